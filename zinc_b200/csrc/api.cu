@@ -30,6 +30,7 @@ struct zc_ctx {
     uint64_t router_mark = 0;            // value of `launches` right after that kernel's last launch (0: never)
     float* merge_scratch = nullptr;      // kMergeScratchFloats f32: a merged attention vector on its way to a matvec
     uint32_t* gemm_flags = nullptr;      // kGemmTileFlags words: tiles of a prefill GEMM that are summed through memory
+    uint8_t* exact_scratch = nullptr;    // kExactScratchBytes: fp16 terms of the activations of a f32-accurate GEMM
     int sm_count = 0;
     // tensor-parallel peer exchange (zc_comm_*)
     zc::CommArgs comm;
@@ -237,7 +238,9 @@ int32_t zc_init(int32_t device, zc_ctx** out_ctx) {
     memset(ctx->status_host, 0, 256);
     ctx->sm_count = prop.multiProcessorCount;
     if (cudaMalloc(reinterpret_cast<void**>(&ctx->scratch_partial), kScratchBytes) != cudaSuccess ||
+        cudaMalloc(reinterpret_cast<void**>(&ctx->exact_scratch), kExactScratchBytes) != cudaSuccess ||
         cudaMemset(ctx->scratch_partial, 0, kScratchBytes) != cudaSuccess) {
+        if (ctx->exact_scratch) cudaFree(ctx->exact_scratch);
         if (ctx->scratch_partial) cudaFree(ctx->scratch_partial);
         cudaFreeHost(ctx->status_host);
         cudaStreamDestroy(ctx->own_stream);
@@ -259,6 +262,7 @@ int32_t zc_destroy(zc_ctx* ctx) {
     zc_comm_destroy(ctx);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
     if (ctx->scratch_partial) cudaFree(ctx->scratch_partial);
+    if (ctx->exact_scratch) cudaFree(ctx->exact_scratch);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
     return ZC_OK;
@@ -785,14 +789,12 @@ int32_t zc_dmmv_batch(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size
     if (num_cols == 0) return fail(ctx, ZC_ERR_INVALID_ARG, "%s: num_cols must be non-zero", fn);
     ZC_TRY(check_vec(ctx, fn, "X", X, x_size, x_offset, (uint64_t)num_cols * K * 4, 16));
     ZC_TRY(check_vec(ctx, fn, "Y", Y, y_size, y_offset, (uint64_t)num_cols * M * 4, 4));
-    cudaError_t e;
-    // Enough columns to amortise tile dequantisation: tensor-core GEMM
-    // (Y[c][M] is D column-major with stride M, X[c][K] is B with stride K).
-    if (num_cols >= 16)
-        e = launch_mul_mm(type, u8(A, a_offset), f32p(X, x_offset), f32m(Y, y_offset), M, num_cols, K, K, M, false,
-                          ctx->status_dev, ctx->gemm_flags, kGemmTileFlags, ctx->stream, &ctx->launches);
-    else
-        e = cudaErrorNotSupported;
+    cudaError_t e = cudaErrorNotSupported;
+    // Y[c][M] is D column-major with stride M, X[c][K] is B with stride K
+    if (num_cols >= 2 && mul_mm_exact_eligible(type, u8(A, a_offset), M, num_cols, K)) {
+        const ExactGemm p{type, u8(A, a_offset), f32p(X, x_offset), f32m(Y, y_offset), M, num_cols, K, K, M, false, ctx->status_dev};
+        e = launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches);
+    }
     if (e == cudaErrorNotSupported)
         e = launch_dmmv_batch(type, u8(A, a_offset), f32p(X, x_offset), f32m(Y, y_offset), M, K, num_cols,
                               ctx->stream, &ctx->launches);
@@ -821,6 +823,11 @@ int32_t zc_mul_mm(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size, co
         mul_mm_cp_async_eligible(type, u8(A, a_offset), Bp, N, K, stride_b))
         e = launch_mul_mm_cp_async(type, u8(A, a_offset), a_size - a_offset, Bp, f32m(D, d_offset * 4), M, N, K,
                                    stride_b, stride_d, ctx->status_dev, ctx->stream, &ctx->launches);
+    if (e == cudaErrorNotSupported && mul_mm_exact_eligible(type, u8(A, a_offset), M, N, K)) {
+        const ExactGemm p{type, u8(A, a_offset), Bp, f32m(D, d_offset * 4), M, N, K, stride_b, stride_d,
+                          act_type == ZC_BF16, ctx->status_dev};
+        e = launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches);
+    }
     if (e == cudaErrorNotSupported)
         e = launch_mul_mm_simple(type, u8(A, a_offset), Bp, f32m(D, d_offset * 4), M, N, K, stride_b, stride_d,
                                  act_type == ZC_BF16, ctx->stream, &ctx->launches);

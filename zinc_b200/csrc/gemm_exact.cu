@@ -1,0 +1,227 @@
+// Preparation of the activations and dispatch of the f32-accurate prefill GEMM (gemm_exact.cuh).
+#include "common.cuh"
+#include "kernels.h"
+
+namespace zc {
+namespace {
+
+constexpr int kPrepThreads = 256;
+
+struct PrepArgs {
+    const void* X;
+    __half* x;          // [N][nblk * 256 * terms]
+    __half* sums;       // [N][nblk * 64], Q4_K / Q5_K
+    float* inv_scale;   // [N]
+    float* D;           // zeroed where tiles are split
+    uint32_t K, nblk, M, stride_b, stride_d;
+    bool sums_on, zero, vec;
+};
+
+// Column of a 64-column group where the two runs of four of chunk c begin: the order in which the type's unpacking
+// yields its weights (gemm_exact.cuh); within a run the order is 0, 2, 1, 3.
+template <int ORDER>
+__device__ __forceinline__ void chunk_columns(int c, uint32_t& a, uint32_t& b) {
+    if (ORDER == 0) {         // Q4_K, Q5_K: low and high nibbles of a word
+        a = 4 * c;
+        b = 32 + 4 * c;
+    } else if (ORDER == 1) {  // Q6_K, Q8_0: two words of a 32-column group
+        a = 32 * (c >> 2) + 8 * (c & 3);
+        b = a + 4;
+    } else {                  // MXFP4: low and high nibbles of a 32-column block
+        a = 32 * (c >> 2) + 4 * (c & 3);
+        b = a + 16;
+    }
+}
+
+template <bool BF16>
+__device__ __forceinline__ float4 load4(const void* row, uint32_t k, uint32_t K, bool vec) {
+    float v[4];
+    if (BF16) {
+        const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(row) + k;
+        if (vec && k + 4 <= K) {
+            const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+            return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16),
+                               __uint_as_float(t.y & 0xFFFF0000u));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = k + i < K ? __bfloat162float(p[i]) : 0.f;
+    } else {
+        const float* p = static_cast<const float*>(row) + k;
+        if (vec && k + 4 <= K) return __ldg(reinterpret_cast<const float4*>(p));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = k + i < K ? p[i] : 0.f;
+    }
+    return make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ uint32_t pack_h2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+// what the fp16 rounding of (a, b) left over
+__device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t h) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&h);
+    return pack_h2(a - __low2float(v), b - __high2float(v));
+}
+
+// One CTA per token: power-of-two scale from the largest element, fp16 terms in the order the GEMM consumes them,
+// sums over 32-column sub-blocks, and (split tiles) the token's row of D set to zero. Bound: the bytes of X, D and
+// the terms, 4 + 4 per element; 4096 x 658: 3 us.
+template <int ORDER, bool BF16>
+__global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    __shared__ float s_max[kPrepThreads / 32];
+    const uint32_t t = blockIdx.x, tid = threadIdx.x;
+    const void* row = static_cast<const uint8_t*>(a.X) + (uint64_t)t * a.stride_b * (BF16 ? 2 : 4);
+    float mx = 0.f;
+    for (uint32_t k = tid * 4; k < a.K; k += kPrepThreads * 4) {
+        const float4 v = load4<BF16>(row, k, a.K, a.vec);
+        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    if ((tid & 31) == 0) s_max[tid >> 5] = mx;
+    if (a.zero) {
+        float* d = a.D + (uint64_t)t * a.stride_d;
+        if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+            for (uint32_t m = tid * 4; m + 4 <= a.M; m += kPrepThreads * 4) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid < (a.M & 3u)) d[(a.M & ~3u) + tid] = 0.f;
+        } else {
+            for (uint32_t m = tid; m < a.M; m += kPrepThreads) d[m] = 0.f;
+        }
+    }
+    __syncthreads();
+    mx = s_max[0];
+#pragma unroll
+    for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, s_max[i]);
+    // largest element to [2^9, 2^10): a sub-block's sum stays below 2^15; the inverse stays a normal number
+    const uint32_t e = __float_as_uint(mx) >> 23;
+    const uint32_t f = min(263u - e, 252u);
+    const float scale = __uint_as_float(f << 23);
+    if (tid == 0) a.inv_scale[t] = __uint_as_float((254u - f) << 23);
+
+    uint4* out = reinterpret_cast<uint4*>(a.x + (uint64_t)t * a.nblk * 256 * (BF16 ? 1 : 2));
+    uint4* sums = reinterpret_cast<uint4*>(a.sums + (uint64_t)t * a.nblk * 64);
+    const uint32_t chunks = a.nblk * 32;
+    for (uint32_t q = tid; q < chunks; q += kPrepThreads) {  // eight lanes per 64-column group, whole warps
+        const uint32_t g = q >> 3;
+        const int c = q & 7;
+        uint32_t ka, kb;
+        chunk_columns<ORDER>(c, ka, kb);
+        float4 va = load4<BF16>(row, g * 64 + ka, a.K, a.vec), vb = load4<BF16>(row, g * 64 + kb, a.K, a.vec);
+        va = make_float4(va.x * scale, va.y * scale, va.z * scale, va.w * scale);
+        vb = make_float4(vb.x * scale, vb.y * scale, vb.z * scale, vb.w * scale);
+        uint4 hi;
+        hi.x = pack_h2(va.x, va.z);
+        hi.y = pack_h2(va.y, va.w);
+        hi.z = pack_h2(vb.x, vb.z);
+        hi.w = pack_h2(vb.y, vb.w);
+        if (BF16) {
+            out[(uint64_t)g * 8 + c] = hi;
+        } else {
+            uint4 lo;
+            lo.x = pack_rest(va.x, va.z, hi.x);
+            lo.y = pack_rest(va.y, va.w, hi.y);
+            lo.z = pack_rest(vb.x, vb.z, hi.z);
+            lo.w = pack_rest(vb.y, vb.w, hi.w);
+            uint4* o = out + (uint64_t)g * 16 + (c >> 2) * 8 + (c & 3);
+            o[0] = hi;
+            o[4] = lo;
+        }
+        if (ORDER == 0 && a.sums_on) {
+            float sa = (va.x + va.y) + (va.z + va.w), sb = (vb.x + vb.y) + (vb.z + vb.w);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                sa += __shfl_xor_sync(0xFFFFFFFFu, sa, o);
+                sb += __shfl_xor_sync(0xFFFFFFFFu, sb, o);
+            }
+            // a block's row: sub-block sums as [high 8][high 8][low 8][zeros 8], against the weights' min terms
+            // [high][low][high][zeros]
+            uint32_t* sp = reinterpret_cast<uint32_t*>(sums + (uint64_t)(g >> 2) * 8) + (g & 3);
+            const uint32_t h = pack_h2(sa, sb);
+            if (c == 0) sp[0] = h;
+            if (c == 1) sp[4] = h;
+            if (c == 2) sp[8] = pack_rest(sa, sb, h);
+            if (c == 3) sp[12] = 0u;
+        }
+    }
+}
+
+template <int ORDER>
+cudaError_t launch_prep(const PrepArgs& a, uint32_t tokens, bool bf16, cudaStream_t s) {
+    if (bf16) exact_prep_kernel<ORDER, true><<<tokens, kPrepThreads, 0, s>>>(a);
+    else exact_prep_kernel<ORDER, false><<<tokens, kPrepThreads, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+    switch (p.type) {
+        case T_Q4_K: return launch_exact_q4k(p, plan, dry, s, grid);
+        case T_Q5_K: return launch_exact_q5k(p, plan, dry, s, grid);
+        case T_Q6_K: return launch_exact_q6k(p, plan, dry, s, grid);
+        case T_Q8_0: return launch_exact_q8(p, plan, dry, s, grid);
+        case T_MXFP4: return launch_exact_mxfp4(p, plan, dry, s, grid);
+        default: return cudaErrorNotSupported;
+    }
+}
+
+}  // namespace
+
+bool mul_mm_exact_eligible(uint32_t type, const uint8_t* A, uint32_t M, uint32_t N, uint32_t K) {
+    if (type != T_Q4_K && type != T_Q5_K && type != T_Q6_K && type != T_Q8_0 && type != T_MXFP4) return false;
+    if (reinterpret_cast<uintptr_t>(A) & 15u) return false;
+    const uint64_t nblk = (K + 255) >> 8;
+    // one token's terms must fit the scratch; unit counts stay in 32 bits
+    return nblk * 256 * 8 < kExactScratchBytes / 64 && ((uint64_t)(M + 255) / 256) * ((N + 31) / 32) * nblk < (1u << 31);
+}
+
+cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaStream_t s, uint64_t* launches) {
+    const uint32_t nblk = (whole.K + 255) >> 8;
+    const bool min_type = whole.type == T_Q4_K || whole.type == T_Q5_K;
+    const size_t per_token = (size_t)nblk * 512 * (whole.bf16 ? 1 : 2) + (min_type ? (size_t)nblk * 128 : 0) + sizeof(float);
+    const uint32_t most = (uint32_t)((kExactScratchBytes - 4096) / per_token) & ~31u;
+    for (uint32_t t0 = 0; t0 < whole.N; t0 += most) {
+        ExactGemm p = whole;
+        p.N = whole.N - t0 < most ? whole.N - t0 : most;
+        p.B = static_cast<const uint8_t*>(whole.B) + (uint64_t)t0 * whole.stride_b * (whole.bf16 ? 2 : 4);
+        p.D = whole.D + (uint64_t)t0 * whole.stride_d;
+        XPlan plan{};
+        plan.nblk = nblk;
+        plan.n_row_pairs = (p.M + 255) / 256;
+        // equal tiles of at most 256 tokens, in steps of 32 (the MMA's N over a CTA pair, eight-row swizzle groups)
+        const uint32_t cols = (p.N + 255) / 256;
+        plan.n_tile = ((p.N + cols - 1) / cols + 31) & ~31u;
+        plan.n_tiles = plan.n_row_pairs * ((p.N + plan.n_tile - 1) / plan.n_tile);
+        uint8_t* q = scratch;
+        plan.x = q;
+        q += (size_t)p.N * nblk * 512 * (p.bf16 ? 1 : 2);
+        plan.sums = q;
+        if (min_type) q += (size_t)p.N * nblk * 128;
+        plan.inv_scale = reinterpret_cast<float*>(q);
+        ExactGrid grid;
+        if (cudaError_t e = launch_type(p, plan, true, s, &grid); e != cudaSuccess) return e;
+        PrepArgs a{};
+        a.X = p.B;
+        a.x = static_cast<__half*>(plan.x);
+        a.sums = static_cast<__half*>(plan.sums);
+        a.inv_scale = plan.inv_scale;
+        a.D = p.D;
+        a.K = p.K;
+        a.nblk = nblk;
+        a.M = p.M;
+        a.stride_b = p.stride_b;
+        a.stride_d = p.stride_d;
+        a.sums_on = min_type;
+        a.zero = grid.split;
+        a.vec = (p.stride_b & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.B) & (p.bf16 ? 7u : 15u)) == 0;
+        const int order = min_type ? 0 : p.type == T_MXFP4 ? 2 : 1;
+        cudaError_t e = order == 0 ? launch_prep<0>(a, p.N, p.bf16, s)
+                        : order == 1 ? launch_prep<1>(a, p.N, p.bf16, s) : launch_prep<2>(a, p.N, p.bf16, s);
+        if (e != cudaSuccess) return e;
+        if ((e = launch_type(p, plan, false, s, &grid)) != cudaSuccess) return e;
+        if (launches) *launches += 2;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace zc

@@ -1,0 +1,847 @@
+// Prefill GEMM with exact weights and f32 (or bf16) activations on the 5th-generation tensor cores:
+// D[n][m] = sum_k W[m][k] * X[n][k], f32 accuracy.
+//
+// The tensor cores take fp16 operands, so both sides are brought to fp16 without losing f32 accuracy:
+//   W  inside a 256-column block a K-quant weight is an integer times the row's d: sc * q (Q4_K 945 at most, Q5_K
+//      1953) is exact in fp16 and the f16 block scale d is applied in f32 afterwards. Q6_K (13 bits) and Q8_0
+//      (d * q over the block's largest power of two, 19 bits) are two exact fp16 terms, the second the rounding
+//      residue of the first. MXFP4 is a power of two times E2M1: exact in one term. A row's min term of Q4_K / Q5_K,
+//      -dmin * m_s * (sum of x over sub-block s), is 32 more columns of the block: (dmin / d) * m_s in two terms
+//      against the sub-block sums of x in two terms.
+//   X  a token is scaled by a power of two (its largest element to [2^9, 2^10)) and split into two fp16 terms: 22
+//      significant bits, absolute error 2^-34 of the token's largest element. bf16 activations are one exact term.
+// Every block is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
+// ("promote") while the next block's MMAs fill the other accumulator.
+//
+// Persistent CTA pairs (cta_group::2, 256 weight rows per pair): tiles of 256 rows x n_tile tokens, their
+// (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over pairs is summed with
+// atomic adds into D, which the preparation kernel zeroes.
+// Bound: tensor pipe (2 or 3 fp16 products per weight and token) from about 100 tokens on; below that the weight
+// bytes and the unpacking of them.
+#pragma once
+
+#include <atomic>
+
+#include "kernels.h"
+#include "tc_common.cuh"
+
+namespace zc {
+namespace {
+
+constexpr int kXThreads = 3 * 32 + 512;  // issuer, loader, spare; sixteen producer warps
+
+template <int TYPE>
+struct XW;  // kTerms: fp16 terms per weight; kBlock: bytes of 256 columns; kBox: bytes a TMA box (or a fetched row) holds
+template <>
+struct XW<T_Q4_K> {
+    static constexpr int kTerms = 1;
+    static constexpr bool kMin = true;
+    static constexpr uint32_t kBlock = 144, kTmaRow = 144, kFetchRow = 176;
+};
+template <>
+struct XW<T_Q5_K> {
+    static constexpr int kTerms = 1;
+    static constexpr bool kMin = true;
+    static constexpr uint32_t kBlock = 176, kTmaRow = 176, kFetchRow = 208;
+};
+template <>
+struct XW<T_Q6_K> {
+    static constexpr int kTerms = 2;
+    static constexpr bool kMin = false;
+    static constexpr uint32_t kBlock = 210, kTmaRow = 240, kFetchRow = 240;
+};
+template <>
+struct XW<T_Q8_0> {
+    static constexpr int kTerms = 2;
+    static constexpr bool kMin = false;
+    static constexpr uint32_t kBlock = 272, kTmaRow = 272, kFetchRow = 304;
+};
+template <>
+struct XW<T_MXFP4> {
+    static constexpr int kTerms = 1;
+    static constexpr bool kMin = false;
+    static constexpr uint32_t kBlock = 136, kTmaRow = 176, kFetchRow = 176;
+};
+
+// Row strides are odd multiples of 16 bytes, so that 16-byte reads of 8 consecutive rows meet no bank twice.
+template <int TYPE, int BN, bool kFetch>
+struct XTile {
+    static constexpr uint32_t kRow = kFetch ? XW<TYPE>::kFetchRow : XW<TYPE>::kTmaRow;
+    static constexpr int kWSlots = 2;
+    static constexpr uint32_t kWBytes = kBM * kRow;
+    static constexpr uint32_t kBBytes = (BN / 2) * 128;  // one step of a CTA's tokens: 128 bytes per token
+    static constexpr uint32_t kMinOffset = kAStages * kABytes;
+    static constexpr uint32_t kWOffset = kMinOffset + (XW<TYPE>::kMin ? kABytes : 0);
+    static constexpr uint32_t kBOffset = kWOffset + ((kWSlots * kWBytes + 1023u) & ~1023u);
+    static constexpr uint32_t kRoom = 232448u - 1024u - 512u - kBOffset;
+    static constexpr int kBSlots = kRoom / kBBytes > 8 ? 8 : kRoom / kBBytes;
+    static_assert(kBSlots >= 3, "activation ring");
+    static constexpr uint32_t kBarOffset = kBOffset + kBSlots * kBBytes;
+    static constexpr uint32_t kSmemBytes = kBarOffset + 512 + 1024;
+};
+
+struct XBars {
+    uint64_t full_a[kAStages], empty_a[kAStages];
+    uint64_t full_m, empty_m;
+    uint64_t full_w[2], empty_w[2];
+    uint64_t full_b[8], empty_b[8];
+    uint64_t accum[2], pfree[2];
+    uint32_t tmem_base;
+    volatile uint32_t failed;
+};
+static_assert(sizeof(XBars) <= 512, "the tiles reserve 512 bytes for the barrier block");
+
+struct XArgs {
+    const uint8_t* A;
+    const uint8_t* a_end;     // first byte past the matrix (fetched rows)
+    float* D;
+    const float* inv_scale;   // [N]: 1 / the token's power of two
+    uint32_t M, N, K, nblk;
+    uint32_t stride_d;
+    uint32_t n_row_pairs, n_tiles, n_tile;  // n_tile tokens per tile (a multiple of 32)
+    uint32_t terms;           // fp16 terms of an activation: 2 (f32) or 1 (bf16)
+    uint32_t* status;
+};
+
+struct XSegment {
+    uint32_t tile, b0, b1;
+};
+__device__ __forceinline__ bool x_next_segment(uint32_t& u, uint32_t u1, uint32_t nblk, XSegment& sg) {
+    if (u >= u1) return false;
+    sg.tile = u / nblk;
+    sg.b0 = u - sg.tile * nblk;
+    sg.b1 = min(nblk, sg.b0 + (u1 - u));
+    u += sg.b1 - sg.b0;
+    return true;
+}
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t rotl(uint32_t v, int r) { return __funnelshift_l(v, v, r & 31); }
+
+// N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p: 16-byte reads (no bank
+// conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four rows per bank), then realigned.
+template <int N>
+__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N]) {
+    constexpr int V = (4 * N + 15 + 15) / 16;
+    uint32_t v[4 * V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
+        v[4 * i] = t.x;
+        v[4 * i + 1] = t.y;
+        v[4 * i + 2] = t.z;
+        v[4 * i + 3] = t.w;
+    }
+    const uint32_t sh = (off & 3u) * 8u;
+    if (off & 8u) {
+#pragma unroll
+        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
+    }
+    if (off & 4u) {
+#pragma unroll
+        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
+}
+
+__device__ __forceinline__ void put_chunk(uint8_t* rowp, int sw, int c, uint4 o) {
+    *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = o;
+}
+
+// 64 columns of Q4_K / Q5_K (w: nibble words, h: the fifth bits' words or unused): chunk i of the stage row holds
+// word i's low nibbles (columns 4i + {0, 2, 1, 3}) and high nibbles (32 + 4i + ...): the order a byte mask yields,
+// which the activations follow. 1024 + q comes from or-ing q into the fp16 pattern of 1024; one fma leaves sc * q.
+template <bool kFive>
+__device__ __forceinline__ void x_deq_k4(const uint32_t (&w)[8], const uint32_t (&h)[8], int j, float s_lo, float s_hi,
+                                         uint8_t* stage, int row) {
+    const __half2 lo = __float2half2_rn(s_lo), lo_c = __float2half2_rn(-1024.f * s_lo);
+    const __half2 hi = __float2half2_rn(s_hi * 0.0625f), hi_c = __float2half2_rn(-64.f * s_hi);
+    uint8_t* rowp = stage + row * 128;
+    const int sw = row & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t a = w[i], b = w[i] >> 8;
+        uint32_t l0 = (a & 0x000F000Fu) | 0x64006400u, l1 = (b & 0x000F000Fu) | 0x64006400u;
+        uint32_t h0 = (a & 0x00F000F0u) | 0x64006400u, h1 = (b & 0x00F000F0u) | 0x64006400u;
+        if constexpr (kFive) {  // bit 2j (low) and 2j + 1 (high) of byte 4i + ... of the qh plane
+            const uint32_t fl = rotl(h[i], 4 - 2 * j), fh = rotl(h[i], 7 - 2 * j);
+            l0 |= fl & 0x00100010u;
+            l1 |= (fl >> 8) & 0x00100010u;
+            h0 |= fh & 0x01000100u;
+            h1 |= rotl(fh, 24) & 0x01000100u;
+        }
+        uint4 o;
+        o.x = h2_bits(__hfma2(bits_h2(l0), lo, lo_c));
+        o.y = h2_bits(__hfma2(bits_h2(l1), lo, lo_c));
+        o.z = h2_bits(__hfma2(bits_h2(h0), hi, hi_c));
+        o.w = h2_bits(__hfma2(bits_h2(h1), hi, hi_c));
+        put_chunk(rowp, sw, i, o);
+    }
+}
+
+// 32 columns as two fp16 terms: chunks 0..3 of the stage row the rounded product v * s, chunks 4..7 its residue.
+// q[i]: the pairs (columns 4i + {0, 2}) and (4i + {1, 3}) as fp16 integers; s: scale of columns 4i .. 4i+3.
+__device__ __forceinline__ void x_put_two(const uint32_t (&q)[16], const __half2 (&s)[8], uint8_t* stage, int row) {
+    uint8_t* rowp = stage + row * 128;
+    const int sw = row & 7;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        uint32_t a[4], r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const __half2 v = bits_h2(q[4 * c + e]), sc = s[2 * c + (e >> 1)];
+            const __half2 p = __hmul2(v, sc);
+            a[e] = h2_bits(p);
+            r[e] = h2_bits(__hfma2(v, sc, __hneg2(p)));
+        }
+        put_chunk(rowp, sw, c, make_uint4(a[0], a[1], a[2], a[3]));
+        put_chunk(rowp, sw, c + 4, make_uint4(r[0], r[1], r[2], r[3]));
+    }
+}
+
+// Columns 32 gg .. of a Q6_K block at p + off (layout: ql[128] qh[64] scales[16] d, element order as dequantRow,
+// src/compute/forward.zig:335-383): half n of the block, low or high nibbles of ql, bit pair of qh.
+__device__ __forceinline__ void x_deq_q6k(const uint8_t* p, uint32_t off, int gg, uint8_t* stage, int row) {
+    const int n = gg >> 2, hi = (gg >> 1) & 1, up = gg & 1;  // columns 128 n + 64 hi + 32 up ..
+    uint32_t ql[8], qh[8];
+    {
+        const uint32_t o = off + 64u * n + 32u * up;
+        lds_words<8>(p + (o & ~15u), o & 15u, ql);
+    }
+    {
+        const uint32_t o = off + 128u + 32u * n;
+        lds_words<8>(p + (o & ~15u), o & 15u, qh);
+    }
+    const uint32_t scw = *reinterpret_cast<const unsigned short*>(p + off + 192u + 8u * n + 4u * hi + 2u * up);
+    const __half2 k1056 = bits_h2(0x64206420u);  // 1024 + 32
+    const __half2 s0 = __float2half2_rn((float)(int)(int8_t)(scw & 0xFFu)), s1 = __float2half2_rn((float)(int)(int8_t)(scw >> 8));
+    const int rot = 4 - 4 * hi - 2 * up;
+    uint32_t q[16];
+    __half2 s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t l = ql[i] >> (4 * hi), t = rotl(qh[i], rot);
+        const uint32_t a = (l & 0x000F000Fu) | (t & 0x00300030u) | 0x64006400u;
+        const uint32_t b = ((l >> 8) & 0x000F000Fu) | ((t >> 8) & 0x00300030u) | 0x64006400u;
+        q[2 * i] = h2_bits(__hsub2(bits_h2(a), k1056));
+        q[2 * i + 1] = h2_bits(__hsub2(bits_h2(b), k1056));
+        s[i] = i < 4 ? s0 : s1;
+    }
+    x_put_two(q, s, stage, row);
+}
+
+// Columns 32 gg .. of eight Q8_0 blocks: block gg at p + off, dn = its d over the row block's power of two.
+__device__ __forceinline__ void x_deq_q8(const uint8_t* p, uint32_t off, float dn, uint8_t* stage, int row) {
+    uint32_t w[8];
+    lds_words<8>(p + (off & ~15u), off & 15u, w);
+    const __half2 k1152 = bits_h2(0x64806480u);  // 1024 + 128
+    const __half2 d2 = __float2half2_rn(dn);
+    uint32_t q[16];
+    __half2 s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t u = w[i] ^ 0x80808080u;
+        q[2 * i] = h2_bits(__hsub2(bits_h2((u & 0x00FF00FFu) | 0x64006400u), k1152));
+        q[2 * i + 1] = h2_bits(__hsub2(bits_h2(((u >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
+        s[i] = d2;
+    }
+    x_put_two(q, s, stage, row);
+}
+
+// One MXFP4 block (16 nibble bytes in q[4]: low nibbles = columns 0..15, high = 16..31) -> chunks c0 .. c0 + 3: the
+// E2M1 bits s|ee|m placed at fp16 bits 15 and 11..9 read as the value times 2^-14; `sc` = 2^14 times the block's
+// power of two.
+__device__ __forceinline__ void x_deq_mx(const uint32_t (&q)[4], __half2 sc, int c0, uint8_t* stage, int row) {
+    uint8_t* rowp = stage + row * 128;
+    const int sw = row & 7;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {  // nibble plane e: (byte 0, 2) low, (1, 3) low, (0, 2) high, (1, 3) high
+            const uint32_t v = e == 0 ? q[i] : e == 1 ? q[i] >> 8 : e == 2 ? q[i] >> 4 : q[i] >> 12;
+            o[e] = h2_bits(__hmul2(bits_h2(((v << 9) & 0x0E000E00u) | ((v << 12) & 0x80008000u)), sc));
+        }
+        put_chunk(rowp, sw, c0 + i, make_uint4(o[0], o[1], o[2], o[3]));
+    }
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+
+template <int TYPE, int BN, bool kFetch>
+__global__ void __launch_bounds__(kXThreads, 1)
+gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_m,
+                  const __grid_constant__ CUtensorMap tmap_w, const XArgs g) {
+    using T = XTile<TYPE, BN, kFetch>;
+    constexpr int kTerms = XW<TYPE>::kTerms;
+    constexpr bool kMin = XW<TYPE>::kMin;
+    constexpr uint32_t kBlock = XW<TYPE>::kBlock, kRow = T::kRow;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* smem_b = smem + T::kBOffset;
+    uint8_t* smem_w = smem + T::kWOffset;
+    XBars* bars = reinterpret_cast<XBars*>(smem + T::kBarOffset);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_ctarank();
+    const uint32_t nblk = g.nblk;
+    const uint32_t U = g.n_tiles * nblk, G = gridDim.x >> 1, slot = blockIdx.x >> 1;
+    const uint32_t u_begin = (uint32_t)part_begin(slot, U, G), u_end = (uint32_t)part_begin(slot + 1, U, G);
+    auto tile_m0 = [&](uint32_t tile) { return ((tile % g.n_row_pairs) * 2 + rank) * (uint32_t)kBM; };
+    auto tile_n0 = [&](uint32_t tile) { return (tile / g.n_row_pairs) * g.n_tile; };
+
+    if (tid == 0) {
+        for (int s = 0; s < kAStages; ++s) {
+            mbar_init(&bars->full_a[s], 8);  // the four producer warps of the owning set, both CTAs
+            mbar_init(&bars->empty_a[s], 1);
+        }
+        mbar_init(&bars->full_m, 32);
+        mbar_init(&bars->empty_m, 1);
+        for (int s = 0; s < T::kBSlots; ++s) {
+            mbar_init(&bars->full_b[s], 2);  // one loader per CTA
+            mbar_init(&bars->empty_b[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&bars->full_w[s], kFetch ? 512 : 1);
+            mbar_init(&bars->empty_w[s], 16);
+            mbar_init(&bars->accum[s], 1);
+            mbar_init(&bars->pfree[s], 32);  // the sixteen producer warps of both CTAs
+        }
+        bars->failed = 0;
+        mbar_fence_init();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
+                     "r"((uint32_t)(2 * BN))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // the peer's barriers exist before anything arrives on them
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+
+    if (warp == 0) {
+        if (lane == 0 && rank == 0) {
+            // ---- MMA issuer (even CTA) ----
+            const uint32_t idesc = (1u << 4) | ((g.n_tile >> 3) << 17) | ((256u >> 4) << 24);  // fp16 x fp16 -> f32
+            const bool two = g.terms == 2;
+            int sb = 0;
+            uint32_t pb = 0;
+            bool ok = true;
+            uint64_t db = 0;
+            auto open_b = [&]() {
+                ok = wait_or_fail<false>(&bars->full_b[sb], pb, bars, g.status, 301);
+                db = smem_desc(smem_u32(smem_b + sb * T::kBBytes));
+                tc_fence_after();
+                return ok;
+            };
+            auto close_b = [&]() {
+                umma_commit_pair(&bars->empty_b[sb]);
+                if (++sb == T::kBSlots) {
+                    sb = 0;
+                    pb ^= 1;
+                }
+            };
+            for (uint32_t gb = 0; gb < u_end - u_begin && ok; ++gb) {
+                const uint32_t d = tmem + (gb & 1) * BN;
+                if (gb >= 2) {
+                    ok = wait_or_fail<false>(&bars->pfree[gb & 1], ((gb >> 1) - 1) & 1, bars, g.status, 302);
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+                constexpr int kSteps = kTerms == 1 ? 4 : 8;
+                for (int st = 0; st < kSteps && ok; ++st) {
+                    const int j = st & 3;
+                    const uint32_t pa = kTerms == 1 ? gb & 1 : (uint32_t)(st >> 2);
+                    ok = wait_or_fail<false>(&bars->full_a[j], pa, bars, g.status, 303);
+                    if (!ok) break;
+                    const uint64_t da = smem_desc(smem_u32(smem + j * kABytes));
+                    const uint32_t acc0 = st > 0 ? 1u : 0u;
+                    if constexpr (kTerms == 1) {
+                        if (two) {
+#pragma unroll
+                            for (int sub = 0; sub < 2; ++sub) {
+                                if (!open_b()) break;
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) {
+                                    umma_bf16_pair(d, da + 4 * sub + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)(sub | k));
+                                    umma_bf16_pair(d, da + 4 * sub + 2 * k, db + 4 + 2 * k, idesc, 1u);
+                                }
+                                close_b();
+                            }
+                        } else if (open_b()) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)k);
+                            close_b();
+                        }
+                    } else {
+                        if (two) {
+                            if (open_b()) {
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) {
+                                    umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)k);
+                                    umma_bf16_pair(d, da + 2 * k, db + 4 + 2 * k, idesc, 1u);
+                                    umma_bf16_pair(d, da + 4 + 2 * k, db + 2 * k, idesc, 1u);
+                                }
+                                close_b();
+                            }
+                        } else if ((st & 1) || open_b()) {  // an activation slot serves two steps
+                            const uint64_t dx = db + 4 * (st & 1);
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                umma_bf16_pair(d, da + 2 * k, dx + 2 * k, idesc, acc0 | (uint32_t)k);
+                                umma_bf16_pair(d, da + 4 + 2 * k, dx + 2 * k, idesc, 1u);
+                            }
+                            if (st & 1) close_b();
+                        }
+                    }
+                    if (!ok) break;
+                    umma_commit_pair(&bars->empty_a[j]);
+                }
+                if constexpr (kMin) {
+                    if (!ok) break;
+                    ok = wait_or_fail<false>(&bars->full_m, gb & 1, bars, g.status, 304);
+                    if (!ok || !open_b()) break;
+                    const uint64_t dm = smem_desc(smem_u32(smem + T::kMinOffset));
+                    umma_bf16_pair(d, dm, db, idesc, 1u);
+                    umma_bf16_pair(d, dm + 2, db + 2, idesc, 1u);
+                    close_b();
+                    umma_commit_pair(&bars->empty_m);
+                }
+                if (!ok) break;
+                umma_commit_pair(&bars->accum[gb & 1]);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // ---- loader of the activations (each CTA its half of a tile's tokens) and, where rows have a 16-byte
+            // pitch, of the raw weight blocks; polls both rings without suspending on either ----
+            const uint32_t steps = (g.terms == 2 ? 8u : 4u) + (kMin ? 1u : 0u);
+            const uint32_t bytes = (g.n_tile / 2) * 128;
+            uint32_t ub = u_begin, uw = u_begin;
+            XSegment bs{0, 0, 0}, ws{0, 0, 0};
+            bool b_live = x_next_segment(ub, u_end, nblk, bs);
+            bool w_live = !kFetch && x_next_segment(uw, u_end, nblk, ws);
+            uint32_t b_b = bs.b0, b_st = 0, w_b = ws.b0;
+            uint32_t b_n0 = tile_n0(bs.tile) + rank * (g.n_tile / 2), w_m0 = tile_m0(ws.tile);
+            int sb = 0, sw = 0;
+            uint32_t pb = 1, pw = 1, idle = 0;
+            bool waited = false;
+            while (b_live || w_live) {
+                bool moved = false;
+                if (w_live && mbar_test_wait(&bars->empty_w[sw], pw)) {
+                    mbar_expect_tx(&bars->full_w[sw], T::kWBytes);
+                    // Q8_0 boxes are wider than 256 bytes: their map counts 16-bit elements
+                    constexpr int kUnit = TYPE == T_Q8_0 ? 2 : 1;
+                    tma_load_2d(smem_w + sw * T::kWBytes, &tmap_w, (int)(((w_b * kBlock) & ~15u) / kUnit), (int)w_m0,
+                                &bars->full_w[sw]);
+                    sw ^= 1;
+                    if (sw == 0) pw ^= 1;
+                    if (++w_b == ws.b1) {
+                        w_live = x_next_segment(uw, u_end, nblk, ws);
+                        w_b = ws.b0;
+                        if (w_live) w_m0 = tile_m0(ws.tile);
+                    }
+                    moved = true;
+                }
+                if (b_live && mbar_test_wait(&bars->empty_b[sb], pb)) {
+                    if (!waited) {  // the weights do not depend on the preparation kernel, the activations do
+                        asm volatile("griddepcontrol.wait;" ::: "memory");
+                        waited = true;
+                    }
+                    const uint32_t fb = leader_addr(&bars->full_b[sb]);
+                    mbar_expect_tx_cluster(fb, bytes);
+                    if (kMin && b_st == steps - 1)
+                        tma_load_2d_pair(smem_b + sb * T::kBBytes, &tmap_m, (int)(b_b * 64), (int)b_n0, fb);
+                    else
+                        tma_load_2d_pair(smem_b + sb * T::kBBytes, &tmap_x,
+                                         (int)((b_b * (steps - (kMin ? 1u : 0u)) + b_st) * 64), (int)b_n0, fb);
+                    if (++sb == T::kBSlots) {
+                        sb = 0;
+                        pb ^= 1;
+                    }
+                    if (++b_st == steps) {
+                        b_st = 0;
+                        if (++b_b == bs.b1) {
+                            b_live = x_next_segment(ub, u_end, nblk, bs);
+                            b_b = bs.b0;
+                            if (b_live) b_n0 = tile_n0(bs.tile) + rank * (g.n_tile / 2);
+                        }
+                    }
+                    moved = true;
+                }
+                if (moved) {
+                    idle = 0;
+                } else {  // bounded like every other wait
+                    __nanosleep(32);
+                    ++idle;
+                    if ((idle & 63u) == 63u && bars->failed) break;
+                    if (idle >= kWaitLimit) {
+                        bars->failed = 1;
+                        if (g.status) {
+                            g.status[0] = 1;
+                            g.status[1] = 305;
+                        }
+                        break;
+                    }
+                }
+            }
+        }
+    } else if (warp >= 3) {
+        // ---- producers: thread = (row, set); the row is the tensor-memory lane the thread promotes, so that a row's
+        // block scale stays in its registers. One-term types: set j owns columns 64 j .. of a block. Two-term types:
+        // columns 32 j .. and 128 + 32 j .., one after the other. ----
+        const int j = (warp - 3) >> 2, row = (warp & 3) * 32 + lane;
+        uint8_t* stage = smem + j * kABytes;
+        const uint32_t full_a = leader_addr(&bars->full_a[j]);
+        const uint32_t pfree0 = leader_addr(&bars->pfree[0]), pfree1 = leader_addr(&bars->pfree[1]);
+        const uint32_t full_m = kMin ? leader_addr(&bars->full_m) : 0u;
+        const uint64_t row_bytes = (uint64_t)(g.K >> 5) * (kBlock / 8);
+        auto row_off = [&](uint32_t tile) {  // rows past M: computed, dropped
+            return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * (TYPE == T_Q8_0 || TYPE == T_MXFP4
+                                                                               ? row_bytes
+                                                                               : (uint64_t)(g.K >> 8) * kBlock);
+        };
+        if constexpr (kMin) {  // columns 24..31 of the min step are zeros
+            if (j == 0) *reinterpret_cast<uint4*>(smem + T::kMinOffset + row * 128 + ((3 ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+        }
+        // fetched rows: thread (row, j) copies pieces j, j + 4, ... of the aligned superset of its row's block
+        uint32_t uf = u_begin, f_b = 0, f_pw = 1;
+        int f_sw = 0;
+        XSegment f_seg{0, 0, 0};
+        bool f_live = false;
+        uint64_t f_off = 0, c_off = 0;
+        auto fetch = [&]() -> bool {
+            if (!f_live) return true;
+            if (!wait_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 306)) return false;
+            const uint64_t o = f_off + (uint64_t)f_b * kBlock;
+            const uint8_t* src = g.A + (o & ~(uint64_t)15);
+            uint8_t* dst = smem_w + f_sw * T::kWBytes + row * kRow;
+            constexpr int kPieces = (kBlock + 15 + 15) / 16;
+            static_assert(!kFetch || kPieces * 16 <= (int)kRow, "a fetched row fits its slot");
+#pragma unroll
+            for (int pc = 0; pc < kPieces; pc += 4) {
+                const int piece = pc + j;
+                if (piece < kPieces) {
+                    const uint8_t* sp = src + piece * 16;
+                    const uint32_t n = sp + 16 <= g.a_end ? 16u : (sp < g.a_end ? (uint32_t)(g.a_end - sp) : 0u);
+                    cp_async16_zfill(dst + piece * 16, n ? sp : g.A, n);
+                }
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[f_sw])) : "memory");
+            f_sw ^= 1;
+            if (f_sw == 0) f_pw ^= 1;
+            if (++f_b == f_seg.b1) {
+                f_live = x_next_segment(uf, u_end, nblk, f_seg);
+                f_b = f_seg.b0;
+                if (f_live) f_off = row_off(f_seg.tile);
+            }
+            return true;
+        };
+        bool ok = true;
+        if constexpr (kFetch) {
+            f_live = x_next_segment(uf, u_end, nblk, f_seg);
+            f_b = f_seg.b0;
+            if (f_live) f_off = row_off(f_seg.tile);
+            ok = fetch();
+        }
+        float acc[BN / 4];
+#pragma unroll
+        for (int i = 0; i < BN / 4; ++i) acc[i] = 0.f;
+        const uint32_t n8 = g.n_tile >> 5;  // groups of 8 columns this set promotes: columns (n_tile / 4) j ..
+        const uint32_t lane_base = ((uint32_t)(warp & 3) * 32u) << 16;
+        uint32_t u = u_begin;
+        XSegment sg{0, 0, 0}, old{0, 0, 0};
+        const uint32_t total = u_end - u_begin;
+        float s_prev = 0.f;
+        uint32_t b = 0;
+        bool fresh = true;
+        for (uint32_t gb = 0; gb <= total && ok; ++gb) {
+            float s_cur = 0.f;
+            const bool boundary = gb > 0 && (gb == total || b == sg.b1);  // the block before this one ended its segment
+            if (boundary) old = sg;
+            if (gb < total) {
+                if (fresh || b == sg.b1) {
+                    x_next_segment(u, u_end, nblk, sg);
+                    b = sg.b0;
+                    fresh = false;
+                    if constexpr (kFetch) c_off = row_off(sg.tile);
+                }
+                const int sw = gb & 1;
+                if (!wait_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 307)) break;
+                if constexpr (kFetch) {
+                    if (!fetch()) break;  // the next block, into the slot the previous one left
+                }
+                const uint8_t* wp = smem_w + sw * T::kWBytes + row * kRow;
+                const uint32_t off = kFetch ? (uint32_t)((c_off + (uint64_t)b * kBlock) & 15u) : (b * kBlock) & 15u;
+                if constexpr (kMin) {  // Q4_K / Q5_K rows and blocks are multiples of 16 bytes: off = 0
+                    const uint4 hd = *reinterpret_cast<const uint4*>(wp);
+                    const uint4 c0 = *reinterpret_cast<const uint4*>(wp + kBlock - 128 + j * 32);
+                    const uint4 c1 = *reinterpret_cast<const uint4*>(wp + kBlock - 112 + j * 32);
+                    uint4 h0 = c0, h1 = c1;
+                    if constexpr (TYPE == T_Q5_K) {
+                        h0 = *reinterpret_cast<const uint4*>(wp + 16);
+                        h1 = *reinterpret_cast<const uint4*>(wp + 32);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                    const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
+                    const float d = __low2float(dd), dmin = __high2float(dd);
+                    // the block's scale is d; where dmin is far above it, dmin / 512, so that the ratio fits fp16
+                    const bool dm_big = fabsf(dmin) > 512.f * fabsf(d);
+                    s_cur = dm_big ? dmin * (1.f / 512.f) : d;
+                    const float ratio = dm_big ? 512.f : (d != 0.f ? dmin / d : 0.f);
+                    const float q_scale = dm_big ? d / s_cur : 1.f;
+                    uint32_t s0, mn0, s1, mn1;
+                    scale_min_k4(2 * j, hd.y, hd.z, hd.w, s0, mn0);
+                    scale_min_k4(2 * j + 1, hd.y, hd.z, hd.w, s1, mn1);
+                    const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+                    const uint32_t h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                    if (!wait_or_fail(&bars->empty_a[j], (gb & 1) ^ 1, bars, g.status, 308)) break;
+                    x_deq_k4<TYPE == T_Q5_K>(w, h, j, q_scale * (float)s0, q_scale * (float)s1, stage, row);
+                    const float v0 = -ratio * (float)mn0, v1 = -ratio * (float)mn1;
+                    const __half2 vh = __floats2half2_rn(v0, v1);
+                    const __half2 vl = __floats2half2_rn(v0 - __low2float(vh), v1 - __high2float(vh));
+                    if (!wait_or_fail(&bars->empty_m, (gb & 1) ^ 1, bars, g.status, 309)) break;
+                    uint8_t* mp = smem + T::kMinOffset + row * 128 + 4 * j;  // chunks 0, 1, 2: high, low, high terms
+                    const int x = row & 7;
+                    *reinterpret_cast<uint32_t*>(mp + ((0 ^ x) << 4)) = h2_bits(vh);
+                    *reinterpret_cast<uint32_t*>(mp + ((1 ^ x) << 4)) = h2_bits(vl);
+                    *reinterpret_cast<uint32_t*>(mp + ((2 ^ x) << 4)) = h2_bits(vh);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive_cluster(full_a);
+                        mbar_arrive_cluster(full_m);
+                    }
+                } else if constexpr (TYPE == T_MXFP4) {
+                    uint32_t emax = 0;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (8 * b + i < (g.K >> 5)) emax = max(emax, (uint32_t)wp[off + 17 * i]);
+                    s_cur = e8m0_to_f32(emax);
+                    uint32_t q[2][4];
+                    __half2 sc[2];
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const uint32_t o = off + 17u * (2 * j + i);
+                        const int diff = (int)emax - (int)wp[o];
+                        lds_words<4>(wp + ((o + 1) & ~15u), (o + 1) & 15u, q[i]);
+                        const bool live = 8 * b + 2 * j + i < (g.K >> 5);
+                        sc[i] = __float2half2_rn(live && diff < 60 ? __uint_as_float((uint32_t)(127 + 14 - diff) << 23) : 0.f);
+                        if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                    if (!wait_or_fail(&bars->empty_a[j], (gb & 1) ^ 1, bars, g.status, 308)) break;
+                    x_deq_mx(q[0], sc[0], 0, stage, row);
+                    x_deq_mx(q[1], sc[1], 4, stage, row);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(full_a);
+                } else {
+                    float up = 1.f;  // Q8_0: 1 / s_cur, a power of two
+                    if constexpr (TYPE == T_Q8_0) {
+                        uint32_t top = 0;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (8 * b + i < (g.K >> 5)) top = max(top, (uint32_t)*reinterpret_cast<const unsigned short*>(wp + off + 34 * i) & 0x7FFFu);
+                        const uint32_t e = __float_as_uint(h2f(top)) >> 23;  // f32 exponent of the largest |d|
+                        s_cur = __uint_as_float(e << 23);
+                        up = e ? __uint_as_float((254u - e) << 23) : 0.f;
+                    } else {
+                        s_cur = h2f(*reinterpret_cast<const unsigned short*>(wp + off + 208));
+                    }
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int gg = j + 4 * hf;
+                        if (!wait_or_fail(&bars->empty_a[j], (uint32_t)hf ^ 1u, bars, g.status, 308)) { ok = false; break; }
+                        if constexpr (TYPE == T_Q6_K) {
+                            x_deq_q6k(wp, off, gg, stage, row);
+                        } else if (8 * b + gg < (g.K >> 5)) {
+                            const uint32_t o = off + 34u * gg;
+                            x_deq_q8(wp, o + 2, h2f(*reinterpret_cast<const unsigned short*>(wp + o)) * up, stage, row);
+                        } else {  // past K
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+                        }
+                        if (hf == 1) {
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                        }
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(full_a);
+                    }
+                    if (!ok) break;
+                }
+                ++b;
+            }
+            if (gb > 0) {
+                // ---- promote the previous block: registers += its scale x its sums ----
+                const uint32_t pv = gb - 1, buf = pv & 1;
+                if (!wait_or_fail(&bars->accum[buf], (pv >> 1) & 1, bars, g.status, 310)) break;
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t ta = tmem + lane_base + buf * BN + j * (g.n_tile >> 2);
+#pragma unroll
+                for (int c = 0; c < BN / 32; c += 2) {
+                    if ((uint32_t)c < n8) {
+                        uint32_t v0[8], v1[8];
+                        tmem_ld8(ta + c * 8, v0);
+                        const bool both = (uint32_t)(c + 1) < n8;
+                        if (both) tmem_ld8(ta + c * 8 + 8, v1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[c * 8 + e] = fmaf(s_prev, __uint_as_float(v0[e]), acc[c * 8 + e]);
+                        if (both) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                acc[c * 8 + 8 + e] = fmaf(s_prev, __uint_as_float(v1[e]), acc[c * 8 + 8 + e]);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(buf ? pfree1 : pfree0);
+                if (boundary) {
+                    // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D ----
+                    asm volatile("griddepcontrol.wait;" ::: "memory");  // D zeroed, scales written
+                    const bool whole = old.b0 == 0 && old.b1 == nblk;
+                    const uint32_t m = tile_m0(old.tile) + row;
+                    const uint32_t n0 = tile_n0(old.tile) + j * (g.n_tile >> 2);
+#pragma unroll
+                    for (int c = 0; c < BN / 4; ++c) {
+                        const uint32_t n = n0 + c;
+                        if ((uint32_t)c < n8 * 8 && n < g.N && m < g.M) {
+                            const float v = acc[c] * __ldcg(g.inv_scale + n);
+                            float* dst = g.D + (uint64_t)n * g.stride_d + m;
+                            if (whole) *dst = v;
+                            else atomicAdd(dst, v);
+                        }
+                        acc[c] = 0.f;
+                    }
+                }
+            }
+            s_prev = s_cur;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * BN)) : "memory");
+    }
+}
+
+// Pairs the device holds at once; every kernel instantiation asks once per device.
+template <typename Kern>
+int x_max_pairs(Kern kern, cudaLaunchConfig_t cfg, std::atomic<int>* cache) {
+    int dev = 0, pairs = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && (pairs = cache[dev].load(std::memory_order_relaxed)) > 0) return pairs;
+    cfg.gridDim = dim3(2, 1, 1);
+    if (cudaOccupancyMaxActiveClusters(&pairs, kern, &cfg) != cudaSuccess || pairs < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (dev < 64) cache[dev].store(pairs, std::memory_order_relaxed);
+    return pairs;
+}
+
+template <int TYPE, int BN, bool kFetch>
+cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+    using T = XTile<TYPE, BN, kFetch>;
+    auto kern = gemm_exact_kernel<TYPE, BN, kFetch>;
+    static std::atomic<uint64_t> attr_done{0};
+    static std::atomic<int> max_pairs[64];
+    if (cudaError_t e = ensure_dynamic_smem(kern, (int)T::kSmemBytes, attr_done); e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kXThreads, 1, 1);
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (dry) {
+        const int pairs = x_max_pairs(kern, cfg, max_pairs);
+        if (pairs < 1) return cudaErrorNotSupported;
+        const uint32_t units = plan.n_tiles * plan.nblk;
+        // whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds
+        uint32_t G = units < (uint32_t)pairs ? units : (uint32_t)pairs;
+        if (plan.n_tiles <= (uint32_t)pairs && plan.n_tiles * 8 >= (uint32_t)pairs * 7) G = plan.n_tiles;
+        grid->pairs = G;
+        grid->split = !(plan.n_tiles % G == 0);
+        return cudaSuccess;
+    }
+    cfg.numAttrs = 2;
+    cfg.gridDim = dim3(2 * grid->pairs, 1, 1);
+    XArgs g{};
+    g.A = p.A;
+    g.a_end = p.A + (uint64_t)p.M * (p.K / block_size(TYPE)) * bytes_per_block(TYPE);
+    g.D = p.D;
+    g.inv_scale = plan.inv_scale;
+    g.M = p.M;
+    g.N = p.N;
+    g.K = p.K;
+    g.nblk = plan.nblk;
+    g.stride_d = p.stride_d;
+    g.n_row_pairs = plan.n_row_pairs;
+    g.n_tiles = plan.n_tiles;
+    g.n_tile = plan.n_tile;
+    g.terms = p.bf16 ? 1u : 2u;
+    g.status = p.status;
+    EncodeFn enc = encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    CUtensorMap mx, mm, mw;
+    const cuuint32_t estr[2] = {1, 1};
+    const cuuint32_t box[2] = {64, plan.n_tile / 2};
+    const cuuint64_t xd[2] = {(cuuint64_t)plan.nblk * 256 * g.terms, p.N}, xs[1] = {(cuuint64_t)plan.nblk * 512 * g.terms};
+    if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, plan.x, xd, xs, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    mm = mx;
+    if constexpr (XW<TYPE>::kMin) {
+        const cuuint64_t md[2] = {(cuuint64_t)plan.nblk * 64, p.N}, ms[1] = {(cuuint64_t)plan.nblk * 128};
+        if (enc(&mm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, plan.sums, md, ms, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    mw = mx;
+    if constexpr (!kFetch) {
+        constexpr int kUnit = TYPE == T_Q8_0 ? 2 : 1;
+        const cuuint64_t row_bytes = (cuuint64_t)plan.nblk * XW<TYPE>::kBlock;
+        const cuuint64_t wd[2] = {row_bytes / kUnit, p.M}, ws[1] = {row_bytes};
+        const cuuint32_t wbox[2] = {XW<TYPE>::kTmaRow / kUnit, kBM};
+        if (enc(&mw, kUnit == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
+                const_cast<uint8_t*>(p.A), wd, ws, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    return cudaLaunchKernelEx(&cfg, kern, mx, mm, mw, g);
+}
+
+template <int TYPE, bool kFetch>
+cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+    if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch>(p, plan, dry, s, grid);
+    if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch>(p, plan, dry, s, grid);
+    return x_launch<TYPE, 256, kFetch>(p, plan, dry, s, grid);
+}
+
+}  // namespace
+}  // namespace zc

@@ -1,0 +1,12 @@
+// Q6_K weights of the f32-accurate prefill GEMM (a translation unit of its own: they compile side by side).
+#include "gemm_exact.cuh"
+
+namespace zc {
+
+cudaError_t launch_exact_q6k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+    // rows have a 16-byte pitch, as a tensor map needs, only where K % 2048 == 0
+    if (p.K & 2047u) return x_launch_bn<T_Q6_K, true>(p, plan, dry, s, grid);
+    return x_launch_bn<T_Q6_K, false>(p, plan, dry, s, grid);
+}
+
+}  // namespace zc

@@ -271,4 +271,35 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
                           uint32_t K, uint32_t stride_b, uint32_t stride_d, bool act_bf16, uint32_t* status,
                           uint32_t* tile_flags, uint32_t n_tile_flags, cudaStream_t s, uint64_t* launches);
 
+// Prefill GEMM at f32 accuracy on the tensor cores (gemm_exact.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4 weights, f32 or
+// bf16 activations. `scratch`: context memory for the fp16 terms of the activations; tokens beyond what it holds go
+// in further passes. cudaErrorNotSupported: the caller takes another path (nothing launched or written).
+constexpr size_t kExactScratchBytes = 64u << 20;
+struct ExactGemm {
+    uint32_t type;
+    const uint8_t* A;
+    const void* B;
+    float* D;
+    uint32_t M, N, K, stride_b, stride_d;
+    bool bf16;
+    uint32_t* status;
+};
+struct XPlan {
+    uint32_t nblk, n_row_pairs, n_tiles, n_tile;
+    void *x, *sums;
+    float* inv_scale;
+};
+struct ExactGrid {
+    uint32_t pairs = 0;
+    bool split = false;
+};
+// one translation unit per weight type; dry: only the grid is computed
+cudaError_t launch_exact_q4k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+cudaError_t launch_exact_q5k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+cudaError_t launch_exact_q6k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+cudaError_t launch_exact_q8(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+cudaError_t launch_exact_mxfp4(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+bool mul_mm_exact_eligible(uint32_t type, const uint8_t* A, uint32_t M, uint32_t N, uint32_t K);
+cudaError_t launch_mul_mm_exact(const ExactGemm& p, uint8_t* scratch, cudaStream_t s, uint64_t* launches);
+
 }  // namespace zc

@@ -186,8 +186,8 @@ __host__ __device__ constexpr uint32_t instr_desc() {
 }
 
 // Bounded wait. kSleep: back off between polls (every role but the tensor-core issuer has slack).
-template <bool kSleep = true>
-__device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, Bars* bars, uint32_t* status,
+template <bool kSleep = true, typename B = Bars>
+__device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, B* bars, uint32_t* status,
                                              uint32_t site) {
     for (uint32_t i = 0; i < kWaitLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
