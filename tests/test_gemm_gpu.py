@@ -193,6 +193,64 @@ def test_mul_mm_mxfp4_block_scaled(gpu, oracle, M, N, K):
     assert rel_l2(got, oracle.gemm_f64(w, t, M, K, Bexact)) <= 1e-5
 
 
+# Relative L2 of the f32-accurate GEMM: 2^-23 for an activation of two fp16 terms, at most 34 tensor-core accumulations
+# of a block and K / 256 f32 additions of 2^-23 each in the worst case, their random sum in practice.
+TOL_EXACT = 5e-6
+
+
+@pytest.mark.parametrize("t,act", [(zb.Q4_K, "f32"), (zb.Q5_K, "f32"), (zb.Q5_K, "bf16"), (zb.Q6_K, "f32"), (zb.Q8_0, "f32"),
+                                   (zb.Q8_0, "bf16"), (zb.MXFP4, "f32")])
+@pytest.mark.parametrize("M,N,K", [(1, 2, 256), (129, 33, 256), (257, 64, 512), (300, 65, 2048), (127, 129, 768),
+                                   (520, 257, 1024), (2050, 17, 2304), (256, 600, 512), (100, 40, 160)])
+def test_mul_mm_exact(gpu, oracle, t, act, M, N, K):
+    """Tile edges in rows and tokens (32, 64, 128, 256), one block, whole and split tiles, block tails past K, rows with
+    and without a 16-byte pitch."""
+    torch, ctx, dd = gpu
+    if K % zb.block_size(t):
+        K = 256
+    g = synth.rng(305, t * 100 + M + N)
+    w = synth.quant_matrix(g, t, M, K)
+    # tokens of very different magnitude: each has a scale of its own
+    X = (synth.activations(g, N, K) * np.exp2(np.arange(N) % 40 - 20)[:, None]).astype(np.float32)
+    if act == "bf16":
+        bits = synth.to_bf16_bits(X)
+        Xd, X = dev(torch, bits.view(np.int16)), synth.bf16_bits_to_f32(bits)
+    else:
+        Xd = dev(torch, X)
+    D = out_with_canary(torch, N * M, init=7.0)
+    wd = dev(torch, w)
+    for _ in range(2):   # the second call finds the context's scratch as the first one left it
+        dd.recordMulMm(t, wd, Xd, D, M, N, K, K, M, act_type=zb.BF16 if act == "bf16" else zb.F32)
+    ctx.submit_and_wait()
+    got = D[:N * M].cpu().numpy().reshape(N, M)
+    want = oracle.gemm_f64(w, t, M, K, X)
+    assert canary_intact(D, N * M)
+    for c in range(N):
+        assert rel_l2(got[c], want[c]) <= (TOL_EXACT if M > 1 else 50 * TOL_EXACT)   # M = 1: one value, cancellation
+
+
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K], ids=["q4_k", "q5_k"])
+def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
+    """Blocks whose d and dmin lie far apart: d = 0, dmin = 0, dmin / d from 2^-14 to 2^17, negative scales."""
+    torch, ctx, dd = gpu
+    M, N, K = 64, 20, 512
+    g = synth.rng(306, t)
+    w = synth.quant_matrix(g, t, M, K).reshape(M * 2, -1)
+    d = np.exp2(-(np.arange(M * 2) % 12)).astype(np.float16) * np.where(np.arange(M * 2) % 5 == 0, -1, 1).astype(np.float16)
+    dmin = np.exp2(np.arange(M * 2) % 17 - 10).astype(np.float16)
+    d[:4], dmin[4:8] = 0, 0
+    d[8:12], dmin[8:12] = np.float16(2.0 ** -14), np.float16(8.0)   # 2^17: the q terms are rounded to 11 bits
+    w[:, 0:2], w[:, 2:4] = d.view(np.uint8).reshape(-1, 2), dmin.view(np.uint8).reshape(-1, 2)
+    X = synth.activations(g, N, K)
+    D = out_with_canary(torch, N * M)
+    dd.recordMulMm(t, dev(torch, w.reshape(-1)), dev(torch, X), D, M, N, K, K, M)
+    ctx.submit_and_wait()
+    got = D[:N * M].cpu().numpy().reshape(N, M)
+    want = oracle.gemm_f64(w.reshape(-1), t, M, K, X)
+    for r in range(M):
+        assert rel_l2(got[:, r], want[:, r]) <= 2 * TOL_EXACT
+
+
 def test_mul_mm_errors(gpu):
     torch, ctx, dd = gpu
     w = torch.zeros(144 * 8, dtype=torch.uint8, device="cuda")

@@ -9,11 +9,11 @@ constexpr int kPrepThreads = 256;
 
 struct PrepArgs {
     const void* X;
-    __half* x;          // [N][nblk * 256 * terms]
+    __half* x;          // [terms][N][nblk * 256]
     __half* sums;       // [N][nblk * 64], Q4_K / Q5_K
     float* inv_scale;   // [N]
     float* D;           // zeroed where tiles are split
-    uint32_t K, nblk, M, stride_b, stride_d;
+    uint32_t tokens, K, nblk, M, stride_b, stride_d;
     bool sums_on, zero, vec;
 };
 
@@ -94,13 +94,14 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
     mx = s_max[0];
 #pragma unroll
     for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, s_max[i]);
-    // largest element to [2^9, 2^10): a sub-block's sum stays below 2^15; the inverse stays a normal number
+    // largest element to [2^4, 2^5): 32 times a sub-block's sum stays below 2^15; the inverse stays a normal number
     const uint32_t e = __float_as_uint(mx) >> 23;
-    const uint32_t f = min(263u - e, 252u);
+    const uint32_t f = min(258u - e, 252u);
     const float scale = __uint_as_float(f << 23);
     if (tid == 0) a.inv_scale[t] = __uint_as_float((254u - f) << 23);
 
-    uint4* out = reinterpret_cast<uint4*>(a.x + (uint64_t)t * a.nblk * 256 * (BF16 ? 1 : 2));
+    uint4* out = reinterpret_cast<uint4*>(a.x + (uint64_t)t * a.nblk * 256);
+    const uint64_t low = (uint64_t)gridDim.x * a.nblk * 32;  // 16-byte chunks to the low term
     uint4* sums = reinterpret_cast<uint4*>(a.sums + (uint64_t)t * a.nblk * 64);
     const uint32_t chunks = a.nblk * 32;
     for (uint32_t q = tid; q < chunks; q += kPrepThreads) {  // eight lanes per 64-column group, whole warps
@@ -116,17 +117,14 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
         hi.y = pack_h2(va.y, va.w);
         hi.z = pack_h2(vb.x, vb.z);
         hi.w = pack_h2(vb.y, vb.w);
-        if (BF16) {
-            out[(uint64_t)g * 8 + c] = hi;
-        } else {
+        out[q] = hi;
+        if (!BF16) {
             uint4 lo;
             lo.x = pack_rest(va.x, va.z, hi.x);
             lo.y = pack_rest(va.y, va.w, hi.y);
             lo.z = pack_rest(vb.x, vb.z, hi.z);
             lo.w = pack_rest(vb.y, vb.w, hi.w);
-            uint4* o = out + (uint64_t)g * 16 + (c >> 2) * 8 + (c & 3);
-            o[0] = hi;
-            o[4] = lo;
+            out[low + q] = lo;
         }
         if (ORDER == 0 && a.sums_on) {
             float sa = (va.x + va.y) + (va.z + va.w), sb = (vb.x + vb.y) + (vb.z + vb.w);
@@ -135,6 +133,8 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
                 sa += __shfl_xor_sync(0xFFFFFFFFu, sa, o);
                 sb += __shfl_xor_sync(0xFFFFFFFFu, sb, o);
             }
+            sa *= 32.f;
+            sb *= 32.f;
             // a block's row: sub-block sums as [high 8][high 8][low 8][zeros 8], against the weights' min terms
             // [high][low][high][zeros]
             uint32_t* sp = reinterpret_cast<uint32_t*>(sums + (uint64_t)(g >> 2) * 8) + (g & 3);
@@ -147,20 +147,21 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
     }
 }
 
-template <int ORDER>
-cudaError_t launch_prep(const PrepArgs& a, uint32_t tokens, bool bf16, cudaStream_t s) {
-    if (bf16) exact_prep_kernel<ORDER, true><<<tokens, kPrepThreads, 0, s>>>(a);
-    else exact_prep_kernel<ORDER, false><<<tokens, kPrepThreads, 0, s>>>(a);
+template <int ORDER, bool BF16>
+cudaError_t launch_prep(const void* args, bool split, cudaStream_t s) {
+    PrepArgs a = *static_cast<const PrepArgs*>(args);
+    a.zero = split;
+    exact_prep_kernel<ORDER, BF16><<<a.tokens, kPrepThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
     switch (p.type) {
-        case T_Q4_K: return launch_exact_q4k(p, plan, dry, s, grid);
-        case T_Q5_K: return launch_exact_q5k(p, plan, dry, s, grid);
-        case T_Q6_K: return launch_exact_q6k(p, plan, dry, s, grid);
-        case T_Q8_0: return launch_exact_q8(p, plan, dry, s, grid);
-        case T_MXFP4: return launch_exact_mxfp4(p, plan, dry, s, grid);
+        case T_Q4_K: return launch_exact_q4k(p, plan, prep, s);
+        case T_Q5_K: return launch_exact_q5k(p, plan, prep, s);
+        case T_Q6_K: return launch_exact_q6k(p, plan, prep, s);
+        case T_Q8_0: return launch_exact_q8(p, plan, prep, s);
+        case T_MXFP4: return launch_exact_mxfp4(p, plan, prep, s);
         default: return cudaErrorNotSupported;
     }
 }
@@ -198,27 +199,25 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         plan.sums = q;
         if (min_type) q += (size_t)p.N * nblk * 128;
         plan.inv_scale = reinterpret_cast<float*>(q);
-        ExactGrid grid;
-        if (cudaError_t e = launch_type(p, plan, true, s, &grid); e != cudaSuccess) return e;
         PrepArgs a{};
         a.X = p.B;
         a.x = static_cast<__half*>(plan.x);
         a.sums = static_cast<__half*>(plan.sums);
         a.inv_scale = plan.inv_scale;
         a.D = p.D;
+        a.tokens = p.N;
         a.K = p.K;
         a.nblk = nblk;
         a.M = p.M;
         a.stride_b = p.stride_b;
         a.stride_d = p.stride_d;
         a.sums_on = min_type;
-        a.zero = grid.split;
         a.vec = (p.stride_b & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.B) & (p.bf16 ? 7u : 15u)) == 0;
         const int order = min_type ? 0 : p.type == T_MXFP4 ? 2 : 1;
-        cudaError_t e = order == 0 ? launch_prep<0>(a, p.N, p.bf16, s)
-                        : order == 1 ? launch_prep<1>(a, p.N, p.bf16, s) : launch_prep<2>(a, p.N, p.bf16, s);
-        if (e != cudaSuccess) return e;
-        if ((e = launch_type(p, plan, false, s, &grid)) != cudaSuccess) return e;
+        const ExactPrep prep{p.bf16 ? (order == 0 ? launch_prep<0, true> : order == 1 ? launch_prep<1, true> : launch_prep<2, true>)
+                                    : (order == 0 ? launch_prep<0, false> : order == 1 ? launch_prep<1, false> : launch_prep<2, false>),
+                             &a};
+        if (cudaError_t e = launch_type(p, plan, prep, s); e != cudaSuccess) return e;
         if (launches) *launches += 2;
     }
     return cudaSuccess;

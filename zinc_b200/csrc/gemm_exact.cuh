@@ -8,8 +8,10 @@
 //      residue of the first. MXFP4 is a power of two times E2M1: exact in one term. A row's min term of Q4_K / Q5_K,
 //      -dmin * m_s * (sum of x over sub-block s), is 32 more columns of the block: (dmin / d) * m_s in two terms
 //      against the sub-block sums of x in two terms.
-//   X  a token is scaled by a power of two (its largest element to [2^9, 2^10)) and split into two fp16 terms: 22
-//      significant bits, absolute error 2^-34 of the token's largest element. bf16 activations are one exact term.
+//   X  a token is scaled by a power of two (its largest element to [2^4, 2^5)) and split into two fp16 terms: 22
+//      significant bits, absolute error 2^-29 of the token's largest element. bf16 activations are one exact term.
+//      (The sub-block sums are scaled up by 2^5 and the min terms down by as much, which leaves dmin / d a range of
+//      2^15 before it no longer fits fp16.)
 // Every block is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
 // ("promote") while the next block's MMAs fill the other accumulator.
 //
@@ -67,24 +69,29 @@ struct XW<T_MXFP4> {
 template <int TYPE, int BN, bool kFetch>
 struct XTile {
     static constexpr uint32_t kRow = kFetch ? XW<TYPE>::kFetchRow : XW<TYPE>::kTmaRow;
+    // With few tokens a block's MMAs are short and the chain unpack -> MMA -> stage free again would set the pace:
+    // every producer set has two stages there (the room the activation slots do not need).
+    static constexpr int kABuf = BN == 64 ? 2 : 1;
     static constexpr int kWSlots = 2;
     static constexpr uint32_t kWBytes = kBM * kRow;
-    static constexpr uint32_t kBBytes = (BN / 2) * 128;  // one step of a CTA's tokens: 128 bytes per token
-    static constexpr uint32_t kMinOffset = kAStages * kABytes;
-    static constexpr uint32_t kWOffset = kMinOffset + (XW<TYPE>::kMin ? kABytes : 0);
+    static constexpr int kPStride = BN == 64 ? 128 : 256;  // tensor-memory columns of one accumulator
+    static constexpr uint32_t kMinOffset = kABuf * kAStages * kABytes;
+    static constexpr uint32_t kMinBytes = kBM * 64;  // 32 columns: 64-byte rows, 64-byte swizzle; two of them
+    static constexpr uint32_t kWOffset = kMinOffset + (XW<TYPE>::kMin ? 2 * kMinBytes : 0);
     static constexpr uint32_t kBOffset = kWOffset + ((kWSlots * kWBytes + 1023u) & ~1023u);
-    static constexpr uint32_t kRoom = 232448u - 1024u - 512u - kBOffset;
-    static constexpr int kBSlots = kRoom / kBBytes > 8 ? 8 : kRoom / kBBytes;
-    static_assert(kBSlots >= 3, "activation ring");
-    static constexpr uint32_t kBarOffset = kBOffset + kBSlots * kBBytes;
-    static constexpr uint32_t kSmemBytes = kBarOffset + 512 + 1024;
+    // The rest is a ring of activation slots of 64 columns of a CTA's n_tile / 2 tokens (128 bytes per token and term):
+    // as many as fit (small tiles need more of them in flight), at most 16.
+    static constexpr uint32_t kSmemBytes = 232448u;
+    static constexpr uint32_t kBRoom = kSmemBytes - 1024u - 512u - kBOffset;
+    static_assert(kBRoom >= 2 * BN * 128, "two slots of the widest tile");
+    static constexpr uint32_t kBarOffset = kBOffset + kBRoom;
 };
 
 struct XBars {
-    uint64_t full_a[kAStages], empty_a[kAStages];
-    uint64_t full_m, empty_m;
+    uint64_t full_a[2 * kAStages], empty_a[2 * kAStages];
+    uint64_t full_m[2], empty_m[2];
     uint64_t full_w[2], empty_w[2];
-    uint64_t full_b[8], empty_b[8];
+    uint64_t full_b[16], empty_b[16];
     uint64_t accum[2], pfree[2];
     uint32_t tmem_base;
     volatile uint32_t failed;
@@ -268,6 +275,28 @@ __device__ __forceinline__ void x_deq_mx(const uint32_t (&q)[4], __half2 sc, int
     }
 }
 
+// acc += s * v, two at a time
+__device__ __forceinline__ void fma_f32x2(float2& acc, float s, float v0, float v1) {
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %2};\n\tmov.b64 b, {%3, %4};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc.x), "+f"(acc.y)
+        : "f"(s), "f"(v0), "f"(v1));
+}
+// Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_64(uint32_t saddr) {
+    const uint32_t lo = ((saddr >> 4) & 0x3FFFu) | (1u << 16);
+    const uint32_t hi = (512u >> 4) | (1u << 14) | (4u << 29);
+    return ((uint64_t)hi << 32) | lo;
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
@@ -295,22 +324,24 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const uint32_t u_begin = (uint32_t)part_begin(slot, U, G), u_end = (uint32_t)part_begin(slot + 1, U, G);
     auto tile_m0 = [&](uint32_t tile) { return ((tile % g.n_row_pairs) * 2 + rank) * (uint32_t)kBM; };
     auto tile_n0 = [&](uint32_t tile) { return (tile / g.n_row_pairs) * g.n_tile; };
+    const uint32_t b_bytes = g.n_tile * 64 * g.terms;  // an activation slot
+    const uint32_t b_slots = min(T::kBRoom / b_bytes, 16u);
 
     if (tid == 0) {
-        for (int s = 0; s < kAStages; ++s) {
+        for (int s = 0; s < T::kABuf * kAStages; ++s) {
             mbar_init(&bars->full_a[s], 8);  // the four producer warps of the owning set, both CTAs
             mbar_init(&bars->empty_a[s], 1);
         }
-        mbar_init(&bars->full_m, 32);
-        mbar_init(&bars->empty_m, 1);
-        for (int s = 0; s < T::kBSlots; ++s) {
-            mbar_init(&bars->full_b[s], 2);  // one loader per CTA
+        for (uint32_t s = 0; s < b_slots; ++s) {
+            mbar_init(&bars->full_b[s], 1);  // the even CTA's loader expects the bytes of both CTAs
             mbar_init(&bars->empty_b[s], 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars->full_w[s], kFetch ? 512 : 1);
             mbar_init(&bars->empty_w[s], 16);
             mbar_init(&bars->accum[s], 1);
+            mbar_init(&bars->full_m[s], 32);
+            mbar_init(&bars->empty_m[s], 1);
             mbar_init(&bars->pfree[s], 32);  // the sixteen producer warps of both CTAs
         }
         bars->failed = 0;
@@ -318,7 +349,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                     "r"((uint32_t)(2 * BN))
+                     "r"((uint32_t)(2 * T::kPStride))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -329,169 +360,154 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const uint32_t tmem = bars->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0 && rank == 0) {
-            // ---- MMA issuer (even CTA) ----
-            const uint32_t idesc = (1u << 4) | ((g.n_tile >> 3) << 17) | ((256u >> 4) << 24);  // fp16 x fp16 -> f32
-            const bool two = g.terms == 2;
-            int sb = 0;
-            uint32_t pb = 0;
+        if (rank == 0) {
+            // ---- MMA issuer (even CTA). Two-term activations: up to 128 tokens the terms lie side by side on the MMA's
+            // N (half the instructions; an instruction costs the issuer some 70 cycles whatever its N), above that they
+            // are two instructions into the same columns. ----
+            const bool two = g.terms == 2, merged = two && g.n_tile <= 128;
+            const uint32_t n_mma = merged ? 2 * g.n_tile : g.n_tile;
+            const uint32_t idesc = (1u << 4) | ((n_mma >> 3) << 17) | ((256u >> 4) << 24);  // fp16 x fp16 -> f32
+            const uint32_t lo = two && !merged ? (g.n_tile / 2) * 128 / 16 : 0;  // descriptor step to the low terms
+            const uint32_t full_a = smem_u32(bars->full_a), full_b = smem_u32(bars->full_b);
+            const uint64_t desc_a = smem_desc(smem_u32(smem)), desc_b = smem_desc(smem_u32(smem_b));
+            uint32_t sb = 0, pb = 0;
             bool ok = true;
-            uint64_t db = 0;
-            auto open_b = [&]() {
-                ok = wait_or_fail<false>(&bars->full_b[sb], pb, bars, g.status, 301);
-                db = smem_desc(smem_u32(smem_b + sb * T::kBBytes));
-                tc_fence_after();
-                return ok;
-            };
-            auto close_b = [&]() {
-                umma_commit_pair(&bars->empty_b[sb]);
-                if (++sb == T::kBSlots) {
-                    sb = 0;
-                    pb ^= 1;
-                }
-            };
-            for (uint32_t gb = 0; gb < u_end - u_begin && ok; ++gb) {
-                const uint32_t d = tmem + (gb & 1) * BN;
-                if (gb >= 2) {
-                    ok = wait_or_fail<false>(&bars->pfree[gb & 1], ((gb >> 1) - 1) & 1, bars, g.status, 302);
+            const uint32_t total = u_end - u_begin;
+            for (uint32_t gb = 0; gb < total && ok; ++gb) {
+                const uint32_t d = tmem + (gb & 1) * T::kPStride;
+                uint64_t db = 0;
+                constexpr int kSteps = kTerms == 1 ? 4 : 8;
+#pragma unroll
+                for (int st = 0; st < kSteps; ++st) {
+                    // fill number f of set st % 4; its stage f % kABuf
+                    const uint32_t f = kTerms == 1 ? gb : 2 * gb + (st >> 2);
+                    const uint32_t sa = (st & 3) * T::kABuf + f % T::kABuf;
+                    const bool open = kTerms == 1 || (st & 1) == 0;  // an activation slot serves two 32-column steps
+                    const bool close = kTerms == 1 || (st & 1) == 1;
+                    // lane 0 watches the weight stage, lane 1 the activation slot, lane 2 the accumulator
+                    uint32_t bar = full_a + sa * 8, par = (f / T::kABuf) & 1;
+                    if (open && lane == 1) {
+                        bar = full_b + sb * 8;
+                        par = pb;
+                    }
+                    if (st == 0 && lane == 2 && gb >= 2) {
+                        bar = smem_u32(&bars->pfree[gb & 1]);
+                        par = ((gb >> 1) - 1) & 1;
+                    }
+                    ok = warp_poll(bar, par, bars, g.status, 301);
                     if (!ok) break;
                     tc_fence_after();
-                }
-                constexpr int kSteps = kTerms == 1 ? 4 : 8;
-                for (int st = 0; st < kSteps && ok; ++st) {
-                    const int j = st & 3;
-                    const uint32_t pa = kTerms == 1 ? gb & 1 : (uint32_t)(st >> 2);
-                    ok = wait_or_fail<false>(&bars->full_a[j], pa, bars, g.status, 303);
-                    if (!ok) break;
-                    const uint64_t da = smem_desc(smem_u32(smem + j * kABytes));
-                    const uint32_t acc0 = st > 0 ? 1u : 0u;
-                    if constexpr (kTerms == 1) {
-                        if (two) {
+                    if (open) db = desc_b + sb * (b_bytes >> 4);
+                    if (elect_one()) {
+                        const uint64_t da = desc_a + sa * (kABytes >> 4);
+                        if constexpr (kTerms == 1) {
 #pragma unroll
-                            for (int sub = 0; sub < 2; ++sub) {
-                                if (!open_b()) break;
-#pragma unroll
-                                for (int k = 0; k < 2; ++k) {
-                                    umma_bf16_pair(d, da + 4 * sub + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)(sub | k));
-                                    umma_bf16_pair(d, da + 4 * sub + 2 * k, db + 4 + 2 * k, idesc, 1u);
-                                }
-                                close_b();
+                            for (int k = 0; k < 4; ++k) {
+                                umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, (uint32_t)(st | k));
+                                if (lo) umma_bf16_pair(d, da + 2 * k, db + lo + 2 * k, idesc, 1u);
                             }
-                        } else if (open_b()) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)k);
-                            close_b();
-                        }
-                    } else {
-                        if (two) {
-                            if (open_b()) {
-#pragma unroll
-                                for (int k = 0; k < 2; ++k) {
-                                    umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, acc0 | (uint32_t)k);
-                                    umma_bf16_pair(d, da + 2 * k, db + 4 + 2 * k, idesc, 1u);
-                                    umma_bf16_pair(d, da + 4 + 2 * k, db + 2 * k, idesc, 1u);
-                                }
-                                close_b();
-                            }
-                        } else if ((st & 1) || open_b()) {  // an activation slot serves two steps
+                        } else {
                             const uint64_t dx = db + 4 * (st & 1);
 #pragma unroll
                             for (int k = 0; k < 2; ++k) {
-                                umma_bf16_pair(d, da + 2 * k, dx + 2 * k, idesc, acc0 | (uint32_t)k);
+                                umma_bf16_pair(d, da + 2 * k, dx + 2 * k, idesc, (uint32_t)(st | k));
                                 umma_bf16_pair(d, da + 4 + 2 * k, dx + 2 * k, idesc, 1u);
+                                if (lo) umma_bf16_pair(d, da + 2 * k, dx + lo + 2 * k, idesc, 1u);
                             }
-                            if (st & 1) close_b();
                         }
+                        umma_commit_pair(&bars->empty_a[sa]);
+                        if (close) umma_commit_pair(&bars->empty_b[sb]);
+                        if (!kMin && st == kSteps - 1) umma_commit_pair(&bars->accum[gb & 1]);
                     }
-                    if (!ok) break;
-                    umma_commit_pair(&bars->empty_a[j]);
-                }
-                if constexpr (kMin) {
-                    if (!ok) break;
-                    ok = wait_or_fail<false>(&bars->full_m, gb & 1, bars, g.status, 304);
-                    if (!ok || !open_b()) break;
-                    const uint64_t dm = smem_desc(smem_u32(smem + T::kMinOffset));
-                    umma_bf16_pair(d, dm, db, idesc, 1u);
-                    umma_bf16_pair(d, dm + 2, db + 2, idesc, 1u);
-                    close_b();
-                    umma_commit_pair(&bars->empty_m);
-                }
-                if (!ok) break;
-                umma_commit_pair(&bars->accum[gb & 1]);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- loader of the activations (each CTA its half of a tile's tokens) and, where rows have a 16-byte
-            // pitch, of the raw weight blocks; polls both rings without suspending on either ----
-            const uint32_t steps = (g.terms == 2 ? 8u : 4u) + (kMin ? 1u : 0u);
-            const uint32_t bytes = (g.n_tile / 2) * 128;
-            uint32_t ub = u_begin, uw = u_begin;
-            XSegment bs{0, 0, 0}, ws{0, 0, 0};
-            bool b_live = x_next_segment(ub, u_end, nblk, bs);
-            bool w_live = !kFetch && x_next_segment(uw, u_end, nblk, ws);
-            uint32_t b_b = bs.b0, b_st = 0, w_b = ws.b0;
-            uint32_t b_n0 = tile_n0(bs.tile) + rank * (g.n_tile / 2), w_m0 = tile_m0(ws.tile);
-            int sb = 0, sw = 0;
-            uint32_t pb = 1, pw = 1, idle = 0;
-            bool waited = false;
-            while (b_live || w_live) {
-                bool moved = false;
-                if (w_live && mbar_test_wait(&bars->empty_w[sw], pw)) {
-                    mbar_expect_tx(&bars->full_w[sw], T::kWBytes);
-                    // Q8_0 boxes are wider than 256 bytes: their map counts 16-bit elements
-                    constexpr int kUnit = TYPE == T_Q8_0 ? 2 : 1;
-                    tma_load_2d(smem_w + sw * T::kWBytes, &tmap_w, (int)(((w_b * kBlock) & ~15u) / kUnit), (int)w_m0,
-                                &bars->full_w[sw]);
-                    sw ^= 1;
-                    if (sw == 0) pw ^= 1;
-                    if (++w_b == ws.b1) {
-                        w_live = x_next_segment(uw, u_end, nblk, ws);
-                        w_b = ws.b0;
-                        if (w_live) w_m0 = tile_m0(ws.tile);
-                    }
-                    moved = true;
-                }
-                if (b_live && mbar_test_wait(&bars->empty_b[sb], pb)) {
-                    if (!waited) {  // the weights do not depend on the preparation kernel, the activations do
-                        asm volatile("griddepcontrol.wait;" ::: "memory");
-                        waited = true;
-                    }
-                    const uint32_t fb = leader_addr(&bars->full_b[sb]);
-                    mbar_expect_tx_cluster(fb, bytes);
-                    if (kMin && b_st == steps - 1)
-                        tma_load_2d_pair(smem_b + sb * T::kBBytes, &tmap_m, (int)(b_b * 64), (int)b_n0, fb);
-                    else
-                        tma_load_2d_pair(smem_b + sb * T::kBBytes, &tmap_x,
-                                         (int)((b_b * (steps - (kMin ? 1u : 0u)) + b_st) * 64), (int)b_n0, fb);
-                    if (++sb == T::kBSlots) {
+                    if (close && ++sb == b_slots) {
                         sb = 0;
                         pb ^= 1;
                     }
-                    if (++b_st == steps) {
-                        b_st = 0;
-                        if (++b_b == bs.b1) {
-                            b_live = x_next_segment(ub, u_end, nblk, bs);
-                            b_b = bs.b0;
-                            if (b_live) b_n0 = tile_n0(bs.tile) + rank * (g.n_tile / 2);
-                        }
-                    }
-                    moved = true;
                 }
-                if (moved) {
-                    idle = 0;
-                } else {  // bounded like every other wait
-                    __nanosleep(32);
-                    ++idle;
-                    if ((idle & 63u) == 63u && bars->failed) break;
-                    if (idle >= kWaitLimit) {
-                        bars->failed = 1;
-                        if (g.status) {
-                            g.status[0] = 1;
-                            g.status[1] = 305;
-                        }
-                        break;
+                if constexpr (kMin) {  // merged: these columns hold the sums' terms; the low-term columns see zeros
+                    if (!ok) break;
+                    ok = warp_poll(lane == 1 ? full_b + sb * 8 : smem_u32(&bars->full_m[gb & 1]), lane == 1 ? pb : (gb >> 1) & 1, bars,
+                                   g.status, 304);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint64_t dm = smem_desc_64(smem_u32(smem + T::kMinOffset + (gb & 1) * T::kMinBytes));
+                        const uint64_t ds = desc_b + sb * (b_bytes >> 4);
+                        umma_bf16_pair(d, dm, ds, idesc, 1u);
+                        umma_bf16_pair(d, dm + 2, ds + 2, idesc, 1u);
+                        umma_commit_pair(&bars->empty_m[gb & 1]);
+                        umma_commit_pair(&bars->empty_b[sb]);
+                        umma_commit_pair(&bars->accum[gb & 1]);
                     }
+                    if (++sb == b_slots) {
+                        sb = 0;
+                        pb ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- loader of the activations (each CTA its half of a tile's tokens): lane l serves slot l, so that every free
+        // slot is seen in one round of polls ----
+        constexpr uint32_t steps = 4u + (kMin ? 1u : 0u);
+        const uint32_t half = (g.n_tile / 2) * 128;
+        const bool merged = g.terms == 2 && g.n_tile <= 128;
+        const uint32_t fills = (u_end - u_begin) * steps;
+        const uint32_t full = smem_u32(&bars->full_b[lane & 15]), full_lead = leader_addr(&bars->full_b[lane & 15]);
+        const uint32_t empty = smem_u32(&bars->empty_b[lane & 15]);
+        uint8_t* dst = smem_b + (lane & 15) * b_bytes;
+        uint32_t f = (uint32_t)lane < b_slots ? (uint32_t)lane : fills, par = 1, idle = 0;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        while (__any_sync(0xFFFFFFFFu, f < fills)) {
+            const bool go = f < fills && mbar_test_addr(empty, par);
+            if (go) {
+                const uint32_t blk = f / steps, st = f - blk * steps, u = u_begin + blk, tile = u / nblk, b = u - tile * nblk;
+                const int n0 = (int)(tile_n0(tile) + rank * (g.n_tile / 2));
+                const bool sums = kMin && st == 4, both = g.terms == 2 && (merged || !sums);
+                if (rank == 0)  // the bytes of both CTAs
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(both ? 4 * half : 2 * half) : "memory");
+                if (sums) {  // merged: the low-term columns get rows past the sums, zeros
+                    tma_load_2d_pair(dst, &tmap_m, (int)(b * 64), n0, full_lead);
+                    if (both) tma_load_2d_pair(dst + half, &tmap_m, (int)(b * 64), (int)g.N, full_lead);
+                } else {
+                    tma_load_2d_pair(dst, &tmap_x, (int)((b * 4 + st) * 64), n0, full_lead);
+                    if (both) tma_load_2d_pair(dst + half, &tmap_x, (int)((b * 4 + st) * 64), (int)g.N + n0, full_lead);
+                }
+                f += b_slots;
+                par ^= 1;
+            }
+            if (__any_sync(0xFFFFFFFFu, go)) {
+                idle = 0;
+            } else {  // bounded like every other wait
+                ++idle;
+                if ((idle & 255u) == 255u && __any_sync(0xFFFFFFFFu, bars->failed != 0)) break;
+                if (idle >= 16u * kWaitLimit) {
+                    bars->failed = 1;
+                    if (g.status) {
+                        g.status[0] = 1;
+                        g.status[1] = 305;
+                    }
+                    break;
+                }
+            }
+        }
+    } else if (warp == 2) {
+        if (!kFetch && lane == 0) {
+            // ---- loader of the raw weight blocks, where rows have a 16-byte pitch. The weights do not depend on the
+            // preparation kernel: they arrive and are unpacked while it still runs. ----
+            uint32_t u = u_begin, i = 0;
+            XSegment ws{0, 0, 0};
+            bool ok = true;
+            while (ok && x_next_segment(u, u_end, nblk, ws)) {
+                const int m0 = (int)tile_m0(ws.tile);
+                for (uint32_t b = ws.b0; b < ws.b1; ++b, ++i) {
+                    const int sw = i & 1;
+                    ok = wait_or_fail(&bars->empty_w[sw], ((i >> 1) & 1) ^ 1, bars, g.status, 311);
+                    if (!ok) break;
+                    mbar_expect_tx(&bars->full_w[sw], T::kWBytes);
+                    // Q8_0 boxes are wider than 256 bytes: their map counts 16-bit elements
+                    constexpr int kUnit = TYPE == T_Q8_0 ? 2 : 1;
+                    tma_load_2d(smem_w + sw * T::kWBytes, &tmap_w, (int)(((b * kBlock) & ~15u) / kUnit), m0, &bars->full_w[sw]);
                 }
             }
         }
@@ -500,10 +516,10 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // block scale stays in its registers. One-term types: set j owns columns 64 j .. of a block. Two-term types:
         // columns 32 j .. and 128 + 32 j .., one after the other. ----
         const int j = (warp - 3) >> 2, row = (warp & 3) * 32 + lane;
-        uint8_t* stage = smem + j * kABytes;
-        const uint32_t full_a = leader_addr(&bars->full_a[j]);
+        const bool merged = g.terms == 2 && g.n_tile <= 128;
+        const uint32_t full_a0 = leader_addr(&bars->full_a[j * T::kABuf]);
         const uint32_t pfree0 = leader_addr(&bars->pfree[0]), pfree1 = leader_addr(&bars->pfree[1]);
-        const uint32_t full_m = kMin ? leader_addr(&bars->full_m) : 0u;
+        const uint32_t full_m = kMin ? leader_addr(&bars->full_m[0]) : 0u;
         const uint64_t row_bytes = (uint64_t)(g.K >> 5) * (kBlock / 8);
         auto row_off = [&](uint32_t tile) {  // rows past M: computed, dropped
             return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * (TYPE == T_Q8_0 || TYPE == T_MXFP4
@@ -511,7 +527,9 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                                                                                : (uint64_t)(g.K >> 8) * kBlock);
         };
         if constexpr (kMin) {  // columns 24..31 of the min step are zeros
-            if (j == 0) *reinterpret_cast<uint4*>(smem + T::kMinOffset + row * 128 + ((3 ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+            if (j < 2)
+                *reinterpret_cast<uint4*>(smem + T::kMinOffset + j * T::kMinBytes + row * 64 + ((3 ^ ((row >> 1) & 3)) << 4)) =
+                    make_uint4(0, 0, 0, 0);
         }
         // fetched rows: thread (row, j) copies pieces j, j + 4, ... of the aligned superset of its row's block
         uint32_t uf = u_begin, f_b = 0, f_pw = 1;
@@ -521,7 +539,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         uint64_t f_off = 0, c_off = 0;
         auto fetch = [&]() -> bool {
             if (!f_live) return true;
-            if (!wait_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 306)) return false;
+            if (!poll_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 306)) return false;
             const uint64_t o = f_off + (uint64_t)f_b * kBlock;
             const uint8_t* src = g.A + (o & ~(uint64_t)15);
             uint8_t* dst = smem_w + f_sw * T::kWBytes + row * kRow;
@@ -553,9 +571,9 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (f_live) f_off = row_off(f_seg.tile);
             ok = fetch();
         }
-        float acc[BN / 4];
+        float2 acc[BN / 8];
 #pragma unroll
-        for (int i = 0; i < BN / 4; ++i) acc[i] = 0.f;
+        for (int i = 0; i < BN / 8; ++i) acc[i] = make_float2(0.f, 0.f);
         const uint32_t n8 = g.n_tile >> 5;  // groups of 8 columns this set promotes: columns (n_tile / 4) j ..
         const uint32_t lane_base = ((uint32_t)(warp & 3) * 32u) << 16;
         uint32_t u = u_begin;
@@ -576,12 +594,18 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     if constexpr (kFetch) c_off = row_off(sg.tile);
                 }
                 const int sw = gb & 1;
-                if (!wait_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 307)) break;
+                if (!poll_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 307)) break;
                 if constexpr (kFetch) {
                     if (!fetch()) break;  // the next block, into the slot the previous one left
                 }
                 const uint8_t* wp = smem_w + sw * T::kWBytes + row * kRow;
                 const uint32_t off = kFetch ? (uint32_t)((c_off + (uint64_t)b * kBlock) & 15u) : (b * kBlock) & 15u;
+                // one-term types: fill number gb of the set, two-term types: 2 gb and 2 gb + 1
+                const int ab = T::kABuf == 1 ? 0 : (int)(gb & 1);
+                uint8_t* stage = smem + (j * T::kABuf + ab) * kABytes;
+                uint64_t* empty_a = &bars->empty_a[j * T::kABuf + ab];
+                const uint32_t pa = ((gb / T::kABuf) & 1) ^ 1;
+                const uint32_t full_a = full_a0 + ab * 8;
                 if constexpr (kMin) {  // Q4_K / Q5_K rows and blocks are multiples of 16 bytes: off = 0
                     const uint4 hd = *reinterpret_cast<const uint4*>(wp);
                     const uint4 c0 = *reinterpret_cast<const uint4*>(wp + kBlock - 128 + j * 32);
@@ -595,24 +619,45 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
                     const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
                     const float d = __low2float(dd), dmin = __high2float(dd);
-                    // the block's scale is d; where dmin is far above it, dmin / 512, so that the ratio fits fp16
-                    const bool dm_big = fabsf(dmin) > 512.f * fabsf(d);
-                    s_cur = dm_big ? dmin * (1.f / 512.f) : d;
-                    const float ratio = dm_big ? 512.f : (d != 0.f ? dmin / d : 0.f);
-                    const float q_scale = dm_big ? d / s_cur : 1.f;
-                    uint32_t s0, mn0, s1, mn1;
-                    scale_min_k4(2 * j, hd.y, hd.z, hd.w, s0, mn0);
-                    scale_min_k4(2 * j + 1, hd.y, hd.z, hd.w, s1, mn1);
+                    // the block's scale is d; where dmin is far above it (and there are mins at all), dmin / 2^15, so that
+                    // the ratio fits fp16: the q terms, at most 945 / 2^15 of a min term there, are then rounded
+                    float ratio = 0.f, q_scale = 1.f;
+                    s_cur = d;
+                    if (fabsf(dmin) > 32768.f * fabsf(d)) {
+                        if (((hd.z | (hd.w & 0xF0F0F0F0u)) != 0u)) {
+                            s_cur = dmin * (1.f / 32768.f);
+                            ratio = 32768.f;
+                            q_scale = d / s_cur;
+                        }
+                    } else if (d != 0.f) {  // dmin / d: an approximate reciprocal and a Newton step
+                        const float r = __fdividef(1.f, d);
+                        ratio = dmin * fmaf(fmaf(-d, r, 1.f), r, r);
+                    }
+                    ratio *= -1.f / 32.f;
+                    // the 6-bit scales and mins of sub-blocks 2j and 2j + 1 (getScaleMinK4, src/compute/forward.zig:229-238),
+                    // four at a time as bytes
+                    uint32_t scw, mnw;
+                    if (j < 2) {
+                        scw = hd.y & 0x3F3F3F3Fu;
+                        mnw = hd.z & 0x3F3F3F3Fu;
+                    } else {
+                        scw = (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u);
+                        mnw = ((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u);
+                    }
+                    scw >>= 16 * (j & 1);
+                    mnw >>= 16 * (j & 1);
+                    const uint32_t s0 = scw & 0xFFu, s1 = (scw >> 8) & 0xFFu, mn0 = mnw & 0xFFu, mn1 = (mnw >> 8) & 0xFFu;
                     const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                     const uint32_t h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    if (!wait_or_fail(&bars->empty_a[j], (gb & 1) ^ 1, bars, g.status, 308)) break;
+                    if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
                     x_deq_k4<TYPE == T_Q5_K>(w, h, j, q_scale * (float)s0, q_scale * (float)s1, stage, row);
-                    const float v0 = -ratio * (float)mn0, v1 = -ratio * (float)mn1;
+                    const float v0 = ratio * (float)mn0, v1 = ratio * (float)mn1;
                     const __half2 vh = __floats2half2_rn(v0, v1);
                     const __half2 vl = __floats2half2_rn(v0 - __low2float(vh), v1 - __high2float(vh));
-                    if (!wait_or_fail(&bars->empty_m, (gb & 1) ^ 1, bars, g.status, 309)) break;
-                    uint8_t* mp = smem + T::kMinOffset + row * 128 + 4 * j;  // chunks 0, 1, 2: high, low, high terms
-                    const int x = row & 7;
+                    if (!poll_or_fail(&bars->empty_m[gb & 1], ((gb >> 1) & 1) ^ 1, bars, g.status, 309)) break;
+                    // chunks 0, 1, 2: high, low, high terms
+                    uint8_t* mp = smem + T::kMinOffset + (gb & 1) * T::kMinBytes + row * 64 + 4 * j;
+                    const int x = (row >> 1) & 3;
                     *reinterpret_cast<uint32_t*>(mp + ((0 ^ x) << 4)) = h2_bits(vh);
                     *reinterpret_cast<uint32_t*>(mp + ((1 ^ x) << 4)) = h2_bits(vl);
                     *reinterpret_cast<uint32_t*>(mp + ((2 ^ x) << 4)) = h2_bits(vh);
@@ -620,7 +665,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive_cluster(full_a);
-                        mbar_arrive_cluster(full_m);
+                        mbar_arrive_cluster(full_m + (gb & 1) * 8);
                     }
                 } else if constexpr (TYPE == T_MXFP4) {
                     uint32_t emax = 0;
@@ -641,7 +686,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
-                    if (!wait_or_fail(&bars->empty_a[j], (gb & 1) ^ 1, bars, g.status, 308)) break;
+                    if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
                     x_deq_mx(q[0], sc[0], 0, stage, row);
                     x_deq_mx(q[1], sc[1], 4, stage, row);
                     fence_proxy_async();
@@ -663,15 +708,19 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         const int gg = j + 4 * hf;
-                        if (!wait_or_fail(&bars->empty_a[j], (uint32_t)hf ^ 1u, bars, g.status, 308)) { ok = false; break; }
+                        // two stages: fill hf goes to stage hf, once a block
+                        const int ab2 = T::kABuf == 1 ? 0 : hf;
+                        uint8_t* stage2 = smem + (j * T::kABuf + ab2) * kABytes;
+                        const uint32_t pa2 = T::kABuf == 1 ? (uint32_t)hf ^ 1u : (gb & 1) ^ 1u;
+                        if (!poll_or_fail(&bars->empty_a[j * T::kABuf + ab2], pa2, bars, g.status, 308)) { ok = false; break; }
                         if constexpr (TYPE == T_Q6_K) {
-                            x_deq_q6k(wp, off, gg, stage, row);
+                            x_deq_q6k(wp, off, gg, stage2, row);
                         } else if (8 * b + gg < (g.K >> 5)) {
                             const uint32_t o = off + 34u * gg;
-                            x_deq_q8(wp, o + 2, h2f(*reinterpret_cast<const unsigned short*>(wp + o)) * up, stage, row);
+                            x_deq_q8(wp, o + 2, h2f(*reinterpret_cast<const unsigned short*>(wp + o)) * up, stage2, row);
                         } else {  // past K
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+                            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage2 + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
                         }
                         if (hf == 1) {
                             __syncwarp();
@@ -679,7 +728,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         }
                         fence_proxy_async();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(full_a);
+                        if (lane == 0) mbar_arrive_cluster(full_a0 + ab2 * 8);
                     }
                     if (!ok) break;
                 }
@@ -688,24 +737,37 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (gb > 0) {
                 // ---- promote the previous block: registers += its scale x its sums ----
                 const uint32_t pv = gb - 1, buf = pv & 1;
-                if (!wait_or_fail(&bars->accum[buf], (pv >> 1) & 1, bars, g.status, 310)) break;
+                if (!poll_or_fail(&bars->accum[buf], (pv >> 1) & 1, bars, g.status, 310)) break;
                 __syncwarp();
                 tc_fence_after();
-                const uint32_t ta = tmem + lane_base + buf * BN + j * (g.n_tile >> 2);
+                // columns of this set's tokens; merged: those of their low terms n_tile / 2 further on (either CTA's
+                // tokens are [high | low] there)
+                const uint32_t q4 = g.n_tile >> 2;
+                const uint32_t ta = tmem + lane_base + buf * T::kPStride + (merged ? (j >> 1) * g.n_tile + (j & 1) * q4 : j * q4);
+                if (BN <= 128 && merged) {
 #pragma unroll
-                for (int c = 0; c < BN / 32; c += 2) {
-                    if ((uint32_t)c < n8) {
-                        uint32_t v0[8], v1[8];
-                        tmem_ld8(ta + c * 8, v0);
-                        const bool both = (uint32_t)(c + 1) < n8;
-                        if (both) tmem_ld8(ta + c * 8 + 8, v1);
-                        tmem_ld_wait();
+                    for (int c = 0; c < BN / 32; ++c) {
+                        if ((uint32_t)c < n8) {
+                            uint32_t v0[8], v1[8];
+                            tmem_ld8(ta + c * 8, v0);
+                            tmem_ld8(ta + c * 8 + 2 * q4, v1);
+                            tmem_ld_wait();
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) acc[c * 8 + e] = fmaf(s_prev, __uint_as_float(v0[e]), acc[c * 8 + e]);
-                        if (both) {
+                            for (int e = 0; e < 8; e += 2)
+                                fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v0[e]) + __uint_as_float(v1[e]),
+                                          __uint_as_float(v0[e + 1]) + __uint_as_float(v1[e + 1]));
+                        }
+                    }
+                } else {  // pairs of groups; the second of the last pair may lie past the set's columns (read, not used)
 #pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                acc[c * 8 + 8 + e] = fmaf(s_prev, __uint_as_float(v1[e]), acc[c * 8 + 8 + e]);
+                    for (int c = 0; c < BN / 32; c += 2) {
+                        if ((uint32_t)c < n8) {
+                            uint32_t v[16];
+                            tmem_ld16(ta + c * 8, v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2)
+                                fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
                         }
                     }
                 }
@@ -718,17 +780,23 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     const bool whole = old.b0 == 0 && old.b1 == nblk;
                     const uint32_t m = tile_m0(old.tile) + row;
                     const uint32_t n0 = tile_n0(old.tile) + j * (g.n_tile >> 2);
+                    // the tokens' scales, one per lane (a load per column would be held back by the add before it)
+                    float inv0 = 0.f, inv1 = 0.f;
+                    if ((uint32_t)lane < n8 * 8 && n0 + lane < g.N) inv0 = __ldcg(g.inv_scale + n0 + lane);
+                    if (BN > 128 && 32u + lane < n8 * 8 && n0 + 32 + lane < g.N) inv1 = __ldcg(g.inv_scale + n0 + 32 + lane);
 #pragma unroll
                     for (int c = 0; c < BN / 4; ++c) {
                         const uint32_t n = n0 + c;
+                        const float inv = __shfl_sync(0xFFFFFFFFu, c < 32 ? inv0 : inv1, c & 31);
                         if ((uint32_t)c < n8 * 8 && n < g.N && m < g.M) {
-                            const float v = acc[c] * __ldcg(g.inv_scale + n);
+                            const float v = ((c & 1) ? acc[c / 2].y : acc[c / 2].x) * inv;
                             float* dst = g.D + (uint64_t)n * g.stride_d + m;
                             if (whole) *dst = v;
                             else atomicAdd(dst, v);
                         }
-                        acc[c] = 0.f;
                     }
+#pragma unroll
+                    for (int c = 0; c < BN / 8; ++c) acc[c] = make_float2(0.f, 0.f);
                 }
             }
             s_prev = s_cur;
@@ -739,7 +807,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * BN)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * T::kPStride)) : "memory");
     }
 }
 
@@ -759,7 +827,7 @@ int x_max_pairs(Kern kern, cudaLaunchConfig_t cfg, std::atomic<int>* cache) {
 }
 
 template <int TYPE, int BN, bool kFetch>
-cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
+cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
     using T = XTile<TYPE, BN, kFetch>;
     auto kern = gemm_exact_kernel<TYPE, BN, kFetch>;
     static std::atomic<uint64_t> attr_done{0};
@@ -778,19 +846,15 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (dry) {
-        const int pairs = x_max_pairs(kern, cfg, max_pairs);
-        if (pairs < 1) return cudaErrorNotSupported;
-        const uint32_t units = plan.n_tiles * plan.nblk;
-        // whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds
-        uint32_t G = units < (uint32_t)pairs ? units : (uint32_t)pairs;
-        if (plan.n_tiles <= (uint32_t)pairs && plan.n_tiles * 8 >= (uint32_t)pairs * 7) G = plan.n_tiles;
-        grid->pairs = G;
-        grid->split = !(plan.n_tiles % G == 0);
-        return cudaSuccess;
-    }
+    const int pairs = x_max_pairs(kern, cfg, max_pairs);
+    if (pairs < 1) return cudaErrorNotSupported;
+    const uint32_t units = plan.n_tiles * plan.nblk;
+    // whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds
+    uint32_t G = units < (uint32_t)pairs ? units : (uint32_t)pairs;
+    if (plan.n_tiles <= (uint32_t)pairs && plan.n_tiles * 8 >= (uint32_t)pairs * 7) G = plan.n_tiles;
+    const bool split = plan.n_tiles % G != 0;
     cfg.numAttrs = 2;
-    cfg.gridDim = dim3(2 * grid->pairs, 1, 1);
+    cfg.gridDim = dim3(2 * G, 1, 1);
     XArgs g{};
     g.A = p.A;
     g.a_end = p.A + (uint64_t)p.M * (p.K / block_size(TYPE)) * bytes_per_block(TYPE);
@@ -811,7 +875,8 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream
     CUtensorMap mx, mm, mw;
     const cuuint32_t estr[2] = {1, 1};
     const cuuint32_t box[2] = {64, plan.n_tile / 2};
-    const cuuint64_t xd[2] = {(cuuint64_t)plan.nblk * 256 * g.terms, p.N}, xs[1] = {(cuuint64_t)plan.nblk * 512 * g.terms};
+    // rows: the high (or only) terms of all tokens, then the low terms
+    const cuuint64_t xd[2] = {(cuuint64_t)plan.nblk * 256, (cuuint64_t)p.N * g.terms}, xs[1] = {(cuuint64_t)plan.nblk * 512};
     if (enc(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, plan.x, xd, xs, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
@@ -833,14 +898,16 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream
                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
+    // the preparation goes out last, so that the GEMM's launch follows it at once and overlaps it
+    if (cudaError_t e = prep.launch(prep.args, split, s); e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, kern, mx, mm, mw, g);
 }
 
 template <int TYPE, bool kFetch>
-cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
-    if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch>(p, plan, dry, s, grid);
-    if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch>(p, plan, dry, s, grid);
-    return x_launch<TYPE, 256, kFetch>(p, plan, dry, s, grid);
+cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
+    if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch>(p, plan, prep, s);
+    if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch>(p, plan, prep, s);
+    return x_launch<TYPE, 256, kFetch>(p, plan, prep, s);
 }
 
 }  // namespace

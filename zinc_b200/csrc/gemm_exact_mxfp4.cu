@@ -3,8 +3,8 @@
 
 namespace zc {
 
-cudaError_t launch_exact_mxfp4(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
-    return x_launch_bn<T_MXFP4, true>(p, plan, dry, s, grid);
+cudaError_t launch_exact_mxfp4(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
+    return x_launch_bn<T_MXFP4, true>(p, plan, prep, s);
 }
 
 }  // namespace zc

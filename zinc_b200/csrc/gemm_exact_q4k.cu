@@ -3,8 +3,8 @@
 
 namespace zc {
 
-cudaError_t launch_exact_q4k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid) {
-    return x_launch_bn<T_Q4_K, false>(p, plan, dry, s, grid);
+cudaError_t launch_exact_q4k(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
+    return x_launch_bn<T_Q4_K, false>(p, plan, prep, s);
 }
 
 }  // namespace zc

@@ -289,16 +289,17 @@ struct XPlan {
     void *x, *sums;
     float* inv_scale;
 };
-struct ExactGrid {
-    uint32_t pairs = 0;
-    bool split = false;
+// launches the preparation of the activations; split: tiles are shared between CTA pairs, D must be zeroed
+struct ExactPrep {
+    cudaError_t (*launch)(const void* args, bool split, cudaStream_t s);
+    const void* args;
 };
-// one translation unit per weight type; dry: only the grid is computed
-cudaError_t launch_exact_q4k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
-cudaError_t launch_exact_q5k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
-cudaError_t launch_exact_q6k(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
-cudaError_t launch_exact_q8(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
-cudaError_t launch_exact_mxfp4(const ExactGemm& p, const XPlan& plan, bool dry, cudaStream_t s, ExactGrid* grid);
+// one translation unit per weight type
+cudaError_t launch_exact_q4k(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s);
+cudaError_t launch_exact_q5k(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s);
+cudaError_t launch_exact_q6k(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s);
+cudaError_t launch_exact_q8(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s);
+cudaError_t launch_exact_mxfp4(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s);
 bool mul_mm_exact_eligible(uint32_t type, const uint8_t* A, uint32_t M, uint32_t N, uint32_t K);
 cudaError_t launch_mul_mm_exact(const ExactGemm& p, uint8_t* scratch, cudaStream_t s, uint64_t* launches);
 

@@ -134,8 +134,8 @@ __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t desc_a,
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // arrives on the barrier at this offset in both CTAs of the pair once the MMAs issued so far are done
@@ -192,6 +192,61 @@ __device__ __forceinline__ bool wait_or_fail(uint64_t* bar, uint32_t parity, B* 
     for (uint32_t i = 0; i < kWaitLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (kSleep) __nanosleep(64);
+        if ((i & 63u) == 63u && bars->failed) return false;
+    }
+    bars->failed = 1;
+    if (status) {
+        status[0] = 1;
+        status[1] = site;
+    }
+    return false;
+}
+
+// One lane of a converged warp. The issuing warp runs its loop with all lanes and only the tensor-core instructions
+// under this predicate: their operands then stay in uniform registers (in a branch on the lane number every operand is
+// moved there anew for every instruction). Elect where the instruction stands: with the answer kept in a variable across
+// the loop, commits went missing.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait of a converged warp for the barriers its lanes name (each lane one: several barriers in one round of
+// polls, one answer). test_wait answers in 10-25 cycles where a try_wait in a loaded kernel took 190-280, and the
+// issuing warp's own instructions are what bounds it.
+template <typename B>
+__device__ __forceinline__ bool warp_poll(uint32_t bar, uint32_t parity, B* bars, uint32_t* status, uint32_t site) {
+    if (__all_sync(0xFFFFFFFFu, mbar_test_addr(bar, parity))) return true;
+    for (uint32_t i = 0; i < 16u * kWaitLimit; ++i) {
+        if (__all_sync(0xFFFFFFFFu, mbar_test_addr(bar, parity))) return true;
+        if ((i & 255u) == 255u && __any_sync(0xFFFFFFFFu, bars->failed != 0)) return false;
+    }
+    bars->failed = 1;
+    if (status) {
+        status[0] = 1;
+        status[1] = site;
+    }
+    return false;
+}
+// Bounded wait of one warp among many: a first poll, then polls with a short sleep between them.
+template <typename B>
+__device__ __forceinline__ bool poll_or_fail(uint64_t* bar, uint32_t parity, B* bars, uint32_t* status, uint32_t site) {
+    const uint32_t a = smem_u32(bar);
+    if (mbar_test_addr(a, parity)) return true;
+    for (uint32_t i = 0; i < 4u * kWaitLimit; ++i) {
+        if (mbar_test_addr(a, parity)) return true;
+        __nanosleep(20);
         if ((i & 63u) == 63u && bars->failed) return false;
     }
     bars->failed = 1;
