@@ -126,33 +126,6 @@ __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cas
 __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t rotl(uint32_t v, int r) { return __funnelshift_l(v, v, r & 31); }
 
-// N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p: 16-byte reads (no bank
-// conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four rows per bank), then realigned.
-template <int N>
-__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N]) {
-    constexpr int V = (4 * N + 15 + 15) / 16;
-    uint32_t v[4 * V];
-#pragma unroll
-    for (int i = 0; i < V; ++i) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
-        v[4 * i] = t.x;
-        v[4 * i + 1] = t.y;
-        v[4 * i + 2] = t.z;
-        v[4 * i + 3] = t.w;
-    }
-    const uint32_t sh = (off & 3u) * 8u;
-    if (off & 8u) {
-#pragma unroll
-        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
-    }
-    if (off & 4u) {
-#pragma unroll
-        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
-}
-
 __device__ __forceinline__ void put_chunk(uint8_t* rowp, int sw, int c, uint4 o) {
     *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = o;
 }

@@ -30,6 +30,18 @@
 namespace zc {
 namespace {
 
+// N consecutive 32-bit words starting `sh` bits (a multiple of 8) into the aligned word at p.
+template <int N>
+__device__ __forceinline__ void lds_shifted(const uint32_t* p, uint32_t sh, uint32_t (&w)[N]) {
+    uint32_t prev = p[0];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t next = p[i + 1];
+        w[i] = __funnelshift_r(prev, next, sh);
+        prev = next;
+    }
+}
+
 constexpr int kMxBN = 128;                 // tokens per item
 constexpr int kMxStageK = 128;             // columns per stage: four MXFP4 blocks, one scale atom
 constexpr int kMxStages = 3;

@@ -109,25 +109,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         // tensor core needs for half the instruction, waits and commits not counted, so one thread alone
         // cannot keep two accumulators fed); both read every weight stage, each its own activation slots ----
         const int w = warp == 0 ? 0 : 1;
-        if (lane == 0 && w < n_iss) {
+        if (w < n_iss) {
             constexpr uint32_t idesc = instr_desc<BN>();
             int sb = w;  // slots are used in the order (iteration, accumulator)
             uint32_t fill = 0;  // how often the ring has wrapped = the number of this slot's fill
             bool ok = true;
             for (int it = 0; it < n_it && ok; ++it) {
                 const int sa = it & 3;
-                ok = wait_or_fail<false>(&bars->full_a[sa], (it >> 2) & 1, bars, g.status, 101);
+                ok = warp_poll(smem_u32(&bars->full_a[sa]), (it >> 2) & 1, bars, g.status, 101);
                 const uint64_t da = smem_desc(smem_u32(smem + sa * kABytes));
                 for (int acc = w; acc < nacc && ok; acc += n_iss) {
-                    ok = wait_or_fail<false>(&bars->full_b[sb + kBSlots * (fill & kFullSets - 1)], (fill / kFullSets) & 1, bars,
-                                             g.status, 102);
+                    ok = warp_poll(smem_u32(&bars->full_b[sb + kBSlots * (fill & kFullSets - 1)]), (fill / kFullSets) & 1,
+                                   bars, g.status, 102);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t db = smem_desc(smem_u32(smem_b + sb * kBSlotBytes));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k)  // 16 columns = 32 bytes per instruction
-                        umma_bf16(tmem + acc * BN, da + 2 * k, db + 2 * k, idesc, (it | k) ? 1u : 0u);
-                    umma_commit(&bars->empty_b[sb]);
+                        for (int k = 0; k < kBK / 16; ++k)  // 16 columns = 32 bytes per instruction
+                            umma_bf16(tmem + acc * BN, da + 2 * k, db + 2 * k, idesc, (it | k) ? 1u : 0u);
+                        umma_commit(&bars->empty_b[sb]);
+                    }
                     sb += n_iss;
                     if (sb >= kBSlots) {
                         sb -= kBSlots;
@@ -135,9 +137,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                     }
                 }
                 if (!ok) break;
-                umma_commit(&bars->empty_a[sa]);
+                if (elect_one()) umma_commit(&bars->empty_a[sa]);
             }
-            umma_commit(&bars->accum);
+            if (elect_one()) umma_commit(&bars->accum);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -234,9 +236,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
             } else {
                 // the block starts (b * 210) & 15 bytes into the box; that offset is even
                 const uint32_t off = ((uint32_t)b * 210u) & 15u;
-                const uint8_t* wp = smem_w + sw * kWBytes + row * 240 + (off & ~3u);
+                const uint8_t* wp = smem_w + sw * kWBytes + row * 240;
                 if (!wait_or_fail(&bars->empty_a[j], ((b - b_begin) & 1) ^ 1, bars, g.status, 104)) break;
-                dequant_group_q6k(reinterpret_cast<const uint32_t*>(wp), (off & 2u) * 8u, j, a_stage, row);
+                dequant_group_q6k(wp, off, j, a_stage, row);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
             }
@@ -398,7 +400,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
         // ---- MMA issuers (even CTA): one thread per accumulator. A thread whose accumulator lies past the last
         // token of a tile still takes part in every hand-off (its commits follow no MMA and arrive at once). ----
         const int w = warp == 0 ? 0 : 1;
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = instr_desc_pair<BN>();
             uint32_t git = 0, fill = 0, seg_i = 0, u = u_begin;
             int sb = 0;
@@ -407,34 +409,36 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
             while (ok && next_segment(u, u_end, nblk, sg)) {
                 const bool live = w < tile_nacc(sg.tile);
                 if (seg_i > 0) {  // the epilogue has read the previous segment's sums out of tensor memory
-                    ok = wait_or_fail<false>(&bars->tmem_free, (seg_i - 1) & 1, bars, g.status, 109);
+                    ok = warp_poll(smem_u32(&bars->tmem_free), (seg_i - 1) & 1, bars, g.status, 109);
                     if (!ok) break;
                     tc_fence_after();
                 }
                 const int n_it = (int)(sg.b1 - sg.b0) * 4;
                 for (int it = 0; it < n_it; ++it, ++git) {
                     const int sa = git & 3;
-                    ok = wait_or_fail<false>(&bars->full_a[sa], (git >> 2) & 1, bars, g.status, 101);
+                    // lane 0 watches the weight stage, lane 1 the activation slot
+                    ok = warp_poll(smem_u32(lane == 1 ? &bars->full_b[sb] : &bars->full_a[sa]), lane == 1 ? fill & 1 : (git >> 2) & 1,
+                                   bars, g.status, 101);
                     if (!ok) break;
-                    ok = wait_or_fail<false>(&bars->full_b[sb], fill & 1, bars, g.status, 102);
-                    if (!ok) break;
-                    if (live) {
-                        tc_fence_after();
-                        const uint64_t da = smem_desc(smem_u32(smem + sa * kABytes));
-                        const uint64_t db = smem_desc(smem_u32(smem_b + sb * kBSlotBytes + w * (kBSlotBytes / 2)));
+                    tc_fence_after();
+                    if (elect_one()) {
+                        if (live) {
+                            const uint64_t da = smem_desc(smem_u32(smem + sa * kABytes));
+                            const uint64_t db = smem_desc(smem_u32(smem_b + sb * kBSlotBytes + w * (kBSlotBytes / 2)));
 #pragma unroll
-                        for (int k = 0; k < kBK / 16; ++k)
-                            umma_bf16_pair(tmem + w * BN, da + 2 * k, db + 2 * k, idesc, (it | k) ? 1u : 0u);
+                            for (int k = 0; k < kBK / 16; ++k)
+                                umma_bf16_pair(tmem + w * BN, da + 2 * k, db + 2 * k, idesc, (it | k) ? 1u : 0u);
+                        }
+                        umma_commit_pair(&bars->empty_b[sb]);
+                        umma_commit_pair(&bars->empty_a[sa]);
                     }
-                    umma_commit_pair(&bars->empty_b[sb]);
                     if (++sb == kRing) {
                         sb = 0;
                         ++fill;
                     }
-                    umma_commit_pair(&bars->empty_a[sa]);
                 }
                 if (!ok) break;
-                umma_commit_pair(&bars->accum);
+                if (elect_one()) umma_commit_pair(&bars->accum);
                 ++seg_i;
             }
         }
@@ -577,7 +581,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
                     if (4 * b + (uint32_t)j < (g.K >> 6)) {
                         const uint32_t off = (uint32_t)((c_row_off + (uint64_t)b * 136u) & 15u) + 34u * (uint32_t)j;
                         const uint8_t* wp = smem_w + sw * kWBytes + row * 176;
-                        dequant_group_mxfp4(reinterpret_cast<const uint32_t*>(wp + (off & ~3u)), (off & 3u) * 8u, a_stage, row);
+                        dequant_group_mxfp4(wp, off, a_stage, row);
                     } else {  // past K: a zero row (the swizzle permutes 16-byte chunks of zeros)
 #pragma unroll
                         for (int c = 0; c < 8; ++c)
@@ -604,9 +608,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
                     // the block starts `off` bytes into the box or (fetched by the threads) into the row's aligned
                     // superset; that offset is even
                     const uint32_t off = kFetch ? (uint32_t)((c_row_off + (uint64_t)b * 210u) & 15u) : (b * 210u) & 15u;
-                    const uint8_t* wp = smem_w + sw * kWBytes + row * 240 + (off & ~3u);
+                    const uint8_t* wp = smem_w + sw * kWBytes + row * 240;
                     if (!wait_or_fail(&bars->empty_a[j], (gb & 1) ^ 1, bars, g.status, 104)) { ok = false; break; }
-                    dequant_group_q6k(reinterpret_cast<const uint32_t*>(wp), (off & 2u) * 8u, j, a_stage, row);
+                    dequant_group_q6k(wp, off, j, a_stage, row);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
                 }
@@ -757,22 +761,24 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs 
     const uint32_t tmem = bars->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {  // ---- MMA issuer: activation stage it & 3, weight stage it & 3 ----
+        {  // ---- MMA issuer: activation stage it & 3, weight stage it & 3 ----
             constexpr uint32_t idesc = instr_desc<kSmRows>();  // M = 128 tokens, N = 256 weight rows
             bool ok = true;
             for (int it = 0; it < n_it && ok; ++it) {
                 const int st = it & 3;
                 const uint32_t ph = (it >> 2) & 1;
-                ok = wait_or_fail<false>(&bars->full_a[st], ph, bars, g.status, 111);  // weights and activations
+                ok = warp_poll(smem_u32(&bars->full_a[st]), ph, bars, g.status, 111);  // weights and activations
                 if (!ok) break;
                 tc_fence_after();
                 const uint64_t dx = smem_desc(smem_u32(smem_x + st * kSmXBytes));
                 const uint64_t dw = smem_desc(smem_u32(smem + st * kSmWBytes));
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < kBK / 16; ++k) umma_bf16(tmem, dx + 2 * k, dw + 2 * k, idesc, (it | k) ? 1u : 0u);
-                umma_commit(&bars->empty_a[st]);  // frees the weight stage and the activation slot
+                    for (int k = 0; k < kBK / 16; ++k) umma_bf16(tmem, dx + 2 * k, dw + 2 * k, idesc, (it | k) ? 1u : 0u);
+                    umma_commit(&bars->empty_a[st]);  // frees the weight stage and the activation slot
+                }
             }
-            umma_commit(&bars->accum);
+            if (elect_one()) umma_commit(&bars->accum);
         }
     } else if (warp == 1) {
         if (lane == 0) {  // ---- TMA loader of the activations ----

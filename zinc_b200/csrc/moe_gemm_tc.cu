@@ -84,22 +84,6 @@ __device__ __forceinline__ uint4 moe_tile(const MoeGemmArgs& g, uint32_t t) {
     return __ldg(&g.tiles[t]);
 }
 
-template <bool kSleep = true>
-__device__ __forceinline__ bool moe_wait(uint64_t* bar, uint32_t parity, MoeBars* bars, uint32_t* status,
-                                         uint32_t site) {
-    for (uint32_t i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (kSleep) __nanosleep(64);
-        if ((i & 63u) == 63u && bars->failed) return false;
-    }
-    bars->failed = 1;
-    if (status) {
-        status[0] = 1;
-        status[1] = site;
-    }
-    return false;
-}
-
 // Position of the dequant warps in the flat sequence of (work item, 256-column block).
 struct BlockCursor {
     uint32_t w;             // work item
@@ -154,29 +138,31 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     const uint32_t tmem = bars->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {  // ---- MMA issuer ----
+        {  // ---- MMA issuer ----
             constexpr uint32_t idesc = instr_desc<BN>();
             uint32_t gs = 0, i = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
                 const uint32_t ab = i & 1;
-                ok = moe_wait<false>(&bars->accum_empty[ab], ((i >> 1) & 1) ^ 1, bars, g.status, 121);
+                ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.status, 121);
                 if (!ok) break;
                 tc_fence_after();
                 for (int s = 0; s < n_stages; ++s, ++gs) {
                     const int st = gs & 3;
                     const uint32_t ph = (gs >> 2) & 1;
-                    ok = moe_wait<false>(&bars->full_a[st], ph, bars, g.status, 122);
+                    ok = warp_poll(smem_u32(&bars->full_a[st]), ph, bars, g.status, 122);
                     if (!ok) break;
                     tc_fence_after();
                     const uint64_t da = smem_desc(smem_u32(smem + st * kABytes));
                     const uint64_t dx = smem_desc(smem_u32(smem_x + st * T::kXBytes));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k)
-                        umma_bf16(tmem + ab * BN, da + 2 * k, dx + 2 * k, idesc, (s | k) ? 1u : 0u);
-                    umma_commit(&bars->empty_a[st]);
+                        for (int k = 0; k < kBK / 16; ++k)
+                            umma_bf16(tmem + ab * BN, da + 2 * k, dx + 2 * k, idesc, (s | k) ? 1u : 0u);
+                        umma_commit(&bars->empty_a[st]);
+                    }
                 }
-                if (ok) umma_commit(&bars->accum_full[ab]);
+                if (ok && elect_one()) umma_commit(&bars->accum_full[ab]);
             }
         }
     } else if (warp == 1) {
@@ -187,7 +173,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                 const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
                 for (int s = 0; s < n_stages; ++s, ++gs) {
                     const int st = gs & 3;
-                    ok = moe_wait(&bars->empty_a[st], ((gs >> 2) & 1) ^ 1, bars, g.status, 124);
+                    ok = poll_or_fail(&bars->empty_a[st], ((gs >> 2) & 1) ^ 1, bars, g.status, 124);
                     if (!ok) break;
                     mbar_expect_tx(&bars->full_a[st], T::kXBytes);
                     tma_load_2d(smem_x + st * T::kXBytes, &tmap_x, s * kBK, (int)tile.y, &bars->full_a[st]);
@@ -244,7 +230,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
         bool dead = false;
         auto issue_fetch = [&]() {
             if (ahead.w >= n_items) return;
-            if (!dead) dead = !moe_wait(&bars->empty_w[slot_f], (use_f & 1) ^ 1, bars, g.status, 127);
+            if (!dead) dead = !poll_or_fail(&bars->empty_w[slot_f], (use_f & 1) ^ 1, bars, g.status, 127);
             if (!dead) fetch(ahead, slot_f);
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[slot_f]))
                          : "memory");
@@ -259,9 +245,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             const int ns = min(4, n_stages - 4 * cur.b);
             const int q = (j - (int)gs) & 3;  // this set's group of the block, if the block has that many
             const bool mine = q < ns;
-            if (mine && !dead) dead = !moe_wait(&bars->full_w[slot_c], use_c & 1, bars, g.status, 128);
+            if (mine && !dead) dead = !poll_or_fail(&bars->full_w[slot_c], use_c & 1, bars, g.status, 128);
             if (mine && !dead)
-                dead = !moe_wait(&bars->empty_a[j], (((gs + q) >> 2) & 1) ^ 1, bars, g.status, 125);
+                dead = !poll_or_fail(&bars->empty_a[j], (((gs + q) >> 2) & 1) ^ 1, bars, g.status, 125);
             if (mine && !dead) {
                 const uint8_t* slot = smem_w + slot_c * T::kRawBytes + row * kBox;
                 if constexpr (TYPE == T_Q4_K) {
@@ -277,12 +263,10 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                                       a_stage, row);
                 } else if constexpr (TYPE == T_Q6_K) {
                     const uint32_t off = (uint32_t)((cur.row_off + (uint64_t)cur.b * kBlock) & 15u);
-                    dequant_group_q6k(reinterpret_cast<const uint32_t*>(slot + (off & ~3u)), (off & 2u) * 8u, q,
-                                      a_stage, row);
+                    dequant_group_q6k(slot, off, q, a_stage, row);
                 } else {
                     const uint32_t off = (uint32_t)((cur.row_off + (uint64_t)cur.b * kBlock) & 15u) + 34u * q;
-                    dequant_group_mxfp4(reinterpret_cast<const uint32_t*>(slot + (off & ~3u)), (off & 3u) * 8u,
-                                        a_stage, row);
+                    dequant_group_mxfp4(slot, off, a_stage, row);
                 }
                 fence_proxy_async();
                 __syncwarp();
@@ -307,7 +291,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             const uint32_t ab = i & 1;
             const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
             const uint32_t m = (w % g.row_tiles) * kBM + q * 32 + lane;
-            if (!moe_wait(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 126)) break;
+            if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 126)) break;
             __syncwarp();
             tc_fence_after();
 #pragma unroll 1

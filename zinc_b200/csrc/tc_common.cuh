@@ -294,16 +294,31 @@ __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& 
     }
 }
 
-// N consecutive 32-bit words starting `sh` bits (0 or 16) into the aligned word at p.
+// N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p: 16-byte reads (no bank
+// conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four rows per bank), then realigned.
 template <int N>
-__device__ __forceinline__ void lds_shifted(const uint32_t* p, uint32_t sh, uint32_t (&w)[N]) {
-    uint32_t prev = p[0];
+__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N]) {
+    constexpr int V = (4 * N + 15 + 15) / 16;
+    uint32_t v[4 * V];
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const uint32_t next = p[i + 1];
-        w[i] = __funnelshift_r(prev, next, sh);
-        prev = next;
+    for (int i = 0; i < V; ++i) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
+        v[4 * i] = t.x;
+        v[4 * i + 1] = t.y;
+        v[4 * i + 2] = t.z;
+        v[4 * i + 3] = t.w;
     }
+    const uint32_t sh = (off & 3u) * 8u;
+    if (off & 8u) {
+#pragma unroll
+        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
+    }
+    if (off & 4u) {
+#pragma unroll
+        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
 }
 
 // Four 6-bit weights (one per byte of q4, values 0..63) -> two bf16x2 words: (128 + q) - 160 = q - 32
@@ -319,17 +334,16 @@ __device__ __forceinline__ void deq4_q6(uint32_t q4, __nv_bfloat162 dsc, uint32_
 // One 64-column group g of a Q6_K block (layout: ql[128] qh[64] scales[16] d, src/model/gguf.zig:38-123;
 // element order as dequantRow, src/compute/forward.zig:335-383): half n = g / 2 of the block, low
 // (g even) or high (g odd) nibbles of ql[64n .. 64n+64), bit pairs 4*(g&1) and 4*(g&1)+2 of
-// qh[32n .. 32n+32), scales[8n + 4*(g&1) .. +4) each covering 16 columns. `blk` points at the aligned
-// word that contains the block's first byte, `sh` = 0 or 16.
-__device__ __forceinline__ void dequant_group_q6k(const uint32_t* blk, uint32_t sh, int g, uint8_t* a_stage,
-                                                  int row) {
+// qh[32n .. 32n+32), scales[8n + 4*(g&1) .. +4) each covering 16 columns. The block starts `off` bytes (even, 0..14)
+// into the 16-byte aligned row at `p`.
+__device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, uint8_t* a_stage, int row) {
     const int n = g >> 1, hi = g & 1;
-    uint32_t ql[16], qh[8], scw[1], dw[1];
-    lds_shifted<16>(blk + 16 * n, sh, ql);
-    lds_shifted<8>(blk + 32 + 8 * n, sh, qh);
-    lds_shifted<1>(blk + 48 + 2 * n + hi, sh, scw);
-    lds_shifted<1>(blk + 52, sh, dw);
-    const float d = __half2float(__ushort_as_half((unsigned short)(dw[0] & 0xFFFFu)));
+    uint32_t ql[16], qh[8];
+    lds_words<16>(p + 64 * n, off, ql);
+    lds_words<8>(p + 128 + 32 * n, off, qh);
+    const unsigned short* tail = reinterpret_cast<const unsigned short*>(p + off + 192);
+    const uint32_t scw[1] = {(uint32_t)tail[4 * n + 2 * hi] | ((uint32_t)tail[4 * n + 2 * hi + 1] << 16)};
+    const float d = __half2float(__ushort_as_half(tail[8]));
     uint8_t* rowp = a_stage + row * 128;
     const int sw = row & 7;
 #pragma unroll
@@ -382,11 +396,10 @@ __device__ __forceinline__ void deq_mx16(uint32_t x16, __nv_bfloat162 scale, uin
 }
 
 // One 64-column group (two 17-byte blocks, 34 bytes) of an MXFP4 row -> the swizzled row `row` of the
-// stage at `a_stage`. `p` points at the aligned word that holds the group's first byte, `sh` = 8 * (its
-// byte position in that word).
-__device__ __forceinline__ void dequant_group_mxfp4(const uint32_t* p, uint32_t sh, uint8_t* a_stage, int row) {
+// stage at `a_stage`. The group starts `off` bytes into the 16-byte aligned row at `p`.
+__device__ __forceinline__ void dequant_group_mxfp4(const uint8_t* p, uint32_t off, uint8_t* a_stage, int row) {
     uint32_t w[9];
-    lds_shifted<9>(p, sh, w);  // bytes 0..35 of the group: e0, 16 nibble bytes, e1, 16 nibble bytes
+    lds_words<9>(p + (off & ~15u), off & 15u, w);  // bytes 0..35 of the group: e0, 16 nibble bytes, e1, 16 nibble bytes
     uint8_t* rowp = a_stage + row * 128;
     const int sw = row & 7;
 #pragma unroll
