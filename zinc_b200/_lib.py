@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(_HERE, "libzinc_b200.so")
@@ -105,6 +106,17 @@ EXPORTS = sorted(list(_OPS) + [
 ])
 
 _lib = None
+CALL_PATH = os.path.join(_HERE, "_call.so")
+
+
+def native_call():
+    """The class of native calls (csrc/call.cpp), or None in a program that has not loaded torch, whose tensors it reads."""
+    if "torch" not in sys.modules:
+        return None
+    if not os.path.exists(CALL_PATH):
+        raise ImportError(f"{CALL_PATH} is missing: build it with `python -m zinc_b200.build`.")
+    from ._call import Call
+    return Call
 
 
 def lib() -> C.CDLL:

@@ -8,6 +8,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO = os.path.join(HERE, "libzinc_b200.so")
+CALL_SO = os.path.join(HERE, "_call.so")   # Python module: calls into the library without ctypes
 SOURCES = ["api.cu", "dmmv.cu", "dmmv_warp.cu", "dmmv_q6k.cu", "misc.cu", "gemm_simple.cu", "gemm_tc.cu",
            "dmmv_static_scratch.cu", "comm.cu", "dmmv_mxfp4.cu", "moe_gemm_tc.cu", "gemm_mx.cu", "gemm_exact.cu",
            "gemm_exact_q4k.cu", "gemm_exact_q5k.cu", "gemm_exact_q6k.cu", "gemm_exact_q8.cu", "gemm_exact_mxfp4.cu"]
@@ -24,10 +25,23 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
+def _call_command() -> list:
+    """g++ on call.cpp, against the headers and libraries of the installed torch (found without importing it)."""
+    import importlib.util
+    import sysconfig
+
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    inc = os.path.join(torch_dir, "include")
+    lib = os.path.join(torch_dir, "lib")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, "call.cpp"), "-o", CALL_SO,
+            "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+            "-I", sysconfig.get_paths()["include"], "-L", lib, "-Wl,-rpath," + lib, "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
 def stale() -> bool:
-    if not os.path.exists(SO):
+    if not os.path.exists(SO) or not os.path.exists(CALL_SO):
         return True
-    t = os.path.getmtime(SO)
+    t = min(os.path.getmtime(SO), os.path.getmtime(CALL_SO))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [
         os.path.join(HERE, "..", "include", "zinc_cuda.h")]
     return any(os.path.getmtime(d) > t for d in deps)
@@ -41,6 +55,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
     procs = []
+    call = subprocess.Popen(_call_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     for src in SOURCES:
         obj = os.path.join(objdir, src.replace(".cu", ".o"))
         cmd = [nvcc, *[f for f in NVCC_FLAGS if f != "--use_fast_math=false"], "-c",
@@ -55,6 +70,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(out)
             raise RuntimeError(f"nvcc failed on {src}")
         objs.append(obj)
+    out, _ = call.communicate()
+    if call.returncode != 0:
+        sys.stderr.write(out)
+        raise RuntimeError("g++ failed on call.cpp")
     with open(os.path.join(objdir, "ptxas.log"), "w") as f:
         f.write("\n".join(log))
     if verbose:

@@ -88,6 +88,7 @@ class Context:
             raise _ERRORS.get(rc, ZincError)(
                 f"zc_init(device={device}) failed: {self._lib.zc_status_string(rc).decode()}")
         self._h = h
+        self.handle = h.value   # the context's address as an integer, 0 once closed
         self.device = device
         if stream is not None:
             self.set_stream(stream)
@@ -96,8 +97,11 @@ class Context:
     def call(self, name: str, *args) -> None:
         rc = getattr(self._lib, name)(self._h, *args)
         if rc != _lib.OK:
-            msg = self._lib.zc_last_error(self._h).decode()
-            raise _ERRORS.get(rc, ZincError)(f"{name}: {msg}")
+            self.fail(name, rc)
+
+    def fail(self, name: str, rc: int) -> None:
+        msg = self._lib.zc_last_error(self._h).decode()
+        raise _ERRORS.get(rc, ZincError)(f"{name}: {msg}")
 
     def set_stream(self, stream: Optional[int]) -> None:
         """Launch on the given cudaStream_t handle (0 / None = CUDA's default stream)."""
@@ -209,6 +213,7 @@ class Context:
         if getattr(self, "_h", None):
             self._lib.zc_destroy(self._h)
             self._h = None
+            self.handle = 0
 
     def __del__(self):
         try:
@@ -238,11 +243,69 @@ def row_bytes(t: int, K: int) -> int:
     return (K // block_size(t)) * bytes_per_block(t)
 
 
+# What each exported function takes, in order: i integer (the context first), f float, b buffer, o buffer or None.
+_CALLS = {
+    "zc_dmmv": "iibbbiiiiii",
+    "zc_dmmv_push": "iibbbiiiiii",
+    "zc_dmmv_batch": "iibbbiiiiii",
+    "zc_moe_dmmv": "iibbbbiiiiiii",
+    "zc_moe_dmmv_batched": "iibbbbiiiiiiii",
+    "zc_moe_dmmv_batched_pair": "iibbbbbbiiiiiiii",
+    "zc_mul_mm_block_scaled": "iibbbiiiiiiiib",
+    "zc_count_experts": "ibbiiiiii",
+    "zc_mul_mm": "iibbbiiiiiiiii",
+    "zc_dmmv_fused_gate_up_swiglu": "iibbbbiiiiii",
+    "zc_dmmv_sigmoid_acc": "iibbbbiiiiii",
+    "zc_moe_fused_gate_up": "iibbbbbbiiiiiii",
+    "zc_moe_fused_gate_up_act": "iibbbbbiiiiiiii",
+    "zc_moe_gate_up_act_ex": "iibboooobbbiiiiiii",
+    "zc_moe_down_acc_ex": "iiboobbbiiiiiii",
+    "zc_moe_router_topk": "iboboobboiiiifiiii",
+    "zc_rms_norm_dmmv_f32": "ibbbobiif",
+    "zc_dmmv_o_proj_merge": "iibbboiiiiiiiii",
+    "zc_rms_norm_dmmv_alpha_beta": "ibbbbobbiif",
+    "zc_moe_weighted_acc": "ibbbiii",
+    "zc_bias_add": "ibbii",
+    "zc_moe_bias_act": "ibboobbiiii",
+    "zc_moe_weighted_bias_acc": "ibbbiii",
+    "zc_moe_ep_filter": "ibbiiiiii",
+    "zc_moe_route_pack": "ibbbiiiii",
+    "zc_moe_route_scatter": "ibbbiiii",
+    "zc_dequant_rows": "iibbiiii",
+}
+
+
+def _calls() -> dict:
+    """One callable per function of _CALLS that returns its status: natively where torch is loaded (its tensors are
+    then read without going through Python), else through ctypes."""
+    L = _lib.lib()
+    native = _lib.native_call()
+    if native is not None:
+        return {name: native(C.cast(getattr(L, name), C.c_void_p).value, spec, _buf) for name, spec in _CALLS.items()}
+
+    def through_ctypes(fn, spec):
+        def call(*args):
+            flat = []
+            for kind, a in zip(spec, args):
+                if kind in "if":
+                    flat.append(a)
+                elif a is None and kind == "o":
+                    flat += (None, 0)
+                else:
+                    b = _buf(a)
+                    flat += (b.ptr, b.size)
+            return fn(*flat)
+        return call
+
+    return {name: through_ctypes(getattr(L, name), spec) for name, spec in _CALLS.items()}
+
+
 class DmmvDispatch:
     """Mirror of DmmvDispatch (src/compute/dmmv.zig:161-297): one object per context."""
 
     def __init__(self, ctx: Context):
         self.ctx = ctx
+        self._f = _calls()
 
     # pipelineForType / moePipelineForType (src/compute/dmmv.zig:678-703)
     def pipelineForType(self, quant_type: int) -> bool:
@@ -253,16 +316,17 @@ class DmmvDispatch:
 
     # recordDispatch (src/compute/dmmv.zig:806-874); buffers in binding order A, x, y
     def recordDispatch(self, quant_type, A, x, y, M, K, a_offset=0, x_offset=0, y_offset=0, acc_mode=0):
-        A, x, y = _buf(A), _buf(x), _buf(y)
-        self.ctx.call("zc_dmmv", quant_type, A.ptr, A.size, x.ptr, x.size, y.ptr, y.size, M, K,
-                      a_offset, x_offset, y_offset, acc_mode)
+        rc = self._f["zc_dmmv"](self.ctx.handle, quant_type, A, x, y, M, K, a_offset, x_offset, y_offset, acc_mode)
+        if rc:
+            self.ctx.fail("zc_dmmv", rc)
 
     # recordDispatch for a K-sharded projection on N GPUs: the partial result is pushed to every rank and
     # summed into dst by the next call on the context (no counterpart in the single-GPU reference)
     def recordDispatchPush(self, quant_type, A, x, dst, M, K, a_offset=0, x_offset=0, dst_offset=0, acc_mode=0):
-        A, x, dst = _buf(A), _buf(x), _buf(dst)
-        self.ctx.call("zc_dmmv_push", quant_type, A.ptr, A.size, x.ptr, x.size, dst.ptr, dst.size, M, K,
-                      a_offset, x_offset, dst_offset, acc_mode)
+        rc = self._f["zc_dmmv_push"](self.ctx.handle, quant_type, A, x, dst, M, K, a_offset, x_offset, dst_offset,
+                                     acc_mode)
+        if rc:
+            self.ctx.fail("zc_dmmv_push", rc)
 
     # recordBatchDispatchPush (src/compute/dmmv.zig:880-926) + dispatchProjectionBatched chunk loop
     def recordDispatchMulti(self, quant_type, As, x, ys, Ms, K, a_offsets=None, x_offset=0, y_offsets=None,
@@ -281,33 +345,35 @@ class DmmvDispatch:
                       u64(*[b.size for b in yb]), u64(*y_offsets), u32(*Ms), K, acc_mode)
 
     def recordBatchDispatchPush(self, quant_type, A, X, Y, M, K, a_offset, x_offset, y_offset, num_cols):
-        A, X, Y = _buf(A), _buf(X), _buf(Y)
-        self.ctx.call("zc_dmmv_batch", quant_type, A.ptr, A.size, X.ptr, X.size, Y.ptr, Y.size, M, K,
-                      a_offset, x_offset, y_offset, num_cols)
+        rc = self._f["zc_dmmv_batch"](self.ctx.handle, quant_type, A, X, Y, M, K, a_offset, x_offset, y_offset,
+                                      num_cols)
+        if rc:
+            self.ctx.fail("zc_dmmv_batch", rc)
 
     # recordMoeDispatch (src/compute/dmmv.zig:709-739); bindings A, x, y, routing
     def recordMoeDispatch(self, quant_type, A, x, y, routing, M, K, expert_stride, n_experts_y,
                           x_expert_stride, x_offset=0, y_offset=0):
-        A, x, y, routing = _buf(A), _buf(x), _buf(y), _buf(routing)
-        self.ctx.call("zc_moe_dmmv", quant_type, A.ptr, A.size, x.ptr, x.size, y.ptr, y.size,
-                      routing.ptr, routing.size, M, K, expert_stride, n_experts_y, x_expert_stride,
-                      x_offset, y_offset)
+        rc = self._f["zc_moe_dmmv"](self.ctx.handle, quant_type, A, x, y, routing, M, K, expert_stride, n_experts_y,
+                                    x_expert_stride, x_offset, y_offset)
+        if rc:
+            self.ctx.fail("zc_moe_dmmv", rc)
 
     # recordMoeBatchedDispatch (src/compute/dmmv.zig:746-792)
     def recordMoeBatchedDispatch(self, quant_type, A, X, Y, routing, M, K, expert_stride, n_experts,
                                  n_experts_used, n_tokens, x_token_stride, y_token_stride):
-        A, X, Y, routing = _buf(A), _buf(X), _buf(Y), _buf(routing)
-        self.ctx.call("zc_moe_dmmv_batched", quant_type, A.ptr, A.size, X.ptr, X.size, Y.ptr, Y.size,
-                      routing.ptr, routing.size, M, K, expert_stride, n_experts, n_experts_used, n_tokens,
-                      x_token_stride, y_token_stride)
+        rc = self._f["zc_moe_dmmv_batched"](self.ctx.handle, quant_type, A, X, Y, routing, M, K, expert_stride,
+                                            n_experts, n_experts_used, n_tokens, x_token_stride, y_token_stride)
+        if rc:
+            self.ctx.fail("zc_moe_dmmv_batched", rc)
 
     # gate and up of a prefill batch on one grouping (the prefill counterpart of dispatchMoeFusedGateUp)
     def recordMoeBatchedDispatchPair(self, quant_type, Wg, Wu, X, Yg, Yu, routing, M, K, expert_stride, n_experts,
                                      n_experts_used, n_tokens, x_token_stride, y_token_stride):
-        Wg, Wu, X, Yg, Yu, routing = map(_buf, (Wg, Wu, X, Yg, Yu, routing))
-        self.ctx.call("zc_moe_dmmv_batched_pair", quant_type, Wg.ptr, Wg.size, Wu.ptr, Wu.size, X.ptr, X.size,
-                      Yg.ptr, Yg.size, Yu.ptr, Yu.size, routing.ptr, routing.size, M, K, expert_stride, n_experts,
-                      n_experts_used, n_tokens, x_token_stride, y_token_stride)
+        rc = self._f["zc_moe_dmmv_batched_pair"](self.ctx.handle, quant_type, Wg, Wu, X, Yg, Yu, routing, M, K,
+                                                 expert_stride, n_experts, n_experts_used, n_tokens, x_token_stride,
+                                                 y_token_stride)
+        if rc:
+            self.ctx.fail("zc_moe_dmmv_batched_pair", rc)
 
     # Lend the library scratch for the grouped MoE prefill path (no counterpart in the reference's
     # DmmvDispatch; its Metal path owns route_ids / route_counts buffers). None removes it.
@@ -323,9 +389,10 @@ class DmmvDispatch:
     # as two exact FP8 terms in `workspace`)
     def recordMulMmBlockScaled(self, quant_type, a_buf, b_buf, d_buf, M, N, K, stride_b, stride_d, workspace,
                                a_offset=0, b_offset=0, d_offset=0):
-        a, b, d, w = map(_buf, (a_buf, b_buf, d_buf, workspace))
-        self.ctx.call("zc_mul_mm_block_scaled", quant_type, a.ptr, a.size, b.ptr, b.size, d.ptr, d.size, M, N, K,
-                      stride_b, stride_d, a_offset, b_offset, d_offset, w.ptr, w.size)
+        rc = self._f["zc_mul_mm_block_scaled"](self.ctx.handle, quant_type, a_buf, b_buf, d_buf, M, N, K, stride_b,
+                                               stride_d, a_offset, b_offset, d_offset, workspace)
+        if rc:
+            self.ctx.fail("zc_mul_mm_block_scaled", rc)
 
     @staticmethod
     def mulMmWorkspaceBytes(quant_type, N, K) -> int:
@@ -340,16 +407,18 @@ class DmmvDispatch:
     # recordCountExperts (src/compute/dmmv.zig:981-1028)
     def recordCountExperts(self, routing, counts, n_tokens, n_layers, layer, n_experts_used, n_experts,
                            d_offset_bytes=0):
-        routing, counts = _buf(routing), _buf(counts)
-        self.ctx.call("zc_count_experts", routing.ptr, routing.size, counts.ptr, counts.size, n_tokens, n_layers,
-                      layer, n_experts_used, n_experts, d_offset_bytes)
+        rc = self._f["zc_count_experts"](self.ctx.handle, routing, counts, n_tokens, n_layers, layer, n_experts_used,
+                                         n_experts, d_offset_bytes)
+        if rc:
+            self.ctx.fail("zc_count_experts", rc)
 
     # recordMulMmQ4K (src/compute/dmmv.zig:1045-1094), widened to every type and to bf16 activations
     def recordMulMm(self, quant_type, A, B, D, M, N, K, stride_b, stride_d, a_offset=0, b_offset=0, d_offset=0,
                     act_type=F32):
-        A, B, D = _buf(A), _buf(B), _buf(D)
-        self.ctx.call("zc_mul_mm", quant_type, A.ptr, A.size, B.ptr, B.size, D.ptr, D.size, M, N, K,
-                      stride_b, stride_d, a_offset, b_offset, d_offset, act_type)
+        rc = self._f["zc_mul_mm"](self.ctx.handle, quant_type, A, B, D, M, N, K, stride_b, stride_d, a_offset,
+                                  b_offset, d_offset, act_type)
+        if rc:
+            self.ctx.fail("zc_mul_mm", rc)
 
     def recordMulMmQ4K(self, A, B, D, M, N, K, stride_b, stride_d, a_offset=0, b_offset=0, d_offset=0):
         self.recordMulMm(Q4_K, A, B, D, M, N, K, stride_b, stride_d, a_offset, b_offset, d_offset, F32)
@@ -358,74 +427,69 @@ class DmmvDispatch:
     # dispatchDmmvFusedGateUpSwiglu (forward.zig:8237-8313)
     def dispatchDmmvFusedGateUpSwiglu(self, quant_type, Wg, Wu, x, out, M, K, gate_offset=0, up_offset=0,
                                       x_offset=0, out_offset=0):
-        Wg, Wu, x, out = _buf(Wg), _buf(Wu), _buf(x), _buf(out)
-        self.ctx.call("zc_dmmv_fused_gate_up_swiglu", quant_type, Wg.ptr, Wg.size, Wu.ptr, Wu.size, x.ptr, x.size,
-                      out.ptr, out.size, M, K, gate_offset, up_offset, x_offset, out_offset)
+        rc = self._f["zc_dmmv_fused_gate_up_swiglu"](self.ctx.handle, quant_type, Wg, Wu, x, out, M, K, gate_offset,
+                                                     up_offset, x_offset, out_offset)
+        if rc:
+            self.ctx.fail("zc_dmmv_fused_gate_up_swiglu", rc)
 
     # dispatchDmmvQ8_0SigmoidAcc (forward.zig:8321-8359)
     def dispatchDmmvSigmoidAcc(self, quant_type, A, x, y, gate, M, K, a_offset=0, x_offset=0, y_offset=0,
                                gate_index=0):
-        A, x, y, gate = _buf(A), _buf(x), _buf(y), _buf(gate)
-        self.ctx.call("zc_dmmv_sigmoid_acc", quant_type, A.ptr, A.size, x.ptr, x.size, y.ptr, y.size,
-                      gate.ptr, gate.size, M, K, a_offset, x_offset, y_offset, gate_index)
+        rc = self._f["zc_dmmv_sigmoid_acc"](self.ctx.handle, quant_type, A, x, y, gate, M, K, a_offset, x_offset,
+                                            y_offset, gate_index)
+        if rc:
+            self.ctx.fail("zc_dmmv_sigmoid_acc", rc)
 
     # fused gate+up MoE dispatch (forward.zig:6206-6222)
     def dispatchMoeFusedGateUp(self, quant_type, Wg, Wu, x, y_gate, y_up, routing, M, K, expert_stride, n_used,
                                x_expert_stride, x_offset=0, y_offset=0):
-        Wg, Wu, x, y_gate, y_up, routing = map(_buf, (Wg, Wu, x, y_gate, y_up, routing))
-        self.ctx.call("zc_moe_fused_gate_up", quant_type, Wg.ptr, Wg.size, Wu.ptr, Wu.size, x.ptr, x.size,
-                      y_gate.ptr, y_gate.size, y_up.ptr, y_up.size, routing.ptr, routing.size, M, K,
-                      expert_stride, n_used, x_expert_stride, x_offset, y_offset)
+        rc = self._f["zc_moe_fused_gate_up"](self.ctx.handle, quant_type, Wg, Wu, x, y_gate, y_up, routing, M, K,
+                                             expert_stride, n_used, x_expert_stride, x_offset, y_offset)
+        if rc:
+            self.ctx.fail("zc_moe_fused_gate_up", rc)
 
     # the same with SwiGLU (or the GPT-OSS form) applied in the epilogue: one launch for the reference's
     # fused gate+up dispatch and its activation dispatch (forward.zig:6206-6240)
     def dispatchMoeFusedGateUpAct(self, quant_type, Wg, Wu, x, y, routing, M, K, expert_stride, n_used,
                                   x_expert_stride, oai=False, x_offset=0, y_offset=0):
-        Wg, Wu, x, y, routing = map(_buf, (Wg, Wu, x, y, routing))
-        self.ctx.call("zc_moe_fused_gate_up_act", quant_type, Wg.ptr, Wg.size, Wu.ptr, Wu.size, x.ptr, x.size,
-                      y.ptr, y.size, routing.ptr, routing.size, M, K, expert_stride, n_used, x_expert_stride,
-                      x_offset, y_offset, 1 if oai else 0)
+        rc = self._f["zc_moe_fused_gate_up_act"](self.ctx.handle, quant_type, Wg, Wu, x, y, routing, M, K,
+                                                 expert_stride, n_used, x_expert_stride, x_offset, y_offset, 1 if oai
+                                                 else 0)
+        if rc:
+            self.ctx.fail("zc_moe_fused_gate_up_act", rc)
 
     # One launch for the routed gate + up dispatch, the shared expert's gate + up (a slot with the id
     # SHARED_EXPERT), the per-expert gate / up biases and the activation (forward.zig:6206-6240, 6455-6500,
     # 6841-6849). shared = (gate, up) matrices or None; biases = (gate_bias, up_bias) [n_experts][M] or None.
     def dispatchMoeGateUpActEx(self, quant_type, Wg, Wu, x, y, routing, M, K, expert_stride, n_used, shared=None,
                                biases=None, oai=False, x_offset=0, y_offset=0):
-        Wg, Wu, x, y, routing = map(_buf, (Wg, Wu, x, y, routing))
-        none = Buffer(None, 0)
-        sg, su = map(_buf, shared) if shared is not None else (none, none)
-        bg, bu = map(_buf, biases) if biases is not None else (none, none)
-        self.ctx.call("zc_moe_gate_up_act_ex", quant_type, Wg.ptr, Wg.size, Wu.ptr, Wu.size, sg.ptr, sg.size,
-                      su.ptr, su.size, bg.ptr, bg.size, bu.ptr, bu.size, x.ptr, x.size, y.ptr, y.size,
-                      routing.ptr, routing.size, M, K, expert_stride, n_used, x_offset, y_offset, 1 if oai else 0)
+        sg, su = shared if shared is not None else (None, None)
+        bg, bu = biases if biases is not None else (None, None)
+        rc = self._f["zc_moe_gate_up_act_ex"](self.ctx.handle, quant_type, Wg, Wu, sg, su, bg, bu, x, y, routing, M,
+                                              K, expert_stride, n_used, x_offset, y_offset, 1 if oai else 0)
+        if rc:
+            self.ctx.fail("zc_moe_gate_up_act_ex", rc)
 
     # fused down + weighted accumulate with the shared expert's down matrix as one more slot and the per-expert
     # down bias inside the weighted sum (forward.zig:6362-6389, 6501-6545, 6923-6927)
     def dispatchMoeDownAccEx(self, quant_type, A, x, y, routing, M, K, expert_stride, n_used, x_expert_stride,
                              shared=None, bias=None, x_offset=0, y_offset=0):
-        A, x, y, routing = map(_buf, (A, x, y, routing))
-        none = Buffer(None, 0)
-        sd = _buf(shared) if shared is not None else none
-        bd = _buf(bias) if bias is not None else none
-        self.ctx.call("zc_moe_down_acc_ex", quant_type, A.ptr, A.size, sd.ptr, sd.size, bd.ptr, bd.size, x.ptr,
-                      x.size, y.ptr, y.size, routing.ptr, routing.size, M, K, expert_stride, n_used,
-                      x_expert_stride, x_offset, y_offset)
+        rc = self._f["zc_moe_down_acc_ex"](self.ctx.handle, quant_type, A, shared, bias, x, y, routing, M, K,
+                                           expert_stride, n_used, x_expert_stride, x_offset, y_offset)
+        if rc:
+            self.ctx.fail("zc_moe_down_acc_ex", rc)
 
     # router DMMV (optionally behind the RMS norm) + softmax_topk (+ the expert-parallel filter) in one launch
     # (forward.zig:6139-6190). routing = [k + shared_slot ids][k + shared_slot weights].
     def dispatchMoeRouterTopk(self, hidden, router_weights, logits, routing, n_experts, K, k,
                               rule=ROUTE_TOPK_THEN_SOFTMAX, bias=None, norm_weights=None, norm_out=None, eps=0.0,
                               shared_slot=False, routing_local=None, e_lo=0, e_hi=0, local_shared=False):
-        h, w, lg, rt = map(_buf, (hidden, router_weights, logits, routing))
-        none = Buffer(None, 0)
-        b = _buf(bias) if bias is not None else none
-        nw = _buf(norm_weights) if norm_weights is not None else none
-        no = _buf(norm_out) if norm_out is not None else none
-        rl = _buf(routing_local) if routing_local is not None else none
-        self.ctx.call("zc_moe_router_topk", h.ptr, h.size, nw.ptr, nw.size, w.ptr, w.size, b.ptr, b.size, no.ptr,
-                      no.size, lg.ptr, lg.size, rt.ptr, rt.size, rl.ptr, rl.size, n_experts, K, k, rule,
-                      C.c_float(eps), 1 if shared_slot else 0, e_lo, e_hi if routing_local is not None else 0,
-                      1 if local_shared else 0)
+        rc = self._f["zc_moe_router_topk"](self.ctx.handle, hidden, norm_weights, router_weights, bias, norm_out,
+                                           logits, routing, routing_local, n_experts, K, k, rule, eps, 1 if
+                                           shared_slot else 0, e_lo, e_hi if routing_local is not None else 0, 1 if
+                                           local_shared else 0)
+        if rc:
+            self.ctx.fail("zc_moe_router_topk", rc)
 
     # fused down + weighted accumulate (forward.zig:6362-6389)
     def dispatchMoeFusedDownAcc(self, quant_type, A, x, y, routing, M, K, expert_stride, n_used, x_expert_stride,
@@ -445,32 +509,33 @@ class DmmvDispatch:
 
     # fused RMS norm + f32 router DMMV (src/shaders/rms_norm_dmmv_f32.comp; src/compute/forward.zig:3469)
     def dispatchRmsNormDmmvF32(self, hidden, norm_weights, router_weights, norm_out, logits, M, K, eps):
-        h, w, r, lg = _buf(hidden), _buf(norm_weights), _buf(router_weights), _buf(logits)
-        no = _buf(norm_out) if norm_out is not None else Buffer(None, 0)
-        self.ctx.call("zc_rms_norm_dmmv_f32", h.ptr, h.size, w.ptr, w.size, r.ptr, r.size, no.ptr, no.size,
-                      lg.ptr, lg.size, M, K, C.c_float(eps))
+        rc = self._f["zc_rms_norm_dmmv_f32"](self.ctx.handle, hidden, norm_weights, router_weights, norm_out, logits,
+                                             M, K, eps)
+        if rc:
+            self.ctx.fail("zc_rms_norm_dmmv_f32", rc)
 
     # dispatchDmmvOprojMerge (src/compute/forward.zig:8360-8411): split-K attention merge + O projection
     def dispatchDmmvOprojMerge(self, quant_type, o_tensor, partial_buf, sinks_buf, hidden_buf, M, K, n_heads,
                                n_i_chunks, sink_offset, head_dim, acc_mode=1, a_offset=0, y_offset=0):
-        A, p, y = map(_buf, (o_tensor, partial_buf, hidden_buf))
-        s = _buf(sinks_buf) if sinks_buf is not None else Buffer(None, 0)
-        self.ctx.call("zc_dmmv_o_proj_merge", quant_type, A.ptr, A.size, p.ptr, p.size, y.ptr, y.size, s.ptr, s.size,
-                      M, K, a_offset, y_offset, acc_mode, n_heads, n_i_chunks, sink_offset, head_dim)
+        rc = self._f["zc_dmmv_o_proj_merge"](self.ctx.handle, quant_type, o_tensor, partial_buf, hidden_buf,
+                                             sinks_buf, M, K, a_offset, y_offset, acc_mode, n_heads, n_i_chunks,
+                                             sink_offset, head_dim)
+        if rc:
+            self.ctx.fail("zc_dmmv_o_proj_merge", rc)
 
     # fused RMS norm + alpha / beta SSM projections (src/shaders/rms_norm_dmmv_q4k_alpha_beta.comp)
     def dispatchRmsNormDmmvAlphaBeta(self, hidden, norm_weights, alpha_weights, beta_weights, norm_out, alpha_out,
                                      beta_out, M, K, eps):
-        h, w, a, b, ao, bo = map(_buf, (hidden, norm_weights, alpha_weights, beta_weights, alpha_out, beta_out))
-        no = _buf(norm_out) if norm_out is not None else Buffer(None, 0)
-        self.ctx.call("zc_rms_norm_dmmv_alpha_beta", h.ptr, h.size, w.ptr, w.size, a.ptr, a.size, b.ptr, b.size,
-                      no.ptr, no.size, ao.ptr, ao.size, bo.ptr, bo.size, M, K, C.c_float(eps))
+        rc = self._f["zc_rms_norm_dmmv_alpha_beta"](self.ctx.handle, hidden, norm_weights, alpha_weights,
+                                                    beta_weights, norm_out, alpha_out, beta_out, M, K, eps)
+        if rc:
+            self.ctx.fail("zc_rms_norm_dmmv_alpha_beta", rc)
 
     # dispatchMoeWeightedAcc (src/shaders/moe_weighted_acc.comp:23-33)
     def dispatchMoeWeightedAcc(self, a, b, routing, n, n_used, src_stride):
-        a, b, routing = map(_buf, (a, b, routing))
-        self.ctx.call("zc_moe_weighted_acc", a.ptr, a.size, b.ptr, b.size, routing.ptr, routing.size, n, n_used,
-                      src_stride)
+        rc = self._f["zc_moe_weighted_acc"](self.ctx.handle, a, b, routing, n, n_used, src_stride)
+        if rc:
+            self.ctx.fail("zc_moe_weighted_acc", rc)
 
     # dispatchFfnActivation (forward.zig:3620-3727): swiglu / swiglu_oai
     def dispatchSwiglu(self, gate, up, y, n, oai=False):
@@ -482,43 +547,46 @@ class DmmvDispatch:
 
     # dispatchBiasAddSlice (forward.zig:3875-3913): out[i] += bias[element_offset + i]
     def dispatchBiasAddSlice(self, out, bias, element_offset, n_elements):
-        out, bias = _buf(out), _buf(bias)
-        self.ctx.call("zc_bias_add", out.ptr, out.size, bias.ptr, bias.size, n_elements, element_offset)
+        rc = self._f["zc_bias_add"](self.ctx.handle, out, bias, n_elements, element_offset)
+        if rc:
+            self.ctx.fail("zc_bias_add", rc)
 
     # per-expert gate / up biases + activation for all selected slots (forward.zig:6841-6860)
     def dispatchMoeBiasAct(self, gate, up, gate_bias, up_bias, routing, y, M, n_used, n_experts, oai=False):
-        gate, up, routing, y = map(_buf, (gate, up, routing, y))
-        gb = _buf(gate_bias) if gate_bias is not None else Buffer(None, 0)
-        ub = _buf(up_bias) if up_bias is not None else Buffer(None, 0)
-        self.ctx.call("zc_moe_bias_act", gate.ptr, gate.size, up.ptr, up.size, gb.ptr, gb.size, ub.ptr, ub.size,
-                      routing.ptr, routing.size, y.ptr, y.size, M, n_used, n_experts, 1 if oai else 0)
+        rc = self._f["zc_moe_bias_act"](self.ctx.handle, gate, up, gate_bias, up_bias, routing, y, M, n_used,
+                                        n_experts, 1 if oai else 0)
+        if rc:
+            self.ctx.fail("zc_moe_bias_act", rc)
 
     # per-expert down bias inside the weighted sum (forward.zig:6923-6927)
     def dispatchMoeWeightedBiasAcc(self, a, bias, routing, n, n_used, n_experts):
-        a, bias, routing = map(_buf, (a, bias, routing))
-        self.ctx.call("zc_moe_weighted_bias_acc", a.ptr, a.size, bias.ptr, bias.size, routing.ptr, routing.size,
-                      n, n_used, n_experts)
+        rc = self._f["zc_moe_weighted_bias_acc"](self.ctx.handle, a, bias, routing, n, n_used, n_experts)
+        if rc:
+            self.ctx.fail("zc_moe_weighted_bias_acc", rc)
 
     # expert parallelism: keep (and renumber) the slots whose expert lies in [expert_lo, expert_hi)
     def dispatchMoeEpFilter(self, routing, out, k, expert_lo, expert_hi, n_tokens=1, routing_stride=None, out_stride=None):
-        routing, out = _buf(routing), _buf(out)
-        self.ctx.call("zc_moe_ep_filter", routing.ptr, routing.size, out.ptr, out.size, k, n_tokens,
-                      2 * k if routing_stride is None else routing_stride, 2 * k if out_stride is None else out_stride,
-                      expert_lo, expert_hi)
+        rc = self._f["zc_moe_ep_filter"](self.ctx.handle, routing, out, k, n_tokens, 2 * k if routing_stride is None
+                                         else routing_stride, 2 * k if out_stride is None else out_stride, expert_lo,
+                                         expert_hi)
+        if rc:
+            self.ctx.fail("zc_moe_ep_filter", rc)
 
     # grouped-by-expert prefill helpers (src/shaders/metal/moe_route_pack.metal, moe_route_scatter.metal)
     def dispatchMoeRoutePack(self, routing, counts, ids, n_tokens, n_experts, k, routing_stride, ids_stride):
-        routing, counts, ids = map(_buf, (routing, counts, ids))
-        self.ctx.call("zc_moe_route_pack", routing.ptr, routing.size, counts.ptr, counts.size, ids.ptr, ids.size,
-                      n_tokens, n_experts, k, routing_stride, ids_stride)
+        rc = self._f["zc_moe_route_pack"](self.ctx.handle, routing, counts, ids, n_tokens, n_experts, k,
+                                          routing_stride, ids_stride)
+        if rc:
+            self.ctx.fail("zc_moe_route_pack", rc)
 
     def dispatchMoeRouteScatter(self, routing, src, dst, n_tokens, hidden_dim, k, routing_stride):
-        routing, src, dst = map(_buf, (routing, src, dst))
-        self.ctx.call("zc_moe_route_scatter", routing.ptr, routing.size, src.ptr, src.size, dst.ptr, dst.size,
-                      n_tokens, hidden_dim, k, routing_stride)
+        rc = self._f["zc_moe_route_scatter"](self.ctx.handle, routing, src, dst, n_tokens, hidden_dim, k,
+                                             routing_stride)
+        if rc:
+            self.ctx.fail("zc_moe_route_scatter", rc)
 
     # dequantRow on the device (forward.zig:242-465), bit-exact
     def dequantRows(self, quant_type, A, out, first_row, n_rows, K, a_offset=0):
-        A, out = _buf(A), _buf(out)
-        self.ctx.call("zc_dequant_rows", quant_type, A.ptr, A.size, out.ptr, out.size, first_row, n_rows, K,
-                      a_offset)
+        rc = self._f["zc_dequant_rows"](self.ctx.handle, quant_type, A, out, first_row, n_rows, K, a_offset)
+        if rc:
+            self.ctx.fail("zc_dequant_rows", rc)
