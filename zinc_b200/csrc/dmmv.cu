@@ -9,6 +9,7 @@
 // dmmv_q4k_moe_fused_down_acc.comp and their per-type siblings).
 #include "kernels.h"
 #include "rowdot.cuh"
+#include "stream_common.cuh"
 
 namespace zc {
 
@@ -31,6 +32,28 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint64_t row_bytes = (uint64_t)(a.K / block_size(TYPE)) * bytes_per_block(TYPE);
+    // A chained launch: the weights depend on no kernel, so a plain matvec asks for the first 4 KB of its rows while the
+    // kernel before drains, and lets its own successor do the same at once (unless its predecessor did that with the
+    // routing still in flight). 512 x 2048 Q8_0, one call after the other: bound by this latency, not by its 1.1 MB.
+    if (MODE == MODE_PLAIN) {
+        if (!a.late) chain_release();
+        const uint32_t r0 = (blockIdx.x * kWarps + warp) * NR;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const uint64_t off = (uint64_t)lane * 128;
+            if (r0 + r < a.M && off < row_bytes)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.A + (uint64_t)(r0 + r) * row_bytes + off));
+        }
+    }
+    chain_wait();
+    if (MODE != MODE_PLAIN || a.late) chain_release();
+    const float *a_x = a.x, *a_gate = a.gate;
+    float* a_y = a.y;
+    const uint32_t* a_routing = a.routing;
+    after_wait(a_x);
+    after_wait(a_y);
+    after_wait(a_routing);
+    after_wait(a_gate);
 
     if constexpr (MODE == MODE_PLAIN || MODE == MODE_SIGMOID_ACC) {
         const uint32_t row0 = (blockIdx.x * kWarps + warp) * NR;
@@ -41,16 +64,16 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
         float acc[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = 0.f;
-        rowdot<TYPE, NR, ALIGNED>(rows, a.x, a.K, lane, acc);
+        rowdot<TYPE, NR, ALIGNED>(rows, a_x, a.K, lane, acc);
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = warp_sum(acc[r]);
         if (lane == 0) {
             float g = 1.f;
-            if constexpr (MODE == MODE_SIGMOID_ACC) g = 1.0f / (1.0f + expf(-__ldg(a.gate)));
+            if constexpr (MODE == MODE_SIGMOID_ACC) g = 1.0f / (1.0f + expf(-__ldg(a_gate)));
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
                 if (row0 + r < a.M) {
-                    float* yp = a.y + row0 + r;
+                    float* yp = a_y + row0 + r;
                     if constexpr (MODE == MODE_SIGMOID_ACC) {
                         *yp += g * acc[r];
                     } else if (a.push.world) {  // fused exchange: the row goes to every rank's receive buffer
@@ -67,22 +90,22 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
         if (row >= a.M) return;
         const uint8_t* rows[2] = {a.A + (uint64_t)row * row_bytes, a.A2 + (uint64_t)row * row_bytes};
         float acc[2] = {0.f, 0.f};
-        rowdot<TYPE, 2, ALIGNED>(rows, a.x, a.K, lane, acc);
+        rowdot<TYPE, 2, ALIGNED>(rows, a_x, a.K, lane, acc);
         const float g = warp_sum(acc[0]), u = warp_sum(acc[1]);
-        if (lane == 0) a.y[row] = (g / (1.0f + expf(-g))) * u;
+        if (lane == 0) a_y[row] = (g / (1.0f + expf(-g))) * u;
     } else if constexpr (MODE == MODE_MOE) {
         const uint32_t slot = blockIdx.y;
         const uint32_t row0 = (blockIdx.x * kWarps + warp) * NR;
         if (row0 >= a.M) return;
-        const uint32_t e_raw = __ldg(a.routing + slot);
+        const uint32_t e_raw = __ldg(a_routing + slot);
         if (e_raw == kSkipExpert) {  // no expert in this slot on this rank: zeros
             if (lane == 0)
                 for (int r = 0; r < NR; ++r)
-                    if (row0 + r < a.M) a.y[(size_t)slot * a.M + row0 + r] = 0.f;
+                    if (row0 + r < a.M) a_y[(size_t)slot * a.M + row0 + r] = 0.f;
             return;
         }
         const uint8_t* base = a.A + (uint64_t)checked_expert(e_raw, a.n_experts_max, a.status) * a.expert_stride;
-        const float* x = a.x + (size_t)slot * a.x_expert_stride;
+        const float* x = a_x + (size_t)slot * a.x_expert_stride;
         const uint8_t* rows[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) rows[r] = base + (uint64_t)min(row0 + r, a.M - 1) * row_bytes;
@@ -95,26 +118,26 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
         if (lane == 0) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-                if (row0 + r < a.M) a.y[(size_t)slot * a.M + row0 + r] = acc[r];
+                if (row0 + r < a.M) a_y[(size_t)slot * a.M + row0 + r] = acc[r];
         }
     } else if constexpr (MODE == MODE_MOE_GATE_UP) {
         // NR row pairs (gate row, up row) per warp: independent load chains share the x loads
         const uint32_t slot = blockIdx.y;
         const uint32_t row0 = (blockIdx.x * kWarps + warp) * NR;
         if (row0 >= a.M) return;
-        const uint32_t e_raw = __ldg(a.routing + slot);
+        const uint32_t e_raw = __ldg(a_routing + slot);
         if (e_raw == kSkipExpert) {  // no expert in this slot on this rank: zeros
             if (lane == 0)
                 for (int r = 0; r < NR; ++r)
                     if (row0 + r < a.M) {
-                        a.y[(size_t)slot * a.M + row0 + r] = 0.f;
+                        a_y[(size_t)slot * a.M + row0 + r] = 0.f;
                         if (!a.act) a.y2[(size_t)slot * a.M + row0 + r] = 0.f;
                     }
             return;
         }
         const uint8_t* mg = expert_matrix(a.A, a.A_sh, e_raw, a.expert_stride, a.n_experts_max, a.status);
         const uint8_t* mu = expert_matrix(a.A2, a.A2_sh, e_raw, a.expert_stride, a.n_experts_max, a.status);
-        const float* x = a.x + (size_t)slot * a.x_expert_stride;
+        const float* x = a_x + (size_t)slot * a.x_expert_stride;
         const uint8_t* rows[2 * NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
@@ -138,9 +161,9 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
                         if (a.bias2) vu += __ldg(a.bias2 + (size_t)e_raw * a.M + row0 + r);
                     }
                     if (a.act) {
-                        a.y[(size_t)slot * a.M + row0 + r] = gate_up_act_v1(a.act, vg, vu);
+                        a_y[(size_t)slot * a.M + row0 + r] = gate_up_act_v1(a.act, vg, vu);
                     } else {
-                        a.y[(size_t)slot * a.M + row0 + r] = vg;
+                        a_y[(size_t)slot * a.M + row0 + r] = vg;
                         a.y2[(size_t)slot * a.M + row0 + r] = vu;
                     }
                 }
@@ -155,27 +178,27 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
         float acc[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = 0.f;
-        rowdot<TYPE, NR, ALIGNED>(rows, a.x + (size_t)col * a.x_expert_stride, a.K, lane, acc);
+        rowdot<TYPE, NR, ALIGNED>(rows, a_x + (size_t)col * a.x_expert_stride, a.K, lane, acc);
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = warp_sum(acc[r]);
         if (lane == 0) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-                if (row0 + r < a.M) a.y[(size_t)col * a.M + row0 + r] = acc[r];
+                if (row0 + r < a.M) a_y[(size_t)col * a.M + row0 + r] = acc[r];
         }
     } else if constexpr (MODE == MODE_MOE_BATCHED) {
         const uint32_t slot = blockIdx.y, tok = blockIdx.z;
         const uint32_t row = blockIdx.x * kWarps + warp;
         if (row >= a.M) return;
-        const uint32_t e_raw = __ldg(a.routing + (size_t)tok * a.n_used + slot);
+        const uint32_t e_raw = __ldg(a_routing + (size_t)tok * a.n_used + slot);
         if (e_raw == kSkipExpert) return;
         const uint32_t e = checked_expert(e_raw, a.n_experts_max, a.status);
         if (e != e_raw) return;  // not an expert: reported, its output row stays untouched (as on the grouped path)
         const uint8_t* rows[1] = {a.A + (uint64_t)e * a.expert_stride + (uint64_t)row * row_bytes};
         float acc[1] = {0.f};
-        rowdot<TYPE, 1, ALIGNED>(rows, a.x + (size_t)tok * a.x_token_stride, a.K, lane, acc);
+        rowdot<TYPE, 1, ALIGNED>(rows, a_x + (size_t)tok * a.x_token_stride, a.K, lane, acc);
         const float v = warp_sum(acc[0]);
-        if (lane == 0) a.y[(size_t)tok * a.y_token_stride + (size_t)slot * a.M + row] = v;
+        if (lane == 0) a_y[(size_t)tok * a.y_token_stride + (size_t)slot * a.M + row] = v;
     } else {  // MODE_MOE_DOWN_ACC: NR rows per warp, the slots in sequence
         const uint32_t row0 = (blockIdx.x * kWarps + warp) * NR;
         if (row0 >= a.M) return;
@@ -183,17 +206,17 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) total[r] = 0.f;
         for (uint32_t s = 0; s < a.n_used; ++s) {
-            const uint32_t e_raw = __ldg(a.routing + s);
+            const uint32_t e_raw = __ldg(a_routing + s);
             if (e_raw == kSkipExpert) continue;
             const uint8_t* base = expert_matrix(a.A, a.A_sh, e_raw, a.expert_stride, a.n_experts_max, a.status);
             const uint8_t* rows[NR];
 #pragma unroll
             for (int r = 0; r < NR; ++r) rows[r] = base + (uint64_t)min(row0 + r, a.M - 1) * row_bytes;
-            const float w = __uint_as_float(__ldg(a.routing + a.n_used + s));
+            const float w = __uint_as_float(__ldg(a_routing + a.n_used + s));
             float acc[NR];
 #pragma unroll
             for (int r = 0; r < NR; ++r) acc[r] = 0.f;
-            rowdot<TYPE, NR, ALIGNED>(rows, a.x + (size_t)s * a.x_expert_stride, a.K, lane, acc);
+            rowdot<TYPE, NR, ALIGNED>(rows, a_x + (size_t)s * a.x_expert_stride, a.K, lane, acc);
 #pragma unroll
             for (int r = 0; r < NR; ++r) total[r] = fmaf(w, acc[r], total[r]);
             if (a.bias && lane == 0 && e_raw < a.n_experts_max) {  // the expert's bias, weighted like its product
@@ -207,7 +230,7 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
         if (lane == 0) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
-                if (row0 + r < a.M) a.y[row0 + r] += total[r];
+                if (row0 + r < a.M) a_y[row0 + r] += total[r];
         }
     }
 }
@@ -220,8 +243,7 @@ cudaError_t launch_one(const DmmvArgs& a, cudaStream_t s) {
                    MODE == MODE_MOE_GATE_UP || MODE == MODE_MOE_DOWN_ACC) ? NR : 1);
     dim3 grid((a.M + rows_per_cta - 1) / rows_per_cta, per_slot ? a.n_used : 1,
               MODE == MODE_MOE_BATCHED ? a.n_tokens : 1);
-    dmmv_kernel<TYPE, MODE, NR, ALIGNED><<<grid, kWarps * 32, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(dmmv_kernel<TYPE, MODE, NR, ALIGNED>, grid, dim3(kWarps * 32), 0, s, a);
 }
 
 template <uint32_t TYPE, bool ALIGNED>

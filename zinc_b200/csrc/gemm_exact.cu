@@ -1,6 +1,7 @@
 // Preparation of the activations and dispatch of the f32-accurate prefill GEMM (gemm_exact.cuh).
 #include "common.cuh"
 #include "kernels.h"
+#include "stream_common.cuh"
 
 namespace zc {
 namespace {
@@ -69,10 +70,13 @@ __device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t h) {
 // the terms, 4 + 4 per element; 4096 x 658: 3 us.
 template <int ORDER, bool BF16>
 __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs a) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    chain_wait();
+    chain_release();  // the GEMM's set-up and its first weight blocks overlap this kernel
     __shared__ float s_max[kPrepThreads / 32];
     const uint32_t t = blockIdx.x, tid = threadIdx.x;
-    const void* row = static_cast<const uint8_t*>(a.X) + (uint64_t)t * a.stride_b * (BF16 ? 2 : 4);
+    const void* X = a.X;
+    after_wait(X);
+    const void* row = static_cast<const uint8_t*>(X) + (uint64_t)t * a.stride_b * (BF16 ? 2 : 4);
     float mx = 0.f;
     for (uint32_t k = tid * 4; k < a.K; k += kPrepThreads * 4) {
         const float4 v = load4<BF16>(row, k, a.K, a.vec);
@@ -151,8 +155,7 @@ template <int ORDER, bool BF16>
 cudaError_t launch_prep(const void* args, bool split, cudaStream_t s) {
     PrepArgs a = *static_cast<const PrepArgs*>(args);
     a.zero = split;
-    exact_prep_kernel<ORDER, BF16><<<a.tokens, kPrepThreads, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(kPrepThreads), 0, s, a);
 }
 
 cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {

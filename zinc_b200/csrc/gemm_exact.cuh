@@ -493,38 +493,38 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         const uint32_t full_a0 = leader_addr(&bars->full_a[j * T::kABuf]);
         const uint32_t pfree0 = leader_addr(&bars->pfree[0]), pfree1 = leader_addr(&bars->pfree[1]);
         const uint32_t full_m = kMin ? leader_addr(&bars->full_m[0]) : 0u;
-        const uint64_t row_bytes = (uint64_t)(g.K >> 5) * (kBlock / 8);
+        const uint64_t pitch = TYPE == T_Q8_0 || TYPE == T_MXFP4 ? (uint64_t)(g.K >> 5) * (kBlock / 8) : (uint64_t)(g.K >> 8) * kBlock;
         auto row_off = [&](uint32_t tile) {  // rows past M: computed, dropped
-            return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * (TYPE == T_Q8_0 || TYPE == T_MXFP4
-                                                                               ? row_bytes
-                                                                               : (uint64_t)(g.K >> 8) * kBlock);
+            return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * pitch;
         };
         if constexpr (kMin) {  // columns 24..31 of the min step are zeros
             if (j < 2)
                 *reinterpret_cast<uint4*>(smem + T::kMinOffset + j * T::kMinBytes + row * 64 + ((3 ^ ((row >> 1) & 3)) << 4)) =
                     make_uint4(0, 0, 0, 0);
         }
-        // fetched rows: thread (row, j) copies pieces j, j + 4, ... of the aligned superset of its row's block
+        // fetched rows: the 16-byte pieces of the aligned supersets of the 128 rows' blocks, dealt to the 512 threads row by
+        // row (a warp's copy instruction then meets a handful of cache lines instead of 32)
         uint32_t uf = u_begin, f_b = 0, f_pw = 1;
         int f_sw = 0;
         XSegment f_seg{0, 0, 0};
         bool f_live = false;
-        uint64_t f_off = 0, c_off = 0;
+        uint32_t f_m0 = 0;
+        uint64_t c_off = 0;
         auto fetch = [&]() -> bool {
             if (!f_live) return true;
             if (!poll_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 306)) return false;
-            const uint64_t o = f_off + (uint64_t)f_b * kBlock;
-            const uint8_t* src = g.A + (o & ~(uint64_t)15);
-            uint8_t* dst = smem_w + f_sw * T::kWBytes + row * kRow;
+            uint8_t* dst = smem_w + f_sw * T::kWBytes;
             constexpr int kPieces = (kBlock + 15 + 15) / 16;
             static_assert(!kFetch || kPieces * 16 <= (int)kRow, "a fetched row fits its slot");
+            const uint32_t pi = (uint32_t)tid - 96;
 #pragma unroll
-            for (int pc = 0; pc < kPieces; pc += 4) {
-                const int piece = pc + j;
-                if (piece < kPieces) {
-                    const uint8_t* sp = src + piece * 16;
+            for (int i = 0; i < (kBM * kPieces + 511) / 512; ++i) {
+                const uint32_t idx = pi + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
+                if ((kBM * kPieces) % 512 == 0 || r < (uint32_t)kBM) {
+                    const uint64_t o = (uint64_t)min(f_m0 + r, g.M - 1) * pitch + (uint64_t)f_b * kBlock;
+                    const uint8_t* sp = g.A + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t n = sp + 16 <= g.a_end ? 16u : (sp < g.a_end ? (uint32_t)(g.a_end - sp) : 0u);
-                    cp_async16_zfill(dst + piece * 16, n ? sp : g.A, n);
+                    cp_async16_zfill(dst + r * kRow + piece * 16, n ? sp : g.A, n);
                 }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[f_sw])) : "memory");
@@ -533,7 +533,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (++f_b == f_seg.b1) {
                 f_live = x_next_segment(uf, u_end, nblk, f_seg);
                 f_b = f_seg.b0;
-                if (f_live) f_off = row_off(f_seg.tile);
+                if (f_live) f_m0 = tile_m0(f_seg.tile);
             }
             return true;
         };
@@ -541,7 +541,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         if constexpr (kFetch) {
             f_live = x_next_segment(uf, u_end, nblk, f_seg);
             f_b = f_seg.b0;
-            if (f_live) f_off = row_off(f_seg.tile);
+            if (f_live) f_m0 = tile_m0(f_seg.tile);
             ok = fetch();
         }
         float2 acc[BN / 8];

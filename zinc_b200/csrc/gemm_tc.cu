@@ -45,6 +45,21 @@ struct GemmArgs {
     uint32_t* status;
 };
 
+// Zeroes an N x M output (row stride stride_d) or a run of tile flags for the GEMM launched behind it, whose set-up and
+// main loop overlap this kernel: released once the kernels before are done, waited for before the GEMM's first add. (A memset node in its
+// place held the GEMM back for 2 us.)
+__global__ void __launch_bounds__(256) zero_kernel(float* D, uint32_t M, uint32_t stride_d) {
+    chain_wait();
+    chain_release();
+    float* d = D + (uint64_t)blockIdx.x * stride_d;
+    if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+        for (uint32_t m = threadIdx.x * 4; m + 4 <= M; m += 1024) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (threadIdx.x < (M & 3u)) d[(M & ~3u) + threadIdx.x] = 0.f;
+    } else {
+        for (uint32_t m = threadIdx.x; m < M; m += 256) d[m] = 0.f;
+    }
+}
+
 template <int TYPE, int BN, int NACC>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_w,
@@ -145,6 +160,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         if (lane == 0) {
             // ---- TMA loader of X and, with two accumulators (whose second issuer has the third control warp),
             // of the raw weight blocks too: polls both rings without suspending on either ----
+            chain_wait();  // the activations; the weights depend on no kernel
             int sb = 0, it = 0, acc = 0;
             uint32_t pb = 1, fill = 0;
             int sw = 0, b = NACC == 2 ? b_begin : b_end;
@@ -253,6 +269,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
         // ---- epilogue: all sixteen producer warps (the stores take the time: the more in flight the better);
         // TMEM lane quarter = warp % 4, set j takes the column chunks c = j mod 4 ----
         {
+            chain_wait();  // D: zeroed, and no longer read or written by the kernels before
             if (wait_or_fail(&bars->accum, 0, bars, g.status, 105)) {
                 __syncwarp();
                 tc_fence_after();
@@ -463,6 +480,20 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
             if (w_live) w_m0 = tile_m0(sw_seg.tile);
             int sbl = 0, sw = 0;
             uint32_t pbl = 1, pw = 1, idle = 0;
+            for (int i = 0; i < kWSlots && w_live; ++i) {  // the first weight blocks depend on no kernel
+                mbar_expect_tx(&bars->full_w[i], kWBytes);
+                tma_load_2d(smem_w + i * kWBytes, &tmap_w, (int)((w_b * Raw<TYPE>::kBlock) & ~15u), (int)w_m0, &bars->full_w[i]);
+                if (++w_b == sw_seg.b1) {
+                    w_live = next_segment(uw, u_end, nblk, sw_seg);
+                    w_b = sw_seg.b0;
+                    if (w_live) w_m0 = tile_m0(sw_seg.tile);
+                }
+                if (++sw == kWSlots) {
+                    sw = 0;
+                    pw ^= 1;
+                }
+            }
+            chain_wait();  // the activations
             while (b_live || w_live) {
                 bool moved = false;
                 if (b_live && mbar_test_wait(&bars->empty_b[sbl], pbl)) {
@@ -523,8 +554,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
         uint32_t pw = 0, gb = 0, seg_i = 0, u = u_begin;
         bool ok = true;
         Segment sg;
-        // kFetch: the dequant threads fetch the raw blocks themselves, one ring slot (a block) ahead: thread (row, j)
-        // copies the 16-byte pieces j, j + 4, ... of the aligned superset of its row's block (136 or 210 bytes)
+        // kFetch: the dequant threads fetch the raw blocks themselves, one ring slot (a block) ahead: the 16-byte pieces
+        // of the aligned supersets of the 128 rows' blocks (136 or 210 bytes), dealt to the threads row by row (a warp's
+        // copy instruction then meets a handful of cache lines instead of 32)
         constexpr uint32_t kRawBlock = Raw<TYPE>::kBlock, kRawRow = Raw<TYPE>::kBox;
         constexpr int kRawPieces = TYPE == T_MXFP4 ? 10 : 15;  // (15 + block bytes) / 16 rounded up
         const uint64_t mx_row_bytes = TYPE == T_MXFP4 ? (uint64_t)(g.K >> 5) * 17u : (uint64_t)(g.K >> 8) * kRawBlock;
@@ -532,23 +564,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
         int f_sw = 0;
         Segment f_seg{0, 0, 0};
         bool f_live = false;
-        uint64_t f_row_off = 0, c_row_off = 0;
+        uint32_t f_m0 = 0;
+        uint64_t c_row_off = 0;
         auto mx_row_off = [&](uint32_t tile) {
             return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * mx_row_bytes;  // rows past M: computed, dropped
         };
         auto mx_fetch = [&]() -> bool {
             if (!f_live) return true;
             if (!wait_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 111)) return false;
-            const uint64_t o = f_row_off + (uint64_t)f_b * kRawBlock;
-            const uint8_t* src = g.A + (o & ~(uint64_t)15);
-            uint8_t* dst = smem_w + f_sw * kWBytes + row * kRawRow;
+            uint8_t* dst = smem_w + f_sw * kWBytes;
 #pragma unroll
-            for (int pc = 0; pc < 16; pc += 4) {
-                const int piece = pc + j;
-                if (piece < kRawPieces) {
-                    const uint8_t* sp = src + piece * 16;
+            for (int i = 0; i < (kBM * kRawPieces + 511) / 512; ++i) {
+                const uint32_t idx = (uint32_t)pi + 512u * i, r = idx / kRawPieces, piece = idx - r * kRawPieces;
+                if ((kBM * kRawPieces) % 512 == 0 || r < (uint32_t)kBM) {
+                    const uint64_t o = (uint64_t)min(f_m0 + r, g.M - 1) * mx_row_bytes + (uint64_t)f_b * kRawBlock;
+                    const uint8_t* sp = g.A + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t nbytes = sp + 16 <= p.a_end ? 16u : (sp < p.a_end ? (uint32_t)(p.a_end - sp) : 0u);
-                    cp_async16_zfill(dst + piece * 16, nbytes ? sp : g.A, nbytes);
+                    cp_async16_zfill(dst + r * kRawRow + piece * 16, nbytes ? sp : g.A, nbytes);
                 }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[f_sw])) : "memory");
@@ -559,14 +591,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
             if (++f_b == f_seg.b1) {
                 f_live = next_segment(uf, u_end, nblk, f_seg);
                 f_b = f_seg.b0;
-                if (f_live) f_row_off = mx_row_off(f_seg.tile);
+                if (f_live) f_m0 = tile_m0(f_seg.tile);
             }
             return true;
         };
         if constexpr (kFetch) {
             f_live = next_segment(uf, u_end, nblk, f_seg);
             f_b = f_seg.b0;
-            if (f_live) f_row_off = mx_row_off(f_seg.tile);
+            if (f_live) f_m0 = tile_m0(f_seg.tile);
             for (int d = 0; d < kWSlots - 1 && ok; ++d) ok = mx_fetch();
         }
         while (ok && next_segment(u, u_end, nblk, sg)) {
@@ -627,6 +659,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
             // the time: the more in flight the better). TMEM lane quarter = warp % 4; set j takes the column chunks
             // c = j mod 4. ----
             {
+                chain_wait();  // D and the flags: zeroed, and no longer read or written by the kernels before
                 if (!wait_or_fail(&bars->accum, seg_i & 1, bars, g.status, 105)) { ok = false; break; }
                 __syncwarp();
                 tc_fence_after();
@@ -782,6 +815,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs 
         }
     } else if (warp == 1) {
         if (lane == 0) {  // ---- TMA loader of the activations ----
+            chain_wait();
             for (int it = 0; it < n_it; ++it) {
                 const int st = it & 3;
                 if (!wait_or_fail(&bars->empty_a[st], ((it >> 2) & 1) ^ 1, bars, g.status, 113)) break;
@@ -833,6 +867,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs 
         // ---- epilogue: all sixteen producer warps, TMEM lane quarter = warp % 4, each group of four warps its own
         // column chunks; a lane is a token, columns are rows ----
         {
+            chain_wait();
             if (wait_or_fail(&bars->accum, 0, bars, g.status, 115)) {
                 __syncwarp();
                 tc_fence_after();
@@ -931,12 +966,10 @@ cudaError_t launch_tile(const uint8_t* A, const void* B, float* D, uint32_t M, u
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 4) --splits;
     if (splits > 1) {
-        cudaError_t e = cudaMemset2DAsync(D, (size_t)stride_d * 4, 0, (size_t)M * 4, N, s);
-        if (e != cudaSuccess) return e;
+        if (cudaError_t e = launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d); e != cudaSuccess) return e;
         grid.z = splits;
     }
-    kern<<<grid, kThreads, Tile<TYPE, BN>::kSmemBytes, s>>>(map, wmap, g);
-    return cudaGetLastError();
+    return launch_chained(kern, grid, dim3(kThreads), Tile<TYPE, BN>::kSmemBytes, s, map, wmap, g);
 }
 
 cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K,
@@ -964,12 +997,10 @@ cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, 
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 2) --splits;
     if (splits > 1) {
-        cudaError_t e = cudaMemset2DAsync(D, (size_t)stride_d * 4, 0, (size_t)M * 4, N, s);
-        if (e != cudaSuccess) return e;
+        if (cudaError_t e = launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d); e != cudaSuccess) return e;
         grid.z = splits;
     }
-    gemm_tc_small_kernel<<<grid, kSmThreads, kSmSmemBytes, s>>>(map, g);
-    return cudaGetLastError();
+    return launch_chained(gemm_tc_small_kernel, grid, dim3(kSmThreads), kSmSmemBytes, s, map, g);
 }
 
 // The persistent pair kernel. cudaErrorNotSupported: the caller takes another path (nothing launched or written).
@@ -994,11 +1025,13 @@ cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, u
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = T::kSmemBytes;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // pairs the device holds at once (every pair of the grid must be resident: pairs wait for each other's tiles)
@@ -1047,11 +1080,10 @@ cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, u
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    if (p.zeroed) {
-        if (cudaError_t e = cudaMemset2DAsync(D, (size_t)stride_d * 4, 0, (size_t)M * 4, N, s); e != cudaSuccess) return e;
-    } else {
-        if (cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)p.n_tiles * 2 * sizeof(uint32_t), s); e != cudaSuccess) return e;
-    }
+    cudaError_t e = p.zeroed ? launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d)
+                             : launch_chained(zero_kernel, dim3(1), dim3(256), 0, s, reinterpret_cast<float*>(flags), p.n_tiles * 2, 0);
+    if (e != cudaSuccess) return e;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, map, wmap, p);
 }
 

@@ -24,6 +24,23 @@ inline cudaError_t ensure_dynamic_smem(Kern kern, int bytes, std::atomic<uint64_
     return cudaSuccess;
 }
 
+// Launch as a programmatic dependent of the kernel before it in the stream: the grid is set up while that kernel drains,
+// and a griddepcontrol.wait in the kernel stands for the dependency (the kernel must execute one in every CTA).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
 // Epilogue / addressing modes of the decode matvec kernel family.
 enum DmmvMode : int {
     MODE_PLAIN = 0,          // y (+)= W x

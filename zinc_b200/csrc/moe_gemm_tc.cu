@@ -34,8 +34,6 @@ constexpr int kMoeThreads = 23 * 32;
 // One activation slot (BN x 64 bf16) per weight stage: its TMA load reports to the stage's own barrier, so the
 // issuing thread waits once and commits once per stage (each wait and each commit costs it a few hundred
 // cycles in this kernel; with a separate activation ring and two waits per stage a layer took 7-20 % longer).
-template <int BN>
-constexpr int moe_x_slots() { return kAStages; }
 constexpr uint32_t kMoeSmemMax = 227u * 1024u;
 
 // The raw-block ring takes what the weight stages and activation slots leave of the 227 KB: its depth is
@@ -44,8 +42,10 @@ template <int TYPE, int BN>
 struct MoeTile {
     static constexpr uint32_t kRawBytes = kBM * Raw<TYPE>::kBox;
     static constexpr uint32_t kXBytes = BN * kBK * 2;
-    static constexpr uint32_t kRawOffset = kAStages * kABytes;
-    static constexpr int kXSlots = moe_x_slots<BN>();
+    // (two stages per dequant set with 32-token tiles took the raw ring its depth: 360 -> 375 us on 256 experts, T = 512)
+    static constexpr int kStages = kAStages;
+    static constexpr uint32_t kRawOffset = kStages * kABytes;
+    static constexpr int kXSlots = kStages;
     static constexpr uint32_t kAvail = kMoeSmemMax - (512 + 1024) - 1024 - kRawOffset - kXSlots * kXBytes;
     static constexpr int kRawSlots = kAvail / kRawBytes > 8 ? 8 : (int)(kAvail / kRawBytes);
     static constexpr uint32_t kXOffset = (kRawOffset + kRawSlots * kRawBytes + 1023u) & ~1023u;
@@ -89,12 +89,19 @@ struct BlockCursor {
     uint32_t w;             // work item
     int b;                  // block of the item
     const uint8_t* expert;  // first byte of the item's expert
+    uint32_t m0;            // first row of the item's row tile
     uint64_t row_off;       // byte offset of this thread's row inside the expert
 };
 
 template <int TYPE, int BN>
 __global__ void __launch_bounds__(kMoeThreads, 1)
-moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs g) {
+moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs args) {
+    // everything this kernel reads but the weights comes from the kernels before it
+    chain_wait();
+    MoeGemmArgs g = args;
+    after_wait(g.header);
+    after_wait(g.tiles);
+    after_wait(g.list);
     using T = MoeTile<TYPE, BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -110,7 +117,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     const uint64_t row_bytes = TYPE == T_MXFP4 ? (uint64_t)(g.K >> 5) * 17u : (uint64_t)nblk * kBlock;
 
     if (tid == 0) {
-        for (int s = 0; s < kAStages; ++s) {
+        for (int s = 0; s < T::kStages; ++s) {
             mbar_init(&bars->full_a[s], 5);  // one arrival per warp of the owning set + the activation box
             mbar_init(&bars->empty_a[s], 1);
         }
@@ -148,8 +155,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                 if (!ok) break;
                 tc_fence_after();
                 for (int s = 0; s < n_stages; ++s, ++gs) {
-                    const int st = gs & 3;
-                    const uint32_t ph = (gs >> 2) & 1;
+                    const int st = gs % T::kStages;
+                    const uint32_t ph = (gs / T::kStages) & 1;
                     ok = warp_poll(smem_u32(&bars->full_a[st]), ph, bars, g.status, 122);
                     if (!ok) break;
                     tc_fence_after();
@@ -172,8 +179,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
                 const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
                 for (int s = 0; s < n_stages; ++s, ++gs) {
-                    const int st = gs & 3;
-                    ok = poll_or_fail(&bars->empty_a[st], ((gs >> 2) & 1) ^ 1, bars, g.status, 124);
+                    const int st = gs % T::kStages;
+                    ok = poll_or_fail(&bars->empty_a[st], ((gs / T::kStages) & 1) ^ 1, bars, g.status, 124);
                     if (!ok) break;
                     mbar_expect_tx(&bars->full_a[st], T::kXBytes);
                     tma_load_2d(smem_x + st * T::kXBytes, &tmap_x, s * kBK, (int)tile.y, &bars->full_a[st]);
@@ -181,34 +188,33 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             }
         }
     } else if (warp >= kMoeDeqWarp0 && warp < kMoeEpiWarp0) {
-        // ---- dequant producers: thread = (row, set j); set j always fills weight stage j. A block that
+        // ---- dequant producers: thread = (row, set j); set j always fills the stages j mod 4. A block that
         // starts at running stage gs hands its group q to set (gs + q) & 3 ----
         const int p = tid - kMoeDeqWarp0 * 32;
         const int row = p & 127, j = p >> 7;
-        uint8_t* a_stage = smem + j * kABytes;
         auto locate = [&](uint32_t w, BlockCursor& c) {
             c.w = w;
             c.b = 0;
             if (w < n_items) {
                 const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
-                const uint32_t m0 = (w % g.row_tiles) * kBM;
-                const uint32_t grow = min(m0 + (uint32_t)row, g.M - 1);  // rows past M are computed and dropped
+                c.m0 = (w % g.row_tiles) * kBM;
+                const uint32_t grow = min(c.m0 + (uint32_t)row, g.M - 1);  // rows past M are computed and dropped
                 c.expert = g.A + (uint64_t)tile.x * g.expert_stride;
                 c.row_off = (uint64_t)grow * row_bytes;
             }
         };
-        // this thread's pieces (j, j + 4, ...) of the aligned superset of its row's block
+        // The 16-byte pieces of the aligned supersets of all rows' blocks, dealt to the 512 threads row by row: a warp's
+        // copy instruction covers three rows' runs of bytes, a handful of cache lines, where one row per lane met 32.
         auto fetch = [&](const BlockCursor& c, uint32_t slot_idx) {
-            const uint64_t o = c.row_off + (uint64_t)c.b * kBlock;
-            const uint8_t* src = c.expert + (o & ~(uint64_t)15);
-            uint8_t* dst = smem_w + slot_idx * T::kRawBytes + row * kBox;
+            uint8_t* slot = smem_w + slot_idx * T::kRawBytes;
 #pragma unroll
-            for (int pc = 0; pc < kPieces; pc += 4) {
-                const int piece = pc + j;
-                if (piece < kPieces) {
-                    const uint8_t* s = src + piece * 16;
+            for (int i = 0; i < (kBM * kPieces + 511) / 512; ++i) {
+                const uint32_t idx = (uint32_t)p + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
+                if ((kBM * kPieces) % 512 == 0 || r < (uint32_t)kBM) {
+                    const uint64_t o = (uint64_t)min(c.m0 + r, g.M - 1) * row_bytes + (uint64_t)c.b * kBlock;
+                    const uint8_t* s = c.expert + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t n = s + 16 <= g.a_end ? 16u : (s < g.a_end ? (uint32_t)(g.a_end - s) : 0u);
-                    cp_async16_zfill(dst + piece * 16, n ? s : g.A, n);
+                    cp_async16_zfill(slot + r * kBox + piece * 16, n ? s : g.A, n);
                 }
             }
         };
@@ -247,8 +253,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             const bool mine = q < ns;
             if (mine && !dead) dead = !poll_or_fail(&bars->full_w[slot_c], use_c & 1, bars, g.status, 128);
             if (mine && !dead)
-                dead = !poll_or_fail(&bars->empty_a[j], (((gs + q) >> 2) & 1) ^ 1, bars, g.status, 125);
+                dead = !poll_or_fail(&bars->empty_a[(gs + q) % T::kStages], (((gs + q) / T::kStages) & 1) ^ 1, bars, g.status, 125);
             if (mine && !dead) {
+                uint8_t* a_stage = smem + ((gs + q) % T::kStages) * kABytes;
                 const uint8_t* slot = smem_w + slot_c * T::kRawBytes + row * kBox;
                 if constexpr (TYPE == T_Q4_K) {
                     const uint4 chdr = *reinterpret_cast<const uint4*>(slot);
@@ -270,7 +277,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->full_a[j]);
+                if (lane == 0) mbar_arrive(&bars->full_a[(gs + q) % T::kStages]);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->empty_w[slot_c]);  // this warp is done with the slot
@@ -339,9 +346,10 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
 // ---- grouping ------------------------------------------------------------------------------------------
 // One CTA. Shared: cnt[n_experts], seg[n_experts] (first list slot, then the running cursor), tstart[n_experts].
 __global__ void __launch_bounds__(1024, 1)
-moe_group_kernel(const uint32_t* __restrict__ routing, uint32_t n_pairs, uint32_t n_experts, uint32_t bn,
-                 uint32_t* __restrict__ header, uint4* __restrict__ tiles, uint32_t* __restrict__ list,
-                 uint32_t* __restrict__ status) {
+moe_group_kernel(const uint32_t* routing, uint32_t n_pairs, uint32_t n_experts, uint32_t bn, uint32_t* header, uint4* tiles,
+                 uint32_t* list, uint32_t* status) {
+    chain_wait();
+    after_wait(routing);
     extern __shared__ uint32_t sh[];
     uint32_t* cnt = sh;
     uint32_t* seg = sh + n_experts;
@@ -402,9 +410,12 @@ moe_group_kernel(const uint32_t* __restrict__ routing, uint32_t n_pairs, uint32_
 
 // One warp per listed pair: its token's activation row as bf16.
 __global__ void __launch_bounds__(256)
-moe_gather_x_kernel(const float* __restrict__ X, const uint32_t* __restrict__ header,
-                    const uint32_t* __restrict__ list, __nv_bfloat16* __restrict__ Xp, uint32_t K, uint32_t n_used,
-                    uint32_t x_token_stride) {
+moe_gather_x_kernel(const float* X, const uint32_t* header, const uint32_t* list, __nv_bfloat16* Xp, uint32_t K,
+                    uint32_t n_used, uint32_t x_token_stride) {
+    chain_wait();
+    after_wait(X);
+    after_wait(header);
+    after_wait(list);
     const uint32_t slot = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (slot >= header[1]) return;
     const uint32_t pair = list[slot];
@@ -448,8 +459,7 @@ cudaError_t launch_gemm(const CUtensorMap& map, const MoeGemmArgs& g, uint32_t m
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t grid = max_items < (uint32_t)sms ? max_items : (uint32_t)sms;
-    kern<<<grid, kMoeThreads, MoeTile<TYPE, BN>::kSmemBytes, s>>>(map, g);
-    return cudaGetLastError();
+    return launch_chained(kern, dim3(grid), dim3(kMoeThreads), MoeTile<TYPE, BN>::kSmemBytes, s, map, g);
 }
 
 // Tokens per tile: 32 when experts see few pairs on average (the activation box then stays small), else 128.
@@ -487,12 +497,11 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
     uint32_t* list = reinterpret_cast<uint32_t*>(base + l.list);
     __nv_bfloat16* xp = reinterpret_cast<__nv_bfloat16*>(base + l.xp);
 
-    moe_group_kernel<<<1, 1024, (size_t)n_experts * 12, s>>>(routing, (uint32_t)n_pairs, n_experts, bn, header, tiles,
-                                                            list, status);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(moe_group_kernel, dim3(1), dim3(1024), n_experts * 12, s, routing, (uint32_t)n_pairs,
+                                   n_experts, bn, header, tiles, list, status);
     if (e != cudaSuccess) return e;
-    moe_gather_x_kernel<<<(uint32_t)((n_pairs + 7) / 8), 256, 0, s>>>(X, header, list, xp, K, n_used, x_token_stride);
-    e = cudaGetLastError();
+    e = launch_chained(moe_gather_x_kernel, dim3((uint32_t)((n_pairs + 7) / 8)), dim3(256), 0, s, X, header, list, xp, K,
+                       n_used, x_token_stride);
     if (e != cudaSuccess) return e;
 
     CUtensorMap map;

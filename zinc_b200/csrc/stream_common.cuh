@@ -11,6 +11,15 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The dependency wait of a chained launch (a no-op in any other). The pointers that lead to other kernels' results are
+// passed through afterwards, so that no load of them, read-only ones included, can be moved ahead of the wait.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename T>
+__device__ __forceinline__ void after_wait(T*& p) {
+    asm volatile("" : "+l"(p)::"memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
