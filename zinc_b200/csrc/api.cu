@@ -25,7 +25,7 @@ struct zc_ctx {
     uint64_t launches = 0;
     uint32_t* status_host = nullptr;  // pinned, mapped: deferred device-side status words
     uint32_t* status_dev = nullptr;
-    uint2* scratch_partial = nullptr;  // split-K partial sums of the streaming matvecs, tagged (zero between launches)
+    uint8_t* scratch = nullptr;          // one allocation, kScratchBytes: what the next three point into
     uint2* router_tagged = nullptr;      // 1024 tagged logits of the fused router + selection kernel (zero between launches)
     uint64_t router_mark = 0;            // value of `launches` right after that kernel's last launch (0: never)
     float* merge_scratch = nullptr;      // kMergeScratchFloats f32: a merged attention vector on its way to a matvec
@@ -54,7 +54,7 @@ constexpr uint32_t kMergeScratchFloats = 16384;
 constexpr size_t kRouterTaggedBytes = 1024 * sizeof(uint2);
 constexpr uint32_t kGemmTileFlags = 32768;  // two per 256 x 512 tile of a prefill GEMM split over CTA pairs
 constexpr size_t kScratchBytes =
-    kStreamPartialBytes + kRouterTaggedBytes + kMergeScratchFloats * sizeof(float) + kGemmTileFlags * sizeof(uint32_t);
+    kRouterTaggedBytes + kMergeScratchFloats * sizeof(float) + kGemmTileFlags * sizeof(uint32_t);
 
 int32_t fail(zc_ctx* ctx, int32_t code, const char* fmt, ...) {
     if (ctx) {
@@ -174,9 +174,7 @@ inline const float* f32p(const void* p, uint64_t off) {
 inline float* f32m(void* p, uint64_t off) { return reinterpret_cast<float*>(static_cast<uint8_t*>(p) + off); }
 
 inline void attach_scratch(zc_ctx* ctx, DmmvArgs& a) {
-    a.scratch_partial = ctx->scratch_partial;
     a.status = ctx->status_dev;
-    if (ctx->wait_limit) a.spin_limit = ctx->wait_limit;
     a.sm_count = ctx->sm_count;
     // nothing was launched since the fused router + selection kernel, which lets its successor start early:
     // that successor must order itself behind it before it trusts the routing buffer
@@ -237,19 +235,18 @@ int32_t zc_init(int32_t device, zc_ctx** out_ctx) {
     }
     memset(ctx->status_host, 0, 256);
     ctx->sm_count = prop.multiProcessorCount;
-    if (cudaMalloc(reinterpret_cast<void**>(&ctx->scratch_partial), kScratchBytes) != cudaSuccess ||
+    if (cudaMalloc(reinterpret_cast<void**>(&ctx->scratch), kScratchBytes) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&ctx->exact_scratch), kExactScratchBytes) != cudaSuccess ||
-        cudaMemset(ctx->scratch_partial, 0, kScratchBytes) != cudaSuccess) {
+        cudaMemset(ctx->scratch, 0, kScratchBytes) != cudaSuccess) {
         if (ctx->exact_scratch) cudaFree(ctx->exact_scratch);
-        if (ctx->scratch_partial) cudaFree(ctx->scratch_partial);
+        if (ctx->scratch) cudaFree(ctx->scratch);
         cudaFreeHost(ctx->status_host);
         cudaStreamDestroy(ctx->own_stream);
         delete ctx;
         return ZC_ERR_OOM;
     }
-    ctx->router_tagged = reinterpret_cast<uint2*>(reinterpret_cast<uint8_t*>(ctx->scratch_partial) + kStreamPartialBytes);
-    ctx->merge_scratch = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ctx->scratch_partial) + kStreamPartialBytes +
-                                                  kRouterTaggedBytes);
+    ctx->router_tagged = reinterpret_cast<uint2*>(ctx->scratch);
+    ctx->merge_scratch = reinterpret_cast<float*>(ctx->scratch + kRouterTaggedBytes);
     ctx->gemm_flags = reinterpret_cast<uint32_t*>(ctx->merge_scratch + kMergeScratchFloats);
     *out_ctx = ctx;
     return ZC_OK;
@@ -261,7 +258,7 @@ int32_t zc_destroy(zc_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     zc_comm_destroy(ctx);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
-    if (ctx->scratch_partial) cudaFree(ctx->scratch_partial);
+    if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->exact_scratch) cudaFree(ctx->exact_scratch);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
@@ -460,10 +457,10 @@ int32_t zc_submit_and_wait(zc_ctx* ctx) {
             return fail(ctx, ZC_ERR_INVALID_ARG,
                         "a routing buffer named expert %u, which the weight buffer does not hold; the results of that "
                         "call are invalid", where);
-        // A wait gave up. Tagged partial sums may be left behind and would be taken for fresh ones by the next
-        // streaming matvec: clear them. A peer exchange that gave up leaves the ranks' epochs out
+        // A wait gave up. Tagged logits may be left behind and would be taken for fresh ones by the next
+        // router kernel: clear them. A peer exchange that gave up leaves the ranks' epochs out
         // of step: the communicator refuses further collectives until it is destroyed and set up again.
-        cudaMemsetAsync(ctx->scratch_partial, 0, kStreamPartialBytes + kRouterTaggedBytes, ctx->stream);
+        cudaMemsetAsync(ctx->router_tagged, 0, kRouterTaggedBytes, ctx->stream);
         cudaStreamSynchronize(ctx->stream);
         if (where >= 200 && ctx->comm_local) ctx->comm_broken = true;
         return fail(ctx, ZC_ERR_TIMEOUT, "device-side wait gave up (code %u, site %u)", code, where);

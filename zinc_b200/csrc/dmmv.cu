@@ -32,21 +32,7 @@ __global__ void __launch_bounds__(kWarps * 32) dmmv_kernel(const DmmvArgs a) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const uint64_t row_bytes = (uint64_t)(a.K / block_size(TYPE)) * bytes_per_block(TYPE);
-    // A chained launch: the weights depend on no kernel, so a plain matvec asks for the first 4 KB of its rows while the
-    // kernel before drains, and lets its own successor do the same at once (unless its predecessor did that with the
-    // routing still in flight). 512 x 2048 Q8_0, one call after the other: bound by this latency, not by its 1.1 MB.
-    if (MODE == MODE_PLAIN) {
-        if (!a.late) chain_release();
-        const uint32_t r0 = (blockIdx.x * kWarps + warp) * NR;
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            const uint64_t off = (uint64_t)lane * 128;
-            if (r0 + r < a.M && off < row_bytes)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(a.A + (uint64_t)(r0 + r) * row_bytes + off));
-        }
-    }
     chain_wait();
-    if (MODE != MODE_PLAIN || a.late) chain_release();
     const float *a_x = a.x, *a_gate = a.gate;
     float* a_y = a.y;
     const uint32_t* a_routing = a.routing;
@@ -282,14 +268,19 @@ cudaError_t launch_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t
     if (wbytes >= kStreamMinBytes) {
         if (warp_dmmv_eligible(type, mode, a)) return launch_warp_dmmv(type, mode, a, s, launches);
         if (q6k_dmmv_eligible(type, mode, a)) return launch_q6k_dmmv(mode, a, s, launches);
+        if (mxfp4_dmmv_eligible(type, mode, a)) return launch_mxfp4_dmmv(a, s, launches);
     }
     // the kernels below do not carry a pending reduction: complete it first
     if (a.consume.n) {
         const cudaError_t ec = launch_consume(a.consume, s, launches);
         if (ec != cudaSuccess) return ec;
     }
-    if (wbytes >= kStreamMinBytes && mxfp4_dmmv_eligible(type, mode, a)) return launch_mxfp4_dmmv(a, s, launches);
     cudaError_t e;
+    if (mode == MODE_PLAIN && row_dmmv_eligible(type, a)) {
+        e = launch_row_dmmv(type, a, s);
+        if (e == cudaSuccess && launches) ++*launches;
+        return e;
+    }
     // 128-bit weight loads need every block start 16-byte aligned: true for the
     // 144/176-byte K-quant blocks when the base, the second base and the expert
     // stride are.

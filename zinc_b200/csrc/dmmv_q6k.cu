@@ -1,7 +1,4 @@
-// Warp-autonomous streaming decode matvec for B200 (Q6_K), integer tensor-core dot engine.
-// Same skeleton as the Q4_K kernel (stream_skel.cuh): every warp owns a contiguous range of
-// (16 rows x one 256-weight super-block) units, prefetches them with coalesced 16-byte
-// asynchronous copies and finishes split tiles in worker order.
+// Streaming decode matvec for Q6_K on the integer tensor cores (dmmv_slice.cuh deals rows to CTAs and K to warps).
 //
 // Stands in for src/shaders/dmmv_q6k.comp:58-156 (and its use for the down projection and the LM
 // head, src/compute/forward.zig:7420, 7714) for the Q6_K layout of src/compute/forward.zig:276-325:
@@ -23,17 +20,13 @@
 // and 8h + 2j + 1 (k slots 16..31). B is block-diagonal to match: column 2d + u holds digit d of x in the k
 // slots of sub-block half u and zeros in the other half, so D column 2d + u is digit d's dot product with
 // sub-block u alone; lane t < 3 ends up with digit t of both sub-blocks for rows g and g+8.
-#include "kernels.h"
-#include "stream_skel.cuh"
+#include "dmmv_slice.cuh"
 
 namespace zc {
 
 namespace {
 
-constexpr int kDepth = 2;
 constexpr int kRow6 = 240;                  // bytes per row slot: 224-byte superset + pad (15 x 16: odd)
-constexpr int kSlot6 = 16 * kRow6;
-constexpr int kRing6 = kDepth * kSlot6;
 constexpr int kPieces6 = 14;                // 16-byte pieces per row superset
 constexpr int kPiecesLane6 = (16 * kPieces6 + 31) / 32;  // 7
 constexpr int kZeroBytes6 = 128;
@@ -41,68 +34,27 @@ constexpr int kFracBits = 20;
 constexpr int kPrepBlocks = 6;
 constexpr int kBBytes = 1536;               // B operand table per super-block: [h 2][j pair 2][column 6][t 4][16 bytes]
 constexpr int kNsxBytes = 256;              // accumulator start values per super-block: [h 2][digit 4][j 4][u 2] s32
-constexpr size_t kTwoPerSm = 113 * 1024;
 
-struct Smem6 {
+struct Tab6 {
     uint8_t* zeros;  // kZeroBytes6 of zeros (B operand of the dead columns 6 and 7)
     uint8_t* bq;     // per super-block kBBytes: {b0, b1} register pairs in B-operand order
     int* nsx;        // per super-block kNsxBytes / 4: -32 * sum of digit d over sub-block (h, j, u)
     float* xs;       // per super-block 2^-f
-    uint8_t* ring;   // [kWarps][kDepth] stages of 16 row slots
-    float* spartial; // [kWarps][32] partial sums published inside the CTA
-    volatile uint32_t* sflags;  // [kWarps]
 };
-
-__host__ __device__ inline size_t smem_bytes6(uint32_t K, int kWarps) {
-    size_t n = (size_t)kZeroBytes6 + (size_t)(K / 256) * (kBBytes + kNsxBytes + 4);
-    n = (n + 127) & ~size_t(127);
-    n += (size_t)kWarps * kRing6;
-    n += (size_t)kWarps * 32 * 4 + (size_t)kWarps * 4 + 16;
-    return n + 128;
-}
-
-__device__ inline Smem6 carve6(uint8_t* base, uint32_t K, int kWarps) {
-    Smem6 s;
-    uintptr_t p = (reinterpret_cast<uintptr_t>(base) + 127) & ~uintptr_t(127);
-    s.zeros = reinterpret_cast<uint8_t*>(p);
-    p += kZeroBytes6;
-    s.bq = reinterpret_cast<uint8_t*>(p);
-    p += (size_t)(K / 256) * kBBytes;
-    s.nsx = reinterpret_cast<int*>(p);
-    p += (size_t)(K / 256) * kNsxBytes;
-    s.xs = reinterpret_cast<float*>(p);
-    p += (size_t)(K / 256) * 4;
-    p = (p + 127) & ~uintptr_t(127);
-    s.ring = reinterpret_cast<uint8_t*>(p);
-    p += (size_t)kWarps * kRing6;
-    s.spartial = reinterpret_cast<float*>(p);
-    p += (size_t)kWarps * 32 * 4;
-    s.sflags = reinterpret_cast<volatile uint32_t*>(p);
-    return s;
-}
 
 struct XRegs6 {
     float4 lo[kPrepBlocks], hi[kPrepBlocks];
 };
-// One warp per super-block; lane l handles the 8 consecutive elements 8l .. 8l+7.
-// K: length of the (concatenated) activation. bpe > 0 (MoE down projection): the activation is n_slots
-// vectors of bpe * 256 elements, x + s * x_stride, each scaled by the slot's routing weight wts[s].
-// Only the n_need super-blocks from b_first on (wrapping at the end of the row) are converted: a CTA whose
-// units cover less than a row does not need the rest.
-__device__ __forceinline__ uint32_t prep_block(uint32_t i, uint32_t b_first, uint32_t nblk) {
-    const uint32_t b = b_first + i;
-    return b >= nblk ? b - nblk : b;
-}
-template <int kWarps>
-__device__ __forceinline__ void load_x6(XRegs6& r, const float* __restrict__ x, uint32_t K, uint32_t bpe,
-                                        uint32_t x_stride, const uint32_t* __restrict__ wts, int warp, int lane,
-                                        uint32_t b_first, uint32_t n_need) {
+// One warp per super-block; lane l handles the 8 consecutive elements 8l .. 8l+7. bpe: blocks of one vector; with more
+// than that (MoE down projection) the activation is several vectors, x + s * x_stride, each scaled by the slot's routing
+// weight wts[s].
+__device__ __forceinline__ void load_x6(XRegs6& r, const float* __restrict__ x, uint32_t nblk, uint32_t bpe, uint32_t x_stride,
+                                        const uint32_t* __restrict__ wts, int warp, int lane, uint32_t n_warps) {
 #pragma unroll
     for (int b = 0; b < kPrepBlocks; ++b) {
-        const uint32_t bi = warp + b * kWarps;
-        if (bi < n_need) {
-            const uint32_t blk = prep_block(bi, b_first, K >> 8);
-            const uint32_t slot = bpe ? blk / bpe : 0u, lb = bpe ? blk - slot * bpe : blk;
+        const uint32_t blk = warp + b * n_warps;
+        if (blk < nblk) {
+            const uint32_t slot = wts ? blk / bpe : 0u, lb = blk - slot * bpe;
             const float* xp = x + (size_t)slot * x_stride + (size_t)lb * 256 + 8 * lane;
             float4 lo = __ldg(reinterpret_cast<const float4*>(xp)), hi = __ldg(reinterpret_cast<const float4*>(xp) + 1);
             if (wts) {
@@ -122,15 +74,12 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
 
 // Lane l's elements 8l .. 8l+7 lie in half h = l/16, quarter j = (l/4)%4, sub-block half u = (l/2)%2, and are
 // the k-slot groups t = 2(l%2) and t+1 of that sub-block half.
-template <int kWarps>
-__device__ __forceinline__ void prep_x6(const Smem6& s, const XRegs6& r, uint32_t K, int warp, int lane,
-                                        uint32_t b_first, uint32_t n_need) {
+__device__ __forceinline__ void prep_x6(const Tab6& s, const XRegs6& r, uint32_t nblk, int warp, int lane, uint32_t n_warps) {
     const uint32_t h = lane >> 4, j = (lane >> 2) & 3, u = (lane >> 1) & 1, t0 = 2 * (lane & 1);
 #pragma unroll
     for (int b = 0; b < kPrepBlocks; ++b) {
-        const uint32_t bi = warp + b * kWarps;
-        if (bi >= n_need) break;
-        const uint32_t blk = prep_block(bi, b_first, K >> 8);
+        const uint32_t blk = warp + b * n_warps;
+        if (blk >= nblk) break;
         const float4 lo = r.lo[b], hi = r.hi[b];
         const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
         float mx = 0.f;
@@ -253,314 +202,164 @@ __device__ __forceinline__ void block6(uint32_t rA, uint32_t rB, uint32_t shA, u
     }
 }
 
-// kMoe: MoE down projection, y += sum_s w_s W[routing[s]] x_s: the n_used selected matrices side by side along
-// K, each with its own activation (scaled by w_s while it is converted to fixed point).
-// kRowsAligned: every row starts on a 16-byte boundary (K a multiple of 2048), so all rows of a unit share
-// one offset inside their aligned supersets; otherwise each row has its own (rows are 2-byte aligned).
-template <int EPI, int kWarps, bool kRowsAligned, bool kMoe = false>
-__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dmmv_q6k_warp_kernel(const WarpArgs a,
-                                                                                 const uint8_t* a_end) {
-    extern __shared__ uint8_t smem_raw[];
-    pdl_begin(a);
-    const uint32_t bpe = a.K >> 8;                        // blocks per row of one matrix
-    const uint32_t bpr = kMoe ? bpe * a.nseg : bpe;       // blocks per (concatenated) row = units per tile
-    const Smem6 s = carve6(smem_raw, bpr * 256, kWarps);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const uint64_t row_bytes = (uint64_t)bpe * 210;
-    // matrix that holds block `b` of the concatenated row, and the block's index inside it
-    auto matrix_of = [&](uint32_t b, uint32_t& lb) -> const uint8_t* {
-        if constexpr (kMoe) {
-            const uint32_t slot = b / bpe;
-            lb = b - slot * bpe;
-            const uint32_t e_raw = __ldg(a.routing + slot);
-            if (e_raw == kSkipExpert) return nullptr;  // no expert in this slot on this rank
-            return expert_matrix(a.A[0], a.A_sh[0], e_raw, a.expert_stride, a.n_experts_max, a.status);
-        } else {
-            lb = b;
-            return a.A[0];
-        }
-    };
-    const uint32_t tiles = (a.M + 15) / 16;
-    const uint32_t U = tiles * bpr, G = gridDim.x * kWarps;
-    const uint32_t me = blockIdx.x * kWarps + warp;
-    const uint32_t u0 = (uint32_t)part_begin(me, U, G), u1 = (uint32_t)part_begin(me + 1, U, G);
-    const uint32_t n = u1 - u0;
-    uint8_t* ring = s.ring + (size_t)warp * kRing6;
+// kAligned: every row starts on a 16-byte boundary (K a multiple of 2048), so all rows of a unit share one offset inside
+// their aligned supersets; otherwise each row has its own (rows are 2-byte aligned).
+template <bool kAligned>
+struct FmtQ6K {
+    using Tab = Tab6;
+    using X = XRegs6;
+    static constexpr uint32_t kSlot = 16 * kRow6;
+    static constexpr uint32_t kCols = 256;
+    static constexpr uint32_t kPrepBlocks = zc::kPrepBlocks;
+    static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes6 + nblk * (kBBytes + kNsxBytes + 4) + 128; }
+    static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
+        Tab t;
+        p += (128u - (smem_u32(p) & 127u)) & 127u;
+        t.zeros = p;
+        t.bq = p + kZeroBytes6;
+        t.nsx = reinterpret_cast<int*>(t.bq + (size_t)nblk * kBBytes);
+        t.xs = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(t.nsx) + (size_t)nblk * kNsxBytes);
+        return t;
+    }
+    template <int kSeg>
+    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, int warp, int lane, uint32_t n_warps) {
+        load_x6(r, a.x, a.nblk, a.bpe, a.x_slot_stride, kSeg == 3 ? a.routing + a.nseg : nullptr, warp, lane, n_warps);
+    }
+    static __device__ __forceinline__ void prep(const Tab& t, const X& r, const SliceArgs& a, int warp, int lane, int tid, uint32_t n_warps) {
+        for (uint32_t i = tid; i < kZeroBytes6 / 16; i += blockDim.x) reinterpret_cast<uint4*>(t.zeros)[i] = make_uint4(0u, 0u, 0u, 0u);
+        prep_x6(t, r, a.nblk, warp, lane, n_warps);
+    }
 
-    uint32_t piece[kPiecesLane6];  // row | column << 8
-#pragma unroll
-    for (int i = 0; i < kPiecesLane6; ++i) {
-        const uint32_t p = i * 32 + lane;
-        const uint32_t r = p / kPieces6;
-        piece[i] = r | ((p - r * kPieces6) << 8);
-    }
-    uint32_t p_tile = u0 / bpr, p_blk = u0 % bpr;
-    // Rows aligned and a whole number of tiles: a piece's place in the slot and its offset from the tile's first
-    // row are fixed per lane
-    const bool whole_tiles = kRowsAligned && (a.M & 15u) == 0;
-    uint32_t pdst[kPiecesLane6], psrc[kPiecesLane6];
-    if constexpr (kRowsAligned) {
-#pragma unroll
-        for (int i = 0; i < kPiecesLane6; ++i) {
-            const uint32_t r = piece[i] & 0xFFu, col = piece[i] >> 8;
-            pdst[i] = r * kRow6 + col * 16;
-            psrc[i] = r * (uint32_t)row_bytes + col * 16;
-        }
-    }
-    const uint32_t ring_addr = smem_u32(ring);
-    auto request = [&](uint32_t slot) {
-        uint8_t* dst = ring + slot * kSlot6;
-        const uint32_t row0 = p_tile * 16;
-        if constexpr (kRowsAligned) {
-            const uint32_t al = (p_blk * 210u) & ~15u;  // aligned start of the block's superset within the row
-            if (whole_tiles) {
-                const uint8_t* base = a.A[0] + (uint64_t)row0 * row_bytes + al;
-                const uint32_t room = (uint32_t)row_bytes - al, ds = ring_addr + slot * kSlot6;
-#pragma unroll
-                for (int i = 0; i < kPiecesLane6; ++i)
-                    if ((piece[i] >> 8) * 16 < room)  // rows are 16-byte aligned: a piece never crosses the row end
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ds + pdst[i]), "l"(base + psrc[i])
-                                     : "memory");
-            } else {
-#pragma unroll
-                for (int i = 0; i < kPiecesLane6; ++i) {
-                    const uint32_t r = piece[i] & 0xFFu, col = piece[i] >> 8;
-                    if (al + col * 16 < (uint32_t)row_bytes) {
-                        const uint32_t row = min(row0 + r, a.M - 1);
-                        cp_async16(dst + r * kRow6 + col * 16, a.A[0] + (uint64_t)row * row_bytes + al + col * 16);
-                    }
-                }
-            }
-        } else {
-            uint32_t lb;
-            const uint8_t* mat = matrix_of(p_blk, lb);
-            // first byte past the buffer that holds `mat` (the shared expert lives in a buffer of its own)
-            const uint8_t* m_end = kMoe && mat == a.A_sh[0] ? a.A_sh_end[0] : a_end;
+    // piece p = i * 32 + lane of a unit: row p / 14, 16-byte column p % 14 of the row's aligned superset
+    struct Copier {
+        uint32_t row[kPiecesLane6], col[kPiecesLane6], src[kPiecesLane6];
+        __device__ __forceinline__ void init(const SliceArgs& a, int lane) {
 #pragma unroll
             for (int i = 0; i < kPiecesLane6; ++i) {
-                if (kMoe && mat == nullptr) break;  // nothing to fetch
-                const uint32_t r = piece[i] & 0xFFu, col = piece[i] >> 8;
-                const uint32_t row = min(row0 + r, a.M - 1);
-                const uint8_t* start = mat + (uint64_t)row * row_bytes + lb * 210u;
-                const uint32_t o = (uint32_t)(reinterpret_cast<uintptr_t>(start) & 15u);
-                if (col * 16 < o + 210u) {  // the piece holds bytes of the block
-                    const uint8_t* src = start - o + col * 16;
-                    uint8_t* d = dst + r * kRow6 + col * 16;
-                    if (src + 16 <= m_end) {
-                        cp_async16(d, src);
-                    } else {  // the very end of the tensor: copy only the bytes that exist
-                        for (const uint8_t* q = src; q < m_end; ++q) d[q - src] = __ldg(q);
+                const uint32_t p = i * 32 + lane;
+                row[i] = p / kPieces6;
+                col[i] = (p - row[i] * kPieces6) * 16;
+                src[i] = row[i] * a.bpe * 210u + col[i];
+            }
+        }
+        __device__ __forceinline__ void copy(const SliceArgs& a, const Unit& u, uint8_t* slot, int) const {
+            const uint32_t row_bytes = a.bpe * 210u, d = smem_u32(slot);
+            const uint8_t* first = u.mat + (uint64_t)u.row0 * row_bytes + u.lb * 210u;  // the block in the tile's first row
+            if constexpr (kAligned) {
+                const uint32_t o = (u.lb * 210u) & 15u, room = row_bytes - (u.lb * 210u - o);
+                const uint8_t* p = first - o;
+#pragma unroll
+                for (int i = 0; i < kPiecesLane6; ++i)
+                    if (row[i] < u.rows && col[i] < room)  // rows are 16-byte aligned: a piece never crosses the row end
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + row[i] * kRow6 + col[i]), "l"(p + src[i])
+                                     : "memory");
+            } else {
+                const uint32_t f = (uint32_t)reinterpret_cast<uintptr_t>(first);
+                // the pieces of a tile away from the end of the buffer are read whole
+                const bool inside = first + (uint64_t)u.rows * row_bytes + 240 <= u.end;
+#pragma unroll
+                for (int i = 0; i < kPiecesLane6; ++i) {
+                    const uint32_t o = (f + row[i] * row_bytes) & 15u;
+                    if (row[i] < u.rows && col[i] < o + 210u) {  // the piece holds bytes of the block
+                        const uint8_t* p = first + src[i] - o;
+                        if (inside || p + 16 <= u.end) {
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + row[i] * kRow6 + col[i]), "l"(p)
+                                         : "memory");
+                        } else {  // the very end of the tensor: copy only the bytes that exist
+                            uint8_t* q = slot + row[i] * kRow6 + col[i];
+                            for (; p < u.end; ++p) *q++ = __ldg(p);
+                        }
                     }
                 }
             }
         }
-        if (++p_blk == bpr) { p_blk = 0; ++p_tile; }
     };
-    // super-blocks of the activation this CTA's units touch
-    const uint32_t cu0 = (uint32_t)part_begin((uint64_t)blockIdx.x * kWarps, U, G);
-    const uint32_t cu1 = (uint32_t)part_begin((uint64_t)(blockIdx.x + 1) * kWarps, U, G);
-    const uint32_t x_first = cu1 - cu0 >= bpr ? 0u : cu0 % bpr, x_need = min(bpr, cu1 - cu0);
-    pdl_late(a);
-    XRegs6 xr;
-    if (a.late)
-        load_x6<kWarps>(xr, a.x, bpr * 256, kMoe ? bpe : 0u, kMoe ? a.x_slot_stride : 0u,
-                        kMoe ? a.routing + a.nseg : nullptr, warp, lane, x_first, x_need);
-#pragma unroll
-    for (int i = 0; i < kDepth; ++i) {
-        if ((uint32_t)i < n) request(i);
-        cp_async_commit();
-    }
-    pdl_wait();
-    if (!a.late)
-        load_x6<kWarps>(xr, a.x, bpr * 256, kMoe ? bpe : 0u, kMoe ? a.x_slot_stride : 0u,
-                        kMoe ? a.routing + a.nseg : nullptr, warp, lane, x_first, x_need);
-    if (a.consume.n) consume_pushed(a.consume, blockIdx.x, gridDim.x, tid, kWarps * 32);
 
-    if (tid < kZeroBytes6 / 16) reinterpret_cast<uint4*>(s.zeros)[tid] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < kWarps) s.sflags[tid] = 0u;
-    prep_x6<kWarps>(s, xr, bpr * 256, warp, lane, x_first, x_need);
-    __syncthreads();
-
-    uint32_t tile = u0 / bpr, blk = u0 % bpr;
-    float acc[2] = {0.f, 0.f};
-    // B operand: lane (g, t) feeds column g; columns 6 and 7 are dead (zeros, one address for the quarter-warp)
-    const bool b_live = g < 6;
-    const uint32_t xb_base = b_live ? smem_u32(s.bq) + (uint32_t)g * 64u + (uint32_t)t * 16u : smem_u32(s.zeros);
-    const uint32_t xb_step = b_live ? (uint32_t)kBBytes : 0u;
-    const uint32_t xh = b_live ? 0xFFFFFFFFu : 0u;
-    const uint32_t nsx_s = smem_u32(s.nsx) + 32u * t, xs_s = smem_u32(s.xs), ring_s = smem_u32(ring);
-    const float dscale = __uint_as_float((127u + 14u - 7u * t) << 23);  // digit t carries 2^(14 - 7t)
-
-    for (uint32_t it = 0; it < n; ++it) {
-        const uint32_t slot = it % kDepth;
-        cp_async_wait<kDepth - 1>();
-        __syncwarp();
-        // byte offset of the block inside each row's aligned superset
-        uint32_t oA, oB;
-        bool skip = false;  // MoE: the block belongs to a slot without an expert on this rank
-        if constexpr (kRowsAligned) {
-            oA = oB = (blk * 210u) & 15u;
-        } else {
-            const uint32_t rowA = min(tile * 16 + g, a.M - 1), rowB = min(tile * 16 + g + 8, a.M - 1);
-            uint32_t lb;
-            const uint8_t* mat = matrix_of(blk, lb);
-            skip = kMoe && mat == nullptr;
-            oA = (uint32_t)(reinterpret_cast<uintptr_t>(mat + (uint64_t)rowA * row_bytes + lb * 210u) & 15u);
-            oB = (uint32_t)(reinterpret_cast<uintptr_t>(mat + (uint64_t)rowB * row_bytes + lb * 210u) & 15u);
+    struct Acc {
+        float s[2];
+        __device__ __forceinline__ void clear() { s[0] = s[1] = 0.f; }
+    };
+    struct Lane {
+        uint32_t xb_base, xb_step, xh, nsx_s, xs_s;
+        int g, t;
+        float dscale;
+        __device__ __forceinline__ void init(const SliceArgs&, const Tab& s, int lane) {
+            g = lane >> 2;
+            t = lane & 3;
+            // B operand: lane (g, t) feeds column g; columns 6 and 7 are dead (zeros, one address for the quarter-warp)
+            const bool b_live = g < 6;
+            xb_base = b_live ? smem_u32(s.bq) + (uint32_t)g * 64u + (uint32_t)t * 16u : smem_u32(s.zeros);
+            xb_step = b_live ? (uint32_t)kBBytes : 0u;
+            xh = b_live ? 0xFFFFFFFFu : 0u;
+            nsx_s = smem_u32(s.nsx) + 32u * t;
+            xs_s = smem_u32(s.xs);
+            dscale = __uint_as_float((127u + 14u - 7u * t) << 23);  // digit t carries 2^(14 - 7t)
         }
-        const uint32_t sb = ring_s + slot * kSlot6;
-        const uint32_t rA = sb + g * kRow6 + oA, rB = sb + (g + 8) * kRow6 + oB;
-        const uint32_t xb = xb_base + blk * xb_step, nb = nsx_s + blk * (uint32_t)kNsxBytes;
-        int IA = 0, IB = 0;
-        uint32_t dA = 0, dB = 0;
-        if (skip) {
-        } else if (kRowsAligned && (oA & 2u) == 0) {  // the same for the whole warp
-            block6<false>(rA, rB, 0u, 0u, xb, xh, nb, t, IA, IB);
-        } else {
-            block6<true>(rA, rB, (oA & 3u) * 8u, (oB & 3u) * 8u, xb, xh, nb, t, IA, IB);
-        }
-        if (!skip) {
-            dA = lds_u16s(rA + 208);
-            dB = lds_u16s(rB + 208);
-        }
-        // every lane has read the stage: refill it
-        __syncwarp();
-        if (it + kDepth < n) request(slot);
-        cp_async_commit();
-        const float xs = lds_f1(xs_s + blk * 4);
-        acc[0] = fmaf(h2f(dA) * xs, (float)IA, acc[0]);
-        acc[1] = fmaf(h2f(dB) * xs, (float)IB, acc[1]);
-
-        const uint32_t T = tile;
-        bool tile_done = false;
-        if (++blk == bpr) { blk = 0; ++tile; tile_done = true; }
-        if (tile_done || it + 1 == n) {
-            float v[1][2];
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                float w = acc[r] * dscale;
-                w += __shfl_xor_sync(0xFFFFFFFFu, w, 1);
-                w += __shfl_xor_sync(0xFFFFFFFFu, w, 2);
-                v[0][r] = w;
-                acc[r] = 0.f;
+        __device__ __forceinline__ void dot(const SliceArgs& a, const Unit& u, uint32_t slot, Acc& acc) const {
+            uint32_t oA, oB;  // byte offset of the block inside each row's aligned superset
+            if constexpr (kAligned) {
+                oA = oB = (u.lb * 210u) & 15u;
+            } else {
+                const uint32_t row_bytes = a.bpe * 210u;
+                const uint32_t f = (uint32_t)reinterpret_cast<uintptr_t>(u.mat) + u.row0 * row_bytes + u.lb * 210u;
+                oA = (f + g * row_bytes) & 15u;
+                oB = (f + (g + 8) * row_bytes) & 15u;
             }
-            finish_tile<1, EPI, kWarps>(a, row_out(a), s.spartial, s.sflags, v, T, bpr, u0, u1, U, G, me, warp, lane);
+            const uint32_t rA = slot + g * kRow6 + oA, rB = slot + (g + 8) * kRow6 + oB;
+            const uint32_t xb = xb_base + u.kb * xb_step, nb = nsx_s + u.kb * (uint32_t)kNsxBytes;
+            int IA, IB;
+            if (kAligned && (oA & 2u) == 0) block6<false>(rA, rB, 0u, 0u, xb, xh, nb, t, IA, IB);  // the same for the whole warp
+            else block6<true>(rA, rB, (oA & 3u) * 8u, (oB & 3u) * 8u, xb, xh, nb, t, IA, IB);
+            const float xs = lds_f1(xs_s + u.kb * 4);
+            acc.s[0] = fmaf(h2f(lds_u16s(rA + 208)) * xs, (float)IA, acc.s[0]);
+            acc.s[1] = fmaf(h2f(lds_u16s(rB + 208)) * xs, (float)IB, acc.s[1]);
         }
-    }
-}
-
-template <int EPI, int kWarps, bool kRowsAligned, bool kMoe = false>
-cudaError_t launch_w6(const WarpArgs& a, const uint8_t* a_end, cudaStream_t st, int sm_count, size_t smem) {
-    auto kern = dmmv_q6k_warp_kernel<EPI, kWarps, kRowsAligned, kMoe>;
-    static std::atomic<uint64_t> attr_done{0};  // per device ordinal
-    if (cudaError_t ea = ensure_dynamic_smem(kern, kWarps == 8 ? (int)kTwoPerSm : 227 * 1024, attr_done); ea != cudaSuccess) return ea;
-    const uint64_t U = (uint64_t)((a.M + 15) / 16) * (a.K >> 8) * (kMoe ? a.nseg : 1u);
-    uint64_t grid = (uint64_t)sm_count * (16 / kWarps);
-    if (grid * kWarps > U) grid = U / kWarps;
-    if (grid * kWarps > kStreamMaxWorkers) grid = kStreamMaxWorkers / kWarps;
-    if (grid == 0) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((uint32_t)grid, 1, 1);
-    cfg.blockDim = dim3(kWarps * 32, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, a, a_end);
-}
+        __device__ __forceinline__ void finish(const Acc& acc, float& v0, float& v1) const {
+            v0 = acc.s[0] * dscale;
+            v1 = acc.s[1] * dscale;
+        }
+    };
+};
 
 template <int EPI>
-cudaError_t launch_cfg6(const WarpArgs& a, const uint8_t* a_end, cudaStream_t st, int sm_count) {
-    const size_t s8 = smem_bytes6(a.K, 8);
-    const bool al = ((a.K >> 8) % 8u) == 0;  // 210 * K/256 bytes per row: a multiple of 16 for K % 2048 == 0
-    if (s8 <= kTwoPerSm)
-        return al ? launch_w6<EPI, 8, true>(a, a_end, st, sm_count, s8) : launch_w6<EPI, 8, false>(a, a_end, st, sm_count, s8);
-    const size_t s16 = smem_bytes6(a.K, 16);
-    return al ? launch_w6<EPI, 16, true>(a, a_end, st, sm_count, s16) : launch_w6<EPI, 16, false>(a, a_end, st, sm_count, s16);
+cudaError_t launch_plain(const SliceArgs& s, int sm_count, cudaStream_t st) {
+    // 210 * K / 256 bytes per row: a multiple of 16 for K % 2048 == 0
+    return ((s.K >> 8) % 8u) == 0 ? slice_launch<FmtQ6K<true>, 1, EPI, 0>(s, sm_count, st)
+                                  : slice_launch<FmtQ6K<false>, 1, EPI, 0>(s, sm_count, st);
 }
 
 }  // namespace
 
 bool q6k_dmmv_eligible(uint32_t type, int mode, const DmmvArgs& a) {
-    if (type != T_Q6_K) return false;
+    if (type != T_Q6_K || (a.K & 255u)) return false;
     if (mode != MODE_PLAIN && mode != MODE_SIGMOID_ACC) return false;
-    if (!a.scratch_partial || !a.status) return false;
-    const uint32_t bpr = a.K >> 8;
+    if (!a.status) return false;
     if (reinterpret_cast<uintptr_t>(a.A) & 15u) return false;  // supersets are fetched in 16-byte pieces from the base
-    if ((bpr % 8u) != 0 && !a.a_end) return false;          // unaligned rows: the end of the buffer must be known
-    if (smem_bytes6(a.K, 16) > 227 * 1024 || bpr > (uint32_t)(kPrepBlocks * 8)) return false;
-    const uint64_t U = (uint64_t)((a.M + 15) / 16) * bpr;
-    if (U < 16 || U > 0xFFFFFFFFull) return false;
-    return true;
+    if (((a.K >> 8) % 8u) != 0 && !a.a_end) return false;      // unaligned rows: the end of the buffer must be known
+    return slice_fits<FmtQ6K<true>>(a.K, 1, 1);
 }
 
 // MoE down projection + weighted accumulate (y += sum_s w_s W[routing[s]] x_s) through the streaming kernel.
 bool q6k_moe_down_acc_eligible(uint32_t type, const DmmvArgs& a) {
-    if (type != T_Q6_K || !a.routing || a.n_used == 0 || !a.a_end) return false;
-    if (!a.scratch_partial || !a.status) return false;
+    if (type != T_Q6_K || !a.routing || a.n_used == 0 || !a.a_end || !a.status) return false;
     if ((reinterpret_cast<uintptr_t>(a.A) & 15u) || (a.expert_stride & 15u) || (a.K & 255u)) return false;
     if ((a.x_expert_stride & 3u) || (reinterpret_cast<uintptr_t>(a.x) & 15u)) return false;
     if (a.A_sh && ((reinterpret_cast<uintptr_t>(a.A_sh) & 15u) || !a.a_sh_end)) return false;
-    const uint32_t bpr = (a.K >> 8) * a.n_used;
-    if (smem_bytes6(bpr * 256, 16) > 227 * 1024 || bpr > (uint32_t)(kPrepBlocks * 8)) return false;
-    const uint64_t U = (uint64_t)((a.M + 15) / 16) * bpr;
-    if ((uint64_t)a.M * bpr * 210u < kStreamMinBytes) return false;  // small expert sets: latency-bound either way
-    return U >= 16 && U <= 0xFFFFFFFFull;
+    if ((uint64_t)a.M * (a.K >> 8) * a.n_used * 210u < kStreamMinBytes) return false;  // small expert sets: latency-bound either way
+    return slice_fits<FmtQ6K<false>>(a.K, a.n_used, 1);
 }
 
 cudaError_t launch_q6k_moe_down_acc(const DmmvArgs& a, cudaStream_t st, uint64_t* launches) {
-    WarpArgs wa;
-    wa.A[0] = wa.A[1] = a.A;
-    wa.x = a.x;
-    wa.y = a.y;
-    wa.gate = nullptr;
-    wa.M = a.M;
-    wa.K = a.K;
-    wa.acc_mode = 1;
-    wa.gpartial = a.scratch_partial;
-    wa.status = a.status;
-    wa.spin_limit = a.spin_limit;
-    wa.nseg = a.n_used;
-    wa.routing = a.routing;
-    wa.n_experts_max = a.n_experts_max;
-    wa.expert_stride = a.expert_stride;
-    wa.x_slot_stride = a.x_expert_stride;
-    wa.A_sh[0] = wa.A_sh[1] = a.A_sh;
-    wa.A_sh_end[0] = wa.A_sh_end[1] = a.a_sh_end;
-    wa.bias[0] = a.bias;
-    wa.late = a.late;
-    const uint32_t Kt = a.K * a.n_used;
-    const size_t s8 = smem_bytes6(Kt, 8);
-    const cudaError_t e = s8 <= kTwoPerSm ? launch_w6<EPI_ACC, 8, false, true>(wa, a.a_end, st, a.sm_count, s8)
-                                          : launch_w6<EPI_ACC, 16, false, true>(wa, a.a_end, st, a.sm_count,
-                                                                                 smem_bytes6(Kt, 16));
+    SliceArgs s = slice_args(a);
+    s.nseg = a.n_used;
+    const cudaError_t e = slice_launch<FmtQ6K<false>, 1, EPI_ACC, 3>(s, a.sm_count, st);
     if (e == cudaSuccess && launches) ++*launches;
     return e;
 }
 
 cudaError_t launch_q6k_dmmv(int mode, const DmmvArgs& a, cudaStream_t st, uint64_t* launches) {
-    WarpArgs wa;
-    wa.A[0] = a.A;
-    wa.A[1] = a.A;
-    wa.x = a.x;
-    wa.y = a.y;
-    wa.gate = a.gate;
-    wa.M = a.M;
-    wa.K = a.K;
-    wa.acc_mode = a.acc_mode;
-    wa.gpartial = a.scratch_partial;
-    wa.status = a.status;
-    wa.spin_limit = a.spin_limit;
-    wa.nseg = 0;
-    wa.push = a.push;
-    wa.consume = a.consume;
-    wa.late = a.late;
-    cudaError_t e = mode == MODE_PLAIN ? launch_cfg6<EPI_PLAIN>(wa, a.a_end, st, a.sm_count)
-                                       : launch_cfg6<EPI_SIGMOID_ACC>(wa, a.a_end, st, a.sm_count);
+    const SliceArgs s = slice_args(a);
+    const cudaError_t e = mode == MODE_PLAIN ? launch_plain<EPI_PLAIN>(s, a.sm_count, st) : launch_plain<EPI_SIGMOID_ACC>(s, a.sm_count, st);
     if (e == cudaSuccess && launches) ++*launches;
     return e;
 }

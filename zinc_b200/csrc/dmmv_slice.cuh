@@ -1,0 +1,395 @@
+// Skeleton of the streaming matvec kernels: rows are dealt to CTAs, K to the warps of a CTA.
+//
+// Every CTA owns a contiguous run of row tiles (at most 16 rows each, the height chosen so that the SMs get equal numbers
+// of rows); inside it, warp (wr, wk) works through the tiles wr, wr + n_wr, ... and owns the blocks (256 columns, MXFP4 512) wk, wk + n_wk,
+// ... of every one of them. So
+//   * x is converted once per CTA, a block or a few per warp, and every row of the CTA uses it;
+//   * a row's partial sums meet in shared memory: one barrier per kRound tiles, no hand-off between CTAs, results
+//     that do not depend on timing;
+//   * the warps of a CTA read adjacent blocks of the same rows at about the same time: whole DRAM pages.
+// (Units dealt to all warps of the GPU in one contiguous range each had every CTA convert all of x and a tile's sums travel
+// through L2: Q/K/V 6144 x 4096 Q4_K 7.2 us, down 4096 x 12288 Q6_K 15.8 us.)
+//
+// A format F supplies: the copies of one unit (16 rows x one block) into a ring slot, the conversion of x, and the
+// unit's dot products. Copies are 16-byte cp.async; a warp keeps `depth` units in flight, requested before the dependency
+// wait: weights depend on no kernel.
+// Bound: HBM for large matrices; a few MB are bound by launch, x and write-back latency.
+#pragma once
+
+#include "kernels.h"
+#include "stream_skel.cuh"
+
+namespace zc {
+namespace {
+
+constexpr int kRound = 4;  // tiles between two meetings of a CTA's warps
+
+struct SliceArgs {
+    const uint8_t* A[2];
+    const uint8_t* a_end[2];   // first byte past the buffers (formats that fetch aligned supersets)
+    const float* x;
+    float* y;
+    float* y2;
+    const float* gate;
+    uint32_t M, K, acc_mode;
+    uint32_t* status;
+    // kSeg 1: matrices that share x; kSeg 2: expert slots, one output block each; kSeg 3: expert slots side by side along K
+    uint32_t nseg;
+    uint32_t seg_end[3];       // last tile + 1 of matrix i
+    const uint8_t* segA[3];
+    float* segY[3];
+    uint32_t segM[3];
+    const uint32_t* routing;
+    uint64_t expert_stride;
+    uint32_t n_experts_max;
+    uint32_t x_slot_stride;    // kSeg 3: elements between the slots' activation vectors
+    PushArgs push;
+    ConsumeArgs consume;
+    uint32_t act;
+    const uint8_t* A_sh[2];
+    const uint8_t* A_sh_end[2];
+    const float* bias[2];
+    uint32_t late;
+    // how the work is cut
+    uint32_t h, tiles, tpe, tpc;   // rows per tile, tiles, tiles per expert slot, tiles per CTA
+    uint32_t n_wk, n_wr, depth;
+    uint32_t nblk, bpe;            // blocks of a (concatenated) row; of one matrix's row
+};
+
+inline SliceArgs slice_args(const DmmvArgs& a) {
+    SliceArgs s = {};
+    s.A[0] = a.A;
+    s.A[1] = a.A2 ? a.A2 : a.A;
+    s.a_end[0] = a.a_end;
+    s.a_end[1] = a.A2 ? a.a2_end : a.a_end;
+    s.x = a.x;
+    s.y = a.y;
+    s.y2 = a.y2;
+    s.gate = a.gate;
+    s.M = a.M;
+    s.K = a.K;
+    s.acc_mode = a.acc_mode;
+    s.status = a.status;
+    s.nseg = 1;
+    s.routing = a.routing;
+    s.expert_stride = a.expert_stride;
+    s.n_experts_max = a.n_experts_max;
+    s.x_slot_stride = a.x_expert_stride;
+    s.push = a.push;
+    s.consume = a.consume;
+    s.act = a.act;
+    s.A_sh[0] = a.A_sh;
+    s.A_sh[1] = a.A2_sh ? a.A2_sh : a.A_sh;
+    s.A_sh_end[0] = a.a_sh_end;
+    s.A_sh_end[1] = a.A2_sh ? a.a2_sh_end : a.a_sh_end;
+    s.bias[0] = a.bias;
+    s.bias[1] = a.bias2;
+    s.late = a.late ? 1u : 0u;
+    return s;
+}
+
+// One block of up to 16 rows.
+struct Unit {
+    const uint8_t* mat;  // the matrix's first byte; nullptr: a slot without an expert on this rank (contributes zeros)
+    const uint8_t* end;
+    uint32_t row0, rows, Mrows;  // first row, valid rows of the tile, rows of the matrix
+    uint32_t lb, kb;     // block within the matrix's row, within the concatenated row
+};
+
+template <int kSeg>
+__device__ __forceinline__ Unit find_unit(const SliceArgs& a, uint32_t T, uint32_t strm, uint32_t kb) {
+    Unit u;
+    u.kb = u.lb = kb;
+    u.Mrows = a.M;
+    if constexpr (kSeg == 1) {
+        const uint32_t sg = (T >= a.seg_end[0] ? 1u : 0u) + (T >= a.seg_end[1] ? 1u : 0u);
+        const uint32_t t0 = sg == 0 ? 0u : sg == 1 ? a.seg_end[0] : a.seg_end[1];
+        u.mat = sg == 0 ? a.segA[0] : sg == 1 ? a.segA[1] : a.segA[2];
+        u.Mrows = sg == 0 ? a.segM[0] : sg == 1 ? a.segM[1] : a.segM[2];
+        u.end = nullptr;
+        u.row0 = (T - t0) * a.h;
+    } else if constexpr (kSeg == 2 || kSeg == 3) {
+        const uint32_t slot = kSeg == 2 ? T / a.tpe : kb / a.bpe;
+        u.row0 = (kSeg == 2 ? T - slot * a.tpe : T) * a.h;
+        if (kSeg == 3) u.lb = kb - slot * a.bpe;
+        const uint32_t e = __ldg(a.routing + slot);
+        u.mat = e == kSkipExpert ? nullptr
+                                 : expert_matrix(a.A[strm], a.A_sh[strm], e, a.expert_stride, a.n_experts_max, a.status);
+        u.end = u.mat && u.mat == a.A_sh[strm] ? a.A_sh_end[strm] : a.a_end[strm];
+    } else {
+        u.mat = a.A[strm];
+        u.end = a.a_end[strm];
+        u.row0 = T * a.h;
+    }
+    u.rows = min(a.h, u.Mrows - u.row0);
+    return u;
+}
+
+// The output row a thread finishes, and what its epilogue reads besides the sums: requested ahead of the barrier.
+struct OutRow {
+    float *y, *y2;
+    uint32_t row;
+    bool ok;
+    float yold, b0, b1;
+};
+
+template <int EPI, int kSeg>
+__device__ __forceinline__ OutRow out_row(const SliceArgs& a, uint32_t T, uint32_t rr, bool live) {
+    OutRow o{nullptr, nullptr, 0u, false, 0.f, 0.f, 0.f};
+    if (!live || rr >= a.h) return o;
+    uint32_t Mrows = a.M, slot = 0;
+    o.y = a.y;
+    o.y2 = a.y2;
+    if constexpr (kSeg == 1) {
+        const uint32_t sg = (T >= a.seg_end[0] ? 1u : 0u) + (T >= a.seg_end[1] ? 1u : 0u);
+        o.row = (T - (sg == 0 ? 0u : sg == 1 ? a.seg_end[0] : a.seg_end[1])) * a.h + rr;
+        Mrows = sg == 0 ? a.segM[0] : sg == 1 ? a.segM[1] : a.segM[2];
+        o.y = sg == 0 ? a.segY[0] : sg == 1 ? a.segY[1] : a.segY[2];
+    } else if constexpr (kSeg == 2) {
+        slot = T / a.tpe;
+        o.row = (T - slot * a.tpe) * a.h + rr;
+        o.y += (size_t)slot * a.M;
+        if (o.y2) o.y2 += (size_t)slot * a.M;
+    } else {
+        o.row = T * a.h + rr;
+    }
+    o.ok = o.row < Mrows;
+    if (!o.ok) return o;
+    const bool adds = EPI == EPI_ACC || EPI == EPI_SIGMOID_ACC || (EPI == EPI_PLAIN && a.acc_mode != 0 && a.push.world == 0);
+    if (adds) o.yold = o.y[o.row];
+    if constexpr (EPI == EPI_SIGMOID_ACC) o.b0 = __ldg(a.gate);
+    if constexpr (EPI == EPI_PAIR) {  // the slot's expert's biases (none for a shared or absent expert)
+        if (a.bias[0]) {
+            const uint32_t e = __ldg(a.routing + slot);
+            if (e < a.n_experts_max) {
+                o.b0 = __ldg(a.bias[0] + (size_t)e * a.M + o.row);
+                if (a.bias[1]) o.b1 = __ldg(a.bias[1] + (size_t)e * a.M + o.row);
+            }
+        }
+    }
+    if constexpr (EPI == EPI_ACC) {  // the selected experts' biases, weighted like their products
+        if (a.bias[0]) {
+#pragma unroll 4
+            for (uint32_t s = 0; s < a.nseg; ++s) {
+                const uint32_t e = __ldg(a.routing + s);
+                if (e < a.n_experts_max)
+                    o.b0 = fmaf(__uint_as_float(__ldg(a.routing + a.nseg + s)), __ldg(a.bias[0] + (size_t)e * a.M + o.row), o.b0);
+            }
+        }
+    }
+    return o;
+}
+
+template <int NS, int EPI>
+__device__ __forceinline__ void write_out(const SliceArgs& a, const OutRow& o, const float (&v)[NS]) {
+    if (!o.ok) return;
+    if constexpr (EPI == EPI_GATE_UP) {
+        o.y[o.row] = (v[0] / (1.0f + expf(-v[0]))) * v[NS - 1];
+    } else if constexpr (EPI == EPI_ACC) {
+        o.y[o.row] = o.yold + (v[0] + o.b0);
+    } else if constexpr (EPI == EPI_PAIR) {
+        const float vg = v[0] + o.b0, vu = v[NS - 1] + o.b1;
+        if (a.act) {
+            o.y[o.row] = gate_up_act(a.act, vg, vu);
+        } else {
+            o.y[o.row] = vg;
+            o.y2[o.row] = vu;
+        }
+    } else if constexpr (EPI == EPI_SIGMOID_ACC) {
+        o.y[o.row] = o.yold + (1.0f / (1.0f + expf(-o.b0))) * v[0];
+    } else if (a.push.world) {
+        const uint2 pv = make_uint2(__float_as_uint(v[0]), 1u);
+        for (uint32_t r = 0; r < a.push.world; ++r) a.push.peers[r][o.row] = pv;
+    } else {
+        o.y[o.row] = a.acc_mode ? o.yold + v[0] : v[0];
+    }
+}
+
+// F: format; Extra: what its activation loader takes besides the arguments (nothing, or the attention partials).
+template <typename F, int NS, int EPI, int kSeg, typename Extra>
+__device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extra) {
+    extern __shared__ uint8_t smem_raw[];
+    pdl_begin(a.late);
+    uint8_t* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    const uint32_t n_warps = blockDim.x >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t* ring = base + (size_t)warp * a.depth * F::kSlot;
+    float* spart = reinterpret_cast<float*>(base + (size_t)n_warps * a.depth * F::kSlot);  // [2][kRound][n_wk][NS * 16]
+    const uint32_t part_tile = a.n_wk * NS * 16;
+    const typename F::Tab tab = F::carve(reinterpret_cast<uint8_t*>(spart + 2 * kRound * part_tile), a.nblk);
+    const uint32_t wk = (uint32_t)warp % a.n_wk, wr = (uint32_t)warp / a.n_wk;
+    const uint32_t ct0 = blockIdx.x * a.tpc, nt = min(a.tpc, a.tiles - ct0);
+
+    typename F::Copier copier;
+    copier.init(a, lane);
+    // the unit to request next: tile, stream, block
+    uint32_t p_tl = wr, p_strm = 0, p_kb = wk;
+    auto request = [&](uint32_t slot) {
+        if (p_tl < nt) {
+            const Unit u = find_unit<kSeg>(a, ct0 + p_tl, p_strm, p_kb);
+            if (u.mat) copier.copy(a, u, ring + slot * F::kSlot, lane);
+            p_kb += a.n_wk;
+            if (p_kb >= a.nblk) {
+                p_kb = wk;
+                if (++p_strm == NS) {
+                    p_strm = 0;
+                    p_tl += a.n_wr;
+                }
+            }
+        }
+        cp_async_commit();
+    };
+    pdl_late(a.late);
+    typename F::X xr;
+    if (a.late) F::template load_x<kSeg>(xr, a, extra, warp, lane, n_warps);
+    for (uint32_t i = 0; i < a.depth; ++i) request(i);
+    pdl_wait();
+    if (!a.late) F::template load_x<kSeg>(xr, a, extra, warp, lane, n_warps);
+    if (a.consume.n) consume_pushed(a.consume, blockIdx.x, gridDim.x, tid, blockDim.x);
+    F::prep(tab, xr, a, warp, lane, tid, n_warps);
+    __syncthreads();
+
+    typename F::Lane ln;
+    ln.init(a, tab, lane);
+    const uint32_t ring_s = smem_u32(ring);
+    uint32_t slot = 0;
+    for (uint32_t r0 = 0, buf = 0; r0 < nt; r0 += kRound, buf ^= 1) {
+        for (uint32_t tl = r0 + wr; tl < min(r0 + (uint32_t)kRound, nt); tl += a.n_wr) {
+            float* part = spart + (buf * kRound + (tl - r0)) * part_tile + wk * (NS * 16);
+#pragma unroll
+            for (int strm = 0; strm < NS; ++strm) {
+                typename F::Acc acc;
+                acc.clear();
+                for (uint32_t kb = wk; kb < a.nblk; kb += a.n_wk) {
+                    if (a.depth == 2) cp_async_wait<1>();
+                    else if (a.depth == 3) cp_async_wait<2>();
+                    else cp_async_wait<3>();
+                    __syncwarp();
+                    const Unit u = find_unit<kSeg>(a, ct0 + tl, strm, kb);
+                    if (u.mat) ln.dot(a, u, ring_s + slot * F::kSlot, acc);
+                    __syncwarp();
+                    request(slot);
+                    if (++slot == a.depth) slot = 0;
+                }
+                float v0, v1;
+                ln.finish(acc, v0, v1);  // rows g and g + 8, this lane's share
+                v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 1);
+                v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 1);
+                v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2);
+                v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
+                if ((lane & 3) == 0) {
+                    part[strm * 16 + (lane >> 2)] = v0;
+                    part[strm * 16 + (lane >> 2) + 8] = v1;
+                }
+            }
+        }
+        // four lanes per row add the warps' shares, in a fixed order
+        const uint32_t n_red = min((uint32_t)kRound, nt - r0) * 64;
+        auto row_of = [&](uint32_t i) { return out_row<EPI, kSeg>(a, ct0 + r0 + (i >> 6), (i >> 2) & 15u, i < n_red && (i & 3u) == 0); };
+        OutRow o = row_of(tid);
+        __syncthreads();
+        for (uint32_t i = tid; i < n_red; i += blockDim.x) {
+            if (i != (uint32_t)tid) o = row_of(i);
+            const float* p = spart + (buf * kRound + (i >> 6)) * part_tile + ((i >> 2) & 15u);
+            float v[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                float w = 0.f;
+                for (uint32_t k = i & 3u; k < a.n_wk; k += 4) w += p[k * (NS * 16) + s * 16];
+                w += __shfl_xor_sync(0xFFFFFFFFu, w, 1);
+                w += __shfl_xor_sync(0xFFFFFFFFu, w, 2);
+                v[s] = w;
+            }
+            write_out<NS, EPI>(a, o, v);
+        }
+    }
+}
+
+struct NoExtra {};
+template <typename F, int NS, int EPI, int kSeg, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dmmv_slice_kernel(const SliceArgs a) {
+    slice_body<F, NS, EPI, kSeg>(a, NoExtra());
+}
+template <typename F, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dmmv_slice_merge_kernel(const SliceArgs a, const MergeArgs m) {
+    slice_body<F, 1, EPI_PLAIN, 0>(a, m);
+}
+
+constexpr uint32_t kSliceSmem1 = 232448u, kSliceSmem2 = 113u * 1024u;  // one, two CTAs per SM
+
+// Cuts the work. `rows(i)`: the row counts of the matrices (kSeg 1) or of one expert slot. False: x does not fit.
+template <typename F>
+bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, uint32_t& grid, uint32_t& smem) {
+    a.bpe = (a.K + F::kCols - 1) / F::kCols;
+    a.nblk = a.bpe * (kSeg == 3 ? a.nseg : 1u);
+    const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 148u;
+    // Few blocks: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen.
+    // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
+    const uint32_t most = a.nblk <= 8 ? 8u : 16u;
+    const uint32_t per = (a.nblk + most - 1) / most;
+    a.n_wk = (a.nblk + per - 1) / per;
+    a.n_wr = most / a.n_wk;
+    if (a.n_wr > (uint32_t)kRound) a.n_wr = kRound;
+    if (a.n_wr == 3) a.n_wr = 2;  // kRound tiles are dealt evenly
+    warps = a.n_wk * a.n_wr;
+    const uint32_t per_sm = most == 8 ? 2u : 1u, room = most == 8 ? kSliceSmem2 : kSliceSmem1;
+    const uint32_t fixed = 128u + 2u * kRound * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
+    if (fixed + warps * 2u * F::kSlot > room) return false;
+    a.depth = (room - fixed) / (warps * F::kSlot);
+    a.depth = a.depth > 4 ? 4 : a.depth;
+    smem = fixed + warps * a.depth * F::kSlot;
+    // Tile height: the one that gives the busiest CTA the least to do (an MMA costs the same for fewer rows: 0.3 per row)
+    uint32_t best = 0xFFFFFFFFu;
+    for (uint32_t h = 16; h >= 4; --h) {
+        uint32_t tiles = 0;
+        if (kSeg == 1) for (uint32_t i = 0; i < a.nseg; ++i) tiles += (a.segM[i] + h - 1) / h;
+        else tiles = ((a.M + h - 1) / h) * (kSeg == 2 ? a.nseg : 1u);
+        const uint32_t tpc = (tiles + sms * per_sm - 1) / (sms * per_sm);
+        const uint32_t cost = tpc * (10 * h + 3 * (16 - h));
+        if (cost < best) {
+            best = cost;
+            a.h = h;
+            a.tiles = tiles;
+            a.tpc = tpc;
+        }
+    }
+    a.tpe = (a.M + a.h - 1) / a.h;
+    if (kSeg == 1) {
+        uint32_t t = 0;
+        for (uint32_t i = 0; i < 3; ++i) {
+            if (i < a.nseg) t += (a.segM[i] + a.h - 1) / a.h;
+            a.seg_end[i] = i < a.nseg ? t : 0xFFFFFFFFu;
+        }
+    }
+    grid = (a.tiles + a.tpc - 1) / a.tpc;
+    return true;
+}
+
+template <typename F, int NS, int EPI, int kSeg>
+cudaError_t slice_launch(SliceArgs a, int sm_count, cudaStream_t s) {
+    uint32_t warps, grid, smem;
+    if (!slice_plan<F>(a, NS, kSeg, sm_count, warps, grid, smem)) return cudaErrorInvalidConfiguration;
+    static std::atomic<uint64_t> attr8{0}, attr16{0};
+    if (warps <= 8) {
+        auto kern = dmmv_slice_kernel<F, NS, EPI, kSeg, 8>;
+        if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, attr8); e != cudaSuccess) return e;
+        return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
+    }
+    auto kern = dmmv_slice_kernel<F, NS, EPI, kSeg, 16>;
+    if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, attr16); e != cudaSuccess) return e;
+    return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
+}
+
+// Does the activation of a launch fit beside two units per warp?
+template <typename F>
+bool slice_fits(uint32_t K, uint32_t slots, int NS) {
+    SliceArgs a = {};
+    a.M = 16;
+    a.K = K;
+    a.nseg = slots;
+    uint32_t w, g, m;
+    return slice_plan<F>(a, NS, slots > 1 ? 3 : 0, 148, w, g, m) && a.nblk <= F::kPrepBlocks * w;
+}
+
+}  // namespace
+}  // namespace zc

@@ -1,26 +1,12 @@
-// zc_dmmv_q4k_static_scratch: the streaming Q4_K matvec with its split-K scratch in a
-// file-scope __device__ array instead of memory a context allocated.
+// zc_dmmv_q4k_static_scratch: the streaming Q4_K matvec without a context.
 //
-// Why: the streaming matvec hands partial row sums between warps of different CTAs through a
-// small global scratch (each sum stored together with a tag word). Every other entry point takes that
-// scratch from a context, and creating a context allocates (device scratch, pinned status
-// words, a stream). A host that has already given all device memory to its own arena (weights
-// and KV cache sized to fill HBM), or that runs where an allocation would synchronise the
-// device (inside its decode loop), cannot afford that. This entry point needs no context and
-// calls no allocating routine: the scratch is part of the loaded module.
+// Why: creating a context allocates (device scratch, pinned status words, a stream). A host that has already given all
+// device memory to its own arena (weights and KV cache sized to fill HBM), or that runs where an allocation would
+// synchronise the device (inside its decode loop), cannot afford that. This entry point needs no context and calls no
+// allocating routine; the kernel keeps its partial sums in shared memory and touches no device memory but its operands.
 //
-// The array is shared by every call on the same device. Consequences:
-//  * the array must be all zero when a launch starts. A __device__ array is zero when the module
-//    is loaded on a device, and each launch leaves it zero (the reader of a tagged sum clears it),
-//    so the set-up writes nothing. A launch that gave up on a bounded wait (status word set) may
-//    leave tagged sums behind; the next call sees the non-zero status word only if the caller
-//    checks it, so a caller that finds status_words[0] != 0 must stop using this entry point on
-//    that device.
-//  * two calls whose kernels can overlap (different streams, or threads without ordering)
-//    race on the array and give wrong results. Calls on one stream are ordered and safe.
-//
-// Set-up happens inside the first call on each device: cudaGetSymbolAddress and one attribute
-// query (no device work). Make the first call on a device before starting any stream capture on it.
+// Set-up happens inside the first call on each device: one attribute query (no device work). Make the first call on a
+// device before starting any stream capture on it.
 #include <cuda_runtime.h>
 #include <stdarg.h>
 #include <stdint.h>
@@ -36,17 +22,11 @@ namespace {
 
 using namespace zc;
 
-// Scratch capacity: kStreamMaxWorkers (4096) worker warps, each 32 partial sums as {f32 bits, tag}
-// pairs: 4096 * 32 * 8 = 1048576 bytes.
-constexpr size_t kStaticScratchBytes = kStreamPartialBytes;
 constexpr uint32_t kStaticMaxK = 12288;  // 48 blocks of 256: what the per-warp staging holds
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
-
 struct DeviceState {
     bool ready = false;
-    unsigned char* scratch = nullptr;  // device address of g_static_scratch on this device
     int sm_count = 0;
 };
 
@@ -68,13 +48,9 @@ cudaError_t setup_device(int device, DeviceState** out) {
     std::lock_guard<std::mutex> lock(g_dev_mutex);
     DeviceState& st = g_dev[device];
     if (!st.ready) {
-        void* ptr = nullptr;
-        cudaError_t e = cudaGetSymbolAddress(&ptr, g_static_scratch);
-        if (e != cudaSuccess) return e;
         int sms = 0;
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (e != cudaSuccess) return e;
-        st.scratch = static_cast<unsigned char*>(ptr);
         st.sm_count = sms;
         st.ready = true;
     }
@@ -121,7 +97,7 @@ extern "C" int32_t zc_dmmv_q4k_static_scratch(void* cuda_stream, const void* A, 
     DeviceState* st = nullptr;
     e = setup_device(device, &st);
     if (e != cudaSuccess)
-        return sfail(err_buf, err_cap, ZC_ERR_CUDA, "%s: set-up of the static scratch: %s", fn, cudaGetErrorString(e));
+        return sfail(err_buf, err_cap, ZC_ERR_CUDA, "%s: device query: %s", fn, cudaGetErrorString(e));
 
     DmmvArgs a;
     a.A = static_cast<const uint8_t*>(A) + a_offset;
@@ -130,10 +106,10 @@ extern "C" int32_t zc_dmmv_q4k_static_scratch(void* cuda_stream, const void* A, 
     a.M = M;
     a.K = K;
     a.acc_mode = acc_mode;
-    a.scratch_partial = reinterpret_cast<uint2*>(st->scratch);
     a.status = status_words;
     a.sm_count = st->sm_count;
-    if (!warp_dmmv_eligible(T_Q4_K, MODE_PLAIN, a))
+    const uint64_t units = ((uint64_t)M + 15) / 16 * ((K / 256 + 1) / 2);
+    if (units < 16 || !warp_dmmv_eligible(T_Q4_K, MODE_PLAIN, a))
         return sfail(err_buf, err_cap, ZC_ERR_INVALID_ARG,
                      "%s: M=%u K=%u is too small for the streaming kernel (needs at least 16 row-tile x k-segment "
                      "units); use zc_dmmv",

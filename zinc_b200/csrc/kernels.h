@@ -101,11 +101,7 @@ struct DmmvArgs {
     uint32_t n_tokens = 1;        // MODE_MOE_BATCHED
     uint32_t x_token_stride = 0;  // MODE_MOE_BATCHED, elements
     uint32_t y_token_stride = 0;  // MODE_MOE_BATCHED, elements
-    // context scratch of the split-K streaming kernels (null: streaming path not used)
-    uint2* scratch_partial = nullptr;   // [kStreamMaxWorkers][32] {f32 bits, tag} partial sums handed across CTAs;
-                                        // all zero between launches (the reader of a value clears it)
     uint32_t* status = nullptr;
-    uint32_t spin_limit = 1u << 26;     // polls after which a device-side wait gives up
     int sm_count = 0;
     PushArgs push;        // MODE_PLAIN: store the result rows into every rank's receive buffer instead of y
     ConsumeArgs consume;  // a pending reduction of pushed vectors that this launch (or a small kernel before it) completes
@@ -130,17 +126,14 @@ struct DmmvArgs {
     MergeArgs merge;  // MODE_PLAIN on the Q4_K streaming kernel: x comes from attention partials
 };
 
-// Capacity of the split-K scratch a context owns.
 // Below this many weight bytes a matvec is latency-bound and the one-warp-per-row kernels (more CTAs) win.
 constexpr uint64_t kStreamMinBytes = 2u << 20;
-constexpr uint32_t kStreamMaxWorkers = 4096;  // warps that may publish a partial tile
-constexpr size_t kStreamPartialBytes = (size_t)kStreamMaxWorkers * 32 * sizeof(uint2);
 
-// Warp-autonomous streaming (cp.async + tensor-core) matvec: eligibility and launch.
+// Streaming (cp.async + tensor-core) matvec, Q4_K: eligibility and launch.
 bool warp_dmmv_eligible(uint32_t type, int mode, const DmmvArgs& a);
 cudaError_t launch_warp_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t s, uint64_t* launches);
 // Grouped form: n (2 or 3) Q4_K matrices that share x and K, one launch. `common` carries x, K, acc_mode,
-// the scratch, the status words and the SM count.
+// the status words and the SM count.
 bool warp_dmmv_multi_eligible(uint32_t type, uint32_t n, const uint8_t* const* A, const uint32_t* M, uint32_t K,
                               const DmmvArgs& common);
 cudaError_t launch_warp_dmmv_multi(uint32_t n, const uint8_t* const* A, float* const* y, const uint32_t* M,
@@ -161,6 +154,10 @@ bool q6k_dmmv_eligible(uint32_t type, int mode, const DmmvArgs& a);
 cudaError_t launch_q6k_dmmv(int mode, const DmmvArgs& a, cudaStream_t s, uint64_t* launches);
 bool q6k_moe_down_acc_eligible(uint32_t type, const DmmvArgs& a);
 cudaError_t launch_q6k_moe_down_acc(const DmmvArgs& a, cudaStream_t s, uint64_t* launches);
+
+// MODE_PLAIN on the row kernel (dmmv_row.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4, any size.
+bool row_dmmv_eligible(uint32_t type, const DmmvArgs& a);
+cudaError_t launch_row_dmmv(uint32_t type, const DmmvArgs& a, cudaStream_t s);
 
 // Returns cudaSuccess or the launch error; *launches is incremented per kernel.
 cudaError_t launch_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t s, uint64_t* launches);

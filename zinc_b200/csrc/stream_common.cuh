@@ -77,9 +77,4 @@ __device__ __forceinline__ float ld_cg_f32(const float* p) {
 // Work units are (16-row tile, k-chunk) pairs in tile-major order; worker (warp) c of G owns the
 // contiguous unit range [c*U/G, (c+1)*U/G). With G <= U every worker owns at least one unit.
 __device__ __forceinline__ uint64_t part_begin(uint64_t c, uint64_t U, uint64_t G) { return c * U / G; }
-// The worker that owns unit u.
-__device__ __forceinline__ uint32_t part_owner(uint64_t u, uint64_t U, uint64_t G) {
-    return (uint32_t)(((u + 1) * G + U - 1) / U - 1);
-}
-
 }  // namespace zc
