@@ -26,7 +26,6 @@ constexpr int kRowSlot = 304;                // 288-byte aligned superset + 16: 
 constexpr int kPiecesRow = 18;
 constexpr int kPiecesLane = 16 * kPiecesRow / 32;  // 9
 constexpr int kZeroUnits = 64;               // zeros the lanes of dead columns read (one step's table is 512 bytes)
-constexpr int kPrepChunks = 6;               // 256-element chunks of x per warp
 
 struct TabX {
     uint4* zeros;
@@ -39,7 +38,7 @@ struct TabX {
 // the slots' vectors, x + s * x_stride, each padded to whole units and scaled by the slot's routing weight wts[s], so
 // that sum_s w_s W_s x_s becomes one long dot product.
 struct XRegsX {
-    float4 lo[kPrepChunks], hi[kPrepChunks];
+    float4 lo, hi;
 };
 
 struct FmtMX {
@@ -47,7 +46,6 @@ struct FmtMX {
     using X = XRegsX;
     static constexpr uint32_t kSlot = 16 * kRowSlot;
     static constexpr uint32_t kCols = 512;
-    static constexpr uint32_t kPrepBlocks = kPrepChunks / 2;  // in units
     static uint32_t table_bytes(uint32_t nblk) { return kZeroUnits * 16 + nblk * (2048 + 8) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
@@ -57,27 +55,19 @@ struct FmtMX {
         t.xs = reinterpret_cast<float*>(t.xf + (size_t)nblk * 128);
         return t;
     }
+    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return 2 * nblk; }  // chunks of 256 elements
     template <int kSeg>
-    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, int warp, int lane, uint32_t n_warps) {
-        const int b = lane >> 2, j = lane & 3;
-#pragma unroll
-        for (int i = 0; i < kPrepChunks; ++i) {
-            const uint32_t chunk = warp + i * n_warps;
-            const uint32_t slot = kSeg == 3 ? chunk / (2 * a.bpe) : 0u, lc = chunk - slot * 2 * a.bpe;
-            const uint32_t e0 = lc * 256 + b * 32 + 4 * j;
-            float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-            if (chunk < 2 * a.nblk && e0 < a.K) {  // K is a multiple of 32: the whole block or none of it
-                const float* xs = a.x + (size_t)slot * a.x_slot_stride;
-                lo = __ldg(reinterpret_cast<const float4*>(xs + e0));
-                hi = __ldg(reinterpret_cast<const float4*>(xs + e0 + 16));
-                if (kSeg == 3) {
-                    const float w = __uint_as_float(__ldg(a.routing + a.nseg + slot));
-                    lo = make_float4(lo.x * w, lo.y * w, lo.z * w, lo.w * w);
-                    hi = make_float4(hi.x * w, hi.y * w, hi.z * w, hi.w * w);
-                }
-            }
-            r.lo[i] = lo;
-            r.hi[i] = hi;
+    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t chunk, int lane) {
+        const uint32_t b = lane >> 2, j = lane & 3;
+        const uint32_t slot = kSeg == 3 ? chunk / (2 * a.bpe) : 0u, lc = chunk - slot * 2 * a.bpe;
+        const uint32_t e0 = lc * 256 + b * 32 + 4 * j;
+        r.lo = r.hi = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e0 < a.K) {  // K is a multiple of 32: the whole block or none of it
+            const float* xs = a.x + (size_t)slot * a.x_slot_stride + e0;
+            const float w = kSeg == 3 ? __uint_as_float(__ldg(a.routing + a.nseg + slot)) : 1.f;
+            const float4 lo = __ldg(reinterpret_cast<const float4*>(xs)), hi = __ldg(reinterpret_cast<const float4*>(xs + 16));
+            r.lo = make_float4(lo.x * w, lo.y * w, lo.z * w, lo.w * w);
+            r.hi = make_float4(hi.x * w, hi.y * w, hi.z * w, hi.w * w);
         }
     }
     static __device__ __forceinline__ uint32_t pack(float a, float b) {
@@ -88,32 +78,29 @@ struct FmtMX {
         const __half2 v = *reinterpret_cast<const __half2*>(&h);
         return pack(a - __low2float(v), b - __high2float(v));
     }
-    static __device__ __forceinline__ void prep(const Tab& s, const X& r, const SliceArgs& a, int warp, int lane, int tid, uint32_t n_warps) {
-        for (uint32_t i = tid; i < kZeroUnits; i += blockDim.x) s.zeros[i] = make_uint4(0u, 0u, 0u, 0u);
+    static __device__ __forceinline__ void clear(const Tab& s, int tid) {
+        if (tid < kZeroUnits) s.zeros[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    static __device__ __forceinline__ void prep(const Tab& s, const X& r, const SliceArgs&, uint32_t chunk, int lane) {
         const uint32_t b = lane >> 2, j = lane & 3;
+        float4 lo = r.lo, hi = r.hi;
+        float mx = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(lo.w))),
+                         fmaxf(fmaxf(fabsf(hi.x), fabsf(hi.y)), fmaxf(fabsf(hi.z), fabsf(hi.w))));
 #pragma unroll
-        for (int i = 0; i < kPrepChunks; ++i) {
-            const uint32_t chunk = warp + i * n_warps;
-            if (chunk >= 2 * a.nblk) break;
-            float4 lo = r.lo[i], hi = r.hi[i];
-            float mx = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(lo.z), fabsf(lo.w))),
-                             fmaxf(fmaxf(fabsf(hi.x), fabsf(hi.y)), fmaxf(fabsf(hi.z), fabsf(hi.w))));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-            uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
-            E = E < 32u ? 32u : E;
-            const float scale = __uint_as_float((263u - E) << 23);
-            lo = make_float4(lo.x * scale, lo.y * scale, lo.z * scale, lo.w * scale);
-            hi = make_float4(hi.x * scale, hi.y * scale, hi.z * scale, hi.w * scale);
-            // byte k of a block's word j holds elements 4j + k and 16 + 4j + k
-            const uint4 h = make_uint4(pack(lo.x, hi.x), pack(lo.y, hi.y), pack(lo.z, hi.z), pack(lo.w, hi.w));
-            const uint4 l = make_uint4(rest(lo.x, hi.x, h.x), rest(lo.y, hi.y, h.y), rest(lo.z, hi.z, h.z), rest(lo.w, hi.w, h.w));
-            // block b of chunk c is block q + 4 t of unit c / 2
-            const uint32_t q = b & 3, t = 2 * (chunk & 1) + (b >> 2), u = (((chunk >> 1) * 4 + q) * 4 + j) * 2;
-            s.xf[u * 4 + t] = h;
-            s.xf[(u + 1) * 4 + t] = l;
-            if (lane == 0) s.xs[chunk] = __uint_as_float((E - 9u) << 23);
-        }
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+        uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
+        E = E < 32u ? 32u : E;
+        const float scale = __uint_as_float((263u - E) << 23);
+        lo = make_float4(lo.x * scale, lo.y * scale, lo.z * scale, lo.w * scale);
+        hi = make_float4(hi.x * scale, hi.y * scale, hi.z * scale, hi.w * scale);
+        // byte k of a block's word j holds elements 4j + k and 16 + 4j + k
+        const uint4 h = make_uint4(pack(lo.x, hi.x), pack(lo.y, hi.y), pack(lo.z, hi.z), pack(lo.w, hi.w));
+        const uint4 l = make_uint4(rest(lo.x, hi.x, h.x), rest(lo.y, hi.y, h.y), rest(lo.z, hi.z, h.z), rest(lo.w, hi.w, h.w));
+        // block b of chunk c is block q + 4 t of unit c / 2
+        const uint32_t q = b & 3, t = 2 * (chunk & 1) + (b >> 2), u = (((chunk >> 1) * 4 + q) * 4 + j) * 2;
+        s.xf[u * 4 + t] = h;
+        s.xf[(u + 1) * 4 + t] = l;
+        if (lane == 0) s.xs[chunk] = __uint_as_float((E - 9u) << 23);
     }
 
     // piece p = i * 32 + lane of a unit: row p / 18, 16-byte column p % 18 of the row's aligned superset
@@ -184,7 +171,7 @@ struct FmtMX {
             const uint32_t pa = slot + g * kRowSlot + oA + 68 * t, pb = slot + (g + 8) * kRowSlot + oB + 68 * t;
             const uint32_t left = nb - u.lb * kUnitBlocks;
             const float xs = lds_f1(xs_s + u.kb * 8);
-#pragma unroll
+#pragma unroll 1
             for (uint32_t q = 0; q < 4; ++q) {
                 // 17 bytes at byte offset o (0..3) inside five aligned words: the scale is byte o, nibble word i is
                 // bytes o + 1 + 4 i .. of them: one funnel shift by 8 (o + 1) bits (a shift of 32 hands back the

@@ -31,7 +31,6 @@ constexpr int kPieces6 = 14;                // 16-byte pieces per row superset
 constexpr int kPiecesLane6 = (16 * kPieces6 + 31) / 32;  // 7
 constexpr int kZeroBytes6 = 128;
 constexpr int kFracBits = 20;
-constexpr int kPrepBlocks = 6;
 constexpr int kBBytes = 1536;               // B operand table per super-block: [h 2][j pair 2][column 6][t 4][16 bytes]
 constexpr int kNsxBytes = 256;              // accumulator start values per super-block: [h 2][digit 4][j 4][u 2] s32
 
@@ -43,29 +42,19 @@ struct Tab6 {
 };
 
 struct XRegs6 {
-    float4 lo[kPrepBlocks], hi[kPrepBlocks];
+    float4 lo, hi;
 };
 // One warp per super-block; lane l handles the 8 consecutive elements 8l .. 8l+7. bpe: blocks of one vector; with more
 // than that (MoE down projection) the activation is several vectors, x + s * x_stride, each scaled by the slot's routing
 // weight wts[s].
-__device__ __forceinline__ void load_x6(XRegs6& r, const float* __restrict__ x, uint32_t nblk, uint32_t bpe, uint32_t x_stride,
-                                        const uint32_t* __restrict__ wts, int warp, int lane, uint32_t n_warps) {
-#pragma unroll
-    for (int b = 0; b < kPrepBlocks; ++b) {
-        const uint32_t blk = warp + b * n_warps;
-        if (blk < nblk) {
-            const uint32_t slot = wts ? blk / bpe : 0u, lb = blk - slot * bpe;
-            const float* xp = x + (size_t)slot * x_stride + (size_t)lb * 256 + 8 * lane;
-            float4 lo = __ldg(reinterpret_cast<const float4*>(xp)), hi = __ldg(reinterpret_cast<const float4*>(xp) + 1);
-            if (wts) {
-                const float w = __uint_as_float(__ldg(wts + slot));
-                lo = make_float4(lo.x * w, lo.y * w, lo.z * w, lo.w * w);
-                hi = make_float4(hi.x * w, hi.y * w, hi.z * w, hi.w * w);
-            }
-            r.lo[b] = lo;
-            r.hi[b] = hi;
-        }
-    }
+__device__ __forceinline__ void load_x6(XRegs6& r, const float* __restrict__ x, uint32_t blk, uint32_t bpe, uint32_t x_stride,
+                                        const uint32_t* __restrict__ wts, int lane) {
+    const uint32_t slot = wts ? blk / bpe : 0u, lb = blk - slot * bpe;
+    const float* xp = x + (size_t)slot * x_stride + (size_t)lb * 256 + 8 * lane;
+    const float w = wts ? __uint_as_float(__ldg(wts + slot)) : 1.f;
+    const float4 lo = __ldg(reinterpret_cast<const float4*>(xp)), hi = __ldg(reinterpret_cast<const float4*>(xp) + 1);
+    r.lo = make_float4(lo.x * w, lo.y * w, lo.z * w, lo.w * w);
+    r.hi = make_float4(hi.x * w, hi.y * w, hi.z * w, hi.w * w);
 }
 
 __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -74,53 +63,48 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
 
 // Lane l's elements 8l .. 8l+7 lie in half h = l/16, quarter j = (l/4)%4, sub-block half u = (l/2)%2, and are
 // the k-slot groups t = 2(l%2) and t+1 of that sub-block half.
-__device__ __forceinline__ void prep_x6(const Tab6& s, const XRegs6& r, uint32_t nblk, int warp, int lane, uint32_t n_warps) {
+__device__ __forceinline__ void prep_x6(const Tab6& s, const XRegs6& r, uint32_t blk, int lane) {
     const uint32_t h = lane >> 4, j = (lane >> 2) & 3, u = (lane >> 1) & 1, t0 = 2 * (lane & 1);
+    const float4 lo = r.lo, hi = r.hi;
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    float mx = 0.f;
 #pragma unroll
-    for (int b = 0; b < kPrepBlocks; ++b) {
-        const uint32_t blk = warp + b * n_warps;
-        if (blk >= nblk) break;
-        const float4 lo = r.lo[b], hi = r.hi[b];
-        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-        float mx = 0.f;
+    for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[e]));
 #pragma unroll
-        for (int e = 0; e < 8; ++e) mx = fmaxf(mx, fabsf(v[e]));
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
+    E = E < 32u ? 32u : E;
+    const float scale = __uint_as_float((127u + 126u + kFracBits - E) << 23);
+    int X[8];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-        uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
-        E = E < 32u ? 32u : E;
-        const float scale = __uint_as_float((127u + 126u + kFracBits - E) << 23);
-        int X[8];
+    for (int e = 0; e < 8; ++e) X[e] = __float2int_rn(v[e] * scale);
+    uint32_t dw[3][2];
+    int ds[3];
+    dw[0][0] = pack4(X[0] >> 14, X[1] >> 14, X[2] >> 14, X[3] >> 14);
+    dw[0][1] = pack4(X[4] >> 14, X[5] >> 14, X[6] >> 14, X[7] >> 14);
+    dw[1][0] = pack4(X[0] >> 7, X[1] >> 7, X[2] >> 7, X[3] >> 7) & 0x7F7F7F7Fu;
+    dw[1][1] = pack4(X[4] >> 7, X[5] >> 7, X[6] >> 7, X[7] >> 7) & 0x7F7F7F7Fu;
+    dw[2][0] = pack4(X[0], X[1], X[2], X[3]) & 0x7F7F7F7Fu;
+    dw[2][1] = pack4(X[4], X[5], X[6], X[7]) & 0x7F7F7F7Fu;
+    ds[0] = ds[1] = ds[2] = 0;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) X[e] = __float2int_rn(v[e] * scale);
-        uint32_t dw[3][2];
-        int ds[3];
-        dw[0][0] = pack4(X[0] >> 14, X[1] >> 14, X[2] >> 14, X[3] >> 14);
-        dw[0][1] = pack4(X[4] >> 14, X[5] >> 14, X[6] >> 14, X[7] >> 14);
-        dw[1][0] = pack4(X[0] >> 7, X[1] >> 7, X[2] >> 7, X[3] >> 7) & 0x7F7F7F7Fu;
-        dw[1][1] = pack4(X[4] >> 7, X[5] >> 7, X[6] >> 7, X[7] >> 7) & 0x7F7F7F7Fu;
-        dw[2][0] = pack4(X[0], X[1], X[2], X[3]) & 0x7F7F7F7Fu;
-        dw[2][1] = pack4(X[4], X[5], X[6], X[7]) & 0x7F7F7F7Fu;
-        ds[0] = ds[1] = ds[2] = 0;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            ds[0] += X[e] >> 14;
-            ds[1] += (X[e] >> 7) & 0x7F;
-            ds[2] += X[e] & 0x7F;
-        }
-        uint8_t* bq = s.bq + (size_t)blk * kBBytes + h * 768 + (j >> 1) * 384 + (j & 1) * 8;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            uint8_t* dst = bq + (2 * d + u) * 64 + t0 * 16;
-            // {b0, b1}: the digit word sits in the register that feeds the k slots of sub-block half u
-            *reinterpret_cast<uint2*>(dst) = u ? make_uint2(0u, dw[d][0]) : make_uint2(dw[d][0], 0u);
-            *reinterpret_cast<uint2*>(dst + 16) = u ? make_uint2(0u, dw[d][1]) : make_uint2(dw[d][1], 0u);
-            const int sum = ds[d] + __shfl_xor_sync(0xFFFFFFFFu, ds[d], 1);
-            if ((lane & 1) == 0) s.nsx[blk * 64 + h * 32 + d * 8 + j * 2 + u] = -32 * sum;
-        }
-        if ((lane & 1) == 0) s.nsx[blk * 64 + h * 32 + 24 + j * 2 + u] = 0;  // digit 3 does not exist: lane t = 3
-        if (lane == 0) s.xs[blk] = __uint_as_float((E + 1u - kFracBits) << 23);
+    for (int e = 0; e < 8; ++e) {
+        ds[0] += X[e] >> 14;
+        ds[1] += (X[e] >> 7) & 0x7F;
+        ds[2] += X[e] & 0x7F;
     }
+    uint8_t* bq = s.bq + (size_t)blk * kBBytes + h * 768 + (j >> 1) * 384 + (j & 1) * 8;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        uint8_t* dst = bq + (2 * d + u) * 64 + t0 * 16;
+        // {b0, b1}: the digit word sits in the register that feeds the k slots of sub-block half u
+        *reinterpret_cast<uint2*>(dst) = u ? make_uint2(0u, dw[d][0]) : make_uint2(dw[d][0], 0u);
+        *reinterpret_cast<uint2*>(dst + 16) = u ? make_uint2(0u, dw[d][1]) : make_uint2(dw[d][1], 0u);
+        const int sum = ds[d] + __shfl_xor_sync(0xFFFFFFFFu, ds[d], 1);
+        if ((lane & 1) == 0) s.nsx[blk * 64 + h * 32 + d * 8 + j * 2 + u] = -32 * sum;
+    }
+    if ((lane & 1) == 0) s.nsx[blk * 64 + h * 32 + 24 + j * 2 + u] = 0;  // digit 3 does not exist: lane t = 3
+    if (lane == 0) s.xs[blk] = __uint_as_float((E + 1u - kFracBits) << 23);
 }
 
 __device__ __forceinline__ uint32_t lds_u32s(uint32_t saddr) {
@@ -210,7 +194,6 @@ struct FmtQ6K {
     using X = XRegs6;
     static constexpr uint32_t kSlot = 16 * kRow6;
     static constexpr uint32_t kCols = 256;
-    static constexpr uint32_t kPrepBlocks = zc::kPrepBlocks;
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes6 + nblk * (kBBytes + kNsxBytes + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
@@ -221,13 +204,16 @@ struct FmtQ6K {
         t.xs = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(t.nsx) + (size_t)nblk * kNsxBytes);
         return t;
     }
+    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return nblk; }
     template <int kSeg>
-    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, int warp, int lane, uint32_t n_warps) {
-        load_x6(r, a.x, a.nblk, a.bpe, a.x_slot_stride, kSeg == 3 ? a.routing + a.nseg : nullptr, warp, lane, n_warps);
+    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t blk, int lane) {
+        load_x6(r, a.x, blk, a.bpe, a.x_slot_stride, kSeg == 3 ? a.routing + a.nseg : nullptr, lane);
     }
-    static __device__ __forceinline__ void prep(const Tab& t, const X& r, const SliceArgs& a, int warp, int lane, int tid, uint32_t n_warps) {
-        for (uint32_t i = tid; i < kZeroBytes6 / 16; i += blockDim.x) reinterpret_cast<uint4*>(t.zeros)[i] = make_uint4(0u, 0u, 0u, 0u);
-        prep_x6(t, r, a.nblk, warp, lane, n_warps);
+    static __device__ __forceinline__ void clear(const Tab& t, int tid) {
+        if (tid < kZeroBytes6 / 16) reinterpret_cast<uint4*>(t.zeros)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    static __device__ __forceinline__ void prep(const Tab& t, const X& r, const SliceArgs&, uint32_t blk, int lane) {
+        prep_x6(t, r, blk, lane);
     }
 
     // piece p = i * 32 + lane of a unit: row p / 14, 16-byte column p % 14 of the row's aligned superset

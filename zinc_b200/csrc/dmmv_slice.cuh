@@ -92,36 +92,56 @@ inline SliceArgs slice_args(const DmmvArgs& a) {
 struct Unit {
     const uint8_t* mat;  // the matrix's first byte; nullptr: a slot without an expert on this rank (contributes zeros)
     const uint8_t* end;
-    uint32_t row0, rows, Mrows;  // first row, valid rows of the tile, rows of the matrix
+    uint32_t row0, rows;  // first row, valid rows of the tile
     uint32_t lb, kb;     // block within the matrix's row, within the concatenated row
 };
 
-template <int kSeg>
-__device__ __forceinline__ Unit find_unit(const SliceArgs& a, uint32_t T, uint32_t strm, uint32_t kb) {
+// The matrices of the expert slots: lane s holds slot s's, found once (a look-up through the routing buffer per unit would
+// put a chain of dependent loads in front of every request). More than 32 slots: looked up each time.
+template <int NS, int kSeg>
+struct Slots {
+    const uint8_t* mat[NS];
+    __device__ __forceinline__ static const uint8_t* find(const SliceArgs& a, uint32_t slot, int strm) {
+        const uint32_t e = __ldg(a.routing + slot);
+        return e == kSkipExpert ? nullptr : expert_matrix(a.A[strm], a.A_sh[strm], e, a.expert_stride, a.n_experts_max, a.status);
+    }
+    __device__ __forceinline__ void init(const SliceArgs& a, int lane) {
+        if constexpr (kSeg >= 2) {
+#pragma unroll
+            for (int i = 0; i < NS; ++i) mat[i] = (uint32_t)lane < a.nseg ? find(a, lane, i) : nullptr;
+        }
+    }
+    __device__ __forceinline__ const uint8_t* get(const SliceArgs& a, uint32_t slot, uint32_t strm) const {
+        if (a.nseg > 32) return find(a, slot, (int)strm);
+        const uint64_t m = reinterpret_cast<uint64_t>(NS == 2 && strm ? mat[NS - 1] : mat[0]);
+        return reinterpret_cast<const uint8_t*>(__shfl_sync(0xFFFFFFFFu, m, slot));
+    }
+};
+
+template <int NS, int kSeg>
+__device__ __forceinline__ Unit find_unit(const SliceArgs& a, const Slots<NS, kSeg>& slots, uint32_t T, uint32_t strm, uint32_t kb) {
     Unit u;
     u.kb = u.lb = kb;
-    u.Mrows = a.M;
+    uint32_t M = a.M;
     if constexpr (kSeg == 1) {
         const uint32_t sg = (T >= a.seg_end[0] ? 1u : 0u) + (T >= a.seg_end[1] ? 1u : 0u);
         const uint32_t t0 = sg == 0 ? 0u : sg == 1 ? a.seg_end[0] : a.seg_end[1];
         u.mat = sg == 0 ? a.segA[0] : sg == 1 ? a.segA[1] : a.segA[2];
-        u.Mrows = sg == 0 ? a.segM[0] : sg == 1 ? a.segM[1] : a.segM[2];
+        M = sg == 0 ? a.segM[0] : sg == 1 ? a.segM[1] : a.segM[2];
         u.end = nullptr;
         u.row0 = (T - t0) * a.h;
     } else if constexpr (kSeg == 2 || kSeg == 3) {
         const uint32_t slot = kSeg == 2 ? T / a.tpe : kb / a.bpe;
         u.row0 = (kSeg == 2 ? T - slot * a.tpe : T) * a.h;
         if (kSeg == 3) u.lb = kb - slot * a.bpe;
-        const uint32_t e = __ldg(a.routing + slot);
-        u.mat = e == kSkipExpert ? nullptr
-                                 : expert_matrix(a.A[strm], a.A_sh[strm], e, a.expert_stride, a.n_experts_max, a.status);
+        u.mat = slots.get(a, slot, strm);
         u.end = u.mat && u.mat == a.A_sh[strm] ? a.A_sh_end[strm] : a.a_end[strm];
     } else {
         u.mat = a.A[strm];
         u.end = a.a_end[strm];
         u.row0 = T * a.h;
     }
-    u.rows = min(a.h, u.Mrows - u.row0);
+    u.rows = min(a.h, M - u.row0);
     return u;
 }
 
@@ -206,6 +226,9 @@ __device__ __forceinline__ void write_out(const SliceArgs& a, const OutRow& o, c
 }
 
 // F: format; Extra: what its activation loader takes besides the arguments (nothing, or the attention partials).
+// One loop requests a unit ahead and works off the oldest one. The request, the dot products and the meeting of the
+// warps each stand in the code once: with several copies (unrolled streams, a prologue of its own) the few units of a
+// launch ran through 20 KB of cold instructions, and "no instruction" was the largest stall.
 template <typename F, int NS, int EPI, int kSeg, typename Extra>
 __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extra) {
     extern __shared__ uint8_t smem_raw[];
@@ -222,12 +245,24 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
 
     typename F::Copier copier;
     copier.init(a, lane);
-    // the unit to request next: tile, stream, block
-    uint32_t p_tl = wr, p_strm = 0, p_kb = wk;
-    auto request = [&](uint32_t slot) {
+    typename F::Lane ln;
+    ln.init(a, tab, lane);
+    pdl_late(a.late);
+    Slots<NS, kSeg> slots;
+    slots.init(a, lane);
+
+    uint32_t p_tl = wr, p_strm = 0, p_kb = wk;  // the unit to request next: tile, stream, block
+    uint32_t tl = wr, strm = 0, kb = wk;        // the unit to work off next
+    uint32_t r0 = 0;                            // first tile of the round the warps meet for next
+    const uint32_t n_prep = F::prep_count(a.nblk), x_at = a.late ? 0u : a.depth - 1;
+    typename F::X x;
+    typename F::Acc acc;
+    acc.clear();
+    uint32_t p_slot = 0, slot = 0;
+    for (uint32_t it = 0;; ++it) {
         if (p_tl < nt) {
-            const Unit u = find_unit<kSeg>(a, ct0 + p_tl, p_strm, p_kb);
-            if (u.mat) copier.copy(a, u, ring + slot * F::kSlot, lane);
+            const Unit u = find_unit<NS, kSeg>(a, slots, ct0 + p_tl, p_strm, p_kb);
+            if (u.mat) copier.copy(a, u, ring + p_slot * F::kSlot, lane);
             p_kb += a.n_wk;
             if (p_kb >= a.nblk) {
                 p_kb = wk;
@@ -238,69 +273,79 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
             }
         }
         cp_async_commit();
-    };
-    pdl_late(a.late);
-    typename F::X xr;
-    if (a.late) F::template load_x<kSeg>(xr, a, extra, warp, lane, n_warps);
-    for (uint32_t i = 0; i < a.depth; ++i) request(i);
-    pdl_wait();
-    if (!a.late) F::template load_x<kSeg>(xr, a, extra, warp, lane, n_warps);
-    if (a.consume.n) consume_pushed(a.consume, blockIdx.x, gridDim.x, tid, blockDim.x);
-    F::prep(tab, xr, a, warp, lane, tid, n_warps);
-    __syncthreads();
-
-    typename F::Lane ln;
-    ln.init(a, tab, lane);
-    const uint32_t ring_s = smem_u32(ring);
-    uint32_t slot = 0;
-    for (uint32_t r0 = 0, buf = 0; r0 < nt; r0 += kRound, buf ^= 1) {
-        for (uint32_t tl = r0 + wr; tl < min(r0 + (uint32_t)kRound, nt); tl += a.n_wr) {
-            float* part = spart + (buf * kRound + (tl - r0)) * part_tile + wk * (NS * 16);
-#pragma unroll
-            for (int strm = 0; strm < NS; ++strm) {
-                typename F::Acc acc;
-                acc.clear();
-                for (uint32_t kb = wk; kb < a.nblk; kb += a.n_wk) {
-                    if (a.depth == 2) cp_async_wait<1>();
-                    else if (a.depth == 3) cp_async_wait<2>();
-                    else cp_async_wait<3>();
-                    __syncwarp();
-                    const Unit u = find_unit<kSeg>(a, ct0 + tl, strm, kb);
-                    if (u.mat) ln.dot(a, u, ring_s + slot * F::kSlot, acc);
-                    __syncwarp();
-                    request(slot);
-                    if (++slot == a.depth) slot = 0;
-                }
+        if (++p_slot == a.depth) p_slot = 0;
+        if (it == x_at) {
+            if (!a.late) pdl_wait();
+            if ((uint32_t)warp < n_prep) F::template load_x<kSeg>(x, a, extra, warp, lane);
+        }
+        if (it + 1 < a.depth) continue;
+        if (it + 1 == a.depth) {  // ---- the activation, once the ring is full ----
+            if (a.consume.n) consume_pushed(a.consume, blockIdx.x, gridDim.x, tid, blockDim.x);
+            F::clear(tab, tid);
+            for (uint32_t b = warp; b < n_prep; b += n_warps) {
+                typename F::X next;
+                if (b + n_warps < n_prep) F::template load_x<kSeg>(next, a, extra, b + n_warps, lane);
+                F::prep(tab, x, a, b, lane);
+                x = next;
+            }
+            __syncthreads();
+        }
+        bool meet = true;
+        if (tl < nt) {
+            if (a.depth == 2) cp_async_wait<1>();
+            else if (a.depth == 3) cp_async_wait<2>();
+            else cp_async_wait<3>();
+            __syncwarp();
+            const Unit u = find_unit<NS, kSeg>(a, slots, ct0 + tl, strm, kb);
+            if (u.mat) ln.dot(a, u, smem_u32(ring) + slot * F::kSlot, acc);
+            __syncwarp();
+            if (++slot == a.depth) slot = 0;
+            kb += a.n_wk;
+            meet = false;
+            if (kb >= a.nblk) {  // the warp's share of a tile's stream is complete
+                float* part = spart + (((tl / kRound) & 1) * kRound + tl % kRound) * part_tile + wk * (NS * 16) + strm * 16;
                 float v0, v1;
                 ln.finish(acc, v0, v1);  // rows g and g + 8, this lane's share
+                acc.clear();
                 v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 1);
                 v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 1);
                 v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2);
                 v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
                 if ((lane & 3) == 0) {
-                    part[strm * 16 + (lane >> 2)] = v0;
-                    part[strm * 16 + (lane >> 2) + 8] = v1;
+                    part[lane >> 2] = v0;
+                    part[(lane >> 2) + 8] = v1;
+                }
+                kb = wk;
+                if (++strm == NS) {
+                    strm = 0;
+                    tl += a.n_wr;
+                    meet = tl >= r0 + kRound || tl >= nt;
                 }
             }
         }
-        // four lanes per row add the warps' shares, in a fixed order
-        const uint32_t n_red = min((uint32_t)kRound, nt - r0) * 64;
-        auto row_of = [&](uint32_t i) { return out_row<EPI, kSeg>(a, ct0 + r0 + (i >> 6), (i >> 2) & 15u, i < n_red && (i & 3u) == 0); };
-        OutRow o = row_of(tid);
-        __syncthreads();
-        for (uint32_t i = tid; i < n_red; i += blockDim.x) {
-            if (i != (uint32_t)tid) o = row_of(i);
-            const float* p = spart + (buf * kRound + (i >> 6)) * part_tile + ((i >> 2) & 15u);
-            float v[NS];
+        if (meet) {
+            // ---- the warps meet: four lanes per row add the warps' shares, in a fixed order ----
+            const uint32_t buf = (r0 / kRound) & 1, n_red = min((uint32_t)kRound, nt - r0) * 64;
+            OutRow o{};
+            if ((uint32_t)tid < n_red) o = out_row<EPI, kSeg>(a, ct0 + r0 + (tid >> 6), (tid >> 2) & 15u, (tid & 3u) == 0);
+            __syncthreads();
+            for (uint32_t i = tid; i < n_red; i += blockDim.x) {
+                if (i != (uint32_t)tid) o = out_row<EPI, kSeg>(a, ct0 + r0 + (i >> 6), (i >> 2) & 15u, (i & 3u) == 0);
+                const float* p = spart + (buf * kRound + (i >> 6)) * part_tile + ((i >> 2) & 15u);
+                float v[NS];
 #pragma unroll
-            for (int s = 0; s < NS; ++s) {
-                float w = 0.f;
-                for (uint32_t k = i & 3u; k < a.n_wk; k += 4) w += p[k * (NS * 16) + s * 16];
-                w += __shfl_xor_sync(0xFFFFFFFFu, w, 1);
-                w += __shfl_xor_sync(0xFFFFFFFFu, w, 2);
-                v[s] = w;
+                for (int s = 0; s < NS; ++s) {
+                    float w = 0.f;
+#pragma unroll 4
+                    for (uint32_t k = i & 3u; k < a.n_wk; k += 4) w += p[k * (NS * 16) + s * 16];
+                    w += __shfl_xor_sync(0xFFFFFFFFu, w, 1);
+                    w += __shfl_xor_sync(0xFFFFFFFFu, w, 2);
+                    v[s] = w;
+                }
+                write_out<NS, EPI>(a, o, v);
             }
-            write_out<NS, EPI>(a, o, v);
+            r0 += kRound;
+            if (r0 >= nt) break;
         }
     }
 }
@@ -388,7 +433,7 @@ bool slice_fits(uint32_t K, uint32_t slots, int NS) {
     a.K = K;
     a.nseg = slots;
     uint32_t w, g, m;
-    return slice_plan<F>(a, NS, slots > 1 ? 3 : 0, 148, w, g, m) && a.nblk <= F::kPrepBlocks * w;
+    return slice_plan<F>(a, NS, slots > 1 ? 3 : 0, 148, w, g, m);
 }
 
 }  // namespace

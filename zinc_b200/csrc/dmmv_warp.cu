@@ -42,59 +42,46 @@ struct Tab {
 
 // Convert x into int8 digit planes. One warp per super-block; lane l handles the 8 consecutive elements
 // 8l .. 8l+7 (a 32-byte coalesced read), so sub-block s is lanes 4s .. 4s+3.
-constexpr int kPrepBlocks = 6;  // x super-blocks per warp
 struct XRegs {
-    float4 lo[kPrepBlocks], hi[kPrepBlocks];
+    float4 lo, hi;
 };
-__device__ __forceinline__ void load_x(XRegs& r, const float* __restrict__ x, uint32_t K, int warp, int lane, uint32_t kWarps) {
-#pragma unroll
-    for (int i = 0; i < kPrepBlocks; ++i) {
-        const uint32_t blk = warp + i * kWarps;
-        if (blk < (K >> 8)) {
-            const float* xp = x + (size_t)blk * 256 + 8 * lane;
-            r.lo[i] = __ldg(reinterpret_cast<const float4*>(xp));
-            r.hi[i] = __ldg(reinterpret_cast<const float4*>(xp) + 1);
-        }
-    }
+__device__ __forceinline__ void load_x(XRegs& r, const float* __restrict__ x, uint32_t blk, int lane) {
+    const float* xp = x + (size_t)blk * 256 + 8 * lane;
+    r.lo = __ldg(reinterpret_cast<const float4*>(xp));
+    r.hi = __ldg(reinterpret_cast<const float4*>(xp) + 1);
 }
 
 // The same eight elements per lane, merged from split-K attention partials (up to four chunks; head_dim a
 // multiple of 8, so a lane's elements share a head).
 constexpr int kMergeChunks = 4;
-__device__ __forceinline__ void load_x_merge(XRegs& r, const MergeArgs& m, uint32_t K, int warp, int lane, uint32_t kWarps) {
+__device__ __forceinline__ void load_x_merge(XRegs& r, const MergeArgs& m, uint32_t blk, int lane) {
+    const uint32_t k0 = blk * 256 + 8 * lane, head = k0 / m.head_dim, d = k0 - head * m.head_dim;
+    float4 pl[kMergeChunks], ph[kMergeChunks];
 #pragma unroll
-    for (int i = 0; i < kPrepBlocks; ++i) {
-        const uint32_t blk = warp + i * kWarps;
-        if (blk < (K >> 8)) {
-            const uint32_t k0 = blk * 256 + 8 * lane, head = k0 / m.head_dim, d = k0 - head * m.head_dim;
-            float4 pl[kMergeChunks], ph[kMergeChunks];
-#pragma unroll
-            for (int c = 0; c < kMergeChunks; ++c) {
-                if ((uint32_t)c < m.n_chunks) {
-                    const float4* p = reinterpret_cast<const float4*>(
-                        m.partial + ((size_t)head * m.n_chunks + c) * m.head_dim + d);
-                    pl[c] = __ldg(p);
-                    ph[c] = __ldg(p + 1);
-                } else {
-                    pl[c] = ph[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-            float w[kMergeChunks];
-            const float inv = attn_merge_weights<kMergeChunks>(
-                m.partial + (size_t)m.n_heads * m.n_chunks * m.head_dim + (size_t)head * m.n_chunks * 2, m.sinks,
-                m.sink_offset + head, m.n_chunks, w);
-            float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-#pragma unroll
-            for (int c = 0; c < kMergeChunks; ++c) {
-                lo = make_float4(fmaf(w[c], pl[c].x, lo.x), fmaf(w[c], pl[c].y, lo.y), fmaf(w[c], pl[c].z, lo.z),
-                                 fmaf(w[c], pl[c].w, lo.w));
-                hi = make_float4(fmaf(w[c], ph[c].x, hi.x), fmaf(w[c], ph[c].y, hi.y), fmaf(w[c], ph[c].z, hi.z),
-                                 fmaf(w[c], ph[c].w, hi.w));
-            }
-            r.lo[i] = make_float4(lo.x * inv, lo.y * inv, lo.z * inv, lo.w * inv);
-            r.hi[i] = make_float4(hi.x * inv, hi.y * inv, hi.z * inv, hi.w * inv);
+    for (int c = 0; c < kMergeChunks; ++c) {
+        if ((uint32_t)c < m.n_chunks) {
+            const float4* p = reinterpret_cast<const float4*>(
+                m.partial + ((size_t)head * m.n_chunks + c) * m.head_dim + d);
+            pl[c] = __ldg(p);
+            ph[c] = __ldg(p + 1);
+        } else {
+            pl[c] = ph[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
+    float w[kMergeChunks];
+    const float inv = attn_merge_weights<kMergeChunks>(
+        m.partial + (size_t)m.n_heads * m.n_chunks * m.head_dim + (size_t)head * m.n_chunks * 2, m.sinks,
+        m.sink_offset + head, m.n_chunks, w);
+    float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+#pragma unroll
+    for (int c = 0; c < kMergeChunks; ++c) {
+        lo = make_float4(fmaf(w[c], pl[c].x, lo.x), fmaf(w[c], pl[c].y, lo.y), fmaf(w[c], pl[c].z, lo.z),
+                         fmaf(w[c], pl[c].w, lo.w));
+        hi = make_float4(fmaf(w[c], ph[c].x, hi.x), fmaf(w[c], ph[c].y, hi.y), fmaf(w[c], ph[c].z, hi.z),
+                         fmaf(w[c], ph[c].w, hi.w));
+    }
+    r.lo = make_float4(lo.x * inv, lo.y * inv, lo.z * inv, lo.w * inv);
+    r.hi = make_float4(hi.x * inv, hi.y * inv, hi.z * inv, hi.w * inv);
 }
 
 // Four values' low bytes as one word.
@@ -102,46 +89,41 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
     return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
 }
 
-__device__ __forceinline__ void prep_x(const Tab& s, const XRegs& r, uint32_t K, int warp, int lane, uint32_t kWarps) {
+__device__ __forceinline__ void prep_x(const Tab& s, const XRegs& r, uint32_t K, uint32_t blk, int lane) {
+    const float4 lo = r.lo, hi = r.hi;
+    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+    float mx = 0.f;
 #pragma unroll
-    for (int bi = 0; bi < kPrepBlocks; ++bi) {
-        const uint32_t blk = warp + bi * kWarps;
-        if (blk >= (K >> 8)) break;
-        const float4 lo = r.lo[bi], hi = r.hi[bi];
-        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-        float mx = 0.f;
+    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
+    // |x| < 2^(E-126)  ->  |x * 2^f| < 2^20 with f = 146 - E (E = biased exponent of the block maximum)
+    uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
+    E = E < 32u ? 32u : E;
+    const float scale = __uint_as_float((127u + 126u + kFracBits - E) << 23);
+    int X[8];
+    int sum = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-        // |x| < 2^(E-126)  ->  |x * 2^f| < 2^20 with f = 146 - E (E = biased exponent of the block maximum)
-        uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
-        E = E < 32u ? 32u : E;
-        const float scale = __uint_as_float((127u + 126u + kFracBits - E) << 23);
-        int X[8];
-        int sum = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            X[i] = __float2int_rn(v[i] * scale);
-            sum += X[i];
-        }
-        uint2 d0, d1, d2;
-        d0.x = pack4(X[0] >> 14, X[1] >> 14, X[2] >> 14, X[3] >> 14);
-        d0.y = pack4(X[4] >> 14, X[5] >> 14, X[6] >> 14, X[7] >> 14);
-        d1.x = pack4(X[0] >> 7, X[1] >> 7, X[2] >> 7, X[3] >> 7) & 0x7F7F7F7Fu;
-        d1.y = pack4(X[4] >> 7, X[5] >> 7, X[6] >> 7, X[7] >> 7) & 0x7F7F7F7Fu;
-        d2.x = pack4(X[0], X[1], X[2], X[3]) & 0x7F7F7F7Fu;
-        d2.y = pack4(X[4], X[5], X[6], X[7]) & 0x7F7F7F7Fu;
-        uint8_t* dst = s.dig + (size_t)blk * 256 + 8 * lane;
-        *reinterpret_cast<uint2*>(dst) = d0;
-        *reinterpret_cast<uint2*>(dst + K) = d1;
-        *reinterpret_cast<uint2*>(dst + 2 * (size_t)K) = d2;
-        // sub-block sums: four lanes per sub-block
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-        if ((lane & 3) == 0) s.sx[blk * 8 + (lane >> 2)] = (float)sum;
-        if (lane == 0) s.xs[blk] = __uint_as_float((E + 1u - kFracBits) << 23);  // 2^-f = 2^(E-146)
+    for (int i = 0; i < 8; ++i) {
+        X[i] = __float2int_rn(v[i] * scale);
+        sum += X[i];
     }
+    uint2 d0, d1, d2;
+    d0.x = pack4(X[0] >> 14, X[1] >> 14, X[2] >> 14, X[3] >> 14);
+    d0.y = pack4(X[4] >> 14, X[5] >> 14, X[6] >> 14, X[7] >> 14);
+    d1.x = pack4(X[0] >> 7, X[1] >> 7, X[2] >> 7, X[3] >> 7) & 0x7F7F7F7Fu;
+    d1.y = pack4(X[4] >> 7, X[5] >> 7, X[6] >> 7, X[7] >> 7) & 0x7F7F7F7Fu;
+    d2.x = pack4(X[0], X[1], X[2], X[3]) & 0x7F7F7F7Fu;
+    d2.y = pack4(X[4], X[5], X[6], X[7]) & 0x7F7F7F7Fu;
+    uint8_t* dst = s.dig + (size_t)blk * 256 + 8 * lane;
+    *reinterpret_cast<uint2*>(dst) = d0;
+    *reinterpret_cast<uint2*>(dst + K) = d1;
+    *reinterpret_cast<uint2*>(dst + 2 * (size_t)K) = d2;
+    // sub-block sums: four lanes per sub-block
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+    if ((lane & 3) == 0) s.sx[blk * 8 + (lane >> 2)] = (float)sum;
+    if (lane == 0) s.xs[blk] = __uint_as_float((E + 1u - kFracBits) << 23);  // 2^-f = 2^(E-146)
 }
 
 struct FmtQ4K {
@@ -149,7 +131,6 @@ struct FmtQ4K {
     using X = XRegs;
     static constexpr uint32_t kSlot = 16 * kRowSeg;
     static constexpr uint32_t kCols = 256;
-    static constexpr uint32_t kPrepBlocks = zc::kPrepBlocks;
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes + nblk * (768 + 32 + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
@@ -160,17 +141,20 @@ struct FmtQ4K {
         t.xs = t.sx + nblk * 8;
         return t;
     }
+    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return nblk; }
     template <int kSeg>
-    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, int warp, int lane, uint32_t n_warps) {
-        zc::load_x(r, a.x, a.K, warp, lane, n_warps);
+    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t blk, int lane) {
+        zc::load_x(r, a.x, blk, lane);
     }
     template <int kSeg>
-    static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const MergeArgs& m, int warp, int lane, uint32_t n_warps) {
-        load_x_merge(r, m, a.K, warp, lane, n_warps);
+    static __device__ __forceinline__ void load_x(X& r, const SliceArgs&, const MergeArgs& m, uint32_t blk, int lane) {
+        load_x_merge(r, m, blk, lane);
     }
-    static __device__ __forceinline__ void prep(const Tab& t, const X& r, const SliceArgs& a, int warp, int lane, int tid, uint32_t n_warps) {
-        for (uint32_t i = tid; i < kZeroBytes / 16; i += blockDim.x) reinterpret_cast<uint4*>(t.zeros)[i] = make_uint4(0u, 0u, 0u, 0u);
-        prep_x(t, r, a.K, warp, lane, n_warps);
+    static __device__ __forceinline__ void clear(const Tab& t, int tid) {
+        if (tid < kZeroBytes / 16) reinterpret_cast<uint4*>(t.zeros)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    static __device__ __forceinline__ void prep(const Tab& t, const X& r, const SliceArgs& a, uint32_t blk, int lane) {
+        prep_x(t, r, a.K, blk, lane);
     }
 
     // piece p = i * 32 + lane of a unit: row p / 9, 16-byte column p % 9
