@@ -171,7 +171,7 @@ struct FmtMX {
             const uint32_t pa = slot + g * kRowSlot + oA + 68 * t, pb = slot + (g + 8) * kRowSlot + oB + 68 * t;
             const uint32_t left = nb - u.lb * kUnitBlocks;
             const float xs = lds_f1(xs_s + u.kb * 8);
-#pragma unroll 1
+#pragma unroll 2
             for (uint32_t q = 0; q < 4; ++q) {
                 // 17 bytes at byte offset o (0..3) inside five aligned words: the scale is byte o, nibble word i is
                 // bytes o + 1 + 4 i .. of them: one funnel shift by 8 (o + 1) bits (a shift of 32 hands back the
@@ -185,7 +185,7 @@ struct FmtMX {
                     wb[i] = lds_u32((qb & ~3u) + 4 * i);
                 }
                 const uint32_t xq = xu + (u.kb * 4 + q) * xu_step;
-                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};  // two chains of MMAs
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint32_t ha[4], hb[4];
@@ -193,12 +193,12 @@ struct FmtMX {
                     e2m1x8_to_f16(__funnelshift_rc(wb[j], wb[j + 1], shb), hb);
                     const uint4 bx = lds_v4(xq + j * 128);
                     mma_f16(d, ha[0], hb[0], ha[1], hb[1], bx.x, bx.y);
-                    mma_f16(d, ha[2], hb[2], ha[3], hb[3], bx.z, bx.w);
+                    mma_f16(e, ha[2], hb[2], ha[3], hb[3], bx.z, bx.w);
                 }
                 if (q + 4 * t < left) {  // blocks past the row end hold stale bytes: their scale must not be used
                     const uint32_t ea = (wa[0] >> (sha - 8u)) & 0xFFu, eb = (wb[0] >> (shb - 8u)) & 0xFFu;
-                    acc.s[0] = fmaf(e8m0_to_f32(ea) * xs, d[0] + d[1], acc.s[0]);
-                    acc.s[1] = fmaf(e8m0_to_f32(eb) * xs, d[2] + d[3], acc.s[1]);
+                    acc.s[0] = fmaf(e8m0_to_f32(ea) * xs, (d[0] + e[0]) + (d[1] + e[1]), acc.s[0]);
+                    acc.s[1] = fmaf(e8m0_to_f32(eb) * xs, (d[2] + e[2]) + (d[3] + e[3]), acc.s[1]);
                 }
             }
         }

@@ -4,7 +4,7 @@
 // of rows); inside it, warp (wr, wk) works through the tiles wr, wr + n_wr, ... and owns the blocks (256 columns, MXFP4 512) wk, wk + n_wk,
 // ... of every one of them. So
 //   * x is converted once per CTA, a block or a few per warp, and every row of the CTA uses it;
-//   * a row's partial sums meet in shared memory: one barrier per kRound tiles, no hand-off between CTAs, results
+//   * a row's partial sums meet in shared memory: one barrier per few tiles, no hand-off between CTAs, results
 //     that do not depend on timing;
 //   * the warps of a CTA read adjacent blocks of the same rows at about the same time: whole DRAM pages.
 // (Units dealt to all warps of the GPU in one contiguous range each had every CTA convert all of x and a tile's sums travel
@@ -22,7 +22,6 @@
 namespace zc {
 namespace {
 
-constexpr int kRound = 4;  // tiles between two meetings of a CTA's warps
 
 struct SliceArgs {
     const uint8_t* A[2];
@@ -53,6 +52,7 @@ struct SliceArgs {
     // how the work is cut
     uint32_t h, tiles, tpe, tpc;   // rows per tile, tiles, tiles per expert slot, tiles per CTA
     uint32_t n_wk, n_wr, depth;
+    uint32_t round;                // tiles between two meetings of a CTA's warps, a multiple of n_wr
     uint32_t nblk, bpe;            // blocks of a (concatenated) row; of one matrix's row
 };
 
@@ -237,9 +237,9 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
     const uint32_t n_warps = blockDim.x >> 5;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t* ring = base + (size_t)warp * a.depth * F::kSlot;
-    float* spart = reinterpret_cast<float*>(base + (size_t)n_warps * a.depth * F::kSlot);  // [2][kRound][n_wk][NS * 16]
+    float* spart = reinterpret_cast<float*>(base + (size_t)n_warps * a.depth * F::kSlot);  // [2][round][n_wk][NS * 16]
     const uint32_t part_tile = a.n_wk * NS * 16;
-    const typename F::Tab tab = F::carve(reinterpret_cast<uint8_t*>(spart + 2 * kRound * part_tile), a.nblk);
+    const typename F::Tab tab = F::carve(reinterpret_cast<uint8_t*>(spart + 2 * a.round * part_tile), a.nblk);
     const uint32_t wk = (uint32_t)warp % a.n_wk, wr = (uint32_t)warp / a.n_wk;
     const uint32_t ct0 = blockIdx.x * a.tpc, nt = min(a.tpc, a.tiles - ct0);
 
@@ -303,7 +303,7 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
             kb += a.n_wk;
             meet = false;
             if (kb >= a.nblk) {  // the warp's share of a tile's stream is complete
-                float* part = spart + (((tl / kRound) & 1) * kRound + tl % kRound) * part_tile + wk * (NS * 16) + strm * 16;
+                float* part = spart + (((tl / a.round) & 1) * a.round + tl % a.round) * part_tile + wk * (NS * 16) + strm * 16;
                 float v0, v1;
                 ln.finish(acc, v0, v1);  // rows g and g + 8, this lane's share
                 acc.clear();
@@ -319,19 +319,19 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
                 if (++strm == NS) {
                     strm = 0;
                     tl += a.n_wr;
-                    meet = tl >= r0 + kRound || tl >= nt;
+                    meet = tl >= r0 + a.round || tl >= nt;
                 }
             }
         }
         if (meet) {
             // ---- the warps meet: four lanes per row add the warps' shares, in a fixed order ----
-            const uint32_t buf = (r0 / kRound) & 1, n_red = min((uint32_t)kRound, nt - r0) * 64;
+            const uint32_t buf = (r0 / a.round) & 1, n_red = min(a.round, nt - r0) * 64;
             OutRow o{};
             if ((uint32_t)tid < n_red) o = out_row<EPI, kSeg>(a, ct0 + r0 + (tid >> 6), (tid >> 2) & 15u, (tid & 3u) == 0);
             __syncthreads();
             for (uint32_t i = tid; i < n_red; i += blockDim.x) {
                 if (i != (uint32_t)tid) o = out_row<EPI, kSeg>(a, ct0 + r0 + (i >> 6), (i >> 2) & 15u, (i & 3u) == 0);
-                const float* p = spart + (buf * kRound + (i >> 6)) * part_tile + ((i >> 2) & 15u);
+                const float* p = spart + (buf * a.round + (i >> 6)) * part_tile + ((i >> 2) & 15u);
                 float v[NS];
 #pragma unroll
                 for (int s = 0; s < NS; ++s) {
@@ -344,7 +344,7 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
                 }
                 write_out<NS, EPI>(a, o, v);
             }
-            r0 += kRound;
+            r0 += a.round;
             if (r0 >= nt) break;
         }
     }
@@ -368,17 +368,17 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     a.bpe = (a.K + F::kCols - 1) / F::kCols;
     a.nblk = a.bpe * (kSeg == 3 ? a.nseg : 1u);
     const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 148u;
-    // Few blocks: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen.
+    // Up to 16 blocks: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen warps.
     // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
-    const uint32_t most = a.nblk <= 8 ? 8u : 16u;
+    const uint32_t most = a.nblk <= 16 ? 8u : 16u;
     const uint32_t per = (a.nblk + most - 1) / most;
     a.n_wk = (a.nblk + per - 1) / per;
     a.n_wr = most / a.n_wk;
-    if (a.n_wr > (uint32_t)kRound) a.n_wr = kRound;
-    if (a.n_wr == 3) a.n_wr = 2;  // kRound tiles are dealt evenly
+    if (a.n_wr > 4) a.n_wr = 4;
+    a.round = a.n_wr == 3 ? 6 : 4;
     warps = a.n_wk * a.n_wr;
     const uint32_t per_sm = most == 8 ? 2u : 1u, room = most == 8 ? kSliceSmem2 : kSliceSmem1;
-    const uint32_t fixed = 128u + 2u * kRound * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
+    const uint32_t fixed = 128u + 2u * a.round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
     if (fixed + warps * 2u * F::kSlot > room) return false;
     a.depth = (room - fixed) / (warps * F::kSlot);
     a.depth = a.depth > 4 ? 4 : a.depth;
