@@ -55,7 +55,7 @@ struct FmtMX {
         t.xs = reinterpret_cast<float*>(t.xf + (size_t)nblk * 128);
         return t;
     }
-    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return 2 * nblk; }  // chunks of 256 elements
+    static __device__ __forceinline__ uint32_t prep_count(const SliceArgs& a) { return 2 * a.nblk; }  // chunks of 256 elements
     template <int kSeg>
     static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t chunk, int lane) {
         const uint32_t b = lane >> 2, j = lane & 3;

@@ -204,7 +204,7 @@ struct FmtQ6K {
         t.xs = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(t.nsx) + (size_t)nblk * kNsxBytes);
         return t;
     }
-    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return nblk; }
+    static __device__ __forceinline__ uint32_t prep_count(const SliceArgs& a) { return a.nblk; }
     template <int kSeg>
     static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t blk, int lane) {
         load_x6(r, a.x, blk, a.bpe, a.x_slot_stride, kSeg == 3 ? a.routing + a.nseg : nullptr, lane);

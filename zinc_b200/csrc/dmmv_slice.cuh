@@ -1,7 +1,7 @@
 // Skeleton of the streaming matvec kernels: rows are dealt to CTAs, K to the warps of a CTA.
 //
 // Every CTA owns a contiguous run of row tiles (at most 16 rows each, the height chosen so that the SMs get equal numbers
-// of rows); inside it, warp (wr, wk) works through the tiles wr, wr + n_wr, ... and owns the blocks (256 columns, MXFP4 512) wk, wk + n_wk,
+// of rows); inside it, warp (wr, wk) works through the tiles wr, wr + n_wr, ... and owns the blocks (512 columns, Q6_K 256) wk, wk + n_wk,
 // ... of every one of them. So
 //   * x is converted once per CTA, a block or a few per warp, and every row of the CTA uses it;
 //   * a row's partial sums meet in shared memory: one barrier per few tiles, no hand-off between CTAs, results
@@ -254,7 +254,7 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
     uint32_t p_tl = wr, p_strm = 0, p_kb = wk;  // the unit to request next: tile, stream, block
     uint32_t tl = wr, strm = 0, kb = wk;        // the unit to work off next
     uint32_t r0 = 0;                            // first tile of the round the warps meet for next
-    const uint32_t n_prep = F::prep_count(a.nblk), x_at = a.late ? 0u : a.depth - 1;
+    const uint32_t n_prep = F::prep_count(a), x_at = a.late ? 0u : a.depth - 1;
     typename F::X x;
     typename F::Acc acc;
     acc.clear();
@@ -368,9 +368,9 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     a.bpe = (a.K + F::kCols - 1) / F::kCols;
     a.nblk = a.bpe * (kSeg == 3 ? a.nseg : 1u);
     const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 148u;
-    // Up to 16 blocks: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen warps.
+    // Up to K = 4096: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen warps.
     // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
-    const uint32_t most = a.nblk <= 16 ? 8u : 16u;
+    const uint32_t most = a.nblk * F::kCols <= 4096 ? 8u : 16u;
     const uint32_t per = (a.nblk + most - 1) / most;
     a.n_wk = (a.nblk + per - 1) / per;
     a.n_wr = most / a.n_wk;

@@ -27,10 +27,11 @@ namespace zc {
 
 namespace {
 
-constexpr int kRowSeg = 192;               // 144 + pad: rows land 64 B apart mod 128 B -> conflict-free 128-bit reads
+constexpr uint32_t kCB = 2;                // super-blocks per unit (one at a time: 10 % more instructions per block)
+constexpr int kRowSeg = kCB * 144 + 32;    // 320: rows land 64 B apart mod 128 B -> conflict-free 128-bit reads
 constexpr int kZeroBytes = 256;            // zeros: B operand of the lanes whose column is dead for their k slots
 constexpr int kFracBits = 20;              // |X| <= 2^20
-constexpr int kPieces = 9;                 // 16-byte pieces of a block
+constexpr int kPieces = kCB * 9;           // 16-byte pieces of a row of a unit
 constexpr int kPiecesPerLane = (16 * kPieces + 31) / 32;
 
 struct Tab {
@@ -130,18 +131,18 @@ struct FmtQ4K {
     using Tab = zc::Tab;
     using X = XRegs;
     static constexpr uint32_t kSlot = 16 * kRowSeg;
-    static constexpr uint32_t kCols = 256;
-    static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes + nblk * (768 + 32 + 4) + 128; }
+    static constexpr uint32_t kCols = kCB * 256;
+    static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes + nblk * kCB * (768 + 32 + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
         p += (128u - (smem_u32(p) & 127u)) & 127u;
         t.zeros = p;
         t.dig = p + kZeroBytes;   // K is a multiple of 256: every plane starts 128-byte aligned
-        t.sx = reinterpret_cast<float*>(t.dig + (size_t)nblk * 768);
-        t.xs = t.sx + nblk * 8;
+        t.sx = reinterpret_cast<float*>(t.dig + (size_t)nblk * kCB * 768);
+        t.xs = t.sx + nblk * kCB * 8;
         return t;
     }
-    static __device__ __forceinline__ uint32_t prep_count(uint32_t nblk) { return nblk; }
+    static __device__ __forceinline__ uint32_t prep_count(const SliceArgs& a) { return a.K >> 8; }
     template <int kSeg>
     static __device__ __forceinline__ void load_x(X& r, const SliceArgs& a, const NoExtra&, uint32_t blk, int lane) {
         zc::load_x(r, a.x, blk, lane);
@@ -157,25 +158,33 @@ struct FmtQ4K {
         prep_x(t, r, a.K, blk, lane);
     }
 
-    // piece p = i * 32 + lane of a unit: row p / 9, 16-byte column p % 9
+    // piece p = i * 32 + lane of a unit: row p / 18, 16-byte column p % 18
     struct Copier {
-        uint32_t src[kPiecesPerLane], dst[kPiecesPerLane], row[kPiecesPerLane];
+        uint32_t src[kPiecesPerLane], dst[kPiecesPerLane];  // dst: row << 16 | offset in the slot
         __device__ __forceinline__ void init(const SliceArgs& a, int lane) {
 #pragma unroll
             for (int i = 0; i < kPiecesPerLane; ++i) {
                 const uint32_t p = i * 32 + lane, r = p / kPieces, c = p - r * kPieces;
-                row[i] = r;
-                src[i] = r * a.bpe * 144u + c * 16;
-                dst[i] = r * kRowSeg + c * 16;
+                src[i] = r * (a.K >> 8) * 144u + c * 16;
+                dst[i] = r << 16 | (r * kRowSeg + c * 16);
             }
         }
         __device__ __forceinline__ void copy(const SliceArgs& a, const Unit& u, uint8_t* slot, int) const {
-            const uint8_t* p = u.mat + (uint64_t)u.row0 * (a.bpe * 144u) + u.lb * 144u;
-            const uint32_t d = smem_u32(slot);
+            const uint32_t bpr = a.K >> 8, d = smem_u32(slot);
+            const uint8_t* p = u.mat + (uint64_t)u.row0 * (bpr * 144u) + u.lb * (kCB * 144u);
+            if (u.rows == 16 && (u.lb + 1) * kCB <= bpr) {
 #pragma unroll
-            for (int i = 0; i < kPiecesPerLane; ++i)
-                if (row[i] < u.rows)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + dst[i]), "l"(p + src[i]) : "memory");
+                for (int i = 0; i < kPiecesPerLane; ++i)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + (dst[i] & 0xFFFFu)), "l"(p + src[i]) : "memory");
+            } else {  // a lower tile, or the last block of an odd number
+                const uint32_t bytes = min(kCB, bpr - u.lb * kCB) * 144u;
+#pragma unroll
+                for (int i = 0; i < kPiecesPerLane; ++i) {
+                    const uint32_t r = dst[i] >> 16, off = dst[i] & 0xFFFFu;
+                    if (r < u.rows && off - r * kRowSeg < bytes)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + off), "l"(p + src[i]) : "memory");
+                }
+            }
         }
     };
 
@@ -204,38 +213,42 @@ struct FmtQ4K {
             // digit t's sum carries 2^(14 - 7t) and the 1/16 of the in-place high nibbles; lane t = 3 holds zeros
             dscale = __uint_as_float((127u + 10u - 7u * t) << 23);
         }
-        __device__ __forceinline__ void dot(const SliceArgs&, const Unit& u, uint32_t slot, Acc& acc) const {
+        __device__ __forceinline__ void dot(const SliceArgs& a, const Unit& u, uint32_t slot, Acc& acc) const {
             constexpr uint32_t kLo = 0x0F0F0F0Fu, kHi = 0xF0F0F0F0u;
-            const uint32_t rA = slot + g * kRowSeg, rB = slot + (g + 8) * kRowSeg;
-            const uint4 hA = lds_v4(rA), hB = lds_v4(rB);
-            const uint32_t xb = xb_base + u.kb * xb_step;
-            // 6-bit scales of sub-blocks 0..3 and 4..7, one per byte (getScaleMinK4, src/compute/forward.zig:229-238)
-            const uint32_t scA[2] = {hA.y & 0x3F3F3F3Fu, (hA.w & 0x0F0F0F0Fu) | ((hA.y >> 2) & 0x30303030u)};
-            const uint32_t scB[2] = {hB.y & 0x3F3F3F3Fu, (hB.w & 0x0F0F0F0Fu) | ((hB.y >> 2) & 0x30303030u)};
-            int IloA = 0, IhiA = 0, IloB = 0, IhiB = 0;
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const uint4 qa = lds_v4(rA + 16 + 64 * p + 16 * t), qb = lds_v4(rB + 16 + 64 * p + 16 * t);
-                const uint4 bl = lds_v4(xb + 128 * p), bh = lds_v4(xb + 128 * p + 32);
-                int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-                mma_u8s8(lo, qa.x & kLo, qb.x & kLo, qa.y & kLo, qb.y & kLo, bl.x, bl.y);
-                mma_u8s8(lo, qa.z & kLo, qb.z & kLo, qa.w & kLo, qb.w & kLo, bl.z, bl.w);
-                mma_u8s8(hi, qa.x & kHi, qb.x & kHi, qa.y & kHi, qb.y & kHi, bh.x, bh.y);
-                mma_u8s8(hi, qa.z & kHi, qb.z & kHi, qa.w & kHi, qb.w & kHi, bh.z, bh.w);
-                // D columns 2t, 2t+1 = digit t of sub-blocks 4p (+1 for the high nibbles) and 4p + 2 (+1)
-                const uint32_t sa = scA[p], sb2 = scB[p];
-                IloA += lo[0] * (int)(sa & 0xFFu) + lo[1] * (int)((sa >> 16) & 0xFFu);
-                IhiA += hi[0] * (int)((sa >> 8) & 0xFFu) + hi[1] * (int)(sa >> 24);
-                IloB += lo[2] * (int)(sb2 & 0xFFu) + lo[3] * (int)((sb2 >> 16) & 0xFFu);
-                IhiB += hi[2] * (int)((sb2 >> 8) & 0xFFu) + hi[3] * (int)(sb2 >> 24);
+            for (uint32_t bi = 0; bi < kCB; ++bi) {
+                const uint32_t blk = u.kb * kCB + bi;
+                if (bi > 0 && blk >= (a.K >> 8)) break;
+                const uint32_t rA = slot + bi * 144 + g * kRowSeg, rB = slot + bi * 144 + (g + 8) * kRowSeg;
+                const uint4 hA = lds_v4(rA), hB = lds_v4(rB);
+                const uint32_t xb = xb_base + blk * xb_step;
+                // 6-bit scales of sub-blocks 0..3 and 4..7, one per byte (getScaleMinK4, src/compute/forward.zig:229-238)
+                const uint32_t scA[2] = {hA.y & 0x3F3F3F3Fu, (hA.w & 0x0F0F0F0Fu) | ((hA.y >> 2) & 0x30303030u)};
+                const uint32_t scB[2] = {hB.y & 0x3F3F3F3Fu, (hB.w & 0x0F0F0F0Fu) | ((hB.y >> 2) & 0x30303030u)};
+                int IloA = 0, IhiA = 0, IloB = 0, IhiB = 0;
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const uint4 qa = lds_v4(rA + 16 + 64 * p + 16 * t), qb = lds_v4(rB + 16 + 64 * p + 16 * t);
+                    const uint4 bl = lds_v4(xb + 128 * p), bh = lds_v4(xb + 128 * p + 32);
+                    int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+                    mma_u8s8(lo, qa.x & kLo, qb.x & kLo, qa.y & kLo, qb.y & kLo, bl.x, bl.y);
+                    mma_u8s8(lo, qa.z & kLo, qb.z & kLo, qa.w & kLo, qb.w & kLo, bl.z, bl.w);
+                    mma_u8s8(hi, qa.x & kHi, qb.x & kHi, qa.y & kHi, qb.y & kHi, bh.x, bh.y);
+                    mma_u8s8(hi, qa.z & kHi, qb.z & kHi, qa.w & kHi, qb.w & kHi, bh.z, bh.w);
+                    // D columns 2t, 2t+1 = digit t of sub-blocks 4p (+1 for the high nibbles) and 4p + 2 (+1)
+                    const uint32_t sa = scA[p], sb2 = scB[p];
+                    IloA += lo[0] * (int)(sa & 0xFFu) + lo[1] * (int)((sa >> 16) & 0xFFu);
+                    IhiA += hi[0] * (int)((sa >> 8) & 0xFFu) + hi[1] * (int)(sa >> 24);
+                    IloB += lo[2] * (int)(sb2 & 0xFFu) + lo[3] * (int)((sb2 >> 16) & 0xFFu);
+                    IhiB += hi[2] * (int)((sb2 >> 8) & 0xFFu) + hi[3] * (int)(sb2 >> 24);
             }
             // the high nibbles were multiplied as 16 q: sum = (16 * lo + hi) / 16, the 1/16 sits in dscale
             const float PA = (float)(IloA * 16 + IhiA), PB = (float)(IloB * 16 + IhiB);
             // mins of sub-blocks 2t, 2t+1
             const uint32_t mnA = __byte_perm(hA.z & 0x3F3F3F3Fu, ((hA.w >> 4) & 0x0F0F0F0Fu) | ((hA.z >> 2) & 0x30303030u), msel);
             const uint32_t mnB = __byte_perm(hB.z & 0x3F3F3F3Fu, ((hB.w >> 4) & 0x0F0F0F0Fu) | ((hB.z >> 2) & 0x30303030u), msel);
-            const float xs = lds_f1(xs_s + u.kb * 4);
-            const float2 sxv = lds_f2(sx_s + u.kb * 32);
+            const float xs = lds_f1(xs_s + blk * 4);
+            const float2 sxv = lds_f2(sx_s + blk * 32);
             const float dA = h2f(hA.x) * xs, dmA = h2f(hA.x >> 16) * xs;
             const float dB = h2f(hB.x) * xs, dmB = h2f(hB.x >> 16) * xs;
             const float mA = (float)(mnA & 0xFFu) * sxv.x + (float)((mnA >> 8) & 0xFFu) * sxv.y;
@@ -244,6 +257,7 @@ struct FmtQ4K {
             acc.M[1] = fmaf(dB, PB, acc.M[1]);
             acc.m[0] = fmaf(dmA, mA, acc.m[0]);
             acc.m[1] = fmaf(dmB, mB, acc.m[1]);
+            }
         }
         __device__ __forceinline__ void finish(const Acc& acc, float& v0, float& v1) const {
             v0 = fmaf(acc.M[0], dscale, -acc.m[0]);
