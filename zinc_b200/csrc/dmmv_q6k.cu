@@ -193,6 +193,7 @@ struct FmtQ6K {
     using Tab = Tab6;
     using X = XRegs6;
     static constexpr uint32_t kSlot = 16 * kRow6;
+    static constexpr uint32_t kMost = 16;
     static constexpr uint32_t kCols = 256;
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes6 + nblk * (kBBytes + kNsxBytes + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {

@@ -352,11 +352,11 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
 
 struct NoExtra {};
 template <typename F, int NS, int EPI, int kSeg, int kWarps>
-__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dmmv_slice_kernel(const SliceArgs a) {
+__global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_slice_kernel(const SliceArgs a) {
     slice_body<F, NS, EPI, kSeg>(a, NoExtra());
 }
 template <typename F, int kWarps>
-__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) dmmv_slice_merge_kernel(const SliceArgs a, const MergeArgs m) {
+__global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_slice_merge_kernel(const SliceArgs a, const MergeArgs m) {
     slice_body<F, 1, EPI_PLAIN, 0>(a, m);
 }
 
@@ -368,16 +368,19 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     a.bpe = (a.K + F::kCols - 1) / F::kCols;
     a.nblk = a.bpe * (kSeg == 3 ? a.nseg : 1u);
     const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 148u;
-    // Up to K = 4096: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else sixteen warps.
+    // Up to K = 4096: eight warps and two CTAs per SM, so that the next kernel's CTAs find room early; else one CTA with as
+    // many warps as the registers allow. A format whose units are bound by latency (kMost > 16) always takes the latter
+    // (MXFP4 gate + up 20.1 -> 17.9 us with 18 warps instead of 12); along slots K is long enough for twelve to sixteen.
     // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
-    const uint32_t most = a.nblk * F::kCols <= 4096 ? 8u : 16u;
+    const bool pair = F::kMost <= 16 && a.nblk * F::kCols <= 4096;
+    const uint32_t most = pair ? 8u : kSeg == 3 ? 16u : F::kMost;
     const uint32_t per = (a.nblk + most - 1) / most;
     a.n_wk = (a.nblk + per - 1) / per;
     a.n_wr = most / a.n_wk;
     if (a.n_wr > 4) a.n_wr = 4;
     a.round = a.n_wr == 3 ? 6 : 4;
     warps = a.n_wk * a.n_wr;
-    const uint32_t per_sm = most == 8 ? 2u : 1u, room = most == 8 ? kSliceSmem2 : kSliceSmem1;
+    const uint32_t per_sm = pair ? 2u : 1u, room = pair ? kSliceSmem2 : kSliceSmem1;
     const uint32_t fixed = 128u + 2u * a.round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
     if (fixed + warps * 2u * F::kSlot > room) return false;
     a.depth = (room - fixed) / (warps * F::kSlot);
@@ -420,7 +423,7 @@ cudaError_t slice_launch(SliceArgs a, int sm_count, cudaStream_t s) {
         if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, attr8); e != cudaSuccess) return e;
         return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
     }
-    auto kern = dmmv_slice_kernel<F, NS, EPI, kSeg, 16>;
+    auto kern = dmmv_slice_kernel<F, NS, EPI, kSeg, kSeg == 3 ? 16 : (int)F::kMost>;
     if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, attr16); e != cudaSuccess) return e;
     return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
 }

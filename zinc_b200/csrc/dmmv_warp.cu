@@ -131,6 +131,7 @@ struct FmtQ4K {
     using Tab = zc::Tab;
     using X = XRegs;
     static constexpr uint32_t kSlot = 16 * kRowSeg;
+    static constexpr uint32_t kMost = 16;
     static constexpr uint32_t kCols = kCB * 256;
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes + nblk * kCB * (768 + 32 + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
