@@ -966,7 +966,7 @@ cudaError_t launch_tile(const uint8_t* A, const void* B, float* D, uint32_t M, u
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 4) --splits;
     if (splits > 1) {
-        if (cudaError_t e = launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d); e != cudaSuccess) return e;
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
         grid.z = splits;
     }
     return launch_chained(kern, grid, dim3(kThreads), Tile<TYPE, BN>::kSmemBytes, s, map, wmap, g);
@@ -997,7 +997,7 @@ cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, 
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 2) --splits;
     if (splits > 1) {
-        if (cudaError_t e = launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d); e != cudaSuccess) return e;
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
         grid.z = splits;
     }
     return launch_chained(gemm_tc_small_kernel, grid, dim3(kSmThreads), kSmSmemBytes, s, map, g);
@@ -1080,8 +1080,8 @@ cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, u
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    cudaError_t e = p.zeroed ? launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d)
-                             : launch_chained(zero_kernel, dim3(1), dim3(256), 0, s, reinterpret_cast<float*>(flags), p.n_tiles * 2, 0);
+    cudaError_t e = p.zeroed ? launch_zero(D, M, N, stride_d, s)
+                             : launch_zero(reinterpret_cast<float*>(flags), p.n_tiles * 2, 1, 0, s);
     if (e != cudaSuccess) return e;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, map, wmap, p);
@@ -1107,6 +1107,10 @@ cudaError_t launch_typed(const uint8_t* A, const void* B, float* D, uint32_t M, 
 }
 
 }  // namespace
+
+cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s) {
+    return launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d);
+}
 
 cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N,
                           uint32_t K, uint32_t stride_b, uint32_t stride_d, bool act_bf16, uint32_t* status,

@@ -195,6 +195,8 @@ bool mul_mm_mx_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t
 cudaError_t launch_mul_mm_mx(const uint8_t* A, uint64_t a_bytes, const void* B, float* D, uint32_t M, uint32_t N,
                              uint32_t K, uint32_t stride_b, uint32_t stride_d, void* workspace, uint32_t* status,
                              int sm_count, cudaStream_t s, uint64_t* launches);
+// Zeroes an N x M output (row stride stride_d) that the GEMM launched behind it adds into.
+cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s);
 bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K,
                               uint32_t stride_b);
 cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_bytes, const void* B, float* D,

@@ -23,6 +23,8 @@
 // Replaces recordMoeBatchedDispatch's per-pair kernel for prefill batches
 // (src/compute/dmmv.zig:746-792; src/shaders/dmmv_q4k_moe_batched.comp:70-164) with the grouping the
 // reference's Metal path does (src/shaders/metal/moe_route_pack.metal:13-36).
+#include <math.h>
+
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -42,6 +44,7 @@ template <int TYPE, int BN>
 struct MoeTile {
     static constexpr uint32_t kRawBytes = kBM * Raw<TYPE>::kBox;
     static constexpr uint32_t kXBytes = BN * kBK * 2;
+    static constexpr uint32_t kAccCols = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;  // tensor memory: powers of two
     // (two stages per dequant set with 32-token tiles took the raw ring its depth: 360 -> 375 us on 256 experts, T = 512)
     static constexpr int kStages = kAStages;
     static constexpr uint32_t kRawOffset = kStages * kABytes;
@@ -74,20 +77,41 @@ struct MoeGemmArgs {
     const uint32_t* list;         // pair ids (token * n_used + slot) grouped by expert
     uint32_t M, K, n_used, y_token_stride, row_tiles;
     uint32_t* status;
-    uint32_t dense_n;             // > 0: plain GEMM over dense_n tokens (one "expert", identity pair list, no tables)
+    uint32_t dense_n;             // > 0: plain GEMM over dense_n tokens (one "expert", identity pair list, no tables) ..
+    uint32_t dense_tile;          // .. in tiles of this many
+    uint32_t splits, slice;       // work items along K per tile, 256-column blocks in each; > 1: they add into a zeroed Y
 };
 
-// Tile t: from the table, or (dense) tokens [t * BN, min(dense_n, (t + 1) * BN)) of the only matrix.
-template <int BN>
+// Work item w: every slice of K of a row tile, then the next row tile, then the next tile of pairs.
+struct Item {
+    uint32_t tile, m0;
+    int b0, b1;  // blocks of 256 columns
+};
+__device__ __forceinline__ Item item_of(const MoeGemmArgs& g, uint32_t w, int nblk) {
+    Item it;
+    uint32_t t = w;
+    it.b0 = 0;
+    it.b1 = nblk;
+    if (g.splits > 1) {
+        t = w / g.splits;
+        it.b0 = (int)((w - t * g.splits) * g.slice);
+        it.b1 = min(nblk, it.b0 + (int)g.slice);
+    }
+    it.tile = t / g.row_tiles;
+    it.m0 = (t - it.tile * g.row_tiles) * kBM;
+    return it;
+}
+
+// Tile t: from the table, or (dense) the t-th run of tokens of the only matrix.
 __device__ __forceinline__ uint4 moe_tile(const MoeGemmArgs& g, uint32_t t) {
-    if (g.dense_n) return make_uint4(0u, t * BN, min((uint32_t)BN, g.dense_n - t * BN), 0u);
+    if (g.dense_n) return make_uint4(0u, t * g.dense_tile, min(g.dense_tile, g.dense_n - t * g.dense_tile), 0u);
     return __ldg(&g.tiles[t]);
 }
 
 // Position of the dequant warps in the flat sequence of (work item, 256-column block).
 struct BlockCursor {
     uint32_t w;             // work item
-    int b;                  // block of the item
+    int b, b1;              // block of the item; one past its last
     const uint8_t* expert;  // first byte of the item's expert
     uint32_t m0;            // first row of the item's row tile
     uint64_t row_off;       // byte offset of this thread's row inside the expert
@@ -109,7 +133,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     uint8_t* smem_x = smem + T::kXOffset;
     MoeBars* bars = reinterpret_cast<MoeBars*>(smem + T::kBarOffset);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n_items = (g.dense_n ? (g.dense_n + BN - 1) / BN : g.header[0]) * g.row_tiles;
+    const uint32_t n_items = (g.dense_n ? (g.dense_n + g.dense_tile - 1) / g.dense_tile : g.header[0]) * g.row_tiles * g.splits;
     const int n_stages = g.K >> 6;           // 64 columns each
     const int nblk = (n_stages + 3) >> 2;    // 256-column blocks, the last one possibly short (MXFP4)
     constexpr uint32_t kBlock = Raw<TYPE>::kBlock, kBox = Raw<TYPE>::kBox;
@@ -135,7 +159,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&bars->tmem_base)),
-                     "r"((uint32_t)(2 * BN))
+                     "r"((uint32_t)(2 * T::kAccCols))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -146,15 +170,19 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
 
     if (warp == 0) {
         {  // ---- MMA issuer ----
-            constexpr uint32_t idesc = instr_desc<BN>();
             uint32_t gs = 0, i = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
                 const uint32_t ab = i & 1;
+                // as many columns as the tile has pairs (N in steps of 16)
+                const Item it = item_of(g, w, nblk);
+                const int s0 = 4 * it.b0, s1 = min(n_stages, 4 * it.b1);
+                const uint32_t cols = (moe_tile(g, it.tile).z + 15u) & ~15u;
+                const uint32_t idesc = instr_desc<16>() + ((cols - 16u) >> 3 << 17);
                 ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.status, 121);
                 if (!ok) break;
                 tc_fence_after();
-                for (int s = 0; s < n_stages; ++s, ++gs) {
+                for (int s = s0; s < s1; ++s, ++gs) {
                     const int st = gs % T::kStages;
                     const uint32_t ph = (gs / T::kStages) & 1;
                     ok = warp_poll(smem_u32(&bars->full_a[st]), ph, bars, g.status, 122);
@@ -165,7 +193,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < kBK / 16; ++k)
-                            umma_bf16(tmem + ab * BN, da + 2 * k, dx + 2 * k, idesc, (s | k) ? 1u : 0u);
+                            umma_bf16(tmem + ab * T::kAccCols, da + 2 * k, dx + 2 * k, idesc, s > s0 || k ? 1u : 0u);
                         umma_commit(&bars->empty_a[st]);
                     }
                 }
@@ -177,8 +205,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             uint32_t gs = 0;
             bool ok = true;
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-                const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
-                for (int s = 0; s < n_stages; ++s, ++gs) {
+                const Item it = item_of(g, w, nblk);
+                const uint4 tile = moe_tile(g, it.tile);
+                for (int s = 4 * it.b0; s < min(n_stages, 4 * it.b1); ++s, ++gs) {
                     const int st = gs % T::kStages;
                     ok = poll_or_fail(&bars->empty_a[st], ((gs / T::kStages) & 1) ^ 1, bars, g.status, 124);
                     if (!ok) break;
@@ -194,10 +223,12 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
         const int row = p & 127, j = p >> 7;
         auto locate = [&](uint32_t w, BlockCursor& c) {
             c.w = w;
-            c.b = 0;
             if (w < n_items) {
-                const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
-                c.m0 = (w % g.row_tiles) * kBM;
+                const Item it = item_of(g, w, nblk);
+                const uint4 tile = moe_tile(g, it.tile);
+                c.m0 = it.m0;
+                c.b = it.b0;
+                c.b1 = it.b1;
                 const uint32_t grow = min(c.m0 + (uint32_t)row, g.M - 1);  // rows past M are computed and dropped
                 c.expert = g.A + (uint64_t)tile.x * g.expert_stride;
                 c.row_off = (uint64_t)grow * row_bytes;
@@ -205,21 +236,40 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
         };
         // The 16-byte pieces of the aligned supersets of all rows' blocks, dealt to the 512 threads row by row: a warp's
         // copy instruction covers three rows' runs of bytes, a handful of cache lines, where one row per lane met 32.
-        auto fetch = [&](const BlockCursor& c, uint32_t slot_idx) {
-            uint8_t* slot = smem_w + slot_idx * T::kRawBytes;
+        constexpr int kFetches = (kBM * kPieces + 511) / 512;
+        uint32_t f_row[kFetches], f_dst[kFetches];  // byte offset of the thread's pieces' rows in a tile; place in the slot
 #pragma unroll
-            for (int i = 0; i < (kBM * kPieces + 511) / 512; ++i) {
-                const uint32_t idx = (uint32_t)p + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
-                if ((kBM * kPieces) % 512 == 0 || r < (uint32_t)kBM) {
+        for (int i = 0; i < kFetches; ++i) {
+            const uint32_t idx = (uint32_t)p + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
+            f_row[i] = r * (uint32_t)row_bytes;
+            f_dst[i] = (kBM * kPieces) % 512 == 0 || r < (uint32_t)kBM ? (r << 20) | (piece << 16) | (r * kBox + piece * 16) : 0xFFFFFFFFu;
+        }
+        auto fetch = [&](const BlockCursor& c, uint32_t slot_idx) {
+            const uint32_t slot = smem_u32(smem_w) + slot_idx * T::kRawBytes;
+            const uint8_t* first = c.expert + (uint64_t)c.m0 * row_bytes + (uint32_t)c.b * kBlock;  // the tile's first row
+            const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(first) & 15u;
+            if (c.m0 + kBM <= g.M && first + (uint64_t)(kBM - 1) * row_bytes + kPieces * 16 <= g.a_end) {
+#pragma unroll
+                for (int i = 0; i < kFetches; ++i) {
+                    if (f_dst[i] != 0xFFFFFFFFu) {
+                        const uint8_t* s = first - low + (((low + f_row[i]) & ~15u) + ((f_dst[i] >> 12) & 0xF0u));
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (f_dst[i] & 0xFFFFu)), "l"(s) : "memory");
+                    }
+                }
+            } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
+#pragma unroll 1
+                for (int i = 0; i < kFetches; ++i) {
+                    if (f_dst[i] == 0xFFFFFFFFu) continue;
+                    const uint32_t r = f_dst[i] >> 20, piece = (f_dst[i] >> 16) & 15u;
                     const uint64_t o = (uint64_t)min(c.m0 + r, g.M - 1) * row_bytes + (uint64_t)c.b * kBlock;
                     const uint8_t* s = c.expert + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t n = s + 16 <= g.a_end ? 16u : (s < g.a_end ? (uint32_t)(g.a_end - s) : 0u);
-                    cp_async16_zfill(slot + r * kBox + piece * 16, n ? s : g.A, n);
+                    cp_async16_zfill(smem_w + slot_idx * T::kRawBytes + (f_dst[i] & 0xFFFFu), n ? s : g.A, n);
                 }
             }
         };
         auto advance = [&](BlockCursor& c) {
-            if (c.b + 1 < nblk)
+            if (c.b + 1 < c.b1)
                 ++c.b;
             else
                 locate(c.w + gridDim.x, c);
@@ -296,15 +346,16 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
         uint32_t i = 0;
         for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ++i) {
             const uint32_t ab = i & 1;
-            const uint4 tile = moe_tile<BN>(g, w / g.row_tiles);
-            const uint32_t m = (w % g.row_tiles) * kBM + q * 32 + lane;
+            const Item it = item_of(g, w, nblk);
+            const uint4 tile = moe_tile(g, it.tile);
+            const uint32_t m = it.m0 + q * 32 + lane;
             if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 126)) break;
             __syncwarp();
             tc_fence_after();
 #pragma unroll 1
             for (uint32_t c = 0; c * 32 < tile.z; ++c) {
                 uint32_t v[32];
-                const uint32_t taddr = tmem + ((q * 32u) << 16) + ab * BN + c * 32;
+                const uint32_t taddr = tmem + ((q * 32u) << 16) + ab * T::kAccCols + c * 32;
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                     "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -325,8 +376,13 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                 for (int jj = 0; jj < 32; ++jj) {
                     const uint32_t t_j = __shfl_sync(0xFFFFFFFFu, tok, jj);
                     const uint32_t s_j = __shfl_sync(0xFFFFFFFFu, slot, jj);
-                    if (c * 32 + jj < tile.z && m < g.M)
-                        g.Y[(uint64_t)t_j * g.y_token_stride + (uint64_t)s_j * g.M + m] = __uint_as_float(v[jj]);
+                    if (c * 32 + jj < tile.z && m < g.M) {
+                        float* y = g.Y + (uint64_t)t_j * g.y_token_stride + (uint64_t)s_j * g.M + m;
+                        if (g.splits > 1)
+                            atomicAdd(y, __uint_as_float(v[jj]));
+                        else
+                            *y = __uint_as_float(v[jj]);
+                    }
                 }
             }
             tc_fence_before();
@@ -338,7 +394,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * BN))
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * T::kAccCols))
                      : "memory");
     }
 }
@@ -398,8 +454,11 @@ moe_group_kernel(const uint32_t* routing, uint32_t n_pairs, uint32_t n_experts, 
     __syncthreads();
     for (uint32_t e = tid; e < n_experts; e += nt) {
         const uint32_t c = cnt[e];
-        for (uint32_t i = 0; i * bn < c; ++i)
-            tiles[tstart[e] + i] = make_uint4(e, seg[e] + i * bn, min(bn, c - i * bn), 0u);
+        const uint32_t parts = (c + bn - 1) / bn;
+        for (uint32_t i = 0; i < parts; ++i) {  // equal shares: the MMAs take as many columns as a tile has pairs
+            const uint32_t lo = (uint32_t)((uint64_t)i * c / parts), hi = (uint32_t)((uint64_t)(i + 1) * c / parts);
+            tiles[tstart[e] + i] = make_uint4(e, seg[e] + lo, hi - lo, 0u);
+        }
     }
     __syncthreads();
     for (uint32_t p = tid; p < n_pairs; p += nt) {
@@ -462,8 +521,24 @@ cudaError_t launch_gemm(const CUtensorMap& map, const MoeGemmArgs& g, uint32_t m
     return launch_chained(kern, dim3(grid), dim3(kMoeThreads), MoeTile<TYPE, BN>::kSmemBytes, s, map, g);
 }
 
-// Tokens per tile: 32 when experts see few pairs on average (the activation box then stays small), else 128.
-uint32_t pick_bn(uint64_t n_pairs, uint32_t n_experts) { return n_pairs <= (uint64_t)n_experts * 48 ? 32u : 128u; }
+// Most pairs per tile. An expert's weights are unpacked once per tile, which is what bounds the kernel, so an expert
+// should need one tile: the average count and two of its standard deviations (about its root each) have to fit.
+// 32 and 64 leave shared memory for a deeper ring of raw blocks.
+uint32_t pick_bn(uint64_t n_pairs, uint32_t n_experts) {
+    const double avg = (double)n_pairs / n_experts, most = avg + 2.0 * sqrt(avg);
+    return most <= 32.0 ? 32u : most <= 64.0 ? 64u : 160u;
+}
+
+template <int BN>
+cudaError_t launch_gemm_type(uint32_t type, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
+    if (type == T_Q4_K) return launch_gemm<T_Q4_K, BN>(map, g, max_items, s);
+    if (type == T_MXFP4) return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
+    return launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+}
+cudaError_t launch_gemm_bn(uint32_t type, uint32_t bn, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
+    return bn == 32 ? launch_gemm_type<32>(type, map, g, max_items, s)
+           : bn == 64 ? launch_gemm_type<64>(type, map, g, max_items, s) : launch_gemm_type<160>(type, map, g, max_items, s);
+}
 
 }  // namespace
 
@@ -514,7 +589,7 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     MoeGemmArgs g{A, A + a_bytes, expert_stride, Y, header, tiles, list, M, K, n_used, y_token_stride,
-                  (M + kBM - 1) / kBM, status, 0u};
+                  (M + kBM - 1) / kBM, status, 0u, 0u, 1u, 0u};
     const uint64_t max_items64 = (uint64_t)l.max_tiles * g.row_tiles;
     const uint32_t max_items = max_items64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)max_items64;
     // one grouping and one packed activation buffer serve both matrices of a pair (gate and up)
@@ -524,15 +599,7 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
             g.a_end = A2 + a2_bytes;
             g.Y = Y2;
         }
-        if (type == T_Q4_K)
-            e = bn == 32 ? launch_gemm<T_Q4_K, 32>(map, g, max_items, s)
-                         : launch_gemm<T_Q4_K, 128>(map, g, max_items, s);
-        else if (type == T_MXFP4)
-            e = bn == 32 ? launch_gemm<T_MXFP4, 32>(map, g, max_items, s)
-                         : launch_gemm<T_MXFP4, 128>(map, g, max_items, s);
-        else
-            e = bn == 32 ? launch_gemm<T_Q6_K, 32>(map, g, max_items, s)
-                         : launch_gemm<T_Q6_K, 128>(map, g, max_items, s);
+        e = launch_gemm_bn(type, bn, map, g, max_items, s);
         if (e != cudaSuccess) return e;
     }
     if (launches) *launches += A2 ? 4 : 3;
@@ -554,7 +621,9 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
                                    uint32_t* status, cudaStream_t s, uint64_t* launches) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    const uint32_t bn = N <= 32 ? 32u : 128u;
+    // equal tiles of at most 160 tokens
+    const uint32_t bn = N <= 32 ? 32u : N <= 64 ? 64u : 160u;
+    const uint32_t per = (N + (N + bn - 1) / bn - 1) / ((N + bn - 1) / bn);
     CUtensorMap map;
     const cuuint64_t dims[2] = {K, N};
     const cuuint64_t strides[1] = {(cuuint64_t)stride_b * 2};
@@ -564,16 +633,23 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    MoeGemmArgs g{A, A + a_bytes, 0, D, nullptr, nullptr, nullptr, M, K, 1u, stride_d, (M + kBM - 1) / kBM, status, N};
-    const uint64_t items64 = (uint64_t)((N + bn - 1) / bn) * g.row_tiles;
+    MoeGemmArgs g{A, A + a_bytes, 0, D, nullptr, nullptr, nullptr, M, K, 1u, stride_d, (M + kBM - 1) / kBM, status, N, per, 1u, 0u};
+    // Fewer tiles than SMs: K is split over as many work items as find an SM, of two 256-column blocks at least, which add
+    // into a zeroed D. (Q6_K 4096 x 11008 on its 32 row tiles alone: 88 us with 32 tokens, 33 split.)
+    const uint64_t tiles = (uint64_t)((N + per - 1) / per) * g.row_tiles;
+    const uint32_t nblk = (K + 255) >> 8;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t most = tiles < (uint64_t)sms ? (uint32_t)(sms / tiles) : 1u;
+    g.slice = max((nblk + most - 1) / most, 2u);
+    g.splits = (nblk + g.slice - 1) / g.slice;
+    if (g.splits > 1) {
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
+    }
+    const uint64_t items64 = tiles * g.splits;
     const uint32_t items = items64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)items64;
-    cudaError_t e;
-    if (type == T_Q4_K)
-        e = bn == 32 ? launch_gemm<T_Q4_K, 32>(map, g, items, s) : launch_gemm<T_Q4_K, 128>(map, g, items, s);
-    else if (type == T_MXFP4)
-        e = bn == 32 ? launch_gemm<T_MXFP4, 32>(map, g, items, s) : launch_gemm<T_MXFP4, 128>(map, g, items, s);
-    else
-        e = bn == 32 ? launch_gemm<T_Q6_K, 32>(map, g, items, s) : launch_gemm<T_Q6_K, 128>(map, g, items, s);
+    const cudaError_t e = launch_gemm_bn(type, bn, map, g, items, s);
     if (e == cudaSuccess && launches) ++*launches;
     return e;
 }
