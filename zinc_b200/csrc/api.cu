@@ -1196,7 +1196,7 @@ int32_t zc_mul_mm_block_scaled(zc_ctx* ctx, uint32_t type, const void* A, uint64
                     "%s: needs 16-byte aligned A and B, stride_b a multiple of 8 and a 256-byte aligned workspace of "
                     "zc_mul_mm_workspace_bytes(type, N, K) bytes", fn);
     const cudaError_t e = launch_mul_mm_mx(u8(A, a_offset), a_size - a_offset, Bp, f32m(D, d_offset * 4), M, N, K, stride_b,
-                                           stride_d, workspace, ctx->status_dev, ctx->sm_count, ctx->stream, &ctx->launches);
+                                           stride_d, workspace, ctx->status_dev, ctx->stream, &ctx->launches);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }
 

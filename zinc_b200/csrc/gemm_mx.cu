@@ -1,22 +1,26 @@
 // MXFP4 prefill GEMM on the block-scaled tensor-core path: D[t][m] = sum_k W[m][k] X[t][k] with the GGUF MXFP4
 // weights as they are (E2M1 nibbles, one E8M0 scale byte per 32 elements: exactly the operand format of
-// tcgen05.mma kind::mxf8f6f4 with block scaling) and the bf16 activations split into two FP8 terms.
+// tcgen05.mma kind::mxf8f6f4 with block scaling) and the activations, rounded to bf16, split into two FP8 terms.
 //
 //   x = x_hi + x_lo, both E4M3 with their own power-of-two scale per 32 elements. A bf16 value has 8 significant
 //   bits and an E4M3 value 4, so x_hi (x rounded to 4 significant bits) and x_lo (the remainder, again at most 4
-//   significant bits) reproduce x exactly unless an element lies more than 2^14 below its block's maximum;
-//   the two products accumulate into the same f32 accumulator. No weight is dequantised: a row's nibbles are only
-//   re-ordered (GGUF keeps element j and j + 16 in one byte, the tensor core wants 16 consecutive elements in 8
-//   bytes of a 16-byte chunk), about 0.6 integer operations per weight instead of 3.6 for the bf16 route.
+//   significant bits) reproduce x exactly unless an element lies more than 2^14 below its block's maximum (then to
+//   2^-22 of that maximum); the two products accumulate into the same f32 accumulator. No weight is dequantised: a
+//   row's nibbles are only re-ordered (GGUF keeps element j and j + 16 in one byte, the tensor core wants 16
+//   consecutive elements in 8 bytes of a 16-byte chunk), about one integer operation per weight instead of the five
+//   of the bf16 route, whose tiles the integer pipe bounds (73 % busy, 3600 cycles per 256 columns of 128 rows).
 //
-//   1. mx_split_kernel   X bf16 [T][K] -> x_hi, x_lo (bytes [T][K]) and their scale bytes in the 512-byte atoms the
-//                        tensor core reads (128 tokens x 4 blocks: byte (t % 32) * 16 + (t / 32) * 4 + block)
-//   2. gemm_mx_kernel    persistent CTAs over (128 weight rows, 128 tokens) items; per 128-column stage: the weight
-//                        stage (16 KB, K-major, 128-byte swizzle) and its 512 scale bytes written by the slot's 128
-//                        producer threads (one per row) from raw bytes they copied into a private slot a stage ahead, x_hi / x_lo tiles
-//                        by TMA, their scale atoms by bulk copies; one thread copies the three scale atoms into tensor
-//                        memory (tcgen05.cp) and issues eight MMAs (four 32-column steps x two terms); two
-//                        accumulators let the epilogue of an item overlap the next item's MMAs.
+//   1. mx_terms_kernel   X -> x_hi, x_lo (bytes [rows][K]) and their scale bytes in the 512-byte atoms the tensor
+//                        core reads (128 tokens x 4 blocks: byte (t % 32) * 16 + (t / 32) * 4 + block), per tile
+//   2. mx_gemm_kernel    persistent CTAs over (up to BN tokens of an expert or of the only matrix, 128 weight rows)
+//                        items; per 128-column stage: the weight stage (16 KB, K-major, 128-byte swizzle) and its 512
+//                        scale bytes written by the slot's 128 producer threads (one per row) from raw bytes they
+//                        copied a stage of theirs ahead, x_hi / x_lo tiles by TMA, their scale atoms by a bulk copy;
+//                        one warp copies the scale atoms into tensor memory (tcgen05.cp) and issues eight MMAs (four
+//                        32-column steps x two terms, as wide as the tile has tokens); two accumulators let the
+//                        epilogue of an item overlap the next item's MMAs. The 128 rows of an item are one run of
+//                        bytes, so the loader has the next item's run brought to L2 chunk by chunk meanwhile: shared
+//                        memory has room for one raw stage per slot only, too little to cover DRAM's latency.
 // Every mbarrier wait is bounded; a wait that gives up records {1, site}, raises the CTA's flag, and every role
 // drains to the common exit where tensor memory is released.
 //
@@ -30,42 +34,39 @@
 namespace zc {
 namespace {
 
-// N consecutive 32-bit words starting `sh` bits (a multiple of 8) into the aligned word at p.
-template <int N>
-__device__ __forceinline__ void lds_shifted(const uint32_t* p, uint32_t sh, uint32_t (&w)[N]) {
-    uint32_t prev = p[0];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const uint32_t next = p[i + 1];
-        w[i] = __funnelshift_r(prev, next, sh);
-        prev = next;
-    }
-}
-
-constexpr int kMxBN = 128;                 // tokens per item
 constexpr int kMxStageK = 128;             // columns per stage: four MXFP4 blocks, one scale atom
 constexpr int kMxStages = 3;
 constexpr uint32_t kMxABytes = kBM * 128;  // 16 KB: 128 rows x 128 padded-FP4 bytes
-constexpr uint32_t kMxXBytes = kMxBN * 128;
-constexpr uint32_t kMxSfBytes = 512;
-// A | x_hi | x_lo | sfa | sfb_hi | sfb_lo, padded to the 1024-byte alignment the swizzled tiles of the next stage need
-constexpr uint32_t kMxStageBytes = (kMxABytes + 2 * kMxXBytes + 3 * kMxSfBytes + 1023u) & ~1023u;
+constexpr uint32_t kMxAtom = 512;          // scale bytes of 128 rows or tokens, four blocks
+// A row's 68 bytes of a stage in their 16-byte aligned superset: up to six pieces, rows 112 bytes apart (8-byte reads
+// of 16 rows meet two per bank pair, at 96 bytes four).
+constexpr uint32_t kMxPieces = 6, kMxRawRow = 112, kMxRawSlot = kBM * kMxRawRow;
 // Warps: 0 tensor memory + MMA issue, 1 loader, then one group of four producer warps per stage slot (a thread
-// per weight row; group j always fills slot j, so the groups work on different stages at the same time: a
-// thread's chain of loads, shifts and stores per stage is latency-bound and four times the issuing thread's time
-// per stage), then four epilogue warps.
+// per weight row; group j always fills slot j, so the groups work on different stages at the same time), then four
+// epilogue warps.
 constexpr int kMxProdWarp0 = 2, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxStages * kMxGroupWarps;
 constexpr int kMxThreads = (kMxEpiWarp0 + 4) * 32;
-constexpr uint32_t kMxRawSlot = 96;        // bytes per producer thread: the 16-byte aligned superset of a row's 68
-constexpr uint32_t kMxRawOffset = kMxStages * kMxStageBytes;
-constexpr uint32_t kMxBarOffset = kMxRawOffset + kMxStages * 128 * kMxRawSlot;
-constexpr uint32_t kMxSmemBytes = kMxBarOffset + 256 + 1024;
-constexpr uint32_t kMxTmemCols = 512;      // two 128-column accumulators, then 12 scale columns per stage
-constexpr uint32_t kMxSfCol0 = 2 * kMxBN;
+
+template <int BN>
+struct MxTile {
+    static constexpr uint32_t kXBytes = BN * 128;
+    static constexpr uint32_t kSfX = BN > 128 ? 2 * kMxAtom : kMxAtom;  // scale bytes of one term of a tile, four blocks
+    // A | x_hi | x_lo | scales of A, x_hi, x_lo, padded to the 1024-byte alignment the swizzled tiles need
+    static constexpr uint32_t kSfOffset = kMxABytes + 2 * kXBytes;
+    static constexpr uint32_t kStageBytes = (kSfOffset + kMxAtom + 2 * kSfX + 1023u) & ~1023u;
+    static constexpr uint32_t kRawOffset = kMxStages * kStageBytes;
+    static constexpr uint32_t kBarOffset = kRawOffset + kMxStages * kMxRawSlot;
+    static constexpr uint32_t kSmemBytes = kBarOffset + 256 + 1024;
+    // tensor memory: two accumulators, then per stage the scale columns of A, x_hi, x_lo
+    static constexpr uint32_t kSfCols = 4 + 2 * (kSfX / 128);
+    static constexpr uint32_t kSfCol0 = 2 * BN;
+    static constexpr uint32_t kCols = kSfCol0 + kMxStages * kSfCols <= 128 ? 128 : kSfCol0 + kMxStages * kSfCols <= 256 ? 256 : 512;
+    static_assert(kSmemBytes <= 227u * 1024u && kSfCol0 + kMxStages * kSfCols <= 512);
+};
 
 struct MxBars {
     uint64_t full[kMxStages];    // the slot's four producer warps + the loader's expect_tx
-    uint64_t empty[kMxStages];   // the issuing thread's commit
+    uint64_t empty[kMxStages];   // the issuing warp's commit
     uint64_t accum_full[2];
     uint64_t accum_empty[2];     // one arrival per epilogue warp
     uint32_t tmem_base;
@@ -73,28 +74,14 @@ struct MxBars {
 };
 
 struct MxArgs {
-    const uint8_t* A;        // MXFP4 rows, K / 32 blocks of 17 bytes
-    const uint8_t* a_end;
-    const uint8_t* sf_hi;    // scale atoms of x_hi: [token tiles][k atoms][512]
-    const uint8_t* sf_lo;
-    float* D;
-    uint32_t M, N, K, stride_d, row_tiles, tok_tiles;
-    uint32_t* status;
+    MxGemm p;
+    const uint8_t* sf;       // scale atoms: [tile][four blocks][x_hi, x_lo][kSfX]
+    uint32_t rows, row_tiles;
 };
 
-template <bool kSleep = true>
-__device__ __forceinline__ bool mx_wait(uint64_t* bar, uint32_t parity, MxBars* bars, uint32_t* status, uint32_t site) {
-    for (uint32_t i = 0; i < kWaitLimit; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (kSleep) __nanosleep(64);
-        if ((i & 63u) == 63u && bars->failed) return false;
-    }
-    bars->failed = 1;
-    if (status) {
-        status[0] = 1;
-        status[1] = site;
-    }
-    return false;
+__device__ __forceinline__ uint4 mx_tile(const MxGemm& p, uint32_t t) {
+    if (p.dense_n) return make_uint4(0u, t * p.dense_tile, min(p.dense_tile, p.dense_n - t * p.dense_tile), 0u);
+    return __ldg(&p.tiles[t]);
 }
 
 // Shared-memory descriptor of a scale atom for tcgen05.cp: 32 rows of 16 bytes, no swizzle, 8-row groups 128 bytes
@@ -108,11 +95,10 @@ __device__ __forceinline__ void tmem_cp_sf(uint32_t tmem_col, uint64_t desc) {
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(desc) : "memory");
 }
 
-// Instruction descriptor of the block-scaled MMA: A = E2M1, B = E4M3, both K-major, E8M0 scales, M = 128, N = 128,
-// K = 32; sfa / sfb: which byte of the scale words this step uses.
-__device__ __forceinline__ uint32_t mx_idesc(uint32_t sfa, uint32_t sfb) {
-    return (sfb << 4) | (5u << 7) | (0u << 10) | ((uint32_t)(kMxBN >> 3) << 17) | (1u << 23) |
-           ((uint32_t)(kBM >> 4) << 24) | (sfa << 29);
+// Instruction descriptor of the block-scaled MMA: A = E2M1, B = E4M3, both K-major, E8M0 scales, M = 128, N = cols,
+// K = 32; sf: which byte of the scale words this step uses.
+__device__ __forceinline__ uint32_t mx_idesc(uint32_t cols, uint32_t sf) {
+    return (sf << 4) | (5u << 7) | (0u << 10) | ((cols >> 3) << 17) | (1u << 23) | ((uint32_t)(kBM >> 4) << 24) | (sf << 29);
 }
 __device__ __forceinline__ void umma_mx(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                         uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
@@ -130,29 +116,35 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
                  "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-
-// Sixteen nibble bytes of a block (four words) -> the two 8-byte halves the tensor core reads: elements 0..15 (the
-// low nibbles) and 16..31 (the high nibbles), two elements per byte, the lower element in the low nibble.
-__device__ __forceinline__ void repack_block(const uint32_t (&q)[4], uint2& lo, uint2& hi) {
-    uint32_t l[4], h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t a = q[i] & 0x0F0F0F0Fu, b = (q[i] >> 4) & 0x0F0F0F0Fu;
-        l[i] = a | (a >> 4);  // bytes 0 and 2 hold the pairs (0,1) and (2,3)
-        h[i] = b | (b >> 4);
-    }
-    lo = make_uint2(__byte_perm(l[0], l[1], 0x6420), __byte_perm(l[2], l[3], 0x6420));
-    hi = make_uint2(__byte_perm(h[0], h[1], 0x6420), __byte_perm(h[2], h[3], 0x6420));
+// `bytes` (a multiple of 16) at the 16-byte aligned address src -> L2
+__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// Eight nibble bytes of a block (two words) -> the four bytes of the low nibbles and of the high nibbles, two
+// consecutive elements per byte, the lower element in the low nibble.
+__device__ __forceinline__ void repack8(uint32_t q0, uint32_t q1, uint32_t& lo, uint32_t& hi) {
+    const uint32_t even = __byte_perm(q0, q1, 0x6420), odd = __byte_perm(q0, q1, 0x7531);
+    lo = (even & 0x0F0F0F0Fu) | ((odd << 4) & 0xF0F0F0F0u);
+    hi = ((even >> 4) & 0x0F0F0F0Fu) | (odd & 0xF0F0F0F0u);
+}
+
+template <int BN>
 __global__ void __launch_bounds__(kMxThreads, 1)
-gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_hi, const __grid_constant__ CUtensorMap tmap_lo, const MxArgs g) {
+mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
+    // everything this kernel reads but the weights comes from the kernels before it
+    chain_wait();
+    MxArgs g = args;
+    after_wait(g.p.header);
+    after_wait(g.p.tiles);
+    after_wait(g.p.list);
+    using T = MxTile<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    MxBars* bars = reinterpret_cast<MxBars*>(smem + kMxBarOffset);
+    MxBars* bars = reinterpret_cast<MxBars*>(smem + T::kBarOffset);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n_items = g.row_tiles * g.tok_tiles;
-    const uint32_t nb = g.K >> 5;                          // blocks per row
+    const uint32_t n_items = (g.p.dense_n ? (g.p.dense_n + g.p.dense_tile - 1) / g.p.dense_tile : g.p.header[0]) * g.row_tiles;
+    const uint32_t nb = g.p.K >> 5;                        // blocks per row
     const int n_stages = (int)((nb + 3) >> 2);             // the last one may hold fewer than four blocks
     const uint64_t row_bytes = (uint64_t)nb * 17u;
 
@@ -170,7 +162,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_hi, const __grid_constan
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                     "r"(kMxTmemCols)
+                     "r"(T::kCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -180,173 +172,230 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_hi, const __grid_constan
     const uint32_t tmem = bars->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {  // ---- scale copies + MMA issuer ----
-            uint32_t gs = 0, i = 0;
-            bool ok = true;
-            for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
-                const uint32_t ab = i & 1;
-                ok = mx_wait<false>(&bars->accum_empty[ab], ((i >> 1) & 1) ^ 1, bars, g.status, 141);
+        // ---- scale copies + MMA issuer (the converged warp walks, one elected lane issues) ----
+        uint32_t st = 0, ph = 0, i = 0;
+        bool ok = true;
+        for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
+            const uint32_t ab = i & 1;
+            // as many columns as the tile has tokens (N in steps of 16)
+            const uint32_t cols = (mx_tile(g.p, w / g.row_tiles).z + 15u) & ~15u;
+            ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.p.status, 141);
+            if (!ok) break;
+            tc_fence_after();
+            for (int s = 0; s < n_stages; ++s) {
+                ok = warp_poll(smem_u32(&bars->full[st]), ph, bars, g.p.status, 142);
                 if (!ok) break;
                 tc_fence_after();
-                for (int s = 0; s < n_stages; ++s, ++gs) {
-                    const uint32_t st = gs % kMxStages, ph = (gs / kMxStages) & 1;
-                    ok = mx_wait<false>(&bars->full[st], ph, bars, g.status, 142);
-                    if (!ok) break;
-                    tc_fence_after();
-                    uint8_t* stage = smem + st * kMxStageBytes;
-                    const uint32_t sf_col = tmem + kMxSfCol0 + st * 12;
-                    const uint32_t sf_s = smem_u32(stage + kMxABytes + 2 * kMxXBytes);
-                    tmem_cp_sf(sf_col, sf_desc(sf_s));
-                    tmem_cp_sf(sf_col + 4, sf_desc(sf_s + kMxSfBytes));
-                    tmem_cp_sf(sf_col + 8, sf_desc(sf_s + 2 * kMxSfBytes));
-                    const uint64_t da = smem_desc(smem_u32(stage));
-                    const uint64_t dh = smem_desc(smem_u32(stage + kMxABytes));
-                    const uint64_t dl = smem_desc(smem_u32(stage + kMxABytes + kMxXBytes));
-                    const int steps = min(4, (int)nb - 4 * s);
+                const uint32_t stage = smem_u32(smem) + st * T::kStageBytes;
+                const uint32_t sf_a = tmem + T::kSfCol0 + st * T::kSfCols, sf_hi = sf_a + 4, sf_lo = sf_hi + T::kSfX / 128;
+                const uint64_t dsf = sf_desc(stage + T::kSfOffset);
+                const uint64_t da = smem_desc(stage), dh = smem_desc(stage + kMxABytes);
+                const int steps = min(4, (int)nb - 4 * s);
+                if (elect_one()) {
+                    tmem_cp_sf(sf_a, dsf);
+                    tmem_cp_sf(sf_hi, dsf + kMxAtom / 16);
+                    tmem_cp_sf(sf_lo, dsf + (kMxAtom + T::kSfX) / 16);
+                    if constexpr (BN > 128) {  // the scales of tokens 128 and up
+                        if (cols > 128) {
+                            tmem_cp_sf(sf_hi + 4, dsf + 2 * kMxAtom / 16);
+                            tmem_cp_sf(sf_lo + 4, dsf + (2 * kMxAtom + T::kSfX) / 16);
+                        }
+                    }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         if (k < steps) {
-                            umma_mx(tmem + ab * kMxBN, da + 2 * k, dh + 2 * k, mx_idesc(k, k), sf_col, sf_col + 4,
-                                    (s | k) ? 1u : 0u);
-                            umma_mx(tmem + ab * kMxBN, da + 2 * k, dl + 2 * k, mx_idesc(k, k), sf_col, sf_col + 8, 1u);
+                            umma_mx(tmem + ab * BN, da + 2 * k, dh + 2 * k, mx_idesc(cols, k), sf_a, sf_hi, (s | k) ? 1u : 0u);
+                            umma_mx(tmem + ab * BN, da + 2 * k, dh + T::kXBytes / 16 + 2 * k, mx_idesc(cols, k), sf_a, sf_lo, 1u);
                         }
                     }
                     umma_commit(&bars->empty[st]);
+                    if (s + 1 == n_stages) umma_commit(&bars->accum_full[ab]);
                 }
-                if (ok) umma_commit(&bars->accum_full[ab]);
+                if (++st == kMxStages) {
+                    st = 0;
+                    ph ^= 1;
+                }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // ---- loader of the activation terms and their scale atoms ----
-            uint32_t gs = 0;
+        if (lane == 0) {  // ---- loader of the activation terms and their scale atoms; the next item's weights to L2 ----
+            uint32_t st = 0, ph = 1;
             bool ok = true;
+            const uint8_t* run = nullptr;  // the item's weight rows: one run of bytes, its end rounded down to 16
+            uint64_t run_bytes = 0;
+            auto locate = [&](uint32_t w) {
+                run_bytes = 0;
+                if (w >= n_items) return;
+                const uint32_t t = w / g.row_tiles, m0 = (w - t * g.row_tiles) * kBM;
+                run = g.p.A + (uint64_t)mx_tile(g.p, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
+                run_bytes = ((uint64_t)min((uint32_t)kBM, g.p.M - m0) * row_bytes) & ~(uint64_t)15;
+            };
+            auto prefetch = [&](int s) {
+                const uint64_t at = (uint64_t)s * (kBM * 68u);
+                if (at < run_bytes) bulk_prefetch(run + at, (uint32_t)min((uint64_t)(kBM * 68u), run_bytes - at));
+            };
+            locate(blockIdx.x);
+            for (int s = 0; s < n_stages; ++s) prefetch(s);
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
                 const uint32_t tt = w / g.row_tiles;
-                for (int s = 0; s < n_stages; ++s, ++gs) {
-                    const uint32_t st = gs % kMxStages;
-                    ok = mx_wait(&bars->empty[st], ((gs / kMxStages) & 1) ^ 1, bars, g.status, 143);
+                const uint32_t row0 = mx_tile(g.p, tt).y;
+                locate(w + gridDim.x);
+                const uint8_t* sf = g.sf + (size_t)tt * n_stages * 2 * T::kSfX;
+                for (int s = 0; s < n_stages; ++s) {
+                    ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 143);
                     if (!ok) break;
-                    uint8_t* stage = smem + st * kMxStageBytes;
-                    mbar_expect_tx(&bars->full[st], 2 * kMxXBytes + 2 * kMxSfBytes);
-                    tma_load_2d(stage + kMxABytes, &tmap_hi, s * kMxStageK, (int)(tt * kMxBN), &bars->full[st]);
-                    tma_load_2d(stage + kMxABytes + kMxXBytes, &tmap_lo, s * kMxStageK, (int)(tt * kMxBN), &bars->full[st]);
-                    const size_t atom = ((size_t)tt * n_stages + s) * kMxSfBytes;
-                    bulk_load(stage + kMxABytes + 2 * kMxXBytes + kMxSfBytes, g.sf_hi + atom, kMxSfBytes, &bars->full[st]);
-                    bulk_load(stage + kMxABytes + 2 * kMxXBytes + 2 * kMxSfBytes, g.sf_lo + atom, kMxSfBytes, &bars->full[st]);
+                    uint8_t* stage = smem + st * T::kStageBytes;
+                    mbar_expect_tx(&bars->full[st], 2 * T::kXBytes + 2 * T::kSfX);
+                    tma_load_2d(stage + kMxABytes, &tmap_x, s * kMxStageK, (int)row0, &bars->full[st]);
+                    tma_load_2d(stage + kMxABytes + T::kXBytes, &tmap_x, s * kMxStageK, (int)(g.rows + row0), &bars->full[st]);
+                    bulk_load(stage + T::kSfOffset + kMxAtom, sf + (size_t)s * 2 * T::kSfX, 2 * T::kSfX, &bars->full[st]);
+                    prefetch(s);
+                    if (++st == kMxStages) {
+                        st = 0;
+                        ph ^= 1;
+                    }
                 }
             }
         }
-    } else if (warp >= kMxProdWarp0 && warp < kMxEpiWarp0) {
+    } else if (warp < kMxEpiWarp0) {
         // ---- weight producers: group = stage slot, thread = weight row; four blocks (68 bytes) per stage ----
-        const int p = tid - kMxProdWarp0 * 32;
-        const int row = p & 127;
-        const uint32_t grp = (uint32_t)p >> 7;
-        const uint32_t my_items = blockIdx.x < n_items ? (n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-        const uint32_t total = my_items * (uint32_t)n_stages;  // stages this CTA walks, in order
-        uint8_t* my_raw = smem + kMxRawOffset + (size_t)p * kMxRawSlot;
-        // byte offset (into A) of this thread's row segment for flat stage gs
-        auto seg_off = [&](uint32_t gs) -> uint64_t {
-            const uint32_t it = gs / (uint32_t)n_stages, s = gs - it * (uint32_t)n_stages;
-            const uint32_t w = blockIdx.x + it * gridDim.x;
-            const uint32_t grow = min((w % g.row_tiles) * kBM + (uint32_t)row, g.M - 1);  // rows past M: computed, dropped
-            return (uint64_t)grow * row_bytes + (uint64_t)s * 68u;
-        };
-        // the segment's 16-byte aligned superset -> this thread's slot; bytes at or beyond the end of the buffer are
-        // not read (zeros are written)
-        auto fetch = [&](uint64_t off) {
-            const uint8_t* src = g.A + (off & ~(uint64_t)15);
+        const uint32_t p = (uint32_t)(tid - kMxProdWarp0 * 32), row = p & 127, grp = p >> 7;
+        const uint32_t slot = smem_u32(smem) + T::kRawOffset + grp * kMxRawSlot;
+        uint8_t* const slot_p = smem + T::kRawOffset + grp * kMxRawSlot;
+        // The pieces of all rows, dealt to the group's threads row by row (a warp's copy instruction covers five rows'
+        // runs of bytes): byte offset of the piece's row in a tile, and row and piece.
+        uint32_t f_row[kMxPieces], f_rp[kMxPieces];
 #pragma unroll
-            for (int pc = 0; pc < (int)kMxRawSlot / 16; ++pc) {
-                const uint8_t* sp = src + pc * 16;
-                const uint32_t n = sp + 16 <= g.a_end ? 16u : (sp < g.a_end ? (uint32_t)(g.a_end - sp) : 0u);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(my_raw + pc * 16)),
-                             "l"(n ? sp : g.A), "r"(n)
-                             : "memory");
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        uint64_t off = 0;
-        if (grp < total) {
-            off = seg_off(grp);
-            fetch(off);
+        for (uint32_t i = 0; i < kMxPieces; ++i) {
+            const uint32_t idx = row + 128u * i, r = idx / kMxPieces;
+            f_row[i] = r * (uint32_t)row_bytes;
+            f_rp[i] = (r << 8) | (idx - r * kMxPieces);
         }
-        bool dead = false;
-        for (uint32_t gs = grp; gs < total; gs += kMxStages) {
-            // this stage's bytes out of the slot (shifted to the segment's first byte); then the slot is free for
-            // the next own stage, whose copies fly while this one is repacked
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            const uint32_t o = (uint32_t)(off & 15u);
-            uint32_t wd[17];
-            lds_shifted<17>(reinterpret_cast<const uint32_t*>(my_raw + (o & ~3u)), (o & 3u) * 8u, wd);
-            const uint32_t s = gs % (uint32_t)n_stages;
-            if (gs + kMxStages < total) {
-                off = seg_off(gs + kMxStages);
-                fetch(off);
+        // the group's next stage: item, stage of it, first byte of the tile's rows and of this thread's row
+        uint32_t w = blockIdx.x, m0 = 0;
+        int s = (int)grp;
+        const uint8_t* expert = g.p.A;
+        auto locate = [&]() {  // normalise (w, s); past the last item nothing is read
+            while (w < n_items && s >= n_stages) {
+                s -= n_stages;
+                w += gridDim.x;
             }
-            const uint32_t use = gs / kMxStages;  // slot grp, use number
-            if (!dead) dead = !mx_wait(&bars->empty[grp], (use & 1) ^ 1, bars, g.status, 144);
+            if (w < n_items) {
+                const uint32_t t = w / g.row_tiles;
+                m0 = (w - t * g.row_tiles) * kBM;
+                expert = g.p.A + (uint64_t)mx_tile(g.p, t).x * g.p.expert_stride;
+            }
+        };
+        auto fetch = [&]() {
+            const uint8_t* first = expert + (uint64_t)m0 * row_bytes + (uint32_t)s * 68u;
+            const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(first) & 15u;
+            if (m0 + kBM <= g.p.M && first + (uint64_t)(kBM - 1) * row_bytes + kMxPieces * 16 <= g.p.A + g.p.a_bytes) {
+#pragma unroll
+                for (uint32_t i = 0; i < kMxPieces; ++i) {
+                    const uint32_t o = low + f_row[i], piece = f_rp[i] & 255u;
+                    if (piece < kMxPieces - 1 || (o & 15u) > 12u)  // 68 bytes from offset 12 end with the fifth piece
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (f_rp[i] >> 8) * kMxRawRow + piece * 16),
+                                     "l"(first - low + ((o & ~15u) + piece * 16))
+                                     : "memory");
+                }
+            } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
+#pragma unroll 1
+                for (uint32_t i = 0; i < kMxPieces; ++i) {
+                    const uint32_t r = f_rp[i] >> 8, piece = f_rp[i] & 255u;
+                    const uint64_t o = (uint64_t)min(m0 + r, g.p.M - 1) * row_bytes + (uint32_t)s * 68u;
+                    const uint8_t* sp = expert + (o & ~(uint64_t)15) + piece * 16;
+                    const uint8_t* end = g.p.A + g.p.a_bytes;
+                    const uint32_t n = sp + 16 <= end ? 16u : (sp < end ? (uint32_t)(end - sp) : 0u);
+                    cp_async16_zfill(slot_p + r * kMxRawRow + piece * 16, n ? sp : g.p.A, n);
+                }
+            }
+        };
+        locate();
+        if (w < n_items) fetch();
+        bool dead = false;
+        uint32_t use = 0;
+        while (w < n_items) {
+            const int blocks = (int)nb - 4 * s;  // of the stage: four or, at the end of a row, fewer
+            const uint32_t off = (uint32_t)(((uint64_t)min(m0 + row, g.p.M - 1) * row_bytes + (uint32_t)s * 68u) & 15u);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            asm volatile("bar.sync %0, 128;" ::"r"(1u + grp) : "memory");
+            // the row's 68 bytes: 8-byte reads from the offset rounded down to 8, then shifted to the first byte
+            uint32_t v[20], wd[18];
+            const uint8_t* src = slot_p + row * kMxRawRow + (off & 8u);
+#pragma unroll
+            for (int k = 0; k < 10; ++k) {
+                const uint2 t = *reinterpret_cast<const uint2*>(src + 8 * k);
+                v[2 * k] = t.x;
+                v[2 * k + 1] = t.y;
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1u + grp) : "memory");
+            // the slot is read: the group's next stage flies while this one is repacked
+            s += kMxStages;
+            locate();
+            if (w < n_items) fetch();
+            if (off & 4u) {
+#pragma unroll
+                for (int k = 0; k < 19; ++k) v[k] = v[k + 1];
+            }
+#pragma unroll
+            for (int k = 0; k < 18; ++k) wd[k] = __funnelshift_r(v[k], v[k + 1], (off & 3u) * 8u);
+            if (!dead) dead = !poll_or_fail(&bars->empty[grp], (use & 1) ^ 1, bars, g.p.status, 144);
+            ++use;
             if (!dead) {
-                uint8_t* stage = smem + grp * kMxStageBytes;
+                uint8_t* stage = smem + grp * T::kStageBytes;
                 uint8_t* rowp = stage + row * 128;
-                const int sw = row & 7;
+                const uint32_t sw = row & 7;
                 uint32_t sf = 0;
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     // block b: scale byte at 17 b, nibble bytes 17 b + 1 .. 17 b + 16
                     constexpr int kW[4] = {0, 4, 8, 13};
                     constexpr int kS[4] = {8, 16, 24, 0};
-                    const bool live = 4u * s + (uint32_t)b < nb;  // the last stage of a row may be short
                     uint32_t q[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         q[i] = kS[b] ? __funnelshift_r(wd[kW[b] + i], wd[kW[b] + i + 1], kS[b]) : wd[kW[b] + i];
-                    const uint32_t e = (wd[(17 * b) >> 2] >> (8 * ((17 * b) & 3))) & 0xFFu;
-                    uint2 lo, hi;
-                    repack_block(q, lo, hi);
-                    if (!live) lo = hi = make_uint2(0u, 0u);
-                    *reinterpret_cast<uint4*>(rowp + (((2 * b) ^ sw) << 4)) = make_uint4(lo.x, lo.y, 0u, 0u);
-                    *reinterpret_cast<uint4*>(rowp + (((2 * b + 1) ^ sw) << 4)) = make_uint4(hi.x, hi.y, 0u, 0u);
-                    sf |= (live ? e : 127u) << (8 * b);
+                    uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+                    repack8(q[0], q[1], lo.x, hi.x);
+                    repack8(q[2], q[3], lo.y, hi.y);
+                    *reinterpret_cast<uint4*>(rowp + (((2 * b) ^ sw) << 4)) = lo;
+                    *reinterpret_cast<uint4*>(rowp + (((2 * b + 1) ^ sw) << 4)) = hi;
+                    sf |= ((wd[(17 * b) >> 2] >> (8 * ((17 * b) & 3))) & 0xFFu) << (8 * b);
                 }
-                *reinterpret_cast<uint32_t*>(stage + kMxABytes + 2 * kMxXBytes + (row & 31) * 16 + (row >> 5) * 4) = sf;
+                // a short stage: neutral scales (its missing blocks take part in no MMA)
+                if (blocks < 4) sf = (sf & ((1u << (8 * blocks)) - 1u)) | (0x7F7F7F7Fu << (8 * blocks));
+                *reinterpret_cast<uint32_t*>(stage + T::kSfOffset + (row & 31) * 16 + (row >> 5) * 4) = sf;
                 fence_proxy_async();
             }
             __syncwarp();
             if (lane == 0 && !dead) mbar_arrive(&bars->full[grp]);
         }
-    } else if (warp >= kMxEpiWarp0) {
-        // ---- epilogue: lane = weight row, column = token ----
+    } else {
+        // ---- epilogue: lane = weight row, column = pair of the tile ----
         const uint32_t q = warp & 3;
         uint32_t i = 0;
         for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ++i) {
             const uint32_t ab = i & 1;
             const uint32_t tt = w / g.row_tiles;
-            const uint32_t m = (w % g.row_tiles) * kBM + q * 32 + lane;
-            const uint32_t t0 = tt * kMxBN, nt = min((uint32_t)kMxBN, g.N - t0);
-            if (!mx_wait(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 145)) break;
+            const uint4 tile = mx_tile(g.p, tt);
+            const uint32_t m = (w - tt * g.row_tiles) * kBM + q * 32 + lane;
+            if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.p.status, 145)) break;
             __syncwarp();
             tc_fence_after();
 #pragma unroll 1
-            for (uint32_t c = 0; c * 32 < nt; ++c) {
+            for (uint32_t c = 0; c * 32 < tile.z; ++c) {
                 uint32_t v[32];
-                const uint32_t taddr = tmem + ((q * 32u) << 16) + ab * kMxBN + c * 32;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                    "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-                      "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                      "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-                      "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-                      "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (m < g.M) {
+                tmem_ld32(tmem + ((q * 32u) << 16) + ab * BN + c * 32, v);
+                // pair of column c*32 + lane: its output row starts at Y + token * y_token_stride + slot * M
+                const uint32_t idx = c * 32 + lane;
+                const uint32_t pair = idx >= tile.z ? 0u : (g.p.dense_n ? tile.y + idx : __ldg(&g.p.list[tile.y + idx]));
+                const uint32_t tok = pair / g.p.n_used;
+                const uint64_t at = (uint64_t)tok * g.p.y_token_stride + (uint64_t)(pair - tok * g.p.n_used) * g.p.M;
+                tmem_ld_wait();
 #pragma unroll
-                    for (int jj = 0; jj < 32; ++jj)
-                        if (c * 32 + jj < nt)
-                            g.D[(uint64_t)(t0 + c * 32 + jj) * g.stride_d + m] = __uint_as_float(v[jj]);
+                for (int jj = 0; jj < 32; ++jj) {
+                    const uint64_t y = __shfl_sync(0xFFFFFFFFu, at, jj);
+                    if (c * 32 + jj < tile.z && m < g.p.M) g.p.Y[y + m] = __uint_as_float(v[jj]);
                 }
             }
             tc_fence_before();
@@ -358,13 +407,11 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_hi, const __grid_constan
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kMxTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols) : "memory");
     }
 }
 
 // ---- activation split ---------------------------------------------------------------------------------
-// One thread per (token, 32-element block). Tokens at or beyond T (the padding of the last 128-token tile) only
-// write neutral scale bytes; their x rows do not exist (the tensor map fills them with zeros).
 __device__ __forceinline__ uint32_t scale_exp(float maxabs) {
     // power of two s = 2^(e - 127) with maxabs / s in [128, 256): inside E4M3's range (448), four bits kept
     const uint32_t E = (__float_as_uint(maxabs) >> 23) & 0xFFu;
@@ -377,140 +424,189 @@ __device__ __forceinline__ float fp8_to_float(uint8_t v) {
     return __half2float(__half(__nv_cvt_fp8_to_halfraw(v, __NV_E4M3)));
 }
 
-__global__ void __launch_bounds__(256) mx_split_kernel(const __nv_bfloat16* __restrict__ X, uint32_t stride_b,
-                                                       uint8_t* __restrict__ x_hi, uint8_t* __restrict__ x_lo,
-                                                       uint8_t* __restrict__ sf_hi, uint8_t* __restrict__ sf_lo,
-                                                       uint32_t T, uint32_t K, uint32_t n_katoms) {
-    const uint32_t nb = K >> 5;
-    const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t Tp = ((T + 127) / 128) * 128;
-    if (id >= (uint64_t)Tp * n_katoms * 4) return;
-    const uint32_t t = (uint32_t)(id / (n_katoms * 4)), b = (uint32_t)(id - (uint64_t)t * (n_katoms * 4));
-    const size_t sf_at = ((size_t)(t >> 7) * n_katoms + (b >> 2)) * 512 + ((t & 127) & 31) * 16 + ((t & 127) >> 5) * 4 + (b & 3);
-    if (t >= T || b >= nb) {
-        sf_hi[sf_at] = 127;
-        sf_lo[sf_at] = 127;
-        return;
-    }
-    const uint4* src = reinterpret_cast<const uint4*>(X + (size_t)t * stride_b + (size_t)b * 32);
-    float v[32];
-    float mx = 0.f;
+
+struct MxTerms {
+    const void* X;           // f32 or bf16 [T][stride]
+    uint32_t T, K, stride, n_used;
+    const uint2* where;      // per (token, slot) pair: {row of the list, tile << 8 | place in the tile}, row 0xFFFFFFFF:
+                             // not listed; nullptr: token t is row t, in tiles of `tile` tokens
+    uint32_t tile;
+    uint8_t* x;              // [2 * rows][K]: x_hi, then x_lo
+    uint8_t* sf;
+    uint32_t rows, sf_x;
+};
+
+// One warp per (token, 256 columns), eight columns per lane: four lanes a block, sixteen a scale atom's four blocks. A
+// token's terms are made once and written to the rows of all its pairs.
+template <bool kBf16>
+__global__ void __launch_bounds__(256) mx_terms_kernel(const MxTerms a) {
+    chain_wait();
+    const uint32_t chunks = (a.K + 255) / 256, lane = threadIdx.x & 31;
+    const uint32_t id = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (id >= a.T * chunks) return;
+    const uint32_t t = id / chunks, col = (id - t * chunks) * 256 + lane * 8;
+    const bool live = col < a.K;  // whole blocks: K % 32 == 0
+    float v[8] = {};
+    if (live) {
+        if constexpr (kBf16) {
+            const uint4 q = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(a.X) + (size_t)t * a.stride + col);
+            const uint32_t ww[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint4 w = __ldg(src + i);
-        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+            for (int j = 0; j < 4; ++j) {
+                v[2 * j] = __uint_as_float(ww[j] << 16);
+                v[2 * j + 1] = __uint_as_float(ww[j] & 0xFFFF0000u);
+            }
+        } else {
+            const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(a.X) + (size_t)t * a.stride + col);
+            const float4 q0 = src[0], q1 = src[1];
+            const float f[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            v[i * 8 + 2 * j] = __uint_as_float(ww[j] << 16);
-            v[i * 8 + 2 * j + 1] = __uint_as_float(ww[j] & 0xFFFF0000u);
+            for (int j = 0; j < 8; ++j) v[j] = __bfloat162float(__float2bfloat16_rn(f[j]));
         }
     }
+    // one term: four lanes' common power of two, eight E4M3 bytes, what is left over
+    auto term = [&](uint2& bytes) -> uint32_t {
+        float mx = 0.f;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) mx = fmaxf(mx, fabsf(v[i]));
-    const uint32_t eh = scale_exp(mx);
-    const float ih = pow2_neg(eh), sh = pow2_pos(eh);
-    uint32_t hi[8], lo[8];
-    float r[32];
-    float mr = 0.f;
+        for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fabsf(v[j]));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+        const uint32_t e = scale_exp(mx);
+        const float inv = pow2_neg(e), s = pow2_pos(e);
+        uint32_t w[2] = {0u, 0u};
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        const uint8_t q = (uint8_t)__nv_cvt_float_to_fp8(v[i] * ih, __NV_SATFINITE, __NV_E4M3);
-        r[i] = v[i] - fp8_to_float(q) * sh;
-        mr = fmaxf(mr, fabsf(r[i]));
-        if ((i & 3) == 0) hi[i >> 2] = 0;
-        hi[i >> 2] |= (uint32_t)q << (8 * (i & 3));
+        for (int j = 0; j < 8; ++j) {
+            const uint8_t q = (uint8_t)__nv_cvt_float_to_fp8(v[j] * inv, __NV_SATFINITE, __NV_E4M3);
+            v[j] -= fp8_to_float(q) * s;
+            w[j >> 2] |= (uint32_t)q << (8 * (j & 3));
+        }
+        bytes = make_uint2(w[0], w[1]);
+        // the atom's four scale bytes, on the lanes that start a block
+        uint32_t word = e << (8 * ((lane >> 2) & 3));
+        word |= __shfl_xor_sync(0xFFFFFFFFu, word, 4);
+        word |= __shfl_xor_sync(0xFFFFFFFFu, word, 8);
+        return word;
+    };
+    uint2 hi, lo;
+    const uint32_t sf_hi = term(hi), sf_lo = term(lo);
+    const uint32_t atoms = (a.K + 127) / 128;
+    for (uint32_t u = 0; u < a.n_used; ++u) {
+        uint32_t row = t, tile, place;
+        if (a.where) {
+            const uint2 at = a.where[(size_t)t * a.n_used + u];
+            row = at.x;
+            tile = at.y >> 8;
+            place = at.y & 255u;
+        } else {
+            tile = t / a.tile;
+            place = t - tile * a.tile;
+        }
+        if (row == 0xFFFFFFFFu || !live) continue;
+        *reinterpret_cast<uint2*>(a.x + (size_t)row * a.K + col) = hi;
+        *reinterpret_cast<uint2*>(a.x + ((size_t)a.rows + row) * a.K + col) = lo;
+        if ((lane & 15) == 0) {
+            uint8_t* sf = a.sf + ((size_t)tile * atoms + (col >> 7)) * 2 * a.sf_x + (place >> 7) * kMxAtom + (place & 31) * 16 +
+                          ((place & 127) >> 5) * 4;
+            *reinterpret_cast<uint32_t*>(sf) = sf_hi;
+            *reinterpret_cast<uint32_t*>(sf + a.sf_x) = sf_lo;
+        }
     }
-    const uint32_t el = scale_exp(mr);
-    const float il = pow2_neg(el);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        const uint8_t q = (uint8_t)__nv_cvt_float_to_fp8(r[i] * il, __NV_SATFINITE, __NV_E4M3);
-        if ((i & 3) == 0) lo[i >> 2] = 0;
-        lo[i >> 2] |= (uint32_t)q << (8 * (i & 3));
-    }
-    uint4* dh = reinterpret_cast<uint4*>(x_hi + (size_t)t * K + (size_t)b * 32);
-    uint4* dl = reinterpret_cast<uint4*>(x_lo + (size_t)t * K + (size_t)b * 32);
-    dh[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    dh[1] = make_uint4(hi[4], hi[5], hi[6], hi[7]);
-    dl[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    dl[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
-    sf_hi[sf_at] = (uint8_t)eh;
-    sf_lo[sf_at] = (uint8_t)el;
+}
+
+template <int BN>
+cudaError_t launch_gemm(const CUtensorMap& map, const MxArgs& g, uint32_t grid, cudaStream_t s) {
+    auto kern = mx_gemm_kernel<BN>;
+    static std::atomic<uint64_t> attr_done{0};  // per device ordinal
+    if (cudaError_t e = ensure_dynamic_smem(kern, (int)MxTile<BN>::kSmemBytes, attr_done); e != cudaSuccess) return e;
+    return launch_chained(kern, dim3(grid), dim3(kMxThreads), MxTile<BN>::kSmemBytes, s, map, g);
 }
 
 struct MxLayout {
-    uint64_t x_bytes, sf_bytes, total;
-    uint32_t n_katoms, tok_tiles;
+    uint64_t sf, total;
+    uint32_t sf_x;
 };
-MxLayout mx_layout(uint32_t N, uint32_t K) {
+MxLayout mx_layout(uint64_t rows, uint32_t K, uint64_t tiles, uint32_t bn) {
     MxLayout l;
-    l.n_katoms = (K + 127) / 128;
-    l.tok_tiles = (N + kMxBN - 1) / kMxBN;
-    l.x_bytes = (((uint64_t)N * K) + 1023) & ~1023ull;
-    l.sf_bytes = (uint64_t)l.tok_tiles * l.n_katoms * 512;
-    l.total = 2 * l.x_bytes + 2 * l.sf_bytes;
+    l.sf_x = bn > 128 ? 2 * kMxAtom : kMxAtom;
+    l.sf = (2 * rows * K + 1023) & ~1023ull;
+    l.total = l.sf + tiles * ((K + 127) / 128) * 2 * l.sf_x;
     return l;
+}
+
+// Tokens per tile of the plain GEMM: equal tiles of at most 160.
+uint32_t dense_bn(uint32_t N) { return N <= 64 ? 64u : 160u; }
+uint32_t dense_tile(uint32_t N) {
+    const uint32_t n = (N + dense_bn(N) - 1) / dense_bn(N);
+    return (N + n - 1) / n;
 }
 
 }  // namespace
 
-uint64_t mul_mm_mx_workspace_bytes(uint32_t N, uint32_t K) { return mx_layout(N, K).total; }
+uint64_t mx_bytes(uint64_t rows, uint32_t K, uint64_t tiles, uint32_t bn) { return mx_layout(rows, K, tiles, bn).total; }
+
+cudaError_t launch_mx_terms(const void* X, bool bf16, uint32_t T, uint32_t K, uint32_t stride, uint32_t n_used,
+                            const uint2* where, uint32_t tile, uint64_t rows, uint64_t tiles, uint32_t bn, uint8_t* ws,
+                            cudaStream_t s) {
+    const MxLayout l = mx_layout(rows, K, tiles, bn);
+    const MxTerms a{X, T, K, stride, n_used, where, tile, ws, ws + l.sf, (uint32_t)rows, l.sf_x};
+    const uint64_t warps = (uint64_t)T * ((K + 255) / 256);
+    if (warps > 0x7FFFFFFFull) return cudaErrorNotSupported;
+    return launch_chained(bf16 ? mx_terms_kernel<true> : mx_terms_kernel<false>, dim3((uint32_t)((warps + 7) / 8)), dim3(256), 0, s, a);
+}
+
+cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint32_t bn, const uint8_t* ws, cudaStream_t s) {
+    EncodeFn enc = encode_fn();
+    if (!enc) return cudaErrorNotSupported;
+    const MxLayout l = mx_layout(rows, p.K, tiles, bn);
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {p.K, 2 * rows};
+    const cuuint64_t strides[1] = {p.K};
+    const cuuint32_t box[2] = {(cuuint32_t)kMxStageK, bn};
+    const cuuint32_t estr[2] = {1, 1};
+    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(ws), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorNotSupported;
+    const MxArgs g{p, ws + l.sf, (uint32_t)rows, (p.M + kBM - 1) / kBM};
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint64_t items = tiles * g.row_tiles;
+    const uint32_t grid = (uint32_t)(items < (uint64_t)sms ? items : (uint64_t)sms);
+    return bn == 32 ? launch_gemm<32>(map, g, grid, s) : bn == 64 ? launch_gemm<64>(map, g, grid, s) : launch_gemm<160>(map, g, grid, s);
+}
+
+uint64_t mul_mm_mx_workspace_bytes(uint32_t N, uint32_t K) {
+    const uint32_t tile = N ? dense_tile(N) : 1;
+    return mx_bytes(N, K, (N + tile - 1) / tile, dense_bn(N));
+}
 
 bool mul_mm_mx_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K, uint32_t stride_b,
                         const void* workspace, uint64_t workspace_size) {
     if (type != T_MXFP4 || (K & 31u) || K < 128 || N < 64) return false;
-    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_size < mx_layout(N, K).total) return false;
+    if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) || workspace_size < mul_mm_mx_workspace_bytes(N, K)) return false;
     return !(reinterpret_cast<uintptr_t>(A) & 15u) && !(reinterpret_cast<uintptr_t>(B) & 15u) && !(stride_b & 7u);
 }
 
 cudaError_t launch_mul_mm_mx(const uint8_t* A, uint64_t a_bytes, const void* B, float* D, uint32_t M, uint32_t N,
                              uint32_t K, uint32_t stride_b, uint32_t stride_d, void* workspace, uint32_t* status,
-                             int sm_count, cudaStream_t s, uint64_t* launches) {
-    EncodeFn enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    const MxLayout l = mx_layout(N, K);
+                             cudaStream_t s, uint64_t* launches) {
+    const uint32_t bn = dense_bn(N), tile = dense_tile(N), tiles = (N + tile - 1) / tile;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
-    uint8_t* x_hi = ws;
-    uint8_t* x_lo = ws + l.x_bytes;
-    uint8_t* sf_hi = ws + 2 * l.x_bytes;
-    uint8_t* sf_lo = sf_hi + l.sf_bytes;
-    CUtensorMap maps[2];
-    for (int i = 0; i < 2; ++i) {
-        const cuuint64_t dims[2] = {K, N};
-        const cuuint64_t strides[1] = {(cuuint64_t)K};
-        const cuuint32_t box[2] = {(cuuint32_t)kMxStageK, (cuuint32_t)kMxBN};
-        const cuuint32_t estr[2] = {1, 1};
-        if (enc(&maps[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, i == 0 ? x_hi : x_lo, dims, strides, box, estr,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorNotSupported;
-    }
-    const uint32_t Tp = l.tok_tiles * kMxBN;
-    const uint64_t threads = (uint64_t)Tp * l.n_katoms * 4;
-    mx_split_kernel<<<(uint32_t)((threads + 255) / 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(B), stride_b, x_hi,
-                                                                      x_lo, sf_hi, sf_lo, N, K, l.n_katoms);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_mx_terms(B, true, N, K, stride_b, 1, nullptr, tile, N, tiles, bn, ws, s);
     if (e != cudaSuccess) return e;
     if (launches) ++*launches;
-    static std::atomic<uint64_t> attr_done{0};
-    if ((e = ensure_dynamic_smem(gemm_mx_kernel, (int)kMxSmemBytes, attr_done)) != cudaSuccess) return e;
-    MxArgs g;
-    g.A = A;
-    g.a_end = A + a_bytes;
-    g.sf_hi = sf_hi;
-    g.sf_lo = sf_lo;
-    g.D = D;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.stride_d = stride_d;
-    g.row_tiles = (M + kBM - 1) / kBM;
-    g.tok_tiles = l.tok_tiles;
-    g.status = status;
-    const uint32_t items = g.row_tiles * g.tok_tiles;
-    const uint32_t grid = items < (uint32_t)sm_count ? items : (uint32_t)sm_count;
-    gemm_mx_kernel<<<grid, kMxThreads, kMxSmemBytes, s>>>(maps[0], maps[1], g);
-    e = cudaGetLastError();
+    MxGemm p{};
+    p.A = A;
+    p.a_bytes = a_bytes;
+    p.Y = D;
+    p.M = M;
+    p.K = K;
+    p.n_used = 1;
+    p.y_token_stride = stride_d;
+    p.dense_n = N;
+    p.dense_tile = tile;
+    p.status = status;
+    e = launch_mx_gemm(p, N, tiles, bn, ws, s);
     if (e == cudaSuccess && launches) ++*launches;
     return e;
 }

@@ -194,7 +194,25 @@ bool mul_mm_mx_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t
                         const void* workspace, uint64_t workspace_size);
 cudaError_t launch_mul_mm_mx(const uint8_t* A, uint64_t a_bytes, const void* B, float* D, uint32_t M, uint32_t N,
                              uint32_t K, uint32_t stride_b, uint32_t stride_d, void* workspace, uint32_t* status,
-                             int sm_count, cudaStream_t s, uint64_t* launches);
+                             cudaStream_t s, uint64_t* launches);
+// The block-scaled GEMM of one matrix or of an expert stack, over activations that launch_mx_terms has split into their two
+// FP8 terms in `ws` (mx_bytes() bytes, 256-byte aligned; bn: 32, 64 or 160, the most tokens of a tile).
+struct MxGemm {
+    const uint8_t* A;             // MXFP4 rows, K / 32 blocks of 17 bytes; 16-byte aligned, as expert_stride
+    uint64_t a_bytes, expert_stride;
+    float* Y;
+    const uint32_t* header;       // grouped: as the grouped GEMM's tables
+    const uint4* tiles;
+    const uint32_t* list;
+    uint32_t M, K, n_used, y_token_stride;
+    uint32_t dense_n, dense_tile; // > 0: plain GEMM over dense_n tokens in tiles of dense_tile
+    uint32_t* status;
+};
+uint64_t mx_bytes(uint64_t rows, uint32_t K, uint64_t tiles, uint32_t bn);
+cudaError_t launch_mx_terms(const void* X, bool bf16, uint32_t T, uint32_t K, uint32_t stride, uint32_t n_used,
+                            const uint2* where, uint32_t tile, uint64_t rows, uint64_t tiles, uint32_t bn, uint8_t* ws,
+                            cudaStream_t s);
+cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint32_t bn, const uint8_t* ws, cudaStream_t s);
 // Zeroes an N x M output (row stride stride_d) that the GEMM launched behind it adds into.
 cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s);
 bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K,

@@ -403,7 +403,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
 // One CTA. Shared: cnt[n_experts], seg[n_experts] (first list slot, then the running cursor), tstart[n_experts].
 __global__ void __launch_bounds__(1024, 1)
 moe_group_kernel(const uint32_t* routing, uint32_t n_pairs, uint32_t n_experts, uint32_t bn, uint32_t* header, uint4* tiles,
-                 uint32_t* list, uint32_t* status) {
+                 uint32_t* list, uint2* where, uint32_t* status) {
     chain_wait();
     after_wait(routing);
     extern __shared__ uint32_t sh[];
@@ -463,7 +463,17 @@ moe_group_kernel(const uint32_t* routing, uint32_t n_pairs, uint32_t n_experts, 
     __syncthreads();
     for (uint32_t p = tid; p < n_pairs; p += nt) {
         const uint32_t e = routing[p];
-        if (e < n_experts) list[atomicAdd(&seg[e], 1u)] = p;
+        if (e < n_experts) {
+            const uint32_t at = atomicAdd(&seg[e], 1u);
+            list[at] = p;
+            if (where) {  // the k-th pair of the expert: its tile, and its place there
+                const uint32_t c = cnt[e], parts = (c + bn - 1) / bn, k = at - tiles[tstart[e]].y;
+                const uint32_t i = (uint32_t)(((uint64_t)(k + 1) * parts - 1) / c);
+                where[p] = make_uint2(at, (tstart[e] + i) << 8 | (k - (uint32_t)((uint64_t)i * c / parts)));
+            }
+        } else if (where) {
+            where[p] = make_uint2(0xFFFFFFFFu, 0u);
+        }
     }
 }
 
@@ -495,17 +505,18 @@ moe_gather_x_kernel(const float* X, const uint32_t* header, const uint32_t* list
 constexpr uint32_t kMoeMaxExperts = 4096;
 
 struct WsLayout {
-    uint64_t header, tiles, list, xp, total;
+    uint64_t header, tiles, list, where, xp, total;
     uint32_t max_tiles;
 };
-WsLayout ws_layout(uint64_t n_pairs, uint32_t K, uint32_t n_experts, uint32_t bn) {
+WsLayout ws_layout(uint64_t n_pairs, uint32_t K, uint32_t n_experts, uint32_t bn, bool mx) {
     WsLayout l;
     l.max_tiles = (uint32_t)(n_pairs / bn + n_experts);
     l.header = 0;
     l.tiles = 256;
     l.list = l.tiles + (uint64_t)l.max_tiles * 16;
-    l.xp = (l.list + n_pairs * 4 + 255) & ~(uint64_t)255;
-    l.total = l.xp + n_pairs * K * 2;
+    l.where = (l.list + n_pairs * 4 + 255) & ~(uint64_t)255;
+    l.xp = mx ? (l.where + n_pairs * 8 + 255) & ~(uint64_t)255 : l.where;
+    l.total = l.xp + (mx ? mx_bytes(n_pairs, K, l.max_tiles, bn) : n_pairs * K * 2);
     return l;
 }
 
@@ -523,27 +534,38 @@ cudaError_t launch_gemm(const CUtensorMap& map, const MoeGemmArgs& g, uint32_t m
 
 // Most pairs per tile. An expert's weights are unpacked once per tile, which is what bounds the kernel, so an expert
 // should need one tile: the average count and two of its standard deviations (about its root each) have to fit.
-// 32 and 64 leave shared memory for a deeper ring of raw blocks.
-uint32_t pick_bn(uint64_t n_pairs, uint32_t n_experts) {
+// 32 and 64 leave shared memory for a deeper ring of raw blocks; Q6_K's blocks are the largest, and beside 160 pairs only
+// two fit (12288 x 1280, 77 tokens in one tile: 16.3 us beside 160, 14.6 beside 128).
+uint32_t bn_most(uint32_t type) { return type == T_Q6_K ? 128u : 160u; }
+uint32_t pick_bn(uint32_t type, uint64_t n_pairs, uint32_t n_experts) {
     const double avg = (double)n_pairs / n_experts, most = avg + 2.0 * sqrt(avg);
-    return most <= 32.0 ? 32u : most <= 64.0 ? 64u : 160u;
+    return most <= 32.0 ? 32u : most <= 64.0 ? 64u : bn_most(type);
 }
 
 template <int BN>
 cudaError_t launch_gemm_type(uint32_t type, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
     if (type == T_Q4_K) return launch_gemm<T_Q4_K, BN>(map, g, max_items, s);
     if (type == T_MXFP4) return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
-    return launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+    if constexpr (BN == 160)
+        return cudaErrorNotSupported;
+    else
+        return launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
 }
 cudaError_t launch_gemm_bn(uint32_t type, uint32_t bn, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
-    return bn == 32 ? launch_gemm_type<32>(type, map, g, max_items, s)
-           : bn == 64 ? launch_gemm_type<64>(type, map, g, max_items, s) : launch_gemm_type<160>(type, map, g, max_items, s);
+    switch (bn) {
+        case 32: return launch_gemm_type<32>(type, map, g, max_items, s);
+        case 64: return launch_gemm_type<64>(type, map, g, max_items, s);
+        case 128: return launch_gemm<T_Q6_K, 128>(map, g, max_items, s);
+        default: return launch_gemm_type<160>(type, map, g, max_items, s);
+    }
 }
 
 }  // namespace
 
 uint64_t moe_grouped_workspace_bytes(uint64_t n_pairs, uint32_t K, uint32_t n_experts) {
-    return ws_layout(n_pairs, K, n_experts, 32).total;  // the smaller tile needs the longer tile table
+    uint64_t most = 0;  // whatever the type and the tiles
+    for (const uint32_t bn : {32u, 64u, 160u}) most = max(most, ws_layout(n_pairs, K, n_experts, bn, true).total);
+    return most;
 }
 
 bool moe_grouped_eligible(uint32_t type, const uint8_t* A, uint32_t K, uint64_t expert_stride, uint32_t n_experts,
@@ -564,17 +586,33 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     const uint64_t n_pairs = (uint64_t)n_tokens * n_used;
-    const uint32_t bn = pick_bn(n_pairs, n_experts);
-    const WsLayout l = ws_layout(n_pairs, K, n_experts, bn);
+    const uint32_t bn = pick_bn(type, n_pairs, n_experts);
+    const bool mx = type == T_MXFP4;
+    const WsLayout l = ws_layout(n_pairs, K, n_experts, bn, mx);
     uint8_t* base = static_cast<uint8_t*>(ws);
     uint32_t* header = reinterpret_cast<uint32_t*>(base + l.header);
     uint4* tiles = reinterpret_cast<uint4*>(base + l.tiles);
     uint32_t* list = reinterpret_cast<uint32_t*>(base + l.list);
+    uint2* where = mx ? reinterpret_cast<uint2*>(base + l.where) : nullptr;
     __nv_bfloat16* xp = reinterpret_cast<__nv_bfloat16*>(base + l.xp);
 
     cudaError_t e = launch_chained(moe_group_kernel, dim3(1), dim3(1024), n_experts * 12, s, routing, (uint32_t)n_pairs,
-                                   n_experts, bn, header, tiles, list, status);
+                                   n_experts, bn, header, tiles, list, where, status);
     if (e != cudaSuccess) return e;
+    if (mx) {  // the weights as they are, the activations as two FP8 terms
+        uint8_t* terms = base + l.xp;
+        e = launch_mx_terms(X, false, n_tokens, K, x_token_stride, n_used, where, 0, n_pairs, l.max_tiles, bn, terms, s);
+        MxGemm p{A, a_bytes, expert_stride, Y, header, tiles, list, M, K, n_used, y_token_stride, 0u, 0u, status};
+        if (e == cudaSuccess) e = launch_mx_gemm(p, n_pairs, l.max_tiles, bn, terms, s);
+        if (e == cudaSuccess && A2) {
+            p.A = A2;
+            p.a_bytes = a2_bytes;
+            p.Y = Y2;
+            e = launch_mx_gemm(p, n_pairs, l.max_tiles, bn, terms, s);
+        }
+        if (e == cudaSuccess && launches) *launches += A2 ? 4 : 3;
+        return e;
+    }
     e = launch_chained(moe_gather_x_kernel, dim3((uint32_t)((n_pairs + 7) / 8)), dim3(256), 0, s, X, header, list, xp, K,
                        n_used, x_token_stride);
     if (e != cudaSuccess) return e;
@@ -621,8 +659,8 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
                                    uint32_t* status, cudaStream_t s, uint64_t* launches) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    // equal tiles of at most 160 tokens
-    const uint32_t bn = N <= 32 ? 32u : N <= 64 ? 64u : 160u;
+    // equal tiles of at most 160 tokens (128: Q6_K)
+    const uint32_t bn = N <= 32 ? 32u : N <= 64 ? 64u : bn_most(type);
     const uint32_t per = (N + (N + bn - 1) / bn - 1) / ((N + bn - 1) / bn);
     CUtensorMap map;
     const cuuint64_t dims[2] = {K, N};
