@@ -14,8 +14,9 @@
 //                        core reads (128 tokens x 4 blocks: byte (t % 32) * 16 + (t / 32) * 4 + block), per tile
 //   2. mx_gemm_kernel    persistent CTAs over (up to BN tokens of an expert or of the only matrix, 128 weight rows)
 //                        items; per 128-column stage: the weight stage (16 KB, K-major, 128-byte swizzle) and its 512
-//                        scale bytes written by the slot's 128 producer threads (one per row) from raw bytes they
-//                        copied a stage of theirs ahead, x_hi / x_lo tiles by TMA, their scale atoms by a bulk copy;
+//                        scale bytes written by the slot's 128 producer threads (one per row) from raw bytes that
+//                        four warps fetch ahead (made by the producers themselves, the copies took a third
+//                        of their time), x_hi / x_lo tiles by TMA, their scale atoms by a bulk copy;
 //                        one warp copies the scale atoms into tensor memory (tcgen05.cp) and issues eight MMAs (four
 //                        32-column steps x two terms, as wide as the tile has tokens); two accumulators let the
 //                        epilogue of an item overlap the next item's MMAs. The 128 rows of an item are one run of
@@ -41,10 +42,11 @@ constexpr uint32_t kMxAtom = 512;          // scale bytes of 128 rows or tokens,
 // A row's 68 bytes of a stage in their 16-byte aligned superset: up to six pieces, rows 112 bytes apart (8-byte reads
 // of 16 rows meet two per bank pair, at 96 bytes four).
 constexpr uint32_t kMxPieces = 6, kMxRawRow = 112, kMxRawSlot = kBM * kMxRawRow;
-// Warps: 0 tensor memory + MMA issue, 1 loader, then one group of four producer warps per stage slot (a thread
+// Warps: 0 tensor memory + MMA issue, 1 loader, four that fetch raw weight bytes, then one group of four producer warps per stage slot (a thread
 // per weight row; group j always fills slot j, so the groups work on different stages at the same time), then four
 // epilogue warps.
-constexpr int kMxProdWarp0 = 2, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxStages * kMxGroupWarps;
+constexpr int kMxFetchWarp0 = 2, kMxFetchWarps = 4;
+constexpr int kMxProdWarp0 = kMxFetchWarp0 + kMxFetchWarps, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxStages * kMxGroupWarps;
 constexpr int kMxThreads = (kMxEpiWarp0 + 4) * 32;
 
 template <int BN>
@@ -55,8 +57,11 @@ struct MxTile {
     static constexpr uint32_t kSfOffset = kMxABytes + 2 * kXBytes;
     static constexpr uint32_t kStageBytes = (kSfOffset + kMxAtom + 2 * kSfX + 1023u) & ~1023u;
     static constexpr uint32_t kRawOffset = kMxStages * kStageBytes;
-    static constexpr uint32_t kBarOffset = kRawOffset + kMxStages * kMxRawSlot;
-    static constexpr uint32_t kSmemBytes = kBarOffset + 256 + 1024;
+    // raw slots: what is left, eight at most
+    static constexpr uint32_t kAvail = 227u * 1024u - 1024 - 512 - kRawOffset;
+    static constexpr uint32_t kRawSlots = kAvail / kMxRawSlot > 8 ? 8 : kAvail / kMxRawSlot;
+    static constexpr uint32_t kBarOffset = kRawOffset + kRawSlots * kMxRawSlot;
+    static constexpr uint32_t kSmemBytes = kBarOffset + 512 + 1024;
     // tensor memory: two accumulators, then per stage the scale columns of A, x_hi, x_lo
     static constexpr uint32_t kSfCols = 4 + 2 * (kSfX / 128);
     static constexpr uint32_t kSfCol0 = 2 * BN;
@@ -67,6 +72,8 @@ struct MxTile {
 struct MxBars {
     uint64_t full[kMxStages];    // the slot's four producer warps + the loader's expect_tx
     uint64_t empty[kMxStages];   // the issuing warp's commit
+    uint64_t full_w[8];          // raw slots: a copy-completion arrival per fetch thread
+    uint64_t empty_w[8];         // the four producer warps that read the slot
     uint64_t accum_full[2];
     uint64_t accum_empty[2];     // one arrival per epilogue warp
     uint32_t tmem_base;
@@ -79,9 +86,9 @@ struct MxArgs {
     uint32_t rows, row_tiles;
 };
 
-__device__ __forceinline__ uint4 mx_tile(const MxGemm& p, uint32_t t) {
+__device__ __forceinline__ uint4 mx_tile(const MxGemm& p, const uint4* tiles, uint32_t t) {
     if (p.dense_n) return make_uint4(0u, t * p.dense_tile, min(p.dense_tile, p.dense_n - t * p.dense_tile), 0u);
-    return __ldg(&p.tiles[t]);
+    return __ldg(&tiles[t]);
 }
 
 // Shared-memory descriptor of a scale atom for tcgen05.cp: 32 rows of 16 bytes, no swizzle, 8-row groups 128 bytes
@@ -134,16 +141,19 @@ __global__ void __launch_bounds__(kMxThreads, 1)
 mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
     // everything this kernel reads but the weights comes from the kernels before it
     chain_wait();
-    MxArgs g = args;
-    after_wait(g.p.header);
-    after_wait(g.p.tiles);
-    after_wait(g.p.list);
+    const MxArgs& g = args;
+    const uint32_t* header = g.p.header;
+    const uint4* tiles = g.p.tiles;
+    const uint32_t* list = g.p.list;
+    after_wait(header);
+    after_wait(tiles);
+    after_wait(list);
     using T = MxTile<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     MxBars* bars = reinterpret_cast<MxBars*>(smem + T::kBarOffset);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t n_items = (g.p.dense_n ? (g.p.dense_n + g.p.dense_tile - 1) / g.p.dense_tile : g.p.header[0]) * g.row_tiles;
+    const uint32_t n_items = (g.p.dense_n ? (g.p.dense_n + g.p.dense_tile - 1) / g.p.dense_tile : header[0]) * g.row_tiles;
     const uint32_t nb = g.p.K >> 5;                        // blocks per row
     const int n_stages = (int)((nb + 3) >> 2);             // the last one may hold fewer than four blocks
     const uint64_t row_bytes = (uint64_t)nb * 17u;
@@ -152,6 +162,10 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         for (int s = 0; s < kMxStages; ++s) {
             mbar_init(&bars->full[s], kMxGroupWarps + 1);
             mbar_init(&bars->empty[s], 1);
+        }
+        for (uint32_t s = 0; s < T::kRawSlots; ++s) {
+            mbar_init(&bars->full_w[s], kMxFetchWarps * 32);
+            mbar_init(&bars->empty_w[s], kMxGroupWarps);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars->accum_full[s], 1);
@@ -169,7 +183,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = bars->tmem_base;
+    const uint32_t tmem = warp_uniform(bars->tmem_base);
 
     if (warp == 0) {
         // ---- scale copies + MMA issuer (the converged warp walks, one elected lane issues) ----
@@ -178,7 +192,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
             const uint32_t ab = i & 1;
             // as many columns as the tile has tokens (N in steps of 16)
-            const uint32_t cols = (mx_tile(g.p, w / g.row_tiles).z + 15u) & ~15u;
+            const uint32_t cols = warp_uniform((mx_tile(g.p, tiles, w / g.row_tiles).z + 15u) & ~15u);
             ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.p.status, 141);
             if (!ok) break;
             tc_fence_after();
@@ -203,10 +217,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                     }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        if (k < steps) {
-                            umma_mx(tmem + ab * BN, da + 2 * k, dh + 2 * k, mx_idesc(cols, k), sf_a, sf_hi, (s | k) ? 1u : 0u);
-                            umma_mx(tmem + ab * BN, da + 2 * k, dh + T::kXBytes / 16 + 2 * k, mx_idesc(cols, k), sf_a, sf_lo, 1u);
-                        }
+                        if (k == steps) break;
+                        umma_mx(tmem + ab * BN, da + 2 * k, dh + 2 * k, mx_idesc(cols, k), sf_a, sf_hi, (s | k) ? 1u : 0u);
+                        umma_mx(tmem + ab * BN, da + 2 * k, dh + T::kXBytes / 16 + 2 * k, mx_idesc(cols, k), sf_a, sf_lo, 1u);
                     }
                     umma_commit(&bars->empty[st]);
                     if (s + 1 == n_stages) umma_commit(&bars->accum_full[ab]);
@@ -227,7 +240,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                 run_bytes = 0;
                 if (w >= n_items) return;
                 const uint32_t t = w / g.row_tiles, m0 = (w - t * g.row_tiles) * kBM;
-                run = g.p.A + (uint64_t)mx_tile(g.p, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
+                run = g.p.A + (uint64_t)mx_tile(g.p, tiles, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
                 run_bytes = ((uint64_t)min((uint32_t)kBM, g.p.M - m0) * row_bytes) & ~(uint64_t)15;
             };
             auto prefetch = [&](int s) {
@@ -238,7 +251,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             for (int s = 0; s < n_stages; ++s) prefetch(s);
             for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
                 const uint32_t tt = w / g.row_tiles;
-                const uint32_t row0 = mx_tile(g.p, tt).y;
+                const uint32_t row0 = mx_tile(g.p, tiles, tt).y;
                 locate(w + gridDim.x);
                 const uint8_t* sf = g.sf + (size_t)tt * n_stages * 2 * T::kSfX;
                 for (int s = 0; s < n_stages; ++s) {
@@ -257,82 +270,106 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                 }
             }
         }
+    } else if (warp < kMxProdWarp0) {
+        // ---- fetchers: the raw bytes of a stage, the 16-byte pieces of all rows dealt to the 128 threads row by row (a
+        // warp's copy instruction covers five rows' runs of bytes). Each copy reports to the slot's barrier by itself. ----
+        const uint32_t p = (uint32_t)(tid - kMxFetchWarp0 * 32);
+        uint32_t f_row[kMxPieces], f_piece[kMxPieces], f_dst[kMxPieces];  // byte offset of the piece's row in a tile, ..
+#pragma unroll
+        for (uint32_t i = 0; i < kMxPieces; ++i) {
+            const uint32_t idx = p + 128u * i, r = idx / kMxPieces;
+            f_row[i] = r * (uint32_t)row_bytes;
+            f_piece[i] = (idx - r * kMxPieces) * 16;
+            f_dst[i] = r * kMxRawRow + f_piece[i];
+        }
+        const uint8_t* const end = g.p.A + g.p.a_bytes;
+        uint32_t slot = 0, ph = 1;
+        bool ok = true;
+        for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
+            const uint32_t t = w / g.row_tiles, m0 = (w - t * g.row_tiles) * kBM;
+            const uint8_t* rows = g.p.A + (uint64_t)mx_tile(g.p, tiles, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
+            // whether every piece of every stage can be read
+            const bool inside = m0 + kBM <= g.p.M && rows + (uint64_t)kBM * row_bytes + kMxPieces * 16 <= end;
+            for (int s = 0; s < n_stages; ++s) {
+                ok = poll_or_fail(&bars->empty_w[slot], ph, bars, g.p.status, 146);
+                if (!ok) break;
+                uint8_t* const raw = smem + T::kRawOffset + slot * kMxRawSlot;
+                if (inside) {
+                    const uint8_t* first = rows + (uint32_t)s * 68u;
+                    const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(first) & 15u;
+                    first -= low;
+#pragma unroll
+                    for (uint32_t i = 0; i < kMxPieces; ++i) {
+                        const uint32_t o = low + f_row[i];
+                        if (f_piece[i] < (kMxPieces - 1) * 16 || (o & 15u) > 12u)  // 68 bytes from offset 12 end with the fifth piece
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(raw) + f_dst[i]),
+                                         "l"(first + ((o & ~15u) + f_piece[i]))
+                                         : "memory");
+                    }
+                } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
+#pragma unroll 1
+                    for (uint32_t i = 0; i < kMxPieces; ++i) {
+                        const uint32_t idx = p + 128u * i, r = idx / kMxPieces, piece = idx - r * kMxPieces;
+                        const uint32_t o = min(r, g.p.M - 1 - m0) * (uint32_t)row_bytes + (uint32_t)s * 68u;
+                        const uint8_t* sp = rows + (o & ~15u) + piece * 16;
+                        const uint32_t n = sp + 16 <= end ? 16u : (sp < end ? (uint32_t)(end - sp) : 0u);
+                        cp_async16_zfill(raw + r * kMxRawRow + piece * 16, n ? sp : g.p.A, n);
+                    }
+                }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[slot])) : "memory");
+                if (++slot == T::kRawSlots) {
+                    slot = 0;
+                    ph ^= 1;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp < kMxEpiWarp0) {
         // ---- weight producers: group = stage slot, thread = weight row; four blocks (68 bytes) per stage ----
         const uint32_t p = (uint32_t)(tid - kMxProdWarp0 * 32), row = p & 127, grp = p >> 7;
-        const uint32_t slot = smem_u32(smem) + T::kRawOffset + grp * kMxRawSlot;
-        uint8_t* const slot_p = smem + T::kRawOffset + grp * kMxRawSlot;
-        // The pieces of all rows, dealt to the group's threads row by row (a warp's copy instruction covers five rows'
-        // runs of bytes): byte offset of the piece's row in a tile, and row and piece.
-        uint32_t f_row[kMxPieces], f_rp[kMxPieces];
-#pragma unroll
-        for (uint32_t i = 0; i < kMxPieces; ++i) {
-            const uint32_t idx = row + 128u * i, r = idx / kMxPieces;
-            f_row[i] = r * (uint32_t)row_bytes;
-            f_rp[i] = (r << 8) | (idx - r * kMxPieces);
-        }
-        // the group's next stage: item, stage of it, first byte of the tile's rows and of this thread's row
-        uint32_t w = blockIdx.x, m0 = 0;
+        // the group's next stage: item, stage of it, offset of this thread's row in the item's run of bytes
+        uint32_t w = blockIdx.x, row_off = 0;
         int s = (int)grp;
-        const uint8_t* expert = g.p.A;
-        auto locate = [&]() {  // normalise (w, s); past the last item nothing is read
-            while (w < n_items && s >= n_stages) {
-                s -= n_stages;
-                w += gridDim.x;
-            }
-            if (w < n_items) {
-                const uint32_t t = w / g.row_tiles;
-                m0 = (w - t * g.row_tiles) * kBM;
-                expert = g.p.A + (uint64_t)mx_tile(g.p, t).x * g.p.expert_stride;
-            }
+        auto locate = [&]() {
+            const uint32_t m0 = (w % g.row_tiles) * kBM;
+            row_off = min(row, g.p.M - 1 - m0) * (uint32_t)row_bytes;
         };
-        auto fetch = [&]() {
-            const uint8_t* first = expert + (uint64_t)m0 * row_bytes + (uint32_t)s * 68u;
-            const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(first) & 15u;
-            if (m0 + kBM <= g.p.M && first + (uint64_t)(kBM - 1) * row_bytes + kMxPieces * 16 <= g.p.A + g.p.a_bytes) {
-#pragma unroll
-                for (uint32_t i = 0; i < kMxPieces; ++i) {
-                    const uint32_t o = low + f_row[i], piece = f_rp[i] & 255u;
-                    if (piece < kMxPieces - 1 || (o & 15u) > 12u)  // 68 bytes from offset 12 end with the fifth piece
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + (f_rp[i] >> 8) * kMxRawRow + piece * 16),
-                                     "l"(first - low + ((o & ~15u) + piece * 16))
-                                     : "memory");
-                }
-            } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
-#pragma unroll 1
-                for (uint32_t i = 0; i < kMxPieces; ++i) {
-                    const uint32_t r = f_rp[i] >> 8, piece = f_rp[i] & 255u;
-                    const uint64_t o = (uint64_t)min(m0 + r, g.p.M - 1) * row_bytes + (uint32_t)s * 68u;
-                    const uint8_t* sp = expert + (o & ~(uint64_t)15) + piece * 16;
-                    const uint8_t* end = g.p.A + g.p.a_bytes;
-                    const uint32_t n = sp + 16 <= end ? 16u : (sp < end ? (uint32_t)(end - sp) : 0u);
-                    cp_async16_zfill(slot_p + r * kMxRawRow + piece * 16, n ? sp : g.p.A, n);
-                }
+        auto settle = [&]() {
+            if (s >= n_stages) {
+                do {
+                    s -= n_stages;
+                    w += gridDim.x;
+                } while (s >= n_stages && w < n_items);
+                locate();
             }
         };
         locate();
-        if (w < n_items) fetch();
+        settle();
         bool dead = false;
-        uint32_t use = 0;
+        uint32_t use = 0, slot = grp, slot_ph = 0;
+        static_assert(T::kRawSlots >= kMxStages);
         while (w < n_items) {
             const int blocks = (int)nb - 4 * s;  // of the stage: four or, at the end of a row, fewer
-            const uint32_t off = (uint32_t)(((uint64_t)min(m0 + row, g.p.M - 1) * row_bytes + (uint32_t)s * 68u) & 15u);
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            asm volatile("bar.sync %0, 128;" ::"r"(1u + grp) : "memory");
+            const uint32_t off = (row_off + (uint32_t)s * 68u) & 15u;
+            if (!dead) dead = !poll_or_fail(&bars->full_w[slot], slot_ph, bars, g.p.status, 147);
             // the row's 68 bytes: 8-byte reads from the offset rounded down to 8, then shifted to the first byte
             uint32_t v[20], wd[18];
-            const uint8_t* src = slot_p + row * kMxRawRow + (off & 8u);
+            const uint8_t* src = smem + T::kRawOffset + slot * kMxRawSlot + row * kMxRawRow + (off & 8u);
 #pragma unroll
             for (int k = 0; k < 10; ++k) {
                 const uint2 t = *reinterpret_cast<const uint2*>(src + 8 * k);
                 v[2 * k] = t.x;
                 v[2 * k + 1] = t.y;
             }
-            asm volatile("bar.sync %0, 128;" ::"r"(1u + grp) : "memory");
-            // the slot is read: the group's next stage flies while this one is repacked
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->empty_w[slot]);
+            slot += kMxStages;
+            if (slot >= T::kRawSlots) {
+                slot -= T::kRawSlots;
+                slot_ph ^= 1;
+            }
             s += kMxStages;
-            locate();
-            if (w < n_items) fetch();
+            settle();
             if (off & 4u) {
 #pragma unroll
                 for (int k = 0; k < 19; ++k) v[k] = v[k + 1];
@@ -377,7 +414,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ++i) {
             const uint32_t ab = i & 1;
             const uint32_t tt = w / g.row_tiles;
-            const uint4 tile = mx_tile(g.p, tt);
+            const uint4 tile = mx_tile(g.p, tiles, tt);
             const uint32_t m = (w - tt * g.row_tiles) * kBM + q * 32 + lane;
             if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.p.status, 145)) break;
             __syncwarp();
@@ -388,7 +425,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                 tmem_ld32(tmem + ((q * 32u) << 16) + ab * BN + c * 32, v);
                 // pair of column c*32 + lane: its output row starts at Y + token * y_token_stride + slot * M
                 const uint32_t idx = c * 32 + lane;
-                const uint32_t pair = idx >= tile.z ? 0u : (g.p.dense_n ? tile.y + idx : __ldg(&g.p.list[tile.y + idx]));
+                const uint32_t pair = idx >= tile.z ? 0u : (g.p.dense_n ? tile.y + idx : __ldg(&list[tile.y + idx]));
                 const uint32_t tok = pair / g.p.n_used;
                 const uint64_t at = (uint64_t)tok * g.p.y_token_stride + (uint64_t)(pair - tok * g.p.n_used) * g.p.M;
                 tmem_ld_wait();

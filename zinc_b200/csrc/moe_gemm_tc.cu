@@ -166,7 +166,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = bars->tmem_base;
+    const uint32_t tmem = warp_uniform(bars->tmem_base);
 
     if (warp == 0) {
         {  // ---- MMA issuer ----
@@ -177,7 +177,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                 // as many columns as the tile has pairs (N in steps of 16)
                 const Item it = item_of(g, w, nblk);
                 const int s0 = 4 * it.b0, s1 = min(n_stages, 4 * it.b1);
-                const uint32_t cols = (moe_tile(g, it.tile).z + 15u) & ~15u;
+                const uint32_t cols = warp_uniform((moe_tile(g, it.tile).z + 15u) & ~15u);
                 const uint32_t idesc = instr_desc<16>() + ((cols - 16u) >> 3 << 17);
                 ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.status, 121);
                 if (!ok) break;
@@ -259,12 +259,12 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
 #pragma unroll 1
                 for (int i = 0; i < kFetches; ++i) {
-                    if (f_dst[i] == 0xFFFFFFFFu) continue;
-                    const uint32_t r = f_dst[i] >> 20, piece = (f_dst[i] >> 16) & 15u;
+                    const uint32_t idx = (uint32_t)p + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
+                    if (r >= (uint32_t)kBM) break;
                     const uint64_t o = (uint64_t)min(c.m0 + r, g.M - 1) * row_bytes + (uint64_t)c.b * kBlock;
                     const uint8_t* s = c.expert + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t n = s + 16 <= g.a_end ? 16u : (s < g.a_end ? (uint32_t)(g.a_end - s) : 0u);
-                    cp_async16_zfill(smem_w + slot_idx * T::kRawBytes + (f_dst[i] & 0xFFFFu), n ? s : g.A, n);
+                    cp_async16_zfill(smem_w + slot_idx * T::kRawBytes + r * kBox + piece * 16, n ? s : g.A, n);
                 }
             }
         };

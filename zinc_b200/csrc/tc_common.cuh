@@ -211,6 +211,9 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
+// A value that all lanes of the warp hold, told to the compiler as such (a shuffle from lane 0): it then keeps to uniform
+// registers what the tensor-core instructions take from there, instead of moving it over for each of them.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
 __device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
