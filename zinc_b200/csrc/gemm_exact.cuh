@@ -784,21 +784,6 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
 }
 
-// Pairs the device holds at once; every kernel instantiation asks once per device.
-template <typename Kern>
-int x_max_pairs(Kern kern, cudaLaunchConfig_t cfg, std::atomic<int>* cache) {
-    int dev = 0, pairs = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && (pairs = cache[dev].load(std::memory_order_relaxed)) > 0) return pairs;
-    cfg.gridDim = dim3(2, 1, 1);
-    if (cudaOccupancyMaxActiveClusters(&pairs, kern, &cfg) != cudaSuccess || pairs < 1) {
-        cudaGetLastError();
-        return 0;
-    }
-    if (dev < 64) cache[dev].store(pairs, std::memory_order_relaxed);
-    return pairs;
-}
-
 template <int TYPE, int BN, bool kFetch>
 cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
     using T = XTile<TYPE, BN, kFetch>;
@@ -819,7 +804,7 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int pairs = x_max_pairs(kern, cfg, max_pairs);
+    const int pairs = max_pairs_of(kern, cfg, max_pairs);
     if (pairs < 1) return cudaErrorNotSupported;
     const uint32_t units = plan.n_tiles * plan.nblk;
     // whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds

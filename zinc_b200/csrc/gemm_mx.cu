@@ -36,7 +36,6 @@ namespace zc {
 namespace {
 
 constexpr int kMxStageK = 128;             // columns per stage: four MXFP4 blocks, one scale atom
-constexpr int kMxStages = 3;
 constexpr uint32_t kMxABytes = kBM * 128;  // 16 KB: 128 rows x 128 padded-FP4 bytes
 constexpr uint32_t kMxAtom = 512;          // scale bytes of 128 rows or tokens, four blocks
 // A row's 68 bytes of a stage in their 16-byte aligned superset: up to six pieces, rows 112 bytes apart (8-byte reads
@@ -45,18 +44,21 @@ constexpr uint32_t kMxPieces = 6, kMxRawRow = 112, kMxRawSlot = kBM * kMxRawRow;
 // Warps: 0 tensor memory + MMA issue, 1 loader, four that fetch raw weight bytes, then one group of four producer warps per stage slot (a thread
 // per weight row; group j always fills slot j, so the groups work on different stages at the same time), then four
 // epilogue warps.
+constexpr int kMxGroups = 3;               // of producer warps; group j fills every third stage
 constexpr int kMxFetchWarp0 = 2, kMxFetchWarps = 4;
-constexpr int kMxProdWarp0 = kMxFetchWarp0 + kMxFetchWarps, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxStages * kMxGroupWarps;
+constexpr int kMxProdWarp0 = kMxFetchWarp0 + kMxFetchWarps, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxGroups * kMxGroupWarps;
 constexpr int kMxThreads = (kMxEpiWarp0 + 4) * 32;
 
 template <int BN>
 struct MxTile {
-    static constexpr uint32_t kXBytes = BN * 128;
+    static constexpr uint32_t kXBytes = BN / 2 * 128;   // one term of the CTA's half of the tokens
+    // Stages: what hides a slot's turn-around (commit, TMA latency, repacking: some 2000 cycles against 500 of MMAs)
+    static constexpr int kStages = BN > 64 ? 4 : 6;
     static constexpr uint32_t kSfX = BN > 128 ? 2 * kMxAtom : kMxAtom;  // scale bytes of one term of a tile, four blocks
     // A | x_hi | x_lo | scales of A, x_hi, x_lo, padded to the 1024-byte alignment the swizzled tiles need
     static constexpr uint32_t kSfOffset = kMxABytes + 2 * kXBytes;
     static constexpr uint32_t kStageBytes = (kSfOffset + kMxAtom + 2 * kSfX + 1023u) & ~1023u;
-    static constexpr uint32_t kRawOffset = kMxStages * kStageBytes;
+    static constexpr uint32_t kRawOffset = kStages * kStageBytes;
     // raw slots: what is left, eight at most
     static constexpr uint32_t kAvail = 227u * 1024u - 1024 - 512 - kRawOffset;
     static constexpr uint32_t kRawSlots = kAvail / kMxRawSlot > 8 ? 8 : kAvail / kMxRawSlot;
@@ -65,24 +67,24 @@ struct MxTile {
     // tensor memory: two accumulators, then per stage the scale columns of A, x_hi, x_lo
     static constexpr uint32_t kSfCols = 4 + 2 * (kSfX / 128);
     static constexpr uint32_t kSfCol0 = 2 * BN;
-    static constexpr uint32_t kCols = kSfCol0 + kMxStages * kSfCols <= 128 ? 128 : kSfCol0 + kMxStages * kSfCols <= 256 ? 256 : 512;
-    static_assert(kSmemBytes <= 227u * 1024u && kSfCol0 + kMxStages * kSfCols <= 512);
+    static constexpr uint32_t kCols = kSfCol0 + kStages * kSfCols <= 128 ? 128 : kSfCol0 + kStages * kSfCols <= 256 ? 256 : 512;
+    static_assert(kSmemBytes <= 227u * 1024u && kSfCol0 + kStages * kSfCols <= 512);
 };
 
 struct MxBars {
-    uint64_t full[kMxStages];    // the slot's four producer warps + the loader's expect_tx
-    uint64_t empty[kMxStages];   // the issuing warp's commit
+    // the pair's, in its even CTA: full, accum_empty; commits arrive in both CTAs
+    uint64_t full[6];            // the stage's four producer warps of both CTAs + the loader's expect_tx
+    uint64_t empty[6];           // the issuing warp's commit
     uint64_t full_w[8];          // raw slots: a copy-completion arrival per fetch thread
     uint64_t empty_w[8];         // the four producer warps that read the slot
     uint64_t accum_full[2];
-    uint64_t accum_empty[2];     // one arrival per epilogue warp
+    uint64_t accum_empty[2];     // one arrival per epilogue warp of both CTAs
     uint32_t tmem_base;
     volatile uint32_t failed;
 };
 
 struct MxArgs {
     MxGemm p;
-    const uint8_t* sf;       // scale atoms: [tile][four blocks][x_hi, x_lo][kSfX]
     uint32_t rows, row_tiles;
 };
 
@@ -99,30 +101,24 @@ __device__ __forceinline__ uint64_t sf_desc(uint32_t saddr) {
     return ((uint64_t)hi << 32) | lo;
 }
 __device__ __forceinline__ void tmem_cp_sf(uint32_t tmem_col, uint64_t desc) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(desc) : "memory");
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(desc) : "memory");
 }
 
-// Instruction descriptor of the block-scaled MMA: A = E2M1, B = E4M3, both K-major, E8M0 scales, M = 128, N = cols,
+// Instruction descriptor of the block-scaled MMA: A = E2M1, B = E4M3, both K-major, E8M0 scales, M = 256, N = cols,
 // K = 32; sf: which byte of the scale words this step uses.
 __device__ __forceinline__ uint32_t mx_idesc(uint32_t cols, uint32_t sf) {
-    return (sf << 4) | (5u << 7) | (0u << 10) | ((cols >> 3) << 17) | (1u << 23) | ((uint32_t)(kBM >> 4) << 24) | (sf << 29);
+    return (sf << 4) | (5u << 7) | (0u << 10) | ((cols >> 3) << 17) | (1u << 23) | ((256u >> 4) << 24) | (sf << 29);
 }
 __device__ __forceinline__ void umma_mx(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
                                         uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
         : "memory");
 }
 
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(smem_dst)),
-                 "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
 // `bytes` (a multiple of 16) at the 16-byte aligned address src -> L2
 __device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
@@ -138,7 +134,7 @@ __device__ __forceinline__ void repack8(uint32_t q0, uint32_t q1, uint32_t& lo, 
 
 template <int BN>
 __global__ void __launch_bounds__(kMxThreads, 1)
-mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
+mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_sf, const MxArgs args) {
     // everything this kernel reads but the weights comes from the kernels before it
     chain_wait();
     const MxArgs& g = args;
@@ -157,10 +153,13 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
     const uint32_t nb = g.p.K >> 5;                        // blocks per row
     const int n_stages = (int)((nb + 3) >> 2);             // the last one may hold fewer than four blocks
     const uint64_t row_bytes = (uint64_t)nb * 17u;
+    const uint32_t rank = cluster_ctarank(), step = gridDim.x >> 1;
+    // The CTA's 128 rows of item w; a CTA wholly past M repeats the last ones (computed, dropped).
+    auto first_row = [&](uint32_t w) { return min(((w % g.row_tiles) * 2 + rank) * (uint32_t)kBM, (g.p.M - 1) & ~(kBM - 1u)); };
 
     if (tid == 0) {
-        for (int s = 0; s < kMxStages; ++s) {
-            mbar_init(&bars->full[s], kMxGroupWarps + 1);
+        for (int s = 0; s < T::kStages; ++s) {
+            mbar_init(&bars->full[s], 2 * kMxGroupWarps + 1);
             mbar_init(&bars->empty[s], 1);
         }
         for (uint32_t s = 0; s < T::kRawSlots; ++s) {
@@ -169,27 +168,28 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars->accum_full[s], 1);
-            mbar_init(&bars->accum_empty[s], 4);
+            mbar_init(&bars->accum_empty[s], 8);
         }
         bars->failed = 0;
         mbar_fence_init();
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
                      "r"(T::kCols)
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all();  // the peer's barriers exist before anything arrives on them
     tc_fence_after();
     const uint32_t tmem = warp_uniform(bars->tmem_base);
 
-    if (warp == 0) {
-        // ---- scale copies + MMA issuer (the converged warp walks, one elected lane issues) ----
+    if (warp == 0 && rank == 0) {
+        // ---- scale copies + MMA issuer of the pair (the converged warp walks, one elected lane issues) ----
         uint32_t st = 0, ph = 0, i = 0;
         bool ok = true;
-        for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++i) {
+        for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step, ++i) {
             const uint32_t ab = i & 1;
             // as many columns as the tile has tokens (N in steps of 16)
             const uint32_t cols = warp_uniform((mx_tile(g.p, tiles, w / g.row_tiles).z + 15u) & ~15u);
@@ -221,10 +221,10 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                         umma_mx(tmem + ab * BN, da + 2 * k, dh + 2 * k, mx_idesc(cols, k), sf_a, sf_hi, (s | k) ? 1u : 0u);
                         umma_mx(tmem + ab * BN, da + 2 * k, dh + T::kXBytes / 16 + 2 * k, mx_idesc(cols, k), sf_a, sf_lo, 1u);
                     }
-                    umma_commit(&bars->empty[st]);
-                    if (s + 1 == n_stages) umma_commit(&bars->accum_full[ab]);
+                    umma_commit_pair(&bars->empty[st]);
+                    if (s + 1 == n_stages) umma_commit_pair(&bars->accum_full[ab]);
                 }
-                if (++st == kMxStages) {
+                if (++st == T::kStages) {
                     st = 0;
                     ph ^= 1;
                 }
@@ -239,38 +239,40 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             auto locate = [&](uint32_t w) {
                 run_bytes = 0;
                 if (w >= n_items) return;
-                const uint32_t t = w / g.row_tiles, m0 = (w - t * g.row_tiles) * kBM;
-                run = g.p.A + (uint64_t)mx_tile(g.p, tiles, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
+                const uint32_t m0 = first_row(w);
+                run = g.p.A + (uint64_t)mx_tile(g.p, tiles, w / g.row_tiles).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
                 run_bytes = ((uint64_t)min((uint32_t)kBM, g.p.M - m0) * row_bytes) & ~(uint64_t)15;
             };
             auto prefetch = [&](int s) {
                 const uint64_t at = (uint64_t)s * (kBM * 68u);
                 if (at < run_bytes) bulk_prefetch(run + at, (uint32_t)min((uint64_t)(kBM * 68u), run_bytes - at));
             };
-            locate(blockIdx.x);
+            locate(blockIdx.x >> 1);
             for (int s = 0; s < n_stages; ++s) prefetch(s);
-            for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
+            for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
                 const uint32_t tt = w / g.row_tiles;
-                const uint32_t row0 = mx_tile(g.p, tiles, tt).y;
-                locate(w + gridDim.x);
-                const uint8_t* sf = g.sf + (size_t)tt * n_stages * 2 * T::kSfX;
+                const uint4 tile = mx_tile(g.p, tiles, tt);
+                const uint32_t row0 = tile.y + rank * (((tile.z + 15u) & ~15u) >> 1);  // the CTA's half of the columns
+                locate(w + step);
+                const uint32_t sf = tt * (uint32_t)n_stages;
                 for (int s = 0; s < n_stages; ++s) {
                     ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 143);
                     if (!ok) break;
                     uint8_t* stage = smem + st * T::kStageBytes;
-                    mbar_expect_tx(&bars->full[st], 2 * T::kXBytes + 2 * T::kSfX);
-                    tma_load_2d(stage + kMxABytes, &tmap_x, s * kMxStageK, (int)row0, &bars->full[st]);
-                    tma_load_2d(stage + kMxABytes + T::kXBytes, &tmap_x, s * kMxStageK, (int)(g.rows + row0), &bars->full[st]);
-                    bulk_load(stage + T::kSfOffset + kMxAtom, sf + (size_t)s * 2 * T::kSfX, 2 * T::kSfX, &bars->full[st]);
+                    if (rank == 0) mbar_expect_tx(&bars->full[st], 2 * (2 * T::kXBytes + 2 * T::kSfX));  // of both CTAs
+                    const uint32_t full = leader_addr(&bars->full[st]);
+                    tma_load_2d_pair(stage + kMxABytes, &tmap_x, s * kMxStageK, (int)row0, full);
+                    tma_load_2d_pair(stage + kMxABytes + T::kXBytes, &tmap_x, s * kMxStageK, (int)(g.rows + row0), full);
+                    tma_load_2d_pair(stage + T::kSfOffset + kMxAtom, &tmap_sf, 0, (int)((sf + s) * (T::kSfX / 128)), full);
                     prefetch(s);
-                    if (++st == kMxStages) {
+                    if (++st == T::kStages) {
                         st = 0;
                         ph ^= 1;
                     }
                 }
             }
         }
-    } else if (warp < kMxProdWarp0) {
+    } else if (warp >= kMxFetchWarp0 && warp < kMxProdWarp0) {
         // ---- fetchers: the raw bytes of a stage, the 16-byte pieces of all rows dealt to the 128 threads row by row (a
         // warp's copy instruction covers five rows' runs of bytes). Each copy reports to the slot's barrier by itself. ----
         const uint32_t p = (uint32_t)(tid - kMxFetchWarp0 * 32);
@@ -285,9 +287,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         const uint8_t* const end = g.p.A + g.p.a_bytes;
         uint32_t slot = 0, ph = 1;
         bool ok = true;
-        for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-            const uint32_t t = w / g.row_tiles, m0 = (w - t * g.row_tiles) * kBM;
-            const uint8_t* rows = g.p.A + (uint64_t)mx_tile(g.p, tiles, t).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
+        for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
+            const uint32_t m0 = first_row(w);
+            const uint8_t* rows = g.p.A + (uint64_t)mx_tile(g.p, tiles, w / g.row_tiles).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
             // whether every piece of every stage can be read
             const bool inside = m0 + kBM <= g.p.M && rows + (uint64_t)kBM * row_bytes + kMxPieces * 16 <= end;
             for (int s = 0; s < n_stages; ++s) {
@@ -324,21 +326,18 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-    } else if (warp < kMxEpiWarp0) {
+    } else if (warp >= kMxProdWarp0 && warp < kMxEpiWarp0) {
         // ---- weight producers: group = stage slot, thread = weight row; four blocks (68 bytes) per stage ----
         const uint32_t p = (uint32_t)(tid - kMxProdWarp0 * 32), row = p & 127, grp = p >> 7;
         // the group's next stage: item, stage of it, offset of this thread's row in the item's run of bytes
-        uint32_t w = blockIdx.x, row_off = 0;
+        uint32_t w = blockIdx.x >> 1, row_off = 0;
         int s = (int)grp;
-        auto locate = [&]() {
-            const uint32_t m0 = (w % g.row_tiles) * kBM;
-            row_off = min(row, g.p.M - 1 - m0) * (uint32_t)row_bytes;
-        };
+        auto locate = [&]() { row_off = min(row, g.p.M - 1 - first_row(w)) * (uint32_t)row_bytes; };
         auto settle = [&]() {
             if (s >= n_stages) {
                 do {
                     s -= n_stages;
-                    w += gridDim.x;
+                    w += step;
                 } while (s >= n_stages && w < n_items);
                 locate();
             }
@@ -346,8 +345,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
         locate();
         settle();
         bool dead = false;
-        uint32_t use = 0, slot = grp, slot_ph = 0;
-        static_assert(T::kRawSlots >= kMxStages);
+        uint32_t st = grp, ph = 1, slot = grp, slot_ph = 0;
+        static_assert(T::kRawSlots >= kMxGroups && T::kStages >= kMxGroups);
         while (w < n_items) {
             const int blocks = (int)nb - 4 * s;  // of the stage: four or, at the end of a row, fewer
             const uint32_t off = (row_off + (uint32_t)s * 68u) & 15u;
@@ -363,12 +362,12 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->empty_w[slot]);
-            slot += kMxStages;
+            slot += kMxGroups;
             if (slot >= T::kRawSlots) {
                 slot -= T::kRawSlots;
                 slot_ph ^= 1;
             }
-            s += kMxStages;
+            s += kMxGroups;
             settle();
             if (off & 4u) {
 #pragma unroll
@@ -376,10 +375,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             }
 #pragma unroll
             for (int k = 0; k < 18; ++k) wd[k] = __funnelshift_r(v[k], v[k + 1], (off & 3u) * 8u);
-            if (!dead) dead = !poll_or_fail(&bars->empty[grp], (use & 1) ^ 1, bars, g.p.status, 144);
-            ++use;
+            if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 144);
             if (!dead) {
-                uint8_t* stage = smem + grp * T::kStageBytes;
+                uint8_t* stage = smem + st * T::kStageBytes;
                 uint8_t* rowp = stage + row * 128;
                 const uint32_t sw = row & 7;
                 uint32_t sf = 0;
@@ -405,17 +403,22 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
                 fence_proxy_async();
             }
             __syncwarp();
-            if (lane == 0 && !dead) mbar_arrive(&bars->full[grp]);
+            if (lane == 0 && !dead) mbar_arrive_cluster(leader_addr(&bars->full[st]));
+            st += kMxGroups;
+            if (st >= T::kStages) {
+                st -= T::kStages;
+                ph ^= 1;
+            }
         }
-    } else {
+    } else if (warp >= kMxEpiWarp0) {
         // ---- epilogue: lane = weight row, column = pair of the tile ----
         const uint32_t q = warp & 3;
         uint32_t i = 0;
-        for (uint32_t w = blockIdx.x; w < n_items; w += gridDim.x, ++i) {
+        for (uint32_t w = blockIdx.x >> 1; w < n_items; w += step, ++i) {
             const uint32_t ab = i & 1;
             const uint32_t tt = w / g.row_tiles;
             const uint4 tile = mx_tile(g.p, tiles, tt);
-            const uint32_t m = (w - tt * g.row_tiles) * kBM + q * 32 + lane;
+            const uint32_t m = ((w - tt * g.row_tiles) * 2 + rank) * kBM + q * 32 + lane;
             if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.p.status, 145)) break;
             __syncwarp();
             tc_fence_after();
@@ -437,14 +440,15 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const MxArgs args) {
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->accum_empty[ab]);
+            if (lane == 0) mbar_arrive_cluster(leader_addr(&bars->accum_empty[ab]));
         }
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols) : "memory");
     }
 }
 
@@ -551,11 +555,29 @@ __global__ void __launch_bounds__(256) mx_terms_kernel(const MxTerms a) {
 }
 
 template <int BN>
-cudaError_t launch_gemm(const CUtensorMap& map, const MxArgs& g, uint32_t grid, cudaStream_t s) {
+cudaError_t launch_gemm(const CUtensorMap& map, const CUtensorMap& sf, const MxArgs& g, uint64_t items, cudaStream_t s) {
     auto kern = mx_gemm_kernel<BN>;
     static std::atomic<uint64_t> attr_done{0};  // per device ordinal
+    static std::atomic<int> max_pairs[64];
     if (cudaError_t e = ensure_dynamic_smem(kern, (int)MxTile<BN>::kSmemBytes, attr_done); e != cudaSuccess) return e;
-    return launch_chained(kern, dim3(grid), dim3(kMxThreads), MxTile<BN>::kSmemBytes, s, map, g);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kMxThreads, 1, 1);
+    cfg.dynamicSmemBytes = MxTile<BN>::kSmemBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int pairs = max_pairs_of(kern, cfg, max_pairs);
+    if (pairs < 1) return cudaErrorNotSupported;
+    cfg.numAttrs = 2;
+    cfg.gridDim = dim3(2 * (uint32_t)(items < (uint64_t)pairs ? items : (uint64_t)pairs), 1, 1);
+    return cudaLaunchKernelEx(&cfg, kern, map, sf, g);
 }
 
 struct MxLayout {
@@ -598,18 +620,25 @@ cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint3
     CUtensorMap map;
     const cuuint64_t dims[2] = {p.K, 2 * rows};
     const cuuint64_t strides[1] = {p.K};
-    const cuuint32_t box[2] = {(cuuint32_t)kMxStageK, bn};
+    const cuuint32_t box[2] = {(cuuint32_t)kMxStageK, bn / 2};
     const cuuint32_t estr[2] = {1, 1};
     if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(ws), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorNotSupported;
-    const MxArgs g{p, ws + l.sf, (uint32_t)rows, (p.M + kBM - 1) / kBM};
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // the scale atoms as rows of 256 bytes: a stage's two terms are one box
+    CUtensorMap sf;
+    const uint32_t atoms = (p.K + 127) / 128;
+    const cuuint64_t sdims[2] = {256, tiles * atoms * (l.sf_x / 128)};
+    const cuuint64_t sstrides[1] = {256};
+    const cuuint32_t sbox[2] = {256, l.sf_x / 128};
+    if (enc(&sf, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(ws) + l.sf, sdims, sstrides, sbox, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorNotSupported;
+    const MxArgs g{p, (uint32_t)rows, (p.M + 255) / 256};
     const uint64_t items = tiles * g.row_tiles;
-    const uint32_t grid = (uint32_t)(items < (uint64_t)sms ? items : (uint64_t)sms);
-    return bn == 32 ? launch_gemm<32>(map, g, grid, s) : bn == 64 ? launch_gemm<64>(map, g, grid, s) : launch_gemm<160>(map, g, grid, s);
+    return bn == 32   ? launch_gemm<32>(map, sf, g, items, s)
+           : bn == 64 ? launch_gemm<64>(map, sf, g, items, s) : launch_gemm<160>(map, sf, g, items, s);
 }
 
 uint64_t mul_mm_mx_workspace_bytes(uint32_t N, uint32_t K) {

@@ -427,6 +427,21 @@ __device__ __forceinline__ void dequant_group_mxfp4(const uint8_t* p, uint32_t o
     }
 }
 
+// Pairs of CTAs the device holds at once; every kernel instantiation asks once per device.
+template <typename Kern>
+int max_pairs_of(Kern kern, cudaLaunchConfig_t cfg, std::atomic<int>* cache) {
+    int dev = 0, pairs = 0;
+    cudaGetDevice(&dev);
+    if (dev < 64 && (pairs = cache[dev].load(std::memory_order_relaxed)) > 0) return pairs;
+    cfg.gridDim = dim3(2, 1, 1);
+    if (cudaOccupancyMaxActiveClusters(&pairs, kern, &cfg) != cudaSuccess || pairs < 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (dev < 64) cache[dev].store(pairs, std::memory_order_relaxed);
+    return pairs;
+}
+
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
