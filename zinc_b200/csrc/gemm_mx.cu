@@ -38,14 +38,16 @@ namespace {
 constexpr int kMxStageK = 128;             // columns per stage: four MXFP4 blocks, one scale atom
 constexpr uint32_t kMxABytes = kBM * 128;  // 16 KB: 128 rows x 128 padded-FP4 bytes
 constexpr uint32_t kMxAtom = 512;          // scale bytes of 128 rows or tokens, four blocks
-// A row's 68 bytes of a stage in their 16-byte aligned superset: up to six pieces, rows 112 bytes apart (8-byte reads
-// of 16 rows meet two per bank pair, at 96 bytes four).
-constexpr uint32_t kMxPieces = 6, kMxRawRow = 112, kMxRawSlot = kBM * kMxRawRow;
-// Warps: 0 tensor memory + MMA issue, 1 loader, four that fetch raw weight bytes, then one group of four producer warps per stage slot (a thread
-// per weight row; group j always fills slot j, so the groups work on different stages at the same time), then four
-// epilogue warps.
 constexpr int kMxGroups = 3;               // of producer warps; group j fills every third stage
-constexpr int kMxFetchWarp0 = 2, kMxFetchWarps = 4;
+// Raw bytes come three stages (204 bytes of a row) at a time, in their 16-byte aligned superset of up to 14 pieces: the
+// load unit takes a copy instruction apart by the lines it meets, some 27 cycles where a run of bytes was one stage's 68.
+// Rows 240 bytes apart: 8-byte reads of 16 rows meet two per bank pair.
+constexpr uint32_t kMxPieces = 14, kMxRawRow = 240, kMxRawSlot = kBM * kMxRawRow, kMxUnit = kMxGroups;
+// Warps: 0 tensor memory + MMA issue; 1 loader of x_hi, 2 of the raw weight bytes, 3 of x_lo, 4 of the scale atoms (one
+// thread each: an issue costs its thread some 100 cycles, and a stage has six); four that copy raw bytes where TMA cannot;
+// then three groups of four producer warps (a thread per weight row; the groups work on different stages at the same
+// time), then four epilogue warps.
+constexpr int kMxFetchWarp0 = 5, kMxFetchWarps = 4;
 constexpr int kMxProdWarp0 = kMxFetchWarp0 + kMxFetchWarps, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxGroups * kMxGroupWarps;
 constexpr int kMxThreads = (kMxEpiWarp0 + 4) * 32;
 
@@ -59,9 +61,9 @@ struct MxTile {
     static constexpr uint32_t kSfOffset = kMxABytes + 2 * kXBytes;
     static constexpr uint32_t kStageBytes = (kSfOffset + kMxAtom + 2 * kSfX + 1023u) & ~1023u;
     static constexpr uint32_t kRawOffset = kStages * kStageBytes;
-    // raw slots: what is left, eight at most
     static constexpr uint32_t kAvail = 227u * 1024u - 1024 - 512 - kRawOffset;
-    static constexpr uint32_t kRawSlots = kAvail / kMxRawSlot > 8 ? 8 : kAvail / kMxRawSlot;
+    static constexpr uint32_t kRawSlots = kAvail / kMxRawSlot > 4 ? 4 : kAvail / kMxRawSlot;
+    static_assert(kRawSlots >= 2);
     static constexpr uint32_t kBarOffset = kRawOffset + kRawSlots * kMxRawSlot;
     static constexpr uint32_t kSmemBytes = kBarOffset + 512 + 1024;
     // tensor memory: two accumulators, then per stage the scale columns of A, x_hi, x_lo
@@ -75,8 +77,8 @@ struct MxBars {
     // the pair's, in its even CTA: full, accum_empty; commits arrive in both CTAs
     uint64_t full[6];            // the stage's four producer warps of both CTAs + the loader's expect_tx
     uint64_t empty[6];           // the issuing warp's commit
-    uint64_t full_w[8];          // raw slots: a copy-completion arrival per fetch thread
-    uint64_t empty_w[8];         // the four producer warps that read the slot
+    uint64_t full_w[4];          // raw slots: a copy-completion arrival per fetch thread
+    uint64_t empty_w[4];         // all producer warps
     uint64_t accum_full[2];
     uint64_t accum_empty[2];     // one arrival per epilogue warp of both CTAs
     uint32_t tmem_base;
@@ -132,9 +134,20 @@ __device__ __forceinline__ void repack8(uint32_t q0, uint32_t q1, uint32_t& lo, 
     hi = ((even >> 4) & 0x0F0F0F0Fu) | (odd & 0xF0F0F0F0u);
 }
 
-template <int BN>
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// kTma: the raw bytes come by TMA. Eight rows are a multiple of 16 bytes (K % 64 == 0), so the matrix is a tensor of
+// eight-row groups, and the segments of the rows c, c + 8, c + 16, .. of a tile are a box: eight boxes of 16 rows a unit,
+// kept in the raw slot by c.
+template <int BN, bool kTma>
 __global__ void __launch_bounds__(kMxThreads, 1)
-mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_sf, const MxArgs args) {
+mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_sf,
+               const __grid_constant__ CUtensorMap tmap_w, const MxArgs args) {
     // everything this kernel reads but the weights comes from the kernels before it
     chain_wait();
     const MxArgs& g = args;
@@ -163,8 +176,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             mbar_init(&bars->empty[s], 1);
         }
         for (uint32_t s = 0; s < T::kRawSlots; ++s) {
-            mbar_init(&bars->full_w[s], kMxFetchWarps * 32);
-            mbar_init(&bars->empty_w[s], kMxGroupWarps);
+            mbar_init(&bars->full_w[s], kTma ? 4 : kMxFetchWarps * 32);
+            mbar_init(&bars->empty_w[s], kMxGroups * kMxGroupWarps);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars->accum_full[s], 1);
@@ -230,8 +243,30 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
             }
         }
-    } else if (warp == 1) {
-        if (lane == 0) {  // ---- loader of the activation terms and their scale atoms; the next item's weights to L2 ----
+    } else if (warp == 1 || warp == 3) {
+        if (lane == 0) {  // ---- loaders of the activation terms ----
+            uint32_t st = 0, ph = 1;
+            bool ok = true;
+            const uint32_t term = warp == 1 ? 0u : 1u;
+            for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
+                const uint4 tile = mx_tile(g.p, tiles, w / g.row_tiles);
+                // the CTA's half of the columns
+                const int y = (int)(term * g.rows + tile.y + rank * (((tile.z + 15u) & ~15u) >> 1));
+                for (int s = 0; s < n_stages; ++s) {
+                    ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 143);
+                    if (!ok) break;
+                    if (rank == 0 && term == 0) mbar_expect_tx(&bars->full[st], 2 * (2 * T::kXBytes + 2 * T::kSfX));  // of both CTAs
+                    tma_load_2d_pair(smem + st * T::kStageBytes + kMxABytes + term * T::kXBytes, &tmap_x, s * kMxStageK, y,
+                                     leader_addr(&bars->full[st]));
+                    if (++st == T::kStages) {
+                        st = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 4) {
+        if (lane == 0) {  // ---- loader of the activations' scale atoms; the next item's weights to L2 ----
             uint32_t st = 0, ph = 1;
             bool ok = true;
             const uint8_t* run = nullptr;  // the item's weight rows: one run of bytes, its end rounded down to 16
@@ -250,20 +285,13 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             locate(blockIdx.x >> 1);
             for (int s = 0; s < n_stages; ++s) prefetch(s);
             for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
-                const uint32_t tt = w / g.row_tiles;
-                const uint4 tile = mx_tile(g.p, tiles, tt);
-                const uint32_t row0 = tile.y + rank * (((tile.z + 15u) & ~15u) >> 1);  // the CTA's half of the columns
+                const uint32_t sf = w / g.row_tiles * (uint32_t)n_stages;
                 locate(w + step);
-                const uint32_t sf = tt * (uint32_t)n_stages;
                 for (int s = 0; s < n_stages; ++s) {
-                    ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 143);
+                    ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 148);
                     if (!ok) break;
-                    uint8_t* stage = smem + st * T::kStageBytes;
-                    if (rank == 0) mbar_expect_tx(&bars->full[st], 2 * (2 * T::kXBytes + 2 * T::kSfX));  // of both CTAs
-                    const uint32_t full = leader_addr(&bars->full[st]);
-                    tma_load_2d_pair(stage + kMxABytes, &tmap_x, s * kMxStageK, (int)row0, full);
-                    tma_load_2d_pair(stage + kMxABytes + T::kXBytes, &tmap_x, s * kMxStageK, (int)(g.rows + row0), full);
-                    tma_load_2d_pair(stage + T::kSfOffset + kMxAtom, &tmap_sf, 0, (int)((sf + s) * (T::kSfX / 128)), full);
+                    tma_load_2d_pair(smem + st * T::kStageBytes + T::kSfOffset + kMxAtom, &tmap_sf, 0, (int)((sf + s) * (T::kSfX / 128)),
+                                     leader_addr(&bars->full[st]));
                     prefetch(s);
                     if (++st == T::kStages) {
                         st = 0;
@@ -272,51 +300,51 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
             }
         }
-    } else if (warp >= kMxFetchWarp0 && warp < kMxProdWarp0) {
-        // ---- fetchers: the raw bytes of a stage, the 16-byte pieces of all rows dealt to the 128 threads row by row (a
-        // warp's copy instruction covers five rows' runs of bytes). Each copy reports to the slot's barrier by itself. ----
-        const uint32_t p = (uint32_t)(tid - kMxFetchWarp0 * 32);
-        uint32_t f_row[kMxPieces], f_piece[kMxPieces], f_dst[kMxPieces];  // byte offset of the piece's row in a tile, ..
+    } else if (kTma && (warp == 2 || (warp >= kMxFetchWarp0 && warp < kMxFetchWarp0 + 3))) {
+        if (lane == 0) {  // ---- loaders of the raw bytes, two boxes each ----
+            const uint32_t c0 = warp == 2 ? 0u : 2u * (uint32_t)(warp - kMxFetchWarp0 + 1);
+            uint32_t slot = 0, ph = 1;
+            bool ok = true;
+            for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
+                const int expert = (int)mx_tile(g.p, tiles, w / g.row_tiles).x, group = (int)(first_row(w) / 8);
+                for (int s = 0; s < n_stages; s += (int)kMxUnit) {
+                    ok = poll_or_fail(&bars->empty_w[slot], ph, bars, g.p.status, 146);
+                    if (!ok) break;
+                    uint8_t* const raw = smem + T::kRawOffset + slot * kMxRawSlot;
+                    mbar_expect_tx(&bars->full_w[slot], kMxRawSlot / 4);
 #pragma unroll
-        for (uint32_t i = 0; i < kMxPieces; ++i) {
-            const uint32_t idx = p + 128u * i, r = idx / kMxPieces;
-            f_row[i] = r * (uint32_t)row_bytes;
-            f_piece[i] = (idx - r * kMxPieces) * 16;
-            f_dst[i] = r * kMxRawRow + f_piece[i];
+                    for (uint32_t c = c0; c < c0 + 2; ++c)
+                        tma_load_3d(raw + c * (kMxRawSlot / 8), &tmap_w, (int)((c * (uint32_t)row_bytes + (uint32_t)s * 68u) & ~15u), group,
+                                    expert, &bars->full_w[slot]);
+                    if (++slot == T::kRawSlots) {
+                        slot = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
         }
+    } else if (!kTma && warp >= kMxFetchWarp0 && warp < kMxProdWarp0) {
+        // ---- fetchers: the 16-byte pieces of all rows dealt to the threads row by row; rows past M repeat the last one
+        // (computed, dropped); bytes past the matrix are zeros, not read ----
         const uint8_t* const end = g.p.A + g.p.a_bytes;
         uint32_t slot = 0, ph = 1;
         bool ok = true;
         for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
             const uint32_t m0 = first_row(w);
             const uint8_t* rows = g.p.A + (uint64_t)mx_tile(g.p, tiles, w / g.row_tiles).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
-            // whether every piece of every stage can be read
-            const bool inside = m0 + kBM <= g.p.M && rows + (uint64_t)kBM * row_bytes + kMxPieces * 16 <= end;
-            for (int s = 0; s < n_stages; ++s) {
-                ok = poll_or_fail(&bars->empty_w[slot], ph, bars, g.p.status, 146);
+            for (int s = 0; s < n_stages; s += (int)kMxUnit) {
+                ok = poll_or_fail(&bars->empty_w[slot], ph, bars, g.p.status, 149);
                 if (!ok) break;
                 uint8_t* const raw = smem + T::kRawOffset + slot * kMxRawSlot;
-                if (inside) {
-                    const uint8_t* first = rows + (uint32_t)s * 68u;
-                    const uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(first) & 15u;
-                    first -= low;
-#pragma unroll
-                    for (uint32_t i = 0; i < kMxPieces; ++i) {
-                        const uint32_t o = low + f_row[i];
-                        if (f_piece[i] < (kMxPieces - 1) * 16 || (o & 15u) > 12u)  // 68 bytes from offset 12 end with the fifth piece
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(raw) + f_dst[i]),
-                                         "l"(first + ((o & ~15u) + f_piece[i]))
-                                         : "memory");
-                    }
-                } else {  // rows past M repeat the last one (computed, dropped); bytes past the stack are zeros, not read
-#pragma unroll 1
-                    for (uint32_t i = 0; i < kMxPieces; ++i) {
-                        const uint32_t idx = p + 128u * i, r = idx / kMxPieces, piece = idx - r * kMxPieces;
-                        const uint32_t o = min(r, g.p.M - 1 - m0) * (uint32_t)row_bytes + (uint32_t)s * 68u;
-                        const uint8_t* sp = rows + (o & ~15u) + piece * 16;
-                        const uint32_t n = sp + 16 <= end ? 16u : (sp < end ? (uint32_t)(end - sp) : 0u);
-                        cp_async16_zfill(raw + r * kMxRawRow + piece * 16, n ? sp : g.p.A, n);
-                    }
+                const uint32_t need = 68u * (uint32_t)min((int)kMxUnit, n_stages - s);
+#pragma unroll 2
+                for (uint32_t idx = (uint32_t)tid - kMxFetchWarp0 * 32; idx < kBM * kMxPieces; idx += kMxFetchWarps * 32) {
+                    const uint32_t r = idx / kMxPieces, piece = (idx - r * kMxPieces) * 16;
+                    const uint32_t o = min(r, g.p.M - 1 - m0) * (uint32_t)row_bytes + (uint32_t)s * 68u;
+                    if (piece >= (o & 15u) + need) continue;
+                    const uint8_t* sp = rows + (o & ~15u) + piece;
+                    const uint32_t n = sp + 16 <= end ? 16u : (sp < end ? (uint32_t)(end - sp) : 0u);
+                    cp_async16_zfill(raw + r * kMxRawRow + piece, n ? sp : g.p.A, n);
                 }
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bars->full_w[slot])) : "memory");
                 if (++slot == T::kRawSlots) {
@@ -328,47 +356,41 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (warp >= kMxProdWarp0 && warp < kMxEpiWarp0) {
         // ---- weight producers: group = stage slot, thread = weight row; four blocks (68 bytes) per stage ----
-        const uint32_t p = (uint32_t)(tid - kMxProdWarp0 * 32), row = p & 127, grp = p >> 7;
-        // the group's next stage: item, stage of it, offset of this thread's row in the item's run of bytes
-        uint32_t w = blockIdx.x >> 1, row_off = 0;
-        int s = (int)grp;
-        auto locate = [&]() { row_off = min(row, g.p.M - 1 - first_row(w)) * (uint32_t)row_bytes; };
-        auto settle = [&]() {
-            if (s >= n_stages) {
-                do {
-                    s -= n_stages;
-                    w += step;
-                } while (s >= n_stages && w < n_items);
-                locate();
-            }
-        };
-        locate();
-        settle();
+        const uint32_t p = (uint32_t)(tid - kMxProdWarp0 * 32) & 127u, grp = (uint32_t)(warp - kMxProdWarp0) / kMxGroupWarps;
+        // kTma: eight lanes take eight different c (distinct swizzles in the stage) of eight different groups (distinct banks
+        // in the raw slot)
+        const uint32_t row = kTma ? ((((p & 7u) + (p >> 3)) & 15u) << 3) | (p & 7u) : p;
+        const uint32_t raw_at = kTma ? (row & 7u) * (kMxRawSlot / 8) + (row >> 3) * kMxRawRow : row * kMxRawRow;
+        // Every group meets every unit and takes one of its stages, the one that is its turn among all stages (the last
+        // unit of a row may hold none for it).
         bool dead = false;
-        uint32_t st = grp, ph = 1, slot = grp, slot_ph = 0;
-        static_assert(T::kRawSlots >= kMxGroups && T::kStages >= kMxGroups);
-        while (w < n_items) {
+        uint32_t st = grp, ph = 1, slot = 0, slot_ph = 0, turn = grp;
+        for (uint32_t w = blockIdx.x >> 1; w < n_items; w += step) {
+          const uint32_t row_off = (kTma ? row & 7u : min(row, g.p.M - 1 - first_row(w))) * (uint32_t)row_bytes;
+          for (int u = 0; u < n_stages; u += (int)kMxUnit) {
+            const int s = u + (int)turn;
             const int blocks = (int)nb - 4 * s;  // of the stage: four or, at the end of a row, fewer
-            const uint32_t off = (row_off + (uint32_t)s * 68u) & 15u;
+            const uint32_t off = ((row_off + (uint32_t)u * 68u) & 15u) + turn * 68u;
             if (!dead) dead = !poll_or_fail(&bars->full_w[slot], slot_ph, bars, g.p.status, 147);
             // the row's 68 bytes: 8-byte reads from the offset rounded down to 8, then shifted to the first byte
             uint32_t v[20], wd[18];
-            const uint8_t* src = smem + T::kRawOffset + slot * kMxRawSlot + row * kMxRawRow + (off & 8u);
+            const uint8_t* src = smem + T::kRawOffset + slot * kMxRawSlot + raw_at + (off & ~7u);
 #pragma unroll
             for (int k = 0; k < 10; ++k) {
                 const uint2 t = *reinterpret_cast<const uint2*>(src + 8 * k);
                 v[2 * k] = t.x;
                 v[2 * k + 1] = t.y;
             }
+            // the reads are done, not only under way, when the slot is given back: with copies that came back faster (TMA), a
+            // release right behind the reads let the next bytes overtake them
+            __threadfence_block();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->empty_w[slot]);
-            slot += kMxGroups;
-            if (slot >= T::kRawSlots) {
-                slot -= T::kRawSlots;
+            if (++slot == T::kRawSlots) {
+                slot = 0;
                 slot_ph ^= 1;
             }
-            s += kMxGroups;
-            settle();
+            if (s >= n_stages) continue;
             if (off & 4u) {
 #pragma unroll
                 for (int k = 0; k < 19; ++k) v[k] = v[k + 1];
@@ -409,6 +431,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 st -= T::kStages;
                 ph ^= 1;
             }
+          }
+          turn = (turn + 2 * (uint32_t)n_stages) % kMxGroups;  // minus the item's stages
         }
     } else if (warp >= kMxEpiWarp0) {
         // ---- epilogue: lane = weight row, column = pair of the tile ----
@@ -554,9 +578,10 @@ __global__ void __launch_bounds__(256) mx_terms_kernel(const MxTerms a) {
     }
 }
 
-template <int BN>
-cudaError_t launch_gemm(const CUtensorMap& map, const CUtensorMap& sf, const MxArgs& g, uint64_t items, cudaStream_t s) {
-    auto kern = mx_gemm_kernel<BN>;
+template <int BN, bool kTma>
+cudaError_t launch_gemm(const CUtensorMap& map, const CUtensorMap& sf, const CUtensorMap& w, const MxArgs& g, uint64_t items,
+                        cudaStream_t s) {
+    auto kern = mx_gemm_kernel<BN, kTma>;
     static std::atomic<uint64_t> attr_done{0};  // per device ordinal
     static std::atomic<int> max_pairs[64];
     if (cudaError_t e = ensure_dynamic_smem(kern, (int)MxTile<BN>::kSmemBytes, attr_done); e != cudaSuccess) return e;
@@ -577,7 +602,7 @@ cudaError_t launch_gemm(const CUtensorMap& map, const CUtensorMap& sf, const MxA
     if (pairs < 1) return cudaErrorNotSupported;
     cfg.numAttrs = 2;
     cfg.gridDim = dim3(2 * (uint32_t)(items < (uint64_t)pairs ? items : (uint64_t)pairs), 1, 1);
-    return cudaLaunchKernelEx(&cfg, kern, map, sf, g);
+    return cudaLaunchKernelEx(&cfg, kern, map, sf, w, g);
 }
 
 struct MxLayout {
@@ -637,8 +662,23 @@ cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint3
         return cudaErrorNotSupported;
     const MxArgs g{p, (uint32_t)rows, (p.M + 255) / 256};
     const uint64_t items = tiles * g.row_tiles;
-    return bn == 32   ? launch_gemm<32>(map, sf, g, items, s)
-           : bn == 64 ? launch_gemm<64>(map, sf, g, items, s) : launch_gemm<160>(map, sf, g, items, s);
+    // eight-row groups of whole 16-byte multiples, none of them reaching past the matrix
+    const bool tma = p.K % 64 == 0 && p.M % 8 == 0;
+    CUtensorMap w = map;
+    if (tma) {
+        const cuuint64_t group = (cuuint64_t)(p.K / 32) * 17 * 8;
+        const cuuint64_t wdims[3] = {group, p.M / 8, p.dense_n ? 1u : p.n_experts};
+        const cuuint64_t wstrides[2] = {group, p.dense_n ? group * (p.M / 8) : p.expert_stride};
+        const cuuint32_t wbox[3] = {kMxRawRow, 16, 1};
+        const cuuint32_t wstr[3] = {1, 1, 1};
+        if (enc(&w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(p.A), wdims, wstrides, wbox, wstr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorNotSupported;
+        return bn == 32   ? launch_gemm<32, true>(map, sf, w, g, items, s)
+               : bn == 64 ? launch_gemm<64, true>(map, sf, w, g, items, s) : launch_gemm<160, true>(map, sf, w, g, items, s);
+    }
+    return bn == 32   ? launch_gemm<32, false>(map, sf, w, g, items, s)
+           : bn == 64 ? launch_gemm<64, false>(map, sf, w, g, items, s) : launch_gemm<160, false>(map, sf, w, g, items, s);
 }
 
 uint64_t mul_mm_mx_workspace_bytes(uint32_t N, uint32_t K) {

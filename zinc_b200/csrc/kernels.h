@@ -204,7 +204,7 @@ struct MxGemm {
     const uint32_t* header;       // grouped: as the grouped GEMM's tables
     const uint4* tiles;
     const uint32_t* list;
-    uint32_t M, K, n_used, y_token_stride;
+    uint32_t M, K, n_experts, n_used, y_token_stride;
     uint32_t dense_n, dense_tile; // > 0: plain GEMM over dense_n tokens in tiles of dense_tile
     uint32_t* status;
 };

@@ -602,7 +602,7 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
     if (mx) {  // the weights as they are, the activations as two FP8 terms
         uint8_t* terms = base + l.xp;
         e = launch_mx_terms(X, false, n_tokens, K, x_token_stride, n_used, where, 0, n_pairs, l.max_tiles, bn, terms, s);
-        MxGemm p{A, a_bytes, expert_stride, Y, header, tiles, list, M, K, n_used, y_token_stride, 0u, 0u, status};
+        MxGemm p{A, a_bytes, expert_stride, Y, header, tiles, list, M, K, n_experts, n_used, y_token_stride, 0u, 0u, status};
         if (e == cudaSuccess) e = launch_mx_gemm(p, n_pairs, l.max_tiles, bn, terms, s);
         if (e == cudaSuccess && A2) {
             p.A = A2;
