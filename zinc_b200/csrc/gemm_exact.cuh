@@ -588,8 +588,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         h0 = *reinterpret_cast<const uint4*>(wp + 16);
                         h1 = *reinterpret_cast<const uint4*>(wp + 32);
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                    release_after(hd.x ^ c0.x ^ c1.x ^ h0.y ^ h1.y, &bars->empty_w[sw], lane);
                     const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
                     const float d = __low2float(dd), dmin = __high2float(dd);
                     // the block's scale is d; where dmin is far above it (and there are mins at all), dmin / 2^15, so that
@@ -657,8 +656,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         sc[i] = __float2half2_rn(live && diff < 60 ? __uint_as_float((uint32_t)(127 + 14 - diff) << 23) : 0.f);
                         if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                    release_after(q[0][0] ^ q[0][3] ^ q[1][0] ^ q[1][3], &bars->empty_w[sw], lane);
                     if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
                     x_deq_mx(q[0], sc[0], 0, stage, row);
                     x_deq_mx(q[1], sc[1], 4, stage, row);

@@ -12,16 +12,19 @@
 //
 //   1. mx_terms_kernel   X -> x_hi, x_lo (bytes [rows][K]) and their scale bytes in the 512-byte atoms the tensor
 //                        core reads (128 tokens x 4 blocks: byte (t % 32) * 16 + (t / 32) * 4 + block), per tile
-//   2. mx_gemm_kernel    persistent CTAs over (up to BN tokens of an expert or of the only matrix, 128 weight rows)
-//                        items; per 128-column stage: the weight stage (16 KB, K-major, 128-byte swizzle) and its 512
-//                        scale bytes written by the slot's 128 producer threads (one per row) from raw bytes that
-//                        four warps fetch ahead (made by the producers themselves, the copies took a third
-//                        of their time), x_hi / x_lo tiles by TMA, their scale atoms by a bulk copy;
+//   2. mx_gemm_kernel    persistent pairs of CTAs (cta_group::2) over (up to BN tokens of an expert or of the only matrix,
+//                        256 weight rows) items: a CTA has 128 of the rows and half of the tokens. Per 128-column stage:
+//                        the weight stage (16 KB, K-major, 128-byte swizzle) and its 512 scale bytes written by 128
+//                        producer threads (one per row) from raw bytes; x_hi / x_lo tiles and their scale atoms by TMA;
 //                        one warp copies the scale atoms into tensor memory (tcgen05.cp) and issues eight MMAs (four
 //                        32-column steps x two terms, as wide as the tile has tokens); two accumulators let the
-//                        epilogue of an item overlap the next item's MMAs. The 128 rows of an item are one run of
-//                        bytes, so the loader has the next item's run brought to L2 chunk by chunk meanwhile: shared
-//                        memory has room for one raw stage per slot only, too little to cover DRAM's latency.
+//                        epilogue of an item overlap the next item's MMAs.
+// What bounds it: the issuing warp's twelve tensor-core instructions a stage (420 cycles, and some 200 of barrier polls)
+// with few tokens, the turn-around of four stages with 160. Measured, down projection of 32 experts 2880 x 2880: 64 tokens,
+// top 4, 99 us with the bf16 tiles, 62 here; 1024 tokens 135 and 96. What it took: CTA pairs (half the activation bytes per
+// SM, and an issue serves twice the rows), a loader thread per stream (a TMA issue costs its thread 150 cycles), raw bytes
+// by TMA three stages at a time (copied by warps they kept the shared-memory pipe from the producers: 1060 cycles to
+// repack a stage instead of 550). Bringing the next item's weights to L2 ahead cost 5 %: TMA serves that too.
 // Every mbarrier wait is bounded; a wait that gives up records {1, site}, raises the CTA's flag, and every role
 // drains to the common exit where tensor memory is released.
 //
@@ -43,9 +46,9 @@ constexpr int kMxGroups = 3;               // of producer warps; group j fills e
 // load unit takes a copy instruction apart by the lines it meets, some 27 cycles where a run of bytes was one stage's 68.
 // Rows 240 bytes apart: 8-byte reads of 16 rows meet two per bank pair.
 constexpr uint32_t kMxPieces = 14, kMxRawRow = 240, kMxRawSlot = kBM * kMxRawRow, kMxUnit = kMxGroups;
-// Warps: 0 tensor memory + MMA issue; 1 loader of x_hi, 2 of the raw weight bytes, 3 of x_lo, 4 of the scale atoms (one
-// thread each: an issue costs its thread some 100 cycles, and a stage has six); four that copy raw bytes where TMA cannot;
-// then three groups of four producer warps (a thread per weight row; the groups work on different stages at the same
+// Warps: 0 tensor memory + MMA issue; 1 loader of x_hi, 3 of x_lo, 4 of the scale atoms, 2 and 5..7 of the raw
+// weight bytes (one thread each: an issue costs its thread some 150 cycles); or, where TMA cannot fetch the
+// raw bytes, 5..8 copy them. Then three groups of four producer warps (a thread per weight row; the groups work on different stages at the same
 // time), then four epilogue warps.
 constexpr int kMxFetchWarp0 = 5, kMxFetchWarps = 4;
 constexpr int kMxProdWarp0 = kMxFetchWarp0 + kMxFetchWarps, kMxGroupWarps = 4, kMxEpiWarp0 = kMxProdWarp0 + kMxGroups * kMxGroupWarps;
@@ -119,11 +122,6 @@ __device__ __forceinline__ void umma_mx(uint32_t tmem_d, uint64_t desc_a, uint64
         "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
         : "memory");
-}
-
-// `bytes` (a multiple of 16) at the 16-byte aligned address src -> L2
-__device__ __forceinline__ void bulk_prefetch(const void* src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
 // Eight nibble bytes of a block (two words) -> the four bytes of the low nibbles and of the high nibbles, two
@@ -266,33 +264,16 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             }
         }
     } else if (warp == 4) {
-        if (lane == 0) {  // ---- loader of the activations' scale atoms; the next item's weights to L2 ----
+        if (lane == 0) {  // ---- loader of the activations' scale atoms ----
             uint32_t st = 0, ph = 1;
             bool ok = true;
-            const uint8_t* run = nullptr;  // the item's weight rows: one run of bytes, its end rounded down to 16
-            uint64_t run_bytes = 0;
-            auto locate = [&](uint32_t w) {
-                run_bytes = 0;
-                if (w >= n_items) return;
-                const uint32_t m0 = first_row(w);
-                run = g.p.A + (uint64_t)mx_tile(g.p, tiles, w / g.row_tiles).x * g.p.expert_stride + (uint64_t)m0 * row_bytes;
-                run_bytes = ((uint64_t)min((uint32_t)kBM, g.p.M - m0) * row_bytes) & ~(uint64_t)15;
-            };
-            auto prefetch = [&](int s) {
-                const uint64_t at = (uint64_t)s * (kBM * 68u);
-                if (at < run_bytes) bulk_prefetch(run + at, (uint32_t)min((uint64_t)(kBM * 68u), run_bytes - at));
-            };
-            locate(blockIdx.x >> 1);
-            for (int s = 0; s < n_stages; ++s) prefetch(s);
             for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
                 const uint32_t sf = w / g.row_tiles * (uint32_t)n_stages;
-                locate(w + step);
                 for (int s = 0; s < n_stages; ++s) {
                     ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 148);
                     if (!ok) break;
                     tma_load_2d_pair(smem + st * T::kStageBytes + T::kSfOffset + kMxAtom, &tmap_sf, 0, (int)((sf + s) * (T::kSfX / 128)),
                                      leader_addr(&bars->full[st]));
-                    prefetch(s);
                     if (++st == T::kStages) {
                         st = 0;
                         ph ^= 1;
@@ -381,11 +362,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 v[2 * k] = t.x;
                 v[2 * k + 1] = t.y;
             }
-            // the reads are done, not only under way, when the slot is given back: with copies that came back faster (TMA), a
-            // release right behind the reads let the next bytes overtake them
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->empty_w[slot]);
+            release_after((v[0] ^ v[2] ^ v[4]) ^ (v[6] ^ v[8] ^ v[10]) ^ (v[12] ^ v[14] ^ v[16]) ^ v[18], &bars->empty_w[slot], lane);
             if (++slot == T::kRawSlots) {
                 slot = 0;
                 slot_ph ^= 1;
@@ -469,6 +446,9 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
     tc_fence_before();
     __syncthreads();
+    if (bars->failed) {  // given up with copies in flight: let them land before the CTA's shared memory is another's
+        for (int i = 0; i < 100; ++i) __nanosleep(1000);
+    }
     cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
     if (warp == 0) {
         tc_fence_after();

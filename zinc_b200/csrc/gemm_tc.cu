@@ -239,8 +239,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                 const uint4 chdr = *reinterpret_cast<const uint4*>(wp);
                 const uint4 c0 = *reinterpret_cast<const uint4*>(wp + 16 + j * 32);
                 const uint4 c1 = *reinterpret_cast<const uint4*>(wp + 32 + j * 32);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                release_after(chdr.x ^ c0.x ^ c1.x, &bars->empty_w[sw], lane);
                 const __half2 dd = *reinterpret_cast<const __half2*>(&chdr.x);
                 const float d = __low2float(dd), dmin = __high2float(dd);
                 uint32_t s0, mn0, s1, mn1;
@@ -626,8 +625,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
                     const uint4 chdr = *reinterpret_cast<const uint4*>(wp);
                     const uint4 c0 = *reinterpret_cast<const uint4*>(wp + 16 + j * 32);
                     const uint4 c1 = *reinterpret_cast<const uint4*>(wp + 32 + j * 32);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
+                    release_after(chdr.x ^ c0.x ^ c1.x, &bars->empty_w[sw], lane);
                     const __half2 dd = *reinterpret_cast<const __half2*>(&chdr.x);
                     const float d = __low2float(dd), dmin = __high2float(dd);
                     uint32_t s0, mn0, s1, mn1;

@@ -260,6 +260,14 @@ __device__ __forceinline__ bool poll_or_fail(uint64_t* bar, uint32_t parity, B* 
     return false;
 }
 
+// Gives a slot of raw bytes back (a converged warp) once its reads are done, not only under way: `x` is made of a word of
+// every one of them, and the branch on it cannot be taken before they return. An arrival that merely followed the reads
+// was seen to overtake them: the refill by TMA then changed single rows, once in some thousand launches.
+__device__ __forceinline__ void release_after(uint32_t x, uint64_t* bar, int lane) {
+    if (__any_sync(0xFFFFFFFFu, x == 0x9E3779B9u)) __nanosleep(1);
+    if (lane == 0) mbar_arrive(bar);
+}
+
 __device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ __nv_bfloat162 bits_bf2(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
 
