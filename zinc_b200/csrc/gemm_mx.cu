@@ -202,8 +202,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         bool ok = true;
         for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step, ++i) {
             const uint32_t ab = i & 1;
-            // as many columns as the tile has tokens (N in steps of 16)
-            const uint32_t cols = warp_uniform((mx_tile(g.p, tiles, w / g.row_tiles).z + 15u) & ~15u);
+            // as many columns as the tile has tokens (N of a pair's MMA in steps of 32)
+            const uint32_t cols = warp_uniform((mx_tile(g.p, tiles, w / g.row_tiles).z + 31u) & ~31u);
             ok = warp_poll(smem_u32(&bars->accum_empty[ab]), ((i >> 1) & 1) ^ 1, bars, g.p.status, 141);
             if (!ok) break;
             tc_fence_after();
@@ -249,7 +249,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             for (uint32_t w = blockIdx.x >> 1; w < n_items && ok; w += step) {
                 const uint4 tile = mx_tile(g.p, tiles, w / g.row_tiles);
                 // the CTA's half of the columns
-                const int y = (int)(term * g.rows + tile.y + rank * (((tile.z + 15u) & ~15u) >> 1));
+                const int y = (int)(term * g.rows + tile.y + rank * (((tile.z + 31u) & ~31u) >> 1));
                 for (int s = 0; s < n_stages; ++s) {
                     ok = poll_or_fail(&bars->empty[st], ph, bars, g.p.status, 143);
                     if (!ok) break;

@@ -195,6 +195,21 @@ bool mul_mm_mx_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t
 cudaError_t launch_mul_mm_mx(const uint8_t* A, uint64_t a_bytes, const void* B, float* D, uint32_t M, uint32_t N,
                              uint32_t K, uint32_t stride_b, uint32_t stride_d, void* workspace, uint32_t* status,
                              cudaStream_t s, uint64_t* launches);
+// The grouped GEMM on CTA pairs (moe_gemm_pair.cu): Q4_K, and Q6_K with M % 8 == 0, K % 256 == 0; xp: the packed bf16
+// activations of the listed pairs; bn: 32, 64 or 128, the most pairs of a tile.
+struct MoePair {
+    const uint8_t* A;             // 16-byte aligned, as expert_stride
+    uint64_t expert_stride;
+    float* Y;
+    const uint32_t* header;
+    const uint4* tiles;
+    const uint32_t* list;
+    uint32_t M, K, n_experts, n_used, y_token_stride;
+    uint32_t* status;
+};
+bool moe_pair_eligible(uint32_t type, uint32_t M, uint32_t K);
+cudaError_t launch_moe_pair(uint32_t type, const MoePair& g, const void* xp, uint64_t n_pairs, uint64_t max_tiles, uint32_t bn,
+                            cudaStream_t s);
 // The block-scaled GEMM of one matrix or of an expert stack, over activations that launch_mx_terms has split into their two
 // FP8 terms in `ws` (mx_bytes() bytes, 256-byte aligned; bn: 32, 64 or 160, the most tokens of a tile).
 struct MxGemm {

@@ -536,7 +536,7 @@ cudaError_t launch_gemm(const CUtensorMap& map, const MoeGemmArgs& g, uint32_t m
 // should need one tile: the average count and two of its standard deviations (about its root each) have to fit.
 // 32 and 64 leave shared memory for a deeper ring of raw blocks; Q6_K's blocks are the largest, and beside 160 pairs only
 // two fit (12288 x 1280, 77 tokens in one tile: 16.3 us beside 160, 14.6 beside 128).
-uint32_t bn_most(uint32_t type) { return type == T_Q6_K ? 128u : 160u; }
+uint32_t bn_most(uint32_t type) { return type == T_MXFP4 ? 160u : 128u; }
 uint32_t pick_bn(uint32_t type, uint64_t n_pairs, uint32_t n_experts) {
     const double avg = (double)n_pairs / n_experts, most = avg + 2.0 * sqrt(avg);
     return most <= 32.0 ? 32u : most <= 64.0 ? 64u : bn_most(type);
@@ -544,18 +544,20 @@ uint32_t pick_bn(uint32_t type, uint64_t n_pairs, uint32_t n_experts) {
 
 template <int BN>
 cudaError_t launch_gemm_type(uint32_t type, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
-    if (type == T_Q4_K) return launch_gemm<T_Q4_K, BN>(map, g, max_items, s);
-    if (type == T_MXFP4) return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
-    if constexpr (BN == 160)
-        return cudaErrorNotSupported;
-    else
-        return launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+    if constexpr (BN == 160) {
+        return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
+    } else if constexpr (BN == 128) {
+        return type == T_Q4_K ? launch_gemm<T_Q4_K, BN>(map, g, max_items, s) : launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+    } else {
+        if (type == T_MXFP4) return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
+        return type == T_Q4_K ? launch_gemm<T_Q4_K, BN>(map, g, max_items, s) : launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+    }
 }
 cudaError_t launch_gemm_bn(uint32_t type, uint32_t bn, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
     switch (bn) {
         case 32: return launch_gemm_type<32>(type, map, g, max_items, s);
         case 64: return launch_gemm_type<64>(type, map, g, max_items, s);
-        case 128: return launch_gemm<T_Q6_K, 128>(map, g, max_items, s);
+        case 128: return launch_gemm_type<128>(type, map, g, max_items, s);
         default: return launch_gemm_type<160>(type, map, g, max_items, s);
     }
 }
@@ -617,6 +619,17 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
                        n_used, x_token_stride);
     if (e != cudaSuccess) return e;
 
+    if (moe_pair_eligible(type, M, K)) {
+        MoePair p{A, expert_stride, Y, header, tiles, list, M, K, n_experts, n_used, y_token_stride, status};
+        e = launch_moe_pair(type, p, xp, n_pairs, l.max_tiles, bn, s);
+        if (e == cudaSuccess && A2) {
+            p.A = A2;
+            p.Y = Y2;
+            e = launch_moe_pair(type, p, xp, n_pairs, l.max_tiles, bn, s);
+        }
+        if (e == cudaSuccess && launches) *launches += A2 ? 4 : 3;
+        return e;
+    }
     CUtensorMap map;
     const cuuint64_t dims[2] = {K, n_pairs};
     const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
