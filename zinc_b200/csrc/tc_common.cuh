@@ -305,28 +305,39 @@ __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& 
     }
 }
 
-// N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p: 16-byte reads (no bank
-// conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four rows per bank), then realigned.
-template <int N>
-__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N]) {
-    constexpr int V = (4 * N + 15 + 15) / 16;
-    uint32_t v[4 * V];
+// N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p, shifted right by `more` bits
+// (< 8) on top: 16-byte reads (no bank conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four
+// rows per bank), or, kWide false, 8-byte reads from the multiple of 8 (two rows per bank, a selection less), then
+// realigned.
+template <int N, bool kWide = true>
+__device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N], uint32_t more = 0) {
+    constexpr int V = kWide ? (4 * N + 15 + 15) / 16 * 4 : (4 * N + 7 + 7) / 8 * 2;
+    uint32_t v[V];
+    if constexpr (kWide) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
-        v[4 * i] = t.x;
-        v[4 * i + 1] = t.y;
-        v[4 * i + 2] = t.z;
-        v[4 * i + 3] = t.w;
-    }
-    const uint32_t sh = (off & 3u) * 8u;
-    if (off & 8u) {
+        for (int i = 0; i < V / 4; ++i) {
+            const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
+            v[4 * i] = t.x;
+            v[4 * i + 1] = t.y;
+            v[4 * i + 2] = t.z;
+            v[4 * i + 3] = t.w;
+        }
+        if (off & 8u) {
 #pragma unroll
-        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
+            for (int i = 0; i + 2 < V; ++i) v[i] = v[i + 2];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < V / 2; ++i) {
+            const uint2 t = *reinterpret_cast<const uint2*>(p + (off & 8u) + 8 * i);
+            v[2 * i] = t.x;
+            v[2 * i + 1] = t.y;
+        }
     }
+    const uint32_t sh = (off & 3u) * 8u + more;
     if (off & 4u) {
 #pragma unroll
-        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
+        for (int i = 0; i + 1 < V; ++i) v[i] = v[i + 1];
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
@@ -347,11 +358,12 @@ __device__ __forceinline__ void deq4_q6(uint32_t q4, __nv_bfloat162 dsc, uint32_
 // (g even) or high (g odd) nibbles of ql[64n .. 64n+64), bit pairs 4*(g&1) and 4*(g&1)+2 of
 // qh[32n .. 32n+32), scales[8n + 4*(g&1) .. +4) each covering 16 columns. The block starts `off` bytes (even, 0..14)
 // into the 16-byte aligned row at `p`.
+template <bool kWide = true>
 __device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, uint8_t* a_stage, int row) {
     const int n = g >> 1, hi = g & 1;
     uint32_t ql[16], qh[8];
-    lds_words<16>(p + 64 * n, off, ql);
-    lds_words<8>(p + 128 + 32 * n, off, qh);
+    lds_words<16, kWide>(p + 64 * n, off, ql, 4 * hi);  // the nibbles wanted are the low ones of their bytes
+    lds_words<8, kWide>(p + 128 + 32 * n, off, qh);
     const unsigned short* tail = reinterpret_cast<const unsigned short*>(p + off + 192);
     const uint32_t scw[1] = {(uint32_t)tail[4 * n + 2 * hi] | ((uint32_t)tail[4 * n + 2 * hi + 1] << 16)};
     const float d = __half2float(__ushort_as_half(tail[8]));
@@ -361,16 +373,16 @@ __device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off
     for (int c = 0; c < 8; ++c) {  // chunk c = columns 8c .. 8c+7 of the group; scale index c / 2
         const float sc = (float)(int)(int8_t)((scw[0] >> (8 * (c >> 1))) & 0xFFu);
         const __nv_bfloat162 dsc = __float2bfloat162_rn(d * sc);
+        const uint32_t turn = (uint32_t)(4 - 2 * (c >> 2) - 4 * hi) & 31u;  // the high bits' place in a byte -> bits 4 and 5
         uint4 o;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             // columns 8c+4e .. +3: ql byte index (c < 4 ? 0 : 32) + 8*(c&3) + 4e, qh byte index 8*(c&3) + 4e
             const uint32_t lw = ql[(c >> 2) * 8 + (c & 3) * 2 + e];
             const uint32_t hw = qh[(c & 3) * 2 + e];
-            const uint32_t nib = (lw >> (4 * hi)) & 0x0F0F0F0Fu;
-            const uint32_t top = ((hw >> (4 * hi + 2 * (c >> 2))) & 0x03030303u) << 4;
+            const uint32_t top = __funnelshift_l(hw, hw, turn) & 0x30303030u;
             uint32_t a, b;
-            deq4_q6(nib | top, dsc, a, b);
+            deq4_q6((lw & 0x0F0F0F0Fu) | top, dsc, a, b);
             if (e == 0) {
                 o.x = a;
                 o.y = b;
