@@ -27,24 +27,34 @@ constexpr int kPairThreads = (kPairEpiWarp0 + 4) * 32;
 
 template <int TYPE, int BN>
 struct PairTile {
-    static constexpr uint32_t kXBytes = BN / 2 * 128;  // 64 columns of the CTA's half of the pairs
-    static constexpr uint32_t kStageBytes = 2 * kABytes + 2 * kXBytes;
-    static constexpr int kStages = BN > 64 ? 3 : 4;
+    static constexpr uint32_t kXBytes = BN / 2 * 128;      // 64 columns of the CTA's half of the pairs
+    static constexpr uint32_t kStageBytes = 2 * kXBytes;
+    static constexpr int kStages = BN > 64 ? 4 : 6;
     static constexpr uint32_t kRawRow = TYPE == T_Q4_K ? 144 : 240;  // odd multiples of 16 (8 rows of 16-byte reads: all banks)
     static constexpr uint32_t kRawSlot = kBM * kRawRow;
     static constexpr uint32_t kRawOffset = kStages * kStageBytes;
-    static constexpr uint32_t kAvail = 227u * 1024u - 1024 - 512 - kRawOffset;
-    static constexpr uint32_t kRawSlots = kAvail / kRawSlot > 4 ? 4 : kAvail / kRawSlot;
+    static constexpr uint32_t kRawSlots = 4;
     static constexpr uint32_t kBarOffset = kRawOffset + kRawSlots * kRawSlot;
     static constexpr uint32_t kSmemBytes = kBarOffset + 512 + 1024;
-    static constexpr uint32_t kCols = 2 * BN;
-    static_assert(kRawSlots >= 2);
+    // tensor memory: two accumulators, then the stages' weights (two bf16 a column)
+    static constexpr uint32_t kACol0 = 2 * BN, kACols = 64;
+    static_assert(kSmemBytes <= 227u * 1024u && kACol0 + kStages * kACols <= 512);
 };
+
+// D[tmem] (+)= A[tmem] * B[smem desc]^T of a CTA pair, bf16 x bf16 -> f32, issued by one thread
+__device__ __forceinline__ void umma_bf16_pair_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 
 struct PairBars {
     // the pair's, in its even CTA: full, accum_empty; commits arrive in both CTAs
-    uint64_t full[4];   // the stage's eight producer warps of both CTAs + the loader's expect_tx
-    uint64_t empty[4];
+    uint64_t full[6];   // the stage's eight producer warps of both CTAs + the loader's expect_tx
+    uint64_t empty[6];
     uint64_t full_w[4], empty_w[4];  // raw slots: the loaders' expect_tx; the sixteen producer warps
     uint64_t accum_full[2], accum_empty[2];
     uint32_t tmem_base;
@@ -56,6 +66,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
+}
+
+// The weight row of a tile that lane l of tensor memory holds.
+template <int TYPE>
+__device__ __forceinline__ uint32_t pair_row(uint32_t l) {
+    return TYPE == T_Q4_K ? l : (l & 64u) + 8u * (l & 7u) + ((l >> 3) & 7u);
 }
 
 template <int TYPE, int BN>
@@ -98,7 +114,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                     "r"(T::kCols)
+                     "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -124,14 +140,12 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                 ok = warp_poll(smem_u32(&bars->full[st]), ph, bars, g.status, 162);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t da = smem_desc(smem_u32(smem) + st * T::kStageBytes);
+                const uint64_t dx = smem_desc(smem_u32(smem) + st * T::kStageBytes);
+                const uint32_t a = tmem + T::kACol0 + st * T::kACols;
                 if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {  // two tiles of 64 columns
-                        const uint64_t a = da + (k >> 2) * (kABytes / 16) + 2 * (k & 3);
-                        const uint64_t x = da + (2 * kABytes + (k >> 2) * T::kXBytes) / 16 + 2 * (k & 3);
-                        umma_bf16_pair(tmem + ab * BN, a, x, idesc, (uint32_t)(s | k));
-                    }
+                    for (int k = 0; k < 8; ++k)  // 16 columns a time; the activations are two tiles of 64
+                        umma_bf16_pair_ta(tmem + ab * BN, a + 8 * k, dx + (k >> 2) * (T::kXBytes / 16) + 2 * (k & 3), idesc, (uint32_t)(s | k));
                     umma_commit_pair(&bars->empty[st]);
                     if (s + 1 == 2 * nblk) umma_commit_pair(&bars->accum_full[ab]);
                 }
@@ -153,7 +167,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     ok = poll_or_fail(&bars->empty[st], ph, bars, g.status, 163);
                     if (!ok) break;
                     if (rank == 0 && half == 0) mbar_expect_tx(&bars->full[st], 4 * T::kXBytes);  // of both CTAs
-                    tma_load_2d_pair(smem + st * T::kStageBytes + 2 * kABytes + half * T::kXBytes, &tmap_x, s * 128 + (int)half * 64, y,
+                    tma_load_2d_pair(smem + st * T::kStageBytes + half * T::kXBytes, &tmap_x, s * 128 + (int)half * 64, y,
                                      leader_addr(&bars->full[st]));
                     if (++st == T::kStages) {
                         st = 0;
@@ -193,19 +207,25 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         }
     } else if (warp >= kPairProdWarp0 && warp < kPairEpiWarp0) {
         // ---- producers ----
-        const uint32_t p = (uint32_t)(tid - kPairProdWarp0 * 32) & 127u, q = (uint32_t)(warp - kPairProdWarp0) >> 2;
-        // Q6_K: eight lanes take eight different c (distinct swizzles in the stage) of eight different groups (distinct banks
-        // in the raw slot)
-        const uint32_t row = TYPE == T_Q4_K ? p : ((((p & 7u) + (p >> 3)) & 15u) << 3) | (p & 7u);
+        // A thread's row goes to its own lane of tensor memory. Q6_K: eight lanes take the same c of eight groups (distinct
+        // banks in the raw slot).
+        const uint32_t q = (uint32_t)(warp - kPairProdWarp0) >> 2, row = pair_row<TYPE>((uint32_t)((warp & 3) * 32 + lane));
         const uint32_t raw_at = TYPE == T_Q4_K ? row * T::kRawRow : (row & 7u) * (T::kRawSlot / 8) + (row >> 3) * T::kRawRow;
         const uint32_t row_off = (row & 7u) * row_bytes;  // eight rows are a multiple of 16 bytes
+        const uint32_t lane_col = tmem + (((uint32_t)(warp & 3) * 32u) << 16) + T::kACol0 + (q & 1u) * (T::kACols / 2);
         uint32_t st = q >> 1, ph = 1, slot = 0, slot_ph = 0;
         bool dead = false;
         for (uint32_t w = blockIdx.x >> 1; w < n_items; w += step) {
             for (int b = 0; b < nblk; ++b) {
                 if (!dead) dead = !poll_or_fail(&bars->full_w[slot], slot_ph, bars, g.status, 165);
                 const uint8_t* raw = smem + T::kRawOffset + slot * T::kRawSlot + raw_at;
-                uint8_t* tile = smem + st * T::kStageBytes + (q & 1u) * kABytes;
+                uint32_t o[32];
+                auto put = [&](int c, const uint4& v) {
+                    o[4 * c] = v.x;
+                    o[4 * c + 1] = v.y;
+                    o[4 * c + 2] = v.z;
+                    o[4 * c + 3] = v.w;
+                };
                 if constexpr (TYPE == T_Q4_K) {
                     const uint4 hd = *reinterpret_cast<const uint4*>(raw);
                     const uint4 c0 = *reinterpret_cast<const uint4*>(raw + 16 + q * 32);
@@ -216,15 +236,19 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     uint32_t s0, mn0, s1, mn1;
                     scale_min_k4(2 * q, hd.y, hd.z, hd.w, s0, mn0);
                     scale_min_k4(2 * q + 1, hd.y, hd.z, hd.w, s1, mn1);
-                    if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 166);
-                    if (!dead) dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1, tile, (int)row);
+                    dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1, put);
                 } else {
-                    if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 166);
-                    if (!dead) dequant_group_q6k(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, tile, (int)row);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->empty_w[slot]);
+                    dequant_group_q6k(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, put);
+                    release_after(o[3] ^ o[7] ^ o[11] ^ o[15] ^ o[19] ^ o[23] ^ o[27] ^ o[31], &bars->empty_w[slot], lane);
                 }
-                fence_proxy_async();
+                if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 166);
+                __syncwarp();
+                tc_fence_after();
+                if (!__any_sync(0xFFFFFFFFu, dead)) {
+                    tmem_st32(lane_col + st * T::kACols, o);
+                    tmem_st_wait();
+                }
+                tc_fence_before();
                 __syncwarp();
                 if (lane == 0 && !dead) mbar_arrive_cluster(leader_addr(&bars->full[st]));
                 st += 2;
@@ -245,7 +269,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         for (uint32_t w = blockIdx.x >> 1; w < n_items; w += step, ++i) {
             const uint32_t ab = i & 1, t = w / row_tiles;
             const uint4 tile = __ldg(&tiles[t]);
-            const uint32_t m = ((w - t * row_tiles) * 2 + rank) * kBM + q * 32 + lane;
+            const uint32_t m = ((w - t * row_tiles) * 2 + rank) * kBM + pair_row<TYPE>(q * 32 + lane);
             if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 167)) break;
             __syncwarp();
             tc_fence_after();
@@ -277,7 +301,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
 }
 

@@ -170,6 +170,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr)
         : "memory");
 }
+// .. and 32 columns into it
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+          "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+          "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
@@ -284,15 +297,13 @@ __device__ __forceinline__ void deq4(uint32_t nib, __nv_bfloat162 dsc, __nv_bflo
     o1 = bf2_bits(__hfma2(__hsub2(bits_bf2(p1), k136), dsc, c));
 }
 
-// One 64-column group of a Q4_K row: 32 bytes of nibbles -> 8 chunks of 8 bf16 written to the
-// swizzled row `row` of the stage at `a_stage`.
+// One 64-column group of a Q4_K row: 32 bytes of nibbles -> 8 chunks of 8 bf16, handed to put(chunk, words).
+template <typename Put>
 __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& q1, float d_sc_lo, float dm_lo,
-                                                  float d_sc_hi, float dm_hi, uint8_t* a_stage, int row) {
+                                                  float d_sc_hi, float dm_hi, Put put) {
     const __nv_bfloat162 s_lo = __float2bfloat162_rn(d_sc_lo), m_lo = __float2bfloat162_rn(8.f * d_sc_lo - dm_lo);
     const __nv_bfloat162 s_hi = __float2bfloat162_rn(d_sc_hi), m_hi = __float2bfloat162_rn(8.f * d_sc_hi - dm_hi);
     const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    uint8_t* rowp = a_stage + row * 128;
-    const int sw = row & 7;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {  // chunk c: bytes 8c..8c+7 -> low nibbles = columns 8c.., high = 32+8c..
         uint4 lo, hi;
@@ -300,44 +311,42 @@ __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& 
         deq4(w[2 * c + 1] & 0x0F0F0F0Fu, s_lo, m_lo, lo.z, lo.w);
         deq4((w[2 * c] >> 4) & 0x0F0F0F0Fu, s_hi, m_hi, hi.x, hi.y);
         deq4((w[2 * c + 1] >> 4) & 0x0F0F0F0Fu, s_hi, m_hi, hi.z, hi.w);
-        *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = lo;
-        *reinterpret_cast<uint4*>(rowp + (((c + 4) ^ sw) << 4)) = hi;
+        put(c, lo);
+        put(c + 4, hi);
     }
+}
+// .. to the swizzled row `row` of the stage at `a_stage`
+__device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& q1, float d_sc_lo, float dm_lo,
+                                                  float d_sc_hi, float dm_hi, uint8_t* a_stage, int row) {
+    uint8_t* rowp = a_stage + row * 128;
+    const int sw = row & 7;
+    dequant_group_q4k(q0, q1, d_sc_lo, dm_lo, d_sc_hi, dm_hi,
+                      [&](int c, const uint4& o) { *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = o; });
 }
 
 // N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p, shifted right by `more` bits
 // (< 8) on top: 16-byte reads (no bank conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four
-// rows per bank), or, kWide false, 8-byte reads from the multiple of 8 (two rows per bank, a selection less), then
-// realigned.
-template <int N, bool kWide = true>
+// rows per bank), then realigned.
+template <int N>
 __device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N], uint32_t more = 0) {
-    constexpr int V = kWide ? (4 * N + 15 + 15) / 16 * 4 : (4 * N + 7 + 7) / 8 * 2;
-    uint32_t v[V];
-    if constexpr (kWide) {
+    constexpr int V = (4 * N + 15 + 15) / 16;
+    uint32_t v[4 * V];
 #pragma unroll
-        for (int i = 0; i < V / 4; ++i) {
-            const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
-            v[4 * i] = t.x;
-            v[4 * i + 1] = t.y;
-            v[4 * i + 2] = t.z;
-            v[4 * i + 3] = t.w;
-        }
-        if (off & 8u) {
-#pragma unroll
-            for (int i = 0; i + 2 < V; ++i) v[i] = v[i + 2];
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < V / 2; ++i) {
-            const uint2 t = *reinterpret_cast<const uint2*>(p + (off & 8u) + 8 * i);
-            v[2 * i] = t.x;
-            v[2 * i + 1] = t.y;
-        }
+    for (int i = 0; i < V; ++i) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
+        v[4 * i] = t.x;
+        v[4 * i + 1] = t.y;
+        v[4 * i + 2] = t.z;
+        v[4 * i + 3] = t.w;
     }
     const uint32_t sh = (off & 3u) * 8u + more;
+    if (off & 8u) {
+#pragma unroll
+        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
+    }
     if (off & 4u) {
 #pragma unroll
-        for (int i = 0; i + 1 < V; ++i) v[i] = v[i + 1];
+        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
@@ -358,17 +367,15 @@ __device__ __forceinline__ void deq4_q6(uint32_t q4, __nv_bfloat162 dsc, uint32_
 // (g even) or high (g odd) nibbles of ql[64n .. 64n+64), bit pairs 4*(g&1) and 4*(g&1)+2 of
 // qh[32n .. 32n+32), scales[8n + 4*(g&1) .. +4) each covering 16 columns. The block starts `off` bytes (even, 0..14)
 // into the 16-byte aligned row at `p`.
-template <bool kWide = true>
-__device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, uint8_t* a_stage, int row) {
+template <typename Put>
+__device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, Put put) {
     const int n = g >> 1, hi = g & 1;
     uint32_t ql[16], qh[8];
-    lds_words<16, kWide>(p + 64 * n, off, ql, 4 * hi);  // the nibbles wanted are the low ones of their bytes
-    lds_words<8, kWide>(p + 128 + 32 * n, off, qh);
+    lds_words<16>(p + 64 * n, off, ql, 4 * hi);  // the nibbles wanted are the low ones of their bytes
+    lds_words<8>(p + 128 + 32 * n, off, qh);
     const unsigned short* tail = reinterpret_cast<const unsigned short*>(p + off + 192);
     const uint32_t scw[1] = {(uint32_t)tail[4 * n + 2 * hi] | ((uint32_t)tail[4 * n + 2 * hi + 1] << 16)};
     const float d = __half2float(__ushort_as_half(tail[8]));
-    uint8_t* rowp = a_stage + row * 128;
-    const int sw = row & 7;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {  // chunk c = columns 8c .. 8c+7 of the group; scale index c / 2
         const float sc = (float)(int)(int8_t)((scw[0] >> (8 * (c >> 1))) & 0xFFu);
@@ -391,8 +398,13 @@ __device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off
                 o.w = b;
             }
         }
-        *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = o;
+        put(c, o);
     }
+}
+__device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, uint8_t* a_stage, int row) {
+    uint8_t* rowp = a_stage + row * 128;
+    const int sw = row & 7;
+    dequant_group_q6k(p, off, g, [&](int c, const uint4& o) { *reinterpret_cast<uint4*>(rowp + ((c ^ sw) << 4)) = o; });
 }
 
 // Byte permute with the full selector semantics (bit 3 of a selector nibble replicates the sign bit of
