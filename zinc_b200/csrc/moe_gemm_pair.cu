@@ -238,7 +238,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     scale_min_k4(2 * q + 1, hd.y, hd.z, hd.w, s1, mn1);
                     dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1, put);
                 } else {
-                    dequant_group_q6k(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, put);
+                    dequant_group_q6k<4>(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, put);
                     release_after(o[3] ^ o[7] ^ o[11] ^ o[15] ^ o[19] ^ o[23] ^ o[27] ^ o[31], &bars->empty_w[slot], lane);
                 }
                 if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 166);
@@ -270,6 +270,13 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
             const uint32_t ab = i & 1, t = w / row_tiles;
             const uint4 tile = __ldg(&tiles[t]);
             const uint32_t m = ((w - t * row_tiles) * 2 + rank) * kBM + pair_row<TYPE>(q * 32 + lane);
+            // pair of column c*32 + lane: its output row starts at Y + token * y_token_stride + slot * M
+            auto place = [&](uint32_t c) {
+                const uint32_t idx = c * 32 + lane, pair = idx >= tile.z ? 0u : __ldg(&list[tile.y + idx]);
+                const uint32_t tok = pair / g.n_used;
+                return (uint64_t)tok * g.y_token_stride + (uint64_t)(pair - tok * g.n_used) * g.M;
+            };
+            uint64_t at = place(0);  // fetched while the accumulator is on its way
             if (!poll_or_fail(&bars->accum_full[ab], (i >> 1) & 1, bars, g.status, 167)) break;
             __syncwarp();
             tc_fence_after();
@@ -277,13 +284,11 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
             for (uint32_t c = 0; c * 32 < tile.z; ++c) {
                 uint32_t v[32];
                 tmem_ld32(tmem + ((q * 32u) << 16) + ab * BN + c * 32, v);
-                // pair of column c*32 + lane: its output row starts at Y + token * y_token_stride + slot * M
-                const uint32_t idx = c * 32 + lane, pair = idx >= tile.z ? 0u : __ldg(&list[tile.y + idx]);
-                const uint32_t tok = pair / g.n_used;
-                const uint64_t at = (uint64_t)tok * g.y_token_stride + (uint64_t)(pair - tok * g.n_used) * g.M;
+                if (c) at = place(c);
                 tmem_ld_wait();
 #pragma unroll
                 for (int jj = 0; jj < 32; ++jj) {
+                    if (jj % 8 == 0 && c * 32 + jj >= tile.z) break;
                     const uint64_t y = __shfl_sync(0xFFFFFFFFu, at, jj);
                     if (c * 32 + jj < tile.z && m < g.M) g.Y[y + m] = __uint_as_float(v[jj]);
                 }

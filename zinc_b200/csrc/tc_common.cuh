@@ -325,28 +325,37 @@ __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& 
 }
 
 // N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p, shifted right by `more` bits
-// (< 8) on top: 16-byte reads (no bank conflicts at odd-multiple-of-16 row strides, where 32-bit reads would meet four
-// rows per bank), then realigned.
-template <int N>
+// (< 8) on top, read kRead bytes at a time and realigned: 16 (no bank conflicts at odd-multiple-of-16 row strides, a
+// selection by every bit of the offset) or fewer (a selection less each, two or four rows to a bank).
+template <int N, int kRead = 16>
 __device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N], uint32_t more = 0) {
-    constexpr int V = (4 * N + 15 + 15) / 16;
-    uint32_t v[4 * V];
+    constexpr int V = kRead == 4 ? N + 1 : (4 * N + 2 * kRead - 2) / kRead * (kRead / 4);
+    uint32_t v[V];
+    const uint8_t* src = p + (off & 15u & ~(uint32_t)(kRead - 1));
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p + 16 * i);
-        v[4 * i] = t.x;
-        v[4 * i + 1] = t.y;
-        v[4 * i + 2] = t.z;
-        v[4 * i + 3] = t.w;
+    for (int i = 0; i < V; i += kRead / 4) {
+        if constexpr (kRead == 16) {
+            const uint4 t = *reinterpret_cast<const uint4*>(src + 4 * i);
+            v[i] = t.x;
+            v[i + 1] = t.y;
+            v[i + 2] = t.z;
+            v[i + 3] = t.w;
+        } else if constexpr (kRead == 8) {
+            const uint2 t = *reinterpret_cast<const uint2*>(src + 4 * i);
+            v[i] = t.x;
+            v[i + 1] = t.y;
+        } else {
+            v[i] = *reinterpret_cast<const uint32_t*>(src + 4 * i);
+        }
     }
     const uint32_t sh = (off & 3u) * 8u + more;
-    if (off & 8u) {
+    if (kRead > 8 && (off & 8u)) {
 #pragma unroll
-        for (int i = 0; i + 2 < 4 * V; ++i) v[i] = v[i + 2];
+        for (int i = 0; i + 2 < V; ++i) v[i] = v[i + 2];
     }
-    if (off & 4u) {
+    if (kRead > 4 && (off & 4u)) {
 #pragma unroll
-        for (int i = 0; i + 1 < 4 * V; ++i) v[i] = v[i + 1];
+        for (int i = 0; i + 1 < V; ++i) v[i] = v[i + 1];
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
@@ -367,12 +376,12 @@ __device__ __forceinline__ void deq4_q6(uint32_t q4, __nv_bfloat162 dsc, uint32_
 // (g even) or high (g odd) nibbles of ql[64n .. 64n+64), bit pairs 4*(g&1) and 4*(g&1)+2 of
 // qh[32n .. 32n+32), scales[8n + 4*(g&1) .. +4) each covering 16 columns. The block starts `off` bytes (even, 0..14)
 // into the 16-byte aligned row at `p`.
-template <typename Put>
+template <int kRead = 16, typename Put>
 __device__ __forceinline__ void dequant_group_q6k(const uint8_t* p, uint32_t off, int g, Put put) {
     const int n = g >> 1, hi = g & 1;
     uint32_t ql[16], qh[8];
-    lds_words<16>(p + 64 * n, off, ql, 4 * hi);  // the nibbles wanted are the low ones of their bytes
-    lds_words<8>(p + 128 + 32 * n, off, qh);
+    lds_words<16, kRead>(p + 64 * n, off, ql, 4 * hi);  // the nibbles wanted are the low ones of their bytes
+    lds_words<8, kRead>(p + 128 + 32 * n, off, qh);
     const unsigned short* tail = reinterpret_cast<const unsigned short*>(p + off + 192);
     const uint32_t scw[1] = {(uint32_t)tail[4 * n + 2 * hi] | ((uint32_t)tail[4 * n + 2 * hi + 1] << 16)};
     const float d = __half2float(__ushort_as_half(tail[8]));
