@@ -414,3 +414,37 @@ def test_o_proj_merge(gpu, oracle, t, M, K, n_heads, nc, sink):
     assert rel_l2(y[:M].cpu().numpy() - h0, want) <= 1e-4
     with pytest.raises(zb.InvalidArgument):
         dd.dispatchDmmvOprojMerge(t, dev(torch, w), dev(torch, buf), None, y, M, K, n_heads + 1, nc, 0, hd)
+
+
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K, zb.Q6_K, zb.Q8_0, zb.MXFP4], ids=IDS[:5])
+@pytest.mark.parametrize("M,blocks", [(7, 2), (33, 7), (130, 17), (1025, 3), (16001, 8)])
+def test_row_and_tall_shapes(gpu, oracle, t, M, blocks):
+    """Rows and blocks that fill neither a CTA of the row kernel nor its warps' rounds, added to y; and rows enough for the
+    streaming kernels' tall cut (half the warps along K, a last tile of one row). The bar: f32 sums of at most 4352 products
+    against f64, 2^-24 each in the worst case."""
+    torch, ctx, dd = gpu
+    K = max(zb.block_size(t), 128) * blocks
+    g = synth.rng(130, t * 1000 + M)
+    w = synth.quant_matrix(g, t, M, K)
+    x, y0 = synth.activations(g, K), synth.activations(g, M)
+    y = out_with_canary(torch, M)
+    y[:M] = dev(torch, y0)
+    dd.recordDispatch(t, dev(torch, w), dev(torch, x), y, M, K, acc_mode=1)
+    ctx.submit_and_wait()
+    assert canary_intact(y, M)
+    assert rel_l2(y[:M].cpu().numpy() - y0, oracle.dmmv_f64(w, t, M, K, x)) <= TOL
+
+
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q6_K, zb.MXFP4], ids=["q4_k", "q6_k", "mxfp4"])
+@pytest.mark.parametrize("M,K,cols", [(1300, 3840, 2), (1304, 3840, 2), (651, 5120, 3), (1302, 2560, 3)])
+def test_batch_few_columns(gpu, oracle, t, M, K, cols):
+    """Both sides of the lines between the small products' kernel, two streaming matvecs and the tensor cores."""
+    torch, ctx, dd = gpu
+    g = synth.rng(131, t * 1000 + M + cols)
+    w = synth.quant_matrix(g, t, M, K)
+    X = synth.activations(g, cols, K)
+    Y = out_with_canary(torch, cols * M)
+    dd.recordBatchDispatchPush(t, dev(torch, w), dev(torch, X), Y, M, K, 0, 0, 0, cols)
+    ctx.submit_and_wait()
+    assert canary_intact(Y, cols * M)
+    assert rel_l2(Y[:cols * M].cpu().numpy().reshape(cols, M), oracle.gemm_f64(w, t, M, K, X)) <= TOL

@@ -821,3 +821,61 @@ def test_moe_prefill_expert_parallel_ranks(gpu, world):
     finally:
         dd.setWorkspace(None)
     assert float(((total - want).norm() / want.norm()).item()) <= 1e-5
+
+
+@pytest.mark.parametrize("t,E,M,K,counts", [
+    (zb.Q4_K, 6, 257, 512, (1, 31, 32, 33, 0, 2)),         # tiles of 32: one pair, full, one more; two rows of the second CTA's
+    (zb.Q4_K, 3, 100, 256, (64, 65, 1)),                   # tiles of 64, one block, no row for the second CTA
+    (zb.Q4_K, 2, 520, 768, (128, 129)),                    # tiles of 128, an odd number of blocks
+    (zb.Q6_K, 6, 264, 256, (1, 31, 32, 33, 0, 2)),         # 210-byte rows in groups of eight
+    (zb.Q6_K, 2, 136, 768, (128, 129)),
+    (zb.Q6_K, 4, 132, 512, (3, 40, 0, 5)),                 # rows not a multiple of eight: the one-CTA kernel
+    (zb.MXFP4, 6, 264, 64, (1, 31, 32, 33, 0, 2)),         # half a scale atom
+    (zb.MXFP4, 3, 100, 512, (64, 65, 1)),                  # rows not a multiple of eight: copied by warps
+    (zb.MXFP4, 2, 520, 832, (160, 161)),                   # tiles of 160, a second atom of activation scales; 6.5 stages
+])
+def test_moe_grouped_tile_edges(gpu, oracle, t, E, M, K, counts):
+    """Pairs per expert at the edges of the tiles (32, 64, 128 or 160, in MMAs 32 wide), rows at those of the CTA pairs (128,
+    256), K at those of blocks and stages. The bar is the grouped tests': products of bf16-rounded operands."""
+    torch, ctx, dd = gpu
+    g = synth.rng(230, E * 1000 + M + K)
+    w, stride = stacked(g, t, E, M, K)
+    if stride % 16:
+        pytest.skip("expert stride not 16-byte aligned: the per-pair kernel serves it")
+    ids = g.permutation(np.repeat(np.arange(E), counts)).astype(np.uint32)
+    T = ids.size
+    X = synth.activations(g, T, K)
+    Y = out_with_canary(torch, T * M)
+    ws = torch.empty(dd.moeGroupedWorkspaceBytes(T, 1, K, E), dtype=torch.uint8, device="cuda")
+    dd.setWorkspace(ws)
+    try:
+        dd.recordMoeBatchedDispatch(t, dev(torch, w), dev(torch, X), Y, dev(torch, ids), M, K, stride, E, 1, T, K, M)
+        ctx.submit_and_wait()
+    finally:
+        dd.setWorkspace(None)
+    got = Y[:T * M].cpu().numpy().reshape(T, M)
+    want = oracle.moe_dmmv_f64(w, t, M, K, stride, ids, K, X)
+    assert canary_intact(Y, T * M)
+    assert rel_l2(got, want) <= TOL_TC
+    assert max(rel_l2(got[i], want[i]) for i in range(T)) <= 2e-2
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 5), (32, 32), (33, 32), (256, 32), (257, 8), (64, 33)])
+def test_router_selection_ties(gpu, oracle, n, k):
+    """Selection by ranks (up to 256 experts and 32 picks) and beyond it, with logits that tie: the lower index first."""
+    torch, ctx, dd = gpu
+    k = min(k, n)
+    K = 64
+    W = np.zeros((n, K), np.float32)
+    W[:, 0] = (np.arange(n) * 7 % 5).astype(np.float32)  # few distinct logits
+    x = np.zeros(K, np.float32)
+    x[0] = 1.0
+    lg = out_with_canary(torch, n)
+    rt = torch.full((2 * k + 8,), 0x7ABCDEF0, dtype=torch.int32, device="cuda")
+    dd.dispatchMoeRouterTopk(dev(torch, x), dev(torch, W.reshape(-1)), lg, rt, n, K, k, rule=zb.ROUTE_TOPK_THEN_SOFTMAX)
+    ctx.submit_and_wait()
+    ids, wt = oracle.topk_softmax_weight(W[:, 0].copy(), k)
+    r = rt[:2 * k].cpu().numpy().view(np.uint32)
+    assert np.array_equal(r[:k], ids)
+    assert np.max(np.abs(r[k:].view(np.float32) - wt)) <= 1e-6
+    assert bool((rt[2 * k:] == 0x7ABCDEF0).all().item())

@@ -374,11 +374,15 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
     const bool pair = F::kMost <= 16 && a.nblk * F::kCols <= 4096;
     const uint32_t most = pair ? 8u : kSeg == 3 ? 16u : F::kMost;
-    const uint32_t per = (a.nblk + most - 1) / most;
+    uint32_t per = (a.nblk + most - 1) / most;
+    // Tall matrices (several tiles per CTA either way): half as many warps along K, as long as all warps find work, and
+    // fewer meetings: Q4_K 65536 x 4096 29.6 -> 27.7 us, Q6_K 151936 x 4096 114.8 -> 109.1.
+    const bool tall = kSeg == 0 && a.M >= 16000 && (a.nblk + 2 * per - 1) / (2 * per) * 4 >= most;
+    if (tall) per *= 2;
     a.n_wk = (a.nblk + per - 1) / per;
     a.n_wr = most / a.n_wk;
     if (a.n_wr > 4) a.n_wr = 4;
-    a.round = a.n_wr == 3 ? 6 : 4;
+    a.round = a.n_wr == 3 ? 6 : tall ? 8 : 4;
     warps = a.n_wk * a.n_wr;
     const uint32_t per_sm = pair ? 2u : 1u, room = pair ? kSliceSmem2 : kSliceSmem1;
     const uint32_t fixed = 128u + 2u * a.round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
