@@ -415,8 +415,8 @@ uint64_t zc_moe_grouped_workspace_bytes(uint32_t n_tokens, uint32_t n_experts_us
  * is the bf16 value exactly, written into `workspace` (zc_mul_mm_workspace_bytes(type, N, K) bytes, 256-byte
  * aligned, caller-owned) by a small kernel before the GEMM. N >= 64 tokens, K >= 128 and a multiple of 32; A and
  * B 16-byte aligned, stride_b a multiple of 8; offsets in elements of B and D as in zc_mul_mm. Results equal
- * zc_mul_mm's to the rounding of the f32 accumulation. As measured it is not yet faster than zc_mul_mm's route
- * (weights dequantised to bf16 tiles), which therefore stays the default. */
+ * zc_mul_mm's to the rounding of the f32 accumulation. It is faster than zc_mul_mm's route (weights dequantised to
+ * bf16 tiles) from about a thousand tokens. */
 uint64_t zc_mul_mm_workspace_bytes(uint32_t type, uint32_t N, uint32_t K);
 int32_t zc_mul_mm_block_scaled(zc_ctx* ctx, uint32_t type,
                                const void* A, uint64_t a_size, const void* B, uint64_t b_size,
@@ -549,12 +549,11 @@ int32_t zc_dmmv_push(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size,
 
 /* ---- matvec without a context and without any allocation ----------------------------------------
  * No counterpart in the reference (its dispatch layer always owns descriptor pools and buffers).
- * The streaming Q4_K matvec of zc_dmmv, y (+)= W x, with its split-K scratch in a __device__
- * array that is part of the library image (1048576 bytes: 4096 worker warps x 32 partial sums,
- * each stored with a tag word) instead of scratch a context allocated. For hosts that cannot let
+ * The streaming Q4_K matvec of zc_dmmv, y (+)= W x, without a context. For hosts that cannot let
  * the library allocate: all device memory already belongs to the host's own arena, or an
  * allocation would synchronise the device in the middle of its decode loop. Neither this call
- * nor its set-up allocates memory of any kind.
+ * nor its set-up allocates memory of any kind (partial sums meet in shared memory; the name is
+ * from when they met in a __device__ array).
  *
  * Uses the calling thread's current device; `cuda_stream` (NULL = default stream), A, x, y and
  * status_words must belong to it. Arguments as zc_dmmv for type Q4_K. Limits: K a multiple of
@@ -565,11 +564,8 @@ int32_t zc_dmmv_push(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size,
  * the call; a bounded wait that gave up stores {1, site} there, the result is then invalid and
  * the entry point must not be used again on that device.
  *
- * The first call on each device does the set-up (symbol address, SM count; the array is all
- * zero when the library is loaded and every launch leaves it zero): make it before any stream
- * capture starts on that device.
- * The scratch is shared by all calls on a device: calls ordered on one stream are safe; calls
- * whose kernels may overlap (different streams, unordered threads) race and give wrong results. */
+ * The first call on each device does the set-up (SM count): make it before any stream capture
+ * starts on that device. */
 int32_t zc_dmmv_q4k_static_scratch(void* cuda_stream,
                                    const void* A, uint64_t a_size,
                                    const void* x, uint64_t x_size,

@@ -185,8 +185,6 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
                                uint64_t* launches, const uint8_t* A2 = nullptr, uint64_t a2_bytes = 0,
                                float* Y2 = nullptr);  // A2 / Y2: a second matrix on the same grouping (gate + up)
 
-// Prefill GEMM for the weight layouts without a 16-byte row pitch (MXFP4, Q6_K with K % 2048 != 0): bf16
-// activations, raw blocks fetched with cp.async, same tile kernel as the grouped MoE path (moe_gemm_tc.cu).
 // MXFP4 weights on the block-scaled tensor-core path (gemm_mx.cu): weights as stored, bf16 activations split into
 // two FP8 terms in a caller-lent workspace.
 uint64_t mul_mm_mx_workspace_bytes(uint32_t N, uint32_t K);
@@ -230,6 +228,8 @@ cudaError_t launch_mx_terms(const void* X, bool bf16, uint32_t T, uint32_t K, ui
 cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint32_t bn, const uint8_t* ws, cudaStream_t s);
 // Zeroes an N x M output (row stride stride_d) that the GEMM launched behind it adds into.
 cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s);
+// Prefill GEMM for the weight layouts without a 16-byte row pitch (MXFP4, Q6_K with K % 2048 != 0): bf16
+// activations, raw blocks fetched with cp.async (moe_gemm_tc.cu).
 bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K,
                               uint32_t stride_b);
 cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_bytes, const void* B, float* D,

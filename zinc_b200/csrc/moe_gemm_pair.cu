@@ -1,17 +1,19 @@
 // Grouped dequant-GEMM of the MoE prefill on CTA pairs: Q4_K and Q6_K expert stacks, tokens grouped by routed expert
 // (moe_gemm_tc.cu makes the groups and packs the activations as bf16). An item is (a tile of up to BN of an expert's pairs,
-// 256 weight rows); each CTA of a pair has 128 of the rows and half of the pairs (tcgen05.mma cta_group::2). Per stage of
-// 128 columns: two bf16 weight tiles (16 KB each, K-major, 128-byte swizzle) written by eight producer warps from raw
-// blocks, two activation tiles by TMA.
+// 256 weight rows); each CTA of a pair has 128 of the rows and half of the pairs (tcgen05.mma cta_group::2). A stage is 128
+// columns: the weights as bf16 in tensor memory, written by eight producer warps (a thread per row, its own lane), two
+// activation tiles in shared memory by TMA.
 //
 // Raw blocks (256 columns) come by TMA. Q4_K rows have a 16-byte pitch: one box of 128 rows. Q6_K rows have not, but eight
 // of them have: the matrix is a tensor of eight-row groups, the segments of the rows c, c + 8, c + 16, .. of a tile are a
 // box of 16, and the slot keeps them by c.
 //
-// What bounds it: with the few pairs an expert has (16 of 256 experts at 512 tokens) the issuing warp (some 30 cycles an
-// instruction) and the turn-around of the stages. The one-CTA kernel, whose sixteen producer warps also copied the raw
-// blocks, had 2800 cycles for 256 columns of 128 rows: a third of it in the copies, which held up the producers' own
-// stores, a third waiting for the one stage a producer warp had.
+// What bounds it, with the 16 pairs an expert of 256 has at 512 tokens: the producers' integer pipe, 1650 (Q4_K) and 2200
+// (Q6_K) cycles for 256 columns of 128 rows. On one-CTA tiles it was 2800: a third in the producers' own copies, which held
+// up their stores, a third waiting for the one stage a warp had (layer 316 us, 242 on pairs). Through shared memory every
+// bf16 weight was written there and read by the MMA, 1024 cycles at 128 bytes each (226 us with tensor memory). Q6_K rows
+// are read four bytes at a time: no selection by the offset's bits, two rows to a bank at worst (down projection 96.6 ->
+// 92.9 us; 8 bytes 98.4).
 // Warp roles (25 warps): 0 MMA issuer, 1 and 3 loaders of the activations, 2 and 4 of raw blocks (a thread each), 5-20
 // producers (group j of four warps = columns 64 j .. of every block, a thread per row), 21-24 epilogue.
 // Every mbarrier wait is bounded; a wait that gives up records {1, site}, raises the CTA's flag, and every role drains to

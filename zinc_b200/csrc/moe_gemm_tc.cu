@@ -3,20 +3,22 @@
 // token tile instead of once per (token, slot) pair.
 //
 //   1. moe_group_kernel     counts the (token, slot) pairs of every expert, lays the experts' pair lists
-//                           side by side (no padding) and writes one tile record per BN pairs of an expert
+//                           side by side (no padding) and writes tile records of at most BN pairs, an expert's pairs
+//                           shared out equally
 //   2. moe_gather_x_kernel  packs the activation row of every pair, in list order, as bf16 [n_pairs][K]
-//   3. moe_gemm_tc_kernel   persistent CTAs walk the (tile, row tile) work items: tcgen05.mma with the
-//                           128 weight rows on the TMEM lanes and the tile's pairs on the columns; the
-//                           activation box (BN rows from the tile's first pair) comes by TMA and may
-//                           run into the next expert's rows, whose columns are never stored
-// Raw weight blocks are fetched by the dequant threads themselves with 16-byte cp.async pieces of the
-// aligned superset of each row's block (Q6_K blocks are only 2-byte aligned and MXFP4 blocks not aligned
-// at all, and their rows have no 16-byte pitch in general, so a tensor map cannot describe them) into a
-// ring as deep as shared memory allows (3 to 8 blocks); each copy reports to the slot's mbarrier itself. Types: Q4_K, Q6_K (K % 256 == 0) and MXFP4 (K % 64 == 0; dequantised exactly to bf16).
+//   3. Q4_K and Q6_K: moe_gemm_pair.cu; MXFP4: gemm_mx.cu (whose activations are split there); Q6_K rows not a multiple of
+//      eight: moe_gemm_tc_kernel. It also serves plain GEMMs on weights without a 16-byte row pitch (MXFP4, Q6_K), K split
+//      over several items where tiles are few.
+// moe_gemm_tc_kernel: persistent CTAs walk the (tile, row tile) work items: tcgen05.mma with the 128 weight rows on the
+// TMEM lanes and the tile's pairs on the columns (as many as it has); the activation box (BN rows from the tile's first
+// pair) comes by TMA and may run into the next expert's rows, whose columns are never stored. Raw weight blocks are fetched
+// by the dequant threads themselves with 16-byte cp.async pieces of the aligned superset of each row's block into a ring as
+// deep as shared memory allows; each copy reports to the slot's mbarrier itself. Types: Q4_K, Q6_K (K % 256 == 0) and
+// MXFP4 (K % 64 == 0; dequantised exactly to bf16).
 // Warp roles (23 warps): 0 tensor-memory owner + MMA issuer, 1 TMA loader of the activations, 2 idle,
 // 3-18 dequant (set j = 4 warps = group j of every 256-column block = weight stage j), 19-22 epilogue.
-// Rings: 4 bf16 weight stages (one per set) each with its activation slot, 4 to 8 raw blocks.
 // Two accumulators in tensor memory let the epilogue of one item overlap the MMAs of the next.
+// Bound: the dequant warps' integer pipe (MXFP4: 73 % busy) and the turn-around of one stage per set.
 // Every mbarrier wait is bounded; a wait that gives up records {1, site}, raises the CTA's flag, and
 // every role drains to the common exit where tensor memory is released.
 //
