@@ -374,22 +374,45 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     // Warps along K: as few as leave the longest share unchanged; the rest along the rows.
     const bool pair = F::kMost <= 16 && a.nblk * F::kCols <= 4096;
     const uint32_t most = pair ? 8u : kSeg == 3 ? 16u : F::kMost;
-    uint32_t per = (a.nblk + most - 1) / most;
-    // Tall matrices (several tiles per CTA either way): half as many warps along K, as long as all warps find work, and
-    // fewer meetings: Q4_K 65536 x 4096 29.6 -> 27.7 us, Q6_K 151936 x 4096 114.8 -> 109.1.
-    const bool tall = kSeg == 0 && a.M >= 16000 && (a.nblk + 2 * per - 1) / (2 * per) * 4 >= most;
-    if (tall) per *= 2;
-    a.n_wk = (a.nblk + per - 1) / per;
-    a.n_wr = most / a.n_wk;
-    if (a.n_wr > 4) a.n_wr = 4;
-    a.round = a.n_wr == 3 ? 6 : tall ? 8 : 4;
-    warps = a.n_wk * a.n_wr;
     const uint32_t per_sm = pair ? 2u : 1u, room = pair ? kSliceSmem2 : kSliceSmem1;
-    const uint32_t fixed = 128u + 2u * a.round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
-    if (fixed + warps * 2u * F::kSlot > room) return false;
-    a.depth = (room - fixed) / (warps * F::kSlot);
-    a.depth = a.depth > 4 ? 4 : a.depth;
-    smem = fixed + warps * a.depth * F::kSlot;
+    uint32_t per = (a.nblk + most - 1) / most;
+    auto cut = [&](uint32_t p, uint32_t wr, uint32_t round) {  // false: two units per warp do not fit beside x
+        a.n_wk = (a.nblk + p - 1) / p;
+        a.n_wr = wr;
+        a.round = round;
+        warps = a.n_wk * wr;
+        const uint32_t fixed = 128u + 2u * round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
+        if (fixed + warps * 2u * F::kSlot > room) return false;
+        a.depth = (room - fixed) / (warps * F::kSlot);
+        a.depth = a.depth > 4 ? 4 : a.depth;
+        smem = fixed + warps * a.depth * F::kSlot;
+        return true;
+    };
+    // Tall matrices (several tiles per CTA either way): the cut whose busiest warp has least to do, tiles of a CTA dealt to
+    // n_wr rows of warps, a longer share of K for each where more rows of warps fit; meetings every eight tiles or so.
+    // (Q4_K 65536 x 4096 29.6 -> 27.7 us, Q6_K 151936 x 4096 114.8 -> 109.1 against the cut below.)
+    uint32_t tall_per = 0, tall_wr = 0;
+    if (kSeg == 0 && a.M >= 16000) {
+        const uint32_t tpc = ((a.M + 15) / 16 + sms * per_sm - 1) / (sms * per_sm);
+        uint32_t least = 0xFFFFFFFFu;
+        for (uint32_t p = a.nblk < per * 4 ? a.nblk : per * 4; p >= per; --p) {
+            const uint32_t wk = (a.nblk + p - 1) / p;
+            for (uint32_t wr = 1; wr <= 4 && wr * wk <= most; ++wr) {
+                // by 5 % at least: between equals the longer share (Q6_K 151936 x 4096: 109 us, 112 with all warps along K)
+                if ((uint64_t)((tpc + wr - 1) / wr * p) * 20 < (uint64_t)least * 19 && cut(p, wr, wr == 3 ? 9 : 8)) {
+                    least = (tpc + wr - 1) / wr * p;
+                    tall_per = p;
+                    tall_wr = wr;
+                }
+            }
+        }
+    }
+    if (tall_per) {
+        cut(tall_per, tall_wr, tall_wr == 3 ? 9 : 8);
+    } else {
+        const uint32_t wk = (a.nblk + per - 1) / per, wr = most / wk > 4 ? 4 : most / wk;
+        if (!cut(per, wr, wr == 3 ? 6 : 4)) return false;
+    }
     // Tile height: the one that gives the busiest CTA the least to do (an MMA costs the same for fewer rows: 0.3 per row)
     uint32_t best = 0xFFFFFFFFu;
     for (uint32_t h = 16; h >= 4; --h) {
