@@ -57,12 +57,18 @@ bool take_attr(PyObject* o, PyObject* name, uint64_t& v) {
 
 // *keep: an object made here that owns the memory (to be released after the call)
 bool take_buffer(Call* c, PyObject* o, uint64_t& ptr, uint64_t& size, PyObject** keep) {
-    if (THPVariable_Check(o)) {
-        const at::Tensor& t = THPVariable_Unpack(o);
-        if (t.is_cuda() && t.is_contiguous()) {
-            ptr = reinterpret_cast<uint64_t>(t.data_ptr());
-            size = t.nbytes();
-            return true;
+    // Plain tensors only: a subclass answers for itself in Python. Tensors without memory of their own (under a
+    // transform or a tracer) answer with a C++ exception, which must not leave through the interpreter's C frames:
+    // they go the Python way too, where the same question raises.
+    if (THPVariable_CheckExact(o)) {
+        try {
+            const at::Tensor& t = THPVariable_Unpack(o);
+            if (t.is_cuda() && t.is_contiguous()) {
+                ptr = reinterpret_cast<uint64_t>(t.data_ptr());
+                size = t.nbytes();
+                return true;
+            }
+        } catch (...) {
         }
     }
     PyObject* b = PyObject_CallOneArg(c->to_buffer, o);  // a Buffer comes back as itself
