@@ -106,16 +106,17 @@ EXPORTS = sorted(list(_OPS) + [
 ])
 
 _lib = None
-CALL_PATH = os.path.join(_HERE, "_call.so")
 
 
 def native_call():
-    """The class of native calls (csrc/call.cpp), or None in a program that has not loaded torch, whose tensors it reads."""
+    """The class of native calls (csrc/call.cpp), or None: in a program that has not loaded torch, whose tensors it reads,
+    and where it was not built or was built against another torch. The same functions are then called through ctypes."""
     if "torch" not in sys.modules:
         return None
-    if not os.path.exists(CALL_PATH):
-        raise ImportError(f"{CALL_PATH} is missing: build it with `python -m zinc_b200.build`.")
-    from ._call import Call
+    try:
+        from ._call import Call
+    except ImportError:
+        return None
     return Call
 
 

@@ -25,12 +25,21 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found")
 
 
-def _call_command() -> list:
-    """g++ on call.cpp, against the headers and libraries of the installed torch (found without importing it)."""
+def _torch_spec():
     import importlib.util
+
+    return importlib.util.find_spec("torch")
+
+
+def _call_command():
+    """g++ on call.cpp, against the headers and libraries of the installed torch (found without importing it); None
+    where there is no torch: the library does not need it."""
     import sysconfig
 
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    spec = _torch_spec()
+    if spec is None or not spec.origin:
+        return None
+    torch_dir = os.path.dirname(spec.origin)
     inc = os.path.join(torch_dir, "include")
     lib = os.path.join(torch_dir, "lib")
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, "call.cpp"), "-o", CALL_SO,
@@ -39,9 +48,10 @@ def _call_command() -> list:
 
 
 def stale() -> bool:
-    if not os.path.exists(SO) or not os.path.exists(CALL_SO):
+    built = [SO] if _call_command() is None else [SO, CALL_SO]
+    if not all(os.path.exists(f) for f in built):
         return True
-    t = min(os.path.getmtime(SO), os.path.getmtime(CALL_SO))
+    t = min(os.path.getmtime(f) for f in built)
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [
         os.path.join(HERE, "..", "include", "zinc_cuda.h")]
     return any(os.path.getmtime(d) > t for d in deps)
@@ -55,7 +65,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
     procs = []
-    call = subprocess.Popen(_call_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    command = _call_command()
+    call = command and subprocess.Popen(command, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     for src in SOURCES:
         obj = os.path.join(objdir, src.replace(".cu", ".o"))
         cmd = [nvcc, *[f for f in NVCC_FLAGS if f != "--use_fast_math=false"], "-c",
@@ -70,10 +81,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
             sys.stderr.write(out)
             raise RuntimeError(f"nvcc failed on {src}")
         objs.append(obj)
-    out, _ = call.communicate()
-    if call.returncode != 0:
-        sys.stderr.write(out)
-        raise RuntimeError("g++ failed on call.cpp")
+    if call is not None:
+        out, _ = call.communicate()
+        if call.returncode != 0:
+            sys.stderr.write(out)
+            raise RuntimeError("g++ failed on call.cpp")
     with open(os.path.join(objdir, "ptxas.log"), "w") as f:
         f.write("\n".join(log))
     if verbose:

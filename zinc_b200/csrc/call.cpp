@@ -1,6 +1,6 @@
 // Python -> C ABI calls without ctypes: one vectorcall object per exported function. A call names its buffers as CUDA
 // tensors or Buffer objects; pointers and byte sizes are taken here, and the function is entered with the interpreter
-// lock released, as ctypes does. A matvec's Python side costs 0.7 us this way instead of 5 us (three tensors, thirteen
+// lock released, as ctypes does. A matvec's Python side costs 1.3 us this way instead of 5 us (three tensors, thirteen
 // arguments), less than its kernel.
 #include <Python.h>
 #include <structmember.h>
@@ -8,24 +8,62 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
+#include <utility>
 
-#if !defined(__x86_64__)
-#error "the call below relies on the x86-64 System V convention"
-#endif
+#include "../../include/zinc_cuda.h"
 
 namespace {
 
 constexpr int kMaxWords = 32;
-// Integer and pointer arguments take one 64-bit slot each, in order, and a float travels in xmm0 whatever its position;
-// slots past the callee's own are ignored.
-#define W4 uint64_t, uint64_t, uint64_t, uint64_t
-using Entry = int32_t (*)(W4, W4, W4, W4, W4, W4, W4, W4, float);
-#undef W4
+
+// Arguments as 64-bit words in order (floats apart: a function has one at most) -> the function's own parameters.
+template <typename P>
+P argument(const uint64_t* w, size_t at, float f) {
+    if constexpr (std::is_same_v<P, float>) return f;
+    else if constexpr (std::is_pointer_v<P>) return reinterpret_cast<P>(static_cast<uintptr_t>(w[at]));
+    else return static_cast<P>(w[at]);
+}
+template <typename Fn>
+struct Invoke;
+template <typename... P>
+struct Invoke<int32_t (*)(P...)> {
+    static constexpr int kWords = ((std::is_same_v<P, float> ? 0 : 1) + ... + 0);
+    static constexpr size_t word_of(size_t param) {  // word of parameter `param`: floats take none
+        constexpr bool is_float[] = {std::is_same_v<P, float>...};
+        size_t at = 0;
+        for (size_t i = 0; i < param; ++i) at += is_float[i] ? 0 : 1;
+        return at;
+    }
+    template <size_t... I>
+    static int32_t run(uint64_t fn, const uint64_t* w, float f, std::index_sequence<I...>) {
+        return reinterpret_cast<int32_t (*)(P...)>(static_cast<uintptr_t>(fn))(argument<P>(w, word_of(I), f)...);
+    }
+    static int32_t go(uint64_t fn, const uint64_t* w, float f) { return run(fn, w, f, std::index_sequence_for<P...>()); }
+};
+
+struct Entry {
+    const char* name;
+    int words;
+    int32_t (*go)(uint64_t fn, const uint64_t* w, float f);
+};
+#define ENTRY(name) {#name, Invoke<decltype(&name)>::kWords, Invoke<decltype(&name)>::go}
+constexpr Entry kEntries[] = {
+    ENTRY(zc_dmmv), ENTRY(zc_dmmv_push), ENTRY(zc_dmmv_batch), ENTRY(zc_moe_dmmv), ENTRY(zc_moe_dmmv_batched),
+    ENTRY(zc_moe_dmmv_batched_pair), ENTRY(zc_mul_mm_block_scaled), ENTRY(zc_count_experts), ENTRY(zc_mul_mm),
+    ENTRY(zc_dmmv_fused_gate_up_swiglu), ENTRY(zc_dmmv_sigmoid_acc), ENTRY(zc_moe_fused_gate_up), ENTRY(zc_moe_fused_gate_up_act),
+    ENTRY(zc_moe_gate_up_act_ex), ENTRY(zc_moe_down_acc_ex), ENTRY(zc_moe_router_topk), ENTRY(zc_rms_norm_dmmv_f32),
+    ENTRY(zc_dmmv_o_proj_merge), ENTRY(zc_rms_norm_dmmv_alpha_beta), ENTRY(zc_moe_weighted_acc), ENTRY(zc_bias_add),
+    ENTRY(zc_moe_bias_act), ENTRY(zc_moe_weighted_bias_acc), ENTRY(zc_moe_ep_filter), ENTRY(zc_moe_route_pack),
+    ENTRY(zc_moe_route_scatter), ENTRY(zc_dequant_rows),
+};
+#undef ENTRY
 
 struct Call {
     PyObject_HEAD
     vectorcallfunc vectorcall;
-    Entry fn;
+    uint64_t fn;
+    int32_t (*go)(uint64_t fn, const uint64_t* w, float f);
     char spec[kMaxWords + 1];  // i integer, f float, b buffer, o buffer or None
     int n;
     PyObject* to_buffer;       // Python: anything else -> Buffer (raises)
@@ -113,9 +151,7 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
     int32_t rc = 0;
     if (ok) {
         Py_BEGIN_ALLOW_THREADS
-        rc = c->fn(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8], w[9], w[10], w[11], w[12], w[13], w[14], w[15],
-                   w[16], w[17], w[18], w[19], w[20], w[21], w[22], w[23], w[24], w[25], w[26], w[27], w[28], w[29], w[30],
-                   w[31], f);
+        rc = c->go(c->fn, w, f);
         Py_END_ALLOW_THREADS
     }
     for (int i = 0; i < kept; ++i) Py_DECREF(keep[i]);
@@ -124,19 +160,23 @@ PyObject* call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* k
 
 PyObject* call_new(PyTypeObject* type, PyObject* args, PyObject*) {
     unsigned long long fn;
-    const char* spec;
+    const char *name, *spec;
     PyObject* to_buffer;
-    if (!PyArg_ParseTuple(args, "KsO", &fn, &spec, &to_buffer)) return nullptr;
+    if (!PyArg_ParseTuple(args, "KssO", &fn, &name, &spec, &to_buffer)) return nullptr;
+    const Entry* entry = nullptr;
+    for (const Entry& e : kEntries)
+        if (!std::strcmp(e.name, name)) entry = &e;
     int words = 0, n = 0;
     for (const char* p = spec; *p; ++p, ++n) words += *p == 'i' ? 1 : *p == 'f' ? 0 : 2;
-    if (words > kMaxWords || n > kMaxWords) {
-        PyErr_SetString(PyExc_ValueError, "too many arguments");
+    if (!entry || words != entry->words || words > kMaxWords || n > kMaxWords) {
+        PyErr_Format(PyExc_ValueError, "%s does not take the arguments '%s'", name, spec);
         return nullptr;
     }
     Call* c = reinterpret_cast<Call*>(type->tp_alloc(type, 0));
     if (!c) return nullptr;
     c->vectorcall = call;
-    c->fn = reinterpret_cast<Entry>(fn);
+    c->fn = fn;
+    c->go = entry->go;
     std::strcpy(c->spec, spec);
     c->n = n;
     Py_INCREF(to_buffer);

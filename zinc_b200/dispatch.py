@@ -281,7 +281,7 @@ def _calls() -> dict:
     L = _lib.lib()
     native = _lib.native_call()
     if native is not None:
-        return {name: native(C.cast(getattr(L, name), C.c_void_p).value, spec, _buf) for name, spec in _CALLS.items()}
+        return {name: native(C.cast(getattr(L, name), C.c_void_p).value, name, spec, _buf) for name, spec in _CALLS.items()}
 
     def through_ctypes(fn, spec):
         def call(*args):
