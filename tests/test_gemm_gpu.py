@@ -251,6 +251,24 @@ def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
         assert rel_l2(got[:, r], want[:, r]) <= 2 * TOL_EXACT
 
 
+@pytest.mark.parametrize("t,K", [(zb.Q6_K, 2048), (zb.Q8_0, 2048), (zb.MXFP4, 2080)], ids=["q6_k", "q8_0", "mxfp4"])
+def test_mul_mm_exact_same_bits_every_time(gpu, t, K):
+    """A raw slot given back while a read of it is under way changes single rows now and then; a repeated launch has to
+    give the same bits. (74 whole tiles: no sum has two writers.)"""
+    torch, ctx, dd = gpu
+    M, N = 256 * 37, 512
+    g = synth.rng(307, t)
+    w, X = dev(torch, synth.quant_matrix(g, t, M, K)), dev(torch, synth.activations(g, N, K))
+    first, bad = None, 0
+    for _ in range(300):
+        D = torch.empty(N * M, device="cuda")
+        dd.recordMulMm(t, w, X, D, M, N, K, K, M)
+        first = D if first is None else first
+        bad = bad + (D != first).sum()
+    ctx.submit_and_wait()
+    assert int(bad) == 0
+
+
 def test_mul_mm_errors(gpu):
     torch, ctx, dd = gpu
     w = torch.zeros(144 * 8, dtype=torch.uint8, device="cuda")

@@ -879,3 +879,27 @@ def test_router_selection_ties(gpu, oracle, n, k):
     assert np.array_equal(r[:k], ids)
     assert np.max(np.abs(r[k:].view(np.float32) - wt)) <= 1e-6
     assert bool((rt[2 * k:] == 0x7ABCDEF0).all().item())
+
+
+@pytest.mark.parametrize("t,M,K", [(zb.Q6_K, 512, 2048), (zb.Q6_K, 2048, 512), (zb.Q4_K, 512, 2048)], ids=["q6_k", "q6_k_short", "q4_k"])
+def test_moe_grouped_same_bits_every_time(gpu, t, M, K):
+    """The raw slots are refilled behind their readers: a slot given back while a read of it is under way changes single
+    rows now and then. Every output has one writer, so that a repeated launch has to give the same bits. (500 launches of
+    32 experts x 2 to 8 row tiles x 2 to 8 blocks: some 300,000 refills.)"""
+    torch, ctx, dd = gpu
+    E, k, T = 32, 4, 64
+    g = synth.rng(240, t + K)
+    w, stride = stacked(g, t, E, M, K)
+    ids = np.stack([g.permutation(E)[:k] for _ in range(T)]).astype(np.uint32)
+    wd, X, idd = dev(torch, w), dev(torch, synth.activations(g, T, K)), dev(torch, ids.view(np.int32))
+    ws = torch.empty(dd.moeGroupedWorkspaceBytes(T, k, K, E), dtype=torch.uint8, device="cuda")
+    dd.setWorkspace(ws)
+    first, bad = None, 0
+    for _ in range(500):
+        Y = torch.empty(T * k * M, device="cuda")
+        dd.recordMoeBatchedDispatch(t, wd, X, Y, idd, M, K, stride, E, k, T, K, k * M)
+        first = Y if first is None else first
+        bad = bad + (Y != first).sum()
+    ctx.submit_and_wait()
+    dd.setWorkspace(None)
+    assert int(bad) == 0

@@ -645,18 +645,19 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     for (int i = 0; i < 8; ++i)
                         if (8 * b + i < (g.K >> 5)) emax = max(emax, (uint32_t)wp[off + 17 * i]);
                     s_cur = e8m0_to_f32(emax);
-                    uint32_t q[2][4];
+                    uint32_t q[2][4], read = emax;  // every word read: nibbles, the block's scales, this set's own
                     __half2 sc[2];
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
-                        const uint32_t o = off + 17u * (2 * j + i);
-                        const int diff = (int)emax - (int)wp[o];
+                        const uint32_t o = off + 17u * (2 * j + i), e = wp[o];
+                        const int diff = (int)emax - (int)e;
                         lds_words<4>(wp + ((o + 1) & ~15u), (o + 1) & 15u, q[i]);
+                        read ^= e ^ q[i][0] ^ q[i][3];
                         const bool live = 8 * b + 2 * j + i < (g.K >> 5);
                         sc[i] = __float2half2_rn(live && diff < 60 ? __uint_as_float((uint32_t)(127 + 14 - diff) << 23) : 0.f);
                         if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
                     }
-                    release_after(q[0][0] ^ q[0][3] ^ q[1][0] ^ q[1][3], &bars->empty_w[sw], lane);
+                    release_after(read, &bars->empty_w[sw], lane);
                     if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
                     x_deq_mx(q[0], sc[0], 0, stage, row);
                     x_deq_mx(q[1], sc[1], 4, stage, row);
@@ -693,10 +694,8 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 #pragma unroll
                             for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage2 + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
                         }
-                        if (hf == 1) {
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&bars->empty_w[sw]);
-                        }
+                        // the weights and their scales are in the stores above; the block's scale is in nothing yet
+                        if (hf == 1) release_after(__float_as_uint(s_cur), &bars->empty_w[sw], lane);
                         fence_proxy_async();
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(full_a0 + ab2 * 8);

@@ -241,7 +241,8 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1, put);
                 } else {
                     dequant_group_q6k<4>(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, put);
-                    release_after(o[3] ^ o[7] ^ o[11] ^ o[15] ^ o[19] ^ o[23] ^ o[27] ^ o[31], &bars->empty_w[slot], lane);
+                    // words 4 k + 3 are made of every word read but the first ones of ql and qh, which word 0 is made of
+                    release_after(o[0] ^ o[3] ^ o[7] ^ o[11] ^ o[15] ^ o[19] ^ o[23] ^ o[27] ^ o[31], &bars->empty_w[slot], lane);
                 }
                 if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 166);
                 __syncwarp();

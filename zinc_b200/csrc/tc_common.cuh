@@ -275,7 +275,9 @@ __device__ __forceinline__ bool poll_or_fail(uint64_t* bar, uint32_t parity, B* 
 
 // Gives a slot of raw bytes back (a converged warp) once its reads are done, not only under way: `x` is made of a word of
 // every one of them, and the branch on it cannot be taken before they return. An arrival that merely followed the reads
-// was seen to overtake them: the refill by TMA then changed single rows, once in some thousand launches.
+// was seen to overtake them: the refill by TMA then changed single rows, once in some thousand launches. Only reads whose
+// values stand in stores ahead of the arrival may be left out of `x` (a store cannot be issued before its operands are
+// there, and the arrival is issued after it): so do the plain arrivals after a Q6_K or MXFP4 group's stores.
 __device__ __forceinline__ void release_after(uint32_t x, uint64_t* bar, int lane) {
     if (__any_sync(0xFFFFFFFFu, x == 0x9E3779B9u)) __nanosleep(1);
     if (lane == 0) mbar_arrive(bar);
