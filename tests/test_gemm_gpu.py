@@ -251,6 +251,62 @@ def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
         assert rel_l2(got[:, r], want[:, r]) <= 2 * TOL_EXACT
 
 
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K, zb.Q6_K, zb.Q8_0, zb.MXFP4], ids=["q4_k", "q5_k", "q6_k", "q8_0", "mxfp4"])
+@pytest.mark.parametrize("N", [20, 150])
+def test_mul_mm_exact_outlier_inside_a_token(gpu, oracle, t, N):
+    """One element of a token 2^16 above the others, against weights that are zero: the others, 2^-16 of the largest or a
+    little less, keep their 22 bits, so that the bound is the one of tokens without outliers."""
+    torch, ctx, dd = gpu
+    M, K = 70, 1024
+    g = synth.rng(308, t)
+    w = synth.quant_matrix(g, t, M, K).reshape(M, -1).copy()
+    one = zb.row_bytes(t, 256)
+    w[:, one:2 * one] = 0   # columns 256 .. 511
+    X = synth.activations(g, N, K)
+    X[:, 300] = np.where(np.arange(N) % 2, -65536.0, 65536.0).astype(np.float32)
+    D = out_with_canary(torch, N * M)
+    dd.recordMulMm(t, dev(torch, w.reshape(-1)), dev(torch, X), D, M, N, K, K, M)
+    ctx.submit_and_wait()
+    want = oracle.gemm_f64(w.reshape(-1), t, M, K, X)
+    got = D[:N * M].cpu().numpy().reshape(N, M)
+    for c in range(N):
+        assert rel_l2(got[c], want[c]) <= TOL_EXACT
+
+
+def test_mul_mm_exact_wide_block_scales(gpu, oracle):
+    """Scales within 256 columns far apart. MXFP4: 2^-20 of the largest, whose block holds zeros: exact. Q8_0: d 2^-12 of the
+    largest: exact. Q4_K: dmin 2^20 times d against mins that cancel: the q terms still count in full."""
+    torch, ctx, dd = gpu
+    M, N, K = 40, 24, 256
+    g = synth.rng(309, 0)
+    X = synth.activations(g, N, K)
+
+    def run(t, w, X):
+        D = out_with_canary(torch, N * M)
+        dd.recordMulMm(t, dev(torch, w.reshape(-1)), dev(torch, X), D, M, N, K, K, M)
+        ctx.submit_and_wait()
+        return D[:N * M].cpu().numpy().reshape(N, M), oracle.gemm_f64(np.ascontiguousarray(w).reshape(-1), t, M, K, X)
+
+    w = synth.quant_matrix(g, zb.MXFP4, M, K).reshape(M, 8, 17).copy()
+    w[:, :, 0] = 110
+    w[:, 3, 0], w[:, 3, 1:] = 130, 0
+    got, want = run(zb.MXFP4, w, X)
+    assert rel_l2(got, want) <= TOL_EXACT
+    w = synth.quant_matrix(g, zb.Q8_0, M, K).reshape(M, 8, 34).copy()
+    w[:, :, 0:2] = np.frombuffer(np.float16(2.0 ** -12 * 1.25).tobytes(), np.uint8)
+    w[:, 5, 0:2], w[:, 5, 2:] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8), 0
+    got, want = run(zb.Q8_0, w, X)
+    assert rel_l2(got, want) <= TOL_EXACT
+    w = synth.quant_matrix(g, zb.Q4_K, M, K).reshape(M, 144).copy()
+    w[:, 0:2] = np.frombuffer(np.float16(2.0 ** -17).tobytes(), np.uint8)
+    w[:, 2:4] = np.frombuffer(np.float16(8.0).tobytes(), np.uint8)
+    Xz = X.copy()
+    Xz[:, 1::2] = -Xz[:, ::2]   # every sub-block sums to zero: the min terms vanish, exactly
+    got, _ = run(zb.Q4_K, w, Xz)
+    w[:, 2:4] = 0               # (a weight dequantised to one f32 would have lost its q term beside the min)
+    assert rel_l2(got, oracle.gemm_f64(np.ascontiguousarray(w).reshape(-1), zb.Q4_K, M, K, Xz)) <= TOL_EXACT
+
+
 @pytest.mark.parametrize("t,K", [(zb.Q6_K, 2048), (zb.Q8_0, 2048), (zb.MXFP4, 2080)], ids=["q6_k", "q8_0", "mxfp4"])
 def test_mul_mm_exact_same_bits_every_time(gpu, t, K):
     """A raw slot given back while a read of it is under way changes single rows now and then; a repeated launch has to

@@ -98,11 +98,13 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
     mx = s_max[0];
 #pragma unroll
     for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, s_max[i]);
-    // largest element to [2^4, 2^5): 32 times a sub-block's sum stays below 2^15; the inverse stays a normal number
+    // Largest element to [2^14, 2^15), the top of fp16's range, so that an element keeps its 22 bits down to 2^-17 of the
+    // largest; the inverse stays a normal number. Types with mins: their weights are 2^-10 of their value (gemm_exact.cuh),
+    // and the sums are brought down to match, below 2^15 too.
     const uint32_t e = __float_as_uint(mx) >> 23;
-    const uint32_t f = min(258u - e, 252u);
+    const uint32_t f = min(268u - e, 252u);
     const float scale = __uint_as_float(f << 23);
-    if (tid == 0) a.inv_scale[t] = __uint_as_float((254u - f) << 23);
+    if (tid == 0) a.inv_scale[t] = __uint_as_float((ORDER == 0 ? 264u - f : 254u - f) << 23);
 
     uint4* out = reinterpret_cast<uint4*>(a.x + (uint64_t)t * a.nblk * 256);
     const uint64_t low = (uint64_t)gridDim.x * a.nblk * 32;  // 16-byte chunks to the low term
@@ -137,8 +139,8 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
                 sa += __shfl_xor_sync(0xFFFFFFFFu, sa, o);
                 sb += __shfl_xor_sync(0xFFFFFFFFu, sb, o);
             }
-            sa *= 32.f;
-            sb *= 32.f;
+            sa *= 1.f / 32.f;
+            sb *= 1.f / 32.f;
             // a block's row: sub-block sums as [high 8][high 8][low 8][zeros 8], against the weights' min terms
             // [high][low][high][zeros]
             uint32_t* sp = reinterpret_cast<uint32_t*>(sums + (uint64_t)(g >> 2) * 8) + (g & 3);

@@ -3,15 +3,20 @@
 //
 // The tensor cores take fp16 operands, so both sides are brought to fp16 without losing f32 accuracy:
 //   W  inside a 256-column block a K-quant weight is an integer times the row's d: sc * q (Q4_K 945 at most, Q5_K
-//      1953) is exact in fp16 and the f16 block scale d is applied in f32 afterwards. Q6_K (13 bits) and Q8_0
-//      (d * q over the block's largest power of two, 19 bits) are two exact fp16 terms, the second the rounding
-//      residue of the first. MXFP4 is a power of two times E2M1: exact in one term. A row's min term of Q4_K / Q5_K,
+//      1953), 2^-10 of it, is exact in fp16 and the f16 block scale d is applied in f32 afterwards. Q6_K (13 bits) is two
+//      exact fp16 terms, the second the rounding residue of the first; so is Q8_0 (d * q over the largest d's power of two
+//      in the block, 19 bits) for a d of 2^-14 of the largest or more, below that to 2^-25 of the largest weight's power
+//      of two. MXFP4 is a power of two times E2M1, one term: exact where the 32-column block's scale is 2^-23 of the largest
+//      in the 256 columns or more, below that to 2^-25 of the largest. A row's min term of Q4_K / Q5_K,
 //      -dmin * m_s * (sum of x over sub-block s), is 32 more columns of the block: (dmin / d) * m_s in two terms
 //      against the sub-block sums of x in two terms.
-//   X  a token is scaled by a power of two (its largest element to [2^4, 2^5)) and split into two fp16 terms: 22
-//      significant bits, absolute error 2^-29 of the token's largest element. bf16 activations are one exact term.
-//      (The sub-block sums are scaled up by 2^5 and the min terms down by as much, which leaves dmin / d a range of
-//      2^15 before it no longer fits fp16.)
+//   X  a token is scaled by a power of two (its largest element to [2^14, 2^15)) and split into two fp16 terms: 22
+//      significant bits down to 2^-17 of the token's largest element, below that an absolute error of 2^-39 of it. bf16
+//      activations are one term, exact down to 2^-31 of the largest. (With the largest at 2^4, as it was first, a token with
+//      one element 2^16 above the others lost half their bits.)
+//      The sub-block sums are scaled by 2^-5 and the min terms too, which with the weights' 2^-10 is the same factor; it
+//      leaves dmin / d a range of 2^15 before it no longer fits fp16, and the block's scale goes up by powers of two beyond.
+// An infinite activation makes its token's row NaN.
 // Every block is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
 // ("promote") while the next block's MMAs fill the other accumulator.
 //
@@ -132,7 +137,7 @@ __device__ __forceinline__ void put_chunk(uint8_t* rowp, int sw, int c, uint4 o)
 
 // 64 columns of Q4_K / Q5_K (w: nibble words, h: the fifth bits' words or unused): chunk i of the stage row holds
 // word i's low nibbles (columns 4i + {0, 2, 1, 3}) and high nibbles (32 + 4i + ...): the order a byte mask yields,
-// which the activations follow. 1024 + q comes from or-ing q into the fp16 pattern of 1024; one fma leaves sc * q.
+// which the activations follow. 1024 + q comes from or-ing q into the fp16 pattern of 1024; one fma leaves s * q.
 template <bool kFive>
 __device__ __forceinline__ void x_deq_k4(const uint32_t (&w)[8], const uint32_t (&h)[8], int j, float s_lo, float s_hi,
                                          uint8_t* stage, int row) {
@@ -591,19 +596,26 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     release_after(hd.x ^ c0.x ^ c1.x ^ h0.y ^ h1.y, &bars->empty_w[sw], lane);
                     const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
                     const float d = __low2float(dd), dmin = __high2float(dd);
-                    // the block's scale is d; where dmin is far above it (and there are mins at all), dmin / 2^15, so that
-                    // the ratio fits fp16: the q terms, at most 945 / 2^15 of a min term there, are then rounded
-                    float ratio = 0.f, q_scale = 1.f;
+                    // The block's scale is d; where dmin is more than 2^15 of it (and there are mins at all), d times the
+                    // power of two that brings the ratio to [2^14, 2^15): the q terms go down by as much, exactly as far
+                    // as fp16 reaches (a ratio of 2^25) and beyond that to 2^-29 of a min term.
+                    float ratio = 0.f, q_scale = 1.f / 1024.f;
+                    bool mins = true;
                     s_cur = d;
                     if (fabsf(dmin) > 32768.f * fabsf(d)) {
-                        if (((hd.z | (hd.w & 0xF0F0F0F0u)) != 0u)) {
+                        mins = (hd.z | (hd.w & 0xF0F0F0F0u)) != 0u;
+                        if (mins && d == 0.f) {
                             s_cur = dmin * (1.f / 32768.f);
-                            ratio = 32768.f;
-                            q_scale = d / s_cur;
+                            q_scale = 0.f;
+                        } else if (mins) {
+                            const uint32_t e = __float_as_uint(__fdividef(fabsf(dmin), fabsf(d))) >> 23;
+                            s_cur = d * __uint_as_float((e - 14u) << 23);
+                            q_scale = __uint_as_float((258u - e) << 23);
                         }
-                    } else if (d != 0.f) {  // dmin / d: an approximate reciprocal and a Newton step
-                        const float r = __fdividef(1.f, d);
-                        ratio = dmin * fmaf(fmaf(-d, r, 1.f), r, r);
+                    }
+                    if (mins && s_cur != 0.f) {  // dmin / s_cur: an approximate reciprocal and a Newton step
+                        const float r = __fdividef(1.f, s_cur);
+                        ratio = dmin * fmaf(fmaf(-s_cur, r, 1.f), r, r);
                     }
                     ratio *= -1.f / 32.f;
                     // the 6-bit scales and mins of sub-blocks 2j and 2j + 1 (getScaleMinK4, src/compute/forward.zig:229-238),
