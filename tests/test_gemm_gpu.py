@@ -252,6 +252,25 @@ def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
 
 
 @pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K, zb.Q6_K, zb.Q8_0, zb.MXFP4], ids=["q4_k", "q5_k", "q6_k", "q8_0", "mxfp4"])
+@pytest.mark.parametrize("cols", [7, 64, 65, 130])
+def test_dmmv_batch_is_as_accurate_as_f32_sums(gpu, oracle, t, cols):
+    """The batched product on the tensor cores against f64. Bound, relative L2: 1.2e-7 for the four truncations of a
+    64-column run (half of 2^-23 each, the partial sums before the last one smaller), 1.7e-7 for the 64 f32 additions of
+    4096 columns (0.29 x 2^-23 each, as a random sum), 0.5e-7 for activations of 22 bits: 2.1e-7 together, some 20 % to
+    spare. (Accumulations of 256 columns have 3.6e-7 and more.)"""
+    torch, ctx, dd = gpu
+    M, K = 512, 4096
+    g = synth.rng(310, t + cols)
+    w = synth.quant_matrix(g, t, M, K)
+    X = synth.activations(g, cols, K)
+    Y = out_with_canary(torch, cols * M)
+    dd.recordBatchDispatchPush(t, dev(torch, w), dev(torch, X), Y, M, K, 0, 0, 0, cols)
+    ctx.submit_and_wait()
+    assert canary_intact(Y, cols * M)
+    assert rel_l2(Y[:cols * M].cpu().numpy(), oracle.gemm_f64(w, t, M, K, X)) <= 2.5e-7
+
+
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K, zb.Q6_K, zb.Q8_0, zb.MXFP4], ids=["q4_k", "q5_k", "q6_k", "q8_0", "mxfp4"])
 @pytest.mark.parametrize("N", [20, 150])
 def test_mul_mm_exact_outlier_inside_a_token(gpu, oracle, t, N):
     """One element of a token 2^16 above the others, against weights that are zero: the others, 2^-16 of the largest or a

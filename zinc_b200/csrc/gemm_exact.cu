@@ -194,8 +194,9 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         XPlan plan{};
         plan.nblk = nblk;
         plan.n_row_pairs = (p.M + 255) / 256;
-        // equal tiles of at most 256 tokens, in steps of 32 (the MMA's N over a CTA pair, eight-row swizzle groups)
-        const uint32_t cols = (p.N + 255) / 256;
+        // equal tiles of at most 256 (fine: 128, types of two fp16 terms 64) tokens, in steps of 32 (the MMA's N over a CTA
+        // pair, eight-row swizzle groups)
+        const uint32_t widest = !p.fine ? 256 : p.type == T_Q6_K || p.type == T_Q8_0 ? 64 : 128, cols = (p.N + widest - 1) / widest;
         plan.n_tile = ((p.N + cols - 1) / cols + 31) & ~31u;
         plan.n_tiles = plan.n_row_pairs * ((p.N + plan.n_tile - 1) / plan.n_tile);
         uint8_t* q = scratch;

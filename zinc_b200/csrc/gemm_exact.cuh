@@ -17,8 +17,17 @@
 //      The sub-block sums are scaled by 2^-5 and the min terms too, which with the weights' 2^-10 is the same factor; it
 //      leaves dmin / d a range of 2^15 before it no longer fits fp16, and the block's scale goes up by powers of two beyond.
 // An infinite activation makes its token's row NaN.
-// Every block is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
-// ("promote") while the next block's MMAs fill the other accumulator.
+// A run of columns is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
+// ("promote") while further runs fill other accumulators. The tensor core cuts an accumulator's last bits off at every
+// instruction, so the length of a run decides how far the result is from the exact one (relative L2, activations N(0, 1),
+// K = 4096):
+//   kRuns 1  a block of 256 columns: 1.8e-7 (MXFP4) to 1e-6 (Q8_0 beyond 128 tokens), where one f32 chain per output
+//            (gemm_simple_kernel) has 1.1e-6. For zc_mul_mm.
+//   kRuns 4  64 columns, their small terms first: 1.2e-7 to 1.8e-7, where f32 sums by lanes (dmmv_kernel) have 1.0e-7 to
+//            1.3e-7 and runs of a block 3.6e-7 to 1e-6. For zc_dmmv_batch, in tiles of at most 128 tokens, where a block's
+//            four accumulators fit: Q4_K 12288 x 4096, 105 tokens 37.3 us (36.7 with runs of a block). Adding a block's
+//            four runs before the registers' sum takes it to 1.4e-7 and 42 us, with the sum's roundings kept too 1.3e-7
+//            and 49 us: the runs' own roundings are what is left.
 //
 // Persistent CTA pairs (cta_group::2, 256 weight rows per pair): tiles of 256 rows x n_tile tokens, their
 // (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over pairs is summed with
@@ -36,6 +45,7 @@ namespace zc {
 namespace {
 
 constexpr int kXThreads = 3 * 32 + 512;  // issuer, loader, spare; sixteen producer warps
+constexpr uint32_t kXBarBytes = 640;
 
 template <int TYPE>
 struct XW;  // kTerms: fp16 terms per weight; kBlock: bytes of 256 columns; kBox: bytes a TMA box (or a fetched row) holds
@@ -71,7 +81,7 @@ struct XW<T_MXFP4> {
 };
 
 // Row strides are odd multiples of 16 bytes, so that 16-byte reads of 8 consecutive rows meet no bank twice.
-template <int TYPE, int BN, bool kFetch>
+template <int TYPE, int BN, bool kFetch, int kRuns>
 struct XTile {
     static constexpr uint32_t kRow = kFetch ? XW<TYPE>::kFetchRow : XW<TYPE>::kTmaRow;
     // With few tokens a block's MMAs are short and the chain unpack -> MMA -> stage free again would set the pace:
@@ -79,7 +89,9 @@ struct XTile {
     static constexpr int kABuf = BN == 64 ? 2 : 1;
     static constexpr int kWSlots = 2;
     static constexpr uint32_t kWBytes = kBM * kRow;
-    static constexpr int kPStride = BN == 64 ? 128 : 256;  // tensor-memory columns of one accumulator
+    // tensor-memory columns of one accumulator, and how many of them there are
+    static constexpr int kPStride = BN == 64 || kRuns == 4 ? 128 : 256, kPBufs = kRuns == 4 ? 4 : 2;
+    static_assert(kRuns == 1 || BN <= (XW<TYPE>::kTerms == 1 ? 128 : 64), "an accumulator for every run, a stage for every fill of a block");
     static constexpr uint32_t kMinOffset = kABuf * kAStages * kABytes;
     static constexpr uint32_t kMinBytes = kBM * 64;  // 32 columns: 64-byte rows, 64-byte swizzle; two of them
     static constexpr uint32_t kWOffset = kMinOffset + (XW<TYPE>::kMin ? 2 * kMinBytes : 0);
@@ -87,7 +99,7 @@ struct XTile {
     // The rest is a ring of activation slots of 64 columns of a CTA's n_tile / 2 tokens (128 bytes per token and term):
     // as many as fit (small tiles need more of them in flight), at most 16.
     static constexpr uint32_t kSmemBytes = 232448u;
-    static constexpr uint32_t kBRoom = kSmemBytes - 1024u - 512u - kBOffset;
+    static constexpr uint32_t kBRoom = kSmemBytes - 1024u - kXBarBytes - kBOffset;
     static_assert(kBRoom >= 2 * BN * 128, "two slots of the widest tile");
     static constexpr uint32_t kBarOffset = kBOffset + kBRoom;
 };
@@ -97,11 +109,11 @@ struct XBars {
     uint64_t full_m[2], empty_m[2];
     uint64_t full_w[2], empty_w[2];
     uint64_t full_b[16], empty_b[16];
-    uint64_t accum[2], pfree[2];
+    uint64_t accum[4], pfree[4];
     uint32_t tmem_base;
     volatile uint32_t failed;
 };
-static_assert(sizeof(XBars) <= 512, "the tiles reserve 512 bytes for the barrier block");
+static_assert(sizeof(XBars) <= kXBarBytes, "the tiles reserve these bytes for the barrier block");
 
 struct XArgs {
     const uint8_t* A;
@@ -282,11 +294,11 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
                  : "memory");
 }
 
-template <int TYPE, int BN, bool kFetch>
+template <int TYPE, int BN, bool kFetch, int kRuns>
 __global__ void __launch_bounds__(kXThreads, 1)
 gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_m,
                   const __grid_constant__ CUtensorMap tmap_w, const XArgs g) {
-    using T = XTile<TYPE, BN, kFetch>;
+    using T = XTile<TYPE, BN, kFetch, kRuns>;
     constexpr int kTerms = XW<TYPE>::kTerms;
     constexpr bool kMin = XW<TYPE>::kMin;
     constexpr uint32_t kBlock = XW<TYPE>::kBlock, kRow = T::kRow;
@@ -317,9 +329,11 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         for (int s = 0; s < 2; ++s) {
             mbar_init(&bars->full_w[s], kFetch ? 512 : 1);
             mbar_init(&bars->empty_w[s], 16);
-            mbar_init(&bars->accum[s], 1);
             mbar_init(&bars->full_m[s], 32);
             mbar_init(&bars->empty_m[s], 1);
+        }
+        for (int s = 0; s < T::kPBufs; ++s) {
+            mbar_init(&bars->accum[s], 1);
             mbar_init(&bars->pfree[s], 32);  // the sixteen producer warps of both CTAs
         }
         bars->failed = 0;
@@ -327,7 +341,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)),
-                     "r"((uint32_t)(2 * T::kPStride))
+                     "r"((uint32_t)(T::kPBufs * T::kPStride))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
@@ -342,7 +356,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             // ---- MMA issuer (even CTA). Two-term activations: up to 128 tokens the terms lie side by side on the MMA's
             // N (half the instructions; an instruction costs the issuer some 70 cycles whatever its N), above that they
             // are two instructions into the same columns. ----
-            const bool two = g.terms == 2, merged = two && g.n_tile <= 128;
+            const bool two = g.terms == 2, merged = kRuns == 1 && two && g.n_tile <= 128;
             const uint32_t n_mma = merged ? 2 * g.n_tile : g.n_tile;
             const uint32_t idesc = (1u << 4) | ((n_mma >> 3) << 17) | ((256u >> 4) << 24);  // fp16 x fp16 -> f32
             const uint32_t lo = two && !merged ? (g.n_tile / 2) * 128 / 16 : 0;  // descriptor step to the low terms
@@ -352,70 +366,126 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             bool ok = true;
             const uint32_t total = u_end - u_begin;
             for (uint32_t gb = 0; gb < total && ok; ++gb) {
-                const uint32_t d = tmem + (gb & 1) * T::kPStride;
-                uint64_t db = 0;
-                constexpr int kSteps = kTerms == 1 ? 4 : 8;
+                if constexpr (kRuns == 1) {
+                    const uint32_t d = tmem + (gb & 1) * T::kPStride;
+                    uint64_t db = 0;
+                    constexpr int kSteps = kTerms == 1 ? 4 : 8;
 #pragma unroll
-                for (int st = 0; st < kSteps; ++st) {
-                    // fill number f of set st % 4; its stage f % kABuf
-                    const uint32_t f = kTerms == 1 ? gb : 2 * gb + (st >> 2);
-                    const uint32_t sa = (st & 3) * T::kABuf + f % T::kABuf;
-                    const bool open = kTerms == 1 || (st & 1) == 0;  // an activation slot serves two 32-column steps
-                    const bool close = kTerms == 1 || (st & 1) == 1;
-                    // lane 0 watches the weight stage, lane 1 the activation slot, lane 2 the accumulator
-                    uint32_t bar = full_a + sa * 8, par = (f / T::kABuf) & 1;
-                    if (open && lane == 1) {
-                        bar = full_b + sb * 8;
-                        par = pb;
-                    }
-                    if (st == 0 && lane == 2 && gb >= 2) {
-                        bar = smem_u32(&bars->pfree[gb & 1]);
-                        par = ((gb >> 1) - 1) & 1;
-                    }
-                    ok = warp_poll(bar, par, bars, g.status, 301);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (open) db = desc_b + sb * (b_bytes >> 4);
-                    if (elect_one()) {
-                        const uint64_t da = desc_a + sa * (kABytes >> 4);
-                        if constexpr (kTerms == 1) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, (uint32_t)(st | k));
-                                if (lo) umma_bf16_pair(d, da + 2 * k, db + lo + 2 * k, idesc, 1u);
-                            }
-                        } else {
-                            const uint64_t dx = db + 4 * (st & 1);
-#pragma unroll
-                            for (int k = 0; k < 2; ++k) {
-                                umma_bf16_pair(d, da + 2 * k, dx + 2 * k, idesc, (uint32_t)(st | k));
-                                umma_bf16_pair(d, da + 4 + 2 * k, dx + 2 * k, idesc, 1u);
-                                if (lo) umma_bf16_pair(d, da + 2 * k, dx + lo + 2 * k, idesc, 1u);
-                            }
+                    for (int st = 0; st < kSteps; ++st) {
+                        // fill number f of set st % 4; its stage f % kABuf
+                        const uint32_t f = kTerms == 1 ? gb : 2 * gb + (st >> 2);
+                        const uint32_t sa = (st & 3) * T::kABuf + f % T::kABuf;
+                        const bool open = kTerms == 1 || (st & 1) == 0;  // an activation slot serves two 32-column steps
+                        const bool close = kTerms == 1 || (st & 1) == 1;
+                        // lane 0 watches the weight stage, lane 1 the activation slot, lane 2 the accumulator
+                        uint32_t bar = full_a + sa * 8, par = (f / T::kABuf) & 1;
+                        if (open && lane == 1) {
+                            bar = full_b + sb * 8;
+                            par = pb;
                         }
-                        umma_commit_pair(&bars->empty_a[sa]);
-                        if (close) umma_commit_pair(&bars->empty_b[sb]);
-                        if (!kMin && st == kSteps - 1) umma_commit_pair(&bars->accum[gb & 1]);
+                        if (st == 0 && lane == 2 && gb >= 2) {
+                            bar = smem_u32(&bars->pfree[gb & 1]);
+                            par = ((gb >> 1) - 1) & 1;
+                        }
+                        ok = warp_poll(bar, par, bars, g.status, 301);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (open) db = desc_b + sb * (b_bytes >> 4);
+                        if (elect_one()) {
+                            const uint64_t da = desc_a + sa * (kABytes >> 4);
+                            if constexpr (kTerms == 1) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, (uint32_t)(st | k));
+                                    if (lo) umma_bf16_pair(d, da + 2 * k, db + lo + 2 * k, idesc, 1u);
+                                }
+                            } else {
+                                const uint64_t dx = db + 4 * (st & 1);
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) {
+                                    umma_bf16_pair(d, da + 2 * k, dx + 2 * k, idesc, (uint32_t)(st | k));
+                                    umma_bf16_pair(d, da + 4 + 2 * k, dx + 2 * k, idesc, 1u);
+                                    if (lo) umma_bf16_pair(d, da + 2 * k, dx + lo + 2 * k, idesc, 1u);
+                                }
+                            }
+                            umma_commit_pair(&bars->empty_a[sa]);
+                            if (close) umma_commit_pair(&bars->empty_b[sb]);
+                            if (!kMin && st == kSteps - 1) umma_commit_pair(&bars->accum[gb & 1]);
+                        }
+                        if (close && ++sb == b_slots) {
+                            sb = 0;
+                            pb ^= 1;
+                        }
                     }
-                    if (close && ++sb == b_slots) {
-                        sb = 0;
-                        pb ^= 1;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {  // a run: one stage or two of 32 columns
+                        // fill number f of the sets, its stage f % kABuf
+                        const uint32_t f = kTerms == 1 ? gb : 2 * gb + (c >> 1);
+                        const uint32_t set = kTerms == 1 ? c : 2 * (c & 1);
+                        const uint32_t sa = set * T::kABuf + f % T::kABuf, sa2 = sa + (kTerms - 1) * T::kABuf;
+                        const uint32_t d = tmem + c * T::kPStride;
+                        // lanes 0 and 3 watch the weight stages, lane 1 the activation slot, lane 2 the accumulator
+                        uint32_t bar = full_a + (lane == 3 ? sa2 : sa) * 8, par = (f / T::kABuf) & 1;
+                        if (lane == 1) {
+                            bar = full_b + sb * 8;
+                            par = pb;
+                        }
+                        if (lane == 2 && gb > 0) {
+                            bar = smem_u32(&bars->pfree[c]);
+                            par = (gb - 1) & 1;
+                        }
+                        ok = warp_poll(bar, par, bars, g.status, 301);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {  // small terms first: what they add up to is all that the accumulator rounds them by
+                            const uint64_t da = desc_a + sa * (kABytes >> 4), db = desc_b + sb * (b_bytes >> 4);
+                            if constexpr (kTerms == 1) {
+                                if (lo) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) umma_bf16_pair(d, da + 2 * k, db + lo + 2 * k, idesc, (uint32_t)k);
+                                }
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_bf16_pair(d, da + 2 * k, db + 2 * k, idesc, lo | (uint32_t)k);
+                            } else {
+                                const uint64_t da2 = desc_a + sa2 * (kABytes >> 4);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k)
+                                    umma_bf16_pair(d, (k < 2 ? da : da2) + 4 + 2 * (k & 1), db + 2 * k, idesc, (uint32_t)k);
+                                if (lo) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k)
+                                        umma_bf16_pair(d, (k < 2 ? da : da2) + 2 * (k & 1), db + lo + 2 * k, idesc, 1u);
+                                }
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_bf16_pair(d, (k < 2 ? da : da2) + 2 * (k & 1), db + 2 * k, idesc, 1u);
+                                umma_commit_pair(&bars->empty_a[sa2]);
+                            }
+                            umma_commit_pair(&bars->empty_a[sa]);
+                            umma_commit_pair(&bars->empty_b[sb]);
+                            if (!kMin || c < 3) umma_commit_pair(&bars->accum[c]);
+                        }
+                        if (++sb == b_slots) {
+                            sb = 0;
+                            pb ^= 1;
+                        }
                     }
                 }
-                if constexpr (kMin) {  // merged: these columns hold the sums' terms; the low-term columns see zeros
+                if constexpr (kMin) {  // into the last run; merged: these columns hold the sums' terms; the low-term columns see zeros
                     if (!ok) break;
                     ok = warp_poll(lane == 1 ? full_b + sb * 8 : smem_u32(&bars->full_m[gb & 1]), lane == 1 ? pb : (gb >> 1) & 1, bars,
                                    g.status, 304);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
+                        const uint32_t last = kRuns == 4 ? 3 : gb & 1, d = tmem + last * T::kPStride;
                         const uint64_t dm = smem_desc_64(smem_u32(smem + T::kMinOffset + (gb & 1) * T::kMinBytes));
                         const uint64_t ds = desc_b + sb * (b_bytes >> 4);
                         umma_bf16_pair(d, dm, ds, idesc, 1u);
                         umma_bf16_pair(d, dm + 2, ds + 2, idesc, 1u);
                         umma_commit_pair(&bars->empty_m[gb & 1]);
                         umma_commit_pair(&bars->empty_b[sb]);
-                        umma_commit_pair(&bars->accum[gb & 1]);
+                        umma_commit_pair(&bars->accum[last]);
                     }
                     if (++sb == b_slots) {
                         sb = 0;
@@ -429,7 +499,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // slot is seen in one round of polls ----
         constexpr uint32_t steps = 4u + (kMin ? 1u : 0u);
         const uint32_t half = (g.n_tile / 2) * 128;
-        const bool merged = g.terms == 2 && g.n_tile <= 128;
+        const bool merged = kRuns == 1 && g.terms == 2 && g.n_tile <= 128;
         const uint32_t fills = (u_end - u_begin) * steps;
         const uint32_t full = smem_u32(&bars->full_b[lane & 15]), full_lead = leader_addr(&bars->full_b[lane & 15]);
         const uint32_t empty = smem_u32(&bars->empty_b[lane & 15]);
@@ -494,9 +564,9 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // block scale stays in its registers. One-term types: set j owns columns 64 j .. of a block. Two-term types:
         // columns 32 j .. and 128 + 32 j .., one after the other. ----
         const int j = (warp - 3) >> 2, row = (warp & 3) * 32 + lane;
-        const bool merged = g.terms == 2 && g.n_tile <= 128;
+        const bool merged = kRuns == 1 && g.terms == 2 && g.n_tile <= 128;
         const uint32_t full_a0 = leader_addr(&bars->full_a[j * T::kABuf]);
-        const uint32_t pfree0 = leader_addr(&bars->pfree[0]), pfree1 = leader_addr(&bars->pfree[1]);
+        const uint32_t pfree0 = leader_addr(&bars->pfree[0]);
         const uint32_t full_m = kMin ? leader_addr(&bars->full_m[0]) : 0u;
         const uint64_t pitch = TYPE == T_Q8_0 || TYPE == T_MXFP4 ? (uint64_t)(g.K >> 5) * (kBlock / 8) : (uint64_t)(g.K >> 8) * kBlock;
         auto row_off = [&](uint32_t tile) {  // rows past M: computed, dropped
@@ -718,44 +788,50 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             }
             if (gb > 0) {
                 // ---- promote the previous block: registers += its scale x its sums ----
-                const uint32_t pv = gb - 1, buf = pv & 1;
-                if (!poll_or_fail(&bars->accum[buf], (pv >> 1) & 1, bars, g.status, 310)) break;
-                __syncwarp();
-                tc_fence_after();
-                // columns of this set's tokens; merged: those of their low terms n_tile / 2 further on (either CTA's
-                // tokens are [high | low] there)
-                const uint32_t q4 = g.n_tile >> 2;
-                const uint32_t ta = tmem + lane_base + buf * T::kPStride + (merged ? (j >> 1) * g.n_tile + (j & 1) * q4 : j * q4);
-                if (BN <= 128 && merged) {
+                const uint32_t pv = gb - 1;
+#pragma unroll 1
+                for (int r = 0; r < kRuns && ok; ++r) {
+                    const uint32_t buf = kRuns == 4 ? (uint32_t)r : pv & 1;
+                    ok = poll_or_fail(&bars->accum[buf], (kRuns == 4 ? pv : pv >> 1) & 1, bars, g.status, 310);
+                    if (!ok) break;
+                    __syncwarp();
+                    tc_fence_after();
+                    // columns of this set's tokens; merged: those of their low terms n_tile / 2 further on (either CTA's
+                    // tokens are [high | low] there)
+                    const uint32_t q4 = g.n_tile >> 2;
+                    const uint32_t ta = tmem + lane_base + buf * T::kPStride + (merged ? (j >> 1) * g.n_tile + (j & 1) * q4 : j * q4);
+                    if (BN <= 128 && merged) {
 #pragma unroll
-                    for (int c = 0; c < BN / 32; ++c) {
-                        if ((uint32_t)c < n8) {
-                            uint32_t v0[8], v1[8];
-                            tmem_ld8(ta + c * 8, v0);
-                            tmem_ld8(ta + c * 8 + 2 * q4, v1);
-                            tmem_ld_wait();
+                        for (int c = 0; c < BN / 32; ++c) {
+                            if ((uint32_t)c < n8) {
+                                uint32_t v0[8], v1[8];
+                                tmem_ld8(ta + c * 8, v0);
+                                tmem_ld8(ta + c * 8 + 2 * q4, v1);
+                                tmem_ld_wait();
 #pragma unroll
-                            for (int e = 0; e < 8; e += 2)
-                                fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v0[e]) + __uint_as_float(v1[e]),
-                                          __uint_as_float(v0[e + 1]) + __uint_as_float(v1[e + 1]));
+                                for (int e = 0; e < 8; e += 2)
+                                    fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v0[e]) + __uint_as_float(v1[e]),
+                                              __uint_as_float(v0[e + 1]) + __uint_as_float(v1[e + 1]));
+                            }
+                        }
+                    } else {  // pairs of groups; the second of the last pair may lie past the set's columns (read, not used)
+#pragma unroll
+                        for (int c = 0; c < BN / 32; c += 2) {
+                            if ((uint32_t)c < n8) {
+                                uint32_t v[16];
+                                tmem_ld16(ta + c * 8, v);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int e = 0; e < 16; e += 2)
+                                    fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
+                            }
                         }
                     }
-                } else {  // pairs of groups; the second of the last pair may lie past the set's columns (read, not used)
-#pragma unroll
-                    for (int c = 0; c < BN / 32; c += 2) {
-                        if ((uint32_t)c < n8) {
-                            uint32_t v[16];
-                            tmem_ld16(ta + c * 8, v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 16; e += 2)
-                                fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-                        }
-                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(pfree0 + buf * 8);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(buf ? pfree1 : pfree0);
+                if (!ok) break;
                 if (boundary) {
                     // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D ----
                     asm volatile("griddepcontrol.wait;" ::: "memory");  // D zeroed, scales written
@@ -789,14 +865,14 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     cluster_sync_all();  // the peer's MMAs read this CTA's stages, its commits arrive here
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * T::kPStride)) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(T::kPBufs * T::kPStride)) : "memory");
     }
 }
 
-template <int TYPE, int BN, bool kFetch>
+template <int TYPE, int BN, bool kFetch, int kRuns>
 cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
-    using T = XTile<TYPE, BN, kFetch>;
-    auto kern = gemm_exact_kernel<TYPE, BN, kFetch>;
+    using T = XTile<TYPE, BN, kFetch, kRuns>;
+    auto kern = gemm_exact_kernel<TYPE, BN, kFetch, kRuns>;
     static std::atomic<uint64_t> attr_done{0};
     static std::atomic<int> max_pairs[64];
     if (cudaError_t e = ensure_dynamic_smem(kern, (int)T::kSmemBytes, attr_done); e != cudaSuccess) return e;
@@ -872,9 +948,17 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
 
 template <int TYPE, bool kFetch>
 cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
-    if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch>(p, plan, prep, s);
-    if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch>(p, plan, prep, s);
-    return x_launch<TYPE, 256, kFetch>(p, plan, prep, s);
+    if (p.fine) {
+        // Two-term types: with one stage per set (tiles above 64 tokens) the second half of a block could be filled only after
+        // the first two runs' accumulators, which the filling warps give back later, are free again: not beyond 64.
+        if constexpr (XW<TYPE>::kTerms == 1) {
+            if (plan.n_tile > 64) return x_launch<TYPE, 128, kFetch, 4>(p, plan, prep, s);
+        }
+        return plan.n_tile <= 64 ? x_launch<TYPE, 64, kFetch, 4>(p, plan, prep, s) : cudaErrorInvalidConfiguration;
+    }
+    if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch, 1>(p, plan, prep, s);
+    if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch, 1>(p, plan, prep, s);
+    return x_launch<TYPE, 256, kFetch, 1>(p, plan, prep, s);
 }
 
 }  // namespace

@@ -331,6 +331,7 @@ struct ExactGemm {
     float* D;
     uint32_t M, N, K, stride_b, stride_d;
     bool bf16;
+    bool fine;         // short accumulations: as near to the exact result as f32 sums by lanes (zc_dmmv_batch)
     uint32_t* status;
 };
 struct XPlan {
