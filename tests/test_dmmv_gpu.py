@@ -448,3 +448,23 @@ def test_batch_few_columns(gpu, oracle, t, M, K, cols):
     ctx.submit_and_wait()
     assert canary_intact(Y, cols * M)
     assert rel_l2(Y[:cols * M].cpu().numpy().reshape(cols, M), oracle.gemm_f64(w, t, M, K, X)) <= TOL
+
+
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q6_K, zb.MXFP4], ids=["q4_k", "q6_k", "mxfp4"])
+@pytest.mark.parametrize("M,K,cols", [(2048, 14336, 1), (700, 12544, 1), (1400, 4096, 2)])
+def test_long_rows_and_two_columns_keep_f32(gpu, oracle, t, M, K, cols):
+    """Matvecs past the streaming kernels' range (K = 12288) and batches of two columns hold x in f32 or 22 bits, not in 21
+    bits of fixed point: 2.5e-7 (test_dmmv_batch_is_as_accurate_as_f32_sums; f32 sums by lanes have half of it), where 21
+    bits leave 1.1e-6."""
+    torch, ctx, dd = gpu
+    g = synth.rng(130, t + K)
+    w = synth.quant_matrix(g, t, M, K)
+    X = synth.activations(g, cols, K)
+    Y = out_with_canary(torch, cols * M)
+    if cols == 1:
+        dd.recordDispatch(t, dev(torch, w), dev(torch, X), Y, M, K)
+    else:
+        dd.recordBatchDispatchPush(t, dev(torch, w), dev(torch, X), Y, M, K, 0, 0, 0, cols)
+    ctx.submit_and_wait()
+    assert canary_intact(Y, cols * M)
+    assert rel_l2(Y[:cols * M].cpu().numpy(), oracle.gemm_f64(w, t, M, K, X)) <= 2.5e-7

@@ -276,7 +276,11 @@ cudaError_t launch_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t
         if (ec != cudaSuccess) return ec;
     }
     cudaError_t e;
-    if (mode == MODE_PLAIN && row_dmmv_eligible(type, a)) {
+    // Large Q4_K and Q6_K matrices come this far with K beyond the streaming kernels' range or without their alignment: one
+    // warp per row with whole blocks per lane has shorter sums there and, Q6_K, half the instructions (4096 x 14336 42 us
+    // against 68 on the row kernel).
+    const bool large_k = (type == T_Q4_K || type == T_Q6_K) && wbytes >= kStreamMinBytes;
+    if (mode == MODE_PLAIN && !large_k && row_dmmv_eligible(type, a)) {
         e = launch_row_dmmv(type, a, s);
         if (e == cudaSuccess && launches) ++*launches;
         return e;

@@ -323,7 +323,7 @@ bool q6k_dmmv_eligible(uint32_t type, int mode, const DmmvArgs& a) {
     if (!a.status) return false;
     if (reinterpret_cast<uintptr_t>(a.A) & 15u) return false;  // supersets are fetched in 16-byte pieces from the base
     if (((a.K >> 8) % 8u) != 0 && !a.a_end) return false;      // unaligned rows: the end of the buffer must be known
-    return slice_fits<FmtQ6K<true>>(a.K, 1, 1);
+    return a.K <= kFixedPointMaxK && slice_fits<FmtQ6K<true>>(a.K, 1, 1);
 }
 
 // MoE down projection + weighted accumulate (y += sum_s w_s W[routing[s]] x_s) through the streaming kernel.
@@ -333,7 +333,7 @@ bool q6k_moe_down_acc_eligible(uint32_t type, const DmmvArgs& a) {
     if ((a.x_expert_stride & 3u) || (reinterpret_cast<uintptr_t>(a.x) & 15u)) return false;
     if (a.A_sh && ((reinterpret_cast<uintptr_t>(a.A_sh) & 15u) || !a.a_sh_end)) return false;
     if ((uint64_t)a.M * (a.K >> 8) * a.n_used * 210u < kStreamMinBytes) return false;  // small expert sets: latency-bound either way
-    return slice_fits<FmtQ6K<false>>(a.K, a.n_used, 1);
+    return (uint64_t)a.K * a.n_used <= kFixedPointMaxK && slice_fits<FmtQ6K<false>>(a.K, a.n_used, 1);
 }
 
 cudaError_t launch_q6k_moe_down_acc(const DmmvArgs& a, cudaStream_t st, uint64_t* launches) {

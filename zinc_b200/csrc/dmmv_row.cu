@@ -1,5 +1,5 @@
-// Row matvec: y (+)= W x for the sizes and types the streaming kernels leave: every matrix of a few hundred KB, and Q5_K
-// and Q8_0 of any size (src/shaders/dmmv_q8_0.comp:80-108, dmmv_q5k.comp and their siblings).
+// Row matvec: y (+)= W x for the sizes and types the streaming kernels leave: every matrix below 2 MB, and Q5_K and Q8_0 of
+// any size (src/shaders/dmmv_q8_0.comp:80-108, dmmv_q5k.comp and their siblings).
 //
 // A warp covers 256 columns of a row per step, eight weights per lane, all lanes' bytes contiguous. Weights become floats
 // exactly (a byte permuted under the exponent of 2^23, one subtraction) and meet x in f32, two at a time. NR rows per warp

@@ -455,6 +455,10 @@ cudaError_t slice_launch(SliceArgs a, int sm_count, cudaStream_t s) {
     return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
 }
 
+// How far the formats reach whose x is 21-bit fixed point per 256 elements (Q4_K, Q6_K; relative L2 error 1.1e-6, f32 sums
+// 1.2e-7): the longest (concatenated) x, and the fewest units of 16 rows x 512 columns. Beyond, the row kernels' f32.
+constexpr uint32_t kFixedPointMaxK = 12288, kFixedPointMinUnits = 16;
+
 // Does the activation of a launch fit beside two units per warp?
 template <typename F>
 bool slice_fits(uint32_t K, uint32_t slots, int NS) {

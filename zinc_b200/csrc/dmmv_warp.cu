@@ -268,6 +268,7 @@ struct FmtQ4K {
 };
 
 bool base_ok(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+uint64_t units(uint32_t M, uint32_t K) { return (uint64_t)((M + 15) / 16) * ((K / 256 + kCB - 1) / kCB); }
 
 }  // namespace
 
@@ -279,7 +280,7 @@ bool warp_dmmv_eligible(uint32_t type, int mode, const DmmvArgs& a) {
     if (mode != MODE_PLAIN && mode != MODE_GATE_UP_SWIGLU && mode != MODE_SIGMOID_ACC) return false;
     if (!a.status || !base_ok(a.A) || !base_ok(a.A2)) return false;
     const int ns = mode == MODE_GATE_UP_SWIGLU ? 2 : 1;
-    return slice_fits<FmtQ4K>(a.K, 1, ns);
+    return a.K <= kFixedPointMaxK && units(a.M, a.K) * ns >= kFixedPointMinUnits && slice_fits<FmtQ4K>(a.K, 1, ns);
 }
 
 cudaError_t launch_warp_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t st, uint64_t* launches) {
@@ -310,10 +311,13 @@ cudaError_t launch_warp_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStr
 // Grouped launch: n <= 3 Q4_K matrices with the same K and the same x, y_i = W_i x, in one kernel.
 bool warp_dmmv_multi_eligible(uint32_t type, uint32_t n, const uint8_t* const* A, const uint32_t* M, uint32_t K,
                               const DmmvArgs& common) {
-    if (type != T_Q4_K || n < 2 || n > 3 || (K & 255u) || !common.status) return false;
-    for (uint32_t i = 0; i < n; ++i)
+    if (type != T_Q4_K || n < 2 || n > 3 || (K & 255u) || K > kFixedPointMaxK || !common.status) return false;
+    uint64_t u = 0;
+    for (uint32_t i = 0; i < n; ++i) {
         if (!base_ok(A[i]) || M[i] == 0) return false;
-    return slice_fits<FmtQ4K>(K, 1, 1);
+        u += units(M[i], K);
+    }
+    return u >= kFixedPointMinUnits && slice_fits<FmtQ4K>(K, 1, 1);
 }
 
 cudaError_t launch_warp_dmmv_multi(uint32_t n, const uint8_t* const* A, float* const* y, const uint32_t* M,
@@ -336,7 +340,7 @@ bool warp_moe_gate_up_eligible(uint32_t type, const DmmvArgs& a) {
         return false;
     if (!base_ok(a.A) || !base_ok(a.A2) || (a.expert_stride & 15u) || !base_ok(a.A_sh) || !base_ok(a.A2_sh) || (a.K & 255u))
         return false;
-    return slice_fits<FmtQ4K>(a.K, 1, 2);
+    return a.K <= kFixedPointMaxK && units(a.M, a.K) * a.n_used * 2 >= kFixedPointMinUnits && slice_fits<FmtQ4K>(a.K, 1, 2);
 }
 
 cudaError_t launch_warp_moe_gate_up(const DmmvArgs& a, cudaStream_t st, uint64_t* launches) {

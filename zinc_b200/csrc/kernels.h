@@ -155,7 +155,7 @@ cudaError_t launch_q6k_dmmv(int mode, const DmmvArgs& a, cudaStream_t s, uint64_
 bool q6k_moe_down_acc_eligible(uint32_t type, const DmmvArgs& a);
 cudaError_t launch_q6k_moe_down_acc(const DmmvArgs& a, cudaStream_t s, uint64_t* launches);
 
-// MODE_PLAIN on the row kernel (dmmv_row.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4, any size.
+// MODE_PLAIN on the row kernel (dmmv_row.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4.
 bool row_dmmv_eligible(uint32_t type, const DmmvArgs& a);
 cudaError_t launch_row_dmmv(uint32_t type, const DmmvArgs& a, cudaStream_t s);
 
