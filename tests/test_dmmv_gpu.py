@@ -468,3 +468,61 @@ def test_long_rows_and_two_columns_keep_f32(gpu, oracle, t, M, K, cols):
     ctx.submit_and_wait()
     assert canary_intact(Y, cols * M)
     assert rel_l2(Y[:cols * M].cpu().numpy(), oracle.gemm_f64(w, t, M, K, X)) <= 2.5e-7
+
+
+@pytest.mark.parametrize("t,M,K", [(zb.Q4_K, 8200, 512), (zb.Q4_K, 18950, 768), (zb.Q4_K, 7110, 4352), (zb.Q6_K, 10001, 256),
+                                   (zb.Q6_K, 4741, 2048), (zb.Q6_K, 9999, 1792), (zb.Q6_K, 10667, 8192), (zb.MXFP4, 8010, 512),
+                                   (zb.MXFP4, 4100, 992), (zb.MXFP4, 23690, 1056)],
+                         ids=lambda v: zb.TYPE_NAMES.get(v, str(v)) if isinstance(v, int) and v < 64 else str(v))
+def test_many_tiles_per_cta(gpu, oracle, t, M, K):
+    """The streaming form whose warps own ranges of their CTA's tiles (148 SMs: the first sizes of every format that take it,
+    one and several blocks per row, a last tile of few rows): tiles of one warp, of two, of three and more; CTAs with fewer
+    units than warps. Stored and accumulated, and the same bits again."""
+    torch, ctx, dd = gpu
+    g = synth.rng(131, t * 31 + M)
+    w = synth.quant_matrix(g, t, M, K)
+    x = synth.activations(g, K)
+    wd, xd = dev(torch, w), dev(torch, x)
+    y, y2, z = out_with_canary(torch, M), out_with_canary(torch, M), out_with_canary(torch, M, init=1.5)
+    dd.recordDispatch(t, wd, xd, y, M, K)
+    dd.recordDispatch(t, wd, xd, y2, M, K)
+    dd.recordDispatch(t, wd, xd, z, M, K, acc_mode=1)
+    ctx.submit_and_wait()
+    want = oracle.dmmv_f64(w, t, M, K, x)
+    assert canary_intact(y, M) and canary_intact(z, M)
+    got = y[:M].cpu().numpy()
+    assert rel_l2(got, want) <= TOL
+    for lo in range(0, M, 1021):   # and everywhere alike
+        assert rel_l2(got[lo:lo + 1021], want[lo:lo + 1021]) <= TOL
+    assert torch.equal(y[:M], y2[:M])
+    assert np.array_equal(z[:M].cpu().numpy(), np.float32(1.5) + got)
+
+
+@pytest.mark.parametrize("M,K", [(9475, 768), (9500, 2048), (3600, 6144)])
+def test_many_tiles_per_cta_gate_up(gpu, oracle, M, K):
+    torch, ctx, dd = gpu
+    g = synth.rng(132, M)
+    wg, wu = synth.quant_matrix(g, zb.Q4_K, M, K), synth.quant_matrix(g, zb.Q4_K, M, K)
+    x = synth.activations(g, K) * np.float32(0.25)
+    y = out_with_canary(torch, M)
+    dd.dispatchDmmvFusedGateUpSwiglu(zb.Q4_K, dev(torch, wg), dev(torch, wu), dev(torch, x), y, M, K)
+    ctx.submit_and_wait()
+    a, b = oracle.dmmv_f64(wg, zb.Q4_K, M, K, x), oracle.dmmv_f64(wu, zb.Q4_K, M, K, x)
+    assert canary_intact(y, M)
+    assert rel_l2(y[:M].cpu().numpy(), a / (1 + np.exp(-a)) * b) <= TOL
+
+
+@pytest.mark.parametrize("t,M,K", [(zb.Q4_K, 12000, 512), (zb.Q6_K, 4750, 2048)], ids=["q4_k", "q6_k"])
+def test_many_tiles_per_cta_sigmoid(gpu, oracle, t, M, K):
+    torch, ctx, dd = gpu
+    g = synth.rng(133, M)
+    w, x = synth.quant_matrix(g, t, M, K), synth.activations(g, K)
+    y0 = synth.activations(g, M)
+    y = out_with_canary(torch, M)
+    y[:M] = dev(torch, y0)
+    gate = np.array([9.0, -0.7], np.float32)
+    dd.dispatchDmmvSigmoidAcc(t, dev(torch, w), dev(torch, x), y, dev(torch, gate), M, K, gate_index=1)
+    ctx.submit_and_wait()
+    want = y0 + oracle.dmmv_f64(w, t, M, K, x) / (1 + np.exp(0.7))
+    assert canary_intact(y, M)
+    assert rel_l2(y[:M].cpu().numpy(), want) <= TOL

@@ -195,6 +195,8 @@ struct FmtQ6K {
     static constexpr uint32_t kSlot = 16 * kRow6;
     static constexpr uint32_t kMost = 16;
     static constexpr uint32_t kCols = 256;
+    static constexpr bool kFlowOne = true;
+    static uint32_t flow_tiles(uint32_t) { return 2; }
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes6 + nblk * (kBBytes + kNsxBytes + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
@@ -235,6 +237,13 @@ struct FmtQ6K {
             if constexpr (kAligned) {
                 const uint32_t o = (u.lb * 210u) & 15u, room = row_bytes - (u.lb * 210u - o);
                 const uint8_t* p = first - o;
+                if (u.rows == 16 && room >= kPieces6 * 16u) {  // away from the ends of the matrix and of its rows
+#pragma unroll
+                    for (int i = 0; i < kPiecesLane6; ++i)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + row[i] * kRow6 + col[i]), "l"(p + src[i])
+                                     : "memory");
+                    return;
+                }
 #pragma unroll
                 for (int i = 0; i < kPiecesLane6; ++i)
                     if (row[i] < u.rows && col[i] < room)  // rows are 16-byte aligned: a piece never crosses the row end

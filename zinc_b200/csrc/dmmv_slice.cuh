@@ -351,6 +351,151 @@ __device__ __forceinline__ void slice_body(const SliceArgs& a, const Extra& extr
 }
 
 struct NoExtra {};
+
+// The form for many tiles per CTA, of one matrix (or pair): the CTA's units (16 rows x one block, tile by tile) are dealt to
+// its warps in equal contiguous ranges. A warp writes the tiles it has to itself; of the at most two it shares with its
+// neighbours, the parts meet in shared memory once, at the end, and are added in the order of the warps. No warp waits for
+// another on the way, and none has more than one unit more to do than the next. A unit is requested into the slot that has
+// just been read, so that the whole ring is in flight while a unit's sums are finished.
+// (The tiles of a CTA shared by all its warps with a meeting every few of them, as above: LM head Q6_K 151936 x 4096 109.9
+// us, here 99.4; Q4_K 40000 x 2816 16.6 and 14.3.)
+template <typename F, int NS, int EPI>
+__device__ __forceinline__ void flow_body(const SliceArgs& a) {
+    extern __shared__ uint8_t smem_raw[];
+    pdl_begin(a.late);
+    uint8_t* base = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    const uint32_t n_warps = blockDim.x >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t* ring = base + (size_t)warp * a.depth * F::kSlot;
+    float* spart = reinterpret_cast<float*>(base + (size_t)n_warps * a.depth * F::kSlot);  // [warp][first, last range][NS * 16]
+    const typename F::Tab tab = F::carve(reinterpret_cast<uint8_t*>(spart + n_warps * 2 * NS * 16), a.nblk);
+    const uint32_t ct0 = (uint32_t)part_begin(blockIdx.x, a.tiles, gridDim.x);
+    const uint32_t U = ((uint32_t)part_begin(blockIdx.x + 1, a.tiles, gridDim.x) - ct0) * a.nblk;
+    auto begin_of = [&](uint32_t w) { return w * U / n_warps; };
+    const uint32_t u0 = begin_of(warp), u1 = begin_of(warp + 1);
+
+    typename F::Copier copier;
+    copier.init(a, lane);
+    typename F::Lane ln;
+    ln.init(a, tab, lane);
+    pdl_late(a.late);
+    auto unit = [&](uint32_t tl, uint32_t strm, uint32_t kb) {
+        Unit u;
+        u.mat = a.A[NS == 2 ? strm : 0];
+        u.end = a.a_end[NS == 2 ? strm : 0];
+        u.row0 = (ct0 + tl) * 16;
+        u.rows = min(16u, a.M - u.row0);
+        u.lb = u.kb = kb;
+        return u;
+    };
+    uint32_t p_u = u0, p_tl = u0 / a.nblk, p_kb = u0 - p_tl * a.nblk, p_strm = 0;  // the unit to request next
+    uint32_t u = u0, tl = p_tl, kb = p_kb, strm = 0;                               // the unit to work off next
+    uint32_t kb0 = kb, seg = 0;                                                    // the range: where it began, its number
+    auto request = [&](uint32_t slot) {
+        if (p_u < u1) {
+            copier.copy(a, unit(p_tl, p_strm, p_kb), ring + slot * F::kSlot, lane);
+            if (NS == 1 || ++p_strm == NS) {
+                p_strm = 0;
+                ++p_u;
+                if (++p_kb == a.nblk) {
+                    p_kb = 0;
+                    ++p_tl;
+                }
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll 1
+    for (uint32_t i = 0; i < a.depth; ++i) request(i);
+    if (!a.late) pdl_wait();
+    // ---- the activation ----
+    const uint32_t n_prep = F::prep_count(a);
+    typename F::X x;
+    if ((uint32_t)warp < n_prep) F::template load_x<0>(x, a, NoExtra(), warp, lane);
+    if (a.consume.n) consume_pushed(a.consume, blockIdx.x, gridDim.x, tid, blockDim.x);
+    F::clear(tab, tid);
+    for (uint32_t b = warp; b < n_prep; b += n_warps) {
+        typename F::X next;
+        if (b + n_warps < n_prep) F::template load_x<0>(next, a, NoExtra(), b + n_warps, lane);
+        F::prep(tab, x, a, b, lane);
+        x = next;
+    }
+    __syncthreads();
+
+    typename F::Acc acc, other;  // of the stream at hand, of the other one
+    acc.clear();
+    other.clear();
+    for (uint32_t slot = 0; u < u1;) {
+        if (a.depth == 2) cp_async_wait<1>();
+        else if (a.depth == 3) cp_async_wait<2>();
+        else cp_async_wait<3>();
+        __syncwarp();
+        ln.dot(a, unit(tl, strm, kb), smem_u32(ring) + slot * F::kSlot, acc);
+        __syncwarp();
+        request(slot);  // into the slot just read
+        if (++slot == a.depth) slot = 0;
+        if (NS == 2) {
+            const typename F::Acc t = acc;
+            acc = other;
+            other = t;
+            if (++strm < NS) continue;
+            strm = 0;
+        }
+        ++u;
+        if (++kb < a.nblk && u < u1) continue;
+        // ---- the warp's part of a tile is complete ----
+        float v[NS][2];
+        ln.finish(acc, v[0][0], v[0][1]);
+        if (NS == 2) ln.finish(other, v[NS - 1][0], v[NS - 1][1]);
+        acc.clear();
+        other.clear();
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {  // rows g and g + 8, the four lanes' shares
+                v[s][i] += __shfl_xor_sync(0xFFFFFFFFu, v[s][i], 1);
+                v[s][i] += __shfl_xor_sync(0xFFFFFFFFu, v[s][i], 2);
+            }
+        const uint32_t half = lane & 3, rr = (lane >> 2) + 8 * (half & 1);  // lanes 0 and 1 of a row's four: rows g and g + 8
+        float r[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) r[s] = half ? v[s][1] : v[s][0];
+        if (kb0 == 0 && kb == a.nblk) {
+            write_out<NS, EPI>(a, out_row<EPI, 0>(a, ct0 + tl, rr, half < 2), r);
+        } else if (half < 2) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s) spart[((warp * 2 + (seg ? 1 : 0)) * NS + s) * 16 + rr] = r[s];
+        }
+        ++seg;
+        kb0 = 0;
+        if (kb == a.nblk) {
+            kb = 0;
+            ++tl;
+        }
+    }
+    // ---- the shared tiles: 16 threads for each, at the first border between warps that lies inside it ----
+    const uint32_t b = (uint32_t)(tid >> 4) + 1, ub = begin_of(b), t0 = ub / a.nblk * a.nblk;  // b, its unit, its tile's first
+    const bool mine = b < n_warps && ub != t0 && begin_of(b - 1) <= t0;
+    const OutRow o = out_row<EPI, 0>(a, ct0 + t0 / a.nblk, tid & 15u, mine);
+    __syncthreads();
+    if (!mine) return;
+    float sum[NS];
+    const float* p = spart + ((b - 1) * 2 + (begin_of(b - 1) == t0 ? 0 : 1)) * NS * 16 + (tid & 15u);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) sum[s] = p[s * 16];
+    for (uint32_t w = b; w < n_warps && begin_of(w) < t0 + a.nblk; ++w) {
+        if (begin_of(w) == begin_of(w + 1)) continue;  // fewer units than warps
+        p = spart + w * 2 * NS * 16 + (tid & 15u);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) sum[s] += p[s * 16];
+    }
+    write_out<NS, EPI>(a, o, sum);
+}
+template <typename F, int NS, int EPI, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_flow_kernel(const SliceArgs a) {
+    flow_body<F, NS, EPI>(a);
+}
+
 template <typename F, int NS, int EPI, int kSeg, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_slice_kernel(const SliceArgs a) {
     slice_body<F, NS, EPI, kSeg>(a, NoExtra());
@@ -388,19 +533,19 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
         smem = fixed + warps * a.depth * F::kSlot;
         return true;
     };
-    // Tall matrices (several tiles per CTA either way): the cut whose busiest warp has least to do, tiles of a CTA dealt to
-    // n_wr rows of warps, a longer share of K for each where more rows of warps fit; meetings every eight tiles or so.
-    // (Q4_K 65536 x 4096 29.6 -> 27.7 us, Q6_K 151936 x 4096 114.8 -> 109.1 against the cut below.)
+    // Four tiles per CTA and more: the cut whose busiest warp has least to do, tiles of a CTA dealt to n_wr rows of warps, a
+    // longer share of K for each where more rows of warps fit; meetings every eight tiles or so. (Q4_K 8192 x 12288 16.3 ->
+    // 14.6 us, 11008 x 5120 12.2 -> 10.1, 65536 x 8192 53.8 -> 52.1 against the cut below.)
+    const uint32_t tpc16 = ((a.M + 15) / 16 + sms * per_sm - 1) / (sms * per_sm);
     uint32_t tall_per = 0, tall_wr = 0;
-    if (kSeg == 0 && a.M >= 16000) {
-        const uint32_t tpc = ((a.M + 15) / 16 + sms * per_sm - 1) / (sms * per_sm);
+    if (kSeg == 0 && tpc16 >= 4) {
         uint32_t least = 0xFFFFFFFFu;
         for (uint32_t p = a.nblk < per * 4 ? a.nblk : per * 4; p >= per; --p) {
             const uint32_t wk = (a.nblk + p - 1) / p;
             for (uint32_t wr = 1; wr <= 4 && wr * wk <= most; ++wr) {
                 // by 5 % at least: between equals the longer share (Q6_K 151936 x 4096: 109 us, 112 with all warps along K)
-                if ((uint64_t)((tpc + wr - 1) / wr * p) * 20 < (uint64_t)least * 19 && cut(p, wr, wr == 3 ? 9 : 8)) {
-                    least = (tpc + wr - 1) / wr * p;
+                if ((uint64_t)((tpc16 + wr - 1) / wr * p) * 20 < (uint64_t)least * 19 && cut(p, wr, wr == 3 ? 9 : 8)) {
+                    least = (tpc16 + wr - 1) / wr * p;
                     tall_per = p;
                     tall_wr = wr;
                 }
@@ -440,9 +585,62 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
     return true;
 }
 
+// The cut of the other form (flow_body), where it is the faster one: many tiles per SM.
+// F::flow_tiles(K): from how many tiles per SM (both streams counted) eight warps on each of two CTAs are ahead where x fits
+// twice on an SM. Measured over 250 shapes, this form against the one above:
+//   Q4_K   K <= 512 always (65536 rows 6.2 and 9.2 us: most warps had no block); K <= 4096 from 8 (K = 4096, 16500 rows 10.4
+//          and 10.2, 20000 rows 11.7 and 12.7, 28672 rows 14.9 and 16.6), beyond from 3 (5120 x 5120 7.5 and 7.7, 14336 x
+//          5120 11.3 and 12.9)
+//   Q6_K   from 2 (5120 x 2816 8.4 and 9.4, 8192 x 4608 13.8 and 17.7, 21669 x 4608 29.6 and 34.2, 128256 x 3072 87.6 and
+//          105.9, 151936 x 4096 99.4 and 109.9; the other way 20000 x 5120 31.1 and 30.1)
+//   MXFP4  K <= 1024 always (20000 x 512 4.1 and 7.8), beyond from 10 (20000 x 2880 14.4 and 13.8, 28672 x 2880 19.3 and 20.4)
+// Where x fits only once, Q6_K takes one CTA of sixteen warps from 4.5 tiles per SM (8192 x 12288 25.5 and 25.0 us, 11008
+// rows 28.7 and 30.1, 28672 rows 62.3 and 70.0); the others stay above (Q4_K 65536 x 12288 76 and 74).
+template <typename F>
+bool flow_plan(SliceArgs& a, int NS, int sm_count, uint32_t& warps, uint32_t& grid, uint32_t& smem) {
+    a.nblk = a.bpe = (a.K + F::kCols - 1) / F::kCols;
+    a.tiles = (a.M + 15) / 16;
+    a.h = 16;
+    const uint32_t sms = sm_count > 0 ? (uint32_t)sm_count : 148u;
+    auto cut = [&](uint32_t n, uint32_t room) {
+        warps = n;
+        const uint32_t fixed = 128u + warps * 2u * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
+        if (fixed + warps * 2u * F::kSlot > room) return false;
+        a.depth = (room - fixed) / (warps * F::kSlot);
+        a.depth = a.depth > 4 ? 4 : a.depth;
+        smem = fixed + warps * a.depth * F::kSlot;
+        return true;
+    };
+    uint32_t ctas = 2 * sms;
+    if (cut(8, kSliceSmem2)) {
+        if (a.tiles * (uint32_t)NS < F::flow_tiles(a.K) * sms) return false;
+    } else {
+        ctas = sms;
+        if (!F::kFlowOne || a.tiles * 2 < 9 * sms || !cut(16, kSliceSmem1)) return false;
+    }
+    const uint32_t busy = (uint32_t)(((uint64_t)a.tiles * a.nblk + warps - 1) / warps);  // CTAs with a unit for every warp
+    grid = ctas < busy ? ctas : busy;
+    return true;
+}
+
 template <typename F, int NS, int EPI, int kSeg>
 cudaError_t slice_launch(SliceArgs a, int sm_count, cudaStream_t s) {
     uint32_t warps, grid, smem;
+    if constexpr (kSeg == 0) {
+        if (flow_plan<F>(a, NS, sm_count, warps, grid, smem)) {
+            static std::atomic<uint64_t> flow8{0}, flow16{0};
+            if (warps == 8) {
+                auto kern = dmmv_flow_kernel<F, NS, EPI, 8>;
+                if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, flow8); e != cudaSuccess) return e;
+                return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
+            }
+            if constexpr (F::kFlowOne) {
+                auto kern = dmmv_flow_kernel<F, NS, EPI, 16>;
+                if (cudaError_t e = ensure_dynamic_smem(kern, kSliceSmem1, flow16); e != cudaSuccess) return e;
+                return launch_chained(kern, dim3(grid), dim3(warps * 32), smem, s, a);
+            }
+        }
+    }
     if (!slice_plan<F>(a, NS, kSeg, sm_count, warps, grid, smem)) return cudaErrorInvalidConfiguration;
     static std::atomic<uint64_t> attr8{0}, attr16{0};
     if (warps <= 8) {
