@@ -344,6 +344,46 @@ def test_mul_mm_exact_same_bits_every_time(gpu, t, K):
     assert int(bad) == 0
 
 
+def test_mul_mm_exact_on_two_streams(gpu):
+    """The f32-accurate GEMM keeps the terms of its activations in the context's scratch: a call on another stream, or a
+    replay there, may not overwrite what a call still under way reads."""
+    torch, _, _ = gpu
+    M, N, K, n = 2048, 300, 2048, 24
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    ctx = zb.Context(0, stream=s1.cuda_stream)
+    dd = zb.DmmvDispatch(ctx)
+    g = synth.rng(311, 0)
+    w = dev(torch, synth.quant_matrix(g, zb.Q4_K, M, K))
+    X = [dev(torch, synth.activations(g, N, K)) for _ in range(4)]
+    want = []
+    for x in X:
+        D = torch.empty(N, M, device="cuda")
+        torch.cuda.synchronize()
+        dd.recordMulMm(zb.Q4_K, w, x, D, M, N, K, K, M)
+        ctx.submit_and_wait()
+        want.append(D)
+    Y = torch.empty(N, M, device="cuda")
+    ctx.begin_record()
+    dd.recordMulMm(zb.Q4_K, w, X[3], Y, M, N, K, K, M)
+    recording = ctx.end_record()
+    got = [torch.empty(N, M, device="cuda") for _ in range(n)]
+    torch.cuda.synchronize()
+    for i in range(n):
+        ctx.set_stream((s1, s2)[i % 2].cuda_stream)
+        if i % 5 == 4:
+            ctx.replay(recording)
+        else:
+            dd.recordMulMm(zb.Q4_K, w, X[i % 3], got[i], M, N, K, K, M)
+    torch.cuda.synchronize()
+    ctx.submit_and_wait()
+    for i in range(n):
+        if i % 5 != 4:
+            assert float((got[i] - want[i % 3]).norm() / want[i % 3].norm()) <= 1e-6
+    assert float((Y - want[3]).norm() / want[3].norm()) <= 1e-6
+    ctx.free_recording(recording)
+    ctx.close()
+
+
 def test_mul_mm_errors(gpu):
     torch, ctx, dd = gpu
     w = torch.zeros(144 * 8, dtype=torch.uint8, device="cuda")
