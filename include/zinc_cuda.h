@@ -229,7 +229,10 @@ int32_t zc_dmmv_sigmoid_acc(zc_ctx* ctx, uint32_t type,
  * recordBatchDispatchPush (src/compute/dmmv.zig:880-926) and the 40-column
  * chunk loop of dispatchProjectionBatched (src/compute/forward.zig:8147-8216):
  * num_cols is unbounded and chunking is internal. The reference supports q4_k
- * and q6_k; every K-quant and 32-block type is accepted. */
+ * and q6_k; every K-quant and 32-block type is accepted. f32 accuracy (an error
+ * of 2.5e-7 of the result and less, activations N(0, 1)); the same bits every time.
+ * Large products run on the tensor cores as in zc_mul_mm with f32 activations: an
+ * infinite activation makes its column NaN there. */
 int32_t zc_dmmv_batch(zc_ctx* ctx, uint32_t type,
                       const void* A, uint64_t a_size, const void* X, uint64_t x_size,
                       void* Y, uint64_t y_size,
@@ -244,8 +247,12 @@ int32_t zc_dmmv_batch(zc_ctx* ctx, uint32_t type,
  * act_type selects B's element type, ZC_F32 or ZC_BF16; D is f32. bf16 activations with Q4_K, Q6_K or
  * MXFP4 weights (A and B 16-byte aligned, N >= 16, stride_b a multiple of 8; MXFP4: K a multiple of 64)
  * run on the tensor cores: weights dequantised to bf16 tiles (exactly, for MXFP4), f32 accumulation in
- * tensor memory. Every other combination (f32 activations included, which keep f32 precision) runs a
- * CUDA-core kernel.
+ * tensor memory. Where few tiles share the SMs, K is split and the parts of Q4_K, of Q6_K with a multiple of 2048
+ * columns and of MXFP4 beyond 256 tokens are added in whatever order they are done: the last bits may vary there.
+ * Every other combination of Q4_K, Q5_K, Q6_K, Q8_0 and MXFP4 weights 16-byte aligned, f32 activations among them, keeps
+ * f32 accuracy on the tensor cores: activations as two fp16 terms (22 bits, down to 2^-17 of a token's largest
+ * element, an absolute error of 2^-39 of that below; an infinite one makes its token's outputs NaN), weights as one or
+ * two, and the same bits every time. The rest runs a CUDA-core kernel.
  * K must be a multiple of 256 for K-quants (InvalidArgument otherwise, as the reference). */
 int32_t zc_mul_mm(zc_ctx* ctx, uint32_t type,
                   const void* A, uint64_t a_size, const void* B, uint64_t b_size,

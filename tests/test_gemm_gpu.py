@@ -344,6 +344,36 @@ def test_mul_mm_exact_same_bits_every_time(gpu, t, K):
     assert int(bad) == 0
 
 
+@pytest.mark.parametrize("t,M,N,K,bf16", [(t, *s, False) for t in (zb.Q4_K, zb.Q6_K, zb.MXFP4) for s in
+                                          ((300, 5, 8192), (1027, 41, 3840), (4096, 64, 4096), (2048, 256, 8192), (4096, 658, 4096))] +
+                         [(zb.Q6_K, 1027, 41, 3840, True), (zb.Q6_K, 4096, 64, 11008, True), (zb.MXFP4, 1027, 41, 3840, True),
+                          (zb.MXFP4, 300, 200, 8192, True)])
+def test_split_gemm_is_reproducible(gpu, oracle, t, M, N, K, bf16):
+    """Few tiles, which K is split for: f32 activations over CTA pairs, bf16 where rows have no pitch of 16 bytes over CTAs.
+    The same bits every time and the right sums (f32: 2e-6, above the 1.1e-6 of one f32 chain per output; rows past M, tokens
+    past N)."""
+    torch, ctx, dd = gpu
+    g = synth.rng(317, M + N + t)
+    raw, X = synth.quant_matrix(g, t, M, K), synth.activations(g, N, K)
+    w, x = dev(torch, raw), dev(torch, X)
+    if bf16:
+        x = x.to(torch.bfloat16)
+        X = x.float().cpu().numpy()
+    first = None
+    for i in range(12):
+        D = torch.full((N + 1, M), 7.0, device="cuda")
+        torch.cuda.synchronize()
+        dd.recordMulMm(t, w, x, D, M, N, K, K, M, act_type=zb.BF16 if bf16 else zb.F32)
+        ctx.submit_and_wait()
+        got = D.cpu()
+        if first is None:
+            first = got
+        assert torch.equal(got, first)
+    assert (first[N:] == 7.0).all()
+    cols = sorted({0, N // 2, N - 1})
+    assert rel_l2(first[cols].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols])) <= (TOL_BF16 if bf16 else 2e-6)
+
+
 def test_mul_mm_exact_on_two_streams(gpu):
     """The f32-accurate GEMM keeps the terms of its activations in the context's scratch: a call on another stream, or a
     replay there, may not overwrite what a call still under way reads."""

@@ -30,7 +30,7 @@ struct zc_ctx {
     uint64_t router_mark = 0;            // value of `launches` right after that kernel's last launch (0: never)
     float* merge_scratch = nullptr;      // kMergeScratchFloats f32: a merged attention vector on its way to a matvec
     uint32_t* gemm_flags = nullptr;      // kGemmTileFlags words: tiles of a prefill GEMM that are summed through memory
-    uint8_t* exact_scratch = nullptr;    // kExactScratchBytes: fp16 terms of the activations of a f32-accurate GEMM
+    uint8_t* exact_scratch = nullptr;    // kExactScratchBytes: fp16 terms of a f32-accurate GEMM's activations, GEMMs' partial sums
     cudaEvent_t exact_done = nullptr;    // behind the last call that used it, or the last replay that may have ..
     unsigned long long exact_stream = 0; // .. on this stream (its id; used: whether there was one)
     bool exact_used = false;
@@ -135,7 +135,7 @@ inline int32_t take_pending(zc_ctx* ctx, DmmvArgs& a) {
     return ZC_OK;
 }
 
-// Use of the f32-accurate GEMM's scratch. A caller may go on to another stream while the work on the one before is still
+// Use of the GEMMs' scratch. A caller may go on to another stream while the work on the one before is still
 // under way: what uses the scratch there waits for what used it here. Calls that are being recorded are ordered where the
 // recording is replayed. (The event costs
 // a call 0.3 us: Q4_K 4096x4096, 658 tokens 56.8 -> 57.2.)
@@ -161,11 +161,15 @@ struct ExactUse {
         return cudaEventRecord(ctx->exact_done, ctx->stream);
     }
 };
-cudaError_t run_mul_mm_exact(zc_ctx* ctx, const ExactGemm& p) {
+template <typename Launch>
+cudaError_t with_exact_scratch(zc_ctx* ctx, Launch launch) {
     ExactUse use{ctx};
     cudaError_t e = use.begin();
-    if (e == cudaSuccess) e = launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches);
+    if (e == cudaSuccess) e = launch();
     return e == cudaSuccess ? use.end() : e;
+}
+cudaError_t run_mul_mm_exact(zc_ctx* ctx, const ExactGemm& p) {
+    return with_exact_scratch(ctx, [&] { return launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches); });
 }
 
 // Common checks of one matvec-shaped call.
@@ -885,8 +889,11 @@ int32_t zc_mul_mm(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size, co
     // layouts a tensor map cannot describe (MXFP4; Q6_K rows without a 16-byte pitch): still tensor cores
     if (e == cudaErrorNotSupported && act_type == ZC_BF16 &&
         mul_mm_cp_async_eligible(type, u8(A, a_offset), Bp, N, K, stride_b))
-        e = launch_mul_mm_cp_async(type, u8(A, a_offset), a_size - a_offset, Bp, f32m(D, d_offset * 4), M, N, K,
-                                   stride_b, stride_d, ctx->status_dev, ctx->stream, &ctx->launches);
+        e = with_exact_scratch(ctx, [&] {
+            return launch_mul_mm_cp_async(type, u8(A, a_offset), a_size - a_offset, Bp, f32m(D, d_offset * 4), M, N, K, stride_b,
+                                          stride_d, ctx->status_dev, reinterpret_cast<float*>(ctx->exact_scratch + kExactTermBytes),
+                                          ctx->stream, &ctx->launches);
+        });
     if (e == cudaErrorNotSupported && mul_mm_exact_eligible(type, u8(A, a_offset), M, N, K)) {
         const ExactGemm p{type, u8(A, a_offset), Bp, f32m(D, d_offset * 4), M, N, K, stride_b, stride_d,
                           act_type == ZC_BF16, false, ctx->status_dev};

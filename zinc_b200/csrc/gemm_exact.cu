@@ -13,7 +13,7 @@ struct PrepArgs {
     __half* x;          // [terms][N][nblk * 256]
     __half* sums;       // [N][nblk * 64], Q4_K / Q5_K
     float* inv_scale;   // [N]
-    float* D;           // zeroed where tiles are split
+    float* D;           // zeroed where tiles lie on two CTA pairs
     uint32_t tokens, K, nblk, M, stride_b, stride_d;
     bool sums_on, zero, vec;
 };
@@ -154,10 +154,45 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
 }
 
 template <int ORDER, bool BF16>
-cudaError_t launch_prep(const void* args, bool split, cudaStream_t s) {
+cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     PrepArgs a = *static_cast<const PrepArgs*>(args);
-    a.zero = split;
+    a.zero = zero;
     return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(kPrepThreads), 0, s, a);
+}
+
+// D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: eight tokens of a tile. Bound: the
+// parts' bytes, which the kernel in front has left in L2, and the launch. It costs the smallest products 2 to 4 us over
+// atomic adds in any order (Q4_K 512 x 2048, 16 tokens 13 -> 17; 1024 x 4096, 64 tokens 17 -> 21) and 4096 x 4096 nothing.
+// (Released early by the GEMM: 2 us more, its CTAs wait where the GEMM's run.)
+template <uint32_t ROWS>
+__global__ void __launch_bounds__(256)
+add_parts_kernel(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t row_tiles, uint32_t n_tile, uint32_t per, uint32_t stride_d) {
+    chain_wait();
+    chain_release();
+    after_wait(parts);
+    const uint32_t tile = blockIdx.x, tok = blockIdx.y * 8, r = threadIdx.x * 4 % ROWS;
+    const uint32_t m = tile % row_tiles * ROWS + r, last = min(tok + 8, n_tile);
+    if (m >= M) return;
+    for (uint32_t c = tok + threadIdx.x * 4 / ROWS; c < last; c += 1024 / ROWS) {
+        const uint32_t n = tile / row_tiles * n_tile + c;
+        if (n >= N) break;
+        const float* p = parts + ((uint64_t)tile * per * n_tile + c) * ROWS + r;
+        float4 s = __ldcg(reinterpret_cast<const float4*>(p));
+#pragma unroll 4
+        for (uint32_t i = 1; i < per; ++i) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(p + (uint64_t)i * n_tile * ROWS));
+            s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+        }
+        float* d = D + (uint64_t)n * stride_d + m;
+        if (m + 4 <= M && (reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+            *reinterpret_cast<float4*>(d) = s;
+        } else {
+            d[0] = s.x;
+            if (m + 1 < M) d[1] = s.y;
+            if (m + 2 < M) d[2] = s.z;
+            if (m + 3 < M) d[3] = s.w;
+        }
+    }
 }
 
 cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
@@ -173,19 +208,25 @@ cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, const ExactPrep& 
 
 }  // namespace
 
+cudaError_t launch_add_parts(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t rows, uint32_t row_tiles, uint32_t n_tile,
+                             uint32_t tiles, uint32_t per, uint32_t stride_d, cudaStream_t s) {
+    return launch_chained(rows == 256 ? add_parts_kernel<256> : add_parts_kernel<128>, dim3(tiles, (n_tile + 7) / 8), dim3(256), 0, s,
+                          parts, D, M, N, row_tiles, n_tile, per, stride_d);
+}
+
 bool mul_mm_exact_eligible(uint32_t type, const uint8_t* A, uint32_t M, uint32_t N, uint32_t K) {
     if (type != T_Q4_K && type != T_Q5_K && type != T_Q6_K && type != T_Q8_0 && type != T_MXFP4) return false;
     if (reinterpret_cast<uintptr_t>(A) & 15u) return false;
     const uint64_t nblk = (K + 255) >> 8;
     // one token's terms must fit the scratch; unit counts stay in 32 bits
-    return nblk * 256 * 8 < kExactScratchBytes / 64 && ((uint64_t)(M + 255) / 256) * ((N + 31) / 32) * nblk < (1u << 31);
+    return nblk * 256 * 8 < kExactTermBytes / 64 && ((uint64_t)(M + 255) / 256) * ((N + 31) / 32) * nblk < (1u << 31);
 }
 
 cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaStream_t s, uint64_t* launches) {
     const uint32_t nblk = (whole.K + 255) >> 8;
     const bool min_type = whole.type == T_Q4_K || whole.type == T_Q5_K;
     const size_t per_token = (size_t)nblk * 512 * (whole.bf16 ? 1 : 2) + (min_type ? (size_t)nblk * 128 : 0) + sizeof(float);
-    const uint32_t most = (uint32_t)((kExactScratchBytes - 4096) / per_token) & ~31u;
+    const uint32_t most = (uint32_t)((kExactTermBytes - 4096) / per_token) & ~31u;
     for (uint32_t t0 = 0; t0 < whole.N; t0 += most) {
         ExactGemm p = whole;
         p.N = whole.N - t0 < most ? whole.N - t0 : most;
@@ -205,6 +246,8 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         plan.sums = q;
         if (min_type) q += (size_t)p.N * nblk * 128;
         plan.inv_scale = reinterpret_cast<float*>(q);
+        plan.parts = reinterpret_cast<float*>(scratch + kExactTermBytes);
+        plan.launches = launches;
         PrepArgs a{};
         a.X = p.B;
         a.x = static_cast<__half*>(plan.x);
@@ -224,7 +267,6 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
                                     : (order == 0 ? launch_prep<0, false> : order == 1 ? launch_prep<1, false> : launch_prep<2, false>),
                              &a};
         if (cudaError_t e = launch_type(p, plan, prep, s); e != cudaSuccess) return e;
-        if (launches) *launches += 2;
     }
     return cudaSuccess;
 }

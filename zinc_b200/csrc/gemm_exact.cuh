@@ -30,8 +30,9 @@
 //            and 49 us: the runs' own roundings are what is left.
 //
 // Persistent CTA pairs (cta_group::2, 256 weight rows per pair): tiles of 256 rows x n_tile tokens, their
-// (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over pairs is summed with
-// atomic adds into D, which the preparation kernel zeroes.
+// (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over two pairs is summed with
+// atomic adds into D, which the preparation kernel zeroes; where there are three pairs or more to a tile, the parts go
+// through the scratch and are added in their order. Either way the result does not depend on timing.
 // Bound: tensor pipe (2 or 3 fp16 products per weight and token) from about 100 tokens on; below that the weight
 // bytes and the unpacking of them.
 #pragma once
@@ -123,9 +124,16 @@ struct XArgs {
     uint32_t M, N, K, nblk;
     uint32_t stride_d;
     uint32_t n_row_pairs, n_tiles, n_tile;  // n_tile tokens per tile (a multiple of 32)
+    uint32_t groups;          // > 0: the pairs form groups, each with one pair more than it has tiles
+    float* parts;             // null, or [pair][token of the tile][256 rows]: every pair has a part of one tile
     uint32_t terms;           // fp16 terms of an activation: 2 (f32) or 1 (bf16)
     uint32_t* status;
 };
+
+// which of `pairs` equal ranges (part_begin) of the units holds unit u
+__device__ __forceinline__ uint32_t x_part_of(uint32_t u, uint32_t units, uint32_t pairs) {
+    return (uint32_t)(((uint64_t)(u + 1) * pairs - 1) / units);
+}
 
 struct XSegment {
     uint32_t tile, b0, b1;
@@ -311,7 +319,16 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     const uint32_t rank = cluster_ctarank();
     const uint32_t nblk = g.nblk;
     const uint32_t U = g.n_tiles * nblk, G = gridDim.x >> 1, slot = blockIdx.x >> 1;
-    const uint32_t u_begin = (uint32_t)part_begin(slot, U, G), u_end = (uint32_t)part_begin(slot + 1, U, G);
+    uint32_t u_begin, u_end;
+    if (g.groups) {
+        const uint32_t e = x_part_of(slot, G, g.groups), at = (uint32_t)part_begin(e, G, g.groups);
+        const uint32_t n = (uint32_t)part_begin(e + 1, G, g.groups) - at, u0 = (at - e) * nblk;  // n pairs share n - 1 tiles
+        u_begin = u0 + (uint32_t)part_begin(slot - at, (n - 1) * nblk, n);
+        u_end = u0 + (uint32_t)part_begin(slot - at + 1, (n - 1) * nblk, n);
+    } else {
+        u_begin = (uint32_t)part_begin(slot, U, G);
+        u_end = (uint32_t)part_begin(slot + 1, U, G);
+    }
     auto tile_m0 = [&](uint32_t tile) { return ((tile % g.n_row_pairs) * 2 + rank) * (uint32_t)kBM; };
     auto tile_n0 = [&](uint32_t tile) { return (tile / g.n_row_pairs) * g.n_tile; };
     const uint32_t b_bytes = g.n_tile * 64 * g.terms;  // an activation slot
@@ -833,11 +850,15 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 }
                 if (!ok) break;
                 if (boundary) {
-                    // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D ----
+                    // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D or wait in
+                    // their slots for add_parts_kernel ----
                     asm volatile("griddepcontrol.wait;" ::: "memory");  // D zeroed, scales written
                     const bool whole = old.b0 == 0 && old.b1 == nblk;
                     const uint32_t m = tile_m0(old.tile) + row;
                     const uint32_t n0 = tile_n0(old.tile) + j * (g.n_tile >> 2);
+                    float* out = g.parts ? g.parts + ((uint64_t)slot * g.n_tile + j * (g.n_tile >> 2)) * 256 + rank * kBM + row
+                                         : g.D + (uint64_t)n0 * g.stride_d + m;
+                    const uint32_t out_stride = g.parts ? 256u : g.stride_d;
                     // the tokens' scales, one per lane (a load per column would be held back by the add before it)
                     float inv0 = 0.f, inv1 = 0.f;
                     if ((uint32_t)lane < n8 * 8 && n0 + lane < g.N) inv0 = __ldcg(g.inv_scale + n0 + lane);
@@ -848,8 +869,8 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         const float inv = __shfl_sync(0xFFFFFFFFu, c < 32 ? inv0 : inv1, c & 31);
                         if ((uint32_t)c < n8 * 8 && n < g.N && m < g.M) {
                             const float v = ((c & 1) ? acc[c / 2].y : acc[c / 2].x) * inv;
-                            float* dst = g.D + (uint64_t)n * g.stride_d + m;
-                            if (whole) *dst = v;
+                            float* dst = out + (uint64_t)c * out_stride;
+                            if (whole || g.parts) *dst = v;
                             else atomicAdd(dst, v);
                         }
                     }
@@ -891,11 +912,23 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     cfg.numAttrs = 1;
     const int pairs = max_pairs_of(kern, cfg, max_pairs);
     if (pairs < 1) return cudaErrorNotSupported;
-    const uint32_t units = plan.n_tiles * plan.nblk;
-    // whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds
-    uint32_t G = units < (uint32_t)pairs ? units : (uint32_t)pairs;
-    if (plan.n_tiles <= (uint32_t)pairs && plan.n_tiles * 8 >= (uint32_t)pairs * 7) G = plan.n_tiles;
-    const bool split = plan.n_tiles % G != 0;
+    // Whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds. The parts of a
+    // split tile are added so that no sum's order depends on timing: two of them by atomics (0 + a + b), more by a kernel
+    // behind this one.
+    const uint32_t n = plan.n_tiles, most = (uint32_t)pairs;
+    uint32_t G = most, groups = 0, per = 1;
+    if (n >= most) {  // ranges of a tile's length or more: a tile lies on two at most
+    } else if (n * 8 >= most * 7) {
+        G = n;
+    } else if (n * 2 > most && plan.nblk > 1) {  // groups of k tiles on k + 1 pairs: every tile on two
+        groups = G - n;
+    } else {  // every tile on as many pairs
+        per = most / n < plan.nblk ? most / n : plan.nblk;
+        const uint64_t room = kExactPartBytes / ((uint64_t)n * plan.n_tile * 1024);
+        if (per > 2 && per > room) per = room > 2 ? (uint32_t)room : 2u;
+        G = n * per;
+    }
+    const bool split = n % G != 0, parts = per > 2;
     cfg.numAttrs = 2;
     cfg.gridDim = dim3(2 * G, 1, 1);
     XArgs g{};
@@ -912,6 +945,8 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     g.n_tiles = plan.n_tiles;
     g.n_tile = plan.n_tile;
     g.terms = p.bf16 ? 1u : 2u;
+    g.groups = groups;
+    g.parts = parts ? plan.parts : nullptr;
     g.status = p.status;
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
@@ -942,8 +977,10 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
             return cudaErrorInvalidValue;
     }
     // the preparation goes out last, so that the GEMM's launch follows it at once and overlaps it
-    if (cudaError_t e = prep.launch(prep.args, split, s); e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, kern, mx, mm, mw, g);
+    if (cudaError_t e = prep.launch(prep.args, split && !parts, s); e != cudaSuccess) return e;
+    if (cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mx, mm, mw, g); e != cudaSuccess) return e;
+    if (plan.launches) *plan.launches += parts ? 3 : 2;
+    return parts ? launch_add_parts(plan.parts, p.D, p.M, p.N, 2 * kBM, plan.n_row_pairs, plan.n_tile, n, per, p.stride_d, s) : cudaSuccess;
 }
 
 template <int TYPE, bool kFetch>

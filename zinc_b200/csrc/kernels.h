@@ -234,7 +234,7 @@ bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, ui
                               uint32_t stride_b);
 cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_bytes, const void* B, float* D,
                                    uint32_t M, uint32_t N, uint32_t K, uint32_t stride_b, uint32_t stride_d,
-                                   uint32_t* status, cudaStream_t s, uint64_t* launches);
+                                   uint32_t* status, float* parts, cudaStream_t s, uint64_t* launches);  // parts: kExactPartBytes
 
 cudaError_t launch_dequant_rows(uint32_t type, const uint8_t* A, float* out, uint64_t first_row, uint32_t n_rows,
                                 uint32_t K, cudaStream_t s, uint64_t* launches);
@@ -323,7 +323,9 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
 // Prefill GEMM at f32 accuracy on the tensor cores (gemm_exact.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4 weights, f32 or
 // bf16 activations. `scratch`: context memory for the fp16 terms of the activations; tokens beyond what it holds go
 // in further passes. cudaErrorNotSupported: the caller takes another path (nothing launched or written).
-constexpr size_t kExactScratchBytes = 64u << 20;
+constexpr size_t kExactTermBytes = 64u << 20;
+constexpr size_t kExactPartBytes = 20u << 20;  // parts of split tiles: 74 CTA pairs, 256 rows and 256 tokens each: 19.4 MB
+constexpr size_t kExactScratchBytes = kExactTermBytes + kExactPartBytes;
 struct ExactGemm {
     uint32_t type;
     const uint8_t* A;
@@ -338,10 +340,16 @@ struct XPlan {
     uint32_t nblk, n_row_pairs, n_tiles, n_tile;
     void *x, *sums;
     float* inv_scale;
+    float* parts;
+    uint64_t* launches;
 };
-// launches the preparation of the activations; split: tiles are shared between CTA pairs, D must be zeroed
+// D[n][m] <- sum of the `per` parts of its tile, in their order: parts [tile][per][n_tile][rows] (rows 256 or 128), tile t at
+// row tile t % row_tiles of n_tile tokens from t / row_tiles * n_tile
+cudaError_t launch_add_parts(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t rows, uint32_t row_tiles, uint32_t n_tile,
+                             uint32_t tiles, uint32_t per, uint32_t stride_d, cudaStream_t s);
+// launches the preparation of the activations; zero: D is set to zero
 struct ExactPrep {
-    cudaError_t (*launch)(const void* args, bool split, cudaStream_t s);
+    cudaError_t (*launch)(const void* args, bool zero, cudaStream_t s);
     const void* args;
 };
 // one translation unit per weight type

@@ -81,7 +81,8 @@ struct MoeGemmArgs {
     uint32_t* status;
     uint32_t dense_n;             // > 0: plain GEMM over dense_n tokens (one "expert", identity pair list, no tables) ..
     uint32_t dense_tile;          // .. in tiles of this many
-    uint32_t splits, slice;       // work items along K per tile, 256-column blocks in each; > 1: they add into a zeroed Y
+    uint32_t splits, slice;       // work items along K per tile, 256-column blocks in each; two: they add into a zeroed Y
+    float* parts;                 // more: [work item][dense_tile][128 rows], added afterwards
 };
 
 // Work item w: every slice of K of a row tile, then the next row tile, then the next tile of pairs.
@@ -380,7 +381,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
                     const uint32_t s_j = __shfl_sync(0xFFFFFFFFu, slot, jj);
                     if (c * 32 + jj < tile.z && m < g.M) {
                         float* y = g.Y + (uint64_t)t_j * g.y_token_stride + (uint64_t)s_j * g.M + m;
-                        if (g.splits > 1)
+                        if (g.parts)
+                            g.parts[((uint64_t)w * g.dense_tile + c * 32 + jj) * kBM + q * 32 + lane] = __uint_as_float(v[jj]);
+                        else if (g.splits > 1)
                             atomicAdd(y, __uint_as_float(v[jj]));
                         else
                             *y = __uint_as_float(v[jj]);
@@ -642,7 +645,7 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     MoeGemmArgs g{A, A + a_bytes, expert_stride, Y, header, tiles, list, M, K, n_used, y_token_stride,
-                  (M + kBM - 1) / kBM, status, 0u, 0u, 1u, 0u};
+                  (M + kBM - 1) / kBM, status, 0u, 0u, 1u, 0u, nullptr};
     const uint64_t max_items64 = (uint64_t)l.max_tiles * g.row_tiles;
     const uint32_t max_items = max_items64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)max_items64;
     // one grouping and one packed activation buffer serve both matrices of a pair (gate and up)
@@ -671,7 +674,7 @@ bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, ui
 
 cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_bytes, const void* B, float* D,
                                    uint32_t M, uint32_t N, uint32_t K, uint32_t stride_b, uint32_t stride_d,
-                                   uint32_t* status, cudaStream_t s, uint64_t* launches) {
+                                   uint32_t* status, float* parts, cudaStream_t s, uint64_t* launches) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     // equal tiles of at most 160 tokens (128: Q6_K)
@@ -686,9 +689,11 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    MoeGemmArgs g{A, A + a_bytes, 0, D, nullptr, nullptr, nullptr, M, K, 1u, stride_d, (M + kBM - 1) / kBM, status, N, per, 1u, 0u};
-    // Fewer tiles than SMs: K is split over as many work items as find an SM, of two 256-column blocks at least, which add
-    // into a zeroed D. (Q6_K 4096 x 11008 on its 32 row tiles alone: 88 us with 32 tokens, 33 split.)
+    MoeGemmArgs g{A, A + a_bytes, 0, D, nullptr, nullptr, nullptr, M, K, 1u, stride_d, (M + kBM - 1) / kBM, status, N, per, 1u, 0u, nullptr};
+    // Fewer tiles than SMs: K is split over as many work items as find an SM, of two 256-column blocks at least. The result
+    // must not depend on which of them is done first: two add into a zeroed D, the parts of more go through the scratch.
+    // (Q6_K 4096 x 11008 on its 32 row tiles alone: 88 us with 32 tokens, 32 split; MXFP4
+    // 2880 x 2880, 32 tokens: 15 us added in any order, 17 in this one.)
     const uint64_t tiles = (uint64_t)((N + per - 1) / per) * g.row_tiles;
     const uint32_t nblk = (K + 255) >> 8;
     int dev = 0, sms = 0;
@@ -697,13 +702,20 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
     const uint32_t most = tiles < (uint64_t)sms ? (uint32_t)(sms / tiles) : 1u;
     g.slice = max((nblk + most - 1) / most, 2u);
     g.splits = (nblk + g.slice - 1) / g.slice;
-    if (g.splits > 1) {
+    if (g.splits > 2 && tiles * g.splits * per * kBM * 4 > kExactPartBytes) {  // more SMs than the scratch is sized for
+        g.slice = (nblk + 1) / 2;
+        g.splits = 2;
+    }
+    if (g.splits > 2) {
+        g.parts = parts;
+    } else if (g.splits == 2) {
         if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
     }
     const uint64_t items64 = tiles * g.splits;
     const uint32_t items = items64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)items64;
-    const cudaError_t e = launch_gemm_bn(type, bn, map, g, items, s);
-    if (e == cudaSuccess && launches) ++*launches;
+    cudaError_t e = launch_gemm_bn(type, bn, map, g, items, s);
+    if (e == cudaSuccess && g.parts) e = launch_add_parts(parts, D, M, N, kBM, g.row_tiles, per, (uint32_t)tiles, g.splits, stride_d, s);
+    if (e == cudaSuccess && launches) *launches += g.parts ? 2 : 1;
     return e;
 }
 
