@@ -374,6 +374,36 @@ def test_split_gemm_is_reproducible(gpu, oracle, t, M, N, K, bf16):
     assert rel_l2(first[cols].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols])) <= (TOL_BF16 if bf16 else 2e-6)
 
 
+@pytest.mark.parametrize("t,M,N,K,bf16", [(zb.Q4_K, 20480, 32, 256, True), (zb.Q6_K, 10240, 32, 2048, True), (zb.Q4_K, 10240, 200, 256, True),
+                                          (zb.MXFP4, 20480, 32, 64, True), (zb.Q4_K, 4096, 40, 256, False)])
+def test_mul_mm_reads_weights_of_the_kernel_before(gpu, t, M, N, K, bf16):
+    """Weights that the kernel directly in front on the stream writes (shapes without a zeroing kernel between them too)."""
+    torch, _, _ = gpu
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        ctx = zb.Context(0, stream=stream.cuda_stream)
+        dd = zb.DmmvDispatch(ctx)
+        g = synth.rng(331, M + N)
+        W = [dev(torch, synth.quant_matrix(g, t, M, K)) for _ in range(2)]
+        x = dev(torch, synth.activations(g, N, K))
+        x = x.to(torch.bfloat16) if bf16 else x
+        w = torch.empty_like(W[0])
+        D = [torch.empty(N, M, device="cuda") for _ in range(10)]
+        for i in range(10):
+            if i < 2:
+                torch.cuda.synchronize()
+            w.copy_(W[i % 2])
+            w.bitwise_or_(0)  # a kernel
+            if i < 2:
+                torch.cuda.synchronize()
+            dd.recordMulMm(t, w, x, D[i], M, N, K, K, M, act_type=zb.BF16 if bf16 else zb.F32)
+        ctx.submit_and_wait()
+        for i in range(2, 10):
+            assert torch.equal(D[i], D[i % 2])
+        assert not torch.equal(D[0], D[1])
+        ctx.close()
+
+
 def test_mul_mm_exact_on_two_streams(gpu):
     """The f32-accurate GEMM keeps the terms of its activations in the context's scratch: a call on another stream, or a
     replay there, may not overwrite what a call still under way reads."""

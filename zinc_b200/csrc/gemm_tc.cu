@@ -114,6 +114,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // Without a zeroing kernel in front (which has waited) the kernel before may still be running, and what it writes may
+    // be this one's weights.
+    if (gridDim.z == 1) chain_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -786,6 +789,9 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs 
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // Without a zeroing kernel in front (which has waited) the kernel before may still be running, and what it writes may
+    // be this one's weights.
+    if (gridDim.z == 1) chain_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
