@@ -393,7 +393,9 @@ int32_t zc_moe_router_topk(zc_ctx* ctx, const void* hidden, uint64_t hidden_size
  * A / expert_stride / X, the pairs are grouped by expert (as the reference's Metal path does,
  * src/shaders/metal/moe_route_pack.metal:13-36) and each expert's weights are dequantised once per
  * tile of its tokens on the tensor cores: bf16 operands, f32 accumulation (relative L2 <= 5e-3).
- * Ids >= n_experts are skipped there (their output rows are left untouched). */
+ * Ids >= n_experts are skipped there (their output rows are left untouched). Q4_K and Q6_K need only the tables
+ * and the activations in bf16 of it, about n_tokens * n_experts_used * (2 * K + 5) bytes; MXFP4 takes its activations as
+ * bf16 where there is no more room, else as two FP8 terms. */
 int32_t zc_moe_dmmv_batched(zc_ctx* ctx, uint32_t type,
                             const void* A, uint64_t a_size, const void* X, uint64_t x_size,
                             void* Y, uint64_t y_size, const void* routing, uint64_t routing_size,

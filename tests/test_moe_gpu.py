@@ -168,6 +168,40 @@ def test_moe_dmmv_batched_grouped(gpu, oracle, t, E, M, K, k, T, pad):
         assert np.all(got[:, k * M:] == got[0, k * M])
 
 
+@pytest.mark.parametrize("t", [zb.Q4_K, zb.Q6_K, zb.MXFP4])
+@pytest.mark.parametrize("K", [512, 2816])
+def test_moe_dmmv_batched_workspace_for_bf16(gpu, oracle, t, K):
+    """A workspace with room for the tables and the activations in bf16, which is less than the largest layout needs, takes
+    the tensor cores as well: its results are those of bf16 operands, not the f32 ones of the call without a workspace."""
+    torch, ctx, dd = gpu
+    E, M, k, T = 8, 192, 2, 200
+    g = synth.rng(223, K + t)
+    w, stride = stacked(g, t, E, M, K)
+    ids = g.integers(0, E, size=(T, k)).astype(np.uint32)
+    X = synth.activations(g, T, K)
+    wd, xd, rd = dev(torch, w), dev(torch, X), dev(torch, ids)
+    n = T * k
+    bf16 = ((256 + (n // 32 + E) * 16 + n * 4 + 255) & ~255) + n * K * 2
+    full = dd.moeGroupedWorkspaceBytes(T, k, K, E)
+    assert bf16 < full
+    out = {}
+    for size in (0, bf16 - 256, bf16, full):
+        Y = torch.full((T, k, M), 7.0, device="cuda")
+        try:
+            if size:
+                dd.setWorkspace(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            dd.recordMoeBatchedDispatch(t, wd, xd, Y, rd, M, K, stride, E, k, T, K, k * M)
+            ctx.submit_and_wait()
+        finally:
+            dd.setWorkspace(None)
+        out[size] = Y.cpu().numpy()
+    want = np.stack([oracle.moe_dmmv_f64(w, t, M, K, stride, ids[i], K, np.repeat(X[i:i + 1], k, axis=0)) for i in range(T)])
+    assert np.array_equal(out[0], out[bf16 - 256]) and not np.array_equal(out[0], out[bf16])
+    assert rel_l2(out[bf16], want) <= TOL_TC
+    if t != zb.MXFP4:
+        assert np.array_equal(out[bf16], out[full])
+
+
 @pytest.mark.parametrize("rule", [zb.ROUTE_SOFTMAX_ALL_RENORM, zb.ROUTE_TOPK_THEN_SOFTMAX])
 @pytest.mark.parametrize("n,k,T", [(8, 3, 1), (256, 8, 64), (32, 4, 17), (1000, 20, 3), (2000, 6, 2), (129, 8, 5)])
 def test_softmax_topk(gpu, oracle, rule, n, k, T):

@@ -1205,7 +1205,7 @@ int32_t zc_moe_dmmv_batched(zc_ctx* ctx, uint32_t type, const void* A, uint64_t 
                              f32p(X, 0), x_token_stride, ctx->workspace_size)) {
         cudaError_t eg = launch_moe_grouped(type, u8(A, 0), a_size, f32p(X, 0), f32m(Y, 0),
                                             static_cast<const uint32_t*>(routing), M, K, expert_stride, n_experts,
-                                            n_experts_used, n_tokens, x_token_stride, y_token_stride, ctx->workspace,
+                                            n_experts_used, n_tokens, x_token_stride, y_token_stride, ctx->workspace, ctx->workspace_size,
                                             ctx->status_dev, ctx->stream, &ctx->launches);
         return eg == cudaSuccess ? ZC_OK : cuda_fail(ctx, eg, fn);
     }
@@ -1239,7 +1239,7 @@ int32_t zc_moe_dmmv_batched_pair(zc_ctx* ctx, uint32_t type, const void* Wg, uin
     }
     cudaError_t e = launch_moe_grouped(type, u8(Wg, 0), wg_size, f32p(X, 0), f32m(Yg, 0),
                                        static_cast<const uint32_t*>(routing), M, K, expert_stride, n_experts,
-                                       n_experts_used, n_tokens, x_token_stride, y_token_stride, ctx->workspace,
+                                       n_experts_used, n_tokens, x_token_stride, y_token_stride, ctx->workspace, ctx->workspace_size,
                                        ctx->status_dev, ctx->stream, &ctx->launches, u8(Wu, 0), wu_size, f32m(Yu, 0));
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }

@@ -181,7 +181,7 @@ bool moe_grouped_eligible(uint32_t type, const uint8_t* A, uint32_t K, uint64_t 
 cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes, const float* X, float* Y,
                                const uint32_t* routing, uint32_t M, uint32_t K, uint64_t expert_stride,
                                uint32_t n_experts, uint32_t n_used, uint32_t n_tokens, uint32_t x_token_stride,
-                               uint32_t y_token_stride, void* ws, uint32_t* status, cudaStream_t s,
+                               uint32_t y_token_stride, void* ws, uint64_t ws_size, uint32_t* status, cudaStream_t s,
                                uint64_t* launches, const uint8_t* A2 = nullptr, uint64_t a2_bytes = 0,
                                float* Y2 = nullptr);  // A2 / Y2: a second matrix on the same grouping (gate + up)
 

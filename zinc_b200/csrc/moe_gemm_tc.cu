@@ -582,19 +582,20 @@ bool moe_grouped_eligible(uint32_t type, const uint8_t* A, uint32_t K, uint64_t 
         return false;
     if ((reinterpret_cast<uintptr_t>(A) & 15u) || (expert_stride & 15u)) return false;
     if ((reinterpret_cast<uintptr_t>(X) & 15u) || (x_token_stride & 3u)) return false;
-    return ws_size >= moe_grouped_workspace_bytes(n_pairs, K, n_experts);
+    return ws_size >= ws_layout(n_pairs, K, n_experts, 32, false).total;  // the smallest tile needs the longest table
 }
 
 cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes, const float* X, float* Y,
                                const uint32_t* routing, uint32_t M, uint32_t K, uint64_t expert_stride,
                                uint32_t n_experts, uint32_t n_used, uint32_t n_tokens, uint32_t x_token_stride,
-                               uint32_t y_token_stride, void* ws, uint32_t* status, cudaStream_t s,
+                               uint32_t y_token_stride, void* ws, uint64_t ws_size, uint32_t* status, cudaStream_t s,
                                uint64_t* launches, const uint8_t* A2, uint64_t a2_bytes, float* Y2) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     const uint64_t n_pairs = (uint64_t)n_tokens * n_used;
     const uint32_t bn = pick_bn(type, n_pairs, n_experts);
-    const bool mx = type == T_MXFP4;
+    // MXFP4 with room for bf16 activations only: the tile kernel on weights unpacked to bf16
+    const bool mx = type == T_MXFP4 && ws_size >= ws_layout(n_pairs, K, n_experts, bn, true).total;
     const WsLayout l = ws_layout(n_pairs, K, n_experts, bn, mx);
     uint8_t* base = static_cast<uint8_t*>(ws);
     uint32_t* header = reinterpret_cast<uint32_t*>(base + l.header);
