@@ -83,6 +83,22 @@ def test_no_cpu_fallback_without_device():
         zb.Context(0)
 
 
+def test_only_peer_waits_break_the_communicator():
+    """A wait that gives up leaves its site number; from 200 on the communicator refuses further collectives. Those of
+    the GEMM kernels, which wait for no peer, are below."""
+    csrc = os.path.join(ROOT, "zinc_b200", "csrc")
+    sites = {}
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh")):
+            text = open(os.path.join(csrc, name)).read()
+            for site in re.findall(r"\bstatus(?:,|\[1\] =)\s*(\d+)\b", text):
+                sites.setdefault(int(site), set()).add(name)
+    assert len(sites) > 30
+    gemm = {n: f for n, f in sites.items() if any("gemm" in x or x.startswith("tc_") for x in f)}
+    assert gemm and max(gemm) < 200, {n: f for n, f in gemm.items() if n >= 200}
+    assert not [n for n, f in gemm.items() if len(f) > 1]   # a number names one kernel
+
+
 def test_product_does_not_import_oracle():
     """Nothing under zinc_b200/ may reference the oracle."""
     pkg = os.path.join(ROOT, "zinc_b200")

@@ -404,7 +404,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                             bar = smem_u32(&bars->pfree[gb & 1]);
                             par = ((gb >> 1) - 1) & 1;
                         }
-                        ok = warp_poll(bar, par, bars, g.status, 301);
+                        ok = warp_poll(bar, par, bars, g.status, 181);
                         if (!ok) break;
                         tc_fence_after();
                         if (open) db = desc_b + sb * (b_bytes >> 4);
@@ -452,7 +452,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                             bar = smem_u32(&bars->pfree[c]);
                             par = (gb - 1) & 1;
                         }
-                        ok = warp_poll(bar, par, bars, g.status, 301);
+                        ok = warp_poll(bar, par, bars, g.status, 181);
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {  // small terms first: what they add up to is all that the accumulator rounds them by
@@ -491,7 +491,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 if constexpr (kMin) {  // into the last run; merged: these columns hold the sums' terms; the low-term columns see zeros
                     if (!ok) break;
                     ok = warp_poll(lane == 1 ? full_b + sb * 8 : smem_u32(&bars->full_m[gb & 1]), lane == 1 ? pb : (gb >> 1) & 1, bars,
-                                   g.status, 304);
+                                   g.status, 184);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -550,7 +550,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     bars->failed = 1;
                     if (g.status) {
                         g.status[0] = 1;
-                        g.status[1] = 305;
+                        g.status[1] = 185;
                     }
                     break;
                 }
@@ -567,7 +567,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 const int m0 = (int)tile_m0(ws.tile);
                 for (uint32_t b = ws.b0; b < ws.b1; ++b, ++i) {
                     const int sw = i & 1;
-                    ok = wait_or_fail(&bars->empty_w[sw], ((i >> 1) & 1) ^ 1, bars, g.status, 311);
+                    ok = wait_or_fail(&bars->empty_w[sw], ((i >> 1) & 1) ^ 1, bars, g.status, 191);
                     if (!ok) break;
                     mbar_expect_tx(&bars->full_w[sw], T::kWBytes);
                     // Q8_0 boxes are wider than 256 bytes: their map counts 16-bit elements
@@ -604,7 +604,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         uint64_t c_off = 0;
         auto fetch = [&]() -> bool {
             if (!f_live) return true;
-            if (!poll_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 306)) return false;
+            if (!poll_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 186)) return false;
             uint8_t* dst = smem_w + f_sw * T::kWBytes;
             constexpr int kPieces = (kBlock + 15 + 15) / 16;
             static_assert(!kFetch || kPieces * 16 <= (int)kRow, "a fetched row fits its slot");
@@ -659,7 +659,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     if constexpr (kFetch) c_off = row_off(sg.tile);
                 }
                 const int sw = gb & 1;
-                if (!poll_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 307)) break;
+                if (!poll_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 187)) break;
                 if constexpr (kFetch) {
                     if (!fetch()) break;  // the next block, into the slot the previous one left
                 }
@@ -720,12 +720,12 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     const uint32_t s0 = scw & 0xFFu, s1 = (scw >> 8) & 0xFFu, mn0 = mnw & 0xFFu, mn1 = (mnw >> 8) & 0xFFu;
                     const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
                     const uint32_t h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
+                    if (!poll_or_fail(empty_a, pa, bars, g.status, 188)) break;
                     x_deq_k4<TYPE == T_Q5_K>(w, h, j, q_scale * (float)s0, q_scale * (float)s1, stage, row);
                     const float v0 = ratio * (float)mn0, v1 = ratio * (float)mn1;
                     const __half2 vh = __floats2half2_rn(v0, v1);
                     const __half2 vl = __floats2half2_rn(v0 - __low2float(vh), v1 - __high2float(vh));
-                    if (!poll_or_fail(&bars->empty_m[gb & 1], ((gb >> 1) & 1) ^ 1, bars, g.status, 309)) break;
+                    if (!poll_or_fail(&bars->empty_m[gb & 1], ((gb >> 1) & 1) ^ 1, bars, g.status, 189)) break;
                     // chunks 0, 1, 2: high, low, high terms
                     uint8_t* mp = smem + T::kMinOffset + (gb & 1) * T::kMinBytes + row * 64 + 4 * j;
                     const int x = (row >> 1) & 3;
@@ -757,7 +757,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
                     }
                     release_after(read, &bars->empty_w[sw], lane);
-                    if (!poll_or_fail(empty_a, pa, bars, g.status, 308)) break;
+                    if (!poll_or_fail(empty_a, pa, bars, g.status, 188)) break;
                     x_deq_mx(q[0], sc[0], 0, stage, row);
                     x_deq_mx(q[1], sc[1], 4, stage, row);
                     fence_proxy_async();
@@ -783,7 +783,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                         const int ab2 = T::kABuf == 1 ? 0 : hf;
                         uint8_t* stage2 = smem + (j * T::kABuf + ab2) * kABytes;
                         const uint32_t pa2 = T::kABuf == 1 ? (uint32_t)hf ^ 1u : (gb & 1) ^ 1u;
-                        if (!poll_or_fail(&bars->empty_a[j * T::kABuf + ab2], pa2, bars, g.status, 308)) { ok = false; break; }
+                        if (!poll_or_fail(&bars->empty_a[j * T::kABuf + ab2], pa2, bars, g.status, 188)) { ok = false; break; }
                         if constexpr (TYPE == T_Q6_K) {
                             x_deq_q6k(wp, off, gg, stage2, row);
                         } else if (8 * b + gg < (g.K >> 5)) {
@@ -809,7 +809,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
 #pragma unroll 1
                 for (int r = 0; r < kRuns && ok; ++r) {
                     const uint32_t buf = kRuns == 4 ? (uint32_t)r : pv & 1;
-                    ok = poll_or_fail(&bars->accum[buf], (kRuns == 4 ? pv : pv >> 1) & 1, bars, g.status, 310);
+                    ok = poll_or_fail(&bars->accum[buf], (kRuns == 4 ? pv : pv >> 1) & 1, bars, g.status, 190);
                     if (!ok) break;
                     __syncwarp();
                     tc_fence_after();
