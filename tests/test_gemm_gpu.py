@@ -374,6 +374,26 @@ def test_split_gemm_is_reproducible(gpu, oracle, t, M, N, K, bf16):
     assert rel_l2(first[cols].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols])) <= (TOL_BF16 if bf16 else 2e-6)
 
 
+@pytest.mark.parametrize("t,M,N,K,bf16,want", [
+    (zb.Q4_K, 256, 40, 4096, True, 2),      # K split: zeroing kernel, GEMM
+    (zb.Q4_K, 40960, 40, 256, True, 1),
+    (zb.Q6_K, 256, 200, 4096, True, 2),
+    (zb.Q4_K, 1024, 600, 4096, True, 2),    # CTA pairs: D or the tiles' flags zeroed, GEMM
+    (zb.MXFP4, 256, 40, 1024, True, 2),     # two slices of K: zeroing kernel, GEMM
+    (zb.MXFP4, 256, 40, 4096, True, 2),     # eight: GEMM, sums of the parts
+    (zb.Q4_K, 256, 40, 4096, False, 3),     # preparation, GEMM, sums of the parts
+    (zb.Q4_K, 20480, 40, 256, False, 2)])
+def test_mul_mm_counts_its_launches(gpu, t, M, N, K, bf16, want):
+    torch, ctx, dd = gpu
+    g = synth.rng(337, M)
+    w, x = dev(torch, synth.quant_matrix(g, t, M, K)), dev(torch, synth.activations(g, N, K))
+    D = torch.empty(N, M, device="cuda")
+    before = ctx.launch_count
+    dd.recordMulMm(t, w, x.to(torch.bfloat16) if bf16 else x, D, M, N, K, K, M, act_type=zb.BF16 if bf16 else zb.F32)
+    assert ctx.launch_count - before == want
+    ctx.submit_and_wait()
+
+
 @pytest.mark.parametrize("t,M,N,K,bf16", [(zb.Q4_K, 20480, 32, 256, True), (zb.Q6_K, 10240, 32, 2048, True), (zb.Q4_K, 10240, 200, 256, True),
                                           (zb.MXFP4, 20480, 32, 64, True), (zb.Q4_K, 4096, 40, 256, False)])
 def test_mul_mm_reads_weights_of_the_kernel_before(gpu, t, M, N, K, bf16):

@@ -933,7 +933,7 @@ gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmArgs 
 
 template <int TYPE, int BN, int NACC>
 cudaError_t launch_tile(const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K,
-                        uint32_t stride_b, uint32_t stride_d, uint32_t* status, cudaStream_t s) {
+                        uint32_t stride_b, uint32_t stride_d, uint32_t* status, cudaStream_t s, uint64_t* launches) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     CUtensorMap map;
@@ -970,14 +970,14 @@ cudaError_t launch_tile(const uint8_t* A, const void* B, float* D, uint32_t M, u
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 4) --splits;
     if (splits > 1) {
-        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s, launches); e != cudaSuccess) return e;
         grid.z = splits;
     }
     return launch_chained(kern, grid, dim3(kThreads), Tile<TYPE, BN>::kSmemBytes, s, map, wmap, g);
 }
 
 cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K,
-                         uint32_t stride_b, uint32_t stride_d, uint32_t* status, cudaStream_t s) {
+                         uint32_t stride_b, uint32_t stride_d, uint32_t* status, cudaStream_t s, uint64_t* launches) {
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     CUtensorMap map;
@@ -1001,7 +1001,7 @@ cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, 
     splits = splits < 1 ? 1 : (splits > 8 ? 8 : splits);
     while (splits > 1 && (K >> 8) / splits < 2) --splits;
     if (splits > 1) {
-        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s, launches); e != cudaSuccess) return e;
         grid.z = splits;
     }
     return launch_chained(gemm_tc_small_kernel, grid, dim3(kSmThreads), kSmSmemBytes, s, map, g);
@@ -1010,7 +1010,7 @@ cudaError_t launch_small(const uint8_t* A, const void* B, float* D, uint32_t M, 
 // The persistent pair kernel. cudaErrorNotSupported: the caller takes another path (nothing launched or written).
 template <int TYPE, bool kFetch = TYPE == T_MXFP4>
 cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K, uint32_t stride_b,
-                        uint32_t stride_d, uint32_t* status, uint32_t* flags, uint32_t n_flags, cudaStream_t s) {
+                        uint32_t stride_d, uint32_t* status, uint32_t* flags, uint32_t n_flags, cudaStream_t s, uint64_t* launches) {
     using T = Tile<TYPE, 256>;
     EncodeFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
@@ -1084,8 +1084,8 @@ cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, u
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return cudaErrorInvalidValue;
     }
-    cudaError_t e = p.zeroed ? launch_zero(D, M, N, stride_d, s)
-                             : launch_zero(reinterpret_cast<float*>(flags), p.n_tiles * 2, 1, 0, s);
+    cudaError_t e = p.zeroed ? launch_zero(D, M, N, stride_d, s, launches)
+                             : launch_zero(reinterpret_cast<float*>(flags), p.n_tiles * 2, 1, 0, s, launches);
     if (e != cudaSuccess) return e;
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, map, wmap, p);
@@ -1094,25 +1094,26 @@ cudaError_t launch_pair(const uint8_t* A, const void* B, float* D, uint32_t M, u
 template <int TYPE>
 cudaError_t launch_typed(const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K,
                          uint32_t stride_b, uint32_t stride_d, uint32_t* status, uint32_t* flags, uint32_t n_flags,
-                         cudaStream_t s) {
+                         cudaStream_t s, uint64_t* launches) {
     if (N <= 128) {
-        if constexpr (TYPE == T_Q4_K) return launch_small(A, B, D, M, N, K, stride_b, stride_d, status, s);
-        return launch_tile<TYPE, 128, 1>(A, B, D, M, N, K, stride_b, stride_d, status, s);
+        if constexpr (TYPE == T_Q4_K) return launch_small(A, B, D, M, N, K, stride_b, stride_d, status, s, launches);
+        return launch_tile<TYPE, 128, 1>(A, B, D, M, N, K, stride_b, stride_d, status, s, launches);
     }
-    if (N <= 256) return launch_tile<TYPE, 256, 1>(A, B, D, M, N, K, stride_b, stride_d, status, s);
+    if (N <= 256) return launch_tile<TYPE, 256, 1>(A, B, D, M, N, K, stride_b, stride_d, status, s, launches);
     // CTA pairs (half the activation traffic per SM, K streamed over the pairs) unless the half-empty pair of an
     // odd number of row tiles would waste more than a seventh of the work
     const uint32_t row_tiles = (M + kBM - 1) / kBM;
     if (g_pair_mode && ((row_tiles & 1u) == 0 || row_tiles >= 7)) {
-        const cudaError_t e = launch_pair<TYPE>(A, B, D, M, N, K, stride_b, stride_d, status, flags, n_flags, s);
+        const cudaError_t e = launch_pair<TYPE>(A, B, D, M, N, K, stride_b, stride_d, status, flags, n_flags, s, launches);
         if (e != cudaErrorNotSupported) return e;
     }
-    return launch_tile<TYPE, 256, 2>(A, B, D, M, N, K, stride_b, stride_d, status, s);
+    return launch_tile<TYPE, 256, 2>(A, B, D, M, N, K, stride_b, stride_d, status, s, launches);
 }
 
 }  // namespace
 
-cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s) {
+cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s, uint64_t* launches) {
+    if (launches) ++*launches;
     return launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d);
 }
 
@@ -1127,7 +1128,7 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
         // leaves, go to the caller's other route (128-token tiles)
         const uint32_t row_tiles = (M + kBM - 1) / kBM;
         if (N <= 256 || (K & 63u) || !g_pair_mode || ((row_tiles & 1u) && row_tiles < 7)) return cudaErrorNotSupported;
-        cudaError_t e = launch_pair<T_MXFP4>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s);
+        cudaError_t e = launch_pair<T_MXFP4>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s, launches);
         if (e == cudaSuccess && launches) ++*launches;
         return e;
     }
@@ -1138,14 +1139,14 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
     if (type == T_Q6_K && (K & 2047u)) {
         const uint32_t row_tiles = (M + kBM - 1) / kBM;
         if (N <= 256 || !g_pair_mode || ((row_tiles & 1u) && row_tiles < 7)) return cudaErrorNotSupported;
-        cudaError_t e = launch_pair<T_Q6_K, true>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s);
+        cudaError_t e = launch_pair<T_Q6_K, true>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s, launches);
         if (e == cudaSuccess && launches) ++*launches;
         return e;
     }
     if (N < 16) return cudaErrorNotSupported;  // a handful of tokens: the matvec-style kernels are the better fit
     cudaError_t e = type == T_Q4_K
-                        ? launch_typed<T_Q4_K>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s)
-                        : launch_typed<T_Q6_K>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s);
+                        ? launch_typed<T_Q4_K>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s, launches)
+                        : launch_typed<T_Q6_K>(A, B, D, M, N, K, stride_b, stride_d, status, tile_flags, n_tile_flags, s, launches);
     if (e == cudaSuccess && launches) ++*launches;
     return e;
 }

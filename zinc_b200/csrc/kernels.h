@@ -227,7 +227,7 @@ cudaError_t launch_mx_terms(const void* X, bool bf16, uint32_t T, uint32_t K, ui
                             cudaStream_t s);
 cudaError_t launch_mx_gemm(const MxGemm& p, uint64_t rows, uint64_t tiles, uint32_t bn, const uint8_t* ws, cudaStream_t s);
 // Zeroes an N x M output (row stride stride_d) that the GEMM launched behind it adds into.
-cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s);
+cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s, uint64_t* launches);
 // Prefill GEMM for the weight layouts without a 16-byte row pitch (MXFP4, Q6_K with K % 2048 != 0): bf16
 // activations, raw blocks fetched with cp.async (moe_gemm_tc.cu).
 bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K,

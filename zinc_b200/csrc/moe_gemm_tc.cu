@@ -710,7 +710,7 @@ cudaError_t launch_mul_mm_cp_async(uint32_t type, const uint8_t* A, uint64_t a_b
     if (g.splits > 2) {
         g.parts = parts;
     } else if (g.splits == 2) {
-        if (cudaError_t e = launch_zero(D, M, N, stride_d, s); e != cudaSuccess) return e;
+        if (cudaError_t e = launch_zero(D, M, N, stride_d, s, launches); e != cudaSuccess) return e;
     }
     const uint64_t items64 = tiles * g.splits;
     const uint32_t items = items64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)items64;
