@@ -419,8 +419,8 @@ def test_o_proj_merge(gpu, oracle, t, M, K, n_heads, nc, sink):
 @pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K, zb.Q6_K, zb.Q8_0, zb.MXFP4], ids=IDS[:5])
 @pytest.mark.parametrize("M,blocks", [(7, 2), (33, 7), (130, 17), (1025, 3), (16001, 8)])
 def test_row_and_tall_shapes(gpu, oracle, t, M, blocks):
-    """Rows and blocks that fill neither a CTA of the row kernel nor its warps' rounds, added to y; and rows enough for the
-    streaming kernels' tall cut (half the warps along K, a last tile of one row). The bar: f32 sums of at most 4352 products
+    """Rows and blocks that fill neither a CTA of the row kernel nor its warps' rounds, added to y; and rows enough for many
+    tiles per CTA of the streaming kernels, a last tile of one row. The bar: f32 sums of at most 4352 products
     against f64, 2^-24 each in the worst case."""
     torch, ctx, dd = gpu
     K = max(zb.block_size(t), 128) * blocks
@@ -496,6 +496,16 @@ def test_many_tiles_per_cta(gpu, oracle, t, M, K):
         assert rel_l2(got[lo:lo + 1021], want[lo:lo + 1021]) <= TOL
     assert torch.equal(y[:M], y2[:M])
     assert np.array_equal(z[:M].cpu().numpy(), np.float32(1.5) + got)
+
+
+@pytest.mark.parametrize("t,M,K", [(zb.Q4_K, 14341, 768), (zb.Q4_K, 9487, 10496), (zb.Q4_K, 19211, 11776), (zb.Q6_K, 7167, 7680),
+                                   (zb.Q6_K, 9487, 7680), (zb.Q6_K, 9487, 8448), (zb.Q6_K, 9487, 9216), (zb.MXFP4, 7167, 1280),
+                                   (zb.MXFP4, 9487, 1280), (zb.MXFP4, 7167, 4352)],
+                         ids=lambda v: zb.TYPE_NAMES.get(v, str(v)) if isinstance(v, int) and v < 64 else str(v))
+def test_tall_cuts(gpu, oracle, t, M, K):
+    """Four tiles per CTA and more that the warps share: on 148 SMs four, two, three rows of warps (Q4_K), four, one, three, two
+    (Q6_K), four, three, two (MXFP4), a last round of few tiles and a last tile of few rows."""
+    test_many_tiles_per_cta(gpu, oracle, t, M, K)
 
 
 @pytest.mark.parametrize("M,K", [(9475, 768), (9500, 2048), (3600, 6144)])

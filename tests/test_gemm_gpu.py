@@ -239,7 +239,7 @@ def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
     d = np.exp2(-(np.arange(M * 2) % 12)).astype(np.float16) * np.where(np.arange(M * 2) % 5 == 0, -1, 1).astype(np.float16)
     dmin = np.exp2(np.arange(M * 2) % 17 - 10).astype(np.float16)
     d[:4], dmin[4:8] = 0, 0
-    d[8:12], dmin[8:12] = np.float16(2.0 ** -14), np.float16(8.0)   # 2^17: the q terms are rounded to 11 bits
+    d[8:12], dmin[8:12] = np.float16(2.0 ** -14), np.float16(8.0)   # 2^17: both go down by powers of two
     w[:, 0:2], w[:, 2:4] = d.view(np.uint8).reshape(-1, 2), dmin.view(np.uint8).reshape(-1, 2)
     X = synth.activations(g, N, K)
     D = out_with_canary(torch, N * M)

@@ -1,6 +1,6 @@
-"""zc_dmmv_q4k_static_scratch (scratch in a __device__ array, no context, no allocation) against
-zc_dmmv on the same inputs. The file name sorts last so the shared scratch is exercised after
-every other test has run; it also passes on its own."""
+"""zc_dmmv_q4k_static_scratch (no context, no allocation, no device memory but its operands) against
+zc_dmmv on the same inputs. The file name sorts last, so that the entry point, whose set-up is its own,
+also runs after every other test; it passes on its own too."""
 import ctypes as C
 
 import numpy as np

@@ -45,7 +45,7 @@ struct FmtMX {
     using Tab = TabX;
     using X = XRegsX;
     static constexpr uint32_t kSlot = 16 * kRowSlot;
-    static constexpr uint32_t kMost = 18;
+    static constexpr uint32_t kMost = 18;  // what the registers allow: three rows of six warps at K = 2561 to 3072
     static constexpr uint32_t kCols = 512;
     static constexpr bool kFlowOne = false;
     static uint32_t flow_tiles(uint32_t K) { return K <= 2 * kCols ? 0 : 10; }

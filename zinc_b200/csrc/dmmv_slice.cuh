@@ -534,7 +534,8 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
         return true;
     };
     // Four tiles per CTA and more: the cut whose busiest warp has least to do, tiles of a CTA dealt to n_wr rows of warps, a
-    // longer share of K for each where more rows of warps fit; meetings every eight tiles or so. (Q4_K 8192 x 12288 16.3 ->
+    // longer share of K for each where more rows of warps fit; meetings every eight tiles, nine with three rows of warps (a
+    // multiple of the rows, so that none idles before one; below, with one to three tiles per CTA, four and six). (Q4_K 8192 x 12288 16.3 ->
     // 14.6 us, 11008 x 5120 12.2 -> 10.1, 65536 x 8192 53.8 -> 52.1 against the cut below.)
     const uint32_t tpc16 = ((a.M + 15) / 16 + sms * per_sm - 1) / (sms * per_sm);
     uint32_t tall_per = 0, tall_wr = 0;

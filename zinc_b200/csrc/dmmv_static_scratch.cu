@@ -22,7 +22,7 @@ namespace {
 
 using namespace zc;
 
-constexpr uint32_t kStaticMaxK = 12288;  // 48 blocks of 256: what the per-warp staging holds
+constexpr uint32_t kStaticMaxK = 12288;  // how far the streaming kernel's 21 bits of x reach; longer rows take f32 in zc_dmmv
 constexpr int kMaxDevices = 64;
 
 struct DeviceState {
@@ -111,8 +111,7 @@ extern "C" int32_t zc_dmmv_q4k_static_scratch(void* cuda_stream, const void* A, 
     const uint64_t units = ((uint64_t)M + 15) / 16 * ((K / 256 + 1) / 2);
     if (units < 16 || !warp_dmmv_eligible(T_Q4_K, MODE_PLAIN, a))
         return sfail(err_buf, err_cap, ZC_ERR_INVALID_ARG,
-                     "%s: M=%u K=%u is too small for the streaming kernel (needs at least 16 row-tile x k-segment "
-                     "units); use zc_dmmv",
+                     "%s: M=%u K=%u is too small (this entry point takes 16 row-tile x k-segment units and more); use zc_dmmv",
                      fn, M, K);
     e = launch_warp_dmmv(T_Q4_K, MODE_PLAIN, a, static_cast<cudaStream_t>(cuda_stream), nullptr);
     if (e != cudaSuccess) return sfail(err_buf, err_cap, ZC_ERR_CUDA, "%s: launch: %s", fn, cudaGetErrorString(e));

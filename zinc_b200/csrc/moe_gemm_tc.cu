@@ -310,18 +310,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const MoeGemmArgs
             if (mine && !dead) {
                 uint8_t* a_stage = smem + ((gs + q) % T::kStages) * kABytes;
                 const uint8_t* slot = smem_w + slot_c * T::kRawBytes + row * kBox;
-                if constexpr (TYPE == T_Q4_K) {
-                    const uint4 chdr = *reinterpret_cast<const uint4*>(slot);
-                    const uint4 c0 = *reinterpret_cast<const uint4*>(slot + 16 + q * 32);
-                    const uint4 c1 = *reinterpret_cast<const uint4*>(slot + 32 + q * 32);
-                    const __half2 dd = *reinterpret_cast<const __half2*>(&chdr.x);
-                    const float d = __low2float(dd), dmin = __high2float(dd);
-                    uint32_t s0, mn0, s1, mn1;
-                    scale_min_k4(2 * q, chdr.y, chdr.z, chdr.w, s0, mn0);
-                    scale_min_k4(2 * q + 1, chdr.y, chdr.z, chdr.w, s1, mn1);
-                    dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1,
-                                      a_stage, row);
-                } else if constexpr (TYPE == T_Q6_K) {
+                if constexpr (TYPE == T_Q6_K) {
                     const uint32_t off = (uint32_t)((cur.row_off + (uint64_t)cur.b * kBlock) & 15u);
                     dequant_group_q6k(slot, off, q, a_stage, row);
                 } else {
@@ -552,10 +541,9 @@ cudaError_t launch_gemm_type(uint32_t type, const CUtensorMap& map, const MoeGem
     if constexpr (BN == 160) {
         return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
     } else if constexpr (BN == 128) {
-        return type == T_Q4_K ? launch_gemm<T_Q4_K, BN>(map, g, max_items, s) : launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+        return launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
     } else {
-        if (type == T_MXFP4) return launch_gemm<T_MXFP4, BN>(map, g, max_items, s);
-        return type == T_Q4_K ? launch_gemm<T_Q4_K, BN>(map, g, max_items, s) : launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
+        return type == T_MXFP4 ? launch_gemm<T_MXFP4, BN>(map, g, max_items, s) : launch_gemm<T_Q6_K, BN>(map, g, max_items, s);
     }
 }
 cudaError_t launch_gemm_bn(uint32_t type, uint32_t bn, const CUtensorMap& map, const MoeGemmArgs& g, uint32_t max_items, cudaStream_t s) {
@@ -580,6 +568,7 @@ bool moe_grouped_eligible(uint32_t type, const uint8_t* A, uint32_t K, uint64_t 
     if (type != T_Q4_K && type != T_Q6_K && type != T_MXFP4) return false;
     if ((type == T_MXFP4 ? (K & 63u) : (K & 255u)) || K < 64 || n_experts > kMoeMaxExperts || n_pairs > 0x7FFFFFFFull)
         return false;
+    if (type == T_Q4_K && !moe_pair_eligible(type, kBM, K)) return false;  // the tile kernel here has no Q4_K
     if ((reinterpret_cast<uintptr_t>(A) & 15u) || (expert_stride & 15u)) return false;
     if ((reinterpret_cast<uintptr_t>(X) & 15u) || (x_token_stride & 3u)) return false;
     return ws_size >= ws_layout(n_pairs, K, n_experts, 32, false).total;  // the smallest tile needs the longest table
@@ -668,7 +657,7 @@ cudaError_t launch_moe_grouped(uint32_t type, const uint8_t* A, uint64_t a_bytes
 // and Q6_K with a row pitch that is not a multiple of 16 bytes. X is bf16 [N][stride_b].
 bool mul_mm_cp_async_eligible(uint32_t type, const uint8_t* A, const void* B, uint32_t N, uint32_t K,
                               uint32_t stride_b) {
-    if (type != T_MXFP4 && type != T_Q6_K && type != T_Q4_K) return false;
+    if (type != T_MXFP4 && type != T_Q6_K) return false;
     if ((type == T_MXFP4 ? (K & 63u) : (K & 255u)) || K < 64 || N < 16) return false;
     return !(reinterpret_cast<uintptr_t>(A) & 15u) && !(reinterpret_cast<uintptr_t>(B) & 15u) && !(stride_b & 7u);
 }

@@ -39,9 +39,6 @@ __device__ __forceinline__ float gate_up_act(uint32_t act, float gate, float up)
     return (gate / (1.0f + expf(-gate))) * up;
 }
 
-
-__device__ __forceinline__ uint4 lds128(const void* p) { return *reinterpret_cast<const uint4*>(p); }
-
 // Loads through the shared window (32-bit addresses from smem_u32): the pointers of the carved shared
 // memory go through integer arithmetic, after which the compiler can no longer prove the address space
 // and would fall back to generic loads.
@@ -61,9 +58,6 @@ __device__ __forceinline__ float lds_f1(uint32_t saddr) {
     return v;
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

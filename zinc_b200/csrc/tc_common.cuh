@@ -328,9 +328,10 @@ __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& 
 
 // N words that start `off` bytes (0..15) into the 16-byte aligned shared-memory address p, shifted right by `more` bits
 // (< 8) on top, read kRead bytes at a time and realigned: 16 (no bank conflicts at odd-multiple-of-16 row strides, a
-// selection by every bit of the offset) or fewer (a selection less each, two or four rows to a bank).
+// selection by every bit of the offset) or 4 (no selection, four rows to a bank).
 template <int N, int kRead = 16>
 __device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32_t (&w)[N], uint32_t more = 0) {
+    static_assert(kRead == 16 || kRead == 4, "the reads written out below");
     constexpr int V = kRead == 4 ? N + 1 : (4 * N + 2 * kRead - 2) / kRead * (kRead / 4);
     uint32_t v[V];
     const uint8_t* src = p + (off & 15u & ~(uint32_t)(kRead - 1));
@@ -342,20 +343,16 @@ __device__ __forceinline__ void lds_words(const uint8_t* p, uint32_t off, uint32
             v[i + 1] = t.y;
             v[i + 2] = t.z;
             v[i + 3] = t.w;
-        } else if constexpr (kRead == 8) {
-            const uint2 t = *reinterpret_cast<const uint2*>(src + 4 * i);
-            v[i] = t.x;
-            v[i + 1] = t.y;
         } else {
             v[i] = *reinterpret_cast<const uint32_t*>(src + 4 * i);
         }
     }
     const uint32_t sh = (off & 3u) * 8u + more;
-    if (kRead > 8 && (off & 8u)) {
+    if (kRead == 16 && (off & 8u)) {
 #pragma unroll
         for (int i = 0; i + 2 < V; ++i) v[i] = v[i + 2];
     }
-    if (kRead > 4 && (off & 4u)) {
+    if (kRead == 16 && (off & 4u)) {
 #pragma unroll
         for (int i = 0; i + 1 < V; ++i) v[i] = v[i + 1];
     }
