@@ -161,9 +161,11 @@ cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
 }
 
 // D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: eight tokens of a tile. Bound: the
-// parts' bytes, which the kernel in front has left in L2, and the launch. It costs the smallest products 2 to 4 us over
-// atomic adds in any order (Q4_K 512 x 2048, 16 tokens 13 -> 17; 1024 x 4096, 64 tokens 17 -> 21) and 4096 x 4096 nothing.
-// (Released early by the GEMM: 2 us more, its CTAs wait where the GEMM's run.)
+// parts' bytes, which the kernel in front has left in L2, and the launch. It costs the smallest products 3 to 5 us over
+// atomic adds in any order (Q4_K 512 x 2048, 16 tokens, call behind call 8.7 -> 11.9, 1024 x 4096, 64 tokens 11.3 -> 15.9) and
+// 4096 x 4096, 64 tokens 1 (17.4 -> 18.5). Released early by the GEMM it was no sooner done. Slots that the last of a
+// tile's warps adds up within the GEMM: 1024 x 4096 25.6 us where this takes 21.5 (with L2 cold), 256 tokens of 4096 x 4096
+// 60 and 40.
 template <uint32_t ROWS>
 __global__ void __launch_bounds__(256)
 add_parts_kernel(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t row_tiles, uint32_t n_tile, uint32_t per, uint32_t stride_d) {
