@@ -19,8 +19,9 @@ flush is needed between steps.
 The same line carries a `workloads` object with the other parts of the metric, each timed the same
 way with its own roofline and the clock samples that fell inside its timed loop: the single
 Q4_K 4096 x 4096 matvec, the batched-prefill dequant-GEMM cases (TFLOP/s) and the two MoE
-configurations at batch 1 and over a prefill batch. `--workload <name>` runs one of them alone and
-prints one line per case.
+configurations at batch 1 and over a prefill batch (value, us per step, share of the roofline on the
+line; `--details FILE` keeps the whole records). `--workload <name>` runs one of them alone and prints
+one line per case.
 
 N>1 (torchrun): tensor parallel over the ranks (strong scaling): Q/K/V, gate/up and LM
 head sharded by rows, O and down along K; hidden-state sums and the logits gather over NVLink
@@ -65,9 +66,9 @@ def measured_peaks():
 
 def ncu_traffic(kernel_key: str):
     """DRAM bytes per launch of the dominant kernel from the committed ncu summary
-    (a line `traffic_bytes <key> <bytes>` in profiles/dmmv_q4k_warp_kernel_gate_up.txt), or None."""
+    (a line `traffic_bytes <key> <bytes>` in profiles/dmmv_and_gemm_kernels.txt), or None."""
     try:
-        with open(os.path.join(ROOT, "profiles", "dmmv_q4k_warp_kernel_gate_up.txt")) as f:
+        with open(os.path.join(ROOT, "profiles", "dmmv_and_gemm_kernels.txt")) as f:
             for line in f:
                 w = line.split()
                 if len(w) == 3 and w[0] == "traffic_bytes" and w[1] == kernel_key:
@@ -191,6 +192,31 @@ def graph_of(torch, stream, fn):
         g.replay()
     stream.synchronize()
     return g
+
+
+def short_records(records):
+    """{"unit": .., what: [value, us per step, share of the roofline], ..} of a side workload's records."""
+    out = {"unit": records[0]["unit"]}
+    for r in records:
+        c = r.get("config", {})
+        what = c.get("workload", r.get("metric", "")).replace("prefill dequant-GEMM ", "").replace(", bf16 activations, f32 out", "")
+        what = what.replace("single Q4_K matvec ", "").replace(", f32 x", "").replace(", T=", " T").split(" MoE layer")[0]
+        if "block-scaled" in c.get("path", ""):
+            what += " block-scaled"
+        if c.get("l2", "").startswith("one weight copy"):
+            what += " L2-hot"
+        roof = r.get("roofline") or {}
+        out[what] = [float(f"{r['value']:.4g}"), float(f"{r['ms_per_step'] * 1e3:.4g}"), round(roof["frac"], 3) if "frac" in roof else None]
+    return out
+
+
+def rounded(o):
+    """Six significant digits: the line stays short enough to be read back from the end of a log."""
+    if isinstance(o, float):
+        return float(f"{o:.6g}")
+    if isinstance(o, dict):
+        return {k: rounded(v) for k, v in o.items()}
+    return [rounded(v) for v in o] if isinstance(o, list) else o
 
 
 def hbm_roofline(bytes_per_launch, us, peak, peak_kind, traffic=None, **extra):
@@ -690,6 +716,7 @@ def main():
     ap.add_argument("--layers", type=int, default=0, help="override the layer count (debug; invalidates the number)")
     ap.add_argument("--tokens", type=int, default=0, help="moe_prefill: override the prefill batch (default 512 / 1024)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
+    ap.add_argument("--details", metavar="FILE", help="decode at one GPU: the side workloads' whole records go here")
     ap.add_argument("--no-extra", action="store_true", help="decode at one GPU: leave the `workloads` object out")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3) if args.impl != "reference" else args.warmup
@@ -902,7 +929,7 @@ def main():
     if rank == 0:
         out = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
-            "warmup": args.warmup, "ms_per_step": ms_per_step, "best_ms_per_step": min(per), "timed_blocks": n_blocks,
+            "warmup": args.warmup, "ms_per_step": ms_per_step, "best_ms_per_step": min(per),
             "higher_is_better": True, "scaling": "strong",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {
@@ -910,13 +937,11 @@ def main():
                 "layers": shape.n_layers, "hidden": shape.hidden, "ffn": shape.ffn, "vocab": shape.vocab,
                 "weight_bytes_per_token": total_bytes,
                 "parallelism": "single GPU" if world == 1 else f"tp{world} (rows: QKV/gate/up/head, K: O/down; hidden-state sums: {dict(fused='rows pushed to every rank from the matvec epilogue, summed in the next matvec prologue, over NVLink peer memory', peer='one-kernel peer all-reduce over NVLink', nccl='NCCL all-reduce')[args.collective]})",
-                "l2": "inputs larger than L2: 4.88 GB of distinct weights per step, no flush needed",
-                "launch": "CUDA graph replay of the recorded op sequence",
-                "timing": f"{n_blocks} blocks of {args.steps} replays, CUDA events per block, median block reported",
+                "l2": "4.88 GB of distinct weights per step: larger than L2, no flush",
+                "launch": "CUDA graph replay",
+                "timing": f"{n_blocks} blocks of {args.steps} replays, CUDA events, median block",
             },
             "tok_s": 1e3 / ms_per_step,
-            "frac_of_nominal_8tbs": value / NOMINAL_HBM_GBS,
-            "frac_of_measured_hbm": value / (peak * world),
             "e2e": {"value": e2e_val, "unit": UNIT, "ms_per_step": e2e_s * 1e3, "steps": e2e_steps,
                     "h2d_bytes_per_step": n_in * 4, "d2h_bytes_per_step": (shape.vocab + shape.hidden) * 4},
             "gpu_launches": launches_per_step * args.steps * n_blocks,
@@ -926,15 +951,18 @@ def main():
                                      kernel="dmmv fused gate+up+SwiGLU (Q4_K), M=%d K=%d" % (M, K)),
             "roofline_step": {"bound": "hbm", "achieved": value, "peak": peak * world, "unit": "GB/s",
                               "frac": value / (peak * world)},
-            "kernels_alone": kernels,
+            "kernels_alone": {k: [v["us"], v["frac"]] for k, v in kernels.items()},  # us, share of the measured HBM rate
             "cpu_baseline": cpu_base,
             "clocks": clocks,
         }
         if check is not None:
             out["tp_check"] = {"rel_l2": check, "ranks": world, "bar": 1e-4}
         if extra is not None:
-            out["workloads"] = extra
-        print(json.dumps(out), flush=True)
+            if args.details:
+                with open(args.details, "w") as f:
+                    json.dump({**out, "workloads": extra}, f, indent=1)
+            out["workloads"] = {k: short_records(v) if isinstance(v, list) else v for k, v in extra.items()}
+        print(json.dumps(rounded(out)), flush=True)
     if dist is not None:
         teardown_distributed(torch, dist, ctx, [graph] if graph is not None else [])
     return 0
