@@ -159,7 +159,12 @@ int32_t zc_moe_dmmv_supported(uint32_t type);
  * the tall-M and batch-shader special cases there are an internal choice here.
  * Types: q4_k, q5_k, q6_k, q8_0, mxfp4, q5_0, q5_1, f16, f32; any other type
  * returns ZC_ERR_UNSUPPORTED_TYPE. K must be a multiple of the block size;
- * x + x_offset must be 16-byte aligned (src/shaders/dmmv_q6k.comp:24-27). */
+ * x + x_offset must be 16-byte aligned (src/shaders/dmmv_q6k.comp:24-27).
+ * Weights of the matvecs (every zc_dmmv_* and the decode calls of zc_moe_*) may be
+ * read while the kernel in front of the call on the stream still runs: they are
+ * uploaded by copies, or written by a kernel that has another one behind it, before
+ * the call. x, y and all other operands may come from the kernel in front. The
+ * GEMMs (zc_mul_mm*, zc_moe_dmmv_batched*) take weights from there too. */
 int32_t zc_dmmv(zc_ctx* ctx, uint32_t type,
                 const void* A, uint64_t a_size, const void* x, uint64_t x_size,
                 void* y, uint64_t y_size,
