@@ -834,14 +834,14 @@ int32_t zc_dmmv_batch(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size
     ZC_TRY(check_vec(ctx, fn, "X", X, x_size, x_offset, (uint64_t)num_cols * K * 4, 16));
     ZC_TRY(check_vec(ctx, fn, "Y", Y, y_size, y_offset, (uint64_t)num_cols * M * 4, 4));
     cudaError_t e = cudaErrorNotSupported;
-    // Small products: the matvec kernel over a grid of columns (Q6_K 500 x 2048, 8 columns: 6.8 us, 9.9 on the tensor cores).
-    // The lines cross at 9 to 11 million products, Q6_K at 13 (1024 x 2048, 5 columns 8.1 and 9.4 us, 8 columns 10.5 and
-    // 9.4), with two columns of a K-quant at 16 to 33 (Q4_K 2048 x 2560 9.0 and 12.0, 4096 x 4096 21.4 and 16.0; Q6_K 8.1
+    // Small products: the matvec kernel over a grid of columns (Q6_K 500 x 2048, 8 columns: 6.8 us, 12 on the tensor cores).
+    // The lines cross at 9 to 11 million products, Q4_K at 17 (1024 x 2048, 8 columns 11.7 and 12.1 us, 12 columns 16.1 and
+    // 12.4), Q6_K at 20 (8 columns 10.1 and 12.6, 12 columns 14.3 and 12.9), with two columns of a K-quant at 16 to 33 (Q4_K 2048 x 2560 9.0 and 12.0, 4096 x 4096 21.4 and 16.0; Q6_K 8.1
     // and 14.0, 19.7 and 19.6). Two columns of a larger MXFP4 matrix: two streaming matvecs (12288 x
     // 4096: 26 us, 31 on the tensor cores). Not so Q4_K and Q6_K, whose streaming matvecs hold x in 21 bits (17 us, 27 on
     // the tensor cores, but a relative L2 error of 1.1e-6 against 1.4e-7). Else the tensor cores.
     const bool kquant = type == T_Q4_K || type == T_Q5_K || type == T_Q6_K;
-    const bool small = (uint64_t)M * K * num_cols <= (num_cols == 2 && kquant ? 28000000u : type == T_Q6_K ? 13000000u : 10000000u);
+    const bool small = (uint64_t)M * K * num_cols <= (num_cols == 2 && kquant ? 28000000u : type == T_Q6_K ? 20000000u : type == T_Q4_K ? 17000000u : 10000000u);
     if (!small && num_cols == 2 && type == T_MXFP4) {
         e = cudaSuccess;
         for (uint32_t c = 0; c < 2 && e == cudaSuccess; ++c) {
