@@ -83,12 +83,15 @@ int32_t zc_init(int32_t device, zc_ctx** out_ctx);
 int32_t zc_destroy(zc_ctx* ctx);
 /* Use a caller-owned cudaStream_t (e.g. the framework's current stream); NULL is
  * CUDA's default stream. zc_use_own_stream goes back to the stream the context
- * created for itself (the initial state). The context's own scratch may be in use
- * on the stream before when the next call comes on another: such a call, or a
- * zc_replay there, waits on the GPU for what used the scratch last. Only graphs that
- * the caller has captured and launches without zc_replay are outside of this: one
- * that holds a zc_mul_mm or a zc_dmmv_batch may not run beside other work of the
- * same context. */
+ * created for itself (the initial state). The activation terms and partial sums
+ * that zc_mul_mm and zc_dmmv_batch keep in the context may be in use on the stream
+ * before when the next call comes on another: such a call, or a zc_replay there,
+ * waits on the GPU for their last use. Only graphs that the caller has captured and
+ * launches without zc_replay are outside of this: one that holds a zc_mul_mm or a
+ * zc_dmmv_batch may not run beside other work of the same context. The context's
+ * small state (tile flags of zc_mul_mm with bf16 activations, the logits of
+ * zc_moe_router_topk, zc_dmmv_o_proj_merge's vector) is not ordered: two of one kind
+ * may not be under way on two streams at once. */
 int32_t zc_set_stream(zc_ctx* ctx, void* cuda_stream);
 int32_t zc_use_own_stream(zc_ctx* ctx);
 void* zc_get_stream(zc_ctx* ctx);

@@ -508,7 +508,7 @@ def test_tall_cuts(gpu, oracle, t, M, K):
     test_many_tiles_per_cta(gpu, oracle, t, M, K)
 
 
-@pytest.mark.parametrize("M,K", [(9475, 768), (9500, 2048), (3600, 6144)])
+@pytest.mark.parametrize("M,K", [(9475, 768), (9500, 2048), (3600, 6144), (7130, 11776)])  # the last: warps that share tiles
 def test_many_tiles_per_cta_gate_up(gpu, oracle, M, K):
     torch, ctx, dd = gpu
     g = synth.rng(132, M)
