@@ -98,7 +98,7 @@ void* zc_get_stream(zc_ctx* ctx);
 /* Text of the last error recorded on this context (never NULL). */
 const char* zc_last_error(zc_ctx* ctx);
 const char* zc_status_string(int32_t status);
-/* Number of kernels this context has launched so far. */
+/* Number of kernels this context has launched or recorded so far. */
 uint64_t zc_launch_count(zc_ctx* ctx);
 
 /* ---- buffers --------------------------------------------------------------
@@ -136,7 +136,16 @@ int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
  * is a CUDA graph: calls made between zc_begin_record and zc_end_record are
  * captured instead of executed; zc_replay enqueues the whole sequence with one
  * launch. Buffers, sizes and offsets are baked in at record time. Host copies
- * recorded this way must use page-locked host memory. */
+ * recorded this way must use page-locked host memory.
+ * zc_end_record joins runs of zc_dmmv, zc_dmmv_multi, zc_dmmv_fused_gate_up_swiglu
+ * and zc_dmmv_sigmoid_acc calls on Q4_K and Q6_K matrices of 2 MB and more, with
+ * nothing else between them on the stream, into one kernel each. Results are those
+ * of the calls in their order; sums are taken in another order than in the calls
+ * themselves, the same one at every replay. Such a kernel uses all SMs, reads
+ * weights of later calls ahead of earlier calls' results (calls that write another
+ * one's weights are not joined) and counts as one launch. A recording owns the
+ * device memory this takes (3.5 MB for a dense 8B token) until zc_free_recording,
+ * which waits for a replay that is under way. */
 int32_t zc_begin_record(zc_ctx* ctx);
 int32_t zc_end_record(zc_ctx* ctx, void** out_recording);
 int32_t zc_replay(zc_ctx* ctx, void* recording);

@@ -1,0 +1,185 @@
+"""Recorded runs of matvecs that zc_end_record joins into one kernel: against the calls themselves and the oracle.
+
+The bars: x is 21-bit fixed point per 256 elements, up to 8 x 2^-20 a step for N(0, 1), 2.2e-6 of it rms (1.1e-6 for blocks
+whose largest is below 4); the recorded form has the same digits of x, so that the two differ by f32 sums; a chain of
+six calls passes its differences on and gate * up adds two: 2e-5.
+"""
+import numpy as np
+import pytest
+
+from helpers import canary_intact, dev, out_with_canary, rel_l2
+
+import zinc_b200 as zb
+from zinc_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+class Run:
+    """Matrices, vectors and calls on a stream of their own; every output is followed by canary words."""
+
+    def __init__(self, torch, seed):
+        self.torch = torch
+        self.stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        self.ctx = zb.Context(0, stream=self.stream.cuda_stream)
+        self.dd = zb.DmmvDispatch(self.ctx)
+        self.g = np.random.default_rng(seed)
+        self.raw = {}
+
+    def mat(self, t, M, K):
+        raw = synth.quant_matrix(self.g, t, M, K)
+        w = dev(self.torch, raw)
+        self.raw[w.data_ptr()] = raw
+        return w
+
+    def vec(self, n):
+        return dev(self.torch, self.g.standard_normal(n).astype(np.float32))
+
+    def out(self, n):
+        return out_with_canary(self.torch, n)
+
+    def eager_and_recorded(self, record, outs, launches, replays=1):
+        """Outputs of the calls and of a replay of the recorded ones, from the same start; every canary must hold."""
+        start = [o.clone() for o in outs]
+        self.torch.cuda.synchronize()
+        record()
+        self.ctx.submit_and_wait()
+        eager = [o.clone() for o in outs]
+        n0 = self.ctx.launch_count
+        with self.torch.cuda.stream(self.stream):
+            self.ctx.begin_record()
+            record()
+            rec = self.ctx.end_record()
+        assert self.ctx.launch_count - n0 == launches
+        got = None
+        for _ in range(replays):
+            for o, s in zip(outs, start):
+                o.copy_(s)
+            self.torch.cuda.synchronize()
+            self.ctx.replay(rec)
+            self.ctx.submit_and_wait()
+            now = [o.clone() for o in outs]
+            assert got is None or all(self.torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0)) for a, b in zip(got, now)), "not the same bits"
+            got = now
+        self.ctx.free_recording(rec)
+        return eager, got
+
+
+# K of one, of an odd number and of many blocks; rows that start on 16-byte boundaries (Q6_K: K % 2048 == 0) and not; row
+# counts around multiples of 16 and of 128
+@pytest.mark.parametrize("t,M,K", [(zb.Q4_K, 16400, 256), (zb.Q4_K, 4097, 1280), (zb.Q4_K, 913, 4096), (zb.Q4_K, 321, 12288),
+                                   (zb.Q6_K, 1251, 2048), (zb.Q6_K, 209, 12288), (zb.Q6_K, 10248, 256), (zb.Q6_K, 1160, 2304),
+                                   (zb.Q6_K, 136, 19 * 1024), (zb.Q6_K, 240, 12032), (zb.Q6_K, 2432, 1280)])
+def test_joined_matvecs_by_shape(gpu, oracle, t, M, K):
+    torch, _, _ = gpu
+    r = Run(torch, M + K)
+    w1, w2, x1, x2 = r.mat(t, M, K), r.mat(t, M, K), r.vec(K), r.vec(K)
+    a, b = r.out(M), r.out(M)
+    b[:M] = 0.5
+    torch.cuda.synchronize()
+
+    def record():
+        r.dd.recordDispatch(t, w1, x1, a, M, K)
+        r.dd.recordDispatch(t, w2, x2, b, M, K, acc_mode=1)
+    fits = K <= 12288   # beyond, the f32 kernels
+    eager, got = r.eager_and_recorded(record, [a, b], 1 if fits else 2, replays=3)
+    for y, e, w, x, add in ((got[0], eager[0], w1, x1, 0.0), (got[1], eager[1], w2, x2, 0.5)):
+        assert canary_intact(y, M)
+        want = oracle.dmmv_f64(r.raw[w.data_ptr()], t, M, K, x.cpu().numpy()) + add
+        assert rel_l2(y[:M].cpu().numpy(), want) <= 2.3e-6
+        assert rel_l2(y[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6
+
+
+def test_joined_calls_are_ordered_by_what_they_read_and_write(gpu):
+    """Every way in which a call can depend on an earlier one, in one run."""
+    torch, _, _ = gpu
+    r = Run(torch, 5)
+    dd, H, F = r.dd, 2304, 2048
+    wq, wk, wv = r.mat(zb.Q4_K, H, H), r.mat(zb.Q4_K, 300, H), r.mat(zb.Q4_K, 17, H)
+    wo, wg, wu, wd, wx, wh = (r.mat(zb.Q6_K, H, H), r.mat(zb.Q4_K, F, H), r.mat(zb.Q4_K, F, H), r.mat(zb.Q6_K, H, F),
+                              r.mat(zb.Q4_K, H, H), r.mat(zb.Q6_K, 1301, F))
+    x, q, k, v, act, h, z = r.out(H), r.out(H), r.out(300), r.out(17), r.out(F), r.out(H), r.out(1301)
+    x[:H], h[:H], z[:1301] = r.vec(H), r.vec(H), r.vec(1301)
+    x2 = r.vec(H)
+
+    def record():
+        dd.recordDispatchMulti(zb.Q4_K, [wq, wk, wv], x, [q, k, v], [H, 300, 17], H)
+        dd.recordDispatch(zb.Q6_K, wo, q, h, H, H, acc_mode=1)                  # reads q
+        dd.dispatchDmmvFusedGateUpSwiglu(zb.Q4_K, wg, wu, h, act, F, H)         # reads h
+        dd.recordDispatch(zb.Q6_K, wd, act, h, H, F, acc_mode=1)                # adds to the h that the call before reads
+        dd.recordDispatch(zb.Q4_K, wx, x2, x, H, H)                             # replaces the first call's x
+        dd.dispatchDmmvSigmoidAcc(zb.Q6_K, wh, x, z, q, 1301, F)                # reads the new x, and q[0]
+        dd.recordDispatchMulti(zb.Q4_K, [wk, wx], x2, [k, q], [300, H], H)      # replaces k and the gate's q
+    outs = [x, q, k, v, act, h, z]
+    for o, n in zip(outs, (H, H, 300, 17, F, H, 1301)):
+        assert canary_intact(o, n)
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=4)
+    for name, e, o, n in zip("x q k v act h z".split(), eager, got, (H, H, 300, 17, F, H, 1301)):
+        assert canary_intact(o, n), name
+        assert bool(torch.isfinite(e[:n]).all()), name
+        assert rel_l2(o[:n].cpu().numpy(), e[:n].cpu().numpy()) <= 2e-5, name
+
+
+def test_calls_that_are_not_joined(gpu):
+    """Work of others between two calls, small matrices, and calls that write what the same run reads ahead."""
+    torch, _, _ = gpu
+    r = Run(torch, 6)
+    M, K = 4096, 1024
+    w1, w2, small = r.mat(zb.Q4_K, M, K), r.mat(zb.Q4_K, M, K), r.mat(zb.Q4_K, 64, K)
+    x, a, b, c = r.vec(K), r.out(M), r.out(M), r.out(64)
+
+    def between():
+        r.dd.recordDispatch(zb.Q4_K, w1, x, a, M, K)
+        with torch.cuda.stream(r.stream):
+            a[:M].mul_(2.0)
+        r.dd.recordDispatch(zb.Q4_K, w2, a, b, M, K)
+    eager, got = r.eager_and_recorded(between, [a, b], 2)
+    for e, o in zip(eager, got):
+        assert torch.equal(e[:M], o[:M])
+
+    def three():
+        r.dd.recordDispatch(zb.Q4_K, small, x, c, 64, K)
+        r.dd.recordDispatch(zb.Q4_K, w1, x, a, M, K)
+        r.dd.recordDispatch(zb.Q4_K, w2, x, b, M, K)
+    eager, got = r.eager_and_recorded(three, [a, b, c], 2)
+    assert torch.equal(eager[2][:64], got[2][:64])
+    assert rel_l2(got[1][:M].cpu().numpy(), eager[1][:M].cpu().numpy()) <= 1.5e-6
+
+    # the second call writes into the first one's weights (a view of them as f32)
+    target = w1.view(torch.float32)[:M]
+    keep = w1.clone()
+
+    def overwrites():
+        r.dd.recordDispatch(zb.Q4_K, w1, x, a, M, K)
+        r.dd.recordDispatch(zb.Q4_K, w2, x, target, M, K)
+    n0 = r.ctx.launch_count
+    r.ctx.begin_record()
+    overwrites()
+    rec = r.ctx.end_record()
+    assert r.ctx.launch_count - n0 == 2
+    r.ctx.replay(rec)
+    r.ctx.submit_and_wait()
+    got = a[:M].clone()
+    w1.copy_(keep)
+    torch.cuda.synchronize()
+    r.dd.recordDispatch(zb.Q4_K, w1, x, a, M, K)
+    r.ctx.submit_and_wait()
+    assert torch.equal(got, a[:M])
+    r.ctx.free_recording(rec)
+
+
+def test_a_long_run_is_several_kernels(gpu):
+    """More calls than one kernel's parameters hold; each adds to the vector that the one before has written."""
+    torch, _, _ = gpu
+    r = Run(torch, 7)
+    M, K, n = 4096, 1024, 450
+    w, x, h, one = r.mat(zb.Q4_K, M, K), r.vec(K), r.out(M), r.out(M)
+
+    def record():
+        for _ in range(n):
+            r.dd.recordDispatch(zb.Q4_K, w, x, h, M, K, acc_mode=1)
+    r.dd.recordDispatch(zb.Q4_K, w, x, one, M, K)
+    _, got = r.eager_and_recorded(record, [h], 3, replays=2)
+    # n additions of equal terms: at most n roundings of 2^-24, half of that on average
+    assert rel_l2(got[0][:M].cpu().numpy(), n * one[:M].double().cpu().numpy()) <= n * 2.0 ** -24 + 2e-6

@@ -7,16 +7,24 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <vector>
 
 #include "../../include/zinc_cuda.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "program.h"
 
 namespace zc {
 cudaError_t launch_mul_mm_simple(uint32_t type, const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N,
                                  uint32_t K, uint32_t stride_b, uint32_t stride_d, bool act_bf16, cudaStream_t s,
                                  uint64_t* launches);
 }
+
+// What zc_end_record hands out.
+struct zc_recording {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<void*> memory;     // of its programs
+};
 
 struct zc_ctx {
     int device = 0;
@@ -47,6 +55,14 @@ struct zc_ctx {
     // caller-owned scratch for the grouped MoE prefill path (zc_set_workspace)
     void* workspace = nullptr;
     uint64_t workspace_size = 0;
+    // calls of the sequence being recorded that may become part of one kernel, and their graph nodes
+    struct Recorded {
+        cudaGraphNode_t node;
+        zc::ProgramOp op;
+    };
+    bool recording = false;
+    std::vector<Recorded> recorded;
+    uint64_t joined = 0;           // recorded launches that became part of another one
     char err[512] = {0};
 };
 
@@ -170,6 +186,142 @@ cudaError_t with_exact_scratch(zc_ctx* ctx, Launch launch) {
 }
 cudaError_t run_mul_mm_exact(zc_ctx* ctx, const ExactGemm& p) {
     return with_exact_scratch(ctx, [&] { return launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches); });
+}
+
+// A call that was just recorded as one kernel, described by `op`: remembered with its graph node.
+void note_op(zc_ctx* ctx, const ProgramOp& op) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v3(ctx->stream, &st, nullptr, &graph, &deps, &edges, &n) != cudaSuccess ||
+        st != cudaStreamCaptureStatusActive || n != 1)
+        return;
+    cudaGraphNodeType type;
+    if (cudaGraphNodeGetType(deps[0], &type) != cudaSuccess || type != cudaGraphNodeTypeKernel) return;
+    try {
+        ctx->recorded.push_back({deps[0], op});
+    } catch (const std::bad_alloc&) {  // the call stays a launch of its own
+    }
+}
+void note_call(zc_ctx* ctx, uint32_t type, int mode, const DmmvArgs& a) {
+    ProgramOp op;
+    if (program_op(type, mode, a, op)) note_op(ctx, op);
+}
+
+// The only neighbour of a node in the recorded graph, on one side; null when there is none, or several.
+cudaGraphNode_t only_neighbour(cudaGraphNode_t node, bool behind) {
+    cudaGraphNode_t o = nullptr;
+    cudaGraphEdgeData e;
+    size_t n = 0;
+    if ((behind ? cudaGraphNodeGetDependentNodes_v2(node, nullptr, nullptr, &n) : cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &n)) !=
+            cudaSuccess || n != 1)
+        return nullptr;
+    if ((behind ? cudaGraphNodeGetDependentNodes_v2(node, &o, &e, &n) : cudaGraphNodeGetDependencies_v2(node, &o, &e, &n)) != cudaSuccess)
+        return nullptr;
+    return o;
+}
+
+// Puts one node in the place of the nodes of a program, which follow one another and nothing else.
+cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t n, Program& p, void* func, uint32_t threads, uint32_t smem) {
+    size_t n_in = 0, n_out = 0;
+    cudaError_t e = cudaGraphNodeGetDependencies_v2(r[0].node, nullptr, nullptr, &n_in);
+    if (e == cudaSuccess) e = cudaGraphNodeGetDependentNodes_v2(r[n - 1].node, nullptr, nullptr, &n_out);
+    if (e != cudaSuccess) return e;
+    std::vector<cudaGraphNode_t> in(n_in + 1), out(n_out + 1);
+    std::vector<cudaGraphEdgeData> edges(n_in + n_out + 1);
+    if (n_in) e = cudaGraphNodeGetDependencies_v2(r[0].node, in.data(), edges.data(), &n_in);
+    if (e == cudaSuccess && n_out) e = cudaGraphNodeGetDependentNodes_v2(r[n - 1].node, out.data(), edges.data(), &n_out);
+    if (e != cudaSuccess) return e;
+    void* args[] = {&p};
+    cudaKernelNodeParams k = {};
+    k.func = func;
+    k.gridDim = dim3(p.grid);
+    k.blockDim = dim3(threads);
+    k.sharedMemBytes = smem;
+    k.kernelParams = args;
+    cudaGraphNode_t node;
+    // the edges become full dependencies: a successor that was to start early finds everything done
+    if ((e = cudaGraphAddKernelNode(&node, graph, in.data(), n_in, &k)) != cudaSuccess) return e;
+    cudaLaunchAttributeValue all_at_once = {};
+    all_at_once.cooperative = 1;
+    e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeCooperative, &all_at_once);
+    for (size_t i = 0; e == cudaSuccess && i < n_out; ++i) e = cudaGraphAddDependencies(graph, &node, &out[i], 1);
+    if (e != cudaSuccess) {
+        cudaGraphDestroyNode(node);
+        return e;
+    }
+    for (uint32_t i = 0; i < n; ++i)
+        if ((e = cudaGraphDestroyNode(r[i].node)) != cudaSuccess) return e;
+    return cudaSuccess;
+}
+
+cudaError_t free_recording(zc_recording* rec) {
+    if (!rec) return cudaSuccess;
+    cudaError_t e = rec->exec ? cudaGraphExecDestroy(rec->exec) : cudaSuccess;
+    for (void* m : rec->memory)
+        if (cudaError_t f = cudaFree(m); e == cudaSuccess) e = f;  // waits for a replay that is under way
+    delete rec;
+    return e;
+}
+
+// Runs of recorded calls with nothing between them become one kernel each (program.h). What does not fit stays as it was.
+cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
+    const std::vector<zc_ctx::Recorded>& r = ctx->recorded;
+    void* func;
+    uint32_t threads, smem;
+    if (r.size() < 2) return cudaSuccess;
+    if (program_kernel(ctx->sm_count, &func, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    std::vector<ProgramOp> ops(r.size());
+    for (size_t i = 0; i < r.size(); ++i) ops[i] = r[i].op;
+    cudaError_t e;
+    std::vector<Program> prog(1);
+    for (size_t i = 0; i + 1 < r.size();) {
+        size_t end = i + 1;
+        while (end < r.size() && only_neighbour(r[end - 1].node, true) == r[end].node && only_neighbour(r[end].node, false) == r[end - 1].node) ++end;
+        if (end - i < 2) {
+            i = end;
+            continue;
+        }
+        Program& p = prog[0];
+        const uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p);
+        if (n == 0) {
+            ++i;
+            continue;
+        }
+        std::vector<CUtensorMap> maps(p.n_maps);
+        if (!program_maps(p, maps.data())) {
+            i += n;
+            continue;
+        }
+        const size_t map_bytes = p.n_maps * sizeof(CUtensorMap), words = (2 * n + 1 + 31) & ~31u;
+        uint8_t* mem = nullptr;
+        rec->memory.reserve(rec->memory.size() + 1);
+        if (cudaMalloc(reinterpret_cast<void**>(&mem), map_bytes + words * 4 + p.table_bytes) != cudaSuccess) {  // the calls stay launches
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        rec->memory.push_back(mem);
+        p.maps = mem;
+        mem += map_bytes;
+        if ((e = cudaMemcpyAsync(const_cast<uint8_t*>(p.maps), maps.data(), map_bytes, cudaMemcpyHostToDevice, ctx->own_stream)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(mem, 0, words * 4, ctx->own_stream)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(ctx->own_stream)) != cudaSuccess) return e;
+        p.done = reinterpret_cast<uint32_t*>(mem);
+        p.converted = p.done + n;
+        p.left = p.converted + n;
+        p.tables = mem + words * 4;
+        p.status = ctx->status_dev;
+        p.spin_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 24);
+        if ((e = replace_nodes(graph, r.data() + i, n, p, func, threads, smem)) != cudaSuccess) return e;
+        ctx->joined += n - 1;
+        i += n;
+    }
+    return cudaSuccess;
 }
 
 // Common checks of one matvec-shaped call.
@@ -441,7 +593,7 @@ const char* zc_status_string(int32_t s) {
     }
 }
 
-uint64_t zc_launch_count(zc_ctx* ctx) { return ctx ? ctx->launches : 0; }
+uint64_t zc_launch_count(zc_ctx* ctx) { return ctx ? ctx->launches - ctx->joined : 0; }
 
 int32_t zc_alloc(zc_ctx* ctx, uint64_t bytes, void** out_dptr) {
     ZC_ENTER(ctx);
@@ -516,21 +668,35 @@ int32_t zc_submit_and_wait(zc_ctx* ctx) {
 int32_t zc_begin_record(zc_ctx* ctx) {
     ZC_ENTER(ctx);
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
-    return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, "zc_begin_record");
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "zc_begin_record");
+    ctx->recording = true;
+    ctx->recorded.clear();
+    return ZC_OK;
 }
 
 int32_t zc_end_record(zc_ctx* ctx, void** out_recording) {
     ZC_ENTER(ctx);
     if (!out_recording) return fail(ctx, ZC_ERR_INVALID_ARG, "zc_end_record: null output");
     *out_recording = nullptr;
+    ctx->recording = false;
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "zc_end_record");
-    cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
+    zc_recording* rec = new (std::nothrow) zc_recording();
+    if (!rec) e = cudaErrorMemoryAllocation;
+    try {
+        if (e == cudaSuccess) e = join_recorded(ctx, graph, rec);
+    } catch (const std::bad_alloc&) {
+        e = cudaErrorMemoryAllocation;
+    }
+    ctx->recorded.clear();
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&rec->exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "zc_end_record (instantiate)");
-    *out_recording = exec;
+    if (e != cudaSuccess) {
+        free_recording(rec);
+        return cuda_fail(ctx, e, "zc_end_record (instantiate)");
+    }
+    *out_recording = rec;
     return ZC_OK;
 }
 
@@ -539,7 +705,7 @@ int32_t zc_replay(zc_ctx* ctx, void* recording) {
     if (!recording) return fail(ctx, ZC_ERR_INVALID_ARG, "zc_replay: null recording");
     ExactUse use{ctx};  // which of the recordings hold a f32-accurate GEMM is not kept: once one does, all are ordered
     cudaError_t e = ctx->exact_recorded ? use.begin() : cudaSuccess;
-    if (e == cudaSuccess) e = cudaGraphLaunch(static_cast<cudaGraphExec_t>(recording), ctx->stream);
+    if (e == cudaSuccess) e = cudaGraphLaunch(static_cast<zc_recording*>(recording)->exec, ctx->stream);
     if (e == cudaSuccess && ctx->exact_recorded) e = use.end();
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, "zc_replay");
 }
@@ -547,7 +713,7 @@ int32_t zc_replay(zc_ctx* ctx, void* recording) {
 int32_t zc_free_recording(zc_ctx* ctx, void* recording) {
     ZC_ENTER(ctx);
     if (!recording) return ZC_OK;
-    cudaError_t e = cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(recording));
+    const cudaError_t e = free_recording(static_cast<zc_recording*>(recording));
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, "zc_free_recording");
 }
 
@@ -591,6 +757,7 @@ int32_t zc_dmmv(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size, cons
                                      ctx->stream, &ctx->launches);
     else
         e = launch_dmmv(type, MODE_PLAIN, a, ctx->stream, &ctx->launches);
+    if (ctx->recording && e == cudaSuccess && !router) note_call(ctx, type, MODE_PLAIN, a);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, "zc_dmmv");
 }
 
@@ -766,6 +933,8 @@ int32_t zc_dmmv_multi(zc_ctx* ctx, uint32_t type, uint32_t n, const void* const*
     cudaError_t e = cudaSuccess;
     if (warp_dmmv_multi_eligible(type, n, Ap, M, K, a)) {
         e = launch_warp_dmmv_multi(n, Ap, yp, M, a, ctx->stream, &ctx->launches);
+        ProgramOp op;
+        if (ctx->recording && e == cudaSuccess && program_op_multi(type, n, Ap, yp, M, a, op)) note_op(ctx, op);
     } else {
         for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) {  // any type, any shape: one launch per matrix
             DmmvArgs ai = a;
@@ -799,6 +968,7 @@ int32_t zc_dmmv_fused_gate_up_swiglu(zc_ctx* ctx, uint32_t type, const void* Wg,
     attach_scratch(ctx, a);
     ZC_TRY(take_pending(ctx, a));
     cudaError_t e = launch_dmmv(type, MODE_GATE_UP_SWIGLU, a, ctx->stream, &ctx->launches);
+    if (ctx->recording && e == cudaSuccess) note_call(ctx, type, MODE_GATE_UP_SWIGLU, a);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }
 
@@ -821,6 +991,7 @@ int32_t zc_dmmv_sigmoid_acc(zc_ctx* ctx, uint32_t type, const void* A, uint64_t 
     a.K = K;
     attach_scratch(ctx, a);
     cudaError_t e = launch_dmmv(type, MODE_SIGMOID_ACC, a, ctx->stream, &ctx->launches);
+    if (ctx->recording && e == cudaSuccess) note_call(ctx, type, MODE_SIGMOID_ACC, a);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }
 
