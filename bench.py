@@ -181,6 +181,26 @@ def timed_blocks(torch, stream, replay, steps: int, barrier=None, min_total_s: f
     return per, t0, t1
 
 
+class Recording:
+    """fn()'s calls through the library's own recording (zc_begin_record / zc_end_record); `launches`: the kernels of one
+    replay."""
+
+    def __init__(self, ctx, fn):
+        n0 = ctx.launch_count
+        ctx.begin_record()
+        fn()
+        self.ctx, self.handle = ctx, ctx.end_record()
+        self.launches = ctx.launch_count - n0
+
+    def replay(self):
+        self.ctx.replay(self.handle)
+
+    def reset(self):
+        if self.handle:
+            self.ctx.free_recording(self.handle)
+        self.handle = 0
+
+
 def graph_of(torch, stream, fn):
     """fn() run once eagerly (warm-up of every kernel variant), then captured into a CUDA graph."""
     fn()
@@ -448,9 +468,13 @@ def moe_decode_results(torch, zb, ctx, dd, stream, sampler, args, rank=0, world=
             continue
         launches = step.record()
         stream.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=stream):
-            step.record()
+        if world == 1:
+            graph = Recording(dd.ctx, step.record)
+            launches = graph.launches
+        else:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                step.record()
         for _ in range(4):
             graph.replay()
         per, t0, t1 = timed_blocks(torch, stream, graph.replay, 20, barrier=barrier if world > 1 else None,
@@ -816,12 +840,16 @@ def main():
         h_out = torch.empty(shape.vocab + shape.hidden, dtype=torch.float32).pin_memory()
         d_in = [step.x_norm, step.attn_out, step.ffn_act_in]
 
-        # one eager token (also the warm-up of every kernel variant), then record the graph
+        # one eager token (also the warm-up of every kernel variant), then record it
         launches_per_step = step.record()
         stream.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=stream):
-            step.record()
+        if world == 1:
+            graph = Recording(ctx, step.record)
+            launches_per_step = graph.launches
+        else:   # collectives of others may be among the calls
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                step.record()
         stream.synchronize()
 
         # ---- device-resident timing: blocks of --steps replays -------------------------------------
@@ -938,7 +966,7 @@ def main():
                 "weight_bytes_per_token": total_bytes,
                 "parallelism": "single GPU" if world == 1 else f"tp{world} (rows: QKV/gate/up/head, K: O/down; hidden-state sums: {dict(fused='rows pushed to every rank from the matvec epilogue, summed in the next matvec prologue, over NVLink peer memory', peer='one-kernel peer all-reduce over NVLink', nccl='NCCL all-reduce')[args.collective]})",
                 "l2": "4.88 GB of distinct weights per step: larger than L2, no flush",
-                "launch": "CUDA graph replay",
+                "launch": "zc_replay of the recorded token" if world == 1 else "CUDA graph replay",
                 "timing": f"{n_blocks} blocks of {args.steps} replays, CUDA events, median block",
             },
             "tok_s": 1e3 / ms_per_step,

@@ -10,7 +10,8 @@
 // one's waits for that one's tiles to be complete on all SMs; no other call waits for anything.
 // The units (16 rows x 512 columns) of a CTA's tiles are dealt to its compute warps one by one; the parts of a tile meet in
 // shared memory and are added in the order of the units: no barrier between warps, and sums that do not depend on timing.
-// Bound: HBM. A dense 8B token (4.88 GB, 145 calls) 834 us, 5.86 TB/s, 0.90 of the measured copy rate; as launches 1575.
+// Bound: HBM for some 20 tokens in a row (a dense 8B token, 4.88 GB in 145 calls, 820 us: 5.95 TB/s, 0.91 of the measured copy
+// rate), then the card's power limit (940 us at 1.66 GHz); as launches 1573 in both.
 // Arithmetic: that of the streaming matvecs (x as 21-bit fixed point per 256 elements, exact integer dot products per block).
 #include "program.h"
 
@@ -47,9 +48,9 @@ constexpr uint32_t kTables = (kSmem - 128 - kRing - kZeros - kParts * kPartBytes
 
 // ---- x tables --------------------------------------------------------------------------------------------
 // Q4_K: three digit planes of K bytes, sums per 32 elements, scale per 256. Q6_K, per 256 elements: digits in the order the
-// lanes read them (768 bytes), start values (192), scale (4).
+// lanes read them (768 bytes), the digits' sums over the sub-blocks in two parts (96), scale (4).
 __host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t K) {
-    return kind == PROG_Q4K ? (K / 256) * (768 + 32 + 4) : (K / 256) * (768 + 192 + 4);
+    return kind == PROG_Q4K ? (K / 256) * (768 + 32 + 4) : (K / 256) * (768 + 96 + 4);
 }
 // A unit in the ring: 16 rows of two blocks each, Q6_K as the 16-byte aligned bytes around them. Its rows lie an odd multiple of
 // 16 bytes apart, so that a 32-bit read of eight rows meets 32 banks.
@@ -136,10 +137,14 @@ __device__ __forceinline__ void prep_q6k(uint8_t* tab, const X8& r, uint32_t K, 
     for (int k = 0; k < 3; ++k) {
         put(b + k * 128, d.w[k][0]);
         put(b + k * 128 + 16, d.w[k][1]);
-        const int sum = s[k] + __shfl_xor_sync(0xFFFFFFFFu, s[k], 1);
-        if ((lane & 1) == 0) put(tab + (K >> 8) * 768 + blk * 192 + h * 96 + k * 32 + (j * 2 + u) * 4, (uint32_t)(-32 * sum));
+        const int sum = s[k] + __shfl_xor_sync(0xFFFFFFFFu, s[k], 1);  // of sub-block 8 h + 2 j + u: -1024 .. 2032 = 64 hi + lo
+        if ((lane & 1) == 0) {
+            uint8_t* q = tab + (K >> 8) * 768 + blk * 96 + k * 32 + 8 * h + 2 * j + u;
+            q[0] = (uint8_t)(sum & 63);
+            q[16] = (uint8_t)(sum >> 6);
+        }
     }
-    if (lane == 0) put(tab + (K >> 8) * 960 + blk * 4, __float_as_uint(d.inv));
+    if (lane == 0) put(tab + (K >> 8) * 864 + blk * 4, __float_as_uint(d.inv));
 }
 
 // ---- dot products ---------------------------------------------------------------------------------------
@@ -200,39 +205,44 @@ __device__ __forceinline__ int signed_byte(uint32_t w) {
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0u), "n"(n | ((8 | n) << 4) | ((8 | n) << 8) | ((8 | n) << 12)));
     return r;
 }
+// D(16x8,s32) += A(16x32,s8,row) * B(32x8,s8,col), k 16 .. 31 zero
+__device__ __forceinline__ void mma_s8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%6}, {%7,%6}, {%0,%1,%2,%3};"
+                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+                 : "r"(a0), "r"(a1), "r"(0u), "r"(b0));
+}
 // One super-block of rows A and B: see the Q6_K streaming matvec. kHalf: it starts in the middle of a word, 2 bytes past rA
 // and rB. x's digits come as one word per MMA; m0 and m1 put it into the register of its sub-block half (the other one, and
-// both in the dead columns, are zero).
+// both in the dead columns, are zero). The quants' offset of -32 is taken off by one MMA of the scales with the digits' sums
+// over the sub-blocks: lane t has both parts of digit t's. (As start values of the accumulators it took 32 moves per block
+// and twice the table: a dense 8B token 834 -> 820 us.)
 template <bool kHalf>
-__device__ __forceinline__ void q6k_block(uint32_t rA, uint32_t rB, uint32_t xb, uint32_t m0, uint32_t m1, uint32_t nb, uint32_t t4, float xs,
+__device__ __forceinline__ void q6k_block(uint32_t rA, uint32_t rB, uint32_t xb, uint32_t m0, uint32_t m1, uint32_t sums, uint32_t t4, float xs,
                                           Acc& acc) {
-    constexpr uint32_t kNib = 0x0F0F0F0Fu, kTop = 0x30303030u;
-    int IA = 0, IB = 0;
+    constexpr uint32_t kNib = 0x0F0F0F0Fu, kPairs = 0x33333333u;
+    int off[4] = {0, 0, 0, 0};
+    mma_s8s8(off, lds_word<kHalf>(rA + 192 + t4), lds_word<kHalf>(rB + 192 + t4), lds_u32(sums));
+    int IA = (off[0] + off[1] * 64) * -32, IB = (off[2] + off[3] * 64) * -32;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         uint32_t vA[4][2], vB[4][2];
+        auto six = [&](uint32_t l0, uint32_t l1, uint32_t q, uint32_t (&v)[4][2], int m) {
+            const uint32_t e = q & kPairs, o = (q >> 2) & kPairs;  // the top bits of quarters 0 and 2, of 1 and 3
+            v[0][m] = (l0 & kNib) | ((e << 4) & ~kNib);
+            v[1][m] = (l1 & kNib) | ((o << 4) & ~kNib);
+            v[2][m] = ((l0 >> 4) & kNib) | (e & ~kNib);
+            v[3][m] = ((l1 >> 4) & kNib) | (o & ~kNib);
+        };
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
             const uint32_t o = 16 * m + 64 * h, oh = 16 * m + 128 + 32 * h;
-            const uint32_t la0 = lds_word<kHalf>(rA + t4 + o), la1 = lds_word<kHalf>(rA + t4 + o + 32), ha = lds_word<kHalf>(rA + t4 + oh);
-            const uint32_t lb0 = lds_word<kHalf>(rB + t4 + o), lb1 = lds_word<kHalf>(rB + t4 + o + 32), hb = lds_word<kHalf>(rB + t4 + oh);
-            vA[0][m] = (la0 & kNib) | ((ha << 4) & kTop);
-            vA[1][m] = (la1 & kNib) | ((ha << 2) & kTop);
-            vA[2][m] = ((la0 >> 4) & kNib) | (ha & kTop);
-            vA[3][m] = ((la1 >> 4) & kNib) | ((ha >> 2) & kTop);
-            vB[0][m] = (lb0 & kNib) | ((hb << 4) & kTop);
-            vB[1][m] = (lb1 & kNib) | ((hb << 2) & kTop);
-            vB[2][m] = ((lb0 >> 4) & kNib) | (hb & kTop);
-            vB[3][m] = ((lb1 >> 4) & kNib) | ((hb >> 2) & kTop);
+            six(lds_word<kHalf>(rA + t4 + o), lds_word<kHalf>(rA + t4 + o + 32), lds_word<kHalf>(rA + t4 + oh), vA, m);
+            six(lds_word<kHalf>(rB + t4 + o), lds_word<kHalf>(rB + t4 + o + 32), lds_word<kHalf>(rB + t4 + oh), vB, m);
         }
         const uint32_t sA0 = lds_word<kHalf>(rA + 192 + 8 * h), sA1 = lds_word<kHalf>(rA + 196 + 8 * h);
         const uint32_t sB0 = lds_word<kHalf>(rB + 192 + 8 * h), sB1 = lds_word<kHalf>(rB + 196 + 8 * h);
         const uint4 b = lds_v4(xb + 384 * h);
-        const uint4 n01 = lds_v4(nb + 96 * h), n23 = lds_v4(nb + 96 * h + 16);
-        int c0[4] = {(int)n01.x, (int)n01.y, (int)n01.x, (int)n01.y};
-        int c1[4] = {(int)n01.z, (int)n01.w, (int)n01.z, (int)n01.w};
-        int c2[4] = {(int)n23.x, (int)n23.y, (int)n23.x, (int)n23.y};
-        int c3[4] = {(int)n23.z, (int)n23.w, (int)n23.z, (int)n23.w};
+        int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0}, c3[4] = {0, 0, 0, 0};
         mma_u8s8(c0, vA[0][0], vB[0][0], vA[0][1], vB[0][1], b.x & m0, b.x & m1);
         mma_u8s8(c1, vA[1][0], vB[1][0], vA[1][1], vB[1][1], b.y & m0, b.y & m1);
         mma_u8s8(c2, vA[2][0], vB[2][0], vA[2][1], vB[2][1], b.z & m0, b.z & m1);
@@ -257,21 +267,8 @@ __device__ __forceinline__ void gave_up(const Program& p, Sync* s, uint32_t site
     p.status[0] = 1;
     p.status[1] = site;
 }
-// The warp sleeps for up to the time given (ns) while the barrier is not there: without it the waiting warps' polls took two
-// thirds of all issued instructions.
-__device__ __forceinline__ bool sleep_on(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
-        : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ bool wait_bar(const Program& p, Sync* s, uint64_t* bar, uint32_t parity, uint32_t site) {
-    for (uint32_t n = 0; !sleep_on(bar, parity);) {
+    for (uint32_t n = 0; !mbar_try_wait(bar, parity);) {  // each sleeps for a while (test and nanosleep instead: 820 -> 834 us)
         if (++n > kWaitLimit || volatile_u32(&s->gave_up)) {
             gave_up(p, s, site);
             return false;
@@ -296,7 +293,7 @@ __device__ __forceinline__ void await_ops(const Program& p, Sync* sync, uint32_t
     if (n == 0) return;
     for (uint32_t d = lane; d < n; d += 32) {
         const uint32_t i = p.deps[first + d], want = p.ops[i].tiles;
-        poll(p, sync, 191, 0, [&] { return ld_acquire_u32(p.done + i) >= want; });
+        poll(p, sync, 191, 100, [&] { return ld_acquire_u32(p.done + i) >= want; });
     }
     __syncwarp();
     __threadfence();
@@ -351,7 +348,7 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
                     gave_up(p, sync, 195);
                     return;
                 }
-                if (polls) __nanosleep(50);
+                if (polls) __nanosleep(250);
             }
             if (lane < k) {
                 const uint32_t q = (i + lane) / units, idx = i + lane - q * units, e = (head + lane) & (kUnits - 1);
@@ -422,7 +419,7 @@ __device__ void fetch_x(const Program& p, Sync* sync, uint32_t tables, int lane)
         const ProgramOp& op = p.ops[j];
         if (tiles_here(p, j)) {
             const uint32_t need = op.wait_warps, nb = op.K >> 8;
-            poll(p, sync, 190, 100, [&] { return __all_sync(0xFFFFFFFFu, lane >= kWarps || volatile_u32(&sync->at[lane]) >= need); });
+            poll(p, sync, 190, 300, [&] { return __all_sync(0xFFFFFFFFu, lane >= kWarps || volatile_u32(&sync->at[lane]) >= need); });
             if (lane == 0) {
                 poll(p, sync, 196, 0, [&] { return ld_acquire_u32(p.converted + j) >= nb; });
                 asm volatile("fence.proxy.async;" ::: "memory");
@@ -464,10 +461,7 @@ __device__ void write_rows(const Program& p, Sync* sync, const float* parts, uin
         }
         const uint32_t n_parts = min((uint32_t)kWarps, (uint32_t)op.units), epi = op.epi;
         const bool two = op.streams == 2, adds = epi == PROG_SIGMOID_ACC || (epi == PROG_PLAIN && op.acc);
-        poll(p, sync, 198, 100, [&] { return volatile_u32(&sync->ready) > j; });  // ops that x waits for are complete
-        await_ops(p, sync, op.dep0 + op.deps_x, op.deps_y, lane);
-        __threadfence();
-        const float gate = epi == PROG_SIGMOID_ACC ? 1.0f / (1.0f + expf(-__ldcg(op.gate))) : 1.f;
+        float gate = 1.f;
         uint32_t tile = first_of(p, op.first);
         for (uint32_t q = 0; q < nt; ++q, tile += p.grid, ++seq) {
             uint32_t m = 0, tl = tile;
@@ -478,10 +472,15 @@ __device__ void write_rows(const Program& p, Sync* sync, const float* parts, uin
             const uint32_t r = op.kind == PROG_Q6K_APART ? (tl >> 3) * 128 + (tl & 7u) + lane * 8 : tl * 16 + lane;
             const bool live = lane < 16 && r < op.M[m];
             float* y = op.y[m] + r;
-            const float old = live && adds ? __ldcg(y) : 0.f;
             const uint32_t s = seq & (kParts - 1);
             wait_bar(p, sync, &sync->parts[s], (seq / kParts) & 1, 199);
             __syncwarp();
+            if (q == 0) {  // parts are there: what x waits for is complete
+                await_ops(p, sync, op.dep0 + op.deps_x, op.deps_y, lane);
+                __threadfence();
+                if (epi == PROG_SIGMOID_ACC) gate = 1.0f / (1.0f + expf(-__ldcg(op.gate)));
+            }
+            const float old = live && adds ? __ldcg(y) : 0.f;
             // lanes 0..15 add the even parts of the rows, lanes 16..31 the odd ones (gate + up: the two streams)
             const volatile float* part = parts + s * (kPartBytes / 4) + (lane & 15);
             float v = 0.f;
@@ -527,7 +526,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
                 xstep = b_live ? 256u : 0u;
             } else {
                 xb = tab + (g < 6 ? g : g - 2) * 64u + t * 16u;
-                xstep = t < 3 ? 192u : 0u;
+                xstep = g < 6 ? 96u : 0u;   // dead columns: zeros
             }
             poll(p, sync, 192, 60, [&] { return volatile_u32(&sync->ready) > cur; });
             __threadfence_block();
@@ -542,7 +541,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
         } else {
             // one of the two blocks starts on a word, the other one in the middle of one: bl, bh
             const uint32_t pitch = unit_pitch(kind), o = d.z >> 20, r = slot + g * pitch + (o & ~3u), half = (o >> 1) & 1u, blk = 2 * kb;
-            const uint32_t nb = (t < 3 ? tab + bpr * 768 + t * 32 : zeros) + blk * xstep, xs = tab + bpr * 960 + blk * 4, x = xb + blk * 768;
+            const uint32_t nb = (g < 6 ? tab + bpr * 768 + g * 16 + 4 * t : zeros) + blk * xstep, xs = tab + bpr * 864 + blk * 4, x = xb + blk * 768;
             const bool both = blk + 1 < bpr;
             if (half == 0 || both) {
                 const uint32_t a = r + half * 212;
@@ -576,7 +575,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
         v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2);
         v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
         const uint32_t seq = d.w;
-        poll(p, sync, 194, 0, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; });  // the place for its parts is free
+        poll(p, sync, 194, 100, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; });  // the place for its parts is free
         __syncwarp();
         if (t == 0) {
             float* q = parts + (seq & (kParts - 1)) * (kPartBytes / 4) + (d.y >> 16) * 16 + (kind == PROG_Q4K ? q4k_row(g) : g);
