@@ -269,13 +269,8 @@ cudaError_t free_recording(zc_recording* rec) {
 // Runs of recorded calls with nothing between them become one kernel each (program.h). What does not fit stays as it was.
 cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     const std::vector<zc_ctx::Recorded>& r = ctx->recorded;
-    void* func;
-    uint32_t threads, smem;
-    if (r.size() < 2) return cudaSuccess;
-    if (program_kernel(ctx->sm_count, &func, threads, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return cudaSuccess;
-    }
+    void* func = nullptr;
+    uint32_t threads = 0, smem = 0;
     std::vector<ProgramOp> ops(r.size());
     for (size_t i = 0; i < r.size(); ++i) ops[i] = r[i].op;
     cudaError_t e;
@@ -286,6 +281,10 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
         if (end - i < 2) {
             i = end;
             continue;
+        }
+        if (!func && program_kernel(ctx->sm_count, &func, threads, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return cudaSuccess;
         }
         Program& p = prog[0];
         const uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p);

@@ -686,9 +686,9 @@ uint32_t round128(uint32_t n) { return (n + 127u) & ~127u; }
 // Where the x tables lie in shared memory. A table can be replaced when all compute warps have passed its op.
 struct Tables {
     uint32_t lo[kProgMaxOps + 1], hi[kProgMaxOps + 1];
-    // ops [0, after) must be passed before op j's table can lie at `at`
-    uint32_t after(uint32_t j, uint32_t at, uint32_t bytes) const {
-        for (uint32_t i = j; i-- > 0;)
+    // ops [0, after) must be passed before op j's table can lie at `at`; no further back than `first`
+    uint32_t after(uint32_t j, uint32_t at, uint32_t bytes, uint32_t first = 0) const {
+        for (uint32_t i = j; i-- > first;)
             if (lo[i] < at + bytes && at < hi[i]) return i + 1;
         return 0;
     }
@@ -697,7 +697,10 @@ struct Tables {
 // in turn then always leave room for the next op's while one is in use (placed one behind the other they waited for the op in
 // use twice in four ops: a dense 8B token 906 us, 834 so).
 void place_table(Tables& t, uint32_t j, uint32_t bytes, uint32_t next) {
-    auto lag = [&](uint32_t i, uint32_t after) { return i - after < 3 ? i - after : 3u; };  // ops in between
+    auto lag = [&](uint32_t i, uint32_t at, uint32_t size) {  // ops in between, up to three
+        const uint32_t after = t.after(i, at, size, i < 4 ? 0 : i - 4);
+        return i - after < 3 ? i - after : 3u;
+    };
     auto candidates = [&](uint32_t i, uint32_t size, auto&& f) {
         f(0u);
         f(kTables - size);
@@ -710,9 +713,9 @@ void place_table(Tables& t, uint32_t j, uint32_t bytes, uint32_t next) {
     candidates(j, bytes, [&](uint32_t at) {
         t.lo[j] = at;
         t.hi[j] = at + bytes;
-        const uint32_t mine = lag(j, t.after(j, at, bytes));
+        const uint32_t mine = lag(j, at, bytes);
         uint32_t then = next ? 0u : 3u;
-        if (next) candidates(j + 1, next, [&](uint32_t b) { then = std::max(then, lag(j + 1, t.after(j + 1, b, next))); });
+        if (next) candidates(j + 1, next, [&](uint32_t b) { then = std::max(then, lag(j + 1, b, next)); });
         const uint32_t score = 1 + std::min(mine, then) * 4 + mine + then;
         if (score > best) {
             best = score;
