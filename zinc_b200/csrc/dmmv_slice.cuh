@@ -54,7 +54,12 @@ struct SliceArgs {
     uint32_t n_wk, n_wr, depth;
     uint32_t round;                // tiles between two meetings of a CTA's warps, a multiple of n_wr
     uint32_t nblk, bpe;            // blocks of a (concatenated) row; of one matrix's row
+    uint32_t tpe_mul, bpe_mul;     // reciprocals of tpe and bpe (quotient)
 };
+
+// n / d by the high word of a product, where 2^32 / d + 1 is exact for every n < limit; 0: it is not (quotient divides).
+inline uint32_t reciprocal(uint32_t d, uint64_t limit) { return d > 1 && limit * d < (1ull << 32) ? (uint32_t)((1ull << 32) / d) + 1 : 0; }
+__device__ __forceinline__ uint32_t quotient(uint32_t n, uint32_t d, uint32_t mul) { return mul ? __umulhi(n, mul) : n / d; }
 
 inline SliceArgs slice_args(const DmmvArgs& a) {
     SliceArgs s = {};
@@ -131,7 +136,7 @@ __device__ __forceinline__ Unit find_unit(const SliceArgs& a, const Slots<NS, kS
         u.end = nullptr;
         u.row0 = (T - t0) * a.h;
     } else if constexpr (kSeg == 2 || kSeg == 3) {
-        const uint32_t slot = kSeg == 2 ? T / a.tpe : kb / a.bpe;
+        const uint32_t slot = kSeg == 2 ? quotient(T, a.tpe, a.tpe_mul) : quotient(kb, a.bpe, a.bpe_mul);
         u.row0 = (kSeg == 2 ? T - slot * a.tpe : T) * a.h;
         if (kSeg == 3) u.lb = kb - slot * a.bpe;
         u.mat = slots.get(a, slot, strm);
@@ -166,7 +171,7 @@ __device__ __forceinline__ OutRow out_row(const SliceArgs& a, uint32_t T, uint32
         Mrows = sg == 0 ? a.segM[0] : sg == 1 ? a.segM[1] : a.segM[2];
         o.y = sg == 0 ? a.segY[0] : sg == 1 ? a.segY[1] : a.segY[2];
     } else if constexpr (kSeg == 2) {
-        slot = T / a.tpe;
+        slot = quotient(T, a.tpe, a.tpe_mul);
         o.row = (T - slot * a.tpe) * a.h + rr;
         o.y += (size_t)slot * a.M;
         if (o.y2) o.y2 += (size_t)slot * a.M;
@@ -507,6 +512,13 @@ __global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_slice_m
 
 constexpr uint32_t kSliceSmem1 = 232448u, kSliceSmem2 = 113u * 1024u;  // one, two CTAs per SM
 
+// Units a warp keeps in flight: four at most; two where there are more than `deep` warps. (Q6_K in sixteen warps, three and two:
+// 28672 x 12288 69.6 and 67.2 us, 5120 x 8192 14.0 and 13.3, 40000 x 10240 79.7 and 76.8.)
+inline uint32_t most_depth(uint32_t depth, uint32_t warps, uint32_t deep) {
+    const uint32_t most = warps > deep ? 2u : 4u;
+    return depth < most ? depth : most;
+}
+
 // Cuts the work. `rows(i)`: the row counts of the matrices (kSeg 1) or of one expert slot. False: x does not fit.
 template <typename F>
 bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, uint32_t& grid, uint32_t& smem) {
@@ -529,7 +541,7 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
         const uint32_t fixed = 128u + 2u * round * a.n_wk * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
         if (fixed + warps * 2u * F::kSlot > room) return false;
         a.depth = (room - fixed) / (warps * F::kSlot);
-        a.depth = a.depth > 4 ? 4 : a.depth;
+        a.depth = most_depth(a.depth, warps, F::kDeepWarps);
         smem = fixed + warps * a.depth * F::kSlot;
         return true;
     };
@@ -575,6 +587,8 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
         }
     }
     a.tpe = (a.M + a.h - 1) / a.h;
+    a.tpe_mul = reciprocal(a.tpe, a.tiles);
+    a.bpe_mul = reciprocal(a.bpe, a.nblk);
     if (kSeg == 1) {
         uint32_t t = 0;
         for (uint32_t i = 0; i < 3; ++i) {
@@ -608,12 +622,12 @@ bool flow_plan(SliceArgs& a, int NS, int sm_count, uint32_t& warps, uint32_t& gr
         const uint32_t fixed = 128u + warps * 2u * (uint32_t)NS * 16u * 4u + F::table_bytes(a.nblk);
         if (fixed + warps * 2u * F::kSlot > room) return false;
         a.depth = (room - fixed) / (warps * F::kSlot);
-        a.depth = a.depth > 4 ? 4 : a.depth;
+        a.depth = most_depth(a.depth, warps, F::kDeepWarps);
         smem = fixed + warps * a.depth * F::kSlot;
         return true;
     };
     uint32_t ctas = 2 * sms;
-    if (cut(8, kSliceSmem2)) {
+    if (a.K <= F::kFlowPairK && cut(8, kSliceSmem2)) {
         if (a.tiles * (uint32_t)NS < F::flow_tiles(a.K) * sms) return false;
     } else {
         ctas = sms;

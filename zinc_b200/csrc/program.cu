@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "kquant_dot.cuh"
 #include "stream_skel.cuh"
 #include "tc_common.cuh"
 
@@ -50,65 +51,17 @@ constexpr uint32_t kTables = (kSmem - 128 - kRing - kZeros - kParts * kPartBytes
 // Q4_K: three digit planes of K bytes, sums per 32 elements, scale per 256. Q6_K, per 256 elements: digits in the order the
 // lanes read them (768 bytes), the digits' sums over the sub-blocks in two parts (96), scale (4).
 __host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t K) {
-    return kind == PROG_Q4K ? (K / 256) * (768 + 32 + 4) : (K / 256) * (768 + 96 + 4);
+    return kind == PROG_Q4K ? (K / 256) * (768 + 32 + 4) : (K / 256) * kQ6kTable;
 }
 // A unit in the ring: 16 rows of two blocks each, Q6_K as the 16-byte aligned bytes around them. Its rows lie an odd multiple of
 // 16 bytes apart, so that a 32-bit read of eight rows meets 32 banks.
 __host__ __device__ constexpr uint32_t unit_pitch(uint32_t kind) { return kind == PROG_Q4K ? 288u : kind == PROG_Q6K ? 432u : 464u; }
 
-struct X8 {
-    float4 lo, hi;
-};
 // x may have been written by another SM within this kernel: read through L2
 __device__ __forceinline__ X8 load_x(const float* x, uint32_t blk, int lane) {
     const float4* p = reinterpret_cast<const float4*>(x + (size_t)blk * 256 + 8 * lane);
     return {__ldcg(p), __ldcg(p + 1)};
 }
-__device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
-}
-__device__ __forceinline__ void put(uint8_t* p, uint32_t v) { *reinterpret_cast<uint32_t*>(p) = v; }
-__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-
-// Lane l holds elements 8 l .. 8 l + 7 of a block of 256: X = round(x 2^f), |X| <= 2^20, as digits b0 2^14 + b1 2^7 + b2.
-struct Digits {
-    int X[8];
-    uint32_t w[3][2];
-    float inv;  // 2^-f
-};
-__device__ __forceinline__ Digits digits_of(const X8& r) {
-    const float v[8] = {r.lo.x, r.lo.y, r.lo.z, r.lo.w, r.hi.x, r.hi.y, r.hi.z, r.hi.w};
-    float mx = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
-    uint32_t E = (__float_as_uint(mx) >> 23) & 0xFFu;
-    E = E < 32u ? 32u : E;
-    const float scale = __uint_as_float((273u - E) << 23);
-    Digits d;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) d.X[i] = __float2int_rn(v[i] * scale);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int* X = d.X + 4 * h;
-        d.w[0][h] = pack4(X[0] >> 14, X[1] >> 14, X[2] >> 14, X[3] >> 14);
-        d.w[1][h] = pack4(X[0] >> 7, X[1] >> 7, X[2] >> 7, X[3] >> 7) & 0x7F7F7F7Fu;
-        d.w[2][h] = pack4(X[0], X[1], X[2], X[3]) & 0x7F7F7F7Fu;
-    }
-    d.inv = __uint_as_float((E - 19u) << 23);
-    return d;
-}
-
 __device__ __forceinline__ void prep_q4k(uint8_t* tab, const X8& r, uint32_t K, uint32_t blk, int lane) {
     const Digits d = digits_of(r);
 #pragma unroll
@@ -121,32 +74,6 @@ __device__ __forceinline__ void prep_q4k(uint8_t* tab, const X8& r, uint32_t K, 
     if ((lane & 3) == 0) put(tab + 3 * K + (blk * 8 + (lane >> 2)) * 4, __float_as_uint((float)sum));
     if (lane == 0) put(tab + 3 * K + (K >> 8) * 32 + blk * 4, __float_as_uint(d.inv));
 }
-// lane l: half h = l / 16, quarter j = (l / 4) % 4, sub-block half u = (l / 2) % 2, k slots t0, t0 + 1 with t0 = 2 (l % 2)
-__device__ __forceinline__ void prep_q6k(uint8_t* tab, const X8& r, uint32_t K, uint32_t blk, int lane) {
-    const Digits d = digits_of(r);
-    const uint32_t h = lane >> 4, j = (lane >> 2) & 3, u = (lane >> 1) & 1, t0 = 2 * (lane & 1);
-    uint8_t* const b = tab + blk * 768 + h * 384 + u * 64 + t0 * 16 + j * 4;
-    int s[3] = {0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        s[0] += d.X[i] >> 14;
-        s[1] += (d.X[i] >> 7) & 0x7F;
-        s[2] += d.X[i] & 0x7F;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        put(b + k * 128, d.w[k][0]);
-        put(b + k * 128 + 16, d.w[k][1]);
-        const int sum = s[k] + __shfl_xor_sync(0xFFFFFFFFu, s[k], 1);  // of sub-block 8 h + 2 j + u: -1024 .. 2032 = 64 hi + lo
-        if ((lane & 1) == 0) {
-            uint8_t* q = tab + (K >> 8) * 768 + blk * 96 + k * 32 + 8 * h + 2 * j + u;
-            q[0] = (uint8_t)(sum & 63);
-            q[16] = (uint8_t)(sum >> 6);
-        }
-    }
-    if (lane == 0) put(tab + (K >> 8) * 864 + blk * 4, __float_as_uint(d.inv));
-}
-
 // ---- dot products ---------------------------------------------------------------------------------------
 struct Acc {
     float M[2], m[2];
@@ -192,68 +119,6 @@ __device__ __forceinline__ void q4k_block(uint32_t rA, uint32_t rB, uint32_t xb,
     acc.M[1] = fmaf(dB, PB, acc.M[1]);
     acc.m[0] = fmaf(dmA, mA, acc.m[0]);
     acc.m[1] = fmaf(dmB, mB, acc.m[1]);
-}
-
-// The word at `a`, or half a word past it.
-template <bool kHalf>
-__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
-    return kHalf ? __byte_perm(lds_u32(a), lds_u32(a + 4), 0x5432) : lds_u32(a);
-}
-template <int n>
-__device__ __forceinline__ int signed_byte(uint32_t w) {
-    int r;  // selector nibble n takes byte n, 8 | n replicates that byte's sign bit
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0u), "n"(n | ((8 | n) << 4) | ((8 | n) << 8) | ((8 | n) << 12)));
-    return r;
-}
-// D(16x8,s32) += A(16x32,s8,row) * B(32x8,s8,col), k 16 .. 31 zero
-__device__ __forceinline__ void mma_s8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%6}, {%7,%6}, {%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-                 : "r"(a0), "r"(a1), "r"(0u), "r"(b0));
-}
-// One super-block of rows A and B: see the Q6_K streaming matvec. kHalf: it starts in the middle of a word, 2 bytes past rA
-// and rB. x's digits come as one word per MMA; m0 and m1 put it into the register of its sub-block half (the other one, and
-// both in the dead columns, are zero). The quants' offset of -32 is taken off by one MMA of the scales with the digits' sums
-// over the sub-blocks: lane t has both parts of digit t's. (As start values of the accumulators it took 32 moves per block
-// and twice the table: a dense 8B token 834 -> 820 us.)
-template <bool kHalf>
-__device__ __forceinline__ void q6k_block(uint32_t rA, uint32_t rB, uint32_t xb, uint32_t m0, uint32_t m1, uint32_t sums, uint32_t t4, float xs,
-                                          Acc& acc) {
-    constexpr uint32_t kNib = 0x0F0F0F0Fu, kPairs = 0x33333333u;
-    int off[4] = {0, 0, 0, 0};
-    mma_s8s8(off, lds_word<kHalf>(rA + 192 + t4), lds_word<kHalf>(rB + 192 + t4), lds_u32(sums));
-    int IA = (off[0] + off[1] * 64) * -32, IB = (off[2] + off[3] * 64) * -32;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t vA[4][2], vB[4][2];
-        auto six = [&](uint32_t l0, uint32_t l1, uint32_t q, uint32_t (&v)[4][2], int m) {
-            const uint32_t e = q & kPairs, o = (q >> 2) & kPairs;  // the top bits of quarters 0 and 2, of 1 and 3
-            v[0][m] = (l0 & kNib) | ((e << 4) & ~kNib);
-            v[1][m] = (l1 & kNib) | ((o << 4) & ~kNib);
-            v[2][m] = ((l0 >> 4) & kNib) | (e & ~kNib);
-            v[3][m] = ((l1 >> 4) & kNib) | (o & ~kNib);
-        };
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const uint32_t o = 16 * m + 64 * h, oh = 16 * m + 128 + 32 * h;
-            six(lds_word<kHalf>(rA + t4 + o), lds_word<kHalf>(rA + t4 + o + 32), lds_word<kHalf>(rA + t4 + oh), vA, m);
-            six(lds_word<kHalf>(rB + t4 + o), lds_word<kHalf>(rB + t4 + o + 32), lds_word<kHalf>(rB + t4 + oh), vB, m);
-        }
-        const uint32_t sA0 = lds_word<kHalf>(rA + 192 + 8 * h), sA1 = lds_word<kHalf>(rA + 196 + 8 * h);
-        const uint32_t sB0 = lds_word<kHalf>(rB + 192 + 8 * h), sB1 = lds_word<kHalf>(rB + 196 + 8 * h);
-        const uint4 b = lds_v4(xb + 384 * h);
-        int c0[4] = {0, 0, 0, 0}, c1[4] = {0, 0, 0, 0}, c2[4] = {0, 0, 0, 0}, c3[4] = {0, 0, 0, 0};
-        mma_u8s8(c0, vA[0][0], vB[0][0], vA[0][1], vB[0][1], b.x & m0, b.x & m1);
-        mma_u8s8(c1, vA[1][0], vB[1][0], vA[1][1], vB[1][1], b.y & m0, b.y & m1);
-        mma_u8s8(c2, vA[2][0], vB[2][0], vA[2][1], vB[2][1], b.z & m0, b.z & m1);
-        mma_u8s8(c3, vA[3][0], vB[3][0], vA[3][1], vB[3][1], b.w & m0, b.w & m1);
-        IA += c0[0] * signed_byte<0>(sA0) + c0[1] * signed_byte<1>(sA0) + c1[0] * signed_byte<2>(sA0) + c1[1] * signed_byte<3>(sA0) +
-              c2[0] * signed_byte<0>(sA1) + c2[1] * signed_byte<1>(sA1) + c3[0] * signed_byte<2>(sA1) + c3[1] * signed_byte<3>(sA1);
-        IB += c0[2] * signed_byte<0>(sB0) + c0[3] * signed_byte<1>(sB0) + c1[2] * signed_byte<2>(sB0) + c1[3] * signed_byte<3>(sB0) +
-              c2[2] * signed_byte<0>(sB1) + c2[3] * signed_byte<1>(sB1) + c3[2] * signed_byte<2>(sB1) + c3[3] * signed_byte<3>(sB1);
-    }
-    acc.M[0] = fmaf(h2f(lds_u16(rA + (kHalf ? 210 : 208))) * xs, (float)IA, acc.M[0]);
-    acc.M[1] = fmaf(h2f(lds_u16(rB + (kHalf ? 210 : 208))) * xs, (float)IB, acc.M[1]);
 }
 
 // ---- waits ------------------------------------------------------------------------------------------------
@@ -403,7 +268,7 @@ __device__ void convert_x(const Program& p, Sync* sync, int lane) {
         for (; b < nb; b += p.grid, ++n) {
             const X8 r = load_x(op.x, b, lane);
             if (op.kind == PROG_Q4K) prep_q4k(tab, r, op.K, b, lane);
-            else prep_q6k(tab, r, op.K, b, lane);
+            else prep_q6k(tab, r, op.K >> 8, b, lane);
         }
         __threadfence();
         asm volatile("fence.proxy.async;" ::: "memory");  // read by bulk copies
@@ -500,7 +365,7 @@ __device__ void write_rows(const Program& p, Sync* sync, const float* parts, uin
 __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t tables, uint32_t zeros, float* parts, uint32_t warp, int lane) {
     const uint32_t g = lane >> 2, t = lane & 3;
     const uint32_t msel = (2u * t) | ((2u * t + 1u) << 4) | 0x7700u;
-    const uint32_t m0 = g < 6 && (g & 1) == 0 ? 0xFFFFFFFFu : 0u, m1 = g < 6 && (g & 1) ? 0xFFFFFFFFu : 0u;
+    const uint32_t m0 = g < 6 && (g & 1) == 0 ? 1u : 0u, m1 = g < 6 && (g & 1) ? 1u : 0u;
     Acc acc;
     acc.clear();
     uint32_t cur = 0xFFFFFFFFu, kind = 0, tab = 0, bpr = 0, xb = 0, xstep = 0;
@@ -545,11 +410,11 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
             const bool both = blk + 1 < bpr;
             if (half == 0 || both) {
                 const uint32_t a = r + half * 212;
-                q6k_block<false>(a, a + 8 * pitch, x + half * 768, m0, m1, nb + half * xstep, 4 * t, lds_f1(xs + half * 4), acc);
+                q6k_block<kWord>(a, a + 8 * pitch, 0u, 0u, x + half * 768, m0, m1, nb + half * xstep, 4 * t, lds_f1(xs + half * 4), acc.M);
             }
             if (half == 1 || both) {
                 const uint32_t a = r + (half ^ 1u) * 208, b = half ^ 1u;
-                q6k_block<true>(a, a + 8 * pitch, x + b * 768, m0, m1, nb + b * xstep, 4 * t, lds_f1(xs + b * 4), acc);
+                q6k_block<kHalfWord>(a, a + 8 * pitch, 0u, 0u, x + b * 768, m0, m1, nb + b * xstep, 4 * t, lds_f1(xs + b * 4), acc.M);
             }
         }
         // The place may be refilled once its reads are done: the sums depend on all of them.
