@@ -183,3 +183,20 @@ def test_a_long_run_is_several_kernels(gpu):
     _, got = r.eager_and_recorded(record, [h], 3, replays=2)
     # n additions of equal terms: at most n roundings of 2^-24, half of that on average
     assert rel_l2(got[0][:M].cpu().numpy(), n * one[:M].double().cpu().numpy()) <= n * 2.0 ** -24 + 2e-6
+
+
+# Q6_K matvecs around the borders of their forms: 4.5 tiles of 16 rows per SM (148), K up to 8192 on 16-byte rows and 7424 else
+@pytest.mark.parametrize("M,K", [(10656, 8192), (10640, 8192), (10656, 7424), (10656, 7680), (4736, 7424), (10656, 10240)])
+def test_q6k_matvec_forms(gpu, oracle, M, K):
+    torch, _, _ = gpu
+    r = Run(torch, M + K)
+    w, x, y = r.mat(zb.Q6_K, M, K), r.vec(K), r.out(M)
+    torch.cuda.synchronize()
+    r.dd.recordDispatch(zb.Q6_K, w, x, y, M, K)
+    r.ctx.submit_and_wait()
+    assert canary_intact(y, M)
+    row = K // 256 * 210
+    raw = r.raw[w.data_ptr()].reshape(-1)
+    for lo in (0, M // 2 // 16 * 16, M - 64):
+        want = oracle.dmmv_f64(raw[lo * row:(lo + 64) * row], zb.Q6_K, 64, K, x.cpu().numpy())
+        assert rel_l2(y[lo:lo + 64].cpu().numpy(), want) <= 2.3e-6

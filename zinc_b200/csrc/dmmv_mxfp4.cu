@@ -48,9 +48,9 @@ struct FmtMX {
     static constexpr uint32_t kMost = 18;  // what the registers allow: three rows of six warps at K = 2561 to 3072
     static constexpr uint32_t kCols = 512;
     static constexpr bool kFlowOne = false;
-    static constexpr uint32_t kFlowPairK = 0xFFFFFFFFu;
     static constexpr uint32_t kDeepWarps = 32;
-    static uint32_t flow_tiles(uint32_t K) { return K <= 2 * kCols ? 0 : 10; }
+    static bool flow_pair(uint32_t) { return true; }
+    static uint32_t flow_tiles(uint32_t K) { return K <= 2 * kCols ? 0 : 20; }
     static uint32_t table_bytes(uint32_t nblk) { return kZeroUnits * 16 + nblk * (2048 + 8) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;

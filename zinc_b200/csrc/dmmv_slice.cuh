@@ -601,16 +601,19 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
 }
 
 // The cut of the other form (flow_body), where it is the faster one: many tiles per SM.
-// F::flow_tiles(K): from how many tiles per SM (both streams counted) eight warps on each of two CTAs are ahead where x fits
-// twice on an SM. Measured over 250 shapes, this form against the one above:
+// F::flow_pair(K): whether eight warps on each of two CTAs are tried, F::flow_tiles(K): from how many tiles per two SMs (both
+// streams counted) they are ahead. In tiles per SM, measured over 250 shapes, this form against the one above:
 //   Q4_K   K <= 512 always (65536 rows 6.2 and 9.2 us: most warps had no block); K <= 4096 from 8 (K = 4096, 16500 rows 10.4
 //          and 10.2, 20000 rows 11.7 and 12.7, 28672 rows 14.9 and 16.6), beyond from 3 (5120 x 5120 7.5 and 7.7, 14336 x
 //          5120 11.3 and 12.9)
 //   Q6_K   from 2 (5120 x 2816 8.4 and 9.4, 8192 x 4608 13.8 and 17.7, 21669 x 4608 29.6 and 34.2, 128256 x 3072 87.6 and
 //          105.9, 151936 x 4096 99.4 and 109.9; the other way 20000 x 5120 31.1 and 30.1)
 //   MXFP4  K <= 1024 always (20000 x 512 4.1 and 7.8), beyond from 10 (20000 x 2880 14.4 and 13.8, 28672 x 2880 19.3 and 20.4)
-// Where x fits only once, Q6_K takes one CTA of sixteen warps from 4.5 tiles per SM (8192 x 12288 25.5 and 25.0 us, 11008
-// rows 28.7 and 30.1, 28672 rows 62.3 and 70.0); the others stay above (Q4_K 65536 x 12288 76 and 74).
+//          K = 8192 (rows on 16-byte boundaries) from 4.5 (12000 rows 23.1 us, one CTA 24.9, the form above 24.2; 28672 rows
+//          43.6, 47.7; below, 8192 rows 18.9 and 16.9)
+// Beyond, Q6_K takes one CTA of sixteen warps from 4.5 tiles per SM (8192 x 12288 25.5 and 25.0 us, 11008 rows 28.7 and 30.1,
+// 28672 rows 62.3 and 70.0; two CTAs of eight, 11008 rows 32.8, 30000 x 12032 90.9 for 78.5, 12000 x 7936 28.9 for 27.5); the
+// others stay above (Q4_K 65536 x 12288 76 and 74).
 template <typename F>
 bool flow_plan(SliceArgs& a, int NS, int sm_count, uint32_t& warps, uint32_t& grid, uint32_t& smem) {
     a.nblk = a.bpe = (a.K + F::kCols - 1) / F::kCols;
@@ -627,8 +630,8 @@ bool flow_plan(SliceArgs& a, int NS, int sm_count, uint32_t& warps, uint32_t& gr
         return true;
     };
     uint32_t ctas = 2 * sms;
-    if (a.K <= F::kFlowPairK && cut(8, kSliceSmem2)) {
-        if (a.tiles * (uint32_t)NS < F::flow_tiles(a.K) * sms) return false;
+    if (F::flow_pair(a.K) && cut(8, kSliceSmem2)) {
+        if (a.tiles * (uint32_t)NS * 2 < F::flow_tiles(a.K) * sms) return false;
     } else {
         ctas = sms;
         if (!F::kFlowOne || a.tiles * 2 < 9 * sms || !cut(16, kSliceSmem1)) return false;

@@ -134,9 +134,9 @@ struct FmtQ4K {
     static constexpr uint32_t kMost = 16;
     static constexpr uint32_t kCols = kCB * 256;
     static constexpr bool kFlowOne = false;
-    static constexpr uint32_t kFlowPairK = 0xFFFFFFFFu;
     static constexpr uint32_t kDeepWarps = 32;
-    static uint32_t flow_tiles(uint32_t K) { return K <= kCols ? 0 : K <= 4096 ? 8 : 3; }
+    static bool flow_pair(uint32_t) { return true; }
+    static uint32_t flow_tiles(uint32_t K) { return K <= kCols ? 0 : K <= 4096 ? 16 : 6; }
     static uint32_t table_bytes(uint32_t nblk) { return kZeroBytes + nblk * kCB * (768 + 32 + 4) + 128; }
     static __device__ __forceinline__ Tab carve(uint8_t* p, uint32_t nblk) {
         Tab t;
