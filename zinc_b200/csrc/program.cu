@@ -4,14 +4,14 @@
 //
 // As launches of their own the matvecs of a dense decode token (145 of them, 5 to 14 us each) spend about 3 us apiece on
 // what is not streaming: CTAs wait for room, convert x, drain. Here one CTA per SM walks through all of them, and its warps
-// have roles: one requests weights, across the borders of the calls, as weights depend on no kernel; twelve compute; one
+// have roles: one requests weights, across the borders of the calls, as weights depend on no kernel; fourteen compute; one
 // converts its share of the calls' x (every block of x is converted once on the GPU, not once per SM) and one brings
 // converted x into shared memory, both ahead; three add up and write finished rows. A call whose x or y meets an earlier
 // one's waits for that one's tiles to be complete on all SMs; no other call waits for anything.
 // The units (16 rows x 512 columns) of a CTA's tiles are dealt to its compute warps one by one; the parts of a tile meet in
 // shared memory and are added in the order of the units: no barrier between warps, and sums that do not depend on timing.
-// Bound: HBM for some 20 tokens in a row (a dense 8B token, 4.88 GB in 145 calls, 820 us: 5.95 TB/s, 0.91 of the measured copy
-// rate), then the card's power limit (940 us at 1.66 GHz); as launches 1573 in both.
+// Bound: HBM for some 20 tokens in a row (a dense 8B token, 4.88 GB in 145 calls, 801 us: 6.1 TB/s, 0.93 of the measured copy
+// rate), then the card's power limit (920-935 us at 1.66 GHz); as launches 1573 in both.
 // Arithmetic: that of the streaming matvecs (x as 21-bit fixed point per 256 elements, exact integer dot products per block).
 #include "program.h"
 
@@ -25,7 +25,8 @@
 namespace zc {
 namespace {
 
-constexpr int kWarps = 12, kWriters = 3, kBlockThreads = (kWarps + 3 + kWriters) * 32;  // warps that compute; that write rows
+// warps that compute (dense 8B token, 8 / 10 / 12 / 14 / 16: 892 / 823 / 815 / 801 / 844 us, the last short of registers); that write rows
+constexpr int kWarps = 14, kWriters = 3, kBlockThreads = (kWarps + 3 + kWriters) * 32;
 constexpr uint32_t kRing = 161280;           // bytes of weights under way: 35 units of Q4_K, 23 of Q6_K (21 where rows are not aligned)
 constexpr uint32_t kUnits = 64;              // barriers and descriptions; at most kUnits - kWarps units are under way
 constexpr uint32_t kParts = 8;               // tiles of a CTA whose parts may be under way
