@@ -91,6 +91,60 @@ def test_joined_matvecs_by_shape(gpu, oracle, t, M, K):
         assert rel_l2(y[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6
 
 
+# Eight tiles of an SM may have their parts under way, and three warps write rows, a call each in turn. Shapes that put 8 to 35
+# tiles of two consecutive calls on an SM (148 SMs), tiles of one unit (K = 256, 512), which complete out of order, and of more.
+@pytest.mark.parametrize("t,shapes", [
+    (zb.Q4_K, [(10240, 1024)] * 3), (zb.Q4_K, [(40000, 512)] * 2), (zb.Q4_K, [(20480, 512)] * 2 + [(10240, 512)]),
+    (zb.Q4_K, [(9480, 1024), (9472, 1024), (18960, 256), (16576, 256), (18944, 512), (18960, 768)]), (zb.Q4_K, [(16576, 256)] * 7),
+    (zb.Q4_K, [(304, 12288), (21312, 256), (304, 12288), (304, 12288), (21312, 256), (4736, 1024)]),
+    (zb.Q6_K, [(16640, 256)] * 5), (zb.Q6_K, [(20024, 512), (300 * 8, 2048), (9472, 1024), (11008, 2048), (9480, 1280)])])
+def test_many_tiles_per_sm(gpu, t, shapes):
+    torch, _, _ = gpu
+    r = Run(torch, 8)
+    w = {s: synth.torch_quant_matrix(t, *s, torch.device("cuda"), 11 + i) for i, s in enumerate(dict.fromkeys(shapes))}
+    xs = {K: r.vec(K) for _, K in shapes}
+    outs = [r.out(M) for M, _ in shapes]
+    torch.cuda.synchronize()
+
+    def record():
+        for y, (M, K) in zip(outs, shapes):
+            r.dd.recordDispatch(t, w[M, K], xs[K], y, M, K)
+        M, K = shapes[0]
+        r.dd.recordDispatch(t, w[M, K], xs[K], outs[0], M, K, acc_mode=1)
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=20)
+    for (M, _), e, o in zip(shapes, eager, got):
+        assert canary_intact(o, M)
+        assert rel_l2(o[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6
+
+
+# A layer and the next one's Q, K and V of dense models from 8B to 70B, each call reading what the ones before wrote. Down
+# projections with K > 12288 stay launches of their own.
+@pytest.mark.parametrize("H,q_dim,kv,F,launches", [(4096, 4096, 1024, 12288, 1), (5120, 5120, 5120, 12288, 1), (5120, 5120, 5120, 13824, 3),
+                                                   (4096, 4096, 1024, 14336, 3), (8192, 8192, 1024, 28672, 3)])
+def test_layers_of_dense_models(gpu, H, q_dim, kv, F, launches):
+    torch, _, _ = gpu
+    r = Run(torch, 9)
+    dd, cuda = r.dd, torch.device("cuda")
+    wq, wk, wv, wo, wg, wu = (synth.torch_quant_matrix(zb.Q4_K, M, K, cuda, 21 + i) for i, (M, K) in
+                              enumerate([(q_dim, H), (kv, H), (kv, H), (H, q_dim), (F, H), (F, H)]))
+    wd = synth.torch_quant_matrix(zb.Q6_K, H, F, cuda, 31)
+    sizes = (q_dim, kv, kv, H, F)
+    q, k, v, h, act = outs = [r.out(n) for n in sizes]
+    h[:H] = r.vec(H).abs()   # the weights are positive in the mean: so are all gates
+
+    def record():
+        dd.recordDispatchMulti(zb.Q4_K, [wq, wk, wv], h, [q, k, v], [q_dim, kv, kv], H)
+        dd.recordDispatch(zb.Q4_K, wo, q, h, H, q_dim, acc_mode=1)
+        dd.dispatchDmmvFusedGateUpSwiglu(zb.Q4_K, wg, wu, h, act, F, H)
+        dd.recordDispatch(zb.Q6_K, wd, act, h, H, F, acc_mode=1)
+        dd.recordDispatchMulti(zb.Q4_K, [wq, wk, wv], h, [q, k, v], [q_dim, kv, kv], H)
+    eager, got = r.eager_and_recorded(record, outs, launches, replays=20)
+    for name, e, o, n in zip("q k v h act".split(), eager, got, sizes):
+        assert canary_intact(o, n), name
+        assert bool(torch.isfinite(e[:n]).all()), name
+        assert rel_l2(o[:n].cpu().numpy(), e[:n].cpu().numpy()) <= 2e-5, name
+
+
 def test_joined_calls_are_ordered_by_what_they_read_and_write(gpu):
     """Every way in which a call can depend on an earlier one, in one run."""
     torch, _, _ = gpu

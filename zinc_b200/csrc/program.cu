@@ -339,6 +339,8 @@ __device__ void write_rows(const Program& p, Sync* sync, const float* parts, uin
             const bool live = lane < 16 && r < op.M[m];
             float* y = op.y[m] + r;
             const uint32_t s = seq & (kParts - 1);
+            // The parity tells a round from the one before only, and the tile before in this place may be another row writer's.
+            poll(p, sync, 198, 60, [&] { return volatile_u32(&sync->added[s]) == seq / kParts; });
             wait_bar(p, sync, &sync->parts[s], (seq / kParts) & 1, 199);
             __syncwarp();
             if (q == 0) {  // parts are there: what x waits for is complete
