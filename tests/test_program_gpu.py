@@ -239,6 +239,26 @@ def test_a_long_run_is_several_kernels(gpu):
     assert rel_l2(got[0][:M].cpu().numpy(), n * one[:M].double().cpu().numpy()) <= n * 2.0 ** -24 + 2e-6
 
 
+@pytest.mark.parametrize("shapes", [[(8200, 1024)] * 2, [(8200, 1024), (4104, 2048)], [(4096, 1024), (2400, 2048), (8200, 1024)]])
+def test_a_recording_in_the_memory_of_an_earlier_one(gpu, shapes):
+    """What a recording left behind (its tensor maps lie in memory that the next one gets) is not used by the next."""
+    torch, _, _ = gpu
+    r = Run(torch, 10)
+    cuda = torch.device("cuda")
+    for i in range(12):
+        M, K = shapes[i % len(shapes)]
+        t = (zb.Q4_K, zb.Q6_K)[i // 2 % 2]
+        ws = [synth.torch_quant_matrix(t, M, K, cuda, 100 * i + n) for n in range(3)]
+        x, outs = r.vec(K), [r.out(M) for _ in ws]
+
+        def record():
+            for w, y in zip(ws, outs):
+                r.dd.recordDispatch(t, w, x, y, M, K)
+        eager, got = r.eager_and_recorded(record, outs, 1)
+        for e, o in zip(eager, got):
+            assert rel_l2(o[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6, i
+
+
 # Q6_K matvecs around the borders of their forms: 4.5 tiles of 16 rows per SM (148), K up to 8192 on 16-byte rows and 7424 else
 @pytest.mark.parametrize("M,K", [(10656, 8192), (10640, 8192), (10656, 7424), (10656, 7680), (4736, 7424), (10656, 10240)])
 def test_q6k_matvec_forms(gpu, oracle, M, K):

@@ -43,6 +43,7 @@ struct Sync {
     uint32_t at[kWarps];                     // the op a compute warp has reached
     uint64_t parts[kParts];                  // the parts of a tile: kWarps arrivals, the first part's makes up for missing ones
     uint32_t added[kParts];                  // tiles that have been added up from that place
+    uint32_t maps_ready;                     // tensor maps that can be used
     uint32_t ready;                          // ops whose x table is there
     uint32_t gave_up;
 };
@@ -178,6 +179,23 @@ __device__ __forceinline__ uint32_t tiles_here(const Program& p, uint32_t op) {
 __device__ __forceinline__ uint32_t units_taken(const Sync* sync, int lane) {
     return __reduce_min_sync(0xFFFFFFFFu, lane < kWarps ? volatile_u32(&sync->taken[lane]) * kWarps + lane : 0xFFFFFFFFu);
 }
+// The tensor maps, before this CTA's first use: they lie in memory that another recording may have had for its own, and are cached
+// by their addresses. (Fenced by the requesting warp itself, an op's at a time, a dense 8B token took 25 us more, by all threads at
+// the start 7.)
+__device__ void acquire_maps(const Program& p, Sync* sync, int lane) {
+    for (uint32_t i = 0; i < p.n_maps; i += 32) {
+        if (i + lane < p.n_maps) {
+            const uint8_t* map = p.maps + (i + lane) * 128u;
+            asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+        }
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence_block();
+            store_volatile(&sync->maps_ready, i + 32);
+        }
+    }
+}
 // Requests the units of the CTA's tiles, in order, into a ring: one tensor copy each, a lane per unit, as many at a time as
 // there is room for. (Five warps with 16-byte copies, 9 or 14 a lane and unit, took so many issue slots that a dense 8B token
 // was 1650 us; nine, beside eight that compute, 1190; this one 1030 before the other roles' changes.)
@@ -189,8 +207,9 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
         const uint32_t tile0 = first_of(p, op.first), pitch = (op.K >> 8) * 210u, end0 = op.tile_end[0], end1 = op.tile_end[1];
         const bool two = op.streams == 2;
         const uint8_t* maps = p.maps + op.map * 128u;
-        if (j + 1 < p.n_ops && lane < 3)  // the next op's descriptors (at least three follow)
-            asm volatile("prefetch.tensormap [%0];" ::"l"(p.maps + (p.ops[j + 1].map + lane) * 128u) : "memory");
+        const uint32_t map_end = j + 1 < p.n_ops ? p.ops[j + 1].map : p.n_maps;
+        poll(p, sync, 189, 60, [&] { return volatile_u32(&sync->maps_ready) >= map_end; });
+        __syncwarp();
         for (uint32_t i = 0; i < n;) {
             uint32_t k = 0;
             for (uint32_t polls = 0;; ++polls) {
@@ -479,7 +498,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) program_kernel_fn(const __gr
     __syncthreads();
     if (tid == 0) {
         mbar_init(&sync->table, 1);
-        sync->ready = sync->gave_up = 0;
+        sync->ready = sync->maps_ready = sync->gave_up = 0;
         mbar_fence_init();
     }
     __syncthreads();
@@ -487,7 +506,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) program_kernel_fn(const __gr
     else if (warp == kWarps) fetch_weights(p, sync, smem_u32(base), lane);
     else if (warp == kWarps + 1) convert_x(p, sync, lane);
     else if (warp == kWarps + 2) fetch_x(p, sync, smem_u32(tables), lane);
-    else write_rows(p, sync, parts, warp - kWarps - 3, lane);
+    else {
+        if (warp == kWarps + 2 + kWriters) acquire_maps(p, sync, lane);  // its first rows are two calls away
+        write_rows(p, sync, parts, warp - kWarps - 3, lane);
+    }
     __syncthreads();
     if (tid == 0) {  // the last CTA to leave clears the counters for the next launch
         __threadfence();
@@ -692,14 +714,13 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
         p.n_ops = j + 1;
     }
     p.table_bytes = x_table * 16;
-    p.n_maps = maps + 3;  // some are prefetched past the last
+    p.n_maps = maps;
     return p.n_ops >= 2 ? p.n_ops : 0;
 }
 
 bool program_maps(const Program& p, CUtensorMap* maps) {
     EncodeFn encode = encode_fn();
     if (!encode) return false;
-    memset(maps, 0, p.n_maps * sizeof(CUtensorMap));
     for (uint32_t j = 0; j < p.n_ops; ++j) {
         const ProgramOp& op = p.ops[j];
         const int n = op.streams == 2 ? 2 : matrices(op);
