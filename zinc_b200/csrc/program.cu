@@ -143,11 +143,24 @@ __device__ __forceinline__ bool wait_bar(const Program& p, Sync* s, uint64_t* ba
     }
     return true;
 }
-// polls `ok` (the same in all lanes that take part) until it holds
+// polls `ok` until it holds, each lane for itself: no warp-wide operations in it
 template <typename Ok>
 __device__ __forceinline__ void poll(const Program& p, Sync* s, uint32_t site, uint32_t sleep, Ok ok) {
     for (uint32_t n = 0; !ok(); ++n) {
         if (volatile_u32(&s->gave_up)) break;
+        if (n > p.spin_limit) {
+            gave_up(p, s, site);
+            break;
+        }
+        if (sleep) __nanosleep(sleep);
+    }
+}
+// The same for a whole warp, whose lanes leave together: those that saw the flag or ran out alone would leave the others in a
+// warp-wide operation that never completes.
+template <typename Ok>
+__device__ __forceinline__ void poll_warp(const Program& p, Sync* s, uint32_t site, uint32_t sleep, Ok ok) {
+    for (uint32_t n = 0; !__all_sync(0xFFFFFFFFu, ok()); ++n) {
+        if (__any_sync(0xFFFFFFFFu, volatile_u32(&s->gave_up))) break;
         if (n > p.spin_limit) {
             gave_up(p, s, site);
             break;
@@ -208,8 +221,7 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
         const bool two = op.streams == 2;
         const uint8_t* maps = p.maps + op.map * 128u;
         const uint32_t map_end = j + 1 < p.n_ops ? p.ops[j + 1].map : p.n_maps;
-        poll(p, sync, 189, 60, [&] { return volatile_u32(&sync->maps_ready) >= map_end; });
-        __syncwarp();
+        poll_warp(p, sync, 189, 60, [&] { return volatile_u32(&sync->maps_ready) >= map_end; });
         for (uint32_t i = 0; i < n;) {
             uint32_t k = 0;
             for (uint32_t polls = 0;; ++polls) {
@@ -229,7 +241,7 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
                     off = o;
                     break;
                 }
-                if (polls > p.spin_limit || volatile_u32(&sync->gave_up)) {
+                if (polls > p.spin_limit || __any_sync(0xFFFFFFFFu, volatile_u32(&sync->gave_up))) {
                     gave_up(p, sync, 195);
                     return;
                 }
@@ -267,7 +279,7 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
         }
         seq0 += nt;
     }
-    poll(p, sync, 195, 50, [&] { return head + kWarps - units_taken(sync, lane) <= kUnits; });  // the barriers have been seen
+    poll_warp(p, sync, 195, 50, [&] { return head + kWarps - units_taken(sync, lane) <= kUnits; });  // the barriers have been seen
     if (lane < kWarps && !volatile_u32(&sync->gave_up)) {  // no more units
         const uint32_t e = (head + lane) & (kUnits - 1);
         sync->unit[e] = make_uint4(0u, kNoOp, 0u, 0u);
@@ -304,7 +316,7 @@ __device__ void fetch_x(const Program& p, Sync* sync, uint32_t tables, int lane)
         const ProgramOp& op = p.ops[j];
         if (tiles_here(p, j)) {
             const uint32_t need = op.wait_warps, nb = op.K >> 8;
-            poll(p, sync, 190, 300, [&] { return __all_sync(0xFFFFFFFFu, lane >= kWarps || volatile_u32(&sync->at[lane]) >= need); });
+            poll_warp(p, sync, 190, 300, [&] { return lane >= kWarps || volatile_u32(&sync->at[lane]) >= need; });
             if (lane == 0) {
                 poll(p, sync, 196, 0, [&] { return ld_acquire_u32(p.converted + j) >= nb; });
                 asm volatile("fence.proxy.async;" ::: "memory");
@@ -359,7 +371,7 @@ __device__ void write_rows(const Program& p, Sync* sync, const float* parts, uin
             float* y = op.y[m] + r;
             const uint32_t s = seq & (kParts - 1);
             // The parity tells a round from the one before only, and the tile before in this place may be another row writer's.
-            poll(p, sync, 198, 60, [&] { return volatile_u32(&sync->added[s]) == seq / kParts; });
+            poll_warp(p, sync, 198, 60, [&] { return volatile_u32(&sync->added[s]) == seq / kParts; });
             wait_bar(p, sync, &sync->parts[s], (seq / kParts) & 1, 199);
             __syncwarp();
             if (q == 0) {  // parts are there: what x waits for is complete
@@ -415,7 +427,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
                 xb = tab + (g < 6 ? g : g - 2) * 64u + t * 16u;
                 xstep = g < 6 ? 96u : 0u;   // dead columns: zeros
             }
-            poll(p, sync, 192, 60, [&] { return volatile_u32(&sync->ready) > cur; });
+            poll_warp(p, sync, 192, 60, [&] { return volatile_u32(&sync->ready) > cur; });
             __threadfence_block();
             __syncwarp();
         }
@@ -462,7 +474,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
         v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2);
         v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
         const uint32_t seq = d.w;
-        poll(p, sync, 194, 100, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; });  // the place for its parts is free
+        poll_warp(p, sync, 194, 100, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; });  // the place for its parts is free
         __syncwarp();
         if (t == 0) {
             float* q = parts + (seq & (kParts - 1)) * (kPartBytes / 4) + (d.y >> 16) * 16 + (kind == PROG_Q4K ? q4k_row(g) : g);
