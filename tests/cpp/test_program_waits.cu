@@ -1,0 +1,168 @@
+// The joined matvec kernel when a wait runs out: it reports, leaves by itself and clears its counters; the next launch is sound.
+// The kernel is compiled in, so that its limit can be set and a count that calls wait for be left out; the calls themselves, the
+// yardstick, come from the library.
+#include <cstdio>
+#include <cstdlib>
+#include <vector>
+
+#include "../../zinc_b200/csrc/program.cu"
+
+namespace zc {
+cudaError_t launch_dmmv(uint32_t type, int mode, const DmmvArgs& a, cudaStream_t s, uint64_t* launches);
+}
+
+using namespace zc;
+
+#define CHECK(e)                                                                                      \
+    do {                                                                                              \
+        const cudaError_t err_ = (e);                                                                 \
+        if (err_ != cudaSuccess) {                                                                    \
+            printf("line %d: %s\n", __LINE__, cudaGetErrorString(err_));                              \
+            exit(1);                                                                                  \
+        }                                                                                             \
+    } while (0)
+#define EXPECT(c, ...)                                \
+    do {                                              \
+        if (!(c)) {                                   \
+            printf("line %d: ", __LINE__);            \
+            printf(__VA_ARGS__);                      \
+            printf("\n");                             \
+            exit(1);                                  \
+        }                                             \
+    } while (0)
+
+__global__ void fill_q4k(uint8_t* w, uint64_t n, uint32_t seed) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t h = (uint32_t)i * 2654435761u + seed;
+        h = (h ^ (h >> 15)) * 0x85EBCA6Bu;
+        const uint32_t at = i % 144;
+        w[i] = at == 1 || at == 3 ? 0x14 + (h >> 30) : (uint8_t)(h >> 16);  // d, dmin: 1e-3 .. 8e-3
+    }
+}
+
+int main() {
+    constexpr uint32_t kSmall = 1024, kRows = 8192;
+    uint8_t* W[3];
+    const uint32_t K[3] = {kSmall, kRows, kSmall};
+    for (int i = 0; i < 3; ++i) {
+        const uint64_t n = (uint64_t)kRows * (K[i] / 256) * 144;
+        CHECK(cudaMalloc(&W[i], n));
+        fill_q4k<<<512, 256>>>(W[i], n, 77u * i);
+    }
+    std::vector<float> x(kSmall);
+    for (uint32_t i = 0; i < kSmall; ++i) x[i] = (float)((i * 37u) % 101u) / 50.f - 1.f;
+    float *dx, *y, *want;  // y: four outputs
+    uint32_t* status;
+    CHECK(cudaMalloc(&dx, kSmall * 4));
+    CHECK(cudaMalloc(&y, 4 * kRows * 4));
+    CHECK(cudaMalloc(&want, 4 * kRows * 4));
+    CHECK(cudaMalloc(&status, 8));
+    CHECK(cudaMemcpy(dx, x.data(), kSmall * 4, cudaMemcpyHostToDevice));
+
+    cudaDeviceProp prop;
+    CHECK(cudaGetDeviceProperties(&prop, 0));
+    const int sms = prop.multiProcessorCount;
+    ProgramOp ops[4];
+    auto call = [&](int i, float* out) {  // 1 reads what 0 writes, 3 what 1 writes; 2 adds to its own rows
+        DmmvArgs a;
+        const int m = i == 3 ? 1 : i;
+        a.A = W[m];
+        a.x = i == 1 ? out : i == 3 ? out + kRows : dx;
+        a.y = out + (uint64_t)i * kRows;
+        a.M = kRows;
+        a.K = K[m];
+        a.acc_mode = i == 2;
+        a.a_end = W[m] + (uint64_t)kRows * (K[m] / 256) * 144;
+        a.status = status;
+        a.sm_count = sms;
+        return a;
+    };
+    CHECK(cudaMemset(want, 0, 4 * kRows * 4));
+    for (int i = 0; i < 4; ++i) {
+        EXPECT(program_op(T_Q4_K, MODE_PLAIN, call(i, y), ops[i]), "call %d is not one of a program", i);
+        CHECK(launch_dmmv(T_Q4_K, MODE_PLAIN, call(i, want), nullptr, nullptr));
+    }
+    CHECK(cudaDeviceSynchronize());
+
+    std::vector<Program> storage(1);
+    Program& p = storage[0];
+    EXPECT(program_plan(ops, 4, sms, p) == 4, "not one program");
+    std::vector<CUtensorMap> maps(p.n_maps);
+    EXPECT(program_maps(p, maps.data()), "tensor maps");
+    constexpr uint32_t kGuard = 4096, kWords = 32;
+    const uint64_t map_bytes = p.n_maps * sizeof(CUtensorMap), total = map_bytes + kGuard + kWords * 4 + p.table_bytes + kGuard;
+    uint8_t* mem;
+    CHECK(cudaMalloc(&mem, total));
+    CHECK(cudaMemset(mem, 0xA5, total));
+    CHECK(cudaMemcpy(mem, maps.data(), map_bytes, cudaMemcpyHostToDevice));
+    uint8_t* counters = mem + map_bytes + kGuard;
+    CHECK(cudaMemset(counters, 0, kWords * 4));
+    p.maps = mem;
+    p.done = reinterpret_cast<uint32_t*>(counters);
+    p.converted = p.done + 4;
+    p.left = p.converted + 4;
+    p.tables = counters + kWords * 4;
+    p.status = status;
+    void* func = nullptr;
+    uint32_t threads = 0, smem = 0;
+    CHECK(program_kernel(sms, &func, threads, smem));
+
+    std::vector<float> first(4 * kRows), now(4 * kRows), ref(4 * kRows);
+    CHECK(cudaMemcpy(ref.data(), want, 4 * kRows * 4, cudaMemcpyDeviceToHost));
+    uint32_t st[2];
+    std::vector<uint8_t> back(total);
+    auto launch = [&](uint32_t limit, int uncounted) {
+        std::vector<Program> copy(1, p);
+        copy[0].spin_limit = limit;
+        if (uncounted >= 0) copy[0].ops[uncounted].awaited = 0;
+        CHECK(cudaMemset(status, 0, 8));
+        CHECK(cudaMemset(y, 0, 4 * kRows * 4));
+        void* args[] = {&copy[0]};
+        CHECK(cudaLaunchCooperativeKernel(func, dim3(p.grid), dim3(threads), args, smem, nullptr));
+        CHECK(cudaDeviceSynchronize());
+        CHECK(cudaMemcpy(st, status, 8, cudaMemcpyDeviceToHost));
+        CHECK(cudaMemcpy(now.data(), y, 4 * kRows * 4, cudaMemcpyDeviceToHost));
+        CHECK(cudaMemcpy(back.data(), mem, total, cudaMemcpyDeviceToHost));
+        for (uint32_t i = 0; i < kWords * 4; ++i) EXPECT(back[map_bytes + kGuard + i] == 0, "counter byte %u after a launch", i);
+        for (uint32_t i = 0; i < kGuard; ++i) EXPECT(back[map_bytes + i] == 0xA5 && back[total - kGuard + i] == 0xA5, "guard byte %u", i);
+    };
+    auto sound = [&](const char* when) {
+        launch(1u << 24, -1);
+        EXPECT(st[0] == 0, "%s: wait %u gave up", when, st[1]);
+        EXPECT(now == first, "%s: not the same bits", when);
+    };
+    launch(1u << 24, -1);
+    EXPECT(st[0] == 0, "wait %u gave up", st[1]);
+    first = now;
+    for (int i = 0; i < 4; ++i) {
+        double diff = 0, sum = 0;
+        for (uint32_t r = i * kRows; r < (i + 1) * kRows; ++r) {
+            diff += ((double)now[r] - ref[r]) * ((double)now[r] - ref[r]);
+            sum += (double)ref[r] * ref[r];
+        }
+        // f32 sums in another order; x of calls 1 and 3 rounded to 21 bits after that
+        EXPECT(sum > 0 && diff <= 4e-6 * 4e-6 * sum, "output %d: %g of %g", i, diff, sum);
+    }
+    int sites[256] = {};
+    for (int round = 0; round < 40; ++round) {
+        // nothing may wait twice: copies have just been requested; then longer, so that other waits run out first
+        for (uint32_t limit : {0u, 1u, 3u, 10u}) {
+            launch(limit, -1);
+            EXPECT(st[0] == 1 || limit > 3, "limit %u: nothing gave up", limit);
+            if (st[0]) ++sites[st[1] & 255];
+            sound("after a short limit");
+        }
+        // calls 1 and 3 wait for a call that is never counted
+        for (int uncounted : {0, 1}) {
+            launch(1000, uncounted);
+            EXPECT(st[0] == 1, "call %d was not counted: nothing gave up", uncounted);
+            ++sites[st[1] & 255];
+            sound("after a call that was not counted");
+        }
+    }
+    printf("ok");
+    for (int i = 0; i < 256; ++i)
+        if (sites[i]) printf(" %d:%d", i, sites[i]);
+    printf("\n");
+    return 0;
+}

@@ -4,6 +4,9 @@ The bars: x is 21-bit fixed point per 256 elements, up to 8 x 2^-20 a step for N
 whose largest is below 4); the recorded form has the same digits of x, so that the two differ by f32 sums; a chain of
 six calls passes its differences on and gate * up adds two: 2e-5.
 """
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
@@ -274,3 +277,17 @@ def test_q6k_matvec_forms(gpu, oracle, M, K):
     for lo in (0, M // 2 // 16 * 16, M - 64):
         want = oracle.dmmv_f64(raw[lo * row:(lo + 64) * row], zb.Q6_K, 64, K, x.cpu().numpy())
         assert rel_l2(y[lo:lo + 64].cpu().numpy(), want) <= 2.3e-6
+
+
+def test_waits_that_run_out(gpu):
+    """tests/cpp/test_program_waits.cu: the kernel with limits that run out, with copies under way; each time a sound launch next."""
+    from zinc_b200 import _lib, build
+
+    here = os.path.dirname(os.path.abspath(__file__))
+    src, exe = (os.path.join(here, "cpp", f) for f in ("test_program_waits.cu", "_build/test_program_waits"))
+    os.makedirs(os.path.dirname(exe), exist_ok=True)
+    lib = os.path.dirname(_lib.SO_PATH)
+    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
+                    "-lzinc_b200", "-Xlinker", "-rpath=" + lib], check=True, capture_output=True, text=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr

@@ -45,6 +45,7 @@ struct Sync {
     uint32_t added[kParts];                  // tiles that have been added up from that place
     uint32_t maps_ready;                     // tensor maps that can be used
     uint32_t ready;                          // ops whose x table is there
+    uint32_t issued;                         // units requested, when the requesting warp is done
     uint32_t gave_up;
 };
 constexpr uint32_t kTables = (kSmem - 128 - kRing - kZeros - kParts * kPartBytes - (uint32_t)sizeof(Sync)) & ~127u;
@@ -124,8 +125,8 @@ __device__ __forceinline__ void q4k_block(uint32_t rA, uint32_t rB, uint32_t xb,
 }
 
 // ---- waits ------------------------------------------------------------------------------------------------
-// Every wait is bounded: one that gives up reports, and all later waits of the CTA are passed by; the results are then wrong
-// and the status says so.
+// Every wait is bounded: one that gives up reports, the compute warps stop, and all other waits of the CTA are passed by; the
+// results are then wrong and the status says so.
 __device__ __forceinline__ uint32_t volatile_u32(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }
 __device__ __forceinline__ void store_volatile(uint32_t* p, uint32_t v) { *reinterpret_cast<volatile uint32_t*>(p) = v; }
 __device__ __forceinline__ void gave_up(const Program& p, Sync* s, uint32_t site) {
@@ -158,15 +159,16 @@ __device__ __forceinline__ void poll(const Program& p, Sync* s, uint32_t site, u
 // The same for a whole warp, whose lanes leave together: those that saw the flag or ran out alone would leave the others in a
 // warp-wide operation that never completes.
 template <typename Ok>
-__device__ __forceinline__ void poll_warp(const Program& p, Sync* s, uint32_t site, uint32_t sleep, Ok ok) {
+__device__ __forceinline__ bool poll_warp(const Program& p, Sync* s, uint32_t site, uint32_t sleep, Ok ok) {
     for (uint32_t n = 0; !__all_sync(0xFFFFFFFFu, ok()); ++n) {
-        if (__any_sync(0xFFFFFFFFu, volatile_u32(&s->gave_up))) break;
+        if (__any_sync(0xFFFFFFFFu, volatile_u32(&s->gave_up))) return false;
         if (n > p.spin_limit) {
             gave_up(p, s, site);
-            break;
+            return false;
         }
         if (sleep) __nanosleep(sleep);
     }
+    return true;
 }
 // until `n` ops are complete on all SMs
 __device__ __forceinline__ void await_ops(const Program& p, Sync* sync, uint32_t first, uint32_t n, int lane) {
@@ -221,7 +223,10 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
         const bool two = op.streams == 2;
         const uint8_t* maps = p.maps + op.map * 128u;
         const uint32_t map_end = j + 1 < p.n_ops ? p.ops[j + 1].map : p.n_maps;
-        poll_warp(p, sync, 189, 60, [&] { return volatile_u32(&sync->maps_ready) >= map_end; });
+        if (!poll_warp(p, sync, 189, 60, [&] { return volatile_u32(&sync->maps_ready) >= map_end; })) {
+            if (lane == 0) sync->issued = head;
+            return;
+        }
         for (uint32_t i = 0; i < n;) {
             uint32_t k = 0;
             for (uint32_t polls = 0;; ++polls) {
@@ -243,6 +248,7 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
                 }
                 if (polls > p.spin_limit || __any_sync(0xFFFFFFFFu, volatile_u32(&sync->gave_up))) {
                     gave_up(p, sync, 195);
+                    if (lane == 0) sync->issued = head;
                     return;
                 }
                 if (polls) __nanosleep(250);
@@ -279,12 +285,21 @@ __device__ void fetch_weights(const Program& p, Sync* sync, uint32_t ring, int l
         }
         seq0 += nt;
     }
+    if (lane == 0) sync->issued = head;
     poll_warp(p, sync, 195, 50, [&] { return head + kWarps - units_taken(sync, lane) <= kUnits; });  // the barriers have been seen
     if (lane < kWarps && !volatile_u32(&sync->gave_up)) {  // no more units
         const uint32_t e = (head + lane) & (kUnits - 1);
         sync->unit[e] = make_uint4(0u, kNoOp, 0u, 0u);
         mbar_arrive(&sync->full[e]);
     }
+}
+
+// After a wait has given up: the units that were requested and that nobody has waited for. Their copies end before the CTA does,
+// whose shared memory another one may have next.
+__device__ void await_copies(Sync* sync, int lane) {
+    const uint32_t head = sync->issued;
+    for (uint32_t u = units_taken(sync, lane) + lane; u < head; u += 32)
+        for (uint32_t n = 0; n < kWaitLimit && !mbar_try_wait(&sync->full[u & (kUnits - 1)], (u / kUnits) & 1);) ++n;
 }
 
 // Converts this CTA's share of the calls' x, a block of 256 at a time, as soon as what they wait for is complete.
@@ -405,10 +420,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
     uint32_t cur = 0xFFFFFFFFu, kind = 0, tab = 0, bpr = 0, xb = 0, xstep = 0;
     for (uint32_t u = warp, n = 1;; u += kWarps, ++n) {
         const uint32_t e = u & (kUnits - 1);
-        if (!__all_sync(0xFFFFFFFFu, wait_bar(p, sync, &sync->full[e], (u / kUnits) & 1, 193))) {
-            if (lane == 0) store_volatile(&sync->at[warp], p.n_ops);
-            break;
-        }
+        if (!__all_sync(0xFFFFFFFFu, wait_bar(p, sync, &sync->full[e], (u / kUnits) & 1, 193))) break;
         const uint4 d = sync->unit[e];
         const uint32_t op_i = d.y & 0xFFFFu;
         if (op_i != cur) {
@@ -427,7 +439,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
                 xb = tab + (g < 6 ? g : g - 2) * 64u + t * 16u;
                 xstep = g < 6 ? 96u : 0u;   // dead columns: zeros
             }
-            poll_warp(p, sync, 192, 60, [&] { return volatile_u32(&sync->ready) > cur; });
+            if (!poll_warp(p, sync, 192, 60, [&] { return volatile_u32(&sync->ready) > cur; })) break;
             __threadfence_block();
             __syncwarp();
         }
@@ -474,8 +486,8 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
         v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2);
         v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
         const uint32_t seq = d.w;
-        poll_warp(p, sync, 194, 100, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; });  // the place for its parts is free
-        __syncwarp();
+        // the place for its parts is free (else no arrival there: it would be one too many)
+        if (!poll_warp(p, sync, 194, 100, [&] { return volatile_u32(&sync->added[seq & (kParts - 1)]) == seq / kParts; })) break;
         if (t == 0) {
             float* q = parts + (seq & (kParts - 1)) * (kPartBytes / 4) + (d.y >> 16) * 16 + (kind == PROG_Q4K ? q4k_row(g) : g);
             q[0] = v0;
@@ -510,7 +522,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) program_kernel_fn(const __gr
     __syncthreads();
     if (tid == 0) {
         mbar_init(&sync->table, 1);
-        sync->ready = sync->maps_ready = sync->gave_up = 0;
+        sync->ready = sync->maps_ready = sync->issued = sync->gave_up = 0;
         mbar_fence_init();
     }
     __syncthreads();
@@ -523,6 +535,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) program_kernel_fn(const __gr
         write_rows(p, sync, parts, warp - kWarps - 3, lane);
     }
     __syncthreads();
+    if (volatile_u32(&sync->gave_up)) {
+        if (warp == kWarps) await_copies(sync, lane);
+        __syncthreads();
+    }
     if (tid == 0) {  // the last CTA to leave clears the counters for the next launch
         __threadfence();
         if (atomicAdd(p.left, 1u) == p.grid - 1) {
