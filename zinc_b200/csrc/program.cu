@@ -195,15 +195,12 @@ __device__ __forceinline__ uint32_t units_taken(const Sync* sync, int lane) {
     return __reduce_min_sync(0xFFFFFFFFu, lane < kWarps ? volatile_u32(&sync->taken[lane]) * kWarps + lane : 0xFFFFFFFFu);
 }
 // The tensor maps, before this CTA's first use: they lie in memory that another recording may have had for its own, and are cached
-// by their addresses. (Fenced by the requesting warp itself, an op's at a time, a dense 8B token took 25 us more, by all threads at
-// the start 7.)
+// by their addresses. (Dense 8B token: 950 us without, 953 so; with each map prefetched behind its fence 959, four at a time 1011;
+// fenced by the requesting warp, an op's at a time, 25 us more, by all threads at the start 7.)
 __device__ void acquire_maps(const Program& p, Sync* sync, int lane) {
     for (uint32_t i = 0; i < p.n_maps; i += 32) {
-        if (i + lane < p.n_maps) {
-            const uint8_t* map = p.maps + (i + lane) * 128u;
-            asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-        }
+        if (lane < 32 && i + lane < p.n_maps)
+            asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(p.maps + (i + lane) * 128u) : "memory");
         __syncwarp();
         if (lane == 0) {
             __threadfence_block();
