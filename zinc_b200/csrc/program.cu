@@ -199,7 +199,7 @@ __device__ __forceinline__ uint32_t units_taken(const Sync* sync, int lane) {
 // fenced by the requesting warp, an op's at a time, 25 us more, by all threads at the start 7.)
 __device__ void acquire_maps(const Program& p, Sync* sync, int lane) {
     for (uint32_t i = 0; i < p.n_maps; i += 32) {
-        if (lane < 32 && i + lane < p.n_maps)
+        if (i + lane < p.n_maps)
             asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(p.maps + (i + lane) * 128u) : "memory");
         __syncwarp();
         if (lane == 0) {
