@@ -226,6 +226,42 @@ def test_calls_that_are_not_joined(gpu):
     r.ctx.free_recording(rec)
 
 
+def test_calls_into_another_capture_are_its_own(gpu):
+    """Between zc_begin_record and zc_end_record the caller goes to another stream, which a graph of the caller's captures."""
+    torch, _, _ = gpu
+    r = Run(torch, 12)
+    M, K = 4096, 1024
+    w1, w2, x = r.mat(zb.Q4_K, M, K), r.mat(zb.Q4_K, M, K), r.vec(K)
+    outs = [r.out(M) for _ in range(4)]
+    ref = [r.out(M) for _ in range(2)]
+    torch.cuda.synchronize()
+    for w, y in zip((w1, w2), ref):
+        r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
+    r.ctx.submit_and_wait()
+    other, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    n0 = r.ctx.launch_count
+    with torch.cuda.graph(graph, stream=other, capture_error_mode="relaxed"):
+        r.ctx.set_stream(r.stream.cuda_stream)
+        r.ctx.begin_record()
+        r.ctx.set_stream(other.cuda_stream)
+        for w, y in zip((w1, w2), outs[2:]):
+            r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
+        r.ctx.set_stream(r.stream.cuda_stream)
+        for w, y in zip((w1, w2), outs):
+            r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
+    rec = r.ctx.end_record()
+    assert r.ctx.launch_count - n0 == 3   # the graph's two, and two joined
+    r.ctx.replay(rec)
+    r.ctx.submit_and_wait()
+    assert not any(bool(o[:M].any()) for o in outs[2:])
+    graph.replay()
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert torch.equal(outs[2 + i][:M], ref[i][:M])
+        assert rel_l2(outs[i][:M].cpu().numpy(), ref[i][:M].cpu().numpy()) <= 1.5e-6
+    r.ctx.free_recording(rec)
+
+
 def test_a_long_run_is_several_kernels(gpu):
     """More calls than one kernel's parameters hold; each adds to the vector that the one before has written."""
     torch, _, _ = gpu

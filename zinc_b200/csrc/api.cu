@@ -61,6 +61,7 @@ struct zc_ctx {
         zc::ProgramOp op;
     };
     bool recording = false;
+    unsigned long long record_id = 0;  // of the capture that zc_begin_record began: calls may go to another one in between
     std::vector<Recorded> recorded;
     uint64_t joined = 0;           // recorded launches that became part of another one
     char err[512] = {0};
@@ -191,12 +192,13 @@ cudaError_t run_mul_mm_exact(zc_ctx* ctx, const ExactGemm& p) {
 // A call that was just recorded as one kernel, described by `op`: remembered with its graph node.
 void note_op(zc_ctx* ctx, const ProgramOp& op) {
     cudaStreamCaptureStatus st;
+    unsigned long long id = 0;
     cudaGraph_t graph = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     const cudaGraphEdgeData* edges = nullptr;
     size_t n = 0;
-    if (cudaStreamGetCaptureInfo_v3(ctx->stream, &st, nullptr, &graph, &deps, &edges, &n) != cudaSuccess ||
-        st != cudaStreamCaptureStatusActive || n != 1)
+    if (cudaStreamGetCaptureInfo_v3(ctx->stream, &st, &id, &graph, &deps, &edges, &n) != cudaSuccess ||
+        st != cudaStreamCaptureStatusActive || id != ctx->record_id || n != 1)
         return;
     cudaGraphNodeType type;
     if (cudaGraphNodeGetType(deps[0], &type) != cudaSuccess || type != cudaGraphNodeTypeKernel) return;
@@ -668,7 +670,9 @@ int32_t zc_begin_record(zc_ctx* ctx) {
     ZC_ENTER(ctx);
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "zc_begin_record");
-    ctx->recording = true;
+    cudaStreamCaptureStatus st;
+    ctx->recording = cudaStreamGetCaptureInfo_v3(ctx->stream, &st, &ctx->record_id, nullptr, nullptr, nullptr, nullptr) == cudaSuccess &&
+                     st == cudaStreamCaptureStatusActive;  // else the calls stay launches
     ctx->recorded.clear();
     return ZC_OK;
 }
