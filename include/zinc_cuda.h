@@ -119,15 +119,16 @@ int32_t zc_memset(zc_ctx* ctx, void* dst, uint64_t dst_offset, int32_t byte_valu
 int32_t zc_barrier(zc_ctx* ctx);
 int32_t zc_submit_and_wait(zc_ctx* ctx);
 /* Device-side errors are deferred to zc_submit_and_wait, as the reference's are to submitAndWait:
- *  - a bounded wait inside a kernel gave up (a split-K hand-off or a peer's flag): ZC_ERR_TIMEOUT. The
- *    results of the calls since the last zc_submit_and_wait are invalid; the context stays usable (its
- *    hand-off flags are cleared), a communicator whose exchange gave up refuses further collectives
- *    until zc_comm_destroy + zc_comm_init on every rank;
+ *  - a bounded wait inside a kernel gave up (a split-K hand-off, a peer's flag, a call joined with
+ *    others): ZC_ERR_TIMEOUT. The results of the calls since the last zc_submit_and_wait are invalid;
+ *    the context stays usable (its hand-off flags are cleared), a communicator whose exchange gave up
+ *    refuses further collectives until zc_comm_destroy + zc_comm_init on every rank;
  *  - a routing buffer named an expert the weight buffer does not hold: ZC_ERR_INVALID_ARG (the id is
  *    replaced by expert 0 or the pair is skipped, so no kernel reads outside the buffer).
  * zc_set_wait_limit sets the number of polls after which such a wait gives up (0 = the defaults,
- * 2^26 for split-K hand-offs and 2^24 for peer flags, i.e. seconds). No counterpart in the reference
- * (Vulkan reports a lost device instead). */
+ * 2^26 for split-K hand-offs and 2^24 for peer flags, i.e. seconds). The waits inside joined calls of a
+ * recording (below) have a limit of their own, 2^24 polls, and report the same way. No counterpart in
+ * the reference (Vulkan reports a lost device instead). */
 int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
 
 /* ---- pre-recorded op sequences ----------------------------------------------

@@ -226,6 +226,21 @@ def test_calls_that_are_not_joined(gpu):
     r.ctx.free_recording(rec)
 
 
+def test_the_limit_for_peers_and_hand_offs_is_not_theirs(gpu):
+    """A limit of one poll (zc_set_wait_limit), under which joined calls could not wait for one another."""
+    torch, _, _ = gpu
+    r = Run(torch, 13)
+    n = 4096
+    w, x, h, y = r.mat(zb.Q4_K, n, n), r.vec(n), r.out(n), r.out(n)
+    r.ctx.set_wait_limit(1)
+
+    def record():
+        r.dd.recordDispatch(zb.Q4_K, w, x, h, n, n)
+        r.dd.recordDispatch(zb.Q4_K, w, h, y, n, n)
+    eager, got = r.eager_and_recorded(record, [h, y], 1, replays=3)
+    assert rel_l2(got[1][:n].cpu().numpy(), eager[1][:n].cpu().numpy()) <= 4e-6
+
+
 def test_calls_into_another_capture_are_its_own(gpu):
     """Between zc_begin_record and zc_end_record the caller goes to another stream, which a graph of the caller's captures."""
     torch, _, _ = gpu

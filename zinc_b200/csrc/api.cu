@@ -317,7 +317,6 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
         p.left = p.converted + n;
         p.tables = mem + words * 4;
         p.status = ctx->status_dev;
-        p.spin_limit = ctx->wait_limit ? ctx->wait_limit : (1u << 24);
         if ((e = replace_nodes(graph, r.data() + i, n, p, func, threads, smem)) != cudaSuccess) return e;
         ctx->joined += n - 1;
         i += n;

@@ -33,6 +33,9 @@ constexpr uint32_t kParts = 8;               // tiles of a CTA whose parts may b
 constexpr uint32_t kPartBytes = kWarps * 16 * 4;
 constexpr uint32_t kZeros = 256;
 constexpr uint32_t kSmem = 232448;
+// Polls of a wait, with sleeps of 50 to 300 ns in between: a second and more. The caller's limit for peers and hand-offs is none for
+// these waits, most of which are for earlier calls to be complete, as long as that takes.
+constexpr uint32_t kPollLimit = 1u << 24;
 constexpr uint32_t kNoOp = 0xFFFFu;          // op of a description: there are no more units
 struct Sync {
     uint4 unit[kUnits];                      // {address, op | part << 16, block | last << 16 | alignment << 20, tile of the CTA}
@@ -690,6 +693,7 @@ bool program_op_multi(uint32_t type, uint32_t n, const uint8_t* const* A, float*
 
 uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p) {
     p.n_ops = 0;
+    p.spin_limit = kPollLimit;
     p.grid = sm_count > 0 ? (uint32_t)sm_count : 148u;
     uint32_t n_deps = 0, first = 0, x_first = 0, x_table = 0, maps = 0;
     bool before[kProgMaxOps][kProgMaxOps];  // [j][i]: i is complete before j writes

@@ -44,7 +44,7 @@ struct Program {
     uint8_t* tables;          // table_bytes of memory for converted x
     const uint8_t* maps;      // n_maps tensor maps of the weights
     uint32_t table_bytes, n_maps;
-    uint32_t spin_limit;
+    uint32_t spin_limit;      // polls after which a wait gives up; program_plan sets it
     uint32_t* status;
     uint16_t deps[kProgMaxDeps];
     ProgramOp ops[kProgMaxOps];
