@@ -241,6 +241,35 @@ def test_the_limit_for_peers_and_hand_offs_is_not_theirs(gpu):
     assert rel_l2(got[1][:n].cpu().numpy(), eager[1][:n].cpu().numpy()) <= 4e-6
 
 
+def test_a_recording_ends_without_waiting(gpu):
+    """Work under way on the context's own stream, which the calls are recorded from."""
+    torch, _, _ = gpu
+    r = Run(torch, 15)
+    M, K = 4096, 1024
+    w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(2)]
+    ctx = zb.Context(0)
+    dd, own = zb.DmmvDispatch(ctx), torch.cuda.ExternalStream(ctx.stream)
+
+    def record():
+        ctx.begin_record()
+        for y in outs:
+            dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
+        return ctx.end_record()
+    ctx.free_recording(record())   # the kernel is loaded
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(own):
+        torch.cuda._sleep(2_000_000_000)   # a second
+        done.record()
+    rec = record()
+    assert not done.query()
+    ctx.replay(rec)
+    ctx.submit_and_wait()
+    assert bool(outs[1][:M].any()) and torch.equal(outs[0][:M], outs[1][:M])
+    ctx.free_recording(rec)
+    ctx.close()
+
+
 def test_calls_into_another_capture_are_its_own(gpu):
     """Between zc_begin_record and zc_end_record the caller goes to another stream, which a graph of the caller's captures."""
     torch, _, _ = gpu

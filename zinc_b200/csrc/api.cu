@@ -268,6 +268,15 @@ cudaError_t free_recording(zc_recording* rec) {
     return e;
 }
 
+// A stream to fill a recording's memory on, so that nothing the caller has under way is waited for.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaError_t open() { return stream ? cudaSuccess : cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking); }
+    ~SideStream() {
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
+
 // Runs of recorded calls with nothing between them become one kernel each (program.h). What does not fit stays as it was.
 cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     const std::vector<zc_ctx::Recorded>& r = ctx->recorded;
@@ -276,6 +285,7 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     std::vector<ProgramOp> ops(r.size());
     for (size_t i = 0; i < r.size(); ++i) ops[i] = r[i].op;
     cudaError_t e;
+    SideStream side;
     std::vector<Program> prog(1);
     for (size_t i = 0; i + 1 < r.size();) {
         size_t end = i + 1;
@@ -309,9 +319,10 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
         rec->memory.push_back(mem);
         p.maps = mem;
         mem += map_bytes;
-        if ((e = cudaMemcpyAsync(const_cast<uint8_t*>(p.maps), maps.data(), map_bytes, cudaMemcpyHostToDevice, ctx->own_stream)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(mem, 0, words * 4, ctx->own_stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamSynchronize(ctx->own_stream)) != cudaSuccess) return e;
+        if ((e = side.open()) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(const_cast<uint8_t*>(p.maps), maps.data(), map_bytes, cudaMemcpyHostToDevice, side.stream)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(mem, 0, words * 4, side.stream)) != cudaSuccess) return e;
+        if ((e = cudaStreamSynchronize(side.stream)) != cudaSuccess) return e;
         p.done = reinterpret_cast<uint32_t*>(mem);
         p.converted = p.done + n;
         p.left = p.converted + n;
