@@ -88,7 +88,7 @@ int main() {
     Program& p = storage[0];
     EXPECT(program_plan(ops, 4, sms, p) == 4, "not one program");
     std::vector<CUtensorMap> maps(p.n_maps);
-    EXPECT(program_maps(p, maps.data()), "tensor maps");
+    EXPECT(program_maps(p, maps.data()) == 4, "tensor maps");
     constexpr uint32_t kGuard = 4096, kWords = 32;
     const uint64_t map_bytes = p.n_maps * sizeof(CUtensorMap), total = map_bytes + kGuard + kWords * 4 + p.table_bytes + kGuard;
     uint8_t* mem;

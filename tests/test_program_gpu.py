@@ -359,15 +359,25 @@ def test_q6k_matvec_forms(gpu, oracle, M, K):
         assert rel_l2(y[lo:lo + 64].cpu().numpy(), want) <= 2.3e-6
 
 
-def test_waits_that_run_out(gpu):
-    """tests/cpp/test_program_waits.cu: the kernel with limits that run out, with copies under way; each time a sound launch next."""
+def run_cpp(name):
+    """Builds tests/cpp/<name>.cu against the library and runs it."""
     from zinc_b200 import _lib, build
 
     here = os.path.dirname(os.path.abspath(__file__))
-    src, exe = (os.path.join(here, "cpp", f) for f in ("test_program_waits.cu", "_build/test_program_waits"))
+    src, exe = os.path.join(here, "cpp", name + ".cu"), os.path.join(here, "cpp", "_build", name)
     os.makedirs(os.path.dirname(exe), exist_ok=True)
     lib = os.path.dirname(_lib.SO_PATH)
     subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
                     "-lzinc_b200", "-Xlinker", "-rpath=" + lib], check=True, capture_output=True, text=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr
+
+
+def test_waits_that_run_out(gpu):
+    """The kernel with limits that run out, with copies under way; each time a sound launch next."""
+    run_cpp("test_program_waits")
+
+
+def test_joining_that_is_refused(gpu):
+    """A matrix without a tensor map, no memory, a node without its attribute: the calls stay launches."""
+    run_cpp("test_joining")

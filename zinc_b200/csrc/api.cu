@@ -225,8 +225,10 @@ cudaGraphNode_t only_neighbour(cudaGraphNode_t node, bool behind) {
     return o;
 }
 
-// Puts one node in the place of the nodes of a program, which follow one another and nothing else.
-cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t n, Program& p, void* func, uint32_t threads, uint32_t smem) {
+// Puts one node in the place of the nodes of a program, which follow one another and nothing else. `replaced` stays false where
+// the new node is refused: the graph is then as it was.
+cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t n, Program& p, void* func, uint32_t threads, uint32_t smem,
+                          bool& replaced) {
     size_t n_in = 0, n_out = 0;
     cudaError_t e = cudaGraphNodeGetDependencies_v2(r[0].node, nullptr, nullptr, &n_in);
     if (e == cudaSuccess) e = cudaGraphNodeGetDependentNodes_v2(r[n - 1].node, nullptr, nullptr, &n_out);
@@ -254,6 +256,7 @@ cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t
         cudaGraphDestroyNode(node);
         return e;
     }
+    replaced = true;
     for (uint32_t i = 0; i < n; ++i)
         if ((e = cudaGraphDestroyNode(r[i].node)) != cudaSuccess) return e;
     return cudaSuccess;
@@ -299,15 +302,18 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
             return cudaSuccess;
         }
         Program& p = prog[0];
-        const uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p);
+        uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p);
         if (n == 0) {
             ++i;
             continue;
         }
         std::vector<CUtensorMap> maps(p.n_maps);
-        if (!program_maps(p, maps.data())) {
-            i += n;
-            continue;
+        if (const uint32_t described = program_maps(p, maps.data()); described < n) {  // that call stays a launch
+            n = described < 2 ? 0 : program_plan(ops.data() + i, described, ctx->sm_count, p);
+            if (n == 0) {
+                i += described + 1;
+                continue;
+            }
         }
         const size_t map_bytes = p.n_maps * sizeof(CUtensorMap), words = (2 * n + 1 + 31) & ~31u;
         uint8_t* mem = nullptr;
@@ -328,7 +334,12 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
         p.left = p.converted + n;
         p.tables = mem + words * 4;
         p.status = ctx->status_dev;
-        if ((e = replace_nodes(graph, r.data() + i, n, p, func, threads, smem)) != cudaSuccess) return e;
+        bool replaced = false;
+        if ((e = replace_nodes(graph, r.data() + i, n, p, func, threads, smem, replaced)) != cudaSuccess) {
+            if (replaced) return e;
+            cudaGetLastError();
+            return cudaSuccess;
+        }
         ctx->joined += n - 1;
         i += n;
     }

@@ -747,9 +747,9 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
     return p.n_ops >= 2 ? p.n_ops : 0;
 }
 
-bool program_maps(const Program& p, CUtensorMap* maps) {
+uint32_t program_maps(const Program& p, CUtensorMap* maps) {
     EncodeFn encode = encode_fn();
-    if (!encode) return false;
+    if (!encode) return 0;
     for (uint32_t j = 0; j < p.n_ops; ++j) {
         const ProgramOp& op = p.ops[j];
         const int n = op.streams == 2 ? 2 : matrices(op);
@@ -760,10 +760,10 @@ bool program_maps(const Program& p, CUtensorMap* maps) {
             if (encode(maps + op.map + i, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<uint8_t*>(op.A[i]), dims, strides, box, steps,
                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-                return false;
+                return j;
         }
     }
-    return true;
+    return p.n_ops;
 }
 
 cudaError_t program_kernel(int sm_count, void** func, uint32_t& threads, uint32_t& smem) {

@@ -58,8 +58,8 @@ bool program_op_multi(uint32_t type, uint32_t n, const uint8_t* const* A, float*
                       ProgramOp& op);
 // Orders the first ops of `list` as a program; returns how many it took (at least two, or none).
 uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p);
-// Fills the program's n_maps tensor maps; false: a matrix that cannot be described.
-bool program_maps(const Program& p, CUtensorMap* maps);
+// Fills the program's n_maps tensor maps; returns how many ops it described: fewer than n_ops where a matrix cannot be.
+uint32_t program_maps(const Program& p, CUtensorMap* maps);
 // The kernel for a graph node: its function, block size and shared memory; cudaErrorNotSupported where it does not fit the device.
 cudaError_t program_kernel(int sm_count, void** func, uint32_t& threads, uint32_t& smem);
 
