@@ -1,4 +1,7 @@
 """Shared helpers of the GPU parity tests."""
+import os
+import subprocess
+
 import numpy as np
 
 CANARY = 0xA5
@@ -33,6 +36,20 @@ def out_with_canary(torch, n_floats: int, back: int = 16, init: float = 0.0):
 
 def canary_intact(t, n_floats: int) -> bool:
     return bool(t[n_floats:].isnan().all().item())
+
+
+def run_cpp(name):
+    """Builds tests/cpp/<name>.cu against the library and runs it."""
+    from zinc_b200 import _lib, build
+
+    here = os.path.dirname(os.path.abspath(__file__))
+    src, exe = os.path.join(here, "cpp", name + ".cu"), os.path.join(here, "cpp", "_build", name)
+    os.makedirs(os.path.dirname(exe), exist_ok=True)
+    lib = os.path.dirname(_lib.SO_PATH)
+    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
+                    "-lzinc_b200", "-Xlinker", "-rpath=" + lib], check=True, capture_output=True, text=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr
 
 
 def oracle_moe_decode_layer(o, x, router, wg, wu, wd, shape, ffn, router_bias=None, bg=None, bu=None, bd=None,

@@ -4,13 +4,10 @@ The bars: x is 21-bit fixed point per 256 elements, up to 8 x 2^-20 a step for N
 whose largest is below 4); the recorded form has the same digits of x, so that the two differ by f32 sums; a chain of
 six calls passes its differences on and gate * up adds two: 2e-5.
 """
-import os
-import subprocess
-
 import numpy as np
 import pytest
 
-from helpers import canary_intact, dev, out_with_canary, rel_l2
+from helpers import canary_intact, dev, out_with_canary, rel_l2, run_cpp
 
 import zinc_b200 as zb
 from zinc_b200 import synth
@@ -176,6 +173,82 @@ def test_joined_calls_are_ordered_by_what_they_read_and_write(gpu):
         assert canary_intact(o, n), name
         assert bool(torch.isfinite(e[:n]).all()), name
         assert rel_l2(o[:n].cpu().numpy(), e[:n].cpu().numpy()) <= 2e-5, name
+
+
+def test_calls_whose_ranges_overlap(gpu):
+    """Outputs that meet a part of another call's x or output: windows of one buffer, 64 floats apart."""
+    torch, _, _ = gpu
+    r = Run(torch, 16)
+    n, K = 4608, 1024
+    ws = [r.mat(zb.Q4_K, n - 64 * i, K) for i in range(4)] + [r.mat(zb.Q6_K, 4096, K)]
+    x, buf, y = r.vec(K), r.out(2 * n), r.out(4096)
+    buf[:2 * n] = r.vec(2 * n)
+
+    def mv(t, w, M, x, x_at, y, y_at, acc=0):
+        r.dd.recordDispatch(t, w, x, y, M, K, x_offset=4 * x_at, y_offset=4 * y_at, acc_mode=acc)
+
+    def record():
+        mv(zb.Q4_K, ws[0], n, x, 0, buf, 1088)                 # the end of the next one's x
+        mv(zb.Q4_K, ws[1], n - 64, buf, 128, buf, 2 * n - 4544, 1)   # adds to most of the first one's rows
+        mv(zb.Q4_K, ws[2], n - 128, x, 0, buf, 64)             # replaces that x, behind it, and more of the first one's rows
+        mv(zb.Q6_K, ws[4], 4096, buf, 2 * n - K, y, 0)         # the end of the second one's rows
+        mv(zb.Q4_K, ws[3], n - 192, x, 0, buf, 2 * n - 4416, 1)  # adds behind the read
+    eager, got = r.eager_and_recorded(record, [buf, y], 1, replays=10)
+    for e, o, m in zip(eager, got, (2 * n, 4096)):
+        assert canary_intact(o, m)
+        assert bool(torch.isfinite(e[:m]).all())
+        assert rel_l2(o[:m].cpu().numpy(), e[:m].cpu().numpy()) <= 6e-6
+
+
+def test_a_long_chain_of_calls(gpu):
+    """Each call reads what the one before wrote, three buffers in turn, and every third is also read two calls later."""
+    torch, _, _ = gpu
+    r = Run(torch, 17)
+    n = 2048
+    ws, v, z = [r.mat(zb.Q6_K, n, n) for _ in range(3)], [r.out(n) for _ in range(3)], r.out(n)
+    v[0][:n] = r.vec(n)
+
+    def record():
+        for i in range(9):
+            r.dd.recordDispatch(zb.Q6_K, ws[i % 3], v[i % 3], v[(i + 1) % 3], n, n)
+            if i % 3 == 2:
+                r.dd.recordDispatch(zb.Q6_K, ws[1], v[1], z, n, n, acc_mode=1)
+    outs = v + [z]
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=10)
+    for e, o in zip(eager, got):
+        assert canary_intact(o, n)
+        assert bool(torch.isfinite(e[:n]).all())
+        # nine calls that each round x and add in another order
+        assert rel_l2(o[:n].cpu().numpy(), e[:n].cpu().numpy()) <= 2e-5
+
+
+def test_two_recordings_on_two_streams(gpu):
+    """Kernels that each want all SMs, launched on two streams without a wait in between."""
+    torch, _, _ = gpu
+    runs = [Run(torch, 18), Run(torch, 19)]
+    M, K, jobs = 20480, 1024, []
+    for r in runs:
+        w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(3)]
+        torch.cuda.synchronize()
+
+        def record(r=r, w=w, x=x, outs=outs):
+            for y in outs:
+                r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K, acc_mode=1)
+        record()
+        r.ctx.submit_and_wait()
+        r.ctx.begin_record()
+        record()
+        jobs.append((r, outs, outs[0].clone(), r.ctx.end_record()))
+    torch.cuda.synchronize()
+    for _ in range(100):
+        for r, _, _, rec in jobs:
+            r.ctx.replay(rec)
+    for r, outs, one, rec in jobs:
+        r.ctx.submit_and_wait()
+        for y in outs:   # 101 additions of equal terms
+            assert canary_intact(y, M)
+            assert rel_l2(y[:M].cpu().numpy(), 101 * one[:M].double().cpu().numpy()) <= 101 * 2.0 ** -24 + 2e-6
+        r.ctx.free_recording(rec)
 
 
 def test_calls_that_are_not_joined(gpu):
@@ -357,20 +430,6 @@ def test_q6k_matvec_forms(gpu, oracle, M, K):
     for lo in (0, M // 2 // 16 * 16, M - 64):
         want = oracle.dmmv_f64(raw[lo * row:(lo + 64) * row], zb.Q6_K, 64, K, x.cpu().numpy())
         assert rel_l2(y[lo:lo + 64].cpu().numpy(), want) <= 2.3e-6
-
-
-def run_cpp(name):
-    """Builds tests/cpp/<name>.cu against the library and runs it."""
-    from zinc_b200 import _lib, build
-
-    here = os.path.dirname(os.path.abspath(__file__))
-    src, exe = os.path.join(here, "cpp", name + ".cu"), os.path.join(here, "cpp", "_build", name)
-    os.makedirs(os.path.dirname(exe), exist_ok=True)
-    lib = os.path.dirname(_lib.SO_PATH)
-    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
-                    "-lzinc_b200", "-Xlinker", "-rpath=" + lib], check=True, capture_output=True, text=True)
-    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
-    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr
 
 
 def test_waits_that_run_out(gpu):

@@ -2,6 +2,8 @@
 import numpy as np
 import pytest
 
+from helpers import run_cpp
+
 
 def reciprocal(d, limit):
     return 2 ** 32 // d + 1 if d > 1 and limit * d < 2 ** 32 else 0
@@ -18,3 +20,8 @@ def test_quotient_is_exact(d):
         n = np.unique(np.concatenate([np.arange(0, limit, step), np.arange(0, limit, d)[:100000], np.arange(d - 1, limit, d)[-100000:],
                                       [limit - 1]])).astype(np.uint64)
         assert np.array_equal((n * np.uint64(mul)) >> np.uint64(32), n // np.uint64(d))
+
+
+def test_the_kernels_own():
+    """reciprocal, quotient and the limits in slice_plan, compiled for the host from the kernels' header."""
+    run_cpp("test_reciprocal")
