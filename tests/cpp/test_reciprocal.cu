@@ -38,7 +38,7 @@ struct Fmt {  // what slice_plan asks of a format
 template <typename F>
 static int plans() {
     int n = 0;
-    for (uint32_t M : {1u, 3u, 16u, 100u, 512u, 2048u, 2880u, 7001u, 16384u, 1200000u})
+    for (uint32_t M : {1u, 3u, 16u, 100u, 512u, 2048u, 2880u, 7001u, 16384u, 400000u})
         for (uint32_t K : {512u, 768u, 1024u, 2048u, 2880u, 4096u})
             for (uint32_t slots : {1u, 2u, 3u, 5u, 8u, 9u, 33u})
                 for (int seg : {2, 3}) {
