@@ -138,15 +138,23 @@ int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
  * captured instead of executed; zc_replay enqueues the whole sequence with one
  * launch. Buffers, sizes and offsets are baked in at record time. Host copies
  * recorded this way must use page-locked host memory.
- * zc_end_record joins runs of zc_dmmv, zc_dmmv_multi, zc_dmmv_fused_gate_up_swiglu
- * and zc_dmmv_sigmoid_acc calls on Q4_K and Q6_K matrices of 2 MB and more, with
- * nothing else between them on the stream, into one kernel each. Results are those
- * of the calls in their order; sums are taken in another order than in the calls
- * themselves, the same one at every replay. Such a kernel uses all SMs, reads
+ * zc_end_record joins runs of zc_dmmv, zc_dmmv_fused_gate_up_swiglu and
+ * zc_dmmv_sigmoid_acc calls on Q4_K and Q6_K matrices of 2 MB and more and of
+ * zc_dmmv_multi calls on Q4_K matrices, with nothing else between them on the
+ * stream, into one kernel each where that is expected to be faster: from two to
+ * five calls on that do not read what the one before wrote (calls that do stay
+ * launches: each such wait costs a joined kernel more than a launch does).
+ * Results are those of the calls in their order; sums are taken in another order
+ * than in the calls themselves, the same one at every replay. Such a kernel reads
  * weights of later calls ahead of earlier calls' results (calls that write another
- * one's weights are not joined) and counts as one launch. A recording owns the
- * device memory this takes (3.5 MB for a dense 8B token) until zc_free_recording,
- * which waits for a replay that is under way. */
+ * one's weights are not joined) and counts as one launch. It runs on all SMs at
+ * once: it starts when each has room for it, behind a kernel of another stream
+ * that keeps an SM to itself. Where that kernel waits for the replay in turn,
+ * capture the calls yourself (cudaStreamBeginCapture): they are launches then.
+ * A recording owns the device memory this takes (3.5 MB for a dense 8B token)
+ * until zc_free_recording, which waits for the work under way on the device.
+ * CUDA refuses zc_end_record and zc_free_recording beside a stream capture in the
+ * global mode, and that capture fails. */
 int32_t zc_begin_record(zc_ctx* ctx);
 int32_t zc_end_record(zc_ctx* ctx, void** out_recording);
 int32_t zc_replay(zc_ctx* ctx, void* recording);

@@ -37,13 +37,13 @@ static bool armed = false;  // between zc_begin_record and the end of zc_end_rec
     } while (0)
 
 int main() {
-    constexpr uint32_t M = 4096, K = 1024, N = 5;
-    constexpr uint64_t kBytes = (uint64_t)M * (K / 256) * 144;
+    constexpr uint32_t M = 12288, K = 4096, N = 5;  // two of these are worth being joined
+    constexpr uint64_t kBytes = (uint64_t)M * (K / 256) * 210;
     zc_ctx* ctx = nullptr;
     EXPECT(zc_init(0, &ctx) == ZC_OK, "no context");
     std::vector<uint8_t> w(kBytes);
     std::vector<float> x(K), out(M);
-    for (uint64_t i = 0; i < kBytes; ++i) w[i] = i % 144 == 1 || i % 144 == 3 ? 0x18 : (uint8_t)(i * 2654435761u >> 20);
+    for (uint64_t i = 0; i < kBytes; ++i) w[i] = i % 210 == 209 ? 0x18 : (uint8_t)(i * 2654435761u >> 20);
     for (uint32_t i = 0; i < K; ++i) x[i] = (float)(i * 37 % 101) / 50.f - 1.f;
     void *W[N], *dx, *y;
     OK(zc_alloc(ctx, K * 4, &dx));
@@ -58,7 +58,7 @@ int main() {
     }
     auto calls = [&](uint32_t first, uint32_t n) {
         for (uint32_t i = first; i < first + n; ++i)
-            OK(zc_dmmv(ctx, zc::T_Q4_K, W[i], kBytes, dx, K * 4, y, (uint64_t)N * M * 4, M, K, 0, 0, (uint64_t)i * M * 4, 0));
+            OK(zc_dmmv(ctx, zc::T_Q6_K, W[i], kBytes, dx, K * 4, y, (uint64_t)N * M * 4, M, K, 0, 0, (uint64_t)i * M * 4, 0));
     };
     auto all_of = [&] {
         std::vector<float> v(N * M);

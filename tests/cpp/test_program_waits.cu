@@ -86,7 +86,7 @@ int main() {
 
     std::vector<Program> storage(1);
     Program& p = storage[0];
-    EXPECT(program_plan(ops, 4, sms, p) == 4, "not one program");
+    EXPECT(program_plan(ops, 4, sms, p, nullptr) == 4, "not one program");
     std::vector<CUtensorMap> maps(p.n_maps);
     EXPECT(program_maps(p, maps.data()) == 4, "tensor maps");
     constexpr uint32_t kGuard = 4096, kWords = 32;

@@ -46,8 +46,9 @@ def run_cpp(name):
     src, exe = os.path.join(here, "cpp", name + ".cu"), os.path.join(here, "cpp", "_build", name)
     os.makedirs(os.path.dirname(exe), exist_ok=True)
     lib = os.path.dirname(_lib.SO_PATH)
-    subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
-                    "-lzinc_b200", "-Xlinker", "-rpath=" + lib], check=True, capture_output=True, text=True)
+    r = subprocess.run([build._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", src, "-o", exe, "-L", lib,
+                        "-lzinc_b200", "-Xlinker", "-rpath=" + lib], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr
 

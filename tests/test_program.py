@@ -1,0 +1,6 @@
+"""Which recorded calls zc_end_record joins: the decision, on the host."""
+from helpers import run_cpp
+
+
+def test_what_is_worth_being_joined():
+    run_cpp("test_program_worth")

@@ -26,6 +26,19 @@ class Run:
         self.dd = zb.DmmvDispatch(self.ctx)
         self.g = np.random.default_rng(seed)
         self.raw = {}
+        self.beside = None
+
+    def pad(self, n):
+        """Calls beside those of a test, each worth some 2.5 us of joining: with enough of them, a run is joined that would be better
+        off as launches."""
+        M, K = 1024, 4096
+        if self.beside is None or len(self.beside[2]) < n:
+            w = synth.torch_quant_matrix(zb.Q6_K, M, K, self.torch.device("cuda"), 3)
+            self.beside = w, self.vec(K), [self.out(M) for _ in range(n)]
+            self.torch.cuda.synchronize()
+        w, x, outs = self.beside
+        for y in outs[:n]:
+            self.dd.recordDispatch(zb.Q6_K, w, x, y, M, K)
 
     def mat(self, t, M, K):
         raw = synth.quant_matrix(self.g, t, M, K)
@@ -39,8 +52,10 @@ class Run:
     def out(self, n):
         return out_with_canary(self.torch, n)
 
-    def eager_and_recorded(self, record, outs, launches, replays=1):
-        """Outputs of the calls and of a replay of the recorded ones, from the same start; every canary must hold."""
+    def eager_and_recorded(self, record, outs, launches, replays=1, pads=0):
+        """Outputs of the calls and of a replay of the recorded ones, from the same start; every canary must hold. `pads`: calls in front
+        of the recorded ones and behind them."""
+        self.pad(pads)
         start = [o.clone() for o in outs]
         self.torch.cuda.synchronize()
         record()
@@ -49,7 +64,9 @@ class Run:
         n0 = self.ctx.launch_count
         with self.torch.cuda.stream(self.stream):
             self.ctx.begin_record()
+            self.pad(pads)
             record()
+            self.pad(pads)
             rec = self.ctx.end_record()
         assert self.ctx.launch_count - n0 == launches
         got = None
@@ -83,7 +100,7 @@ def test_joined_matvecs_by_shape(gpu, oracle, t, M, K):
         r.dd.recordDispatch(t, w1, x1, a, M, K)
         r.dd.recordDispatch(t, w2, x2, b, M, K, acc_mode=1)
     fits = K <= 12288   # beyond, the f32 kernels
-    eager, got = r.eager_and_recorded(record, [a, b], 1 if fits else 2, replays=3)
+    eager, got = r.eager_and_recorded(record, [a, b], 1 if fits else 4, replays=3, pads=24)
     for y, e, w, x, add in ((got[0], eager[0], w1, x1, 0.0), (got[1], eager[1], w2, x2, 0.5)):
         assert canary_intact(y, M)
         want = oracle.dmmv_f64(r.raw[w.data_ptr()], t, M, K, x.cpu().numpy()) + add
@@ -111,7 +128,7 @@ def test_many_tiles_per_sm(gpu, t, shapes):
             r.dd.recordDispatch(t, w[M, K], xs[K], y, M, K)
         M, K = shapes[0]
         r.dd.recordDispatch(t, w[M, K], xs[K], outs[0], M, K, acc_mode=1)
-    eager, got = r.eager_and_recorded(record, outs, 1, replays=20)
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=20, pads=24)
     for (M, _), e, o in zip(shapes, eager, got):
         assert canary_intact(o, M)
         assert rel_l2(o[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6
@@ -136,9 +153,11 @@ def test_layers_of_dense_models(gpu, H, q_dim, kv, F, launches):
         dd.recordDispatchMulti(zb.Q4_K, [wq, wk, wv], h, [q, k, v], [q_dim, kv, kv], H)
         dd.recordDispatch(zb.Q4_K, wo, q, h, H, q_dim, acc_mode=1)
         dd.dispatchDmmvFusedGateUpSwiglu(zb.Q4_K, wg, wu, h, act, F, H)
+        if launches > 1:
+            r.pad(24)
         dd.recordDispatch(zb.Q6_K, wd, act, h, H, F, acc_mode=1)
         dd.recordDispatchMulti(zb.Q4_K, [wq, wk, wv], h, [q, k, v], [q_dim, kv, kv], H)
-    eager, got = r.eager_and_recorded(record, outs, launches, replays=20)
+    eager, got = r.eager_and_recorded(record, outs, launches, replays=20, pads=24)
     for name, e, o, n in zip("q k v h act".split(), eager, got, sizes):
         assert canary_intact(o, n), name
         assert bool(torch.isfinite(e[:n]).all()), name
@@ -168,7 +187,7 @@ def test_joined_calls_are_ordered_by_what_they_read_and_write(gpu):
     outs = [x, q, k, v, act, h, z]
     for o, n in zip(outs, (H, H, 300, 17, F, H, 1301)):
         assert canary_intact(o, n)
-    eager, got = r.eager_and_recorded(record, outs, 1, replays=4)
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=4, pads=24)
     for name, e, o, n in zip("x q k v act h z".split(), eager, got, (H, H, 300, 17, F, H, 1301)):
         assert canary_intact(o, n), name
         assert bool(torch.isfinite(e[:n]).all()), name
@@ -193,7 +212,7 @@ def test_calls_whose_ranges_overlap(gpu):
         mv(zb.Q4_K, ws[2], n - 128, x, 0, buf, 64)             # replaces that x, behind it, and more of the first one's rows
         mv(zb.Q6_K, ws[4], 4096, buf, 2 * n - K, y, 0)         # the end of the second one's rows
         mv(zb.Q4_K, ws[3], n - 192, x, 0, buf, 2 * n - 4416, 1)  # adds behind the read
-    eager, got = r.eager_and_recorded(record, [buf, y], 1, replays=10)
+    eager, got = r.eager_and_recorded(record, [buf, y], 1, replays=10, pads=24)
     for e, o, m in zip(eager, got, (2 * n, 4096)):
         assert canary_intact(o, m)
         assert bool(torch.isfinite(e[:m]).all())
@@ -214,7 +233,7 @@ def test_a_long_chain_of_calls(gpu):
             if i % 3 == 2:
                 r.dd.recordDispatch(zb.Q6_K, ws[1], v[1], z, n, n, acc_mode=1)
     outs = v + [z]
-    eager, got = r.eager_and_recorded(record, outs, 1, replays=10)
+    eager, got = r.eager_and_recorded(record, outs, 1, replays=10, pads=32)
     for e, o in zip(eager, got):
         assert canary_intact(o, n)
         assert bool(torch.isfinite(e[:n]).all())
@@ -228,17 +247,20 @@ def test_two_recordings_on_two_streams(gpu):
     runs = [Run(torch, 18), Run(torch, 19)]
     M, K, jobs = 20480, 1024, []
     for r in runs:
-        w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(3)]
+        w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(8)]
         torch.cuda.synchronize()
 
         def record(r=r, w=w, x=x, outs=outs):
             for y in outs:
                 r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K, acc_mode=1)
+            r.pad(24)
         record()
         r.ctx.submit_and_wait()
+        n0 = r.ctx.launch_count
         r.ctx.begin_record()
         record()
         jobs.append((r, outs, outs[0].clone(), r.ctx.end_record()))
+        assert r.ctx.launch_count - n0 == 1
     torch.cuda.synchronize()
     for _ in range(100):
         for r, _, _, rec in jobs:
@@ -272,7 +294,7 @@ def test_calls_that_are_not_joined(gpu):
         r.dd.recordDispatch(zb.Q4_K, small, x, c, 64, K)
         r.dd.recordDispatch(zb.Q4_K, w1, x, a, M, K)
         r.dd.recordDispatch(zb.Q4_K, w2, x, b, M, K)
-    eager, got = r.eager_and_recorded(three, [a, b, c], 2)
+    eager, got = r.eager_and_recorded(three, [a, b, c], 3, pads=24)   # what is in front, the small one, the rest
     assert torch.equal(eager[2][:64], got[2][:64])
     assert rel_l2(got[1][:M].cpu().numpy(), eager[1][:M].cpu().numpy()) <= 1.5e-6
 
@@ -286,6 +308,7 @@ def test_calls_that_are_not_joined(gpu):
     n0 = r.ctx.launch_count
     r.ctx.begin_record()
     overwrites()
+    r.pad(24)
     rec = r.ctx.end_record()
     assert r.ctx.launch_count - n0 == 2
     r.ctx.replay(rec)
@@ -310,7 +333,7 @@ def test_the_limit_for_peers_and_hand_offs_is_not_theirs(gpu):
     def record():
         r.dd.recordDispatch(zb.Q4_K, w, x, h, n, n)
         r.dd.recordDispatch(zb.Q4_K, w, h, y, n, n)
-    eager, got = r.eager_and_recorded(record, [h, y], 1, replays=3)
+    eager, got = r.eager_and_recorded(record, [h, y], 1, replays=3, pads=24)
     assert rel_l2(got[1][:n].cpu().numpy(), eager[1][:n].cpu().numpy()) <= 4e-6
 
 
@@ -319,7 +342,7 @@ def test_a_recording_ends_without_waiting(gpu):
     torch, _, _ = gpu
     r = Run(torch, 15)
     M, K = 4096, 1024
-    w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(2)]
+    w, x, outs = r.mat(zb.Q4_K, M, K), r.vec(K), [r.out(M) for _ in range(12)]
     ctx = zb.Context(0)
     dd, own = zb.DmmvDispatch(ctx), torch.cuda.ExternalStream(ctx.stream)
 
@@ -352,6 +375,7 @@ def test_calls_into_another_capture_are_its_own(gpu):
     outs = [r.out(M) for _ in range(4)]
     ref = [r.out(M) for _ in range(2)]
     torch.cuda.synchronize()
+    r.pad(24)
     for w, y in zip((w1, w2), ref):
         r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
     r.ctx.submit_and_wait()
@@ -366,8 +390,9 @@ def test_calls_into_another_capture_are_its_own(gpu):
         r.ctx.set_stream(r.stream.cuda_stream)
         for w, y in zip((w1, w2), outs):
             r.dd.recordDispatch(zb.Q4_K, w, x, y, M, K)
+        r.pad(24)
     rec = r.ctx.end_record()
-    assert r.ctx.launch_count - n0 == 3   # the graph's two, and two joined
+    assert r.ctx.launch_count - n0 == 3   # the graph's two, and the joined ones
     r.ctx.replay(rec)
     r.ctx.submit_and_wait()
     assert not any(bool(o[:M].any()) for o in outs[2:])
@@ -383,14 +408,14 @@ def test_a_long_run_is_several_kernels(gpu):
     """More calls than one kernel's parameters hold; each adds to the vector that the one before has written."""
     torch, _, _ = gpu
     r = Run(torch, 7)
-    M, K, n = 4096, 1024, 450
+    M, K, n = 1024, 4096, 450
     w, x, h, one = r.mat(zb.Q4_K, M, K), r.vec(K), r.out(M), r.out(M)
 
     def record():
         for _ in range(n):
             r.dd.recordDispatch(zb.Q4_K, w, x, h, M, K, acc_mode=1)
     r.dd.recordDispatch(zb.Q4_K, w, x, one, M, K)
-    _, got = r.eager_and_recorded(record, [h], 3, replays=2)
+    _, got = r.eager_and_recorded(record, [h], 3, replays=2, pads=24)
     # n additions of equal terms: at most n roundings of 2^-24, half of that on average
     assert rel_l2(got[0][:M].cpu().numpy(), n * one[:M].double().cpu().numpy()) <= n * 2.0 ** -24 + 2e-6
 
@@ -410,7 +435,7 @@ def test_a_recording_in_the_memory_of_an_earlier_one(gpu, shapes):
         def record():
             for w, y in zip(ws, outs):
                 r.dd.recordDispatch(t, w, x, y, M, K)
-        eager, got = r.eager_and_recorded(record, outs, 1)
+        eager, got = r.eager_and_recorded(record, outs, 1, pads=24)
         for e, o in zip(eager, got):
             assert rel_l2(o[:M].cpu().numpy(), e[:M].cpu().numpy()) <= 1.5e-6, i
 
@@ -435,6 +460,27 @@ def test_q6k_matvec_forms(gpu, oracle, M, K):
 def test_waits_that_run_out(gpu):
     """The kernel with limits that run out, with copies under way; each time a sound launch next."""
     run_cpp("test_program_waits")
+
+
+def test_runs_that_are_faster_as_launches(gpu):
+    """Calls that read one another's results, and runs of a few small ones, stay what they are; calls beside one another are joined."""
+    torch, _, _ = gpu
+    r = Run(torch, 20)
+    n = 2048
+    w, bufs = r.mat(zb.Q4_K, n, n), [r.out(n) for _ in range(9)]
+    bufs[0][:n] = 1e-3
+
+    def chain():
+        for a, b in zip(bufs, bufs[1:]):
+            r.dd.recordDispatch(zb.Q4_K, w, a, b, n, n)
+
+    def beside(k):
+        for b in bufs[1:1 + k]:
+            r.dd.recordDispatch(zb.Q4_K, w, bufs[0], b, n, n)
+    eager, got = r.eager_and_recorded(chain, bufs, 8)
+    assert all(torch.equal(e[:n], o[:n]) for e, o in zip(eager, got))
+    r.eager_and_recorded(lambda: beside(2), bufs, 2)
+    r.eager_and_recorded(lambda: beside(8), bufs, 1)
 
 
 def test_joining_that_is_refused(gpu):

@@ -280,7 +280,8 @@ struct SideStream {
     }
 };
 
-// Runs of recorded calls with nothing between them become one kernel each (program.h). What does not fit stays as it was.
+// Runs of recorded calls with nothing between them become one kernel each (program.h), where that is the faster form. What does not
+// fit stays as it was.
 cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     const std::vector<zc_ctx::Recorded>& r = ctx->recorded;
     void* func = nullptr;
@@ -289,10 +290,10 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     for (size_t i = 0; i < r.size(); ++i) ops[i] = r[i].op;
     cudaError_t e;
     SideStream side;
-    std::vector<Program> prog(1);
+    std::vector<Program> prog(2);
     for (size_t i = 0; i + 1 < r.size();) {
         size_t end = i + 1;
-        while (end < r.size() && only_neighbour(r[end - 1].node, true) == r[end].node && only_neighbour(r[end].node, false) == r[end - 1].node) ++end;
+        while (end < r.size() && end - i < kProgMaxOps && only_neighbour(r[end - 1].node, true) == r[end].node && only_neighbour(r[end].node, false) == r[end - 1].node) ++end;
         if (end - i < 2) {
             i = end;
             continue;
@@ -302,14 +303,17 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
             return cudaSuccess;
         }
         Program& p = prog[0];
-        uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p);
+        float gain = 0.f, without = 0.f;
+        uint32_t n = program_plan(ops.data() + i, (uint32_t)(end - i), ctx->sm_count, p, &gain);
+        // a first call that the second one waits for may be better left a launch
+        if (n && p.ops[1].deps_x && program_plan(ops.data() + i + 1, (uint32_t)(end - i - 1), ctx->sm_count, prog[1], &without) && without > gain) n = 0;
         if (n == 0) {
             ++i;
             continue;
         }
         std::vector<CUtensorMap> maps(p.n_maps);
         if (const uint32_t described = program_maps(p, maps.data()); described < n) {  // that call stays a launch
-            n = described < 2 ? 0 : program_plan(ops.data() + i, described, ctx->sm_count, p);
+            n = described < 2 ? 0 : program_plan(ops.data() + i, described, ctx->sm_count, p, &gain);
             if (n == 0) {
                 i += described + 1;
                 continue;

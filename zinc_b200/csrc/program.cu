@@ -644,6 +644,53 @@ void place_table(Tables& t, uint32_t j, uint32_t bytes, uint32_t next) {
     t.hi[j] = best_at + bytes;
 }
 
+// What joining gains or costs: estimates in us, fitted to 382 runs of 2 to 8 calls of 2.4 to 510 MB with another kernel between the
+// runs, joined and as launches. None of the runs that pay by them was slower joined; of those that do not, 27 would have been 5 to 24 %
+// faster, nearly all of 2 to 4 calls. Measured, joined and as launches:
+//   start and end of a joined kernel cost more than those of launches: two calls of Q4_K 4096 x 1024 10.2 and 8.1, four 12.9 and 14.3,
+//     eight 18.4 and 26.6; two of Q6_K 12288 x 4096 26.2 and 29.2
+//   three warps of an SM write rows: eight calls of Q4_K 65536 x 512, 28 tiles on an SM each, 111.2 and 52.3, of 65536 x 2048 129.0 and 119.6
+//   a call that reads what the call before wrote waits for all SMs, has that converted and fetched: eight of Q4_K 4096 x 4096 in a
+//     chain 72.7 and 41.1, eight beside one another 24.2 and 41.0; an 8B token whose calls read one another's results 1894 and 1527,
+//     one whose calls only add to one vector 900 and 1557
+//   one that adds to what the call before wrote waits with its rows only: eight of Q4_K 4096 x 1024 35.2 and 26.7, of 1024 x 4096 29.4
+//     and 35.3, of Q6_K 4096 x 4096 47.3 and 55.6; with a call between the two Q4_K 4096 x 4096 31.3 and 41.0
+constexpr float kStartUs = 6.7f, kStartTileUs = 0.21f, kReadUs = 6.7f, kAddUs = 1.8f, kAddTileUs = 1.2f, kFullUs = 2.6f;
+constexpr float kSafety = 0.97f;      // of the launches' time
+constexpr float kHopelessUs = 100.f;  // so far behind its best part a run is looked at no further
+float mega_bytes(const ProgramOp& op) {
+    const float pitch = (float)(op.K >> 8) * (op.kind == PROG_Q4K ? 144.f : 210.f);
+    return ((float)op.M[0] * op.streams + (float)op.M[1] + (float)op.M[2]) * pitch * 1e-6f;
+}
+float launch_us(const ProgramOp& op) {
+    const float mb = mega_bytes(op), start = 2.7f + 0.21f * (float)op.K / 1024.f;
+    return op.kind == PROG_Q4K ? start + std::min(mb, 28.f) / 6.5f + std::max(0.f, mb - 28.f) / 6.1f
+                               : start + std::min(mb, 40.f) / 4.4f + std::max(0.f, mb - 40.f) / 5.3f;
+}
+
+// Adds ops to a program's estimate one by one.
+struct Worth {
+    float end[kProgMaxOps];  // when an op's rows are written
+    float t = 0.f, launches = 0.f;
+    void add(const Program& p, uint32_t j) {
+        const ProgramOp& op = p.ops[j];
+        const uint32_t sm_tiles = (op.tiles + p.grid - 1) / p.grid;
+        const float tiles = (float)sm_tiles, stream = std::max(0.63f + mega_bytes(op) / 6.0f, 0.4f * tiles);
+        if (j == 0) t = kStartUs + kStartTileUs * tiles;
+        t += stream;
+        for (uint32_t d = 0; d < op.deps_x; ++d) t = std::max(t, end[p.deps[op.dep0 + d]] + kReadUs + stream);
+        for (uint32_t d = op.deps_x; d < (uint32_t)op.deps_x + op.deps_y; ++d) {
+            const uint32_t i = p.deps[op.dep0 + d];
+            // the tiles on hold and the next ones have no places left
+            if (i + 1 == j && sm_tiles + (p.ops[i].tiles + p.grid - 1) / p.grid > kParts) t += kFullUs;
+            t = std::max(t, end[i] + kAddUs + kAddTileUs * tiles);
+        }
+        end[j] = t;
+        launches += launch_us(op);
+    }
+    float gain() const { return kSafety * launches - t; }
+};
+
 }  // namespace
 
 bool program_op(uint32_t type, int mode, const DmmvArgs& a, ProgramOp& op) {
@@ -691,13 +738,16 @@ bool program_op_multi(uint32_t type, uint32_t n, const uint8_t* const* A, float*
     return true;
 }
 
-uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p) {
+uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p, float* gain) {
     p.n_ops = 0;
     p.spin_limit = kPollLimit;
     p.grid = sm_count > 0 ? (uint32_t)sm_count : 148u;
     uint32_t n_deps = 0, first = 0, x_first = 0, x_table = 0, maps = 0;
     bool before[kProgMaxOps][kProgMaxOps];  // [j][i]: i is complete before j writes
     Tables place;
+    Worth worth;
+    float most = 0.f;
+    uint32_t best = 0, best_maps = 0, best_table = 0;
     for (uint32_t j = 0; j < n && j < kProgMaxOps; ++j) {
         ProgramOp op = list[j];
         bool clash = false;
@@ -741,6 +791,21 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
         op.table = (uint16_t)(place.lo[j] / 16);
         p.ops[j] = op;
         p.n_ops = j + 1;
+        if (!gain) continue;
+        worth.add(p, j);
+        if (j > 0 && worth.gain() > most) {
+            most = worth.gain();
+            best = j + 1;
+            best_maps = maps;
+            best_table = x_table;
+        }
+        if (worth.gain() < most - kHopelessUs) break;
+    }
+    if (gain) {
+        *gain = most;
+        p.n_ops = best;
+        maps = best_maps;
+        x_table = best_table;
     }
     p.table_bytes = x_table * 16;
     p.n_maps = maps;

@@ -56,8 +56,9 @@ static_assert(sizeof(Program) <= 32764, "kernel parameters");
 bool program_op(uint32_t type, int mode, const DmmvArgs& a, ProgramOp& op);
 bool program_op_multi(uint32_t type, uint32_t n, const uint8_t* const* A, float* const* y, const uint32_t* M, const DmmvArgs& common,
                       ProgramOp& op);
-// Orders the first ops of `list` as a program; returns how many it took (at least two, or none).
-uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p);
+// Orders the first ops of `list` as a program; returns how many it took (at least two, or none). With `gain`: as many as are worth
+// being joined, and what that is to gain in us; else as many as there can be.
+uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& p, float* gain);
 // Fills the program's n_maps tensor maps; returns how many ops it described: fewer than n_ops where a matrix cannot be.
 uint32_t program_maps(const Program& p, CUtensorMap* maps);
 // The kernel for a graph node: its function, block size and shared memory; cudaErrorNotSupported where it does not fit the device.
