@@ -514,8 +514,8 @@ __global__ void __launch_bounds__(kWarps * 32, kWarps == 8 ? 2 : 1) dmmv_slice_m
 
 constexpr uint32_t kSliceSmem1 = 232448u, kSliceSmem2 = 113u * 1024u;  // one, two CTAs per SM
 
-// Units a warp keeps in flight: four at most; two where there are more than `deep` warps. (Q6_K in sixteen warps, three and two:
-// 28672 x 12288 69.6 and 67.2 us, 5120 x 8192 14.0 and 13.3, 40000 x 10240 79.7 and 76.8.)
+// Units a warp keeps in flight: four at most; two where there are more than `deep` warps. (Q6_K in sixteen warps, as many as fit and
+// two: 8192 x 12288 23.2 and 22.6 us, 5120 x 8192 13.4 and 12.9, 28672 x 12288 66.3 and 65.8, 40000 x 10240 71.9 and 71.8.)
 inline uint32_t most_depth(uint32_t depth, uint32_t warps, uint32_t deep) {
     const uint32_t most = warps > deep ? 2u : 4u;
     return depth < most ? depth : most;
@@ -608,14 +608,14 @@ bool slice_plan(SliceArgs& a, int NS, int kSeg, int sm_count, uint32_t& warps, u
 //   Q4_K   K <= 512 always (65536 rows 6.2 and 9.2 us: most warps had no block); K <= 4096 from 8 (K = 4096, 16500 rows 10.4
 //          and 10.2, 20000 rows 11.7 and 12.7, 28672 rows 14.9 and 16.6), beyond from 3 (5120 x 5120 7.5 and 7.7, 14336 x
 //          5120 11.3 and 12.9)
-//   Q6_K   from 2 (5120 x 2816 8.4 and 9.4, 8192 x 4608 13.8 and 17.7, 21669 x 4608 29.6 and 34.2, 128256 x 3072 87.6 and
-//          105.9, 151936 x 4096 99.4 and 109.9; the other way 20000 x 5120 31.1 and 30.1)
+//   Q6_K   K <= 7424 from 2 (5120 x 2816 8.3 and 9.0, 8192 x 4608 13.3 and 13.8, 21669 x 4608 27.3 and 31.4, 65536 x 6144 67.2 and
+//          73.0, 128256 x 3072 85.8 and 101.6, 151936 x 4096 99.1 and 108.6; the other way 20000 x 5120 29.2 and 27.7); K = 8192 (rows
+//          on 16-byte boundaries) from 4.5 (28672 rows 44.2, one CTA 47.7, the form above 45.9; 12000 rows 22.6, 24.5, 22.2; below,
+//          8192 rows 17.0 and 16.2)
 //   MXFP4  K <= 1024 always (20000 x 512 4.1 and 7.8), beyond from 10 (20000 x 2880 14.4 and 13.8, 28672 x 2880 19.3 and 20.4)
-//          K = 8192 (rows on 16-byte boundaries) from 4.5 (12000 rows 23.1 us, one CTA 24.9, the form above 24.2; 28672 rows
-//          43.6, 47.7; below, 8192 rows 18.9 and 16.9)
-// Beyond, Q6_K takes one CTA of sixteen warps from 4.5 tiles per SM (8192 x 12288 25.5 and 25.0 us, 11008 rows 28.7 and 30.1,
-// 28672 rows 62.3 and 70.0; two CTAs of eight, 11008 rows 32.8, 30000 x 12032 90.9 for 78.5, 12000 x 7936 28.9 for 27.5); the
-// others stay above (Q4_K 65536 x 12288 76 and 74).
+// Beyond, Q6_K takes one CTA of sixteen warps from 4.5 tiles per SM (11008 x 12288 27.9 us in both forms, 28672 rows 65.8 and 69.0,
+// 30000 x 12032 75.9 and 84.2; two CTAs of eight 32.4, 64.7, 85.1, 12000 x 7936 28.8 for 27.6, 40000 x 10240 69.3 for 71.8); the others
+// stay above (Q4_K 65536 x 12288 76 and 74).
 template <typename F>
 bool flow_plan(SliceArgs& a, int NS, int sm_count, uint32_t& warps, uint32_t& grid, uint32_t& smem) {
     a.nblk = a.bpe = (a.K + F::kCols - 1) / F::kCols;
