@@ -10,8 +10,9 @@
 // one's waits for that one's tiles to be complete on all SMs; no other call waits for anything.
 // The units (16 rows x 512 columns) of a CTA's tiles are dealt to its compute warps one by one; the parts of a tile meet in
 // shared memory and are added in the order of the units: no barrier between warps, and sums that do not depend on timing.
-// Bound: HBM for some 20 tokens in a row (a dense 8B token, 4.88 GB in 145 calls, 801 us: 6.1 TB/s, 0.93 of the measured copy
-// rate), then the card's power limit (920-935 us at 1.66 GHz); as launches 1573 in both.
+// Bound: HBM for some 20 tokens in a row (a dense 8B token, 4.88 GB in 145 calls, 807 us: 6.05 TB/s, 0.92 of the measured copy
+// rate), then the card's power limit (900-960 us at 1.66 GHz); as launches 1557. That is with calls that do not read one another's
+// results; those that do are better off as launches (What joining gains, below).
 // Arithmetic: that of the streaming matvecs (x as 21-bit fixed point per 256 elements, exact integer dot products per block).
 #include "program.h"
 
