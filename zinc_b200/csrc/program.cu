@@ -743,12 +743,10 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
     p.n_ops = 0;
     p.spin_limit = kPollLimit;
     p.grid = sm_count > 0 ? (uint32_t)sm_count : 148u;
-    uint32_t n_deps = 0, first = 0, x_first = 0, x_table = 0, maps = 0;
+    uint32_t n_deps = 0, best = 0;
     bool before[kProgMaxOps][kProgMaxOps];  // [j][i]: i is complete before j writes
-    Tables place;
     Worth worth;
     float most = 0.f;
-    uint32_t best = 0, best_maps = 0, best_table = 0;
     for (uint32_t j = 0; j < n && j < kProgMaxOps; ++j) {
         ProgramOp op = list[j];
         bool clash = false;
@@ -778,18 +776,6 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
         if (n_deps == kProgMaxDeps) break;
         op.deps_x = (uint16_t)added[0];
         op.deps_y = (uint16_t)added[1];
-        op.map = (uint16_t)maps;
-        maps += op.streams == 2 ? 2 : (uint32_t)matrices(op);
-        op.first = (uint16_t)first;
-        first = (uint32_t)((first + op.tiles) % p.grid);
-        const uint32_t need = round128(table_bytes(op.kind, op.K)), next = j + 1 < n ? round128(table_bytes(list[j + 1].kind, list[j + 1].K)) : 0u;
-        place_table(place, j, need, next);
-        op.x_first = (uint16_t)x_first;
-        x_first = (x_first + (op.K >> 8)) % p.grid;
-        op.x_table = x_table;
-        x_table += need / 16;
-        op.wait_warps = (uint16_t)place.after(j, place.lo[j], need);
-        op.table = (uint16_t)(place.lo[j] / 16);
         p.ops[j] = op;
         p.n_ops = j + 1;
         if (!gain) continue;
@@ -797,16 +783,29 @@ uint32_t program_plan(const ProgramOp* list, uint32_t n, int sm_count, Program& 
         if (j > 0 && worth.gain() > most) {
             most = worth.gain();
             best = j + 1;
-            best_maps = maps;
-            best_table = x_table;
         }
         if (worth.gain() < most - kHopelessUs) break;
     }
     if (gain) {
         *gain = most;
         p.n_ops = best;
-        maps = best_maps;
-        x_table = best_table;
+    }
+    Tables place;
+    uint32_t first = 0, x_first = 0, x_table = 0, maps = 0;
+    for (uint32_t j = 0; j < p.n_ops; ++j) {
+        ProgramOp& op = p.ops[j];
+        op.map = (uint16_t)maps;
+        maps += op.streams == 2 ? 2 : (uint32_t)matrices(op);
+        op.first = (uint16_t)first;
+        first = (uint32_t)((first + op.tiles) % p.grid);
+        const uint32_t need = round128(table_bytes(op.kind, op.K));
+        place_table(place, j, need, j + 1 < p.n_ops ? round128(table_bytes(p.ops[j + 1].kind, p.ops[j + 1].K)) : 0u);
+        op.x_first = (uint16_t)x_first;
+        x_first = (x_first + (op.K >> 8)) % p.grid;
+        op.x_table = x_table;
+        x_table += need / 16;
+        op.wait_warps = (uint16_t)place.after(j, place.lo[j], need);
+        op.table = (uint16_t)(place.lo[j] / 16);
     }
     p.table_bytes = x_table * 16;
     p.n_maps = maps;
