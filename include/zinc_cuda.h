@@ -127,7 +127,7 @@ int32_t zc_submit_and_wait(zc_ctx* ctx);
  *    replaced by expert 0 or the pair is skipped, so no kernel reads outside the buffer).
  * zc_set_wait_limit sets the number of polls after which such a wait gives up (0 = the defaults,
  * 2^26 for split-K hand-offs and 2^24 for peer flags, i.e. seconds). The waits inside joined calls of a
- * recording (below) have a limit of their own, 2^24 polls, and report the same way. No counterpart in
+ * recording (below) have limits of their own, 2^22 polls and more, and report the same way. No counterpart in
  * the reference (Vulkan reports a lost device instead). */
 int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
 
@@ -144,6 +144,12 @@ int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
  * stream, into one kernel each where that is expected to be faster: from two to
  * five calls on that do not read what the one before wrote (calls that do stay
  * launches: each such wait costs a joined kernel more than a launch does).
+ * So are MoE decode layers of three calls in a row each, zc_moe_router_topk
+ * (without norm_weights and routing_local; up to 256 experts), zc_moe_gate_up_act_ex
+ * on its input and zc_moe_down_acc_ex on its output, of one shape and with the
+ * same buffers or ones apart, on Q4_K gate and up and Q6_K down matrices or MXFP4
+ * throughout (rows of whole 16 bytes times eight): any number of them, up to 160
+ * a kernel, whether or not a layer reads what the one before added to.
  * Results are those of the calls in their order; sums are taken in another order
  * than in the calls themselves, the same one at every replay. Such a kernel reads
  * weights of later calls ahead of earlier calls' results (calls that write another

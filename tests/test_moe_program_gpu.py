@@ -1,0 +1,170 @@
+"""Recorded MoE decode layers that zc_end_record joins into one kernel: against the calls themselves.
+
+The bars: the same digits (Q4_K, Q6_K) or terms (MXFP4) of x and of the activations, so that the joined form differs by the order of f32
+sums: 1e-6 of the logits, as much of gate and of up, whose product is the activation, and 21 bits of it (2.2e-6 rms) again in the
+down projection: 1e-5. Where x is what the layer before added to, its differences go through a layer: 1e-3, and a layer that read x too
+early is off by more than half."""
+import pytest
+
+from helpers import canary_intact, out_with_canary, rel_l2, run_cpp
+
+import zinc_b200 as zb
+from zinc_b200.moe_step import MoeDecode, MoeShape
+
+pytestmark = pytest.mark.gpu
+
+
+def shape(arch, H, E, k, F, L):
+    q = arch == "kquant"
+    return MoeShape(hidden=H, n_experts=E, top_k=k, ffn=F, t_gate_up=zb.Q4_K if q else zb.MXFP4, t_down=zb.Q6_K if q else zb.MXFP4,
+                    rule=zb.ROUTE_SOFTMAX_ALL_RENORM if q else zb.ROUTE_TOPK_THEN_SOFTMAX, shared=q, oai=not q, n_layers=L, biases=not q)
+
+
+class Layers:
+    def __init__(self, torch, s, seed=7, layers=None):
+        self.torch, self.s = torch, s
+        self.stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(self.stream):
+            self.ctx = zb.Context(0, stream=self.stream.cuda_stream)
+            self.dd = zb.DmmvDispatch(self.ctx)
+            self.step = MoeDecode.build(torch, self.dd, s, seed=seed)
+        if layers:
+            self.step.layers = [self.step.layers[i % len(self.step.layers)] for i in range(layers)]
+        slots = self.step.routing.numel() // 2
+        self.sizes = {"hidden": s.hidden, "logits": s.n_experts, "act": slots * s.ffn, "routing": 2 * slots}
+        for name, n in self.sizes.items():
+            setattr(self.step, name, out_with_canary(torch, n))
+        self.step.routing = self.step.routing_local = self.step.routing.view(torch.int32)
+
+    def outs(self):
+        return {n: getattr(self.step, n) for n in self.sizes}
+
+    def reset(self, hidden):
+        for n, t in self.outs().items():
+            t[:self.sizes[n]] = 0
+        self.step.hidden[:self.s.hidden] = hidden
+
+    def eager_and_recorded(self, record, launches, hidden=0.25, replays=3):
+        torch = self.torch
+        with torch.cuda.stream(self.stream):
+            self.reset(hidden)
+            record()
+            self.ctx.submit_and_wait()
+            eager = {n: t.clone() for n, t in self.outs().items()}
+            n0 = self.ctx.launch_count
+            self.ctx.begin_record()
+            record()
+            rec = self.ctx.end_record()
+            assert self.ctx.launch_count - n0 == launches
+            got = None
+            for _ in range(replays):
+                self.reset(hidden)
+                self.ctx.replay(rec)
+                self.ctx.submit_and_wait()
+                now = {n: t.clone() for n, t in self.outs().items()}
+                assert got is None or all(torch.equal(got[n].view(torch.int32), now[n].view(torch.int32)) for n in now), "not the same bits"
+                got = now
+            self.ctx.free_recording(rec)
+        return eager, got
+
+    def check(self, eager, got, bar=1e-5):
+        slots = self.sizes["routing"] // 2
+        assert self.torch.equal(eager["routing"][:slots], got["routing"][:slots])
+        for n in ("logits", "act", "hidden"):
+            e, g = eager[n][:self.sizes[n]].cpu().numpy(), got[n][:self.sizes[n]].cpu().numpy()
+            assert rel_l2(g, e) <= (2e-6 if n == "logits" and bar == 1e-5 else bar), n
+        w = [r["routing"][slots:2 * slots].view(self.torch.float32).cpu().numpy() for r in (eager, got)]
+        assert rel_l2(w[1], w[0]) <= bar
+        for n, t in got.items():
+            assert canary_intact(t.view(self.torch.float32), self.sizes[n]), n
+
+
+# experts, slots and widths at the edges: widths of an odd number of blocks of 512, widths of 64 beyond a multiple of 128, more down rows
+# than SMs have tiles for, more gate and up units than the ring holds, fewer experts than SMs and several of them to a CTA
+@pytest.mark.parametrize("arch,H,E,k,F,L", [
+    ("kquant", 2048, 256, 8, 512, 3), ("kquant", 1280, 96, 5, 768, 2), ("kquant", 4096, 128, 8, 1024, 2), ("kquant", 1024, 64, 4, 512, 1),
+    ("mxfp4", 2880, 32, 4, 2880, 2), ("mxfp4", 1088, 16, 2, 1024, 3), ("mxfp4", 1984, 24, 3, 1472, 2), ("mxfp4", 1024, 200, 4, 2624, 1)])
+def test_joined_layers_by_shape(gpu, arch, H, E, k, F, L):
+    torch, _, _ = gpu
+    r = Layers(torch, shape(arch, H, E, k, F, L))
+    r.check(*r.eager_and_recorded(r.step.record, 1, replays=20))
+
+
+@pytest.mark.parametrize("arch,H,E,k,F", [("kquant", 2048, 64, 8, 512), ("mxfp4", 1984, 24, 3, 1472)])
+def test_layers_that_read_what_the_one_before_wrote(gpu, arch, H, E, k, F):
+    torch, _, _ = gpu
+    r = Layers(torch, shape(arch, H, E, k, F, 2))
+    hidden = 0.1 * torch.randn(H, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    r.step.x = r.step.hidden
+    r.check(*r.eager_and_recorded(r.step.record, 1, hidden=hidden, replays=20), bar=1e-3)
+
+
+def test_a_long_run_is_several_kernels(gpu):
+    torch, _, _ = gpu
+    r = Layers(torch, shape("kquant", 1024, 64, 4, 512, 2), layers=170)   # 160 in a kernel
+    r.check(*r.eager_and_recorded(r.step.record, 2))
+
+
+def test_calls_that_are_not_joined(gpu):
+    """Layers whose calls are not one another's, whose buffers meet, or with something in between."""
+    torch, _, _ = gpu
+    r = Layers(torch, shape("kquant", 1024, 64, 4, 512, 2))
+    step, dd = r.step, r.dd
+    act, act2 = step.act, out_with_canary(torch, 5 * 512 + 256)
+    x, x2 = step.x, step.x + 1.0
+    layers = step.layers
+
+    def run(*parts):
+        def record():
+            for layer, a, xx, between in parts:
+                step.layers, step.act, step.x = [layers[layer]], a, xx
+                if between:
+                    between()
+                step.record()
+            step.layers, step.act, step.x = layers, act, x
+        return record
+
+    r.check(*r.eager_and_recorded(run((0, act, x, None), (1, act, x, None)), 1))
+    r.check(*r.eager_and_recorded(run((0, act, x, None), (1, act, x2, None)), 1))
+    r.check(*r.eager_and_recorded(run((0, act, x, None), (1, act2, x, None)), 1))       # other buffers throughout
+    r.check(*r.eager_and_recorded(run((0, act2[256:], x, None), (1, act2, x, None)), 2))  # activations that overlap
+    spare = out_with_canary(torch, 1024)
+    r.check(*r.eager_and_recorded(run((0, act, x, None), (1, act, x, lambda: dd.dispatchSwiglu(x2, x2, spare, 512))), 3))
+    # selections into a place of their own in between
+    other = torch.zeros_like(step.routing)
+
+    def route_again():
+        w = layers[1]
+        dd.dispatchMoeRouterTopk(x2, w.router, r.step.logits, other, 64, 1024, 4, rule=r.s.rule, shared_slot=True)
+    r.check(*r.eager_and_recorded(run((0, act, x, None), (1, act, x, route_again)), 3))
+
+
+def test_two_recordings_on_two_streams(gpu):
+    torch, _, _ = gpu
+    a, b = Layers(torch, shape("kquant", 2048, 64, 8, 512, 3)), Layers(torch, shape("mxfp4", 1920, 24, 3, 1920, 3))
+    recs = []
+    for r in (a, b):
+        with torch.cuda.stream(r.stream):
+            r.reset(0.25)
+            r.step.record()
+            r.ctx.submit_and_wait()
+            r.eager = {n: t.clone() for n, t in r.outs().items()}
+            r.ctx.begin_record()
+            r.step.record()
+            recs.append(r.ctx.end_record())
+            r.ctx.submit_and_wait()
+    for _ in range(20):
+        for r, rec in zip((a, b), recs):
+            with torch.cuda.stream(r.stream):
+                r.reset(0.25)
+                r.ctx.replay(rec)
+    for r, rec in zip((a, b), recs):
+        r.ctx.submit_and_wait()
+        r.check(r.eager, r.outs())
+        r.ctx.free_recording(rec)
+
+
+def test_waits_that_run_out(gpu):
+    """The kernel with limits that run out, with copies under way; each time a sound launch next."""
+    run_cpp("test_moe_waits")

@@ -4,3 +4,7 @@ from helpers import run_cpp
 
 def test_what_is_worth_being_joined():
     run_cpp("test_program_worth")
+
+
+def test_how_moe_layers_are_laid_out():
+    run_cpp("test_moe_layout")

@@ -12,6 +12,7 @@
 #include "../../include/zinc_cuda.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "moe_program.h"
 #include "program.h"
 
 namespace zc {
@@ -63,6 +64,15 @@ struct zc_ctx {
     bool recording = false;
     unsigned long long record_id = 0;  // of the capture that zc_begin_record began: calls may go to another one in between
     std::vector<Recorded> recorded;
+    // .. and the calls of MoE decode layers
+    struct RecordedMoe {
+        cudaGraphNode_t node;
+        int stage;                     // 0 router + selection, 1 gate + up + activation, 2 down + weighted sum
+        uint32_t type;
+        zc::MoeRouterCall router;
+        zc::DmmvArgs args;
+    };
+    std::vector<RecordedMoe> recorded_moe;
     uint64_t joined = 0;           // recorded launches that became part of another one
     char err[512] = {0};
 };
@@ -189,8 +199,8 @@ cudaError_t run_mul_mm_exact(zc_ctx* ctx, const ExactGemm& p) {
     return with_exact_scratch(ctx, [&] { return launch_mul_mm_exact(p, ctx->exact_scratch, ctx->stream, &ctx->launches); });
 }
 
-// A call that was just recorded as one kernel, described by `op`: remembered with its graph node.
-void note_op(zc_ctx* ctx, const ProgramOp& op) {
+// The graph node of a call that was just recorded as one kernel; null: it is none, or not of the recording's own capture.
+cudaGraphNode_t recorded_node(zc_ctx* ctx) {
     cudaStreamCaptureStatus st;
     unsigned long long id = 0;
     cudaGraph_t graph = nullptr;
@@ -199,12 +209,24 @@ void note_op(zc_ctx* ctx, const ProgramOp& op) {
     size_t n = 0;
     if (cudaStreamGetCaptureInfo_v3(ctx->stream, &st, &id, &graph, &deps, &edges, &n) != cudaSuccess ||
         st != cudaStreamCaptureStatusActive || id != ctx->record_id || n != 1)
-        return;
+        return nullptr;
     cudaGraphNodeType type;
-    if (cudaGraphNodeGetType(deps[0], &type) != cudaSuccess || type != cudaGraphNodeTypeKernel) return;
+    return cudaGraphNodeGetType(deps[0], &type) == cudaSuccess && type == cudaGraphNodeTypeKernel ? deps[0] : nullptr;
+}
+void note_op(zc_ctx* ctx, const ProgramOp& op) {
+    const cudaGraphNode_t node = recorded_node(ctx);
+    if (!node) return;
     try {
-        ctx->recorded.push_back({deps[0], op});
+        ctx->recorded.push_back({node, op});
     } catch (const std::bad_alloc&) {  // the call stays a launch of its own
+    }
+}
+void note_moe(zc_ctx* ctx, int stage, uint32_t type, const MoeRouterCall& router, const DmmvArgs& args) {
+    const cudaGraphNode_t node = recorded_node(ctx);
+    if (!node) return;
+    try {
+        ctx->recorded_moe.push_back({node, stage, type, router, args});
+    } catch (const std::bad_alloc&) {
     }
 }
 void note_call(zc_ctx* ctx, uint32_t type, int mode, const DmmvArgs& a) {
@@ -227,8 +249,9 @@ cudaGraphNode_t only_neighbour(cudaGraphNode_t node, bool behind) {
 
 // Puts one node in the place of the nodes of a program, which follow one another and nothing else. `replaced` stays false where
 // the new node is refused: the graph is then as it was.
-cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t n, Program& p, void* func, uint32_t threads, uint32_t smem,
-                          bool& replaced) {
+template <typename Recorded>
+cudaError_t replace_nodes(cudaGraph_t graph, const Recorded* r, uint32_t n, void* params, uint32_t grid, void* func, uint32_t threads,
+                          uint32_t smem, bool& replaced) {
     size_t n_in = 0, n_out = 0;
     cudaError_t e = cudaGraphNodeGetDependencies_v2(r[0].node, nullptr, nullptr, &n_in);
     if (e == cudaSuccess) e = cudaGraphNodeGetDependentNodes_v2(r[n - 1].node, nullptr, nullptr, &n_out);
@@ -238,10 +261,10 @@ cudaError_t replace_nodes(cudaGraph_t graph, const zc_ctx::Recorded* r, uint32_t
     if (n_in) e = cudaGraphNodeGetDependencies_v2(r[0].node, in.data(), edges.data(), &n_in);
     if (e == cudaSuccess && n_out) e = cudaGraphNodeGetDependentNodes_v2(r[n - 1].node, out.data(), edges.data(), &n_out);
     if (e != cudaSuccess) return e;
-    void* args[] = {&p};
+    void* args[] = {params};
     cudaKernelNodeParams k = {};
     k.func = func;
-    k.gridDim = dim3(p.grid);
+    k.gridDim = dim3(grid);
     k.blockDim = dim3(threads);
     k.sharedMemBytes = smem;
     k.kernelParams = args;
@@ -280,6 +303,75 @@ struct SideStream {
     }
 };
 
+// b follows a and nothing else does, and b follows nothing else
+bool in_a_row(cudaGraphNode_t a, cudaGraphNode_t b) { return only_neighbour(a, true) == b && only_neighbour(b, false) == a; }
+
+// Memory of a recording's own: `copied` bytes from `from`, `zeroed` bytes of zeros behind them, `more` behind those; null: none to be had.
+cudaError_t recording_memory(zc_recording* rec, SideStream& side, const void* from, size_t copied, size_t zeroed, size_t more, uint8_t** out) {
+    uint8_t* mem = nullptr;
+    *out = nullptr;
+    rec->memory.reserve(rec->memory.size() + 1);
+    if (cudaMalloc(reinterpret_cast<void**>(&mem), copied + zeroed + more) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    rec->memory.push_back(mem);
+    cudaError_t e = side.open();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(mem, from, copied, cudaMemcpyHostToDevice, side.stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(mem + copied, 0, zeroed, side.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(side.stream);
+    *out = mem;
+    return e;
+}
+
+// Runs of recorded MoE decode layers, three calls each and nothing between them, become one kernel each (moe_program.h).
+cudaError_t join_recorded_moe(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
+    const std::vector<zc_ctx::RecordedMoe>& r = ctx->recorded_moe;
+    SideStream side;
+    std::vector<MoeCalls> calls;
+    std::vector<MoeProgram> prog(1);
+    MoeProgram& p = prog[0];
+    for (size_t i = 0; i + 2 < r.size();) {
+        calls.clear();
+        for (size_t j = i; j + 2 < r.size() && calls.size() < kMoeMaxLayers; j += 3) {
+            if (r[j].stage != 0 || r[j + 1].stage != 1 || r[j + 2].stage != 2 || !in_a_row(r[j].node, r[j + 1].node) ||
+                !in_a_row(r[j + 1].node, r[j + 2].node) || (j > i && !in_a_row(r[j - 1].node, r[j].node)))
+                break;
+            calls.push_back({r[j].router, r[j + 1].type, r[j + 2].type, r[j + 1].args, r[j + 2].args});
+        }
+        const uint32_t n = moe_plan(calls.data(), (uint32_t)calls.size(), ctx->sm_count, p);
+        if (n == 0) {
+            ++i;
+            continue;
+        }
+        void* func = nullptr;
+        uint32_t threads = 0;
+        std::vector<CUtensorMap> maps((size_t)n * p.n_maps);
+        if (moe_program_kernel(calls[0].gate_up_type == T_MXFP4, ctx->sm_count, p, &func, threads) != cudaSuccess || !moe_maps(calls.data(), p, maps.data())) {
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        const size_t map_bytes = maps.size() * sizeof(CUtensorMap);
+        uint8_t* mem;
+        cudaError_t e = recording_memory(rec, side, maps.data(), map_bytes, moe_exchange_bytes(p), 0, &mem);
+        if (e != cudaSuccess || !mem) return e;  // the calls stay launches
+        p.maps = mem;
+        p.words = reinterpret_cast<uint32_t*>(mem + map_bytes);
+        p.logits_x = reinterpret_cast<uint64_t*>(mem + map_bytes + 256);
+        p.act_x = p.logits_x + 2 * p.E;
+        p.status = ctx->status_dev;
+        bool replaced = false;
+        if ((e = replace_nodes(graph, r.data() + i, 3 * n, &p, p.grid, func, threads, p.smem, replaced)) != cudaSuccess) {
+            if (replaced) return e;
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        ctx->joined += 3 * n - 1;
+        i += 3 * n;
+    }
+    return cudaSuccess;
+}
+
 // Runs of recorded calls with nothing between them become one kernel each (program.h), where that is the faster form. What does not
 // fit stays as it was.
 cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
@@ -293,7 +385,7 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
     std::vector<Program> prog(2);
     for (size_t i = 0; i + 1 < r.size();) {
         size_t end = i + 1;
-        while (end < r.size() && end - i < kProgMaxOps && only_neighbour(r[end - 1].node, true) == r[end].node && only_neighbour(r[end].node, false) == r[end - 1].node) ++end;
+        while (end < r.size() && end - i < kProgMaxOps && in_a_row(r[end - 1].node, r[end].node)) ++end;
         if (end - i < 2) {
             i = end;
             continue;
@@ -320,26 +412,17 @@ cudaError_t join_recorded(zc_ctx* ctx, cudaGraph_t graph, zc_recording* rec) {
             }
         }
         const size_t map_bytes = p.n_maps * sizeof(CUtensorMap), words = (2 * n + 1 + 31) & ~31u;
-        uint8_t* mem = nullptr;
-        rec->memory.reserve(rec->memory.size() + 1);
-        if (cudaMalloc(reinterpret_cast<void**>(&mem), map_bytes + words * 4 + p.table_bytes) != cudaSuccess) {  // the calls stay launches
-            cudaGetLastError();
-            return cudaSuccess;
-        }
-        rec->memory.push_back(mem);
+        uint8_t* mem;
+        if ((e = recording_memory(rec, side, maps.data(), map_bytes, words * 4, p.table_bytes, &mem)) != cudaSuccess || !mem) return e;  // the calls stay launches
         p.maps = mem;
         mem += map_bytes;
-        if ((e = side.open()) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(const_cast<uint8_t*>(p.maps), maps.data(), map_bytes, cudaMemcpyHostToDevice, side.stream)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(mem, 0, words * 4, side.stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamSynchronize(side.stream)) != cudaSuccess) return e;
         p.done = reinterpret_cast<uint32_t*>(mem);
         p.converted = p.done + n;
         p.left = p.converted + n;
         p.tables = mem + words * 4;
         p.status = ctx->status_dev;
         bool replaced = false;
-        if ((e = replace_nodes(graph, r.data() + i, n, p, func, threads, smem, replaced)) != cudaSuccess) {
+        if ((e = replace_nodes(graph, r.data() + i, n, &p, p.grid, func, threads, smem, replaced)) != cudaSuccess) {
             if (replaced) return e;
             cudaGetLastError();
             return cudaSuccess;
@@ -699,6 +782,7 @@ int32_t zc_begin_record(zc_ctx* ctx) {
     ctx->recording = cudaStreamGetCaptureInfo_v3(ctx->stream, &st, &ctx->record_id, nullptr, nullptr, nullptr, nullptr) == cudaSuccess &&
                      st == cudaStreamCaptureStatusActive;  // else the calls stay launches
     ctx->recorded.clear();
+    ctx->recorded_moe.clear();
     return ZC_OK;
 }
 
@@ -713,11 +797,13 @@ int32_t zc_end_record(zc_ctx* ctx, void** out_recording) {
     zc_recording* rec = new (std::nothrow) zc_recording();
     if (!rec) e = cudaErrorMemoryAllocation;
     try {
+        if (e == cudaSuccess) e = join_recorded_moe(ctx, graph, rec);
         if (e == cudaSuccess) e = join_recorded(ctx, graph, rec);
     } catch (const std::bad_alloc&) {
         e = cudaErrorMemoryAllocation;
     }
     ctx->recorded.clear();
+    ctx->recorded_moe.clear();
     if (e == cudaSuccess) e = cudaGraphInstantiate(&rec->exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
@@ -1217,6 +1303,7 @@ static int32_t moe_gate_up_common(zc_ctx* ctx, const char* fn, uint32_t type, co
         e = launch_mxfp4_moe_gate_up(a, ctx->stream, &ctx->launches);
     else
         e = launch_dmmv(type, MODE_MOE_GATE_UP, a, ctx->stream, &ctx->launches);
+    if (ctx->recording && e == cudaSuccess) note_moe(ctx, 1, type, MoeRouterCall(), a);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }
 
@@ -1280,6 +1367,7 @@ static int32_t moe_down_acc_common(zc_ctx* ctx, const char* fn, uint32_t type, c
         e = launch_q6k_moe_down_acc(a, ctx->stream, &ctx->launches);
     else
         e = launch_dmmv(type, MODE_MOE_DOWN_ACC, a, ctx->stream, &ctx->launches);
+    if (ctx->recording && e == cudaSuccess) note_moe(ctx, 2, type, MoeRouterCall(), a);
     return e == cudaSuccess ? ZC_OK : cuda_fail(ctx, e, fn);
 }
 
@@ -1367,6 +1455,12 @@ int32_t zc_moe_router_topk(zc_ctx* ctx, const void* hidden, uint64_t hidden_size
         rule, shared_slot, e_lo, e_hi, local_shared, eps, ctx->stream, &ctx->launches);
     if (e != cudaSuccess) return cuda_fail(ctx, e, fn);
     ctx->router_mark = ctx->launches;
+    if (ctx->recording)
+        note_moe(ctx, 0, T_F32,
+                 MoeRouterCall{f32p(hidden, 0), static_cast<const float*>(norm_weights), f32p(router_weights, 0), static_cast<const float*>(bias),
+                               f32m(logits, 0), static_cast<uint32_t*>(routing), static_cast<const uint32_t*>(routing_local), n_experts, K, k, rule,
+                               shared_slot},
+                 DmmvArgs());
     return ZC_OK;
 }
 

@@ -57,12 +57,6 @@ struct SliceArgs {
     uint32_t tpe_mul, bpe_mul;     // reciprocals of tpe and bpe (quotient)
 };
 
-// n / d by the high word of a product, where 2^32 / d + 1 is exact for every n < limit; 0: it is not (quotient divides).
-inline uint32_t reciprocal(uint32_t d, uint64_t limit) { return d > 1 && limit * d < (1ull << 32) ? (uint32_t)((1ull << 32) / d) + 1 : 0; }
-__host__ __device__ __forceinline__ uint32_t quotient(uint32_t n, uint32_t d, uint32_t mul) {
-    return mul ? (uint32_t)(((uint64_t)n * mul) >> 32) : n / d;
-}
-
 inline SliceArgs slice_args(const DmmvArgs& a) {
     SliceArgs s = {};
     s.A[0] = a.A;

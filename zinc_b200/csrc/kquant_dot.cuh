@@ -1,5 +1,5 @@
 // The parts of the K-quant matvecs that their kernels share: x as 21-bit fixed point in three digits, and the exact integer dot
-// product of a Q6_K block with it (src/shaders/dmmv_q6k.comp:58-156; layout: src/compute/forward.zig:276-325).
+// products of Q4_K and Q6_K blocks with it (src/shaders/dmmv_q6k.comp:58-156; layout: src/compute/forward.zig:276-325).
 #pragma once
 
 #include "stream_skel.cuh"
@@ -55,10 +55,73 @@ __device__ __forceinline__ Digits digits_of(const X8& r) {
     return d;
 }
 
+constexpr uint32_t kQ4kTable = 768 + 32 + 4;  // bytes per block of x
+// Block blk of x into a Q4_K table: three digit planes of K bytes, sums per 32 elements, scale per 256.
+__device__ __forceinline__ void prep_q4k(uint8_t* tab, const X8& r, uint32_t K, uint32_t blk, int lane) {
+    const Digits d = digits_of(r);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(tab + j * K + blk * 256 + 8 * lane) = make_uint2(d.w[j][0], d.w[j][1]);
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum += d.X[i];
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
+    if ((lane & 3) == 0) put(tab + 3 * K + (blk * 8 + (lane >> 2)) * 4, __float_as_uint((float)sum));
+    if (lane == 0) put(tab + 3 * K + (K >> 8) * 32 + blk * 4, __float_as_uint(d.inv));
+}
+
+struct Q4kAcc {
+    float M[2], m[2];
+    __device__ __forceinline__ void clear() { M[0] = M[1] = m[0] = m[1] = 0.f; }
+};
+
+// A unit's rows lie 288 bytes apart. 128-bit reads take eight lanes, rows of two lane groups, at a time: rows two apart start
+// 64 bytes apart modulo 128, so lane groups 2 i and 2 i + 1 get such rows (the low two bits of the group swapped).
+__device__ __forceinline__ uint32_t q4k_row(uint32_t g) { return (g & 4u) | ((g & 1u) << 1) | ((g >> 1) & 1u); }
+
+// One super-block of rows A and B: see the Q4_K streaming matvec for the layout of the operands.
+__device__ __forceinline__ void q4k_block(uint32_t rA, uint32_t rB, uint32_t xb, uint32_t sxa, uint32_t xsa, uint32_t t, uint32_t msel, Q4kAcc& acc) {
+    constexpr uint32_t kLo = 0x0F0F0F0Fu, kHi = 0xF0F0F0F0u;
+    const uint4 hA = lds_v4(rA), hB = lds_v4(rB);
+    const uint32_t scA[2] = {hA.y & 0x3F3F3F3Fu, (hA.w & 0x0F0F0F0Fu) | ((hA.y >> 2) & 0x30303030u)};
+    const uint32_t scB[2] = {hB.y & 0x3F3F3F3Fu, (hB.w & 0x0F0F0F0Fu) | ((hB.y >> 2) & 0x30303030u)};
+    int IloA = 0, IhiA = 0, IloB = 0, IhiB = 0;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const uint4 qa = lds_v4(rA + 16 + 64 * p + 16 * t), qb = lds_v4(rB + 16 + 64 * p + 16 * t);
+        const uint4 bl = lds_v4(xb + 128 * p), bh = lds_v4(xb + 128 * p + 32);
+        int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+        mma_u8s8(lo, qa.x & kLo, qb.x & kLo, qa.y & kLo, qb.y & kLo, bl.x, bl.y);
+        mma_u8s8(lo, qa.z & kLo, qb.z & kLo, qa.w & kLo, qb.w & kLo, bl.z, bl.w);
+        mma_u8s8(hi, qa.x & kHi, qb.x & kHi, qa.y & kHi, qb.y & kHi, bh.x, bh.y);
+        mma_u8s8(hi, qa.z & kHi, qb.z & kHi, qa.w & kHi, qb.w & kHi, bh.z, bh.w);
+        const uint32_t sa = scA[p], sb = scB[p];
+        IloA += lo[0] * (int)(sa & 0xFFu) + lo[1] * (int)((sa >> 16) & 0xFFu);
+        IhiA += hi[0] * (int)((sa >> 8) & 0xFFu) + hi[1] * (int)(sa >> 24);
+        IloB += lo[2] * (int)(sb & 0xFFu) + lo[3] * (int)((sb >> 16) & 0xFFu);
+        IhiB += hi[2] * (int)((sb >> 8) & 0xFFu) + hi[3] * (int)(sb >> 24);
+    }
+    const float PA = (float)(IloA * 16 + IhiA), PB = (float)(IloB * 16 + IhiB);
+    const uint32_t mnA = __byte_perm(hA.z & 0x3F3F3F3Fu, ((hA.w >> 4) & 0x0F0F0F0Fu) | ((hA.z >> 2) & 0x30303030u), msel);
+    const uint32_t mnB = __byte_perm(hB.z & 0x3F3F3F3Fu, ((hB.w >> 4) & 0x0F0F0F0Fu) | ((hB.z >> 2) & 0x30303030u), msel);
+    const float xs = lds_f1(xsa);
+    const float2 sxv = lds_f2(sxa);
+    const float dA = h2f(hA.x) * xs, dmA = h2f(hA.x >> 16) * xs;
+    const float dB = h2f(hB.x) * xs, dmB = h2f(hB.x >> 16) * xs;
+    const float mA = (float)(mnA & 0xFFu) * sxv.x + (float)((mnA >> 8) & 0xFFu) * sxv.y;
+    const float mB = (float)(mnB & 0xFFu) * sxv.x + (float)((mnB >> 8) & 0xFFu) * sxv.y;
+    acc.M[0] = fmaf(dA, PA, acc.M[0]);
+    acc.M[1] = fmaf(dB, PB, acc.M[1]);
+    acc.m[0] = fmaf(dmA, mA, acc.m[0]);
+    acc.m[1] = fmaf(dmB, mB, acc.m[1]);
+}
+
 constexpr uint32_t kQ6kTable = 768 + 96 + 4;  // bytes per block of x
 // Block blk of nb into a Q6_K table: the digits in the order the lanes read them (768 bytes a block), their sums over the
 // sub-blocks in two parts (96), the scales (4). Lane l: half h = l / 16, quarter j = (l / 4) % 4, sub-block half u = (l / 2) % 2, k slots t0, t0 + 1 with t0 = 2 (l % 2)
-__device__ __forceinline__ void prep_q6k(uint8_t* tab, const X8& r, uint32_t nb, uint32_t blk, int lane) {
+// kTwice: written to another CTA of the cluster too, whose shared memory is `also` on from this one's.
+template <bool kTwice = false>
+__device__ __forceinline__ void prep_q6k(uint8_t* tab, const X8& r, uint32_t nb, uint32_t blk, int lane, uint32_t also = 0) {
     const Digits d = digits_of(r);
     const uint32_t h = lane >> 4, j = (lane >> 2) & 3, u = (lane >> 1) & 1, t0 = 2 * (lane & 1);
     uint8_t* const b = tab + blk * 768 + h * 384 + u * 64 + t0 * 16 + j * 4;
@@ -73,14 +136,25 @@ __device__ __forceinline__ void prep_q6k(uint8_t* tab, const X8& r, uint32_t nb,
     for (int k = 0; k < 3; ++k) {
         put(b + k * 128, d.w[k][0]);
         put(b + k * 128 + 16, d.w[k][1]);
+        if constexpr (kTwice) {
+            st_cluster(smem_u32(b) + also + k * 128, d.w[k][0]);
+            st_cluster(smem_u32(b) + also + k * 128 + 16, d.w[k][1]);
+        }
         const int sum = s[k] + __shfl_xor_sync(0xFFFFFFFFu, s[k], 1);  // of sub-block 8 h + 2 j + u: -1024 .. 2032 = 64 hi + lo
         if ((lane & 1) == 0) {
             uint8_t* q = tab + nb * 768 + blk * 96 + k * 32 + 8 * h + 2 * j + u;
             q[0] = (uint8_t)(sum & 63);
             q[16] = (uint8_t)(sum >> 6);
+            if constexpr (kTwice) {
+                st_cluster_u8(smem_u32(q) + also, sum & 63);
+                st_cluster_u8(smem_u32(q) + also + 16, sum >> 6);
+            }
         }
     }
-    if (lane == 0) put(tab + nb * 864 + blk * 4, __float_as_uint(d.inv));
+    if (lane == 0) {
+        put(tab + nb * 864 + blk * 4, __float_as_uint(d.inv));
+        if constexpr (kTwice) st_cluster(smem_u32(tab) + also + nb * 864 + blk * 4, __float_as_uint(d.inv));
+    }
 }
 
 // Where a row's words lie: on word boundaries, in the middle of words (2 bytes past `a`), or anywhere (sh = 8 x the byte past `a`).

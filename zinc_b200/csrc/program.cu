@@ -55,11 +55,7 @@ struct Sync {
 constexpr uint32_t kTables = (kSmem - 128 - kRing - kZeros - kParts * kPartBytes - (uint32_t)sizeof(Sync)) & ~127u;
 
 // ---- x tables --------------------------------------------------------------------------------------------
-// Q4_K: three digit planes of K bytes, sums per 32 elements, scale per 256. Q6_K, per 256 elements: digits in the order the
-// lanes read them (768 bytes), the digits' sums over the sub-blocks in two parts (96), scale (4).
-__host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t K) {
-    return kind == PROG_Q4K ? (K / 256) * (768 + 32 + 4) : (K / 256) * kQ6kTable;
-}
+__host__ __device__ constexpr uint32_t table_bytes(uint32_t kind, uint32_t K) { return (K / 256) * (kind == PROG_Q4K ? kQ4kTable : kQ6kTable); }
 // A unit in the ring: 16 rows of two blocks each, Q6_K as the 16-byte aligned bytes around them. Its rows lie an odd multiple of
 // 16 bytes apart, so that a 32-bit read of eight rows meets 32 banks.
 __host__ __device__ constexpr uint32_t unit_pitch(uint32_t kind) { return kind == PROG_Q4K ? 288u : kind == PROG_Q6K ? 432u : 464u; }
@@ -68,64 +64,6 @@ __host__ __device__ constexpr uint32_t unit_pitch(uint32_t kind) { return kind =
 __device__ __forceinline__ X8 load_x(const float* x, uint32_t blk, int lane) {
     const float4* p = reinterpret_cast<const float4*>(x + (size_t)blk * 256 + 8 * lane);
     return {__ldcg(p), __ldcg(p + 1)};
-}
-__device__ __forceinline__ void prep_q4k(uint8_t* tab, const X8& r, uint32_t K, uint32_t blk, int lane) {
-    const Digits d = digits_of(r);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) *reinterpret_cast<uint2*>(tab + j * K + blk * 256 + 8 * lane) = make_uint2(d.w[j][0], d.w[j][1]);
-    int sum = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) sum += d.X[i];
-    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-    sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-    if ((lane & 3) == 0) put(tab + 3 * K + (blk * 8 + (lane >> 2)) * 4, __float_as_uint((float)sum));
-    if (lane == 0) put(tab + 3 * K + (K >> 8) * 32 + blk * 4, __float_as_uint(d.inv));
-}
-// ---- dot products ---------------------------------------------------------------------------------------
-struct Acc {
-    float M[2], m[2];
-    __device__ __forceinline__ void clear() { M[0] = M[1] = m[0] = m[1] = 0.f; }
-};
-
-// A unit's rows lie 288 bytes apart. 128-bit reads take eight lanes, rows of two lane groups, at a time: rows two apart start
-// 64 bytes apart modulo 128, so lane groups 2 i and 2 i + 1 get such rows (the low two bits of the group swapped).
-__device__ __forceinline__ uint32_t q4k_row(uint32_t g) { return (g & 4u) | ((g & 1u) << 1) | ((g >> 1) & 1u); }
-
-// One super-block of rows A and B: see the Q4_K streaming matvec for the layout of the operands.
-__device__ __forceinline__ void q4k_block(uint32_t rA, uint32_t rB, uint32_t xb, uint32_t sxa, uint32_t xsa, uint32_t t, uint32_t msel, Acc& acc) {
-    constexpr uint32_t kLo = 0x0F0F0F0Fu, kHi = 0xF0F0F0F0u;
-    const uint4 hA = lds_v4(rA), hB = lds_v4(rB);
-    const uint32_t scA[2] = {hA.y & 0x3F3F3F3Fu, (hA.w & 0x0F0F0F0Fu) | ((hA.y >> 2) & 0x30303030u)};
-    const uint32_t scB[2] = {hB.y & 0x3F3F3F3Fu, (hB.w & 0x0F0F0F0Fu) | ((hB.y >> 2) & 0x30303030u)};
-    int IloA = 0, IhiA = 0, IloB = 0, IhiB = 0;
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const uint4 qa = lds_v4(rA + 16 + 64 * p + 16 * t), qb = lds_v4(rB + 16 + 64 * p + 16 * t);
-        const uint4 bl = lds_v4(xb + 128 * p), bh = lds_v4(xb + 128 * p + 32);
-        int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-        mma_u8s8(lo, qa.x & kLo, qb.x & kLo, qa.y & kLo, qb.y & kLo, bl.x, bl.y);
-        mma_u8s8(lo, qa.z & kLo, qb.z & kLo, qa.w & kLo, qb.w & kLo, bl.z, bl.w);
-        mma_u8s8(hi, qa.x & kHi, qb.x & kHi, qa.y & kHi, qb.y & kHi, bh.x, bh.y);
-        mma_u8s8(hi, qa.z & kHi, qb.z & kHi, qa.w & kHi, qb.w & kHi, bh.z, bh.w);
-        const uint32_t sa = scA[p], sb = scB[p];
-        IloA += lo[0] * (int)(sa & 0xFFu) + lo[1] * (int)((sa >> 16) & 0xFFu);
-        IhiA += hi[0] * (int)((sa >> 8) & 0xFFu) + hi[1] * (int)(sa >> 24);
-        IloB += lo[2] * (int)(sb & 0xFFu) + lo[3] * (int)((sb >> 16) & 0xFFu);
-        IhiB += hi[2] * (int)((sb >> 8) & 0xFFu) + hi[3] * (int)(sb >> 24);
-    }
-    const float PA = (float)(IloA * 16 + IhiA), PB = (float)(IloB * 16 + IhiB);
-    const uint32_t mnA = __byte_perm(hA.z & 0x3F3F3F3Fu, ((hA.w >> 4) & 0x0F0F0F0Fu) | ((hA.z >> 2) & 0x30303030u), msel);
-    const uint32_t mnB = __byte_perm(hB.z & 0x3F3F3F3Fu, ((hB.w >> 4) & 0x0F0F0F0Fu) | ((hB.z >> 2) & 0x30303030u), msel);
-    const float xs = lds_f1(xsa);
-    const float2 sxv = lds_f2(sxa);
-    const float dA = h2f(hA.x) * xs, dmA = h2f(hA.x >> 16) * xs;
-    const float dB = h2f(hB.x) * xs, dmB = h2f(hB.x >> 16) * xs;
-    const float mA = (float)(mnA & 0xFFu) * sxv.x + (float)((mnA >> 8) & 0xFFu) * sxv.y;
-    const float mB = (float)(mnB & 0xFFu) * sxv.x + (float)((mnB >> 8) & 0xFFu) * sxv.y;
-    acc.M[0] = fmaf(dA, PA, acc.M[0]);
-    acc.M[1] = fmaf(dB, PB, acc.M[1]);
-    acc.m[0] = fmaf(dmA, mA, acc.m[0]);
-    acc.m[1] = fmaf(dmB, mB, acc.m[1]);
 }
 
 // ---- waits ------------------------------------------------------------------------------------------------
@@ -416,7 +354,7 @@ __device__ __forceinline__ void compute(const Program& p, Sync* sync, uint32_t t
     const uint32_t g = lane >> 2, t = lane & 3;
     const uint32_t msel = (2u * t) | ((2u * t + 1u) << 4) | 0x7700u;
     const uint32_t m0 = g < 6 && (g & 1) == 0 ? 1u : 0u, m1 = g < 6 && (g & 1) ? 1u : 0u;
-    Acc acc;
+    Q4kAcc acc;
     acc.clear();
     uint32_t cur = 0xFFFFFFFFu, kind = 0, tab = 0, bpr = 0, xb = 0, xstep = 0;
     for (uint32_t u = warp, n = 1;; u += kWarps, ++n) {

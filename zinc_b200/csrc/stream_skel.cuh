@@ -58,6 +58,13 @@ __device__ __forceinline__ float lds_f1(uint32_t saddr) {
     return v;
 }
 
+// Stores to the cluster's shared window
+__device__ __forceinline__ void st_cluster(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void st_cluster(uint32_t a, const uint4& v) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u8(uint32_t a, int v) { asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -86,6 +93,12 @@ __device__ __forceinline__ uint2 ld_volatile_u2(const uint2* p) {
     uint2 v;
     asm volatile("ld.volatile.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
     return v;
+}
+
+// n / d by the high word of a product, where 2^32 / d + 1 is exact for every n < limit; 0: it is not (quotient divides).
+inline uint32_t reciprocal(uint32_t d, uint64_t limit) { return d > 1 && limit * d < (1ull << 32) ? (uint32_t)((1ull << 32) / d) + 1 : 0; }
+__host__ __device__ __forceinline__ uint32_t quotient(uint32_t n, uint32_t d, uint32_t mul) {
+    return mul ? (uint32_t)(((uint64_t)n * mul) >> 32) : n / d;
 }
 
 // The consumer half of the fused exchange, spread over the grid: element i belongs to thread i / n_ctas of CTA
