@@ -374,6 +374,36 @@ def test_split_gemm_is_reproducible(gpu, oracle, t, M, N, K, bf16):
     assert rel_l2(first[cols].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols])) <= (TOL_BF16 if bf16 else 2e-6)
 
 
+# Shapes that K is cut for over 1, 2, 4, 6, 10 and 16 CTAs and whole tiles; tokens on both sides of a tile's 192 and of 16, one block of K,
+# rows on both sides of 8 and 128 (Q6_K: boxes of every eighth row), rows of D that start anywhere and at 16 bytes only
+@pytest.mark.parametrize("t,M,N,K", [(t, *s) for t in (zb.Q4_K, zb.Q6_K) for s in
+                                     ((1, 16, 256), (127, 17, 512), (130, 192, 1024), (263, 193, 2560), (1024, 77, 4096), (1027, 385, 768),
+                                      (300, 40, 11520), (641, 209, 3328), (2050, 31, 1280), (515, 1500, 256))])
+@pytest.mark.parametrize("pad_b,pad_d,d_off", [(0, 0, 0), (8, 3, 1), (24, 4, 4)])
+def test_mul_mm_cut(gpu, oracle, t, M, N, K, pad_b, pad_d, d_off):
+    torch, ctx, dd = gpu
+    g = synth.rng(341, M + N + t)
+    raw, X = synth.quant_matrix(g, t, M, K), synth.activations(g, N, K)
+    X = synth.bf16_bits_to_f32(synth.to_bf16_bits(X))
+    Xp = np.zeros((N, K + pad_b), np.float32)
+    Xp[:, :K] = X
+    w, x = dev(torch, raw), dev(torch, Xp).to(torch.bfloat16)
+    first = None
+    for i in range(4):
+        D = torch.full((d_off + (N + 1) * (M + pad_d),), 7.0, device="cuda")
+        torch.cuda.synchronize()
+        dd.recordMulMm(t, w, x, D, M, N, K, K + pad_b, M + pad_d, 0, 0, d_off, zb.BF16)
+        ctx.submit_and_wait()
+        got = D.cpu()
+        first = got if first is None else first
+        assert torch.equal(got, first), "not the same bits"
+    assert (first[:d_off] == 7.0).all()
+    first = first[d_off:].view(N + 1, M + pad_d)
+    assert (first[N:] == 7.0).all() and (first[:, M:] == 7.0).all()
+    cols = sorted({0, 15, N // 2, N - 1})
+    assert rel_l2(first[cols, :M].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols], round_bf16=True)) <= TOL_BF16_OPERANDS
+
+
 @pytest.mark.parametrize("t,M,N,K,bf16,want", [
     (zb.Q4_K, 256, 40, 4096, True, 2),      # K split: zeroing kernel, GEMM
     (zb.Q4_K, 40960, 40, 256, True, 1),

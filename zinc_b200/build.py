@@ -9,7 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO = os.path.join(HERE, "libzinc_b200.so")
 CALL_SO = os.path.join(HERE, "_call.so")   # Python module: calls into the library without ctypes
-SOURCES = ["api.cu", "dmmv.cu", "dmmv_warp.cu", "dmmv_q6k.cu", "dmmv_row.cu", "misc.cu", "gemm_simple.cu", "gemm_tc.cu",
+SOURCES = ["api.cu", "dmmv.cu", "dmmv_warp.cu", "dmmv_q6k.cu", "dmmv_row.cu", "misc.cu", "gemm_simple.cu", "gemm_tc.cu", "gemm_cut.cu",
            "dmmv_static_scratch.cu", "comm.cu", "dmmv_mxfp4.cu", "program.cu", "moe_program.cu", "moe_gemm_tc.cu", "moe_gemm_pair.cu", "gemm_mx.cu", "gemm_exact.cu",
            "gemm_exact_q4k.cu", "gemm_exact_q5k.cu", "gemm_exact_q6k.cu", "gemm_exact_q8.cu", "gemm_exact_mxfp4.cu"]
 NVCC_FLAGS = [

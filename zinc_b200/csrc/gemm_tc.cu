@@ -5,7 +5,8 @@
 //   X  bf16 activations [N][stride_b], fetched by TMA (cp.async.bulk.tensor, 128-byte swizzle)
 //   D  f32 [N][stride_d]; accumulators live in tensor memory and are read back with tcgen05.ld
 //
-// Three kernels. More than 256 tokens: gemm_tc_pair_kernel, persistent CTA pairs (cta_group::2, one MMA of 256
+// Few tiles of Q4_K and Q6_K take gemm_cut.cu where that is expected to be faster; here are the others, three
+// kernels. More than 256 tokens: gemm_tc_pair_kernel, persistent CTA pairs (cta_group::2, one MMA of 256
 // rows x 256 tokens per pair and accumulator, K streamed over the pairs). Up to 256 tokens (and the few shapes the
 // pair kernel leaves): gemm_tc_kernel, one CTA per 128-row x (NACC x BN)-token tile. At most 128 tokens of Q4_K:
 // gemm_tc_small_kernel, tokens on the MMA's M side. In all of them a dequantised weight stage is used for every
@@ -48,15 +49,18 @@ struct GemmArgs {
 // Zeroes an N x M output (row stride stride_d) or a run of tile flags for the GEMM launched behind it, whose set-up and
 // main loop overlap this kernel: released once the kernels before are done, waited for before the GEMM's first add. (A memset node in its
 // place held the GEMM back for 2 us.)
-__global__ void __launch_bounds__(256) zero_kernel(float* D, uint32_t M, uint32_t stride_d) {
+// Few rows: several tokens a CTA, 4096 floats (11264 tokens of 128 rows took 8 us with a CTA each).
+__global__ void __launch_bounds__(256) zero_kernel(float* D, uint32_t M, uint32_t N, uint32_t per, uint32_t stride_d) {
     chain_wait();
     chain_release();
-    float* d = D + (uint64_t)blockIdx.x * stride_d;
-    if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
-        for (uint32_t m = threadIdx.x * 4; m + 4 <= M; m += 1024) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (threadIdx.x < (M & 3u)) d[(M & ~3u) + threadIdx.x] = 0.f;
-    } else {
-        for (uint32_t m = threadIdx.x; m < M; m += 256) d[m] = 0.f;
+    for (uint32_t n = blockIdx.x * per; n < min(N, blockIdx.x * per + per); ++n) {
+        float* d = D + (uint64_t)n * stride_d;
+        if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+            for (uint32_t m = threadIdx.x * 4; m + 4 <= M; m += 1024) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (threadIdx.x < (M & 3u)) d[(M & ~3u) + threadIdx.x] = 0.f;
+        } else {
+            for (uint32_t m = threadIdx.x; m < M; m += 256) d[m] = 0.f;
+        }
     }
 }
 
@@ -1114,7 +1118,8 @@ cudaError_t launch_typed(const uint8_t* A, const void* B, float* D, uint32_t M, 
 
 cudaError_t launch_zero(float* D, uint32_t M, uint32_t N, uint32_t stride_d, cudaStream_t s, uint64_t* launches) {
     if (launches) ++*launches;
-    return launch_chained(zero_kernel, dim3(N), dim3(256), 0, s, D, M, stride_d);
+    const uint32_t per = M < 4096 ? 4096 / M : 1;
+    return launch_chained(zero_kernel, dim3((N + per - 1) / per), dim3(256), 0, s, D, M, N, per, stride_d);
 }
 
 cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N,
@@ -1133,6 +1138,10 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
         return e;
     }
     if (K & 255u) return cudaErrorNotSupported;
+    if (N >= 16) {
+        const cudaError_t e = launch_mul_mm_cut(type, A, B, D, M, N, K, stride_b, stride_d, status, s, launches);
+        if (e != cudaErrorNotSupported) return e;
+    }
     // Q6_K rows are 210 bytes per block: the TMA row pitch is a multiple of 16 only for K % 2048 == 0. Other K:
     // the pair kernel with the dequant threads fetching their rows (more than 256 tokens), else the caller's
     // 128-token-tile route.

@@ -320,6 +320,11 @@ cudaError_t launch_mul_mm(uint32_t type, const uint8_t* A, const void* B, float*
                           uint32_t K, uint32_t stride_b, uint32_t stride_d, bool act_bf16, uint32_t* status,
                           uint32_t* tile_flags, uint32_t n_tile_flags, cudaStream_t s, uint64_t* launches);
 
+// The same for few tiles, K cut over CTAs (gemm_cut.cu): Q4_K and Q6_K, bf16 activations. cudaErrorNotSupported: another path is faster
+// (nothing launched or written).
+cudaError_t launch_mul_mm_cut(uint32_t type, const uint8_t* A, const void* B, float* D, uint32_t M, uint32_t N, uint32_t K, uint32_t stride_b,
+                              uint32_t stride_d, uint32_t* status, cudaStream_t s, uint64_t* launches);
+
 // Prefill GEMM at f32 accuracy on the tensor cores (gemm_exact.cu): Q4_K, Q5_K, Q6_K, Q8_0, MXFP4 weights, f32 or
 // bf16 activations. `scratch`: context memory for the fp16 terms of the activations; tokens beyond what it holds go
 // in further passes. cudaErrorNotSupported: the caller takes another path (nothing launched or written).
