@@ -233,12 +233,8 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
                     const uint4 c0 = *reinterpret_cast<const uint4*>(raw + 16 + q * 32);
                     const uint4 c1 = *reinterpret_cast<const uint4*>(raw + 32 + q * 32);
                     release_after(hd.x ^ c0.x ^ c1.x, &bars->empty_w[slot], lane);
-                    const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
-                    const float d = __low2float(dd), dmin = __high2float(dd);
-                    uint32_t s0, mn0, s1, mn1;
-                    scale_min_k4(2 * q, hd.y, hd.z, hd.w, s0, mn0);
-                    scale_min_k4(2 * q + 1, hd.y, hd.z, hd.w, s1, mn1);
-                    dequant_group_q4k(c0, c1, d * (float)s0, dmin * (float)mn0, d * (float)s1, dmin * (float)mn1, put);
+                    const GroupQ4k k = group_q4k(hd, q);
+                    dequant_group_q4k(c0, c1, k.s_lo, k.m_lo, k.s_hi, k.m_hi, put);
                 } else {
                     dequant_group_q6k<4>(raw, (row_off + (uint32_t)b * 210u) & 15u, (int)q, put);
                     // words 4 k + 3 are made of every word read but the first ones of ql and qh, which word 0 is made of

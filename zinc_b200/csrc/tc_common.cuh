@@ -299,6 +299,28 @@ __device__ __forceinline__ void deq4(uint32_t nib, __nv_bfloat162 dsc, __nv_bflo
     o1 = bf2_bits(__hfma2(__hsub2(bits_bf2(p1), k136), dsc, c));
 }
 
+// The scales and mins of the 64-column group g of a Q4_K block with header hd (getScaleMinK4, src/compute/forward.zig:229-238), four
+// at a time as bytes; g is the same for the whole warp. (One by one, with their places chosen by tests: 50 instructions more of some
+// 170 a group.)
+struct GroupQ4k {
+    float s_lo, m_lo, s_hi, m_hi;   // d * scale and dmin * min of the columns 0..31 and 32..63
+};
+__device__ __forceinline__ GroupQ4k group_q4k(const uint4& hd, uint32_t g) {
+    uint32_t sc, mn;
+    if (g < 2) {
+        sc = hd.y & 0x3F3F3F3Fu;
+        mn = hd.z & 0x3F3F3F3Fu;
+    } else {
+        sc = (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u);
+        mn = ((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u);
+    }
+    sc >>= 16 * (g & 1u);
+    mn >>= 16 * (g & 1u);
+    const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
+    const float d = __low2float(dd), dmin = __high2float(dd);
+    return {d * (float)(sc & 0xFFu), dmin * (float)(mn & 0xFFu), d * (float)((sc >> 8) & 0xFFu), dmin * (float)((mn >> 8) & 0xFFu)};
+}
+
 // One 64-column group of a Q4_K row: 32 bytes of nibbles -> 8 chunks of 8 bf16, handed to put(chunk, words).
 template <typename Put>
 __device__ __forceinline__ void dequant_group_q4k(const uint4& q0, const uint4& q1, float d_sc_lo, float dm_lo,
