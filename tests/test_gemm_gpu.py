@@ -229,6 +229,31 @@ def test_mul_mm_exact(gpu, oracle, t, act, M, N, K):
         assert rel_l2(got[c], want[c]) <= (TOL_EXACT if M > 1 else 50 * TOL_EXACT)   # M = 1: one value, cancellation
 
 
+@pytest.mark.parametrize("t,act", [(zb.Q4_K, "f32"), (zb.Q5_K, "bf16"), (zb.Q6_K, "f32"), (zb.Q8_0, "bf16"), (zb.MXFP4, "f32")])
+@pytest.mark.parametrize("M,N,K", [(5000, 145, 768), (5000, 209, 768), (4400, 193, 2048), (9000, 257, 512), (9000, 481, 512),
+                                   (9000, 700, 512)])
+def test_mul_mm_exact_tile_widths(gpu, oracle, t, act, M, N, K):
+    """Tiles of 48 to 256 tokens that are no multiples of 32, of both splits of the warps (to 192 tokens and beyond), raw
+    blocks by TMA and fetched."""
+    torch, ctx, dd = gpu
+    g = synth.rng(311, t * 100 + M + N)
+    w = synth.quant_matrix(g, t, M, K)
+    X = synth.activations(g, N, K)
+    if act == "bf16":
+        bits = synth.to_bf16_bits(X)
+        Xd, X = dev(torch, bits.view(np.int16)), synth.bf16_bits_to_f32(bits)
+    else:
+        Xd = dev(torch, X)
+    D = out_with_canary(torch, N * M, init=7.0)
+    dd.recordMulMm(t, dev(torch, w), Xd, D, M, N, K, K, M, act_type=zb.BF16 if act == "bf16" else zb.F32)
+    ctx.submit_and_wait()
+    got = D[:N * M].cpu().numpy().reshape(N, M)
+    assert canary_intact(D, N * M)
+    want = oracle.gemm_f64(w, t, M, K, X)
+    for c in range(N):
+        assert rel_l2(got[c], want[c]) <= TOL_EXACT
+
+
 @pytest.mark.parametrize("t", [zb.Q4_K, zb.Q5_K], ids=["q4_k", "q5_k"])
 def test_mul_mm_exact_scale_ratios(gpu, oracle, t):
     """Blocks whose d and dmin lie far apart: d = 0, dmin = 0, dmin / d from 2^-14 to 2^17, negative scales."""

@@ -1,4 +1,6 @@
 // Preparation of the activations and dispatch of the f32-accurate prefill GEMM (gemm_exact.cuh).
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "stream_common.cuh"
@@ -6,7 +8,7 @@
 namespace zc {
 namespace {
 
-constexpr int kPrepThreads = 256;
+constexpr int kPrepMost = 1024;  // threads
 
 struct PrepArgs {
     const void* X;
@@ -67,20 +69,42 @@ __device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t h) {
 
 // One CTA per token: power-of-two scale from the largest element, fp16 terms in the order the GEMM consumes them,
 // sums over 32-column sub-blocks, and (split tiles) the token's row of D set to zero. Bound: the bytes of X, D and
-// the terms, 4 + 4 per element; 4096 x 658: 3 us.
+// the terms, 4 + 4 per element, and for few tokens the latency of one read behind the other: a thread's two chunks of a row of
+// up to 16384 columns stay in its registers between the scale and the terms (read twice, four elements at a time: 4096 columns,
+// 128 tokens
+// 5.8 us, 658 tokens with D to zero 9.0; now 4.5 and 8.1, both with L2 cold).
 template <int ORDER, bool BF16>
-__global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs a) {
+__global__ void __maxnreg__(40) exact_prep_kernel(const PrepArgs a) {
     chain_wait();
     chain_release();  // the GEMM's set-up and its first weight blocks overlap this kernel
-    __shared__ float s_max[kPrepThreads / 32];
-    const uint32_t t = blockIdx.x, tid = threadIdx.x;
+    __shared__ float s_max[kPrepMost / 32];
+    const uint32_t t = blockIdx.x, tid = threadIdx.x, threads = blockDim.x;
     const void* X = a.X;
     after_wait(X);
     const void* row = static_cast<const uint8_t*>(X) + (uint64_t)t * a.stride_b * (BF16 ? 2 : 4);
+    const uint32_t chunks = a.nblk * 32;  // eight lanes per 64-column group, whole warps
+    float4 va[2], vb[2];
+    auto load = [&](uint32_t q0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t q = q0 + i * threads;
+            uint32_t ka, kb;
+            chunk_columns<ORDER>(q & 7, ka, kb);
+            va[i] = vb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q < chunks) {
+                va[i] = load4<BF16>(row, (q >> 3) * 64 + ka, a.K, a.vec);
+                vb[i] = load4<BF16>(row, (q >> 3) * 64 + kb, a.K, a.vec);
+            }
+        }
+    };
     float mx = 0.f;
-    for (uint32_t k = tid * 4; k < a.K; k += kPrepThreads * 4) {
-        const float4 v = load4<BF16>(row, k, a.K, a.vec);
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    for (uint32_t q0 = tid; q0 < chunks; q0 += 2 * threads) {
+        load(q0);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(va[i].x), fabsf(va[i].y)), fmaxf(fabsf(va[i].z), fabsf(va[i].w))));
+            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(vb[i].x), fabsf(vb[i].y)), fmaxf(fabsf(vb[i].z), fabsf(vb[i].w))));
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
@@ -88,16 +112,16 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
     if (a.zero) {
         float* d = a.D + (uint64_t)t * a.stride_d;
         if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
-            for (uint32_t m = tid * 4; m + 4 <= a.M; m += kPrepThreads * 4) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t m = tid * 4; m + 4 <= a.M; m += threads * 4) *reinterpret_cast<float4*>(d + m) = make_float4(0.f, 0.f, 0.f, 0.f);
             if (tid < (a.M & 3u)) d[(a.M & ~3u) + tid] = 0.f;
         } else {
-            for (uint32_t m = tid; m < a.M; m += kPrepThreads) d[m] = 0.f;
+            for (uint32_t m = tid; m < a.M; m += threads) d[m] = 0.f;
         }
     }
     __syncthreads();
-    mx = s_max[0];
+    mx = s_max[tid & 31 & (threads / 32 - 1)];  // the number of warps is a power of two
 #pragma unroll
-    for (int i = 1; i < kPrepThreads / 32; ++i) mx = fmaxf(mx, s_max[i]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
     // Largest element to [2^14, 2^15), the top of fp16's range, so that an element keeps its 22 bits down to 2^-17 of the
     // largest; the inverse stays a normal number. Types with mins: their weights are 2^-10 of their value (gemm_exact.cuh),
     // and the sums are brought down to match, below 2^15 too.
@@ -109,46 +133,49 @@ __global__ void __launch_bounds__(kPrepThreads) exact_prep_kernel(const PrepArgs
     uint4* out = reinterpret_cast<uint4*>(a.x + (uint64_t)t * a.nblk * 256);
     const uint64_t low = (uint64_t)gridDim.x * a.nblk * 32;  // 16-byte chunks to the low term
     uint4* sums = reinterpret_cast<uint4*>(a.sums + (uint64_t)t * a.nblk * 64);
-    const uint32_t chunks = a.nblk * 32;
-    for (uint32_t q = tid; q < chunks; q += kPrepThreads) {  // eight lanes per 64-column group, whole warps
-        const uint32_t g = q >> 3;
-        const int c = q & 7;
-        uint32_t ka, kb;
-        chunk_columns<ORDER>(c, ka, kb);
-        float4 va = load4<BF16>(row, g * 64 + ka, a.K, a.vec), vb = load4<BF16>(row, g * 64 + kb, a.K, a.vec);
-        va = make_float4(va.x * scale, va.y * scale, va.z * scale, va.w * scale);
-        vb = make_float4(vb.x * scale, vb.y * scale, vb.z * scale, vb.w * scale);
-        uint4 hi;
-        hi.x = pack_h2(va.x, va.z);
-        hi.y = pack_h2(va.y, va.w);
-        hi.z = pack_h2(vb.x, vb.z);
-        hi.w = pack_h2(vb.y, vb.w);
-        out[q] = hi;
-        if (!BF16) {
-            uint4 lo;
-            lo.x = pack_rest(va.x, va.z, hi.x);
-            lo.y = pack_rest(va.y, va.w, hi.y);
-            lo.z = pack_rest(vb.x, vb.z, hi.z);
-            lo.w = pack_rest(vb.y, vb.w, hi.w);
-            out[low + q] = lo;
-        }
-        if (ORDER == 0 && a.sums_on) {
-            float sa = (va.x + va.y) + (va.z + va.w), sb = (vb.x + vb.y) + (vb.z + vb.w);
+    const bool held = chunks <= 2 * threads;
+    for (uint32_t q0 = tid; q0 < chunks; q0 += 2 * threads) {
+        if (!held) load(q0);
 #pragma unroll
-            for (int o = 4; o > 0; o >>= 1) {
-                sa += __shfl_xor_sync(0xFFFFFFFFu, sa, o);
-                sb += __shfl_xor_sync(0xFFFFFFFFu, sb, o);
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t q = q0 + i * threads;
+            if (q >= chunks) break;
+            const uint32_t g = q >> 3;
+            const int c = q & 7;
+            const float4 xa = make_float4(va[i].x * scale, va[i].y * scale, va[i].z * scale, va[i].w * scale);
+            const float4 xb = make_float4(vb[i].x * scale, vb[i].y * scale, vb[i].z * scale, vb[i].w * scale);
+            uint4 hi;
+            hi.x = pack_h2(xa.x, xa.z);
+            hi.y = pack_h2(xa.y, xa.w);
+            hi.z = pack_h2(xb.x, xb.z);
+            hi.w = pack_h2(xb.y, xb.w);
+            out[q] = hi;
+            if (!BF16) {
+                uint4 lo;
+                lo.x = pack_rest(xa.x, xa.z, hi.x);
+                lo.y = pack_rest(xa.y, xa.w, hi.y);
+                lo.z = pack_rest(xb.x, xb.z, hi.z);
+                lo.w = pack_rest(xb.y, xb.w, hi.w);
+                out[low + q] = lo;
             }
-            sa *= 1.f / 32.f;
-            sb *= 1.f / 32.f;
-            // a block's row: sub-block sums as [high 8][high 8][low 8][zeros 8], against the weights' min terms
-            // [high][low][high][zeros]
-            uint32_t* sp = reinterpret_cast<uint32_t*>(sums + (uint64_t)(g >> 2) * 8) + (g & 3);
-            const uint32_t h = pack_h2(sa, sb);
-            if (c == 0) sp[0] = h;
-            if (c == 1) sp[4] = h;
-            if (c == 2) sp[8] = pack_rest(sa, sb, h);
-            if (c == 3) sp[12] = 0u;
+            if (ORDER == 0 && a.sums_on) {
+                float sa = (xa.x + xa.y) + (xa.z + xa.w), sb = (xb.x + xb.y) + (xb.z + xb.w);
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) {
+                    sa += __shfl_xor_sync(0xFFFFFFFFu, sa, o);
+                    sb += __shfl_xor_sync(0xFFFFFFFFu, sb, o);
+                }
+                sa *= 1.f / 32.f;
+                sb *= 1.f / 32.f;
+                // a block's row: sub-block sums as [high 8][high 8][low 8][zeros 8], against the weights' min terms
+                // [high][low][high][zeros]
+                uint32_t* sp = reinterpret_cast<uint32_t*>(sums + (uint64_t)(g >> 2) * 8) + (g & 3);
+                const uint32_t h = pack_h2(sa, sb);
+                if (c == 0) sp[0] = h;
+                if (c == 1) sp[4] = h;
+                if (c == 2) sp[8] = pack_rest(sa, sb, h);
+                if (c == 3) sp[12] = 0u;
+            }
         }
     }
 }
@@ -157,7 +184,11 @@ template <int ORDER, bool BF16>
 cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     PrepArgs a = *static_cast<const PrepArgs*>(args);
     a.zero = zero;
-    return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(kPrepThreads), 0, s, a);
+    // a whole row in the threads' registers where there are few tokens; beyond two CTAs to an SM the second read costs less than
+    // the occupancy (10752 columns, 1268 tokens: 1024 threads 12 us, 256 3)
+    uint32_t threads = 256;
+    while (a.tokens <= 2 * 148 && threads < kPrepMost && threads < a.nblk * 16) threads *= 2;
+    return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(threads), 0, s, a);
 }
 
 // D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: eight tokens of a tile. Bound: the
@@ -224,6 +255,35 @@ bool mul_mm_exact_eligible(uint32_t type, const uint8_t* A, uint32_t M, uint32_t
     return nblk * 256 * 8 < kExactTermBytes / 64 && ((uint64_t)(M + 255) / 256) * ((N + 31) / 32) * nblk < (1u << 31);
 }
 
+// equal tiles in steps of 16 tokens (the MMA's N over a CTA pair, eight-row swizzle groups)
+static uint32_t equal_tiles(uint32_t N, uint32_t cols) { return ((N + cols - 1) / cols + 15) & ~15u; }
+
+// Tokens of a tile, at most 256. Wide tiles unpack the weights fewer times, narrow ones waste fewer columns and leave no pairs
+// idle; which of them wins depends on the shape, so every width's cost is estimated. 110 shapes (types, 96 to 2048 tokens, K to
+// 11 Ki): the widths it picks take 1 % more than the best of each shape in the mean, the widest ones 5 %.
+// 4096 x 4096, 512 tokens: 256 40.7 us, 176 42.7; 892 x 3072, 287 tokens: 96 17.2, 144 18.5.
+static uint32_t tile_width(const ExactGemm& p, uint32_t n_row_pairs, uint32_t nblk) {
+    const uint32_t least = (p.N + 255) / 256, pairs = 74;
+    uint32_t best = 0;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t cols = least; cols <= 2 * least + 4; ++cols) {
+        const uint32_t w = equal_tiles(p.N, cols), tiles = n_row_pairs * ((p.N + w - 1) / w);
+        if (best && w < 48) break;
+        const XCost c = x_cost(p, p.type == T_Q6_K || p.type == T_Q8_0, w);
+        const XDeal d = x_deal(tiles, w, nblk, pairs, c);
+        const uint64_t blocks = ((uint64_t)tiles * nblk + d.pairs - 1) / d.pairs;
+        uint64_t cost = blocks * c.block + c.epilogue;
+        if (d.groups) cost += c.epilogue;
+        else if (tiles >= pairs) cost += c.epilogue * tiles / pairs;
+        if (tiles * nblk % d.pairs != 0 || d.groups || d.per == 2) cost += c.zero;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = w;
+        }
+    }
+    return best;
+}
+
 cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaStream_t s, uint64_t* launches) {
     const uint32_t nblk = (whole.K + 255) >> 8;
     const bool min_type = whole.type == T_Q4_K || whole.type == T_Q5_K;
@@ -237,10 +297,9 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         XPlan plan{};
         plan.nblk = nblk;
         plan.n_row_pairs = (p.M + 255) / 256;
-        // equal tiles of at most 256 (fine: 128, types of two fp16 terms 64) tokens, in steps of 32 (the MMA's N over a CTA
-        // pair, eight-row swizzle groups)
-        const uint32_t widest = !p.fine ? 256 : p.type == T_Q6_K || p.type == T_Q8_0 ? 64 : 128, cols = (p.N + widest - 1) / widest;
-        plan.n_tile = ((p.N + cols - 1) / cols + 31) & ~31u;
+        // fine: the widest tiles there are (128 tokens, types of two fp16 terms 64)
+        const uint32_t widest = p.type == T_Q6_K || p.type == T_Q8_0 ? 64 : 128;
+        plan.n_tile = p.fine ? equal_tiles(p.N, (p.N + widest - 1) / widest) : tile_width(p, plan.n_row_pairs, nblk);
         plan.n_tiles = plan.n_row_pairs * ((p.N + plan.n_tile - 1) / plan.n_tile);
         uint8_t* q = scratch;
         plan.x = q;

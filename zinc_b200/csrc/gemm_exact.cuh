@@ -17,24 +17,28 @@
 //      The sub-block sums are scaled by 2^-5 and the min terms too, which with the weights' 2^-10 is the same factor; it
 //      leaves dmin / d a range of 2^15 before it no longer fits fp16, and the block's scale goes up by powers of two beyond.
 // An infinite activation makes its token's row NaN.
-// A run of columns is one accumulation in tensor memory; the producer warps then add scale * sum to f32 registers
-// ("promote") while further runs fill other accumulators. The tensor core cuts an accumulator's last bits off at every
+// A run of columns is one accumulation in tensor memory; eight warps of their own then add scale * sum to f32 registers
+// ("promote") while further runs fill other accumulators and the producer warps unpack what follows. (With both in the same
+// warps a block took the sum of the two: MXFP4 4096 x 4096, 512 tokens 53.3 us, now 39.3, Q6_K 50.0 and 46.5; Q4_K, which has
+// little to unpack and long MMAs, 39.7 and 40.7 there, 30.9 and 27.5 at 256 tokens.) The tensor core cuts an accumulator's last bits off at every
 // instruction, so the length of a run decides how far the result is from the exact one (relative L2, activations N(0, 1),
 // K = 4096):
 //   kRuns 1  a block of 256 columns: 1.8e-7 (MXFP4) to 1e-6 (Q8_0 beyond 128 tokens), where one f32 chain per output
 //            (gemm_simple_kernel) has 1.1e-6. For zc_mul_mm.
 //   kRuns 4  64 columns, their small terms first: 1.2e-7 to 1.8e-7, where f32 sums by lanes (dmmv_kernel) have 1.0e-7 to
 //            1.3e-7 and runs of a block 3.6e-7 to 1e-6. For zc_dmmv_batch, in tiles of at most 128 tokens, where a block's
-//            four accumulators fit: Q4_K 12288 x 4096, 105 tokens 37.3 us (36.7 with runs of a block). Adding a block's
-//            four runs before the registers' sum takes it to 1.4e-7 and 42 us, with the sum's roundings kept too 1.3e-7
-//            and 49 us: the runs' own roundings are what is left.
+//            four accumulators fit: Q4_K 12288 x 4096, 105 tokens 38.3 us (37 with runs of a block). Adding a block's
+//            four runs before the registers' sum takes it to 1.4e-7 and 12 % more time, with the sum's roundings kept too
+//            1.3e-7 and 30 %: the runs' own roundings are what is left.
 //
 // Persistent CTA pairs (cta_group::2, 256 weight rows per pair): tiles of 256 rows x n_tile tokens, their
 // (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over two pairs is summed with
 // atomic adds into D, which the preparation kernel zeroes; where there are three pairs or more to a tile, the parts go
 // through the scratch and are added in their order. Either way the result does not depend on timing.
-// Bound: tensor pipe (2 or 3 fp16 products per weight and token) from about 100 tokens on; below that the weight
-// bytes and the unpacking of them.
+// Bound: tensor pipe (2 or 3 fp16 products per weight and token) and the shared memory that feeds it from about 160 tokens to
+// a tile on (Q4_K, 192 tokens: 3900 cycles a block, of which 34 MMAs take 3264); below that the chain raw block -> unpacked
+// stage -> MMA, 2600 to 3000 cycles a block whatever the tokens. Around it: the preparation kernel (4.5 to 8 us), 2 us from
+// the launch to the first raw block, 2 to 4 us of epilogue.
 #pragma once
 
 #include <atomic>
@@ -45,8 +49,11 @@
 namespace zc {
 namespace {
 
-constexpr int kXThreads = 3 * 32 + 512;  // issuer, loader, spare; sixteen producer warps
-constexpr uint32_t kXBarBytes = 640;
+constexpr int kXProdWarp0 = 4, kXPromoters = 8;  // warps: issuer, the two loaders, a spare one; the producers; the promoters
+constexpr uint32_t kXBarBytes = 768;
+// Blocks whose rows' scales are kept. A producer that passes on block b's has filled block b - 1, so with two stages a set the
+// MMAs of block b - 3 are under way, which waited for the promotion of block b - 5: eight (a power of two of more than four).
+constexpr uint32_t kXScales = 8;
 
 template <int TYPE>
 struct XW;  // kTerms: fp16 terms per weight; kBlock: bytes of 256 columns; kBox: bytes a TMA box (or a fetched row) holds
@@ -89,6 +96,16 @@ struct XTile {
     // every producer set has two stages there (the room the activation slots do not need).
     static constexpr int kABuf = BN == 64 ? 2 : 1;
     static constexpr int kWSlots = 2;
+    // Producer warps. The warps that promote get the registers that the others give back (setmaxnreg); tiles beyond 192 tokens
+    // need so many there (half a tile's sums) that there is room for eight producers of two sets each, which such a tile's
+    // long MMAs leave the time for.
+    static constexpr int kProducers = BN <= 192 ? 16 : 8, kSets = 16 / kProducers, kPromWarp0 = kXProdWarp0 + kProducers;
+    static constexpr int kThreads = (kPromWarp0 + kXPromoters) * 32;
+    static constexpr int kLaunchRegs = BN <= 192 ? 72 : 96, kControlRegs = BN <= 192 ? 72 : 48, kProducerRegs = BN <= 192 ? 48 : 56,
+                         kPromoterRegs = BN <= 192 ? 120 : 160;
+    static_assert(4 * kControlRegs + kProducers * kProducerRegs + kXPromoters * kPromoterRegs <= kThreads / 32 * kLaunchRegs &&
+                      kThreads * kLaunchRegs <= 65536,
+                  "what the block was launched with");
     static constexpr uint32_t kWBytes = kBM * kRow;
     // tensor-memory columns of one accumulator, and how many of them there are
     static constexpr int kPStride = BN == 64 || kRuns == 4 ? 128 : 256, kPBufs = kRuns == 4 ? 4 : 2;
@@ -100,9 +117,9 @@ struct XTile {
     // The rest is a ring of activation slots of 64 columns of a CTA's n_tile / 2 tokens (128 bytes per token and term):
     // as many as fit (small tiles need more of them in flight), at most 16.
     static constexpr uint32_t kSmemBytes = 232448u;
-    static constexpr uint32_t kBRoom = kSmemBytes - 1024u - kXBarBytes - kBOffset;
+    static constexpr uint32_t kBRoom = (kSmemBytes - 1024u - kXBarBytes - kXScales * kBM * 4u - kBOffset) & ~1023u;
     static_assert(kBRoom >= 2 * BN * 128, "two slots of the widest tile");
-    static constexpr uint32_t kBarOffset = kBOffset + kBRoom;
+    static constexpr uint32_t kScaleOffset = kBOffset + kBRoom, kBarOffset = kScaleOffset + kXScales * kBM * 4u;
 };
 
 struct XBars {
@@ -111,6 +128,7 @@ struct XBars {
     uint64_t full_w[2], empty_w[2];
     uint64_t full_b[16], empty_b[16];
     uint64_t accum[4], pfree[4];
+    uint64_t scales[kXScales];
     uint32_t tmem_base;
     volatile uint32_t failed;
 };
@@ -123,7 +141,7 @@ struct XArgs {
     const float* inv_scale;   // [N]: 1 / the token's power of two
     uint32_t M, N, K, nblk;
     uint32_t stride_d;
-    uint32_t n_row_pairs, n_tiles, n_tile;  // n_tile tokens per tile (a multiple of 32)
+    uint32_t n_row_pairs, n_tiles, n_tile;  // n_tile tokens per tile (a multiple of 16)
     uint32_t groups;          // > 0: the pairs form groups, each with one pair more than it has tiles
     float* parts;             // null, or [pair][token of the tile][256 rows]: every pair has a part of one tile
     uint32_t terms;           // fp16 terms of an activation: 2 (f32) or 1 (bf16)
@@ -302,8 +320,14 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
                  : "memory");
 }
 
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float2* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "f"(v[0].x), "f"(v[0].y),
+                 "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y)
+                 : "memory");
+}
+
 template <int TYPE, int BN, bool kFetch, int kRuns>
-__global__ void __launch_bounds__(kXThreads, 1)
+__global__ void __launch_bounds__(XTile<TYPE, BN, kFetch, kRuns>::kThreads, 1)
 gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_m,
                   const __grid_constant__ CUtensorMap tmap_w, const XArgs g) {
     using T = XTile<TYPE, BN, kFetch, kRuns>;
@@ -344,15 +368,16 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             mbar_init(&bars->empty_b[s], 1);
         }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&bars->full_w[s], kFetch ? 512 : 1);
-            mbar_init(&bars->empty_w[s], 16);
-            mbar_init(&bars->full_m[s], 32);
+            mbar_init(&bars->full_w[s], kFetch ? T::kProducers * 32 : 1);
+            mbar_init(&bars->empty_w[s], T::kProducers);
+            mbar_init(&bars->full_m[s], 2 * T::kProducers);
             mbar_init(&bars->empty_m[s], 1);
         }
         for (int s = 0; s < T::kPBufs; ++s) {
             mbar_init(&bars->accum[s], 1);
-            mbar_init(&bars->pfree[s], 32);  // the sixteen producer warps of both CTAs
+            mbar_init(&bars->pfree[s], 2 * kXPromoters);  // of both CTAs
         }
+        for (uint32_t s = 0; s < kXScales; ++s) mbar_init(&bars->scales[s], 4);  // the producer warps that have them
         bars->failed = 0;
         mbar_fence_init();
     }
@@ -368,6 +393,9 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
 
+    if constexpr (T::kControlRegs < T::kLaunchRegs) {
+        if (warp < kXProdWarp0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T::kControlRegs));
+    }
     if (warp == 0) {
         if (rank == 0) {
             // ---- MMA issuer (even CTA). Two-term activations: up to 128 tokens the terms lie side by side on the MMA's
@@ -544,9 +572,10 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (__any_sync(0xFFFFFFFFu, go)) {
                 idle = 0;
             } else {  // bounded like every other wait
+                __nanosleep(40);  // the unpacking warps' stores go through the same pipe as polls (1 %)
                 ++idle;
                 if ((idle & 255u) == 255u && __any_sync(0xFFFFFFFFu, bars->failed != 0)) break;
-                if (idle >= 16u * kWaitLimit) {
+                if (idle >= 4u * kWaitLimit) {
                     bars->failed = 1;
                     if (g.status) {
                         g.status[0] = 1;
@@ -576,25 +605,25 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 }
             }
         }
-    } else if (warp >= 3) {
-        // ---- producers: thread = (row, set); the row is the tensor-memory lane the thread promotes, so that a row's
-        // block scale stays in its registers. One-term types: set j owns columns 64 j .. of a block. Two-term types:
-        // columns 32 j .. and 128 + 32 j .., one after the other. ----
-        const int j = (warp - 3) >> 2, row = (warp & 3) * 32 + lane;
-        const bool merged = kRuns == 1 && g.terms == 2 && g.n_tile <= 128;
-        const uint32_t full_a0 = leader_addr(&bars->full_a[j * T::kABuf]);
-        const uint32_t pfree0 = leader_addr(&bars->pfree[0]);
+    } else if (warp >= kXProdWarp0 && warp < T::kPromWarp0) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(T::kProducerRegs));
+        // ---- producers: thread = (row, set j0 or the sets j0 and j0 + 2). One-term types: set j holds columns 64 j .. of a block.
+        // Two-term types: columns 32 j .. and 128 + 32 j .., one after the other. ----
+        constexpr int kSets = T::kSets, kStep = 4 / kSets;
+        const int j0 = (warp - kXProdWarp0) >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t full_a0 = leader_addr(&bars->full_a[j0 * T::kABuf]);
         const uint32_t full_m = kMin ? leader_addr(&bars->full_m[0]) : 0u;
+        float* const scales = reinterpret_cast<float*>(smem + T::kScaleOffset) + row;
         const uint64_t pitch = TYPE == T_Q8_0 || TYPE == T_MXFP4 ? (uint64_t)(g.K >> 5) * (kBlock / 8) : (uint64_t)(g.K >> 8) * kBlock;
         auto row_off = [&](uint32_t tile) {  // rows past M: computed, dropped
             return (uint64_t)min(tile_m0(tile) + (uint32_t)row, g.M - 1) * pitch;
         };
         if constexpr (kMin) {  // columns 24..31 of the min step are zeros
-            if (j < 2)
-                *reinterpret_cast<uint4*>(smem + T::kMinOffset + j * T::kMinBytes + row * 64 + ((3 ^ ((row >> 1) & 3)) << 4)) =
+            if (j0 < 2)
+                *reinterpret_cast<uint4*>(smem + T::kMinOffset + j0 * T::kMinBytes + row * 64 + ((3 ^ ((row >> 1) & 3)) << 4)) =
                     make_uint4(0, 0, 0, 0);
         }
-        // fetched rows: the 16-byte pieces of the aligned supersets of the 128 rows' blocks, dealt to the 512 threads row by
+        // fetched rows: the 16-byte pieces of the aligned supersets of the 128 rows' blocks, dealt to the threads row by
         // row (a warp's copy instruction then meets a handful of cache lines instead of 32)
         uint32_t uf = u_begin, f_b = 0, f_pw = 1;
         int f_sw = 0;
@@ -606,13 +635,13 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (!f_live) return true;
             if (!poll_or_fail(&bars->empty_w[f_sw], f_pw, bars, g.status, 186)) return false;
             uint8_t* dst = smem_w + f_sw * T::kWBytes;
-            constexpr int kPieces = (kBlock + 15 + 15) / 16;
+            constexpr int kPieces = (kBlock + 15 + 15) / 16, kFetchers = T::kProducers * 32;
             static_assert(!kFetch || kPieces * 16 <= (int)kRow, "a fetched row fits its slot");
-            const uint32_t pi = (uint32_t)tid - 96;
+            const uint32_t pi = (uint32_t)tid - kXProdWarp0 * 32;
 #pragma unroll
-            for (int i = 0; i < (kBM * kPieces + 511) / 512; ++i) {
-                const uint32_t idx = pi + 512u * i, r = idx / kPieces, piece = idx - r * kPieces;
-                if ((kBM * kPieces) % 512 == 0 || r < (uint32_t)kBM) {
+            for (int i = 0; i < (kBM * kPieces + kFetchers - 1) / kFetchers; ++i) {
+                const uint32_t idx = pi + (uint32_t)kFetchers * i, r = idx / kPieces, piece = idx - r * kPieces;
+                if ((kBM * kPieces) % kFetchers == 0 || r < (uint32_t)kBM) {
                     const uint64_t o = (uint64_t)min(f_m0 + r, g.M - 1) * pitch + (uint64_t)f_b * kBlock;
                     const uint8_t* sp = g.A + (o & ~(uint64_t)15) + piece * 16;
                     const uint32_t n = sp + 16 <= g.a_end ? 16u : (sp < g.a_end ? (uint32_t)(g.a_end - sp) : 0u);
@@ -636,75 +665,79 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             if (f_live) f_m0 = tile_m0(f_seg.tile);
             ok = fetch();
         }
-        float2 acc[BN / 8];
-#pragma unroll
-        for (int i = 0; i < BN / 8; ++i) acc[i] = make_float2(0.f, 0.f);
-        const uint32_t n8 = g.n_tile >> 5;  // groups of 8 columns this set promotes: columns (n_tile / 4) j ..
-        const uint32_t lane_base = ((uint32_t)(warp & 3) * 32u) << 16;
-        uint32_t u = u_begin;
-        XSegment sg{0, 0, 0}, old{0, 0, 0};
+        uint32_t u = u_begin, b = 0;
+        XSegment sg{0, 0, 0};
         const uint32_t total = u_end - u_begin;
-        float s_prev = 0.f;
-        uint32_t b = 0;
-        bool fresh = true;
-        for (uint32_t gb = 0; gb <= total && ok; ++gb) {
-            float s_cur = 0.f;
-            const bool boundary = gb > 0 && (gb == total || b == sg.b1);  // the block before this one ended its segment
-            if (boundary) old = sg;
-            if (gb < total) {
-                if (fresh || b == sg.b1) {
-                    x_next_segment(u, u_end, nblk, sg);
-                    b = sg.b0;
-                    fresh = false;
-                    if constexpr (kFetch) c_off = row_off(sg.tile);
+        // the scale of the row's block, for the warps that promote
+        auto pass_on = [&](uint32_t gb, float sc) {
+            if (j0 == 0) {
+                scales[(gb & (kXScales - 1)) * kBM] = sc;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->scales[gb & (kXScales - 1)]);
+            }
+        };
+        for (uint32_t gb = 0; gb < total && ok; ++gb, ++b) {
+            if (gb == 0 || b == sg.b1) {
+                x_next_segment(u, u_end, nblk, sg);
+                b = sg.b0;
+                if constexpr (kFetch) c_off = row_off(sg.tile);
+            }
+            const int sw = gb & 1;
+            if (!poll_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 187)) break;
+            if constexpr (kFetch) {
+                if (!fetch()) break;  // the next block, into the slot the previous one left
+            }
+            const uint8_t* wp = smem_w + sw * T::kWBytes + row * kRow;
+            const uint32_t off = kFetch ? (uint32_t)((c_off + (uint64_t)b * kBlock) & 15u) : (b * kBlock) & 15u;
+            // one-term types: fill number gb of a set, two-term types: 2 gb and 2 gb + 1
+            const int ab = T::kABuf == 1 ? 0 : (int)(gb & 1);
+            const uint32_t pa = ((gb / T::kABuf) & 1) ^ 1;
+            float s_cur;
+            if constexpr (kMin) {  // Q4_K / Q5_K rows and blocks are multiples of 16 bytes: off = 0
+                const uint4 hd = *reinterpret_cast<const uint4*>(wp);
+                uint4 c[2 * kSets];
+                uint32_t read = hd.x;
+#pragma unroll
+                for (int e = 0; e < kSets; ++e) {
+                    c[2 * e] = *reinterpret_cast<const uint4*>(wp + kBlock - 128 + (j0 + kStep * e) * 32);
+                    c[2 * e + 1] = *reinterpret_cast<const uint4*>(wp + kBlock - 112 + (j0 + kStep * e) * 32);
+                    read ^= c[2 * e].x ^ c[2 * e + 1].x;
                 }
-                const int sw = gb & 1;
-                if (!poll_or_fail(&bars->full_w[sw], (gb >> 1) & 1, bars, g.status, 187)) break;
-                if constexpr (kFetch) {
-                    if (!fetch()) break;  // the next block, into the slot the previous one left
+                uint4 h0 = c[0], h1 = c[1];
+                if constexpr (TYPE == T_Q5_K) {
+                    h0 = *reinterpret_cast<const uint4*>(wp + 16);
+                    h1 = *reinterpret_cast<const uint4*>(wp + 32);
                 }
-                const uint8_t* wp = smem_w + sw * T::kWBytes + row * kRow;
-                const uint32_t off = kFetch ? (uint32_t)((c_off + (uint64_t)b * kBlock) & 15u) : (b * kBlock) & 15u;
-                // one-term types: fill number gb of the set, two-term types: 2 gb and 2 gb + 1
-                const int ab = T::kABuf == 1 ? 0 : (int)(gb & 1);
-                uint8_t* stage = smem + (j * T::kABuf + ab) * kABytes;
-                uint64_t* empty_a = &bars->empty_a[j * T::kABuf + ab];
-                const uint32_t pa = ((gb / T::kABuf) & 1) ^ 1;
-                const uint32_t full_a = full_a0 + ab * 8;
-                if constexpr (kMin) {  // Q4_K / Q5_K rows and blocks are multiples of 16 bytes: off = 0
-                    const uint4 hd = *reinterpret_cast<const uint4*>(wp);
-                    const uint4 c0 = *reinterpret_cast<const uint4*>(wp + kBlock - 128 + j * 32);
-                    const uint4 c1 = *reinterpret_cast<const uint4*>(wp + kBlock - 112 + j * 32);
-                    uint4 h0 = c0, h1 = c1;
-                    if constexpr (TYPE == T_Q5_K) {
-                        h0 = *reinterpret_cast<const uint4*>(wp + 16);
-                        h1 = *reinterpret_cast<const uint4*>(wp + 32);
+                release_after(read ^ h0.y ^ h1.y, &bars->empty_w[sw], lane);
+                const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
+                const float d = __low2float(dd), dmin = __high2float(dd);
+                // The block's scale is d; where dmin is more than 2^15 of it (and there are mins at all), d times the
+                // power of two that brings the ratio to [2^14, 2^15): the q terms go down by as much, exactly as far
+                // as fp16 reaches (a ratio of 2^25) and beyond that to 2^-29 of a min term.
+                float ratio = 0.f, q_scale = 1.f / 1024.f;
+                bool mins = true;
+                s_cur = d;
+                if (fabsf(dmin) > 32768.f * fabsf(d)) {
+                    mins = (hd.z | (hd.w & 0xF0F0F0F0u)) != 0u;
+                    if (mins && d == 0.f) {
+                        s_cur = dmin * (1.f / 32768.f);
+                        q_scale = 0.f;
+                    } else if (mins) {
+                        const uint32_t e = __float_as_uint(__fdividef(fabsf(dmin), fabsf(d))) >> 23;
+                        s_cur = d * __uint_as_float((e - 14u) << 23);
+                        q_scale = __uint_as_float((258u - e) << 23);
                     }
-                    release_after(hd.x ^ c0.x ^ c1.x ^ h0.y ^ h1.y, &bars->empty_w[sw], lane);
-                    const __half2 dd = *reinterpret_cast<const __half2*>(&hd.x);
-                    const float d = __low2float(dd), dmin = __high2float(dd);
-                    // The block's scale is d; where dmin is more than 2^15 of it (and there are mins at all), d times the
-                    // power of two that brings the ratio to [2^14, 2^15): the q terms go down by as much, exactly as far
-                    // as fp16 reaches (a ratio of 2^25) and beyond that to 2^-29 of a min term.
-                    float ratio = 0.f, q_scale = 1.f / 1024.f;
-                    bool mins = true;
-                    s_cur = d;
-                    if (fabsf(dmin) > 32768.f * fabsf(d)) {
-                        mins = (hd.z | (hd.w & 0xF0F0F0F0u)) != 0u;
-                        if (mins && d == 0.f) {
-                            s_cur = dmin * (1.f / 32768.f);
-                            q_scale = 0.f;
-                        } else if (mins) {
-                            const uint32_t e = __float_as_uint(__fdividef(fabsf(dmin), fabsf(d))) >> 23;
-                            s_cur = d * __uint_as_float((e - 14u) << 23);
-                            q_scale = __uint_as_float((258u - e) << 23);
-                        }
-                    }
-                    if (mins && s_cur != 0.f) {  // dmin / s_cur: an approximate reciprocal and a Newton step
-                        const float r = __fdividef(1.f, s_cur);
-                        ratio = dmin * fmaf(fmaf(-s_cur, r, 1.f), r, r);
-                    }
-                    ratio *= -1.f / 32.f;
+                }
+                if (mins && s_cur != 0.f) {  // dmin / s_cur: an approximate reciprocal and a Newton step
+                    const float r = __fdividef(1.f, s_cur);
+                    ratio = dmin * fmaf(fmaf(-s_cur, r, 1.f), r, r);
+                }
+                ratio *= -1.f / 32.f;
+                pass_on(gb, s_cur);
+                uint32_t vh[kSets], vl[kSets];
+#pragma unroll
+                for (int e = 0; e < kSets; ++e) {
+                    const int j = j0 + kStep * e;
                     // the 6-bit scales and mins of sub-blocks 2j and 2j + 1 (getScaleMinK4, src/compute/forward.zig:229-238),
                     // four at a time as bytes
                     uint32_t scw, mnw;
@@ -718,167 +751,224 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                     scw >>= 16 * (j & 1);
                     mnw >>= 16 * (j & 1);
                     const uint32_t s0 = scw & 0xFFu, s1 = (scw >> 8) & 0xFFu, mn0 = mnw & 0xFFu, mn1 = (mnw >> 8) & 0xFFu;
-                    const uint32_t w[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-                    const uint32_t h[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    if (!poll_or_fail(empty_a, pa, bars, g.status, 188)) break;
-                    x_deq_k4<TYPE == T_Q5_K>(w, h, j, q_scale * (float)s0, q_scale * (float)s1, stage, row);
+                    const uint32_t w[8] = {c[2 * e].x, c[2 * e].y, c[2 * e].z, c[2 * e].w, c[2 * e + 1].x, c[2 * e + 1].y, c[2 * e + 1].z, c[2 * e + 1].w};
+                    const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                    if (!poll_or_fail(&bars->empty_a[j0 * T::kABuf + kStep * e * T::kABuf + ab], pa, bars, g.status, 188)) { ok = false; break; }
+                    x_deq_k4<TYPE == T_Q5_K>(w, hw, j, q_scale * (float)s0, q_scale * (float)s1, smem + (j0 * T::kABuf + kStep * e * T::kABuf + ab) * kABytes, row);
                     const float v0 = ratio * (float)mn0, v1 = ratio * (float)mn1;
-                    const __half2 vh = __floats2half2_rn(v0, v1);
-                    const __half2 vl = __floats2half2_rn(v0 - __low2float(vh), v1 - __high2float(vh));
-                    if (!poll_or_fail(&bars->empty_m[gb & 1], ((gb >> 1) & 1) ^ 1, bars, g.status, 189)) break;
-                    // chunks 0, 1, 2: high, low, high terms
-                    uint8_t* mp = smem + T::kMinOffset + (gb & 1) * T::kMinBytes + row * 64 + 4 * j;
-                    const int x = (row >> 1) & 3;
-                    *reinterpret_cast<uint32_t*>(mp + ((0 ^ x) << 4)) = h2_bits(vh);
-                    *reinterpret_cast<uint32_t*>(mp + ((1 ^ x) << 4)) = h2_bits(vl);
-                    *reinterpret_cast<uint32_t*>(mp + ((2 ^ x) << 4)) = h2_bits(vh);
+                    const __half2 hi = __floats2half2_rn(v0, v1);
+                    vh[e] = h2_bits(hi);
+                    vl[e] = h2_bits(__floats2half2_rn(v0 - __low2float(hi), v1 - __high2float(hi)));
                     fence_proxy_async();
                     __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive_cluster(full_a);
-                        mbar_arrive_cluster(full_m + (gb & 1) * 8);
-                    }
-                } else if constexpr (TYPE == T_MXFP4) {
-                    uint32_t emax = 0;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (8 * b + i < (g.K >> 5)) emax = max(emax, (uint32_t)wp[off + 17 * i]);
-                    s_cur = e8m0_to_f32(emax);
-                    uint32_t q[2][4], read = emax;  // every word read: nibbles, the block's scales, this set's own
-                    __half2 sc[2];
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const uint32_t o = off + 17u * (2 * j + i), e = wp[o];
-                        const int diff = (int)emax - (int)e;
-                        lds_words<4>(wp + ((o + 1) & ~15u), (o + 1) & 15u, q[i]);
-                        read ^= e ^ q[i][0] ^ q[i][3];
-                        const bool live = 8 * b + 2 * j + i < (g.K >> 5);
-                        sc[i] = __float2half2_rn(live && diff < 60 ? __uint_as_float((uint32_t)(127 + 14 - diff) << 23) : 0.f);
-                        if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
-                    }
-                    release_after(read, &bars->empty_w[sw], lane);
-                    if (!poll_or_fail(empty_a, pa, bars, g.status, 188)) break;
-                    x_deq_mx(q[0], sc[0], 0, stage, row);
-                    x_deq_mx(q[1], sc[1], 4, stage, row);
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(full_a);
-                } else {
-                    float up = 1.f;  // Q8_0: 1 / s_cur, a power of two
-                    if constexpr (TYPE == T_Q8_0) {
-                        uint32_t top = 0;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (8 * b + i < (g.K >> 5)) top = max(top, (uint32_t)*reinterpret_cast<const unsigned short*>(wp + off + 34 * i) & 0x7FFFu);
-                        const uint32_t e = __float_as_uint(h2f(top)) >> 23;  // f32 exponent of the largest |d|
-                        s_cur = __uint_as_float(e << 23);
-                        up = e ? __uint_as_float((254u - e) << 23) : 0.f;
-                    } else {
-                        s_cur = h2f(*reinterpret_cast<const unsigned short*>(wp + off + 208));
-                    }
-#pragma unroll
-                    for (int hf = 0; hf < 2; ++hf) {
-                        const int gg = j + 4 * hf;
-                        // two stages: fill hf goes to stage hf, once a block
-                        const int ab2 = T::kABuf == 1 ? 0 : hf;
-                        uint8_t* stage2 = smem + (j * T::kABuf + ab2) * kABytes;
-                        const uint32_t pa2 = T::kABuf == 1 ? (uint32_t)hf ^ 1u : (gb & 1) ^ 1u;
-                        if (!poll_or_fail(&bars->empty_a[j * T::kABuf + ab2], pa2, bars, g.status, 188)) { ok = false; break; }
-                        if constexpr (TYPE == T_Q6_K) {
-                            x_deq_q6k(wp, off, gg, stage2, row);
-                        } else if (8 * b + gg < (g.K >> 5)) {
-                            const uint32_t o = off + 34u * gg;
-                            x_deq_q8(wp, o + 2, h2f(*reinterpret_cast<const unsigned short*>(wp + o)) * up, stage2, row);
-                        } else {  // past K
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage2 + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
-                        }
-                        // the weights and their scales are in the stores above; the block's scale is in nothing yet
-                        if (hf == 1) release_after(__float_as_uint(s_cur), &bars->empty_w[sw], lane);
-                        fence_proxy_async();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(full_a0 + ab2 * 8);
-                    }
-                    if (!ok) break;
-                }
-                ++b;
-            }
-            if (gb > 0) {
-                // ---- promote the previous block: registers += its scale x its sums ----
-                const uint32_t pv = gb - 1;
-#pragma unroll 1
-                for (int r = 0; r < kRuns && ok; ++r) {
-                    const uint32_t buf = kRuns == 4 ? (uint32_t)r : pv & 1;
-                    ok = poll_or_fail(&bars->accum[buf], (kRuns == 4 ? pv : pv >> 1) & 1, bars, g.status, 190);
-                    if (!ok) break;
-                    __syncwarp();
-                    tc_fence_after();
-                    // columns of this set's tokens; merged: those of their low terms n_tile / 2 further on (either CTA's
-                    // tokens are [high | low] there)
-                    const uint32_t q4 = g.n_tile >> 2;
-                    const uint32_t ta = tmem + lane_base + buf * T::kPStride + (merged ? (j >> 1) * g.n_tile + (j & 1) * q4 : j * q4);
-                    if (BN <= 128 && merged) {
-#pragma unroll
-                        for (int c = 0; c < BN / 32; ++c) {
-                            if ((uint32_t)c < n8) {
-                                uint32_t v0[8], v1[8];
-                                tmem_ld8(ta + c * 8, v0);
-                                tmem_ld8(ta + c * 8 + 2 * q4, v1);
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int e = 0; e < 8; e += 2)
-                                    fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v0[e]) + __uint_as_float(v1[e]),
-                                              __uint_as_float(v0[e + 1]) + __uint_as_float(v1[e + 1]));
-                            }
-                        }
-                    } else {  // pairs of groups; the second of the last pair may lie past the set's columns (read, not used)
-#pragma unroll
-                        for (int c = 0; c < BN / 32; c += 2) {
-                            if ((uint32_t)c < n8) {
-                                uint32_t v[16];
-                                tmem_ld16(ta + c * 8, v);
-                                tmem_ld_wait();
-#pragma unroll
-                                for (int e = 0; e < 16; e += 2)
-                                    fma_f32x2(acc[c * 4 + e / 2], s_prev, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-                            }
-                        }
-                    }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(pfree0 + buf * 8);
+                    if (lane == 0) mbar_arrive_cluster(full_a0 + (kStep * e * T::kABuf + ab) * 8);
                 }
                 if (!ok) break;
-                if (boundary) {
-                    // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D or wait in
-                    // their slots for add_parts_kernel ----
-                    asm volatile("griddepcontrol.wait;" ::: "memory");  // D zeroed, scales written
-                    const bool whole = old.b0 == 0 && old.b1 == nblk;
-                    const uint32_t m = tile_m0(old.tile) + row;
-                    const uint32_t n0 = tile_n0(old.tile) + j * (g.n_tile >> 2);
-                    float* out = g.parts ? g.parts + ((uint64_t)slot * g.n_tile + j * (g.n_tile >> 2)) * 256 + rank * kBM + row
-                                         : g.D + (uint64_t)n0 * g.stride_d + m;
-                    const uint32_t out_stride = g.parts ? 256u : g.stride_d;
-                    // the tokens' scales, one per lane (a load per column would be held back by the add before it)
-                    float inv0 = 0.f, inv1 = 0.f;
-                    if ((uint32_t)lane < n8 * 8 && n0 + lane < g.N) inv0 = __ldcg(g.inv_scale + n0 + lane);
-                    if (BN > 128 && 32u + lane < n8 * 8 && n0 + 32 + lane < g.N) inv1 = __ldcg(g.inv_scale + n0 + 32 + lane);
+                if (!poll_or_fail(&bars->empty_m[gb & 1], ((gb >> 1) & 1) ^ 1, bars, g.status, 189)) break;
+                // chunks 0, 1, 2: high, low, high terms
+                uint8_t* mp = smem + T::kMinOffset + (gb & 1) * T::kMinBytes + row * 64 + 4 * j0;
+                const int x = (row >> 1) & 3;
 #pragma unroll
-                    for (int c = 0; c < BN / 4; ++c) {
-                        const uint32_t n = n0 + c;
-                        const float inv = __shfl_sync(0xFFFFFFFFu, c < 32 ? inv0 : inv1, c & 31);
-                        if ((uint32_t)c < n8 * 8 && n < g.N && m < g.M) {
-                            const float v = ((c & 1) ? acc[c / 2].y : acc[c / 2].x) * inv;
-                            float* dst = out + (uint64_t)c * out_stride;
-                            if (whole || g.parts) *dst = v;
-                            else atomicAdd(dst, v);
+                for (int e = 0; e < kSets; ++e) {
+                    *reinterpret_cast<uint32_t*>(mp + 8 * e + ((0 ^ x) << 4)) = vh[e];
+                    *reinterpret_cast<uint32_t*>(mp + 8 * e + ((1 ^ x) << 4)) = vl[e];
+                    *reinterpret_cast<uint32_t*>(mp + 8 * e + ((2 ^ x) << 4)) = vh[e];
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(full_m + (gb & 1) * 8);
+            } else if constexpr (TYPE == T_MXFP4) {
+                uint32_t emax = 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (8 * b + i < (g.K >> 5)) emax = max(emax, (uint32_t)wp[off + 17 * i]);
+                s_cur = e8m0_to_f32(emax);
+                pass_on(gb, s_cur);
+                uint32_t q[2 * kSets][4], read = emax;  // every word read: nibbles, the block's scales, these sets' own
+                __half2 sc[2 * kSets];
+#pragma unroll
+                for (int i = 0; i < 2 * kSets; ++i) {
+                    const int blk = 2 * (j0 + kStep * (i >> 1)) + (i & 1);
+                    const uint32_t o = off + 17u * blk, e = wp[o];
+                    const int diff = (int)emax - (int)e;
+                    lds_words<4>(wp + ((o + 1) & ~15u), (o + 1) & 15u, q[i]);
+                    read ^= e ^ q[i][0] ^ q[i][3];
+                    const bool live = 8 * b + blk < (g.K >> 5);
+                    sc[i] = __float2half2_rn(live && diff < 60 ? __uint_as_float((uint32_t)(127 + 14 - diff) << 23) : 0.f);
+                    if (!live) q[i][0] = q[i][1] = q[i][2] = q[i][3] = 0u;
+                }
+                release_after(read, &bars->empty_w[sw], lane);
+#pragma unroll
+                for (int e = 0; e < kSets; ++e) {
+                    uint8_t* stage = smem + (j0 * T::kABuf + kStep * e * T::kABuf + ab) * kABytes;
+                    if (!poll_or_fail(&bars->empty_a[j0 * T::kABuf + kStep * e * T::kABuf + ab], pa, bars, g.status, 188)) { ok = false; break; }
+                    x_deq_mx(q[2 * e], sc[2 * e], 0, stage, row);
+                    x_deq_mx(q[2 * e + 1], sc[2 * e + 1], 4, stage, row);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(full_a0 + (kStep * e * T::kABuf + ab) * 8);
+                }
+            } else {
+                float up = 1.f;  // Q8_0: 1 / s_cur, a power of two
+                if constexpr (TYPE == T_Q8_0) {
+                    uint32_t top = 0;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (8 * b + i < (g.K >> 5)) top = max(top, (uint32_t)*reinterpret_cast<const unsigned short*>(wp + off + 34 * i) & 0x7FFFu);
+                    const uint32_t e = __float_as_uint(h2f(top)) >> 23;  // f32 exponent of the largest |d|
+                    s_cur = __uint_as_float(e << 23);
+                    up = e ? __uint_as_float((254u - e) << 23) : 0.f;
+                } else {
+                    s_cur = h2f(*reinterpret_cast<const unsigned short*>(wp + off + 208));
+                }
+                pass_on(gb, s_cur);
+#pragma unroll
+                for (int f = 0; f < 2 * kSets; ++f) {  // in the order in which the issuer takes them: the second halves last
+                    const int hf = f / kSets, st = kStep * (f % kSets), gg = j0 + st + 4 * hf;
+                    // two stages: fill hf goes to stage hf, once a block
+                    const int ab2 = T::kABuf == 1 ? 0 : hf;
+                    uint8_t* stage2 = smem + (j0 * T::kABuf + st * T::kABuf + ab2) * kABytes;
+                    const uint32_t pa2 = T::kABuf == 1 ? (uint32_t)hf ^ 1u : (gb & 1) ^ 1u;
+                    if (!poll_or_fail(&bars->empty_a[j0 * T::kABuf + st * T::kABuf + ab2], pa2, bars, g.status, 188)) { ok = false; break; }
+                    if constexpr (TYPE == T_Q6_K) {
+                        x_deq_q6k(wp, off, gg, stage2, row);
+                    } else if (8 * b + gg < (g.K >> 5)) {
+                        const uint32_t o = off + 34u * gg;
+                        x_deq_q8(wp, o + 2, h2f(*reinterpret_cast<const unsigned short*>(wp + o)) * up, stage2, row);
+                    } else {  // past K
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(stage2 + row * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+                    }
+                    // the weights and their scales are in the stores above; the block's scale is in nothing yet
+                    if (f == 2 * kSets - 1) release_after(__float_as_uint(s_cur), &bars->empty_w[sw], lane);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(full_a0 + (st * T::kABuf + ab2) * 8);
+                }
+                if (!ok) break;
+            }
+        }
+    } else if (warp >= T::kPromWarp0) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(T::kPromoterRegs));
+        // ---- promoters: thread = (row, half of the tile's tokens): registers += the row's scale x the runs' sums ----
+        const int hp = (warp - T::kPromWarp0) >> 2, row = (warp & 3) * 32 + lane;
+        const bool merged = kRuns == 1 && g.terms == 2 && g.n_tile <= 128;
+        const uint32_t pfree0 = leader_addr(&bars->pfree[0]), half = g.n_tile / 2;
+        const float* const scales = reinterpret_cast<const float*>(smem + T::kScaleOffset) + row;
+        const uint32_t lane_base = ((uint32_t)(warp & 3) * 32u) << 16;
+        float2 acc[BN / 4];
+#pragma unroll
+        for (int i = 0; i < BN / 4; ++i) acc[i] = make_float2(0.f, 0.f);
+        uint32_t u = u_begin, b = 0;
+        XSegment sg{0, 0, 0};
+        const uint32_t total = u_end - u_begin;
+        bool ok = true;
+        for (uint32_t gb = 0; gb < total && ok; ++gb) {
+            if (gb == 0 || b == sg.b1) {
+                x_next_segment(u, u_end, nblk, sg);
+                b = sg.b0;
+            }
+            if (!poll_or_fail(&bars->scales[gb & (kXScales - 1)], (gb / kXScales) & 1, bars, g.status, 192)) break;
+            const float sc = scales[(gb & (kXScales - 1)) * kBM];
+#pragma unroll 1
+            for (int r = 0; r < kRuns && ok; ++r) {
+                const uint32_t buf = kRuns == 4 ? (uint32_t)r : gb & 1;
+                ok = poll_or_fail(&bars->accum[buf], (kRuns == 4 ? gb : gb >> 1) & 1, bars, g.status, 190);
+                if (!ok) break;
+                __syncwarp();
+                tc_fence_after();
+                // columns of these tokens; merged: those of their low terms n_tile / 2 further on (either CTA's
+                // tokens are [high | low] there)
+                const uint32_t ta = tmem + lane_base + buf * T::kPStride + (merged ? hp * g.n_tile : hp * half);
+                if (BN <= 128 && merged) {
+#pragma unroll
+                    for (int c = 0; c < BN / 32; ++c) {
+                        if ((uint32_t)c * 16 < half) {
+                            uint32_t v0[16], v1[16];
+                            tmem_ld16(ta + c * 16, v0);
+                            tmem_ld16(ta + c * 16 + half, v1);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < 16; e += 2)
+                                fma_f32x2(acc[c * 8 + e / 2], sc, __uint_as_float(v0[e]) + __uint_as_float(v1[e]),
+                                          __uint_as_float(v0[e + 1]) + __uint_as_float(v1[e + 1]));
                         }
                     }
+                } else {  // pairs of loads where the registers allow it: a load's latency is what a run's promotion consists of
+                    constexpr int kLoads = BN <= 128 ? 2 : 1;
 #pragma unroll
-                    for (int c = 0; c < BN / 8; ++c) acc[c] = make_float2(0.f, 0.f);
+                    for (int c = 0; c < BN / 32; c += kLoads) {
+                        if ((uint32_t)c * 16 < half) {
+                            uint32_t v[kLoads][16];
+#pragma unroll
+                            for (int l = 0; l < kLoads; ++l) tmem_ld16(ta + (c + l) * 16, v[l]);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int l = 0; l < kLoads; ++l)
+#pragma unroll
+                                for (int e = 0; e < 16; e += 2)
+                                    fma_f32x2(acc[(c + l) * 8 + e / 2], sc, __uint_as_float(v[l][e]), __uint_as_float(v[l][e + 1]));
+                        }
+                    }
                 }
+                if (r == kRuns - 1 && b + 1 == sg.b1) break;  // the columns are needed once more
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(pfree0 + buf * 8);
             }
-            s_prev = s_cur;
+            if (!ok) break;
+            if (++b == sg.b1) {
+                // ---- the segment's sums leave: a whole tile is stored, the parts of a split tile add up in D or wait in
+                // their slots for add_parts_kernel. They go back to the columns that the last run was read from, so that a
+                // loop of a few instructions can store them: with one store per register in a row, code that is fetched for
+                // one pass, 64 columns a thread took 3.9 us and 96 6.2 (now 2.1 and 3.8). ----
+                asm volatile("griddepcontrol.wait;" ::: "memory");  // D zeroed, scales written
+                const bool whole = sg.b0 == 0 && sg.b1 == nblk;
+                const uint32_t m = tile_m0(sg.tile) + row;
+                const uint32_t n0 = tile_n0(sg.tile) + hp * half;
+                float* out = g.parts ? g.parts + ((uint64_t)slot * g.n_tile + hp * half) * 256 + rank * kBM + row : g.D + (uint64_t)n0 * g.stride_d + m;
+                const uint32_t out_stride = g.parts ? 256u : g.stride_d;
+                // the tokens' scales, one per lane (a load per column would be held back by the add before it)
+                float inv[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    inv[i] = 32u * i + lane < half && n0 + 32 * i + lane < g.N ? __ldcg(g.inv_scale + n0 + 32 * i + lane) : 0.f;
+                const uint32_t last = kRuns == 4 ? 3u : gb & 1;
+                const uint32_t ta = tmem + lane_base + last * T::kPStride + (merged ? hp * g.n_tile : hp * half);
+#pragma unroll
+                for (int c = 0; c < BN / 16; ++c) {
+                    if ((uint32_t)c * 8 < half) tmem_st8(ta + c * 8, acc + c * 4);
+                    acc[c * 4] = acc[c * 4 + 1] = acc[c * 4 + 2] = acc[c * 4 + 3] = make_float2(0.f, 0.f);
+                }
+                tmem_st_wait();
+                const uint32_t cols = m < g.M && n0 < g.N ? min(half, g.N - n0) : 0u;  // that this thread stores
+                const bool plain = whole || g.parts;
+#pragma unroll 1
+                for (uint32_t c = 0; c < half; c += 8) {
+                    uint32_t v[8];
+                    tmem_ld8(ta + c, v);
+                    const float iv = c < 64 ? (c < 32 ? inv[0] : inv[1]) : (c < 96 ? inv[2] : inv[3]);
+                    float x[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = __shfl_sync(0xFFFFFFFFu, iv, (c & 31) + e);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] *= __uint_as_float(v[e]);
+                    if (plain) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (c + e < cols) out[(uint64_t)e * out_stride] = x[e];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (c + e < cols) atomicAdd(out + (uint64_t)e * out_stride, x[e]);
+                    }
+                    out += 8 * (uint64_t)out_stride;
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(pfree0 + last * 8);
+            }
         }
     }
     tc_fence_before();
@@ -898,7 +988,7 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     static std::atomic<int> max_pairs[64];
     if (cudaError_t e = ensure_dynamic_smem(kern, (int)T::kSmemBytes, attr_done); e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kXThreads, 1, 1);
+    cfg.blockDim = dim3(T::kThreads, 1, 1);
     cfg.dynamicSmemBytes = T::kSmemBytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -912,24 +1002,15 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     cfg.numAttrs = 1;
     const int pairs = max_pairs_of(kern, cfg, max_pairs);
     if (pairs < 1) return cudaErrorNotSupported;
-    // Whole tiles where there are nearly as many as pairs: a split tile costs a second epilogue of atomic adds. The parts of a
-    // split tile are added so that no sum's order depends on timing: two of them by atomics (0 + a + b), more by a kernel
-    // behind this one.
-    const uint32_t n = plan.n_tiles, most = (uint32_t)pairs;
-    uint32_t G = most, groups = 0, per = 1;
-    if (n >= most) {  // ranges of a tile's length or more: a tile lies on two at most
-    } else if (n * 8 >= most * 7) {
-        G = n;
-    } else if (n * 2 > most && plan.nblk > 1) {  // groups of k tiles on k + 1 pairs: every tile on two
-        groups = G - n;
-    } else {  // every tile on as many pairs
-        per = most / n < plan.nblk ? most / n : plan.nblk;
-        const uint64_t room = kExactPartBytes / ((uint64_t)n * plan.n_tile * 1024);
-        if (per > 2 && per > room) per = room > 2 ? (uint32_t)room : 2u;
-        // two, where that makes a part two blocks longer at most: no third launch (1024 x 1024, 8 tokens 11.2 -> 9.7 us)
-        if (per > 2 && (plan.nblk + 1) / 2 <= (plan.nblk + per - 1) / per + 2) per = 2;
-        G = n * per;
-    }
+    // the promoters wait for registers that the others give back: the sum is that of T's static_assert
+    static const bool registers = [&] {
+        cudaFuncAttributes fa{};
+        return cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs == T::kLaunchRegs;
+    }();
+    if (!registers) return cudaErrorNotSupported;
+    const uint32_t n = plan.n_tiles;
+    const XDeal deal = x_deal(n, plan.n_tile, plan.nblk, (uint32_t)pairs, x_cost(p, XW<TYPE>::kTerms == 2, plan.n_tile));
+    const uint32_t G = deal.pairs, per = deal.per;
     const bool split = n % G != 0, parts = per > 2;
     cfg.numAttrs = 2;
     cfg.gridDim = dim3(2 * G, 1, 1);
@@ -947,7 +1028,7 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     g.n_tiles = plan.n_tiles;
     g.n_tile = plan.n_tile;
     g.terms = p.bf16 ? 1u : 2u;
-    g.groups = groups;
+    g.groups = deal.groups;
     g.parts = parts ? plan.parts : nullptr;
     g.status = p.status;
     EncodeFn enc = encode_fn();
@@ -997,7 +1078,7 @@ cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, const ExactPrep& 
     }
     if (plan.n_tile <= 64) return x_launch<TYPE, 64, kFetch, 1>(p, plan, prep, s);
     if (plan.n_tile <= 128) return x_launch<TYPE, 128, kFetch, 1>(p, plan, prep, s);
-    return x_launch<TYPE, 256, kFetch, 1>(p, plan, prep, s);
+    return plan.n_tile <= 192 ? x_launch<TYPE, 192, kFetch, 1>(p, plan, prep, s) : x_launch<TYPE, 256, kFetch, 1>(p, plan, prep, s);
 }
 
 }  // namespace

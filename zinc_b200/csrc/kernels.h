@@ -348,6 +348,39 @@ struct XPlan {
     float* parts;
     uint64_t* launches;
 };
+// What a tile costs a CTA pair, in cycles: a block at the tensor cores' pace (10 per fp16 product and token, 20 in
+// short accumulations) or the producers',
+// an epilogue, and D to be zeroed before parts can be added into it (a pair's share of its bytes' time).
+struct XCost {
+    uint64_t block, epilogue, zero;
+};
+inline XCost x_cost(const ExactGemm& p, bool two, uint32_t n_tile) {  // two: weights of two fp16 terms
+    const uint64_t mma = (p.fine ? 20ull : 10ull) * ((two ? 2 : 1) + (p.bf16 ? 0 : 1)) * n_tile, unpack = two ? 5000 : 2600;
+    return {mma > unpack ? mma : unpack, 1500 + 40ull * n_tile, (uint64_t)p.M * p.N / 450};
+}
+// How the tiles are dealt to CTA pairs: whole ones where the pairs that stay idle cost less than a second epilogue and the
+// zeroing of D (Q4_K 4096 x 4096, 658 tokens, 64 tiles on 64 of 74 pairs 55.7 us, on all 74 57.5). The parts of a split tile
+// are added so that no sum's order depends on timing: two of them by atomics (0 + a + b), more by a kernel behind this one.
+struct XDeal {
+    uint32_t pairs, groups, per;  // per: parts of a tile, where all are split alike
+};
+inline XDeal x_deal(uint32_t n, uint32_t n_tile, uint32_t nblk, uint32_t most, const XCost& c) {
+    XDeal d{most, 0, 1};
+    if (n >= most) {  // ranges of a tile's length or more: a tile lies on two at most
+    } else if (n * 2 > most && nblk > 1) {
+        const uint64_t spread = ((uint64_t)n * nblk + most - 1) / most;
+        if ((nblk - spread) * c.block <= c.epilogue + c.zero) d.pairs = n;
+        else d.groups = most - n;  // groups of k tiles on k + 1 pairs: every tile on two
+    } else {  // every tile on as many pairs
+        d.per = most / n < nblk ? most / n : nblk;
+        const uint64_t room = kExactPartBytes / ((uint64_t)n * n_tile * 1024);
+        if (d.per > 2 && d.per > room) d.per = room > 2 ? (uint32_t)room : 2u;
+        // two, where that makes a part two blocks longer at most: no third launch (1024 x 1024, 8 tokens 11.2 -> 9.7 us)
+        if (d.per > 2 && (nblk + 1) / 2 <= (nblk + d.per - 1) / d.per + 2) d.per = 2;
+        d.pairs = n * d.per;
+    }
+    return d;
+}
 // D[n][m] <- sum of the `per` parts of its tile, in their order: parts [tile][per][n_tile][rows] (rows 256 or 128), tile t at
 // row tile t % row_tiles of n_tile tokens from t / row_tiles * n_tile
 cudaError_t launch_add_parts(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t rows, uint32_t row_tiles, uint32_t n_tile,
