@@ -405,13 +405,14 @@ float cut_us(uint32_t type, uint32_t tn, uint32_t most, uint32_t cluster, uint32
     const float one = 3.3f + (float)most * (type == T_Q4_K ? 0.83f : 1.39f) + 0.018f * (float)tn;
     return (float)rounds * one + (parts > 1 ? 2.1f : 0.f) + (cluster > 1 ? 0.9f : 0.f);
 }
-float others_us(uint32_t type, uint32_t M, uint32_t N, uint32_t K, uint32_t sms) {
+float others_us(uint32_t type, uint32_t M, uint32_t N, uint32_t K, uint32_t sms, bool vec) {  // vec: D's columns on 16 bytes
     const uint32_t nblk = K >> 8, row_tiles = (M + kBM - 1) / kBM;
     if (N > 256) {  // CTA pairs over 256 rows x 512 tokens
         const uint32_t tiles = (row_tiles + 1) / 2 * ((N + 511) / 512), pairs = sms / 2;
         uint32_t G = tiles * nblk / 4;
         G = G < 1 ? 1 : G > pairs ? pairs : G;
-        if (tiles <= pairs && tiles * 5 >= pairs * 3) G = tiles;
+        // whole tiles: 31 shapes within 8 % rms (Q4_K 4096 x 4096, 2048 tokens there 52.5, here 60.7)
+        if (tiles <= pairs && tiles * 5 >= pairs * 3) return 16.f + 2.4f * (float)nblk;
         return 28.f + 2.2f * (float)(tiles * nblk) / (float)G;
     }
     if (type == T_Q6_K && (K & 2047u)) return 1e9f;  // one CTA per 128 x 128, by cp.async
@@ -421,13 +422,15 @@ float others_us(uint32_t type, uint32_t M, uint32_t N, uint32_t K, uint32_t sms)
     splits = splits < 1 ? 1 : splits > 8 ? 8 : splits;
     while (splits > 1 && nblk / splits < least) --splits;
     const float blocks = (float)((nblk + splits - 1) / splits), rounds = (float)((tiles * splits + sms - 1) / sms);
-    return swapped ? 7.5f + 2.3f * blocks * rounds : N <= 128 ? 6.f + 1.9f * blocks * rounds : 8.f + (type == T_Q4_K ? 1.55f : 1.8f) * blocks * rounds;
+    // (single additions: 4075 x 4096, 100 tokens 26 us, 4976 x 5120, 128 tokens with vectors of four 17)
+    return swapped ? 7.5f + 2.3f * blocks * rounds + (vec || splits == 1 ? 0.f : 0.12f * (float)N) : N <= 128 ? 6.f + 1.9f * blocks * rounds : 8.f + (type == T_Q4_K ? 1.55f : 1.8f) * blocks * rounds;
 }
 
-bool best_cut(uint32_t type, uint32_t M, uint32_t N, uint32_t K, uint32_t sms, Cut& best) {
+bool best_cut(uint32_t type, uint32_t M, uint32_t N, uint32_t K, uint32_t sms, bool vec, Cut& best) {
     const uint32_t nblk = K >> 8, row_tiles = (M + kBM - 1) / kBM;
     const int* held = most_clusters();
-    float least = 0.94f * others_us(type, M, N, K, sms);
+    // the estimates are some 10 % off either way, between 128 and 256 tokens of Q4_K more (4814 x 5120, 159 tokens: 20.2 us, the other 17.9)
+    float least = (type == T_Q4_K && N > 128 && N <= 256 ? 0.8f : 0.9f) * others_us(type, M, N, K, sms, vec);
     bool found = false;
     uint32_t last = 0;
     for (uint32_t nt = (N + kCutMaxTokens - 1) / kCutMaxTokens, tries = 0; nt <= (N + 15) / 16 && tries < 16; ++nt) {
@@ -459,7 +462,8 @@ cudaError_t launch_mul_mm_cut(uint32_t type, const uint8_t* A, const void* B, fl
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     Cut cut;
-    if (!best_cut(type, M, N, K, (uint32_t)sms, cut)) return cudaErrorNotSupported;
+    const bool vec = (stride_d & 3u) == 0 && (reinterpret_cast<uintptr_t>(D) & 15u) == 0;
+    if (!best_cut(type, M, N, K, (uint32_t)sms, vec, cut)) return cudaErrorNotSupported;
     const cudaError_t e = type == T_Q4_K ? launch_typed<T_Q4_K>(A, B, D, M, N, K, stride_b, stride_d, cut, status, s, launches)
                                          : launch_typed<T_Q6_K>(A, B, D, M, N, K, stride_b, stride_d, cut, status, s, launches);
     if (e == cudaSuccess && launches) ++*launches;
