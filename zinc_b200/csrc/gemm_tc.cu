@@ -297,18 +297,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_constant
                         : "r"(taddr)
                         : "memory");
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (m < g.M) {
+                    const uint32_t nc = n0 + c * 32, cols = m < g.M && nc < g.N ? g.N - nc : 0u;  // that this thread writes
+                    float* dst = g.D + (uint64_t)nc * g.stride_d + m;
+                    if (gridDim.z == 1) {
 #pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) {
-                            const uint32_t n = n0 + c * 32 + jj;
-                            if (n < g.N) {
-                                float* dst = g.D + (uint64_t)n * g.stride_d + m;
-                                if (gridDim.z == 1)
-                                    *dst = __uint_as_float(v[jj]);
-                                else
-                                    atomicAdd(dst, __uint_as_float(v[jj]));
-                            }
-                        }
+                        for (uint32_t jj = 0; jj < 32; ++jj)
+                            if (jj < cols) dst[(uint64_t)jj * g.stride_d] = __uint_as_float(v[jj]);
+                    } else {
+#pragma unroll
+                        for (uint32_t jj = 0; jj < 32; ++jj)
+                            if (jj < cols) atomicAdd(dst + (uint64_t)jj * g.stride_d, __uint_as_float(v[jj]));
                     }
                 }
             }
@@ -701,18 +699,16 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_b, const __grid_con
                     return n0 + (uint32_t)(c >> 3) * (BN / 2) + col + (col >= (uint32_t)(BN / 2) ? BN / 2 : 0);
                 };
                 auto put = [&](uint32_t nc, const uint32_t (&v)[32]) {
-                    if (m < g.M && go && nc < g.N) {
+                    const uint32_t cols = m < g.M && go && nc < g.N ? g.N - nc : 0u;  // that this thread writes
+                    float* dst = g.D + (uint64_t)nc * g.stride_d + m;
+                    if (store) {  // asked once: a branch for each column costs more than the column's store
 #pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) {
-                            const uint32_t n = nc + jj;
-                            if (n < g.N) {
-                                float* dst = g.D + (uint64_t)n * g.stride_d + m;
-                                if (store)
-                                    *dst = __uint_as_float(v[jj]);
-                                else
-                                    atomicAdd(dst, __uint_as_float(v[jj]));
-                            }
-                        }
+                        for (uint32_t jj = 0; jj < 32; ++jj)
+                            if (jj < cols) dst[(uint64_t)jj * g.stride_d] = __uint_as_float(v[jj]);
+                    } else {
+#pragma unroll
+                        for (uint32_t jj = 0; jj < 32; ++jj)
+                            if (jj < cols) atomicAdd(dst + (uint64_t)jj * g.stride_d, __uint_as_float(v[jj]));
                     }
                 };
 #pragma unroll 1
