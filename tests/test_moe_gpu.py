@@ -894,6 +894,37 @@ def test_moe_grouped_tile_edges(gpu, oracle, t, E, M, K, counts):
     assert max(rel_l2(got[i], want[i]) for i in range(T)) <= 2e-2
 
 
+@pytest.mark.parametrize("t,M,K", [(zb.MXFP4, 32, 64), (zb.Q4_K, 8, 256)])
+@pytest.mark.parametrize("E,T", [(1, 16), (31, 1025), (1025, 4096), (1025, 4097), (4096, 5000)])
+def test_moe_grouped_pair_counts(gpu, oracle, t, M, K, E, T):
+    """The grouping at the edges of what a thread holds: one expert to the most there may be, pairs that a CTA keeps in its
+    registers (4096) and one more, a pair of no expert. The bar is the grouped tests'."""
+    torch, ctx, dd = gpu
+    g = synth.rng(232, E + T)
+    w, stride = stacked(g, t, E, M, K)
+    ids = g.integers(0, E, size=T).astype(np.uint32)
+    ids[: T // 3] = E - 1
+    ids[5] = 0xFFFFFFFF
+    X = synth.activations(g, T, K)
+    Y = out_with_canary(torch, T * M, init=-7.0)
+    ws = torch.empty(dd.moeGroupedWorkspaceBytes(T, 1, K, E), dtype=torch.uint8, device="cuda")
+    dd.setWorkspace(ws)
+    try:
+        dd.recordMoeBatchedDispatch(t, dev(torch, w), dev(torch, X), Y, dev(torch, ids), M, K, stride, E, 1, T, K, M)
+        ctx.submit_and_wait()
+    finally:
+        dd.setWorkspace(None)
+    got = Y[:T * M].cpu().numpy().reshape(T, M)
+    assert canary_intact(Y, T * M)
+    assert np.all(got[5] == -7.0)
+    ok = np.arange(T) != 5
+    want = oracle.moe_dmmv_f64(w, t, M, K, stride, ids[ok], K, X[ok])
+    assert rel_l2(got[ok], want) <= TOL_TC
+    # a token's own eight sums: the error goes with their terms (twice its mean in 5000 draws), the norm falls to a fifth of its
+    # mean by cancellation (chi of 8 degrees of freedom: 1 in 5000 below 0.2)
+    assert max(rel_l2(a, b) for a, b in zip(got[ok], want)) <= 10 * TOL_TC
+
+
 @pytest.mark.parametrize("n,k", [(1, 1), (31, 5), (32, 32), (33, 32), (256, 32), (257, 8), (64, 33)])
 def test_router_selection_ties(gpu, oracle, n, k):
     """Selection by ranks (up to 256 experts and 32 picks) and beyond it, with logits that tie: the lower index first."""
