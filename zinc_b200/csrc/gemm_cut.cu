@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
         if (lane == 0) {  // ---- loader of the activations ----
             uint32_t st = 0, ph = 1;
             for (int s = 0; s < 2 * nb; ++s) {
-                if (!poll_or_fail(&bars->empty[st], ph, bars, g.status, 172)) break;
+                if (!poll_or_fail<true>(&bars->empty[st], ph, bars, g.status, 172)) break;
                 mbar_expect_tx(&bars->full[st], stage_bytes);
                 for (int h = 0; h < 2; ++h)
                     tma_load_2d(smem + st * stage_bytes + h * x_bytes, &maps.x, (b0 * 4 + s * 2 + h) * 64, (int)n0, &bars->full[st]);
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
         if (lane == 0) {  // ---- loaders of the raw blocks; rows past M: zeros ----
             uint32_t slot = 0, ph = 1;
             for (int b = b0; b < b0 + nb; ++b) {
-                if (!poll_or_fail(&bars->empty_w[slot], ph, bars, g.status, 173)) break;
+                if (!poll_or_fail<true>(&bars->empty_w[slot], ph, bars, g.status, 173)) break;
                 uint8_t* const raw = raw0 + slot * R::kSlot;
                 if constexpr (TYPE == T_Q4_K) {
                     mbar_expect_tx(&bars->full_w[slot], R::kSlot);
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
         uint32_t st = (q >> 1) % g.stages, ph = 1, slot = 0, slot_ph = 0;
         bool dead = false;
         for (int b = b0; b < b0 + nb; ++b) {
-            if (!dead) dead = !poll_or_fail(&bars->full_w[slot], slot_ph, bars, g.status, 174);
+            if (!dead) dead = !poll_or_fail<true>(&bars->full_w[slot], slot_ph, bars, g.status, 174);
             const uint8_t* raw = raw0 + slot * R::kSlot + raw_at;
             uint32_t o[32];
             auto put = [&](int c, const uint4& v) {
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
                 // words 4 k + 3 are made of every word read but the first ones of ql and qh, which word 0 is made of
                 release_after(o[0] ^ o[3] ^ o[7] ^ o[11] ^ o[15] ^ o[19] ^ o[23] ^ o[27] ^ o[31], &bars->empty_w[slot], lane);
             }
-            if (!dead) dead = !poll_or_fail(&bars->empty[st], ph, bars, g.status, 175);
+            if (!dead) dead = !poll_or_fail<true>(&bars->empty[st], ph, bars, g.status, 175);
             __syncwarp();
             tc_fence_after();
             if (!__any_sync(0xFFFFFFFFu, dead)) {
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
             }
         }
         // ---- the tile, or this CTA's part of it: lane = weight row, column = token ----
-        if (!dead) dead = !poll_or_fail(&bars->accum, 0, bars, g.status, 176);
+        if (!dead) dead = !poll_or_fail<true>(&bars->accum, 0, bars, g.status, 176);
         __syncwarp();
         tc_fence_after();
         dead = __any_sync(0xFFFFFFFFu, dead);
