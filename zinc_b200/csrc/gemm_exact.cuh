@@ -432,7 +432,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                             bar = smem_u32(&bars->pfree[gb & 1]);
                             par = ((gb >> 1) - 1) & 1;
                         }
-                        ok = warp_poll(bar, par, bars, g.status, 181);
+                        ok = warp_poll<true>(bar, par, bars, g.status, 181);
                         if (!ok) break;
                         tc_fence_after();
                         if (open) db = desc_b + sb * (b_bytes >> 4);
@@ -480,7 +480,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                             bar = smem_u32(&bars->pfree[c]);
                             par = (gb - 1) & 1;
                         }
-                        ok = warp_poll(bar, par, bars, g.status, 181);
+                        ok = warp_poll<true>(bar, par, bars, g.status, 181);
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {  // small terms first: what they add up to is all that the accumulator rounds them by
@@ -518,7 +518,7 @@ gemm_exact_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 }
                 if constexpr (kMin) {  // into the last run; merged: these columns hold the sums' terms; the low-term columns see zeros
                     if (!ok) break;
-                    ok = warp_poll(lane == 1 ? full_b + sb * 8 : smem_u32(&bars->full_m[gb & 1]), lane == 1 ? pb : (gb >> 1) & 1, bars,
+                    ok = warp_poll<true>(lane == 1 ? full_b + sb * 8 : smem_u32(&bars->full_m[gb & 1]), lane == 1 ? pb : (gb >> 1) & 1, bars,
                                    g.status, 184);
                     if (!ok) break;
                     tc_fence_after();

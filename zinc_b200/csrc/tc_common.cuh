@@ -238,14 +238,26 @@ __device__ __forceinline__ bool mbar_test_addr(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait of a converged warp for the barriers its lanes name (each lane one: several barriers in one round of
-// polls, one answer). test_wait answers in 10-25 cycles where a try_wait in a loaded kernel took 190-280, and the
-// issuing warp's own instructions are what bounds it.
-template <typename B>
+__device__ __forceinline__ bool mbar_try_addr(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait of a converged warp for the barriers its lanes name (each lane one: several barriers in one round, one answer):
+// a first poll, then waits that suspend the lanes. kSpin: polls only, which the f32-accurate GEMM's issuer keeps (its Q5_K
+// products of 4096 x 4096 took 2 % more suspended); elsewhere the spinning cost the others more than the issuer gained (MoE
+// prefill of 256 experts 208.2 -> 205.7 us, the cut GEMM's few tokens 2 to 3 %).
+template <bool kSpin = false, typename B>
 __device__ __forceinline__ bool warp_poll(uint32_t bar, uint32_t parity, B* bars, uint32_t* status, uint32_t site) {
     if (__all_sync(0xFFFFFFFFu, mbar_test_addr(bar, parity))) return true;
-    for (uint32_t i = 0; i < 16u * kWaitLimit; ++i) {
-        if (__all_sync(0xFFFFFFFFu, mbar_test_addr(bar, parity))) return true;
+    for (uint32_t i = 0; i < (kSpin ? 16u : 1u) * kWaitLimit; ++i) {
+        if (__all_sync(0xFFFFFFFFu, kSpin ? mbar_test_addr(bar, parity) : mbar_try_addr(bar, parity))) return true;
         if ((i & 255u) == 255u && __any_sync(0xFFFFFFFFu, bars->failed != 0)) return false;
     }
     bars->failed = 1;
