@@ -496,7 +496,7 @@ def moe_decode_results(torch, zb, ctx, dd, stream, sampler, args, rank=0, world=
                 "dtype": "f32", "data": "synthetic",
                 "config": {"workload": name + ", decode batch 1", "layers": shape.n_layers,
                            "weight_bytes_per_token": shape.weight_bytes(), "parallelism": par,
-                           "dispatch": "router + selection / gate + up + activation / down + sum: three launches per layer"
+                           "dispatch": "router + selection / gate + up + activation / down + sum: three calls per layer"
                            if step.fused else "one launch per dispatch of the reference's sequence",
                            "l2": "weights touched per token (all layers) are larger than L2"},
                 "gpu_launches": launches * len(per) * 20, "gpu_launches_per_step": launches,
@@ -731,7 +731,7 @@ def main():
                          "moe_decode: the two MoE configurations at batch 1; moe_prefill: one MoE layer's routed experts "
                          "over a prefill batch")
     ap.add_argument("--moe-dispatch", default="fused", choices=["fused", "reference"],
-                    help="moe_decode: fused = three launches per layer (default); reference = one launch per dispatch of "
+                    help="moe_decode: fused = three calls per layer (default); reference = one launch per dispatch of "
                          "the reference's sequence")
     ap.add_argument("--collective", default="fused", choices=["fused", "peer", "nccl"],
                     help="N > 1, hidden-state sums: fused = partial rows pushed to every rank from the matvec's epilogue "
