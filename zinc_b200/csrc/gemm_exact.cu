@@ -185,7 +185,7 @@ cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     PrepArgs a = *static_cast<const PrepArgs*>(args);
     a.zero = zero;
     // a whole row in the threads' registers where there are few tokens; beyond two CTAs to an SM the second read costs less than
-    // the occupancy (10752 columns, 1268 tokens: 1024 threads 12 us, 256 3)
+    // the occupancy (Q5_K 407 x 10752, 1268 tokens: the whole product 61.6 us with 1024 threads, 49.2 with 256)
     uint32_t threads = 256;
     while (a.tokens <= 2 * 148 && threads < kPrepMost && threads < a.nblk * 16) threads *= 2;
     return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(threads), 0, s, a);

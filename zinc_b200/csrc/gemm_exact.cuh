@@ -19,17 +19,17 @@
 // An infinite activation makes its token's row NaN.
 // A run of columns is one accumulation in tensor memory; eight warps of their own then add scale * sum to f32 registers
 // ("promote") while further runs fill other accumulators and the producer warps unpack what follows. (With both in the same
-// warps a block took the sum of the two: MXFP4 4096 x 4096, 512 tokens 53.3 us, now 39.3, Q6_K 50.0 and 46.5; Q4_K, which has
-// little to unpack and long MMAs, 39.7 and 40.7 there, 30.9 and 27.5 at 256 tokens.) The tensor core cuts an accumulator's last bits off at every
+// warps a block took the sum of the two: MXFP4 4096 x 4096, 512 tokens 53.2 us, now 43.4, Q6_K 50.4 and 46.3; Q4_K, which has
+// little to unpack and long MMAs, 40.3 and 40.7 there, 30.9 and 27.5 at 256 tokens.) The tensor core cuts an accumulator's last bits off at every
 // instruction, so the length of a run decides how far the result is from the exact one (relative L2, activations N(0, 1),
 // K = 4096):
 //   kRuns 1  a block of 256 columns: 1.8e-7 (MXFP4) to 1e-6 (Q8_0 beyond 128 tokens), where one f32 chain per output
 //            (gemm_simple_kernel) has 1.1e-6. For zc_mul_mm.
 //   kRuns 4  64 columns, their small terms first: 1.2e-7 to 1.8e-7, where f32 sums by lanes (dmmv_kernel) have 1.0e-7 to
 //            1.3e-7 and runs of a block 3.6e-7 to 1e-6. For zc_dmmv_batch, in tiles of at most 128 tokens, where a block's
-//            four accumulators fit: Q4_K 12288 x 4096, 105 tokens 38.3 us (37 with runs of a block). Adding a block's
-//            four runs before the registers' sum takes it to 1.4e-7 and 12 % more time, with the sum's roundings kept too
-//            1.3e-7 and 30 %: the runs' own roundings are what is left.
+//            four accumulators fit: Q4_K 12288 x 4096, 105 tokens 36.4 us. (Measured while the same warps unpacked and
+//            promoted, 37.3 us: runs of a block 36.7; adding a block's four runs before the registers' sum 1.4e-7 and 42 us, with
+//            the sum's roundings kept too 1.3e-7 and 49 us: the runs' own roundings are what is left.)
 //
 // Persistent CTA pairs (cta_group::2, 256 weight rows per pair): tiles of 256 rows x n_tile tokens, their
 // (tile, block) units dealt in equal contiguous ranges to the pairs. A tile that is split over two pairs is summed with
