@@ -191,30 +191,35 @@ cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(threads), 0, s, a);
 }
 
-// D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: eight tokens of a tile. Bound: the
+// D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: 1024 / rows tokens of a tile. Bound: the
 // parts' bytes, which the kernel in front has left in L2, and the launch. It costs the smallest products 3 to 5 us over
 // atomic adds in any order (Q4_K 512 x 2048, 16 tokens, call behind call 8.7 -> 11.9, 1024 x 4096, 64 tokens 11.3 -> 15.9) and
 // 4096 x 4096, 64 tokens 1 (17.4 -> 18.5). Released early by the GEMM it was no sooner done. Slots that the last of a
 // tile's warps adds up within the GEMM: 1024 x 4096 25.6 us where this takes 21.5 (with L2 cold), 256 tokens of 4096 x 4096
 // 60 and 40.
+// Four rows of one column a thread, four parts read at once: with two columns behind one another and an unrolled loop and its
+// rest (code that is fetched for one pass) Q4_K f32 4096 x 4096, 32 tokens took 17.5 us, now 16.2, Q8_0 417 x 9248, 19 tokens
+// 22.5 and 19.0.
 template <uint32_t ROWS>
 __global__ void __launch_bounds__(256)
 add_parts_kernel(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t row_tiles, uint32_t n_tile, uint32_t per, uint32_t stride_d) {
     chain_wait();
     chain_release();
     after_wait(parts);
-    const uint32_t tile = blockIdx.x, tok = blockIdx.y * 8, r = threadIdx.x * 4 % ROWS;
-    const uint32_t m = tile % row_tiles * ROWS + r, last = min(tok + 8, n_tile);
-    if (m >= M) return;
-    for (uint32_t c = tok + threadIdx.x * 4 / ROWS; c < last; c += 1024 / ROWS) {
-        const uint32_t n = tile / row_tiles * n_tile + c;
-        if (n >= N) break;
+    const uint32_t tile = blockIdx.x, r = threadIdx.x * 4 % ROWS, c = blockIdx.y * (1024 / ROWS) + threadIdx.x * 4 / ROWS;
+    const uint32_t m = tile % row_tiles * ROWS + r, n = tile / row_tiles * n_tile + c;
+    if (m < M && c < n_tile && n < N) {
         const float* p = parts + ((uint64_t)tile * per * n_tile + c) * ROWS + r;
-        float4 s = __ldcg(reinterpret_cast<const float4*>(p));
-#pragma unroll 4
-        for (uint32_t i = 1; i < per; ++i) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(p + (uint64_t)i * n_tile * ROWS));
-            s = make_float4(s.x + v.x, s.y + v.y, s.z + v.z, s.w + v.w);
+        float4 s = make_float4(-0.f, -0.f, -0.f, -0.f);  // leaves what is added to it as it is
+#pragma unroll 1
+        for (uint32_t i = 0; i < per; i += 4) {
+            float4 v[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (i + j < per) v[j] = __ldcg(reinterpret_cast<const float4*>(p + (uint64_t)(i + j) * n_tile * ROWS));
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (i + j < per) s = make_float4(s.x + v[j].x, s.y + v[j].y, s.z + v[j].z, s.w + v[j].w);
         }
         float* d = D + (uint64_t)n * stride_d + m;
         if (m + 4 <= M && (reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
@@ -243,7 +248,7 @@ cudaError_t launch_type(const ExactGemm& p, const XPlan& plan, const ExactPrep& 
 
 cudaError_t launch_add_parts(const float* parts, float* D, uint32_t M, uint32_t N, uint32_t rows, uint32_t row_tiles, uint32_t n_tile,
                              uint32_t tiles, uint32_t per, uint32_t stride_d, cudaStream_t s) {
-    return launch_chained(rows == 256 ? add_parts_kernel<256> : add_parts_kernel<128>, dim3(tiles, (n_tile + 7) / 8), dim3(256), 0, s,
+    return launch_chained(rows == 256 ? add_parts_kernel<256> : add_parts_kernel<128>, dim3(tiles, (n_tile * rows + 1023) / 1024), dim3(256), 0, s,
                           parts, D, M, N, row_tiles, n_tile, per, stride_d);
 }
 
