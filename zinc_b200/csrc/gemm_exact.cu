@@ -36,23 +36,21 @@ __device__ __forceinline__ void chunk_columns(int c, uint32_t& a, uint32_t& b) {
     }
 }
 
-template <bool BF16>
-__device__ __forceinline__ float4 load4(const void* row, uint32_t k, uint32_t K, bool vec) {
+// VEC: rows of whole, aligned groups of four (the code is fetched for one pass: without the general case there is less of it)
+template <bool BF16, bool VEC>
+__device__ __forceinline__ float4 load4(const void* row, uint32_t k, uint32_t K) {
+    if (VEC) {
+        if (k >= K) return make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!BF16) return __ldg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k));
+        const uint2 t = __ldg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(row) + k));
+        return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16),
+                           __uint_as_float(t.y & 0xFFFF0000u));
+    }
     float v[4];
-    if (BF16) {
-        const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(row) + k;
-        if (vec && k + 4 <= K) {
-            const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
-            return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xFFFF0000u), __uint_as_float(t.y << 16),
-                               __uint_as_float(t.y & 0xFFFF0000u));
-        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = k + i < K ? __bfloat162float(p[i]) : 0.f;
-    } else {
-        const float* p = static_cast<const float*>(row) + k;
-        if (vec && k + 4 <= K) return __ldg(reinterpret_cast<const float4*>(p));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = k + i < K ? p[i] : 0.f;
+    for (int i = 0; i < 4; ++i) {
+        if (BF16) v[i] = k + i < K ? __bfloat162float(static_cast<const __nv_bfloat16*>(row)[k + i]) : 0.f;
+        else v[i] = k + i < K ? static_cast<const float*>(row)[k + i] : 0.f;
     }
     return make_float4(v[0], v[1], v[2], v[3]);
 }
@@ -73,7 +71,7 @@ __device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t h) {
 // up to 16384 columns stay in its registers between the scale and the terms (read twice, four elements at a time: 4096 columns,
 // 128 tokens
 // 5.8 us, 658 tokens with D to zero 9.0; now 4.5 and 8.1, both with L2 cold).
-template <int ORDER, bool BF16>
+template <int ORDER, bool BF16, bool VEC>
 __global__ void __maxnreg__(40) exact_prep_kernel(const PrepArgs a) {
     chain_wait();
     chain_release();  // the GEMM's set-up and its first weight blocks overlap this kernel
@@ -92,8 +90,8 @@ __global__ void __maxnreg__(40) exact_prep_kernel(const PrepArgs a) {
             chunk_columns<ORDER>(q & 7, ka, kb);
             va[i] = vb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (q < chunks) {
-                va[i] = load4<BF16>(row, (q >> 3) * 64 + ka, a.K, a.vec);
-                vb[i] = load4<BF16>(row, (q >> 3) * 64 + kb, a.K, a.vec);
+                va[i] = load4<BF16, VEC>(row, (q >> 3) * 64 + ka, a.K);
+                vb[i] = load4<BF16, VEC>(row, (q >> 3) * 64 + kb, a.K);
             }
         }
     };
@@ -188,7 +186,7 @@ cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     // the occupancy (Q5_K 407 x 10752, 1268 tokens: the whole product 61.6 us with 1024 threads, 49.2 with 256)
     uint32_t threads = 256;
     while (a.tokens <= 2 * 148 && threads < kPrepMost && threads < a.nblk * 16) threads *= 2;
-    return launch_chained(exact_prep_kernel<ORDER, BF16>, dim3(a.tokens), dim3(threads), 0, s, a);
+    return launch_chained(a.vec ? exact_prep_kernel<ORDER, BF16, true> : exact_prep_kernel<ORDER, BF16, false>, dim3(a.tokens), dim3(threads), 0, s, a);
 }
 
 // D = the sum of a tile's parts, in their order: [tile][part][token][rows]. One CTA: 1024 / rows tokens of a tile. Bound: the
@@ -327,7 +325,7 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         a.stride_b = p.stride_b;
         a.stride_d = p.stride_d;
         a.sums_on = min_type;
-        a.vec = (p.stride_b & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.B) & (p.bf16 ? 7u : 15u)) == 0;
+        a.vec = ((p.stride_b | p.K) & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.B) & (p.bf16 ? 7u : 15u)) == 0;
         const int order = min_type ? 0 : p.type == T_MXFP4 ? 2 : 1;
         const ExactPrep prep{p.bf16 ? (order == 0 ? launch_prep<0, true> : order == 1 ? launch_prep<1, true> : launch_prep<2, true>)
                                     : (order == 0 ? launch_prep<0, false> : order == 1 ? launch_prep<1, false> : launch_prep<2, false>),
