@@ -19,8 +19,8 @@
 // An infinite activation makes its token's row NaN.
 // A run of columns is one accumulation in tensor memory; eight warps of their own then add scale * sum to f32 registers
 // ("promote") while further runs fill other accumulators and the producer warps unpack what follows. (With both in the same
-// warps a block took the sum of the two: MXFP4 4096 x 4096, 512 tokens 53.2 us, now 43.4, Q6_K 50.4 and 46.3; Q4_K, which has
-// little to unpack and long MMAs, 40.3 and 40.7 there, 30.9 and 27.5 at 256 tokens.) The tensor core cuts an accumulator's last bits off at every
+// warps a block took the sum of the two: MXFP4 4096 x 4096, 512 tokens 53.2 us, now 43.2, Q6_K 50.1 and 45.6; Q4_K, which has
+// little to unpack and long MMAs, 39.8 and 40.0 there, 30.7 and 27.0 at 256 tokens.) The tensor core cuts an accumulator's last bits off at every
 // instruction, so the length of a run decides how far the result is from the exact one (relative L2, activations N(0, 1),
 // K = 4096):
 //   kRuns 1  a block of 256 columns: 1.8e-7 (MXFP4) to 1e-6 (Q8_0 beyond 128 tokens), where one f32 chain per output
