@@ -54,6 +54,8 @@ static void check(uint32_t mx, uint32_t H, uint32_t E, uint32_t k, uint32_t F, i
     for (int v : seen) EXPECT(v == 1, "a tile of nobody");
     EXPECT(p.at_parts_d - p.at_parts_g >= units_g * 64 && p.at_sync - p.at_parts_d >= units_d * 64, "room for the parts");
     EXPECT(most * 16 <= kComputeThreads && (p.d_tiles + p.grid - 1) / p.grid * 64 <= kComputeThreads, "a thread a row");
+    const uint32_t table = mx ? UnitOf<UNIT_MX>::table(F, s.slots) : UnitOf<UNIT_Q6K>::table(F, s.slots);
+    EXPECT((p.act_step == 0 || p.act_step >= table) && p.at_zeros - p.at_act >= table + p.act_step, "room for the activations' tables");
     auto over_is_exact = [&](uint32_t limit, uint32_t d, uint32_t mul) {
         for (uint32_t n = 0; n < limit; ++n)
             if ((mul ? (uint32_t)(((uint64_t)n * mul) >> 32) : n) != n / d) return false;

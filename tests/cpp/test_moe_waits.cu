@@ -1,8 +1,15 @@
 // The kernel of recorded MoE layers when its waits run out: it reports, leaves by itself, writes nothing past its buffers and leaves its
-// counters clean; the next launch is sound. The kernel is compiled in, so that its limit can be set.
+// counters clean; the next launch is sound. And when one CTA falls some 40 us behind ahead of its down products, layer after layer: the
+// same bits (the other CTA of its pair, which writes half of its table of activations, is a layer ahead by then). The kernel is compiled
+// in, so that its limit can be set and a CTA be held up.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
+
+__device__ int late_cta = -1;
+#define ZC_MOE_BEFORE_DOWN(layer)    \
+    if ((int)blockIdx.x == late_cta) \
+        for (int i_ = 0; i_ < 20; ++i_) __nanosleep(2000)
 
 #include "../../zinc_b200/csrc/moe_program.cu"
 
@@ -40,8 +47,8 @@ __global__ void fill_f32(float* x, uint32_t n, float scale) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = ((float)((i * 2654435761u) >> 16 & 1023u) / 512.f - 1.f) * scale;
 }
 
-static void run(bool mx, int sms) {
-    constexpr uint32_t H = 1024, E = 64, k = 4, F = 768, L = 3;
+static void run(bool mx, int sms, uint32_t H, uint32_t F, uint32_t E, bool one_table) {
+    constexpr uint32_t k = 4, L = 3;
     const uint32_t shared = mx ? 0 : 1, slots = k + shared, gb = mx ? 17 : 144, db = mx ? 17 : 210, ge = mx ? 32 : 256;
     const uint64_t gs = (uint64_t)F * (H / ge) * gb, ds = (uint64_t)H * (F / ge) * db;
     uint8_t *wg, *wu, *wd, *sg, *su, *sd;
@@ -102,6 +109,7 @@ static void run(bool mx, int sms) {
     std::vector<MoeProgram> storage(1);
     MoeProgram& p = storage[0];
     EXPECT(moe_plan(calls.data(), L, sms, p) == L, "not one program");
+    EXPECT((p.act_step == 0) == one_table, "%u x %u: not the tables that were to be tested", H, F);
     std::vector<CUtensorMap> maps((size_t)L * p.n_maps);
     EXPECT(moe_maps(calls.data(), p, maps.data()), "tensor maps");
     constexpr uint32_t kGuard = 4096;
@@ -151,6 +159,14 @@ static void run(bool mx, int sms) {
         sum += (double)v * v;
     }
     EXPECT(sum > 0, "hidden is zero");
+    for (int cta : {0, 1, 2, 37, 74, 75, (int)p.grid - 2, (int)p.grid - 1, -1}) {
+        CHECK(cudaMemcpyToSymbol(late_cta, &cta, sizeof cta));
+        for (int round = 0; round < 3; ++round) {
+            launch(1u << 24, 0);
+            EXPECT(st[0] == 0, "CTA %d late: wait %u gave up", cta, st[1]);
+            EXPECT(now == first, "CTA %d late: not the same bits", cta);
+        }
+    }
     int gave_up = 0;
     for (int round = 0; round < 30; ++round) {
         for (uint32_t limit : {0u, 1u, 3u, 10u}) {
@@ -166,14 +182,16 @@ static void run(bool mx, int sms) {
     }
     EXPECT(gave_up >= 30, "%d launches gave up", gave_up);
     for (uint8_t** s : stacks) CHECK(cudaFree(*s));
-    CHECK(cudaFree(mem));
+    for (void* m : {(void*)mem, (void*)x, (void*)router, (void*)out, (void*)status}) CHECK(cudaFree(m));
 }
 
 int main() {
     cudaDeviceProp prop;
     CHECK(cudaGetDeviceProperties(&prop, 0));
-    run(false, prop.multiProcessorCount);
-    run(true, prop.multiProcessorCount);
+    for (bool mx : {false, true}) {
+        run(mx, prop.multiProcessorCount, 1024, 768, 64, false);
+        run(mx, prop.multiProcessorCount, mx ? 2880 : 1024, mx ? 2880 : 2304, 16, true);
+    }
     printf("ok\n");
     return 0;
 }

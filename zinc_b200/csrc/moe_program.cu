@@ -21,6 +21,10 @@
 // Arithmetic: that of the streaming matvecs.
 #include "moe_program.h"
 
+#ifndef ZC_MOE_BEFORE_DOWN
+#define ZC_MOE_BEFORE_DOWN(layer)  // where a test lets a CTA fall behind its pair
+#endif
+
 #include <algorithm>
 #include <cstring>
 
@@ -65,7 +69,8 @@ struct Sync {
     uint64_t full[kUnits];
     uint64_t empty[kMaxRing];             // by places
     uint64_t rows;                        // arrival of x and of the router's rows
-    uint64_t table;                       // the activations' table: the compute warps of both CTAs of the pair
+    uint64_t table;                       // the activations' table is filled: the compute warps of both CTAs of the pair
+    uint64_t read;                        // one table: the pair's other CTA has read its own
     uint32_t ids[kIds][32], weights[kIds][32];  // the selections of a layer
     float row_part[kMaxRouterRows][kRouters];
     uint32_t routed;                      // layers whose experts are known and whose x is in its table
@@ -560,6 +565,10 @@ __device__ __forceinline__ void activate(const MoeProgram& p, Sync* s, uint32_t 
 
 // All activations of layer l, scaled by their slots' weights, into the table of the down projection: every other block of 256 by each
 // CTA of a pair, written to both. (All by every CTA: 18 blocks took 1.9 us, 48 took 4.2.)
+// The other CTA must have read what is written over there, and nothing awaited here says so of the layer before: the words are other
+// CTAs' for most blocks, and its part in s->table of that layer came ahead of its down products. With two tables by the layers' parity
+// s->table of the layer between does (every warp arrives there behind its down products of the layer that is written over); with one,
+// s->read (compute()).
 template <int GU, int KIND>
 __device__ __forceinline__ void collect(const MoeProgram& p, Sync* s, uint32_t l, uint8_t* table, uint32_t tag, uint32_t warp, int lane) {
     const uint64_t* src = p.act_x + (uint64_t)(l & 1) * p.slots * p.F;
@@ -679,7 +688,6 @@ __device__ __forceinline__ void add_row(const MoeProgram& p, Sync* s, uint32_t l
 
 template <int GU, int D>
 __device__ void compute(const MoeProgram& p, Sync* s, uint8_t* smem, uint32_t base_tag, uint32_t warp, int lane) {
-    uint8_t* act_table = smem + p.at_act;
     float *parts_g = reinterpret_cast<float*>(smem + p.at_parts_g), *parts_d = reinterpret_cast<float*>(smem + p.at_parts_d);
     const uint32_t ring = smem_u32(smem), zeros = ring + p.at_zeros, tid = warp * 32 + lane;
     const uint32_t n_g = Stage<GU, false>(p).n, n_d = Stage<D, true>(p).n;
@@ -687,16 +695,26 @@ __device__ void compute(const MoeProgram& p, Sync* s, uint8_t* smem, uint32_t ba
 #pragma unroll 1
     for (uint32_t l = 0; l < p.n_layers; ++l, first += n_g + n_d) {
         const uint32_t tag = base_tag + l + 1;
+        uint8_t* act_table = smem + p.at_act + (l & 1) * p.act_step;
         await(p, s, &s->routed, l + 1, 20, 218);
         const GateUpRow gu = gate_up_row<GU>(p, s, l, tid);
         dots<GU, false>(p, s, first, ring, ring + p.at_table + (l & 1) * p.table_bytes, zeros, parts_g, warp, lane);
+        // One table: the other CTA has read its own before this one writes there (collect()). For all warps by the barrier, in one warp:
+        // 24 layers of 2880 505 -> 509 us; each warp waiting ahead of its first store 528, a warp of its own for it (fewer registers) 541.
+        if (p.act_step == 0 && l > 0 && warp == kWarps - 1) {
+            wait_pair(p, s, &s->read, (l - 1) & 1, 220);
+            __syncwarp();
+        }
         bar_compute();
         activate(p, s, l, parts_g, tag, gu);
         collect<GU, D>(p, s, l, act_table, tag, warp, lane);
         if (tid == 0) store_volatile(&s->collected, l + 1);  // by all warps
         const DownRow dr = down_row<D>(p, s, l, tid);
+        ZC_MOE_BEFORE_DOWN(l);
         dots<D, true>(p, s, first + n_g, ring, smem_u32(act_table), zeros, parts_d, warp, lane);
         bar_compute();
+        if (p.act_step == 0 && tid == kComputeThreads - 1 && l + 1 < p.n_layers) arrive_at(&s->read, cluster_ctarank() ^ 1u);
+        __syncwarp();
         add_row(p, s, l, parts_d, tid, dr);
         if (l + 1 < p.n_layers && p.layers[l + 1].x_waits) {  // the next layer's x is what was just written, on all SMs
             ++waits;
@@ -731,6 +749,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMoeThreads, 1) moe_
     if (tid == 0) {
         mbar_init(&s->rows, 1);
         mbar_init(&s->table, 2 * kWarps);
+        mbar_init(&s->read, 1);
         s->routed = s->collected = s->rows_issued = s->gave_up = 0;
     }
     mbar_fence_init();
@@ -820,7 +839,7 @@ bool lay_out(const MoeShape& s, int sm_count, MoeProgram& p) {
     p.d_tiles = W::tiles(s.H);
     p.d_units_slot = W::units(s.F);
     p.d_units = p.d_units_slot * s.slots;
-    // Every CTA has gate and up rows: its activations show that it has read what the next layer but one writes over.
+    // Every CTA has gate and up rows: its activations show that it has read what the next layer but one writes over in the exchange.
     p.grid = std::min(sms, p.gu_tiles) & ~1u;   // in pairs
     if (p.grid < sms / 2) return false;
     p.router_rows = (s.E + p.grid - 1) / p.grid;
@@ -845,12 +864,17 @@ bool lay_out(const MoeShape& s, int sm_count, MoeProgram& p) {
     const uint32_t ng = most_tiles * p.gu_units;
     auto up = [](uint32_t n) { return (n + 127u) & ~127u; };
     p.table_bytes = up(G::table(s.H, 1));
-    const uint32_t x_bytes = up(s.H * 4 * (1 + p.router_rows)), act_bytes = up(W::table(s.F, s.slots));
+    const uint32_t x_bytes = up(s.H * 4 * (1 + p.router_rows));
+    const uint32_t act_bytes = up(W::table(s.F, s.slots));
     const uint32_t fixed = 128 + x_bytes + 2 * p.table_bytes + act_bytes + kMxZeros + up(ng * 64) + up(nd * 64) + up(sizeof(Sync));
     if (ng / p.gu_units * 16 > kComputeThreads || nd / p.d_units * 64 > kComputeThreads) return false;
     p.place_bytes = std::max(G::kBytes, W::kBytes);
     if (fixed + kMinRing * p.place_bytes > kMoeSmem) return false;
-    p.ring = std::min(kMaxRing, (kMoeSmem - fixed) / p.place_bytes);
+    auto ring = [&](uint32_t taken) { return taken > kMoeSmem ? 0u : std::min(kMaxRing, (kMoeSmem - taken) / p.place_bytes); };
+    p.ring = ring(fixed);
+    // a second table where the ring stays as long: 40 layers of 256 experts take 400 us with it, 414 with one table; the MXFP4 layers of
+    // 2880, whose ring it would take from 25 places to 15, 622 and 509
+    p.act_step = ring(fixed + act_bytes) == p.ring ? act_bytes : 0;
     bool exact = true;
     auto mul = [&](uint32_t d, uint64_t limit) {
         const uint32_t m = reciprocal(d, limit);
@@ -873,7 +897,7 @@ bool lay_out(const MoeShape& s, int sm_count, MoeProgram& p) {
     };
     p.at_x = take(x_bytes);
     p.at_table = take(2 * p.table_bytes);
-    p.at_act = take(act_bytes);
+    p.at_act = take(act_bytes + p.act_step);
     p.at_zeros = take(kMxZeros);
     p.at_parts_g = take(ng * 64);
     p.at_parts_d = take(nd * 64);

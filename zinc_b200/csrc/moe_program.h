@@ -57,8 +57,8 @@ struct MoeProgram {
     uint32_t ring, place_bytes;                   // units of weights under way, bytes of one
     uint32_t gu_tiles_slot_mul, gu_units_mul, d_units_mul, d_units_slot_mul, blocks_slot_mul, ring_mul;   // reciprocals
     uint32_t router_rows;                         // of a CTA, at most
-    // shared memory: the ring, x and the router's rows, two tables of x, the activations' table, zeros, parts
-    uint32_t at_x, at_table, table_bytes, at_act, at_zeros, at_parts_g, at_parts_d, at_sync, smem;
+    // shared memory: the ring, x and the router's rows, two tables of x, the activations' table or two (act_step apart; 0: one), zeros, parts
+    uint32_t at_x, at_table, table_bytes, at_act, act_step, at_zeros, at_parts_g, at_parts_d, at_sync, smem;
     uint64_t* logits_x;       // [2][E] {value, tag}: how the CTAs exchange logits ..
     uint64_t* act_x;          // [2][slots * F] .. and activations
     uint32_t* words;          // tags used so far, CTAs that have left, CTAs whose rows of hidden are written
