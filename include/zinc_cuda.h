@@ -148,8 +148,10 @@ int32_t zc_set_wait_limit(zc_ctx* ctx, uint32_t polls);
  * (without norm_weights and routing_local; up to 256 experts), zc_moe_gate_up_act_ex
  * on its input and zc_moe_down_acc_ex on its output, of one shape and with the
  * same buffers or ones apart, on Q4_K gate and up and Q6_K down matrices or MXFP4
- * throughout (rows of whole 16 bytes times eight): any number of them, up to 160
- * a kernel, whether or not a layer reads what the one before added to.
+ * throughout (rows of whole 16 bytes times eight), from 2 MB of Q6_K down weights
+ * of the selected experts on (below, the calls hold activations in f32): any
+ * number of them, up to 160 a kernel, whether or not a layer reads what the one
+ * before added to.
  * Results are those of the calls in their order; sums are taken in another order
  * than in the calls themselves, the same one at every replay. Such a kernel reads
  * weights of later calls ahead of earlier calls' results (calls that write another

@@ -100,6 +100,17 @@ def test_layers_that_read_what_the_one_before_wrote(gpu, arch, H, E, k, F):
     r.check(*r.eager_and_recorded(r.step.record, 1, hidden=hidden, replays=20), bar=1e-3)
 
 
+# Q6_K down matrices of the selected experts below 2 MB (1.94 and 1.61): the calls hold the activations in f32 there
+@pytest.mark.parametrize("H,E,k,F", [(1024, 64, 8, 256), (768, 32, 4, 512)])
+def test_layers_whose_calls_hold_f32_stay_launches(gpu, H, E, k, F):
+    torch, _, _ = gpu
+    r = Layers(torch, shape("kquant", H, E, k, F, 2))
+    eager, got = r.eager_and_recorded(r.step.record, 6)
+    r.check(eager, got)
+    # 21-bit activations would be 1.7e-6 off; two orders of f32 sums 1e-7
+    assert rel_l2(got["hidden"][:H].cpu().numpy(), eager["hidden"][:H].cpu().numpy()) <= 5e-7
+
+
 def test_a_long_run_is_several_kernels(gpu):
     torch, _, _ = gpu
     r = Layers(torch, shape("kquant", 1024, 64, 4, 512, 2), layers=170)   # 160 in a kernel
