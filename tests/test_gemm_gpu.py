@@ -10,7 +10,7 @@ import pytest
 
 import zinc_b200 as zb
 from zinc_b200 import synth
-from helpers import canary_intact, dev, out_with_canary, rel_l2
+from helpers import canary_intact, dev, out_with_canary, rel_l2, run_cpp
 
 pytestmark = pytest.mark.gpu
 TOL_F32, TOL_BF16, TOL_BF16_OPERANDS = 1e-4, 5e-3, 4e-3
@@ -397,6 +397,11 @@ def test_split_gemm_is_reproducible(gpu, oracle, t, M, N, K, bf16):
     assert (first[N:] == 7.0).all()
     cols = sorted({0, N // 2, N - 1})
     assert rel_l2(first[cols].numpy(), oracle.gemm_f64(raw, t, M, K, X[cols])) <= (TOL_BF16 if bf16 else 2e-6)
+
+
+def test_mul_mm_cut_in_every_form(gpu):
+    """Every number of CTAs and every cluster that K can be cut over, and waits that run out, with copies and MMAs under way."""
+    run_cpp("test_cut")
 
 
 # Shapes that K is cut for over 1, 2, 4, 6, 10 and 16 CTAs and whole tiles; tokens on both sides of a tile's 192 and of 16, one block of K,

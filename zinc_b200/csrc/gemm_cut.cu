@@ -12,7 +12,8 @@
 // (such rows lie eight rows' bytes apart, a multiple of 16), so that any number of rows can be described.
 // Warp roles (20 warps): 0 MMA issuer, 1 loader of the activations, 2 and 3 of raw blocks, 4-19 producers (group j of four warps =
 // columns 64 j .. of every block, a thread per row) and epilogue. Every mbarrier wait is bounded; a wait that gives up records {1, site},
-// raises the CTA's flag, and every role drains to the common exit where tensor memory is released.
+// raises the flag of all CTAs of the cluster, none of which adds its sums then, and every role drains to the common exit, where copies
+// and MMAs in flight are awaited and tensor memory is released.
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -41,9 +42,9 @@ struct CutRaw {
 };
 
 struct CutBars {
-    uint64_t full[kCutMaxStages], empty[kCutMaxStages];   // eight producer warps + the loader's expect_tx; a commit
-    uint64_t full_w[4], empty_w[4];                       // raw slots: the loaders' expect_tx; sixteen producer warps
-    uint64_t accum;
+    uint64_t full[kCutMaxStages], full_x[kCutMaxStages], empty[kCutMaxStages];  // eight producer warps; the loader's expect_tx; a commit
+    uint64_t full_w[2][4], empty_w[4];                    // raw slots: each loader's expect_tx; sixteen producer warps
+    uint64_t accum, drained;
     uint32_t tmem_base;
     volatile uint32_t failed;
 };
@@ -69,10 +70,24 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t a, uint32_t rank) {
         : "memory");
     return v;
 }
+__device__ __forceinline__ void raise_cluster(volatile uint32_t* flag, uint32_t rank) {
+    asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\tst.shared::cluster.u32 [r], %2;\n\t}" ::"r"(
+                     smem_u32(const_cast<uint32_t*>(flag))),
+                 "r"(rank), "r"(1u)
+                 : "memory");
+}
 // The weight row of a tile that lane l of tensor memory holds: for Q6_K eight lanes take the same c of eight groups (distinct banks).
 template <int TYPE>
 __device__ __forceinline__ uint32_t cut_row(uint32_t l) {
     return TYPE == T_Q4_K ? l : (l & 64u) + 8u * (l & 7u) + ((l >> 3) & 7u);
+}
+
+// After a wait has given up: until the last copies into a ring of n slots have landed, of `issued` that one thread requested. (The
+// barriers are arrived at by that thread only, so every copy's phase ends.)
+__device__ __forceinline__ void cut_await_copies(uint64_t* bars, uint32_t n, uint32_t issued) {
+    for (uint32_t i = issued > n ? issued - n : 0u; i < issued; ++i)
+        for (uint32_t tries = 0; tries < kDrainLimit && !mbar_try_wait(&bars[i % n], (i / n) & 1); ++tries) {
+        }
 }
 
 template <int TYPE>
@@ -89,14 +104,17 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
 
     if (tid == 0) {
         for (uint32_t s = 0; s < kCutMaxStages; ++s) {
-            mbar_init(&bars->full[s], 9);
+            mbar_init(&bars->full[s], 8);
+            mbar_init(&bars->full_x[s], 1);
             mbar_init(&bars->empty[s], 1);
         }
         for (int s = 0; s < 4; ++s) {
-            mbar_init(&bars->full_w[s], TYPE == T_Q4_K ? 1 : 2);
+            mbar_init(&bars->full_w[0][s], 1);
+            mbar_init(&bars->full_w[1][s], 1);
             mbar_init(&bars->empty_w[s], 16);
         }
         mbar_init(&bars->accum, 1);
+        mbar_init(&bars->drained, 1);
         bars->failed = 0;
         mbar_fence_init();
     }
@@ -113,12 +131,13 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem = warp_uniform(bars->tmem_base), tmem_w = tmem + (g.tn <= 128 ? 128u : 256u);
 
+    uint32_t requested = 0;  // copies, by a loader
     if (warp == 0) {
         // ---- MMA issuer (the converged warp walks, one elected lane issues) ----
         const uint32_t idesc = instr_desc<16>() + ((g.tn - 16u) >> 3 << 17);
         uint32_t st = 0, ph = 0;
         for (int s = 0; s < 2 * nb; ++s) {
-            if (!warp_poll(smem_u32(&bars->full[st]), ph, bars, g.status, 171)) break;
+            if (!warp_poll(smem_u32(lane == 1 ? &bars->full_x[st] : &bars->full[st]), ph, bars, g.status, 171)) break;
             tc_fence_after();
             const uint64_t dx = smem_desc(smem_u32(smem) + st * stage_bytes);
             const uint32_t a = tmem_w + st * 64;
@@ -139,9 +158,10 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
             uint32_t st = 0, ph = 1;
             for (int s = 0; s < 2 * nb; ++s) {
                 if (!poll_or_fail<true>(&bars->empty[st], ph, bars, g.status, 172)) break;
-                mbar_expect_tx(&bars->full[st], stage_bytes);
+                mbar_expect_tx(&bars->full_x[st], stage_bytes);
                 for (int h = 0; h < 2; ++h)
-                    tma_load_2d(smem + st * stage_bytes + h * x_bytes, &maps.x, (b0 * 4 + s * 2 + h) * 64, (int)n0, &bars->full[st]);
+                    tma_load_2d(smem + st * stage_bytes + h * x_bytes, &maps.x, (b0 * 4 + s * 2 + h) * 64, (int)n0, &bars->full_x[st]);
+                ++requested;
                 if (++st == g.stages) {
                     st = 0;
                     ph ^= 1;
@@ -151,20 +171,22 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
     } else if (warp == 2 || (warp == 3 && TYPE != T_Q4_K)) {
         if (lane == 0) {  // ---- loaders of the raw blocks; rows past M: zeros ----
             uint32_t slot = 0, ph = 1;
+            uint64_t* const full_w = bars->full_w[warp - 2];
             for (int b = b0; b < b0 + nb; ++b) {
                 if (!poll_or_fail<true>(&bars->empty_w[slot], ph, bars, g.status, 173)) break;
                 uint8_t* const raw = raw0 + slot * R::kSlot;
                 if constexpr (TYPE == T_Q4_K) {
-                    mbar_expect_tx(&bars->full_w[slot], R::kSlot);
-                    tma_load_2d(raw, &maps.w[0], b * 144, (int)m0, &bars->full_w[slot]);
+                    mbar_expect_tx(&full_w[slot], R::kSlot);
+                    tma_load_2d(raw, &maps.w[0], b * 144, (int)m0, &full_w[slot]);
                 } else {
                     const uint32_t c0 = warp == 2 ? 0u : 4u, row_bytes = g.nblk * 210u;
-                    mbar_expect_tx(&bars->full_w[slot], R::kSlot / 2);
+                    mbar_expect_tx(&full_w[slot], R::kSlot / 2);
 #pragma unroll
                     for (uint32_t c = c0; c < c0 + 4; ++c)
                         tma_load_2d(raw + c * (R::kSlot / 8), &maps.w[c], (int)((((c * row_bytes) & 15u) + (uint32_t)b * 210u) & ~15u), (int)(m0 / 8),
-                                    &bars->full_w[slot]);
+                                    &full_w[slot]);
                 }
+                ++requested;
                 if (++slot == g.raw_slots) {
                     slot = 0;
                     ph ^= 1;
@@ -176,11 +198,13 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
         const uint32_t q = (uint32_t)(warp - kCutProdWarp0) >> 2, quarter = (uint32_t)warp & 3u, row = cut_row<TYPE>(quarter * 32 + lane);
         const uint32_t raw_at = TYPE == T_Q4_K ? row * R::kRow : (row & 7u) * (R::kSlot / 8) + (row >> 3) * R::kRow;
         const uint32_t row_off = ((row & 7u) * g.nblk * 210u) & 15u;   // eight rows are a multiple of 16 bytes
+        // Q6_K: the rows of a warp are of one loader's boxes
+        uint64_t* const full_w = bars->full_w[TYPE == T_Q4_K ? 0 : (row & 7u) >> 2];
         const uint32_t lane_col = tmem_w + ((quarter * 32u) << 16) + (q & 1u) * 32;
         uint32_t st = (q >> 1) % g.stages, ph = 1, slot = 0, slot_ph = 0;
         bool dead = false;
         for (int b = b0; b < b0 + nb; ++b) {
-            if (!dead) dead = !poll_or_fail<true>(&bars->full_w[slot], slot_ph, bars, g.status, 174);
+            if (!dead) dead = !poll_or_fail<true>(&full_w[slot], slot_ph, bars, g.status, 174);
             const uint8_t* raw = raw0 + slot * R::kSlot + raw_at;
             uint32_t o[32];
             auto put = [&](int c, const uint4& v) {
@@ -253,6 +277,8 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
     if (g.parts > 1) {
         // ---- the parts of the cluster's CTAs, each CTA's share of the tokens, in the order of the parts ----
         if (g.cluster > 1) {
+            if (bars->failed)
+                for (uint32_t r = 0; r < g.cluster; ++r) raise_cluster(&bars->failed, r);
             __syncwarp();
             cluster_sync_all();
         } else {
@@ -292,8 +318,18 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
     chain_wait();
     tc_fence_before();
     __syncthreads();
-    if (bars->failed) {  // given up with copies in flight: let them land before the CTA's shared memory is another's
-        for (int i = 0; i < 100; ++i) __nanosleep(1000);
+    if (bars->failed) {  // nothing is in flight when shared and tensor memory become another's
+        if (warp == 0) {
+            if (elect_one()) umma_commit(&bars->drained);
+            __syncwarp();
+            for (uint32_t tries = 0; tries < kDrainLimit && !mbar_try_wait(&bars->drained, 0); ++tries) {
+            }
+        } else if (lane == 0 && warp == 1) {
+            cut_await_copies(bars->full_x, g.stages, requested);
+        } else if (lane == 0 && warp < kCutProdWarp0) {
+            cut_await_copies(bars->full_w[warp - 2], g.raw_slots, requested);
+        }
+        __syncthreads();
     }
     if (g.cluster > 1) cluster_sync_all();  // the others read this CTA's sums
     if (warp == 0) {
@@ -341,7 +377,7 @@ cudaError_t launch_typed(const uint8_t* A, const void* B, float* D, uint32_t M, 
     g.stages = g.stages < kCutMaxStages ? g.stages : kCutMaxStages;
     g.stages = g.stages < 2 * most ? g.stages : 2 * most;
     if (TYPE == T_Q4_K && most > 2 && room - g.stages * stage >= 4 * R::kSlot) g.raw_slots = 4;
-    if (g.stages < 2) return cudaErrorNotSupported;
+    if (g.stages < 2) return cudaErrorNotSupported;  // two hold a tile's sums, which take the place of the stages
     auto kern = gemm_cut_kernel<TYPE>;
     static std::atomic<uint64_t> attr_done{0};
     if (cudaError_t e = ensure_dynamic_smem(kern, kCutSmem, attr_done); e != cudaSuccess) return e;
@@ -350,7 +386,6 @@ cudaError_t launch_typed(const uint8_t* A, const void* B, float* D, uint32_t M, 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cut.parts, (M + kBM - 1) / kBM, (N + cut.tn - 1) / cut.tn);
     cfg.blockDim = dim3(kCutThreads, 1, 1);
-    // the sums take the place of the stages and, where they are more, of raw blocks
     const uint32_t rings = g.stages * stage + g.raw_slots * R::kSlot;
     cfg.dynamicSmemBytes = rings + kCutBars + 1024;
     cfg.stream = s;

@@ -60,7 +60,12 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 
 // Iteration limit of every mbarrier wait: a waiter that reaches it records an error status and leaves
 // its loop instead of spinning forever (each failed try_wait already suspends for a while).
+#ifdef ZC_WAIT_LIMIT
+#define kWaitLimit ZC_WAIT_LIMIT  // a test's, whose waits run out
+#else
 constexpr uint32_t kWaitLimit = 1u << 22;
+#endif
+constexpr uint32_t kDrainLimit = 1u << 22;  // of what ends by itself: copies and MMAs in flight when a wait has given up
 
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
     uint32_t v;
