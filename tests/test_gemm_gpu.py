@@ -404,11 +404,13 @@ def test_mul_mm_cut_in_every_form(gpu):
     run_cpp("test_cut")
 
 
-# Shapes that K is cut for over 1, 2, 4, 6, 10 and 16 CTAs and whole tiles; tokens on both sides of a tile's 192 and of 16, one block of K,
-# rows on both sides of 8 and 128 (Q6_K: boxes of every eighth row), rows of D that start anywhere and at 16 bytes only
+# Shapes that the rule cuts K of over 1, 2, 4, 6, 8, 10 and 16 CTAs (148 SMs; every form by itself: the test above); tokens on both sides
+# of a tile's 192 and of 16, one block of K, rows on both sides of 8 and 128 (Q6_K: boxes of every eighth row), rows of D that start
+# anywhere and at 16 bytes only
 @pytest.mark.parametrize("t,M,N,K", [(t, *s) for t in (zb.Q4_K, zb.Q6_K) for s in
                                      ((1, 16, 256), (127, 17, 512), (130, 192, 1024), (263, 193, 2560), (1024, 77, 4096), (1027, 385, 768),
-                                      (300, 40, 11520), (641, 209, 3328), (2050, 31, 1280), (515, 1500, 256))])
+                                      (300, 40, 11520), (641, 209, 3328), (2050, 31, 1280), (515, 1500, 256),
+                                      (1743, 378, 3072), (1152, 130, 2560))])
 @pytest.mark.parametrize("pad_b,pad_d,d_off", [(0, 0, 0), (8, 3, 1), (24, 4, 4)])
 def test_mul_mm_cut(gpu, oracle, t, M, N, K, pad_b, pad_d, d_off):
     torch, ctx, dd = gpu
