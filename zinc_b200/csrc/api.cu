@@ -1148,7 +1148,7 @@ int32_t zc_dmmv_batch(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size
     // Y[c][M] is D column-major with stride M, X[c][K] is B with stride K
     if (!small && num_cols >= 2 && mul_mm_exact_eligible(type, u8(A, a_offset), M, num_cols, K)) {
         const ExactGemm p{type, u8(A, a_offset), f32p(X, x_offset), f32m(Y, y_offset), M, num_cols, K, K, M,
-                          false, true, ctx->status_dev};
+                          false, true, ctx->status_dev, (uint32_t)ctx->sm_count};
         e = run_mul_mm_exact(ctx, p);
     }
     if (e == cudaErrorNotSupported)
@@ -1184,7 +1184,7 @@ int32_t zc_mul_mm(zc_ctx* ctx, uint32_t type, const void* A, uint64_t a_size, co
         });
     if (e == cudaErrorNotSupported && mul_mm_exact_eligible(type, u8(A, a_offset), M, N, K)) {
         const ExactGemm p{type, u8(A, a_offset), Bp, f32m(D, d_offset * 4), M, N, K, stride_b, stride_d,
-                          act_type == ZC_BF16, false, ctx->status_dev};
+                          act_type == ZC_BF16, false, ctx->status_dev, (uint32_t)ctx->sm_count};
         e = run_mul_mm_exact(ctx, p);
     }
     if (e == cudaErrorNotSupported)

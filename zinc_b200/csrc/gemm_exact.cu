@@ -17,6 +17,7 @@ struct PrepArgs {
     float* inv_scale;   // [N]
     float* D;           // zeroed where tiles lie on two CTA pairs
     uint32_t tokens, K, nblk, M, stride_b, stride_d;
+    uint32_t sms;
     bool sums_on, zero, vec;
 };
 
@@ -185,7 +186,7 @@ cudaError_t launch_prep(const void* args, bool zero, cudaStream_t s) {
     // a whole row in the threads' registers where there are few tokens; beyond two CTAs to an SM the second read costs less than
     // the occupancy (Q5_K 407 x 10752, 1268 tokens: the whole product 61.6 us with 1024 threads, 49.2 with 256)
     uint32_t threads = 256;
-    while (a.tokens <= 2 * 148 && threads < kPrepMost && threads < a.nblk * 16) threads *= 2;
+    while (a.tokens <= 2 * a.sms && threads < kPrepMost && threads < a.nblk * 16) threads *= 2;
     return launch_chained(a.vec ? exact_prep_kernel<ORDER, BF16, true> : exact_prep_kernel<ORDER, BF16, false>, dim3(a.tokens), dim3(threads), 0, s, a);
 }
 
@@ -265,20 +266,25 @@ static uint32_t equal_tiles(uint32_t N, uint32_t cols) { return ((N + cols - 1) 
 // idle; which of them wins depends on the shape, so every width's cost is estimated. 110 shapes (types, 96 to 2048 tokens, K to
 // 11 Ki): the widths it picks take 1 % more than the best of each shape in the mean, the widest ones 5 %.
 // 4096 x 4096, 512 tokens: 256 40.7 us, 176 42.7; 892 x 3072, 287 tokens: 96 17.2, 144 18.5.
+static uint64_t width_cost(const ExactGemm& p, uint32_t w, uint32_t n_row_pairs, uint32_t nblk) {
+    const uint32_t tiles = n_row_pairs * ((p.N + w - 1) / w), pairs = p.sms > 1 ? p.sms / 2 : 1;
+    const XCost c = x_cost(p, p.type == T_Q6_K || p.type == T_Q8_0, w);
+    const XDeal d = x_deal(tiles, w, nblk, pairs, c);
+    const uint64_t blocks = ((uint64_t)tiles * nblk + d.pairs - 1) / d.pairs;
+    uint64_t cost = blocks * c.block + c.epilogue;
+    if (d.groups) cost += c.epilogue;
+    else if (tiles >= pairs) cost += c.epilogue * tiles / pairs;
+    if (tiles * nblk % d.pairs != 0 || d.groups || d.per == 2) cost += c.zero;
+    return cost;
+}
 static uint32_t tile_width(const ExactGemm& p, uint32_t n_row_pairs, uint32_t nblk) {
-    const uint32_t least = (p.N + 255) / 256, pairs = 74;
+    const uint32_t least = (p.N + 255) / 256;
     uint32_t best = 0;
     uint64_t best_cost = ~0ull;
     for (uint32_t cols = least; cols <= 2 * least + 4; ++cols) {
-        const uint32_t w = equal_tiles(p.N, cols), tiles = n_row_pairs * ((p.N + w - 1) / w);
+        const uint32_t w = equal_tiles(p.N, cols);
         if (best && w < 48) break;
-        const XCost c = x_cost(p, p.type == T_Q6_K || p.type == T_Q8_0, w);
-        const XDeal d = x_deal(tiles, w, nblk, pairs, c);
-        const uint64_t blocks = ((uint64_t)tiles * nblk + d.pairs - 1) / d.pairs;
-        uint64_t cost = blocks * c.block + c.epilogue;
-        if (d.groups) cost += c.epilogue;
-        else if (tiles >= pairs) cost += c.epilogue * tiles / pairs;
-        if (tiles * nblk % d.pairs != 0 || d.groups || d.per == 2) cost += c.zero;
+        const uint64_t cost = width_cost(p, w, n_row_pairs, nblk);
         if (cost < best_cost) {
             best_cost = cost;
             best = w;
@@ -324,6 +330,7 @@ cudaError_t launch_mul_mm_exact(const ExactGemm& whole, uint8_t* scratch, cudaSt
         a.M = p.M;
         a.stride_b = p.stride_b;
         a.stride_d = p.stride_d;
+        a.sms = p.sms;
         a.sums_on = min_type;
         a.vec = ((p.stride_b | p.K) & 3u) == 0 && (reinterpret_cast<uintptr_t>(p.B) & (p.bf16 ? 7u : 15u)) == 0;
         const int order = min_type ? 0 : p.type == T_MXFP4 ? 2 : 1;

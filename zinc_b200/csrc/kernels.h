@@ -340,6 +340,7 @@ struct ExactGemm {
     bool bf16;
     bool fine;         // short accumulations: as near to the exact result as f32 sums by lanes (zc_dmmv_batch)
     uint32_t* status;
+    uint32_t sms;      // of the device
 };
 struct XPlan {
     uint32_t nblk, n_row_pairs, n_tiles, n_tile;
