@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 
@@ -57,6 +58,22 @@ def stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def check_registers(log: str) -> int:
+    """Raises where a kernel of the f32-accurate GEMM got another number of registers than gemm_exact.cuh counts on: the launch would be
+    refused then (its promoting warps would wait for registers that nobody gives back), and the product left to a kernel some thirty
+    times slower. Returns the number of kernels."""
+    with open(os.path.join(CSRC, "gemm_exact.cuh")) as f:
+        widest, few, many = map(int, re.search(r"kLaunchRegs = BN <= (\d+) \? (\d+) : (\d+)", f.read()).groups())
+    found = re.findall(r"entry function '(\w*gemm_exact_kernelILi\d+ELi(\d+)E\w*)'(?:(?!entry function).)*?Used (\d+) registers", log, re.S)
+    for name, width, used in found:
+        want = few if int(width) <= widest else many
+        if int(used) != want:
+            raise RuntimeError(f"{name}: {used} registers, not {want}")
+    if not found:
+        raise RuntimeError("no kernel of the f32-accurate GEMM among the compiled ones")
+    return len(found)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu into objects (in parallel) and link the shared library."""
     if not force and not stale():
@@ -90,6 +107,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         f.write("\n".join(log))
     if verbose:
         print("\n".join(log))
+    check_registers("\n".join(log))
     subprocess.check_call([nvcc, "-shared", "-o", SO, *objs, "-gencode", "arch=compute_100a,code=sm_100a"])
     return SO
 

@@ -1002,7 +1002,8 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
     cfg.numAttrs = 1;
     const int pairs = max_pairs_of(kern, cfg, max_pairs);
     if (pairs < 1) return cudaErrorNotSupported;
-    // the promoters wait for registers that the others give back: the sum is that of T's static_assert
+    // the promoters wait for registers that the others give back: the sum is that of T's static_assert (the build fails where a kernel
+    // got another number: build.py)
     static const bool registers = [&] {
         cudaFuncAttributes fa{};
         return cudaFuncGetAttributes(&fa, kern) == cudaSuccess && fa.numRegs == T::kLaunchRegs;
