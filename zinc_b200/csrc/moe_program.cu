@@ -828,7 +828,6 @@ bool lay_out(const MoeShape& s, int sm_count, MoeProgram& p) {
     p.E = s.E;
     p.k = s.k;
     p.slots = s.slots;
-    p.shared = s.shared;
     p.rule = s.rule;
     p.act = s.act;
     p.H = s.H;
