@@ -111,6 +111,65 @@ def test_layers_whose_calls_hold_f32_stay_launches(gpu, H, E, k, F):
     assert rel_l2(got["hidden"][:H].cpu().numpy(), eager["hidden"][:H].cpu().numpy()) <= 5e-7
 
 
+NAN, INF = float("nan"), float("inf")
+
+
+def logits_of(kind, E):
+    """Router logits at the edges of a selection; what is not named is 0.5."""
+    v = [0.5] * E
+    named = {"all the same": {}, "two levels": {i: 1.5 for i in range(3, E, 7)}, "negative zero": {i: -0.0 if i % 2 else 0.0 for i in range(E)},
+             "some NaN": {0: NAN, 5: NAN, 33: 2.0, E - 1: NAN}, "all NaN": {i: NAN for i in range(E)},
+             "one infinity": {40: INF, 7: 1.0}, "two infinities": {40: INF, 7: INF}, "nearly all out": {i: -INF for i in range(E) if i not in (9, E - 2)},
+             "all out": {i: -INF for i in range(E)}, "lowest": {i: -3.4028234663852886e38 for i in range(2, E)}}[kind]
+    for i, x in named.items():
+        v[i] = x
+    return v
+
+
+@pytest.mark.parametrize("kind", ["all the same", "two levels", "negative zero", "some NaN", "all NaN", "one infinity", "two infinities",
+                                  "nearly all out", "all out", "lowest"])
+@pytest.mark.parametrize("rule", [zb.ROUTE_SOFTMAX_ALL_RENORM, zb.ROUTE_TOPK_THEN_SOFTMAX])
+@pytest.mark.parametrize("E,k", [(96, 5), (250, 8)])
+def test_selections_at_the_edges(gpu, kind, rule, E, k):
+    """The joined kernel's selection against the router kernel's, on logits that the biases make exactly."""
+    torch, _, _ = gpu
+    s = shape("kquant", 1024, E, k, 512, 1)
+    s.rule = rule
+    r = Layers(torch, s)
+    w = r.step.layers[0]
+    w.router.zero_()
+    w.router_bias = torch.tensor(logits_of(kind, E), device="cuda")
+    torch.cuda.synchronize()
+    eager, got = r.eager_and_recorded(r.step.record, 1)
+    slots = k + 1
+    assert torch.equal(eager["routing"][:slots], got["routing"][:slots])
+    a, b = (v["routing"][slots:2 * slots].view(torch.float32) for v in (eager, got))
+    assert torch.allclose(a, b, rtol=1e-6, atol=0, equal_nan=True)  # the softmax's sum in another order
+    assert torch.allclose(eager["hidden"][:1024], got["hidden"][:1024], rtol=1e-4, atol=1e-5 * eager["hidden"][:1024].abs().max().item(), equal_nan=True)
+
+
+@pytest.mark.parametrize("arch,H,E,k,F", [("kquant", 1024, 64, 4, 512), ("mxfp4", 1088, 16, 2, 1024)])
+@pytest.mark.parametrize("odd", [NAN, INF, -INF, 3e38])
+def test_an_element_of_x_that_is_no_ordinary_number(gpu, arch, H, E, k, F, odd):
+    """What the calls make of it, the joined layer makes of it."""
+    torch, _, _ = gpu
+    r = Layers(torch, shape(arch, H, E, k, F, 1))
+    r.step.x = r.step.x.clone()
+    r.step.x[77] = odd
+    r.step.layers[0].router[:, 77] = 0.0 if odd == 3e38 else 1.0  # (finite: the selection does not hang on the order of a sum)
+    torch.cuda.synchronize()
+    eager, got = r.eager_and_recorded(r.step.record, 1)
+    assert torch.equal(eager["routing"][:k], got["routing"][:k])
+    # activations beyond 1e30 (an infinity among the K-quants' fixed point): whether the sums over them overflow hangs on their order
+    large = eager["act"][:r.sizes["act"]].abs().nan_to_num().max().item() > 1e30
+    for n in ("logits", "act") if large else ("logits", "act", "hidden"):
+        e, g = eager[n][:r.sizes[n]].double(), got[n][:r.sizes[n]].double()
+        ordinary = e.isfinite()
+        assert torch.equal(ordinary, g.isfinite()) and torch.equal(e.isnan(), g.isnan()), n
+        assert torch.equal(e[~ordinary & ~e.isnan()], g[~ordinary & ~e.isnan()]), n
+        assert rel_l2(g[ordinary].cpu().numpy(), e[ordinary].cpu().numpy()) <= 1e-5, n
+
+
 def test_a_long_run_is_several_kernels(gpu):
     torch, _, _ = gpu
     r = Layers(torch, shape("kquant", 1024, 64, 4, 512, 2), layers=170)   # 160 in a kernel
