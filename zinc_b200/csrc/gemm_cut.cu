@@ -14,6 +14,8 @@
 // columns 64 j .. of every block, a thread per row) and epilogue. Every mbarrier wait is bounded; a wait that gives up records {1, site},
 // raises the flag of all CTAs of the cluster, none of which adds its sums then, and every role drains to the common exit, where copies
 // and MMAs in flight are awaited and tensor memory is released.
+#include <cstddef>
+
 #include "kernels.h"
 #include "tc_common.cuh"
 
@@ -102,20 +104,11 @@ __global__ void __launch_bounds__(kCutThreads, 1) gemm_cut_kernel(const __grid_c
     const uint32_t part = blockIdx.x, m0 = blockIdx.y * kBM, n0 = blockIdx.z * g.tn;
     const int b0 = (int)(part * g.nblk / g.parts), nb = (int)((part + 1) * g.nblk / g.parts) - b0;
 
-    if (tid == 0) {
-        for (uint32_t s = 0; s < kCutMaxStages; ++s) {
-            mbar_init(&bars->full[s], 8);
-            mbar_init(&bars->full_x[s], 1);
-            mbar_init(&bars->empty[s], 1);
-        }
-        for (int s = 0; s < 4; ++s) {
-            mbar_init(&bars->full_w[0][s], 1);
-            mbar_init(&bars->full_w[1][s], 1);
-            mbar_init(&bars->empty_w[s], 16);
-        }
-        mbar_init(&bars->accum, 1);
-        mbar_init(&bars->drained, 1);
-        bars->failed = 0;
+    if (tid < (int)(offsetof(CutBars, tmem_base) / 8)) {  // a thread each
+        static_assert(offsetof(CutBars, tmem_base) / 8 <= 32, "by the warp that goes on to the allocation");
+        constexpr int kEmptyW = offsetof(CutBars, empty_w) / 8;
+        mbar_init(bars->full + tid, tid < (int)kCutMaxStages ? 8u : tid >= kEmptyW && tid < kEmptyW + 4 ? 16u : 1u);
+        if (tid == 0) bars->failed = 0;
         mbar_fence_init();
     }
     if (warp == 0) {
