@@ -1070,8 +1070,7 @@ cudaError_t x_launch(const ExactGemm& p, const XPlan& plan, const ExactPrep& pre
 template <int TYPE, bool kFetch>
 cudaError_t x_launch_bn(const ExactGemm& p, const XPlan& plan, const ExactPrep& prep, cudaStream_t s) {
     if (p.fine) {
-        // Two-term types: with one stage per set (tiles above 64 tokens) the second half of a block could be filled only after
-        // the first two runs' accumulators, which the filling warps give back later, are free again: not beyond 64.
+        // Two-term types: tiles of at most 64 tokens, whose sets have two stages, a fill of a block each.
         if constexpr (XW<TYPE>::kTerms == 1) {
             if (plan.n_tile > 64) return x_launch<TYPE, 128, kFetch, 4>(p, plan, prep, s);
         }

@@ -9,9 +9,10 @@
 // The warps have roles: one requests weights as soon as a layer's experts are known, across the layers' borders; three do the routing, up
 // to two layers ahead (where x is not what the layer before adds to), so that the next layer's weights are under way before it begins;
 // sixteen compute.
-// Measured (launches / this kernel): 40 layers of the first kind 783 / 405 us, 24 of the second 918 / 506; the same with each layer's x
-// what the one before added to 780 / 700 and 912 / 750; single layers with another kernel before each 21.0 / 20.8 and 39.7 / 32.4, of
-// six other shapes 0 to 21 % less: so every layer is joined, whatever is around it.
+// Measured (launches / this kernel): 40 layers of the first kind 780 / 403 us, 24 of the second 886 / 511; the same with each layer's x
+// what the one before added to 769 / 699 and 906 / 763; single layers behind a kernel that makes their x 21.3 / 20.5 and 41.4 / 35.4,
+// of 15 other shapes between 4 % more and 24 % less, K-quants 4 % less in the mean, with no rule found that tells them apart: so every
+// layer is joined, whatever is around it.
 // Bound: for the first kind by the exchange of the activations (half of a layer: 0.5 us until the last word is seen, 2 until they are
 // converted) and by the latency of one unit per warp; for MXFP4 by the instructions of the dot product. What it took: polls of one
 // word per tile instead of all words (12.1 -> 10 us and 27.8 -> 26.3 a layer), code that is not unrolled (26.3 -> 23.4), conversion
@@ -700,7 +701,7 @@ __device__ void compute(const MoeProgram& p, Sync* s, uint8_t* smem, uint32_t ba
         const GateUpRow gu = gate_up_row<GU>(p, s, l, tid);
         dots<GU, false>(p, s, first, ring, ring + p.at_table + (l & 1) * p.table_bytes, zeros, parts_g, warp, lane);
         // One table: the other CTA has read its own before this one writes there (collect()). For all warps by the barrier, in one warp:
-        // 24 layers of 2880 505 -> 509 us; each warp waiting ahead of its first store 528, a warp of its own for it (fewer registers) 541.
+        // 24 layers of 2880 508 -> 511 us; each warp waiting ahead of its first store 528, a warp of its own for it (fewer registers) 541.
         if (p.act_step == 0 && l > 0 && warp == kWarps - 1) {
             wait_pair(p, s, &s->read, (l - 1) & 1, 220);
             __syncwarp();
@@ -871,7 +872,7 @@ bool lay_out(const MoeShape& s, int sm_count, MoeProgram& p) {
     if (fixed + kMinRing * p.place_bytes > kMoeSmem) return false;
     auto ring = [&](uint32_t taken) { return taken > kMoeSmem ? 0u : std::min(kMaxRing, (kMoeSmem - taken) / p.place_bytes); };
     p.ring = ring(fixed);
-    // a second table where the ring stays as long: 40 layers of 256 experts take 400 us with it, 414 with one table; the MXFP4 layers of
+    // a second table where the ring stays as long: 40 layers of 256 experts take 403 us with it, 414 with one table; the MXFP4 layers of
     // 2880, whose ring it would take from 25 places to 15, 622 and 509
     p.act_step = ring(fixed + act_bytes) == p.ring ? act_bytes : 0;
     bool exact = true;
